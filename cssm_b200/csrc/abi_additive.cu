@@ -7,7 +7,7 @@
 // z planes); this file adds the gate-map kernel and the sequencing.
 #include <string.h>
 #include "kernels.cuh"
-#include "gemm_simt.cuh"
+#include "gemm.cuh"
 
 namespace cssm {
 

@@ -7,7 +7,7 @@
 // routines (any H, W).  A_t and U_t are never materialised.
 #include <string.h>
 #include "kernels.cuh"
-#include "gemm_simt.cuh"
+#include "gemm.cuh"
 #include "generic_dft.cuh"
 
 namespace cssm {

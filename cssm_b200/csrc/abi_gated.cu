@@ -3,7 +3,7 @@
 #include <stdio.h>
 #include <cuda_bf16.h>
 #include "kernels.cuh"
-#include "gemm_simt.cuh"
+#include "gemm.cuh"
 
 namespace cssm {
 

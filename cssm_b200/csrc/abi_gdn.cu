@@ -1,7 +1,7 @@
 // extern "C" entry points of the GDN (GatedDeltaNetCSSM) block.
 #include <string.h>
 #include "kernels.cuh"
-#include "gemm_simt.cuh"
+#include "gemm.cuh"
 
 namespace cssm {
 

@@ -2,7 +2,7 @@
 // S_t = K_hat S_{t-1} + X_hat_t, irfft2, out_proj, minus the input (src/models/cssm.py:6101-6175).
 #include <string.h>
 #include "kernels.cuh"
-#include "gemm_simt.cuh"
+#include "gemm.cuh"
 
 namespace cssm {
 

@@ -62,6 +62,21 @@ __device__ __forceinline__ float rcp_fast(float d) {
 __device__ __forceinline__ float silu_f(float v) { return v * rcp_fast(1.0f + __expf(-v)); }
 __device__ __forceinline__ float sigmoid_f(float v) { return rcp_fast(1.0f + __expf(-v)); }
 
+// n / d for 0 <= n < 2^31 by one multiply-high: d's rounded-up reciprocal, 2^l >= d.
+struct FastDiv {
+  uint32_t mul, shift, one;
+  FastDiv() = default;
+  explicit FastDiv(int d) {
+    shift = 0;
+    while ((1u << shift) < (uint32_t)d) ++shift;
+    mul = (uint32_t)((((uint64_t)1 << 32) * (((uint64_t)1 << shift) - (uint64_t)d)) / (uint64_t)d + 1);
+    one = d == 1 ? 1 : 0;
+  }
+  __device__ __forceinline__ int div(int n) const {
+    return one ? n : (int)((__umulhi((uint32_t)n, mul) + (uint32_t)n) >> shift);
+  }
+};
+
 // Host-side record of the last CUDA error seen on this thread.
 void set_cuda_error(cudaError_t e);
 int check_launch();

@@ -1,0 +1,600 @@
+// tcgen05 / TMEM GEMM of the float32 channel projections, any K, N and plane size.
+//
+// Every float32 operand is split into three bfloat16 parts, x = x0 + x1 + x2 (8 significant bits
+// each: the sum is exact to float32's own 24), and the product is taken as the six partial products
+// whose weight reaches 2^-16 of the leading one (00, 01, 10, 11, 02, 20), accumulated in float32 in
+// TMEM.  What is dropped is below 2^-24 of |a||b|.  A bf16 MMA runs at twice the tf32 rate, so six of them
+// cost what three tf32 passes cost, in three quarters of the shared memory.  The accumulator truncates
+// at every MMA, so with more than one K block the 00 products have an accumulator of their own and the
+// five small ones another (24 truncations of the full sum at K = 384 instead of 144: relative error 2.2e-6 before).
+//
+// Persistent kernel, one CTA per SM, 544 threads, warp-specialised:
+//   warps 0-7  producers : 128-row x 64-k A blocks from global memory (channels-last rows with RoPE
+//                          applied, or planar planes times scale and gate), fetched one block ahead
+//                          into registers, split, and written into the 128-byte-swizzled K-major
+//                          operand layout of the ring; with streamed weights also the B blocks;
+//   warp  8    MMA issuer: one lane issues 6 x (K block / 16) tcgen05.mma per block into one of two
+//                          TMEM accumulators and commits to mbarriers;
+//   warps 9-16 epilogue  : tcgen05.ld (lane = pixel row; two warps per TMEM lane quadrant, half of the
+//                          32-column chunks each), 1/rms, bias, activation; planar stores (coalesced
+//                          over pixels) or channels-last rows through a per-warp TMA tensor store.
+// RES: the whole (K, BN) weight tile is split once per CTA and stays in shared memory (the ring then
+// carries A only); without it the producers split the weight block of every stage again.
+// Rows are flat pixels m = frame * HW + px, so a tile may cross frames and HW may be anything.
+// Every mbarrier wait is bounded; on expiry the kernel records an error code and winds down.
+//
+// Bound: the producers (about 300 instructions a thread and tile, twice that with RoPE; a clock trace of
+// one CTA shows the MMA warp waiting for them), not memory: at K = 64 it reaches 0.6 of the HBM rate.
+// Against the CUDA-core GEMM that covered these sizes before (batch x frames, plane, channels):
+// in_proj 48 x 8 x 14^2, 256 -> 512: 884 -> 211 us; in_proj + B_k/B_v + qkv of 12 x 8 x 28^2, 64: 271 -> 56 us;
+// out_proj 33 x 16^2, 256 -> 256: 121 -> 36 us; 16 x 8 x 56^2, 32 -> 64: 150 -> 67 us, 32 -> 32: 134 -> 37 us.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <string.h>
+#include "kernels.cuh"
+#include "gemm.cuh"
+#include "tc05.cuh"
+
+namespace cssm {
+
+__device__ int g_split_error = 0;
+
+// 8 producer warps, 1 MMA warp, 8 epilogue warps (with 16 producer warps 72 registers a thread are left
+// and the kernel is slower throughout).
+constexpr int GS_PROD = 256;
+constexpr int GS_THREADS = GS_PROD + 32 + 256;
+constexpr int GS_MMA_WARP = GS_PROD / 32;
+constexpr int GS_BM = 128, GS_BK = 64;
+constexpr uint32_t GS_A_PART = GS_BM * 128u;           // one bf16 part of an A block
+constexpr uint32_t GS_A_BYTES = 3u * GS_A_PART;
+constexpr int GS_SS = 8;             // row-sum buffers (producers run at most five tiles ahead of the epilogue)
+
+// streaming loads that leave the L1 (a few KB beside the shared memory in use) to the RoPE tables
+__device__ __forceinline__ void ld_stream4(const float* p, float* v) {
+  asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
+}
+
+template <int V> struct Int { static constexpr int value = V; };
+
+struct SplitGeom {
+  int BN, n_tiles, m_tiles, kblocks, stages;
+  int corr;                           // 1: separate accumulator for the small partial products
+  FastDiv hw, w, t, fdiv;             // divisions by HW, W, T and the source-frame divisor
+};
+
+// x -> three bf16 parts for a pair of values, packed (low half = first value)
+__device__ __forceinline__ void split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p0) : "f"(y), "f"(x));
+  const cf r = mk(x, y) - mk(__uint_as_float(p0 << 16), __uint_as_float(p0 & 0xffff0000u));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1) : "f"(r.y), "f"(r.x));
+  const cf u = r - mk(__uint_as_float(p1 << 16), __uint_as_float(p1 & 0xffff0000u));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p2) : "f"(u.y), "f"(u.x));
+}
+// eight consecutive k values -> one 16-byte chunk in each of the three parts
+__device__ __forceinline__ void store_split8(unsigned char* base, uint32_t off, uint32_t part, const float (&v)[8]) {
+  uint4 a, b, c;
+  split3(v[0], v[1], a.x, b.x, c.x);
+  split3(v[2], v[3], a.y, b.y, c.y);
+  split3(v[4], v[5], a.z, b.z, c.z);
+  split3(v[6], v[7], a.w, b.w, c.w);
+  *reinterpret_cast<uint4*>(base + off) = a;
+  *reinterpret_cast<uint4*>(base + part + off) = b;
+  *reinterpret_cast<uint4*>(base + 2 * part + off) = c;
+}
+__device__ __forceinline__ uint32_t idesc_bf16_f32(uint32_t M, uint32_t N) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
+}
+// issued by the lanes with lead != 0 (one of the warp)
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                        uint32_t accumulate, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, l;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 l, %5, 0;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+}
+
+// GATE: planar A times the gate planes.
+template <bool A_PLANAR, bool RES, bool GATE>
+__global__ void __launch_bounds__(GS_THREADS, 1)
+gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ CUtensorMap omap) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  // operand tiles need 1024-byte alignment (swizzle atoms); the launch adds 1024 bytes of slack
+  unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
+  const uint32_t sbase = tc::smem_u32(smem);
+  const uint32_t BN = (uint32_t)q.BN, b_part = BN * 128u, b_block = 3u * b_part;
+  const int NS = q.stages, kblocks = q.kblocks;
+  const uint32_t res_bytes = RES ? (uint32_t)kblocks * b_block : 0u;
+  const uint32_t stage_bytes = GS_A_BYTES + (RES ? 0u : b_block);
+  unsigned char* ring = smem + res_bytes;
+  unsigned char* stg = ring + (uint32_t)NS * stage_bytes;         // 8 x 4 KB when the output is channels-last
+  float* bias_s = reinterpret_cast<float*>(stg + (A_PLANAR ? 8u * 4096u : 0u));
+  float* ss_s = bias_s + 256;                                     // [GS_SS][2][128] row sums (RMS prologue)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ss_s + (A_PLANAR ? GS_SS * 256 : 0));
+  uint64_t* full = bars;           // [4] block written (8 producer warps)
+  uint64_t* empty = bars + 4;      // [4] block consumed (tcgen05.commit)
+  uint64_t* accfull = bars + 8;    // [2] accumulator complete (tcgen05.commit)
+  uint64_t* accempty = bars + 10;  // [2] accumulator drained (8 epilogue warps)
+  uint64_t* done = bars + 12;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int num_tiles = q.m_tiles * q.n_tiles;
+  const uint32_t acc_cols = q.corr ? 2u * BN : BN;                // TMEM columns of one accumulator (pair)
+  uint32_t tmem_cols = 32;
+  while (tmem_cols < 2u * acc_cols) tmem_cols <<= 1;
+
+  if (tid == 0) {
+    for (int s = 0; s < NS; ++s) { tc::mbar_init(&full[s], GS_PROD / 32); tc::mbar_init(&empty[s], 1); }
+    for (int a = 0; a < 2; ++a) { tc::mbar_init(&accfull[a], 1); tc::mbar_init(&accempty[a], 8); }
+    tc::mbar_init(done, 1);
+    tc::fence_mbar_init();
+  }
+  if (warp == GS_MMA_WARP) {
+    tc::tmem_alloc(tmem_slot, tmem_cols);
+    tc::tmem_relinquish();
+  }
+  // one 8-k chunk of weight row n (columns of the (K, N) matrix), zero outside the matrix
+  auto load_w8 = [&](int n, int k0, float (&v)[8]) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int k = k0 + e;
+      float w = (n < g.N && k < g.K) ? __ldg(g.Wk + (size_t)k * g.N + n) : 0.f;
+      if (A_PLANAR && g.rms_scale != nullptr && k < g.K) w *= __ldg(g.rms_scale + k);
+      v[e] = w;
+    }
+  };
+  const int n_first = (blockIdx.x % q.n_tiles) * q.BN;            // RES: the N tile of this CTA
+  if (RES) {
+    for (int item = tid; item < q.BN * kblocks * 8; item += GS_THREADS) {
+      const int n = item % q.BN, ck = item / q.BN;                // ck: 8-k chunk over all K blocks
+      float v[8];
+      load_w8(n_first + n, ck * 8, v);
+      store_split8(smem + (uint32_t)(ck >> 3) * b_block, tc::sw128_offset(n, ck & 7), b_part, v);
+    }
+    for (int n = tid; n < q.BN; n += GS_THREADS) bias_s[n] = (g.bias && n_first + n < g.N) ? g.bias[n_first + n] : 0.f;
+  }
+  tc::fence_proxy_async();
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp < GS_MMA_WARP) {
+    // ================================ producers ================================
+    // channels-last: item i of a thread is the 4-k chunk (lane & 7) + 8 (i >> 2) of row prow0 + 32 (i & 3), so
+    // a warp load covers four rows x 128 contiguous bytes.  Most RoPE modes rotate the low channel pairs
+    // only: with this order they are the first half of the items of six lanes in eight, not all items of
+    // three.  The four rows of a warp are four apart, which keeps its 8-byte stores free of conflicts.
+    // planar: thread = (pixel row tid & 127, k half tid >> 7).
+    float pre[32], gpre[GATE ? 32 : 1];
+    const int chunk = lane & 7, prow0 = (lane >> 3) * 4 + (warp & 3) + 16 * (warp >> 2);
+    // the lane's two chunks inside a part, rows prow0 (+ 32 r)
+    const uint32_t dst0 = tc::sw128_offset(prow0, chunk >> 1) + (chunk & 1) * 8;
+    const uint32_t dst1 = tc::sw128_offset(prow0, (chunk >> 1) + 4) + (chunk & 1) * 8;
+    const int prow = tid & 127, kh = tid >> 7;
+    const bool rope = !A_PLANAR && g.rope_t != nullptr;
+    const bool remap = g.a_fmul != 0 || g.a_fadd != 0;
+    auto fetch = [&](int tile, int kb) {
+      const int m0 = (tile / q.n_tiles) * GS_BM, k0 = kb * GS_BK;
+      if constexpr (!A_PLANAR) {
+        if (!remap && m0 + GS_BM <= g.M && k0 + GS_BK <= g.K) {      // whole block, rows one after another
+          const float* p = g.A + (size_t)(m0 + prow0) * g.K + k0 + chunk * 4;
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            ld_stream4(p, pre + 4 * r);
+            ld_stream4(p + 32, pre + 16 + 4 * r);
+            p += 32 * g.K;
+          }
+          return;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const int m = m0 + prow0 + 32 * r;
+          size_t row = (size_t)m;
+          if (remap) {
+            const int fo = q.hw.div(m);
+            row = (size_t)(q.fdiv.div(fo) * g.a_fmul + g.a_fadd) * g.HW + (m - fo * g.HW);
+          }
+          const float* p = g.A + row * g.K + k0 + chunk * 4;
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            float* v = pre + 16 * hf + 4 * r;
+            if (m < g.M && k0 + (chunk + 8 * hf) * 4 < g.K) ld_stream4(p + 32 * hf, v);
+            else v[0] = v[1] = v[2] = v[3] = 0.f;
+          }
+        }
+      } else {
+        const int m = m0 + prow, kk = k0 + kh * 32;
+        const int nk = m < g.M ? g.K - kk : 0;             // valid k values from kk on
+        const int fo = q.hw.div(min(m, g.M - 1)), px = min(m, g.M - 1) - fo * g.HW;
+        const int fr = remap ? q.fdiv.div(fo) * g.a_fmul + g.a_fadd : fo;
+        const float* ap = g.A + ((size_t)fr * g.a_planes + g.a_plane0 + kk) * g.HW + px;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) pre[j] = j < nk ? __ldg(ap + (size_t)j * g.HW) : 0.f;
+        if constexpr (GATE) {
+          const float* gp = g.gate + ((size_t)(g.g_compact ? fo : fr) * g.g_planes + g.g_plane0 + kk) * g.HW + px;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) gpre[j] = j < nk ? __ldg(gp + (size_t)j * g.HW) : 0.f;
+        }
+      }
+    };
+    int tile = blockIdx.x, kb = 0, it = 0, tcnt = 0, rot_kb = -1;
+    float ss = 0.f;
+    bool rot[2] = {false, false};       // this lane's chunk in either half of the block holds rotated pairs
+    if (tile < num_tiles) fetch(tile, 0);
+    while (tile < num_tiles) {
+      const int s = it % NS;
+      const int m0 = (tile / q.n_tiles) * GS_BM, k0 = kb * GS_BK;
+      int ntile = tile, nkb = kb + 1;
+      if (nkb == kblocks) { nkb = 0; ntile += gridDim.x; }
+      unsigned char* a_s = ring + (uint32_t)s * stage_bytes;
+      if constexpr (!A_PLANAR) {
+        if (rope && rot_kb != kb) {
+          rot_kb = kb;
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            const int k = k0 + (chunk + 8 * hf) * 4;
+            rot[hf] = k < g.K && (g.rope_nz == nullptr || __ldg(g.rope_nz + (k >> 1)) != 0.f ||
+                                  __ldg(g.rope_nz + (k >> 1) + 1) != 0.f);
+          }
+        }
+        if (rot[0] || rot[1]) {
+          const int n2 = g.K >> 1, pi = (k0 >> 1) + 2 * chunk;
+          const int fr0 = q.hw.div(m0), px0 = m0 - fr0 * g.HW;
+          const int t0 = g.rope_tlast ? g.T - 1 : fr0 - q.t.div(fr0) * g.T;
+          const bool crosses = px0 + GS_BM > g.HW;            // the tile runs into the next frame(s)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            int px = px0 + prow0 + 32 * r, t = t0;
+            if (crosses && px >= g.HW) {
+              const int m = min(m0 + prow0 + 32 * r, g.M - 1), fr = q.hw.div(m);
+              px = m - fr * g.HW;
+              if (!g.rope_tlast) t = fr - q.t.div(fr) * g.T;
+            }
+            const int h = q.w.div(px), w = px - h * g.W;
+            const float2* pt = g.rope_t + t * n2 + pi;
+            const float2* ph = g.rope_h + h * n2 + pi;
+            const float2* pw = g.rope_w + w * n2 + pi;
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+              if (!rot[hf]) continue;
+              // two pairs per 16-byte table load (K % 4 == 0)
+              const float4 ct = __ldg(reinterpret_cast<const float4*>(pt + 16 * hf));
+              const float4 ch = __ldg(reinterpret_cast<const float4*>(ph + 16 * hf));
+              const float4 cw = __ldg(reinterpret_cast<const float4*>(pw + 16 * hf));
+              float* x = pre + 16 * hf + 4 * r;
+              // (cos, sin) of the summed angle, then the rotation of one pair
+              auto turn = [](float tx, float ty, float hx, float hy, float wx, float wy, float& u, float& v) {
+                const float cx = tx * hx - ty * hy, sx = tx * hy + ty * hx;
+                const float c2 = cx * wx - sx * wy, s2 = cx * wy + sx * wx;
+                const float ne = u * c2 - v * s2, no = u * s2 + v * c2;
+                u = ne; v = no;
+              };
+              turn(ct.x, ct.y, ch.x, ch.y, cw.x, cw.y, x[0], x[1]);
+              turn(ct.z, ct.w, ch.z, ch.w, cw.z, cw.w, x[2], x[3]);
+            }
+          }
+        }
+        // warp-uniform exit: the lanes of a warp meet again at the __syncwarp before the arrive
+        if (__any_sync(0xffffffffu, !tc::mbar_wait(&empty[s], ((it / NS) & 1) ^ 1))) { atomicExch(&g_split_error, 1); break; }
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          unsigned char* dst = a_s + (hf ? dst1 : dst0);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const float* x = pre + 16 * hf + 4 * r;
+            uint2 a, b, c;
+            split3(x[0], x[1], a.x, b.x, c.x);
+            split3(x[2], x[3], a.y, b.y, c.y);
+            *reinterpret_cast<uint2*>(dst + r * 4096) = a;                       // 32 rows = 4096 bytes on
+            *reinterpret_cast<uint2*>(dst + r * 4096 + GS_A_PART) = b;
+            *reinterpret_cast<uint2*>(dst + r * 4096 + 2 * GS_A_PART) = c;
+          }
+        }
+        if (ntile < num_tiles) fetch(ntile, nkb);
+      } else {
+        if (g.rms_scale != nullptr) {
+          // the sum of squares of this part of the row; 1/rms is a row factor, applied to the accumulator
+#pragma unroll
+          for (int j = 0; j < 32; ++j) ss = fmaf(pre[j], pre[j], ss);
+        }
+        if (__any_sync(0xffffffffu, !tc::mbar_wait(&empty[s], ((it / NS) & 1) ^ 1))) { atomicExch(&g_split_error, 1); break; }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          float v[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = GATE ? pre[8 * c + e] * gpre[GATE ? 8 * c + e : 0] : pre[8 * c + e];
+          store_split8(a_s, tc::sw128_offset(prow, kh * 4 + c), GS_A_PART, v);
+        }
+        if (g.rms_scale != nullptr && nkb == 0) { ss_s[((tcnt % GS_SS) * 2 + kh) * 128 + prow] = ss; ss = 0.f; }
+        if (ntile < num_tiles) fetch(ntile, nkb);
+      }
+      if (!RES) {
+        unsigned char* b_s = a_s + GS_A_BYTES;
+        const int n0 = (tile % q.n_tiles) * q.BN;
+        for (int item = tid; item < q.BN * 8; item += GS_PROD) {
+          const int n = item % q.BN, c = item / q.BN;
+          float v[8];
+          load_w8(n0 + n, k0 + c * 8, v);
+          store_split8(b_s, tc::sw128_offset(n, c), b_part, v);
+        }
+      }
+      tc::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&full[s]);
+      if (nkb == 0) ++tcnt;
+      tile = ntile; kb = nkb; ++it;
+    }
+  } else if (warp == GS_MMA_WARP) {
+    // ================================ MMA issuer ================================
+    // The whole warp walks the loop and only the instruction itself is predicated on lane 0: in a
+    // one-lane branch the compiler has to move every descriptor into uniform registers again, and that
+    // set the pace (about 125 clocks an MMA).
+    const uint32_t idesc = idesc_bf16_f32(GS_BM, BN);
+    const uint32_t lead = lane == 0 ? 1u : 0u;
+    // (A part, B part) of the six partial products, smallest first
+    constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
+    int s = 0, sph = 0, ac = 0, aph = 1;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      if (!tc::mbar_wait(&accempty[ac], aph)) { atomicExch(&g_split_error, 2); ok = false; break; }
+      tc::fence_after_sync();
+      const uint32_t d = tmem_base + (uint32_t)ac * acc_cols;
+      for (int kb = 0; kb < kblocks; ++kb) {
+        if (!tc::mbar_wait(&full[s], sph)) { atomicExch(&g_split_error, 2); ok = false; break; }
+        tc::fence_after_sync();
+        const uint32_t a_s = sbase + res_bytes + (uint32_t)s * stage_bytes;
+        const uint32_t b_s = RES ? sbase + (uint32_t)kb * b_block : a_s + GS_A_BYTES;
+        const uint64_t ad0 = tc::make_desc_sw128(a_s), bd0 = tc::make_desc_sw128(b_s);
+        const uint64_t bp = (uint64_t)(b_part >> 4);
+        const uint64_t bd[3] = {bd0, bd0 + bp, bd0 + 2 * bp};
+        const uint32_t d00 = q.corr ? d + BN : d, first = kb == 0 ? 0u : 1u;
+        auto issue = [&](auto steps) {
+          constexpr int KS = decltype(steps)::value;
+#pragma unroll
+          for (int p = 0; p < 6; ++p)
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks)
+              mma_f16(p == 5 ? d00 : d, ad0 + PA[p] * (GS_A_PART >> 4) + ks * 2, bd[PB[p]] + ks * 2, idesc,
+                      p == 5 && ks == 0 ? (q.corr ? first : 1u) : (p | ks ? 1u : first), lead);
+        };
+        const int krem = g.K - kb * GS_BK;
+        if (krem > 48) issue(Int<4>());
+        else if (krem > 32) issue(Int<3>());
+        else if (krem > 16) issue(Int<2>());
+        else issue(Int<1>());
+        if (lane == 0) tc::commit(&empty[s]);
+        if (++s == NS) { s = 0; sph ^= 1; }
+      }
+      if (ok && lane == 0) tc::commit(&accfull[ac]);
+      if (ac == 1) aph ^= 1;
+      ac ^= 1;
+    }
+    // nothing of lane 0's tensor work may be in flight when TMEM is freed
+    if (lane == 0) tc::commit(done);
+    if (!tc::mbar_wait(done, 0) && ok) atomicExch(&g_split_error, 3);
+    __syncwarp();
+  } else {
+    // ================================ epilogue ================================
+    const int quad = warp & 3;                          // TMEM lane quadrant this warp may read
+    const int half = (warp - (GS_MMA_WARP + 1)) >> 2;   // even or odd 32-column chunks
+    const int row = quad * 32 + lane;
+    unsigned char* my_stg = stg + (uint32_t)(warp - (GS_MMA_WARP + 1)) * 4096u;
+    int tcnt = 0;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++tcnt) {
+      const int ac = tcnt & 1, ph = (tcnt >> 1) & 1;
+      const int m0 = (tile / q.n_tiles) * GS_BM, n0 = (tile % q.n_tiles) * q.BN;
+      const int m = m0 + row;
+      int fr = 0, px = 0;
+      bool zrow = true;                                 // this row's z columns are wanted
+      if (!A_PLANAR) {
+        fr = q.hw.div(min(m, g.M - 1)); px = m - fr * g.HW;
+        zrow = !g.z_last_only || fr - q.t.div(fr) * g.T == g.T - 1;
+      }
+      if (__any_sync(0xffffffffu, !tc::mbar_wait(&accfull[ac], ph))) { atomicExch(&g_split_error, 4); break; }
+      tc::fence_after_sync();
+      float rinv = 1.f;
+      if (A_PLANAR && g.rms_scale != nullptr) {
+        const float* sp = ss_s + (tcnt % GS_SS) * 256 + row;
+        rinv = rsqrtf((sp[0] + sp[128]) / (float)g.K + 1e-6f);
+      }
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)ac * acc_cols;
+#pragma unroll 1
+      for (int cc = half; cc * 32 < q.BN; cc += 2) {
+        const int n = n0 + cc * 32;
+        if (n >= g.N) break;
+        const bool zcols = n >= g.act_n0;               // all 32 columns are activated ones
+        if (!A_PLANAR && zcols && g.z_last_only && !__any_sync(0xffffffffu, zrow)) continue;
+        float v[32];
+        {
+          uint32_t r[32];
+          tc::ld_32x32b_x32(taddr + cc * 32, r);
+          tc::wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+        }
+        if (q.corr) {
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            uint32_t r[16];
+            tc::ld_32x32b_x16(taddr + BN + cc * 32 + hf * 16, r);
+            tc::wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[hf * 16 + j] += __uint_as_float(r[j]);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (RES) b = *reinterpret_cast<const float4*>(bias_s + cc * 32 + j);
+          else if (g.bias && n + j < g.N) b = __ldg(reinterpret_cast<const float4*>(g.bias + n + j));
+          v[j] = fmaf(v[j], rinv, b.x);         v[j + 1] = fmaf(v[j + 1], rinv, b.y);
+          v[j + 2] = fmaf(v[j + 2], rinv, b.z); v[j + 3] = fmaf(v[j + 3], rinv, b.w);
+        }
+        if (!A_PLANAR) {
+          if (g.out_act != 0 && n + 32 > g.act_n0) {
+            // (a branch on the kind inside the loops: 82 -> 137 us at K = 64, N = 128, 524 K rows)
+            if (!zcols) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                const float sg = sigmoid_f(v[j]);
+                if (n + j >= g.act_n0) v[j] = g.out_act == 1 ? v[j] * sg : sg;
+              }
+            } else if (g.out_act == 1) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = silu_f(v[j]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = sigmoid_f(v[j]);
+            }
+          }
+          // planar: lanes are consecutive pixels, so every column is a coalesced store
+          if (m < g.M) {
+            float* op = g.out + ((size_t)fr * g.o_planes + g.o_plane0 + n) * g.HW + px;
+            const int nw = zrow ? g.N - n : min(g.N, g.act_n0) - n;     // columns of this row to store
+            if (nw >= 32) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) op[(size_t)j * g.HW] = v[j];
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (j < nw) op[(size_t)j * g.HW] = v[j];
+            }
+          }
+        } else {
+          if (g.sub != nullptr && m < g.M) {
+            const float4* sp = reinterpret_cast<const float4*>(g.sub + (size_t)m * g.N + n);
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              if (n + j >= g.N) continue;
+              const float4 sv = __ldg(sp + (j >> 2));
+              v[j] -= sv.x; v[j + 1] -= sv.y; v[j + 2] -= sv.z; v[j + 3] -= sv.w;
+            }
+          }
+          // 32 rows x 32 columns in the 128-byte swizzle, one TMA store per warp; rows beyond M and
+          // columns beyond N are clipped by the tensor map
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(my_stg + tc::sw128_offset(lane, j >> 2)) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+          tc::fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            tc::tma_store_2d(&omap, my_stg, n, m0 + quad * 32);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        }
+      }
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&accempty[ac]);
+    }
+    // shared memory must outlive the last TMA stores that read it
+    if (A_PLANAR && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == GS_MMA_WARP) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem_base, tmem_cols);
+  }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                                  CUtensorMapFloatOOBfill);
+static EncodeTiledFn encode_fn() {
+  static EncodeTiledFn fn = []() -> EncodeTiledFn {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult qr;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qr) != cudaSuccess ||
+        qr != cudaDriverEntryPointSuccess)
+      return nullptr;
+    return reinterpret_cast<EncodeTiledFn>(p);
+  }();
+  return fn;
+}
+
+int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
+  if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.HW <= 0) return CSSM_ERR_DIMS;
+  if (g.K % 4 != 0 || g.N % 4 != 0) return CSSM_ERR_UNSUPPORTED;
+  SplitGeom q;
+  memset(&q, 0, sizeof(q));
+  q.kblocks = (g.K + GS_BK - 1) / GS_BK;
+  q.m_tiles = (g.M + GS_BM - 1) / GS_BM;
+  q.hw = FastDiv(g.HW); q.w = FastDiv(g.W > 0 ? g.W : 1); q.t = FastDiv(g.T > 0 ? g.T : 1);
+  q.fdiv = FastDiv(g.a_fdiv > 1 ? g.a_fdiv : 1);
+  constexpr size_t LIMIT = 227 * 1024;
+  const size_t fixed = 1024 + 1024 + 128 + (a_planar ? 8 * 4096 + GS_SS * 1024 : 0);   // slack, bias, barriers, staging, sums
+  auto round32 = [](int v) { return (v + 31) / 32 * 32; };
+  auto res_size = [&](int bn) { return (size_t)q.kblocks * 3 * bn * 128; };
+  // Weights resident when a tile of at least 64 columns (or all of N) leaves room for two A stages:
+  // every CTA then splits its weights once.  Otherwise 128-column tiles with the weights streamed.
+  q.corr = q.kblocks > 1 ? 1 : 0;
+  int nt = q.corr ? (g.N + 127) / 128 : (g.N + 255) / 256;
+  while (round32((g.N + nt - 1) / nt) > 32 && res_size(round32((g.N + nt - 1) / nt)) + 2 * GS_A_BYTES + fixed > LIMIT) ++nt;
+  q.BN = round32((g.N + nt - 1) / nt);
+  const bool res = (q.BN >= 64 || nt == 1) && res_size(q.BN) + 2 * GS_A_BYTES + fixed <= LIMIT;
+  if (!res) {
+    const int most = a_planar ? 96 : 128;
+    nt = (g.N + most - 1) / most;
+    q.BN = round32((g.N + nt - 1) / nt);
+  }
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  // few row tiles: narrower column tiles until two thirds of the SMs have one (each CTA then splits
+  // fewer weights too; the row tile is split once more per column tile, which idle SMs do for free)
+  for (int k = nt + 1; q.BN > 32 && q.m_tiles * ((g.N + q.BN - 1) / q.BN) * 3 < sms * 2; ++k)
+    q.BN = round32((g.N + k - 1) / k);
+  q.n_tiles = (g.N + q.BN - 1) / q.BN;
+  const size_t stage = GS_A_BYTES + (res ? 0 : (size_t)3 * q.BN * 128);
+  const size_t base = (res ? res_size(q.BN) : 0) + fixed;
+  q.stages = 4;
+  while (q.stages > 1 && base + q.stages * stage > LIMIT) --q.stages;
+  if (base + q.stages * stage > LIMIT) return CSSM_ERR_UNSUPPORTED;
+  const size_t smem = base + q.stages * stage;
+  const long long tiles = (long long)q.m_tiles * q.n_tiles;
+  if (tiles > 0x7fffffffLL) return CSSM_ERR_DIMS;
+  // a multiple of n_tiles, so that a CTA keeps one N tile (resident weights, bias)
+  int grid = (int)(tiles < sms ? tiles : sms);
+  if (res && grid > q.n_tiles) grid -= grid % q.n_tiles;
+  if (res && grid < q.n_tiles) return CSSM_ERR_UNSUPPORTED;
+  CUtensorMap map;
+  memset(&map, 0, sizeof(map));
+  if (a_planar) {
+    EncodeTiledFn enc = encode_fn();
+    const cuuint64_t dims[2] = {(cuuint64_t)g.N, (cuuint64_t)g.M}, strides[1] = {(cuuint64_t)g.N * 4};
+    const cuuint32_t box[2] = {32, 32}, es[2] = {1, 1};
+    if (enc == nullptr ||
+        enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, g.out, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return CSSM_ERR_CUDA;
+  }
+  const bool gate = g.gate != nullptr;
+  auto kern = a_planar ? (gate ? (res ? gemm_split_kernel<true, true, true> : gemm_split_kernel<true, false, true>)
+                               : (res ? gemm_split_kernel<true, true, false> : gemm_split_kernel<true, false, false>))
+                       : (res ? gemm_split_kernel<false, true, false> : gemm_split_kernel<false, false, false>);
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  kern<<<grid, GS_THREADS, smem, st>>>(g, q, map);
+  return check_launch();
+}
+
+int read_split_error(int* out, int clear) {
+  cudaError_t e = cudaMemcpyFromSymbol(out, g_split_error, sizeof(int));
+  if (e == cudaSuccess && clear && *out != 0) {
+    const int zero = 0;
+    e = cudaMemcpyToSymbol(g_split_error, &zero, sizeof(int));
+  }
+  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  return CSSM_OK;
+}
+
+}  // namespace cssm

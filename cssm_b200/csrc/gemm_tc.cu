@@ -4,8 +4,7 @@
 // Persistent kernel, one CTA per SM, 544 threads, warp-specialised:
 //   warps 0-7  producers : read a 128-pixel A tile from global memory (channels-last rows with
 //                          RoPE fused, loaded one tile ahead into registers so a whole tile is
-//                          in flight per SM; or planar planes with the RMSNorm/gate prologue
-//                          fused), split every value into tf32 hi + remainder, and
+//                          in flight per SM; or planar planes times gate planes), split every value into tf32 hi + remainder, and
 //                          write both into the 128-byte-swizzled K-major operand layout of a
 //                          2-stage ring;
 //   warp  8    MMA issuer: one lane issues 24 tcgen05.mma (M128 x N x K8) per tile into one of
@@ -18,12 +17,24 @@
 #include <cuda.h>
 #include <string.h>
 #include "kernels.cuh"
-#include "gemm_simt.cuh"
+#include "gemm.cuh"
 #include "tc05.cuh"
 
 namespace cssm {
 
 __device__ int g_tc_error = 0;
+
+__device__ inline int gemm_src_frame(const GemmArgs& g, int f) {
+  if (g.a_fmul == 0 && g.a_fadd == 0) return f;
+  return (g.a_fdiv > 1 ? f / g.a_fdiv : f) * g.a_fmul + g.a_fadd;
+}
+__device__ inline int gemm_rope_t(const GemmArgs& g, int f) { return g.rope_tlast ? g.T - 1 : f % g.T; }
+// channels-last A: source row of output row m
+__device__ inline size_t gemm_src_row(const GemmArgs& g, int m) {
+  if (g.a_fmul == 0 && g.a_fadd == 0) return (size_t)m;
+  const int fo = m / g.HW;
+  return (size_t)gemm_src_frame(g, fo) * g.HW + (m - fo * g.HW);
+}
 
 constexpr int TC_THREADS = 544;      // 8 producer warps, 1 MMA warp, 8 epilogue warps
 constexpr int TC_MMA_WARP = 8;
@@ -208,18 +219,6 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
           const float* ap = g.A + ((size_t)fr * g.a_planes + g.a_plane0 + kh * 32) * g.HW + px;
 #pragma unroll
           for (int k = 0; k < 32; ++k) v[k] = __ldg(ap + (size_t)k * g.HW);
-          if (g.rms_scale != nullptr) {
-            // the other K half of the row is re-read (cache hit: the partner thread loads it)
-            const float* op = g.A + ((size_t)fr * g.a_planes + g.a_plane0 + (1 - kh) * 32) * g.HW + px;
-            float ss = 0.f;
-#pragma unroll
-            for (int k = 0; k < 32; ++k) { const float o = op[(size_t)k * g.HW]; ss = fmaf(o, o, ss); }
-#pragma unroll
-            for (int k = 0; k < 32; ++k) ss = fmaf(v[k], v[k], ss);
-            const float rinv = rsqrtf(ss * (1.0f / TC_K) + 1e-6f);
-#pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] *= rinv * __ldg(&g.rms_scale[kh * 32 + k]);
-          }
           if (g.gate != nullptr) {
             const float* gp = g.gate + ((size_t)(g.g_compact ? fo : fr) * g.g_planes + g.g_plane0 + kh * 32) * g.HW + px;
 #pragma unroll
@@ -419,8 +418,12 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
   }
 }
 
-// Whether the tensor-core kernel covers this problem (else the CUDA-core GEMM runs).
+// Whether this kernel takes the problem (else gemm_split_kernel, csrc/gemm_split.cu): 64 channels, tiles
+// inside one frame, no RMS prologue.  Splitting into two tf32 parts costs the producers half of what
+// three bf16 parts do, and at K = 64 the producers set the pace: in_proj of 4.2 M rows 649 against
+// 788 us.  With the RMS prologue (row sums over K) the other kernel is ahead, 683 against 847 us.
 bool gemm_tc_supported(const GemmArgs& g, bool a_planar) {
+  if (g.rms_scale != nullptr) return false;
   if (g.K != TC_K || (g.N != 64 && g.N != 128 && g.N != 192)) return false;
   if (g.HW % TC_BM != 0 || g.M % TC_BM != 0) return false;
   if (g.out_act != 0 && g.act_n0 % 32 != 0) return false;
@@ -527,8 +530,10 @@ extern "C" {
 int cssm_device_error(int* out, int clear) {
   if (!out) return CSSM_ERR_NULL;
   int a = 0, b = 0;
-  int rc = cssm::read_tc_error(&a, clear);
+  int rc = cssm::read_tc_error(&a, clear), a2 = 0;
+  if (rc == CSSM_OK) rc = cssm::read_split_error(&a2, clear);
   if (rc != CSSM_OK) return rc;
+  a |= a2;
   rc = cssm::read_spec_error(&b, clear);
   if (rc != CSSM_OK) return rc;
   int c = 0, m = 0;
