@@ -411,7 +411,10 @@ int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weigh
     if ((s = launch_deltanet_spectral_r64(sp, st)) != CSSM_OK) return s;
   } else if (deltanet_path(*d) == PATH_R32) {
     if ((s = launch_deltanet_spectral_r32(sp, st)) != CSSM_OK) return s;
+  } else if ((s = launch_deltanet_spectral_dft(sp, st)) != CSSM_ERR_UNSUPPORTED) {
+    if (s != CSSM_OK) return s;
   } else {
+    // long thin planes whose DFT tables do not fit beside them
     const size_t smem = deltanet_smem_bytes(d->H, d->W);
     cudaError_t e = cudaFuncSetAttribute(deltanet_spectral_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -476,6 +476,8 @@ int launch_spectral(int B, int T, int H, int W, int C, const cf* khat, const flo
     if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
     kern<<<grid, R64_THREADS, smem, st>>>(xz, khat, reinterpret_cast<const float4*>(gates), d.T,
                                           d.C, pmap, dchan);
+  } else if (gated_spectral_dft_fits(d.H, d.W, d.T)) {
+    return launch_gated_spectral_dft(d.B, d.T, d.H, d.W, d.C, khat, gates, xz, last_only, nogate, st, dchan);
   } else if (d.H * d.W <= SMALL_MAX_HW) {
     const size_t smem = small_smem_bytes(d.H, d.W);
     cudaError_t e = cudaFuncSetAttribute(gated_spectral_small,

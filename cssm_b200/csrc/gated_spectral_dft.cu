@@ -1,0 +1,168 @@
+// Fused spectral kernel of the gated block for planes of any size (64x64 and 32x32 have their own):
+// rfft2 -> gated recurrence over T -> irfft2 -> * silu(z), on the folded-DFT products of dft_plane.cuh.
+//
+// A CTA takes P consecutive channels of one batch element and walks t = 0 .. T-1 with their state in
+// shared memory; CTAs are persistent and loop over the channel groups, so the DFT tables are made once.
+// A thread always owns the same (column, row frequency pair) cells, so the state needs no barrier.
+// P is chosen by the launcher so that the register tiles of a pass fill the 256 threads.
+//
+// Bound: the packed FMAs of the four products and the shared-memory reads that feed them
+// (4 P Hp Wp (Hp + Wp) / 2 packed multiply-adds a step); below 20 x 20 pixels the loads and barriers.
+#include <math.h>
+#include <string.h>
+#include "kernels.cuh"
+#include "dft_plane.cuh"
+
+namespace cssm {
+
+struct GatedDftArgs {
+  float* xz; const cf* khat; const float4* gates; const float* dchan;
+  int B, T, C, P, groups, last_only, mode;        // mode: see launch_spectral
+  size_t region; int ldx, ldc;
+  DpGeom g;
+};
+
+template <int RT, int YT>
+__global__ void __launch_bounds__(DP_THREADS, 2) gated_spectral_dft(const GatedDftArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const DpGeom& g = a.g;
+  float2* TW = reinterpret_cast<float2*>(smem_raw);
+  float2* TH = TW + g.Wp * g.ldw;
+  unsigned char* base = reinterpret_cast<unsigned char*>(TH + g.Hp * g.ldh);
+  float4* RA = reinterpret_cast<float4*>(base);
+  float4* RB = reinterpret_cast<float4*>(base + a.region);
+  float4* ST = reinterpret_cast<float4*>(base + 2 * a.region);       // [k][col] {h_k, h_{H-k}}
+  const int HW = g.H * g.W, NB = g.H * g.Wp, ldx = a.ldx, ldc = a.ldc;
+  dp_fill_table(TW, g.W, g.ldw);
+  dp_fill_table(TH, g.H, g.ldh);
+  const int cgroups = (a.C + a.P - 1) / a.P;
+  const float invHW = 1.0f / (float)HW;
+  const bool keep = a.T > 1;
+
+  for (int grp = blockIdx.x; grp < a.groups; grp += gridDim.x) {
+    const int b = grp / cgroups, c0 = (grp - b * cgroups) * a.P, P = min(a.P, a.C - c0);
+    for (int t = 0; t < a.T; ++t) {
+      const size_t frame = (size_t)(b * a.T + t);
+      float* xp = a.xz + (frame * 2 * a.C + c0) * HW;
+      const bool emit = !a.last_only || t == a.T - 1;                // same for the whole CTA
+      __syncthreads();                                               // tables written; RA free again
+      dp_load_fold(g, xp, RA, ldx, P);
+      __syncthreads();
+      dp_rows<RT, YT>(g, RA, ldx, TW, RB, ldc, P);
+      __syncthreads();
+      const float4* gp = a.gates + frame * NB;
+      dp_cols<RT, YT>(g, RB, ldc, TH, P, [&](int x, int kr, int m, const cf* f0, const cf* f1) {
+        const int pl = g.dWp.div(x), kw = x - pl * g.Wp;
+        const float4* gx = gp + kw;
+        const cf* kx = a.khat + (size_t)(c0 + pl) * NB + kw;
+        float4 g0[YT], g1[YT];
+        cf k0[YT], k1[YT];
+#pragma unroll
+        for (int e = 0; e < YT; ++e) {
+          const int k = min(kr + e, g.Hp - 1), o0 = k * g.Wp, o1 = k == 0 ? 0 : (g.H - k) * g.Wp;
+          g0[e] = g1[e] = make_float4(1.f, 1.f, invHW, 0.f);         // ungated: A = K_hat, U = X_hat
+          if (a.mode != 1) { g0[e] = __ldg(gx + o0); g1[e] = __ldg(gx + o1); }
+          k0[e] = k1[e] = mk(0.f, 0.f);
+          if (t > 0) {
+            const float2 u0 = __ldg(reinterpret_cast<const float2*>(kx + o0)), u1 = __ldg(reinterpret_cast<const float2*>(kx + o1));
+            k0[e] = mk(u0.x, u0.y); k1[e] = mk(u1.x, u1.y);
+          }
+        }
+        const float dc = (a.mode == 3 && t > 0) ? __ldg(a.dchan + frame * a.C + c0 + pl) : 1.f;
+        auto step = [](float4 gt, cf kh, cf f, cf h) {
+          cf U = mk(gt.y * f.x, gt.y * f.y);
+          if (U.x * U.x + U.y * U.y < gt.w * gt.w) U = mk(gt.w, 0.f);
+          const cf A = mk(kh.x * gt.x, kh.y * gt.x);
+          const cf n = cmul(A, h);
+          return mk(n.x + U.x, n.y + U.y);
+        };
+#pragma unroll
+        for (int e = 0; e < YT; ++e) {
+          if (e >= m) continue;
+          const int k = kr + e;
+          float4 st = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (t > 0) st = ST[k * ldc + x];
+          g0[e].x *= dc; g1[e].x *= dc;
+          const cf h0 = step(g0[e], k0[e], f0[e], mk(st.x, st.y)), h1 = step(g1[e], k1[e], f1[e], mk(st.z, st.w));
+          if (keep) ST[k * ldc + x] = make_float4(h0.x, h0.y, h1.x, h1.y);
+          if (emit)
+            RA[k * ldc + x] = dp_fold_spec(k == 0 || 2 * k == g.H, mk(g0[e].z * h0.x, g0[e].z * h0.y),
+                                           mk(g1[e].z * h1.x, g1[e].z * h1.y));
+        }
+      });
+      if (!emit) continue;
+      __syncthreads();
+      dp_inv_cols<RT, YT>(g, RA, ldc, TH, RB, ldx, P);
+      __syncthreads();
+      float* out = reinterpret_cast<float*>(RA);
+      dp_inv_rows<RT, YT>(g, RB, ldx, TW, out, P);
+      __syncthreads();
+      dp_store(g, out, xp, a.mode == 0 ? xp + (size_t)a.C * HW : nullptr, P);
+    }
+  }
+}
+
+// Planes per CTA and register tile for a launch of `items` channel planes per batch element of a kind:
+// the estimate adds up, for a wave of CTAs, the multiply-add time of a step (throughput of the SM, or the
+// latency of a pass when its tiles do not fill the threads) and a fixed part for the loads and barriers.
+// The search is a few microseconds of host time, so each thread remembers its last few answers.
+DpChoice dp_choose(int H, int W, int C, int B, int unit, size_t limit, size_t (*bytes)(const DpGeom&, int, int), int arg) {
+  struct Memo { int H, W, C, B, unit, arg; size_t (*bytes)(const DpGeom&, int, int); DpChoice c; };
+  static thread_local Memo memo[8] = {};
+  Memo& m = memo[(H * 31 + W * 17 + C + B * 7 + arg + unit) & 7];
+  if (m.bytes == bytes && m.H == H && m.W == W && m.C == C && m.B == B && m.unit == unit && m.arg == arg) return m.c;
+  const DpGeom g = dp_geom(H, W);
+  DpChoice best;
+  best.P = 0; best.cost = 1e30; best.wide = 0; best.ctas = 1; best.smem = 0;
+  for (int P = unit; P <= C && P <= 128 * unit; P += unit) {
+    const size_t smem = bytes(g, P, arg);
+    if (smem > limit) break;
+    const int fit = (int)((227 * 1024) / (smem + 1024)), occ = fit > 2 ? 2 : (fit < 1 ? 1 : fit);
+    const double groups = (double)B * ((C + P - 1) / P);
+    for (int wide = 0; wide < 2; ++wide) {
+      const int RT = wide ? 2 : 1, YT = wide ? 4 : 2;
+      auto up = [](int a, int b) { return (a + b - 1) / b; };
+      const double tr = (double)up(P * g.Hp, RT) * up(g.Wp, YT), tc = (double)up(P * g.Wp, RT) * up(g.Hp, YT);
+      const double per = wide ? 0.31 : 0.16, lat = wide ? 45 : 25;
+      auto pass = [&](double tiles, int n, double q) {
+        const double rounds = ceil(tiles / DP_THREADS);
+        const double thr = q * tiles * n * per, ltn = rounds * (n * lat + 150);
+        return thr > ltn ? thr : ltn;
+      };
+      const double resident = groups < 148.0 * occ ? ceil(groups / 148) : occ;
+      const double step = 2 * pass(tr, g.Wp, resident) + 2 * pass(tc, g.Hp, resident) + 1500 + resident * P * H * W * 0.8;
+      const double cost = ceil(groups / (148.0 * resident)) * step;
+      if (cost < best.cost) { best.cost = cost; best.P = P; best.wide = wide; best.ctas = occ; best.smem = smem; }
+    }
+  }
+  m = Memo{H, W, C, B, unit, arg, bytes, best};
+  return best;
+}
+
+static size_t gated_dft_bytes(const DpGeom& g, int P, int T) {
+  return dp_table_bytes(g) + 2 * dp_region_bytes(g, P) + (T > 1 ? (size_t)g.Hp * dp_ld_cols(g, P) * 16 : 0);
+}
+
+bool gated_spectral_dft_fits(int H, int W, int T) { return gated_dft_bytes(dp_geom(H, W), 1, T) <= 226 * 1024; }
+
+int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat, const float* gates, float* xz,
+                              int last_only, int mode, cudaStream_t st, const float* dchan) {
+  const DpChoice ch = dp_choose(H, W, C, B, 1, 226 * 1024, gated_dft_bytes, T);
+  if (ch.P == 0) return CSSM_ERR_UNSUPPORTED;
+  GatedDftArgs a;
+  memset(&a, 0, sizeof(a));
+  a.xz = xz; a.khat = khat; a.gates = reinterpret_cast<const float4*>(gates); a.dchan = dchan;
+  a.B = B; a.T = T; a.C = C; a.P = ch.P; a.last_only = last_only; a.mode = mode;
+  a.g = dp_geom(H, W);
+  a.groups = B * ((C + ch.P - 1) / ch.P);
+  a.region = dp_region_bytes(a.g, ch.P);
+  a.ldx = dp_ld_rows(a.g, ch.P); a.ldc = dp_ld_cols(a.g, ch.P);
+  auto kern = ch.wide ? gated_spectral_dft<2, 4> : gated_spectral_dft<1, 2>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ch.smem);
+  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  const int slots = 148 * ch.ctas;
+  kern<<<a.groups < slots ? a.groups : slots, DP_THREADS, ch.smem, st>>>(a);
+  return check_launch();
+}
+
+}  // namespace cssm

@@ -166,6 +166,9 @@ int launch_gdn_spectral(const GdnSpectralArgs& a, cudaStream_t st) {
   if (a.dk < 1 || a.dk > GDN_MAXDK || a.C % a.dk != 0) return CSSM_ERR_UNSUPPORTED;
   if (spectral_path(a.H, a.W) == PATH_R64 && a.dk == 4) return launch_gdn_spectral_r64(a, st);
   if (spectral_path(a.H, a.W) == PATH_R32 && a.dk == 4) return launch_gdn_spectral_r32(a, st);
+  const int rc = launch_gdn_spectral_dft(a, st);
+  if (rc != CSSM_ERR_UNSUPPORTED) return rc;
+  // long thin planes whose DFT tables do not fit beside them
   const size_t smem = gdn_generic_smem_bytes(a.H, a.W, a.dk);
   if (smem > 220 * 1024) return CSSM_ERR_UNSUPPORTED;
   cudaError_t e = cudaFuncSetAttribute(gdn_spectral_generic,

@@ -50,6 +50,10 @@ int launch_gated_spectral(const cssm_gated_desc& d, const cf* khat, const float*
 int launch_spectral(int B, int T, int H, int W, int C, const cf* khat, const float* gates,
                     float* xz, int last_only, int nogate, cudaStream_t st, const float* dchan = nullptr);
 size_t generic_smem_bytes(int H, int W);
+// folded-DFT kernel for any plane size (csrc/gated_spectral_dft.cu); same arguments as launch_spectral
+bool gated_spectral_dft_fits(int H, int W, int T);
+int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat, const float* gates, float* xz,
+                              int last_only, int mode, cudaStream_t st, const float* dchan);
 int read_spec_error(int* out, int clear);
 
 // ---- DeltaNet block (scalar delta rule) ----
@@ -66,6 +70,8 @@ struct DnSpectralArgs {
 };
 int launch_deltanet_spectral_r64(const DnSpectralArgs& a, cudaStream_t st);
 int launch_deltanet_spectral_r32(const DnSpectralArgs& a, cudaStream_t st);
+// any plane size; CSSM_ERR_UNSUPPORTED when one channel does not fit an SM's shared memory
+int launch_deltanet_spectral_dft(const DnSpectralArgs& a, cudaStream_t st);
 
 // ---- GDN block ----
 struct GdnDwArgs {
@@ -104,6 +110,7 @@ struct GdnSpectralArgs {
                              // transforms, readout and inverse transforms of earlier steps are skipped)
 };
 int launch_gdn_spectral(const GdnSpectralArgs& a, cudaStream_t st);
+int launch_gdn_spectral_dft(const GdnSpectralArgs& a, cudaStream_t st);    // as launch_deltanet_spectral_dft
 size_t gdn_generic_smem_bytes(int H, int W, int dk);
 
 // ---- bf16 tensor-core GEMM with a K loop (csrc/gemm_bf16.cu) ----
