@@ -21,7 +21,7 @@
 
 namespace cssm {
 
-constexpr int DP_THREADS = 256;
+// A CTA has NT = 256 threads (two per SM) or 128 (four).  (NT from blockDim instead: 10 % slower.)
 
 typedef unsigned long long dp_u64;
 
@@ -37,9 +37,10 @@ __device__ __forceinline__ float2 dp_unpack(dp_u64 v) {
 }
 
 // tw[n][y], n, y = 0 .. N/2, row stride ld >= N/2 + 1 (a multiple of 4; the rest is zero)
+template <int NT>
 __device__ inline void dp_fill_table(float2* tw, int N, int ld) {
   const int M = N / 2 + 1;
-  for (int i = threadIdx.x; i < M * ld; i += DP_THREADS) {
+  for (int i = threadIdx.x; i < M * ld; i += NT) {
     const int n = i / ld, y = i - n * ld;
     float2 v = make_float2(0.f, 0.f);
     if (y < M) sincospif(-2.0f * (float)((n * y) % N) / (float)N, &v.y, &v.x);
@@ -49,11 +50,11 @@ __device__ inline void dp_fill_table(float2* tw, int N, int ld) {
 
 // One pass: op [Nred][ldx] 16-byte entries, tw [Nred][ldy] pairs.  epi(x, y0, m, lo, hi) takes the first m of
 // the YT cells (x, y0 ..) of a tile row at once, so that it can have their loads in flight together.
-template <int RT, int YT, class Epi>
+template <int RT, int YT, int NT, class Epi>
 __device__ __forceinline__ void dp_pass(const ulonglong2* __restrict__ op, int ldx, const dp_u64* __restrict__ tw,
                                         int ldy, int Nred, int X, int Y, Epi&& epi) {
   const int nx = (X + RT - 1) / RT, ny = (Y + YT - 1) / YT;
-  for (int tile = threadIdx.x; tile < nx * ny; tile += DP_THREADS) {
+  for (int tile = threadIdx.x; tile < nx * ny; tile += NT) {
     const int ty = tile / nx, tx = tile - ty * nx;
     dp_u64 lo[RT][YT], hi[RT][YT];
     const ulonglong2* po[RT];
@@ -128,15 +129,16 @@ inline size_t dp_table_bytes(const DpGeom& g) {
 
 // P planes from global memory (consecutive, HW apart) -> folded row operand [pixel pair][row pair].
 // Four entries (16 loads) in flight per thread.
+template <int NT>
 __device__ __forceinline__ void dp_load_fold(const DpGeom& g, const float* __restrict__ src, float4* S, int ldx, int P) {
   const int total = P * g.Hp * g.Wp;
-  for (int i0 = threadIdx.x; i0 < total; i0 += 4 * DP_THREADS) {
+  for (int i0 = threadIdx.x; i0 < total; i0 += 4 * NT) {
     float v[4][4];
     int dst[4];
     bool sn[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int i = min(i0 + u * DP_THREADS, total - 1);
+      const int i = min(i0 + u * NT, total - 1);
       const int x = g.dWp.div(i), n = i - x * g.Wp;
       const int pl = g.dHp.div(x), p = x - pl * g.Hp;
       const float* r0 = src + (pl * g.H + p) * g.W;
@@ -146,7 +148,7 @@ __device__ __forceinline__ void dp_load_fold(const DpGeom& g, const float* __res
       const float* r1 = r0 + (g.H - 2 * p) * g.W;
       v[u][0] = r0[n]; v[u][1] = r0[m];
       v[u][2] = self_p ? 0.f : r1[n]; v[u][3] = self_p ? 0.f : r1[m];
-      dst[u] = i0 + u * DP_THREADS < total ? n * ldx + x : -1;
+      dst[u] = i0 + u * NT < total ? n * ldx + x : -1;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
@@ -157,9 +159,9 @@ __device__ __forceinline__ void dp_load_fold(const DpGeom& g, const float* __res
 }
 
 // rows: folded pixels -> folded column operand [row pair][plane * Wp + k]
-template <int RT, int YT>
+template <int RT, int YT, int NT>
 __device__ __forceinline__ void dp_rows(const DpGeom& g, const float4* S, int ldx, const float2* TW, float4* U, int ldc, int P) {
-  dp_pass<RT, YT>(reinterpret_cast<const ulonglong2*>(S), ldx, reinterpret_cast<const dp_u64*>(TW), g.ldw, g.Wp,
+  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(S), ldx, reinterpret_cast<const dp_u64*>(TW), g.ldw, g.Wp,
                   P * g.Hp, g.Wp, [&](int x, int k0, int m, const float2* y0, const float2* y1) {
     const int pl = g.dHp.div(x), p = x - pl * g.Hp;
     const bool self = p == 0 || 2 * p == g.H;
@@ -174,9 +176,9 @@ __device__ __forceinline__ void dp_rows(const DpGeom& g, const float4* S, int ld
 
 // columns: epi(col, k0, m, F, G) with F[e] = F_{k0+e} and G[e] = F_{H-k0-e} of that column, k = 0 .. H/2
 // (G is meaningless for a self-paired k)
-template <int RT, int YT, class Epi>
+template <int RT, int YT, int NT, class Epi>
 __device__ __forceinline__ void dp_cols(const DpGeom& g, const float4* U, int ldc, const float2* TH, int P, Epi&& epi) {
-  dp_pass<RT, YT>(reinterpret_cast<const ulonglong2*>(U), ldc, reinterpret_cast<const dp_u64*>(TH), g.ldh, g.Hp,
+  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(U), ldc, reinterpret_cast<const dp_u64*>(TH), g.ldh, g.Hp,
                   P * g.Wp, g.Hp, [&](int x, int k0, int m, const float2* lo, const float2* hi) {
     cf f0[YT], f1[YT];
 #pragma unroll
@@ -195,9 +197,9 @@ __device__ __forceinline__ float4 dp_fold_spec(bool self, cf g0, cf g1) {
 }
 
 // inverse columns: [k][col] -> inverse row operand [column k][row pair]
-template <int RT, int YT>
+template <int RT, int YT, int NT>
 __device__ __forceinline__ void dp_inv_cols(const DpGeom& g, const float4* V, int ldc, const float2* TH, float4* R, int ldx, int P) {
-  dp_pass<RT, YT>(reinterpret_cast<const ulonglong2*>(V), ldc, reinterpret_cast<const dp_u64*>(TH), g.ldh, g.Hp,
+  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(V), ldc, reinterpret_cast<const dp_u64*>(TH), g.ldh, g.Hp,
                   P * g.Wp, g.Hp, [&](int x, int p0, int m, const float2* lo, const float2* hi) {
     const int pl = g.dWp.div(x), k = x - pl * g.Wp;
     const float f = (k == 0 || 2 * k == g.W) ? 1.f : 2.f;
@@ -211,10 +213,10 @@ __device__ __forceinline__ void dp_inv_cols(const DpGeom& g, const float4* V, in
 
 // inverse rows (C2R; the imaginary parts of columns 0 and W/2 meet a zero sine) -> planes in shared
 // memory, rows of W | 1 floats
-template <int RT, int YT>
+template <int RT, int YT, int NT>
 __device__ __forceinline__ void dp_inv_rows(const DpGeom& g, const float4* R, int ldx, const float2* TW, float* out, int P) {
   const int pitch = g.W | 1;
-  dp_pass<RT, YT>(reinterpret_cast<const ulonglong2*>(R), ldx, reinterpret_cast<const dp_u64*>(TW), g.ldw, g.Wp,
+  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(R), ldx, reinterpret_cast<const dp_u64*>(TW), g.ldw, g.Wp,
                   P * g.Hp, g.Wp, [&](int x, int w0, int m, const float2* lo, const float2* hi) {
     const int pl = g.dHp.div(x), p = x - pl * g.Hp;
     float* r0 = out + (pl * g.H + p) * pitch;
@@ -236,18 +238,19 @@ __device__ __forceinline__ void dp_inv_rows(const DpGeom& g, const float4* R, in
 }
 
 // planes in shared memory (rows of W | 1 floats) -> global memory, times the planes z unless it is null
+template <int NT>
 __device__ __forceinline__ void dp_store(const DpGeom& g, const float* out, float* __restrict__ dst, const float* __restrict__ z, int P) {
   const int total = P * g.H * g.W, pitch = g.W | 1;
-  for (int i0 = threadIdx.x; i0 < total; i0 += 8 * DP_THREADS) {
+  for (int i0 = threadIdx.x; i0 < total; i0 += 8 * NT) {
     float zv[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const int i = i0 + u * DP_THREADS;
+      const int i = i0 + u * NT;
       zv[u] = (z != nullptr && i < total) ? __ldg(z + i) : 1.f;
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const int i = i0 + u * DP_THREADS;
+      const int i = i0 + u * NT;
       if (i < total) {
         const int row = g.dW.div(i);
         dst[i] = out[row * pitch + (i - row * g.W)] * zv[u];
@@ -257,8 +260,8 @@ __device__ __forceinline__ void dp_store(const DpGeom& g, const float* out, floa
 }
 
 // Launch choice of the plane-group kernels: P planes per CTA (a multiple of `unit`), wide = 2 x 4 register
-// tiles instead of 1 x 2, CTAs per SM, dynamic shared memory.  bytes(g, P, arg): shared memory of P planes.
-struct DpChoice { int P, wide, ctas; size_t smem; double cost; };
+// tiles instead of 1 x 2, CTAs per SM, threads, dynamic shared memory.  bytes(g, P, arg): shared memory of P planes.
+struct DpChoice { int P, wide, ctas, threads; size_t smem; double cost; };
 DpChoice dp_choose(int H, int W, int C, int B, int unit, size_t limit, size_t (*bytes)(const DpGeom&, int, int), int arg);
 
 }  // namespace cssm

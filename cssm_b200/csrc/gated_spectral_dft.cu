@@ -8,6 +8,8 @@
 //
 // Bound: the packed FMAs of the four products and the shared-memory reads that feed them
 // (4 P Hp Wp (Hp + Wp) / 2 packed multiply-adds a step); below 20 x 20 pixels the loads and barriers.
+// 16 x 8 x 56 x 56 x 32: 1074 (direct DFTs, one thread per output) -> 210 us; 48 x 8 x 14 x 14 x 256 and
+// 7 x 7 x 384, last frame only: 676 -> 283 us for the three launches of a forward.
 #include <math.h>
 #include <string.h>
 #include "kernels.cuh"
@@ -22,8 +24,8 @@ struct GatedDftArgs {
   DpGeom g;
 };
 
-template <int RT, int YT>
-__global__ void __launch_bounds__(DP_THREADS, 2) gated_spectral_dft(const GatedDftArgs a) {
+template <int RT, int YT, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDftArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DpGeom& g = a.g;
   float2* TW = reinterpret_cast<float2*>(smem_raw);
@@ -33,8 +35,8 @@ __global__ void __launch_bounds__(DP_THREADS, 2) gated_spectral_dft(const GatedD
   float4* RB = reinterpret_cast<float4*>(base + a.region);
   float4* ST = reinterpret_cast<float4*>(base + 2 * a.region);       // [k][col] {h_k, h_{H-k}}
   const int HW = g.H * g.W, NB = g.H * g.Wp, ldx = a.ldx, ldc = a.ldc;
-  dp_fill_table(TW, g.W, g.ldw);
-  dp_fill_table(TH, g.H, g.ldh);
+  dp_fill_table<NT>(TW, g.W, g.ldw);
+  dp_fill_table<NT>(TH, g.H, g.ldh);
   const int cgroups = (a.C + a.P - 1) / a.P;
   const float invHW = 1.0f / (float)HW;
   const bool keep = a.T > 1;
@@ -46,12 +48,12 @@ __global__ void __launch_bounds__(DP_THREADS, 2) gated_spectral_dft(const GatedD
       float* xp = a.xz + (frame * 2 * a.C + c0) * HW;
       const bool emit = !a.last_only || t == a.T - 1;                // same for the whole CTA
       __syncthreads();                                               // tables written; RA free again
-      dp_load_fold(g, xp, RA, ldx, P);
+      dp_load_fold<NT>(g, xp, RA, ldx, P);
       __syncthreads();
-      dp_rows<RT, YT>(g, RA, ldx, TW, RB, ldc, P);
+      dp_rows<RT, YT, NT>(g, RA, ldx, TW, RB, ldc, P);
       __syncthreads();
       const float4* gp = a.gates + frame * NB;
-      dp_cols<RT, YT>(g, RB, ldc, TH, P, [&](int x, int kr, int m, const cf* f0, const cf* f1) {
+      dp_cols<RT, YT, NT>(g, RB, ldc, TH, P, [&](int x, int kr, int m, const cf* f0, const cf* f1) {
         const int pl = g.dWp.div(x), kw = x - pl * g.Wp;
         const float4* gx = gp + kw;
         const cf* kx = a.khat + (size_t)(c0 + pl) * NB + kw;
@@ -92,19 +94,20 @@ __global__ void __launch_bounds__(DP_THREADS, 2) gated_spectral_dft(const GatedD
       });
       if (!emit) continue;
       __syncthreads();
-      dp_inv_cols<RT, YT>(g, RA, ldc, TH, RB, ldx, P);
+      dp_inv_cols<RT, YT, NT>(g, RA, ldc, TH, RB, ldx, P);
       __syncthreads();
       float* out = reinterpret_cast<float*>(RA);
-      dp_inv_rows<RT, YT>(g, RB, ldx, TW, out, P);
+      dp_inv_rows<RT, YT, NT>(g, RB, ldx, TW, out, P);
       __syncthreads();
-      dp_store(g, out, xp, a.mode == 0 ? xp + (size_t)a.C * HW : nullptr, P);
+      dp_store<NT>(g, out, xp, a.mode == 0 ? xp + (size_t)a.C * HW : nullptr, P);
     }
   }
 }
 
-// Planes per CTA and register tile for a launch of `items` channel planes per batch element of a kind:
-// the estimate adds up, for a wave of CTAs, the multiply-add time of a step (throughput of the SM, or the
-// latency of a pass when its tiles do not fill the threads) and a fixed part for the loads and barriers.
+// Planes per CTA, register tile and threads: the estimate adds up, for a wave of CTAs, the time of the four
+// passes of a step (throughput of the SM, or the latency of a pass when its tiles do not fill the threads)
+// and a fixed part for the loads and barriers.  The constants were fitted to 19 shapes from 1 x 14 x 14 x 256
+// to 16 x 8 x 56 x 56 x 32 (some 40 choices each); the choice is within 5 % of the best of them everywhere.
 // The search is a few microseconds of host time, so each thread remembers its last few answers.
 DpChoice dp_choose(int H, int W, int C, int B, int unit, size_t limit, size_t (*bytes)(const DpGeom&, int, int), int arg) {
   struct Memo { int H, W, C, B, unit, arg; size_t (*bytes)(const DpGeom&, int, int); DpChoice c; };
@@ -117,22 +120,23 @@ DpChoice dp_choose(int H, int W, int C, int B, int unit, size_t limit, size_t (*
   for (int P = unit; P <= C && P <= 128 * unit; P += unit) {
     const size_t smem = bytes(g, P, arg);
     if (smem > limit) break;
-    const int fit = (int)((227 * 1024) / (smem + 1024)), occ = fit > 2 ? 2 : (fit < 1 ? 1 : fit);
     const double groups = (double)B * ((C + P - 1) / P);
-    for (int wide = 0; wide < 2; ++wide) {
+    for (int v = 0; v < 4; ++v) {
+      const int wide = v & 1, nt = v & 2 ? 256 : 128;
+      const int fit = (int)((227 * 1024) / (smem + 1024)), most = 512 / nt, occ = fit > most ? most : (fit < 1 ? 1 : fit);
       const int RT = wide ? 2 : 1, YT = wide ? 4 : 2;
       auto up = [](int a, int b) { return (a + b - 1) / b; };
       const double tr = (double)up(P * g.Hp, RT) * up(g.Wp, YT), tc = (double)up(P * g.Wp, RT) * up(g.Hp, YT);
-      const double per = wide ? 0.31 : 0.16, lat = wide ? 45 : 25;
+      // clocks: SM time of a tile and reduction step, latency of a step, of an epilogue
+      const double per = wide ? 0.094 : 0.163, lat = wide ? 129 : 30, epi = wide ? 180 : 320;
       auto pass = [&](double tiles, int n, double q) {
-        const double rounds = ceil(tiles / DP_THREADS);
-        const double thr = q * tiles * n * per, ltn = rounds * (n * lat + 150);
+        const double thr = q * tiles * (n * per + 0.029 * RT * YT), ltn = ceil(tiles / nt) * (n * lat + epi);
         return thr > ltn ? thr : ltn;
       };
       const double resident = groups < 148.0 * occ ? ceil(groups / 148) : occ;
-      const double step = 2 * pass(tr, g.Wp, resident) + 2 * pass(tc, g.Hp, resident) + 1500 + resident * P * H * W * 0.8;
+      const double step = 2 * pass(tr, g.Wp, resident) + 2 * pass(tc, g.Hp, resident) + 2930 + resident * P * H * W;
       const double cost = ceil(groups / (148.0 * resident)) * step;
-      if (cost < best.cost) { best.cost = cost; best.P = P; best.wide = wide; best.ctas = occ; best.smem = smem; }
+      if (cost < best.cost) { best.cost = cost; best.P = P; best.wide = wide; best.ctas = occ; best.threads = nt; best.smem = smem; }
     }
   }
   m = Memo{H, W, C, B, unit, arg, bytes, best};
@@ -157,11 +161,12 @@ int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat,
   a.groups = B * ((C + ch.P - 1) / ch.P);
   a.region = dp_region_bytes(a.g, ch.P);
   a.ldx = dp_ld_rows(a.g, ch.P); a.ldc = dp_ld_cols(a.g, ch.P);
-  auto kern = ch.wide ? gated_spectral_dft<2, 4> : gated_spectral_dft<1, 2>;
+  auto kern = ch.threads == 256 ? (ch.wide ? gated_spectral_dft<2, 4, 256> : gated_spectral_dft<1, 2, 256>)
+                                : (ch.wide ? gated_spectral_dft<2, 4, 128> : gated_spectral_dft<1, 2, 128>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ch.smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   const int slots = 148 * ch.ctas;
-  kern<<<a.groups < slots ? a.groups : slots, DP_THREADS, ch.smem, st>>>(a);
+  kern<<<a.groups < slots ? a.groups : slots, ch.threads, ch.smem, st>>>(a);
   return check_launch();
 }
 

@@ -1,0 +1,61 @@
+"""The folded-DFT spectral kernels (planes without a radix kernel) at the sizes where they can go wrong:
+one-pixel, odd, even, prime and unequal sides, channel counts that leave a ragged plane group, T = 1 (no
+state), and a plane too long for the tables (direct-DFT kernel), against the float64 oracle.
+
+Tolerance: a plane value is four nested sums of at most 50 terms with exactly rounded twiddles, each
+within sqrt(50) * 2^-24 of its norm (4e-7); the recurrence over at most three steps adds its own few
+roundings, the norms of the delta rules one division: below 5e-6 of the 2-norm, checked at 1e-5."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import cssm_oracle as orc
+from cssm_b200 import AdditiveCSSM, DeltaNetCSSM, GatedCSSM, GatedDeltaNetCSSM, NoGateCSSM
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-5
+SIZES = [(1, 1, 1, 7, 4), (2, 3, 2, 3, 4), (1, 2, 5, 4, 8), (3, 1, 7, 7, 20), (2, 3, 8, 13, 12), (1, 3, 14, 14, 68),
+         (2, 2, 16, 15, 8), (1, 2, 29, 31, 12), (1, 2, 50, 56, 8), (1, 2, 33, 90, 4), (1, 2, 2, 700, 4)]
+
+
+def _check(got, ref):
+    got = got.cpu().numpy()
+    assert np.isfinite(got).all()
+    assert orc.rel_l2(got, ref) <= TOL
+
+
+@pytest.mark.parametrize("B,T,H,W,C", SIZES)
+def test_gated_family(B, T, H, W, C):
+    rng = np.random.default_rng(H * 100 + W)
+    x = rng.standard_normal((B, T, H, W, C)).astype(np.float32)
+    xd = torch.from_numpy(x).cuda()
+    kw = dict(kernel_size=1, rope_mode="none", gate_type="factored")
+    p = orc.init_gated_params(1, C, H, W, bias_scale=0.1, kernel_size=1, gate_type="factored")
+    b = GatedCSSM(channels=C, **kw).bind({"params": p})
+    ref = orc.gated_forward(p, x, **kw)
+    _check(b(xd), ref)
+    _check(b(xd, last_frame_only=True), ref[:, -1])
+    m = NoGateCSSM(channels=C, kernel_size=1)
+    p = m.init(2, x.shape, bias_scale=0.1)["params"]
+    _check(m.apply({"params": p}, xd), orc.nogate_forward(p, x, kernel_size=1))
+    kw["gate_type"] = "channel"
+    p = orc.init_additive1_params(3, C, H, W, kernel_size=1, gate_type="channel", bias_scale=0.1)
+    _check(AdditiveCSSM(channels=C, single_state=True, **kw).apply({"params": p}, xd), orc.additive1_forward(p, x, **kw))
+
+
+@pytest.mark.parametrize("dk", [1, 2, 4])
+@pytest.mark.parametrize("B,T,H,W,C", SIZES)
+def test_delta_rules(B, T, H, W, C, dk):
+    rng = np.random.default_rng(H * 100 + W + dk)
+    x = rng.standard_normal((B, T, H, W, C)).astype(np.float32)
+    xd = torch.from_numpy(x).cuda()
+    kw = dict(delta_key_dim=dk, kernel_size=1, rope_mode="none", gate_type="factored")
+    p = orc.init_gdn_params(1, C, H, W, bias_scale=0.1, perturb_rms=True, **{k: kw[k] for k in kw if k != "rope_mode"})
+    b = GatedDeltaNetCSSM(channels=C, **kw).bind({"params": p})
+    ref = orc.gdn_forward(p, x, **kw)
+    _check(b(xd), ref)
+    _check(b(xd, last_frame_only=True), ref[:, -1])
+    if dk == 1:
+        kw = dict(kernel_size=1, rope_mode="none", gate_type="dense" if H % 2 else "channel")
+        p = orc.init_deltanet_params(3, C, H, W, kernel_size=1, gate_type=kw["gate_type"], bias_scale=0.1)
+        _check(DeltaNetCSSM(channels=C, **kw).apply({"params": p}, xd), orc.deltanet_forward(p, x, **kw))
