@@ -8,6 +8,7 @@
 #include <string.h>
 #include "kernels.cuh"
 #include "gemm.cuh"
+#include "gates.cuh"
 
 namespace cssm {
 
@@ -20,59 +21,52 @@ struct AddGateArgs {
 
 __device__ __forceinline__ float add_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-// One CTA per (frame, chunk of bins).  The map entry has the layout the fused spectral kernel
-// reads: {factor on K_hat, factor on X_hat, factor on the state for the output (with the 1/(HW)
-// of the inverse transform folded in), magnitude floor of the input term}.
-__global__ void __launch_bounds__(256) additive_gates_kernel(const AddGateArgs g) {
-  extern __shared__ float sh[];
-  const int Wf = g.W / 2 + 1, NB = g.H * Wf;
+// The map entry has the layout the fused spectral kernel reads: {factor on K_hat, factor on X_hat, factor
+// on the state for the output (with the 1/(HW) of the inverse transform folded in), magnitude floor of
+// the input term}.
+__device__ __forceinline__ float4 add_map(float rd, float rb, float rc, float inv, int floor) {
+  return make_float4(0.1f + 0.89f * add_sigmoid(rd), add_sigmoid(rb), add_sigmoid(rc) * inv, floor ? 1e-7f : 0.f);
+}
+// factored: one frame per CTA row, its bins over gridDim.y CTAs
+__global__ void __launch_bounds__(256) additive_gates_factored_kernel(const AddGateArgs g) {
+  extern __shared__ __align__(16) float sh[];
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, per = g.H + Wf, fr = blockIdx.x;
   float* ctx = sh;                 // [C]
-  float* vec = sh + g.C;           // factored: 3 x (H + Wf)
-  const int fr = blockIdx.x, tid = threadIdx.x, t = fr % g.T;
+  float* vec = sh + g.C;           // 3 x (H + Wf)
+  float* scratch = vec + 3 * per;  // [256]
   const float inv = 1.0f / (float)(g.H * g.W);
-  for (int c = tid; c < g.C; c += blockDim.x) {
-    float s = 0.f;
-    for (int h = 0; h < g.H; ++h) s += g.ctx_part[((size_t)fr * g.H + h) * g.C + c];
-    ctx[c] = s * inv + g.tcode[t * g.C + c];
-  }
-  __syncthreads();
-  const int per = g.H + Wf;
-  if (g.gate_type == CSSM_GATE_FACTORED) {
-    for (int o = tid; o < 3 * per; o += blockDim.x) {
-      const int gi = o / per, r = o % per;
-      const bool isw = r >= g.H;
-      const int col = isw ? r - g.H : r, ncol = isw ? Wf : g.H;
-      const float* kk = g.gk[2 * gi + (isw ? 1 : 0)];
-      float acc = g.gb[2 * gi + (isw ? 1 : 0)][col];
-      for (int c = 0; c < g.C; ++c) acc = fmaf(ctx[c], kk[(size_t)c * ncol + col], acc);
-      vec[o] = acc;
-    }
-    __syncthreads();
-  }
+  pdl_sync();
+  const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, 0, inv};
+  gate_ctx(src, fr, 1, ctx, scratch);
+  const int off[7] = {0, g.H, per, per + g.H, 2 * per, 2 * per + g.H, 3 * per};
+  gate_vectors<6>(g.gk, g.gb, off, 6, ctx, g.C, vec, scratch);
   const int per_cta = (NB + gridDim.y - 1) / gridDim.y;
   const int bin_end = min(NB, (int)(blockIdx.y + 1) * per_cta);
-  for (int bin = blockIdx.y * per_cta + tid; bin < bin_end; bin += blockDim.x) {
-    const int kh = bin / Wf, kw = bin % Wf;
+  for (int bin = blockIdx.y * per_cta + threadIdx.x; bin < bin_end; bin += 256) {
+    const int kh = bin / Wf, kw = bin - kh * Wf;
     float r[3];
-    if (g.gate_type == CSSM_GATE_FACTORED) {
 #pragma unroll
-      for (int gi = 0; gi < 3; ++gi) r[gi] = vec[gi * per + kh] + vec[gi * per + g.H + kw];
-    } else {
-#pragma unroll
-      for (int gi = 0; gi < 3; ++gi) {
-        float acc = g.gb[gi][bin];
-        const float* kk = g.gk[gi];
-        for (int c = 0; c < g.C; ++c) acc = fmaf(ctx[c], kk[(size_t)c * NB + bin], acc);
-        r[gi] = acc;
-      }
-    }
-    float4 o;
-    o.x = 0.1f + 0.89f * add_sigmoid(r[0]);
-    o.y = add_sigmoid(r[1]);
-    o.z = add_sigmoid(r[2]) * inv;
-    o.w = g.goom_floor ? 1e-7f : 0.f;
-    g.maps[(size_t)fr * NB + bin_index(g.path, kh, kw, g.H, Wf)] = o;
+    for (int gi = 0; gi < 3; ++gi) r[gi] = vec[gi * per + kh] + vec[gi * per + g.H + kw];
+    g.maps[(size_t)fr * NB + bin_index(g.path, kh, kw, g.H, Wf)] = add_map(r[0], r[1], r[2], inv, g.goom_floor);
   }
+}
+// dense: a thread owns one bin of G frames
+template <int G>
+__global__ void __launch_bounds__(128) additive_gates_dense_kernel(const AddGateArgs g) {
+  extern __shared__ __align__(16) float sh[];
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, f0 = blockIdx.y * G, nf = min(G, g.BT - f0);
+  const float inv = 1.0f / (float)(g.H * g.W);
+  pdl_sync();
+  const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, 0, inv};
+  gate_ctx(src, f0, nf, sh, sh + G * g.C);
+  const int bin = blockIdx.x * 128 + threadIdx.x;
+  if (bin >= NB) return;
+  float r[3][G];
+  gate_dense<3, G>(g.gk, g.gb, NB, bin, g.C, sh, r);
+  const int kh = bin / Wf, o = bin_index(g.path, kh, bin - kh * Wf, g.H, Wf);
+#pragma unroll
+  for (int f = 0; f < G; ++f)
+    if (f < nf) g.maps[(size_t)(f0 + f) * NB + o] = add_map(r[0][f], r[1][f], r[2][f], inv, g.goom_floor);
 }
 
 // gate_type 'channel' (cssm.py:3168-3178): d_X = 0.1 + 0.89 sigmoid(Dense(C)(ctx)) per (frame,
@@ -85,22 +79,20 @@ struct AddChanArgs {
   float* dchan;                            // (BT, C)
   float4* maps;                            // (BT, H*Wf)
 };
-__global__ void __launch_bounds__(128) additive_chan_gates_kernel(const AddChanArgs g) {
-  extern __shared__ float sh[];            // ctx [C]
-  const int fr = blockIdx.x, tid = threadIdx.x, t = fr % g.T;
+__global__ void __launch_bounds__(256) additive_chan_gates_kernel(const AddChanArgs g) {
+  extern __shared__ __align__(16) float sh[];     // ctx [C], vec [C], scratch [256]
+  const int fr = blockIdx.x, tid = threadIdx.x;
   const int NB = g.H * (g.W / 2 + 1);
   const float inv = 1.0f / (float)(g.H * g.W);
-  for (int c = tid; c < g.C; c += blockDim.x) {
-    float s = 0.f;
-    for (int h = 0; h < g.H; ++h) s += g.ctx_part[((size_t)fr * g.H + h) * g.C + c];
-    sh[c] = s * inv + g.tcode[t * g.C + c];
-  }
-  __syncthreads();
-  for (int o = tid; o < g.C; o += blockDim.x) {
-    float a = g.db[o];
-    for (int c = 0; c < g.C; ++c) a = fmaf(sh[c], g.dk[(size_t)c * g.C + o], a);
-    g.dchan[(size_t)fr * g.C + o] = 0.1f + 0.89f * add_sigmoid(a);
-  }
+  float* vec = sh + g.C;
+  pdl_sync();
+  const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, 0, inv};
+  gate_ctx(src, fr, 1, sh, vec + g.C);
+  const float* const gk[1] = {g.dk};
+  const float* const gb[1] = {g.db};
+  const int off[2] = {0, g.C};
+  gate_vectors<1>(gk, gb, off, 1, sh, g.C, vec, vec + g.C);
+  for (int o = tid; o < g.C; o += blockDim.x) g.dchan[(size_t)fr * g.C + o] = 0.1f + 0.89f * add_sigmoid(vec[o]);
   const float4 m = make_float4(1.f, 1.f, inv, g.goom_floor ? 1e-7f : 0.f);
   for (int i = tid; i < NB; i += blockDim.x) g.maps[(size_t)fr * NB + i] = m;
 }
@@ -108,6 +100,7 @@ __global__ void __launch_bounds__(128) additive_chan_gates_kernel(const AddChanA
 // planes [0, C) of every frame of the (frames, 2C, HW) buffer times its planes [C, 2C)
 __global__ void __launch_bounds__(256) additive_in_gate_kernel(float* __restrict__ planar, size_t per_frame4,
                                                                size_t total4) {
+  pdl_sync();
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= total4) return;
   const size_t fr = i / per_frame4, r = i - fr * per_frame4;
@@ -120,14 +113,17 @@ __global__ void __launch_bounds__(256) additive_in_gate_kernel(float* __restrict
 
 static int launch_additive_gates(const AddGateArgs& g, cudaStream_t st) {
   const int Wf = g.W / 2 + 1, NB = g.H * Wf;
-  const size_t smem = (size_t)(g.C + 3 * (g.H + Wf)) * sizeof(float);
-  int chunks = 1;
-  if (g.BT < 296) {
-    chunks = (296 + g.BT - 1) / g.BT;
-    const int maxc = (NB + 255) / 256;
-    if (chunks > maxc) chunks = maxc;
+  if (g.gate_type == CSSM_GATE_FACTORED) {
+    const size_t smem = (size_t)(g.C + 3 * (g.H + Wf) + 256) * sizeof(float);
+    launch_k(additive_gates_factored_kernel, dim3(g.BT, gate_chunks(g.BT, NB)), 256, smem, st, g);
+    return check_launch();
   }
-  additive_gates_kernel<<<dim3(g.BT, chunks), 256, smem, st>>>(g);
+  const int chunks = (NB + 127) / 128, G = gate_dense_frames(g.BT, chunks);
+  const dim3 grid(chunks, (g.BT + G - 1) / G);
+  const size_t smem = (size_t)(G * g.C + 128) * sizeof(float);
+  if (G == 8) launch_k(additive_gates_dense_kernel<8>, grid, 128, smem, st, g);
+  else if (G == 4) launch_k(additive_gates_dense_kernel<4>, grid, 128, smem, st, g);
+  else launch_k(additive_gates_dense_kernel<1>, grid, 128, smem, st, g);
   return check_launch();
 }
 
@@ -237,6 +233,7 @@ int cssm_additive_plan_init(const cssm_additive_desc* d, const cssm_additive_wei
 int cssm_additive_forward(const cssm_additive_desc* d, const cssm_additive_weights* w,
                           const void* plan, const float* x, float* y, void* workspace,
                           size_t workspace_bytes, void* stream) {
+  PdlScope pdl(d != nullptr && (size_t)d->B * d->T * d->H * d->W * d->C * 4 <= PDL_MAX_BYTES);
   int s = additive_validate(d);
   if (s != CSSM_OK) return s;
   if (!w || !plan || !x || !y || !workspace) return CSSM_ERR_NULL;
@@ -289,7 +286,7 @@ int cssm_additive_forward(const cssm_additive_desc* d, const cssm_additive_weigh
     if (((size_t)C * HW) % 4 != 0) return CSSM_ERR_UNSUPPORTED;
     // x_proj *= B_X in the spatial domain
     const size_t per_frame4 = (size_t)C * HW / 4, total4 = per_frame4 * BT;
-    additive_in_gate_kernel<<<(unsigned)((total4 + 255) / 256), 256, 0, st>>>(planar, per_frame4, total4);
+    launch_k(additive_in_gate_kernel, (unsigned)((total4 + 255) / 256), 256, 0, st, planar, per_frame4, total4);
     if ((s = check_launch()) != CSSM_OK) return s;
     AddChanArgs ca;
     memset(&ca, 0, sizeof(ca));
@@ -297,7 +294,7 @@ int cssm_additive_forward(const cssm_additive_desc* d, const cssm_additive_weigh
     ca.BT = BT; ca.T = d->T; ca.C = C; ca.H = d->H; ca.W = d->W; ca.goom_floor = d->goom_floor;
     ca.dk = w->gate_kernel[0]; ca.db = w->gate_bias[0];
     ca.dchan = (float*)(ws + l.dchan); ca.maps = (float4*)(ws + l.maps);
-    additive_chan_gates_kernel<<<BT, 128, (size_t)C * sizeof(float), st>>>(ca);
+    launch_k(additive_chan_gates_kernel, BT, 256, (size_t)(2 * C + 256) * sizeof(float), st, ca);
     if ((s = check_launch()) != CSSM_OK) return s;
     // C_gate planes sigmoid(Conv1x1(rotated x))
     memset(&g, 0, sizeof(g));

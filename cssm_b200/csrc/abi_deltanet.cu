@@ -8,6 +8,7 @@
 #include <string.h>
 #include "kernels.cuh"
 #include "gemm.cuh"
+#include "gates.cuh"
 #include "generic_dft.cuh"
 
 namespace cssm {
@@ -22,60 +23,61 @@ struct DnGateArgs {
 
 __device__ __forceinline__ float dn_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-// One CTA per (frame, chunk of bins): ctx = mean of the rotated input + temporal code, then the
-// five gate maps sigmoid(Dense(ctx)) (dense) or sigmoid(row + col) (factored); alpha is mapped
-// to [0.1, 0.99] (cssm.py:3756-3793).
-__global__ void __launch_bounds__(256) deltanet_gates_kernel(const DnGateArgs g) {
-  extern __shared__ float sh[];
-  const int Wf = g.W / 2 + 1, NB = g.H * Wf;
+// Five gate maps sigmoid(Dense(ctx)) (dense) or sigmoid(row + col) (factored), ctx = mean of the rotated
+// input + temporal code; alpha is mapped to [0.1, 0.99] (cssm.py:3756-3793).
+__device__ __forceinline__ void dn_write(const DnGateArgs& g, size_t oi, const float (&r)[5], float inv) {
+  g.abkv[oi] = make_float4(0.1f + 0.89f * dn_sigmoid(r[0]), dn_sigmoid(r[1]), dn_sigmoid(r[2]), dn_sigmoid(r[3]));
+  g.cg[oi] = dn_sigmoid(r[4]) * inv;
+}
+// factored: one frame per CTA row, its bins over gridDim.y CTAs
+__global__ void __launch_bounds__(256) deltanet_gates_factored_kernel(const DnGateArgs g) {
+  extern __shared__ __align__(16) float sh[];
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, per = g.H + Wf, fr = blockIdx.x;
   float* ctx = sh;                 // [C]
-  float* vec = sh + g.C;           // factored: 5 x (H + Wf)
-  const int fr = blockIdx.x, tid = threadIdx.x, t = fr % g.T;
+  float* vec = sh + g.C;           // 5 x (H + Wf)
+  float* scratch = vec + 5 * per;  // [256]
   const float inv = 1.0f / (float)(g.H * g.W);
-  for (int c = tid; c < g.C; c += blockDim.x) {
-    float s = 0.f;
-    for (int h = 0; h < g.H; ++h) s += g.ctx_part[((size_t)fr * g.H + h) * g.C + c];
-    ctx[c] = s * inv + g.tcode[t * g.C + c];
-  }
-  __syncthreads();
-  const int per = g.H + Wf;
-  if (g.gate_type == CSSM_GATE_FACTORED) {
-    for (int o = tid; o < 5 * per; o += blockDim.x) {
-      const int gi = o / per, r = o % per;
-      const bool isw = r >= g.H;
-      const int col = isw ? r - g.H : r, ncol = isw ? Wf : g.H;
-      const float* kk = g.gk[2 * gi + (isw ? 1 : 0)];
-      float acc = g.gb[2 * gi + (isw ? 1 : 0)][col];
-      for (int c = 0; c < g.C; ++c) acc = fmaf(ctx[c], kk[(size_t)c * ncol + col], acc);
-      vec[o] = acc;
-    }
-    __syncthreads();
-  }
+  pdl_sync();
+  const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, 0, inv};
+  gate_ctx(src, fr, 1, ctx, scratch);
+  int off[11];
+#pragma unroll
+  for (int q = 0; q <= 10; ++q) off[q] = (q >> 1) * per + ((q & 1) ? g.H : 0);
+  gate_vectors<10>(g.gk, g.gb, off, 10, ctx, g.C, vec, scratch);
   const int per_cta = (NB + gridDim.y - 1) / gridDim.y;
   const int bin_end = min(NB, (int)(blockIdx.y + 1) * per_cta);
-  for (int bin = blockIdx.y * per_cta + tid; bin < bin_end; bin += blockDim.x) {
-    const int kh = bin / Wf, kw = bin % Wf;
+  for (int bin = blockIdx.y * per_cta + threadIdx.x; bin < bin_end; bin += 256) {
+    const int kh = bin / Wf, kw = bin - kh * Wf;
     float r[5];
-    if (g.gate_type == CSSM_GATE_FACTORED) {
 #pragma unroll
-      for (int gi = 0; gi < 5; ++gi) r[gi] = vec[gi * per + kh] + vec[gi * per + g.H + kw];
-    } else {
+    for (int gi = 0; gi < 5; ++gi) r[gi] = vec[gi * per + kh] + vec[gi * per + g.H + kw];
+    dn_write(g, (size_t)fr * NB + bin_index(g.path, kh, kw, g.H, Wf), r, inv);
+  }
+}
+// dense: a thread owns one bin of G frames
+template <int G>
+__global__ void __launch_bounds__(128) deltanet_gates_dense_kernel(const DnGateArgs g) {
+  extern __shared__ __align__(16) float sh[];
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, f0 = blockIdx.y * G, nf = min(G, g.BT - f0);
+  const float inv = 1.0f / (float)(g.H * g.W);
+  pdl_sync();
+  const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, 0, inv};
+  gate_ctx(src, f0, nf, sh, sh + G * g.C);
+  const int bin = blockIdx.x * 128 + threadIdx.x;
+  if (bin >= NB) return;
+  float r[5][G];
+  gate_dense<5, G>(g.gk, g.gb, NB, bin, g.C, sh, r);
+  const int kh = bin / Wf, o = bin_index(g.path, kh, bin - kh * Wf, g.H, Wf);
 #pragma unroll
-      for (int gi = 0; gi < 5; ++gi) {
-        float acc = g.gb[gi][bin];
-        const float* kk = g.gk[gi];
-        for (int c = 0; c < g.C; ++c) acc = fmaf(ctx[c], kk[(size_t)c * NB + bin], acc);
-        r[gi] = acc;
-      }
-    }
-    const size_t oi = (size_t)fr * NB + bin_index(g.path, kh, kw, g.H, Wf);
-    g.abkv[oi] = make_float4(0.1f + 0.89f * dn_sigmoid(r[0]), dn_sigmoid(r[1]),
-                                                dn_sigmoid(r[2]), dn_sigmoid(r[3]));
-    g.cg[oi] = dn_sigmoid(r[4]) * inv;
+  for (int f = 0; f < G; ++f) {
+    if (f >= nf) continue;
+    const float v[5] = {r[0][f], r[1][f], r[2][f], r[3][f], r[4][f]};
+    dn_write(g, (size_t)(f0 + f) * NB + o, v, inv);
   }
 }
 
 __global__ void __launch_bounds__(GG_THREADS) deltanet_spectral_kernel(const DnSpectralArgs a) {
+  pdl_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int H = a.H, W = a.W;
   const int Wf = W / 2 + 1, HW = H * W, NB = H * Wf;
@@ -162,24 +164,19 @@ struct DnChanArgs {
   const float* ak; const float* ab; const float* bk; const float* bb;   // (C,C), (C) x 2
   float2* chan;                                                          // (BT, C) {alpha, beta}
 };
-__global__ void __launch_bounds__(128) deltanet_chan_gates_kernel(const DnChanArgs g) {
-  extern __shared__ float sh[];          // ctx [C]
-  const int fr = blockIdx.x, tid = threadIdx.x, t = fr % g.T;
-  const float inv = 1.0f / (float)(g.H * g.W);
-  for (int c = tid; c < g.C; c += blockDim.x) {
-    float s = 0.f;
-    for (int h = 0; h < g.H; ++h) s += g.ctx_part[((size_t)fr * g.H + h) * g.C + c];
-    sh[c] = s * inv + g.tcode[t * g.C + c];
-  }
-  __syncthreads();
-  for (int o = tid; o < g.C; o += blockDim.x) {
-    float aa = g.ab[o], bb = g.bb[o];
-    for (int c = 0; c < g.C; ++c) {
-      aa = fmaf(sh[c], g.ak[(size_t)c * g.C + o], aa);
-      bb = fmaf(sh[c], g.bk[(size_t)c * g.C + o], bb);
-    }
-    g.chan[(size_t)fr * g.C + o] = make_float2(0.1f + 0.89f * dn_sigmoid(aa), dn_sigmoid(bb));
-  }
+__global__ void __launch_bounds__(256) deltanet_chan_gates_kernel(const DnChanArgs g) {
+  extern __shared__ __align__(16) float sh[];          // ctx [C], vec [2C], scratch [256]
+  const int fr = blockIdx.x;
+  float* vec = sh + g.C;
+  pdl_sync();
+  const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, 0, 1.0f / (float)(g.H * g.W)};
+  gate_ctx(src, fr, 1, sh, vec + 2 * g.C);
+  const float* const gk[2] = {g.ak, g.bk};
+  const float* const gb[2] = {g.ab, g.bb};
+  const int off[3] = {0, g.C, 2 * g.C};
+  gate_vectors<2>(gk, gb, off, 2, sh, g.C, vec, vec + 2 * g.C);
+  for (int o = threadIdx.x; o < g.C; o += blockDim.x)
+    g.chan[(size_t)fr * g.C + o] = make_float2(0.1f + 0.89f * dn_sigmoid(vec[o]), dn_sigmoid(vec[g.C + o]));
 }
 
 // k, v planes times their spatial gate planes: for every frame the 2C planes C..3C of the
@@ -188,6 +185,7 @@ __global__ void __launch_bounds__(256) deltanet_kv_gate_kernel(float* __restrict
                                                                const float* __restrict__ gsp,
                                                                size_t per_frame4, size_t fstride4,
                                                                size_t total4, size_t koff4) {
+  pdl_sync();
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= total4) return;
   const size_t fr = i / per_frame4, r = i - fr * per_frame4;
@@ -309,6 +307,7 @@ int cssm_deltanet_plan_init(const cssm_deltanet_desc* d, const cssm_deltanet_wei
 int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weights* w,
                           const void* plan, const float* x, float* y, void* workspace,
                           size_t workspace_bytes, void* stream) {
+  PdlScope pdl(d != nullptr && (size_t)d->B * d->T * d->H * d->W * d->C * 4 <= PDL_MAX_BYTES);
   int s = deltanet_validate(d);
   if (s != CSSM_OK) return s;
   if (!w || !plan || !x || !y || !workspace) return CSSM_ERR_NULL;
@@ -368,7 +367,7 @@ int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weigh
     ca.BT = BT; ca.T = d->T; ca.C = C; ca.H = d->H; ca.W = d->W;
     ca.ak = w->gate_kernel[0]; ca.ab = w->gate_bias[0]; ca.bk = w->gate_kernel[1]; ca.bb = w->gate_bias[1];
     ca.chan = (float2*)(ws + l.chan);
-    deltanet_chan_gates_kernel<<<BT, 128, (size_t)C * sizeof(float), st>>>(ca);
+    launch_k(deltanet_chan_gates_kernel, BT, 256, (size_t)(3 * C + 256) * sizeof(float), st, ca);
     if ((s = check_launch()) != CSSM_OK) return s;
     // spatial gates sigmoid(Conv1x1(rotated x)) -> planes (BT, 3C, H, W): B_k, B_v, C_gate
     float* gsp = (float*)(ws + l.gsp);
@@ -384,19 +383,21 @@ int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weigh
     // C is a multiple of 4, so every frame's planes start and end on a float4 boundary
     const size_t per_frame4 = (size_t)2 * C * HW / 4, fstride4 = (size_t)3 * C * HW / 4;
     const size_t total4 = per_frame4 * BT;
-    deltanet_kv_gate_kernel<<<(unsigned)((total4 + 255) / 256), 256, 0, st>>>(
-        qkv, gsp, per_frame4, fstride4, total4, (size_t)C * HW / 4);
+    launch_k(deltanet_kv_gate_kernel, (unsigned)((total4 + 255) / 256), 256, 0, st, qkv, gsp, per_frame4, fstride4, total4, (size_t)C * HW / 4);
     if ((s = check_launch()) != CSSM_OK) return s;
   } else {
     const int Wf = d->W / 2 + 1, NB = d->H * Wf;
-    const size_t smem = (size_t)(C + 5 * (d->H + Wf)) * sizeof(float);
-    int chunks = 1;
-    if (BT < 296) {
-      chunks = (296 + BT - 1) / BT;
-      const int maxc = (NB + 255) / 256;
-      if (chunks > maxc) chunks = maxc;
+    if (d->gate_type == CSSM_GATE_FACTORED) {
+      const size_t smem = (size_t)(C + 5 * (d->H + Wf) + 256) * sizeof(float);
+      launch_k(deltanet_gates_factored_kernel, dim3(BT, gate_chunks(BT, NB)), 256, smem, st, ga);
+    } else {
+      const int chunks = (NB + 127) / 128, G = gate_dense_frames(BT, chunks);
+      const dim3 grid(chunks, (BT + G - 1) / G);
+      const size_t smem = (size_t)(G * C + 128) * sizeof(float);
+      if (G == 8) launch_k(deltanet_gates_dense_kernel<8>, grid, 128, smem, st, ga);
+      else if (G == 4) launch_k(deltanet_gates_dense_kernel<4>, grid, 128, smem, st, ga);
+      else launch_k(deltanet_gates_dense_kernel<1>, grid, 128, smem, st, ga);
     }
-    deltanet_gates_kernel<<<dim3(BT, chunks), 256, smem, st>>>(ga);
     if ((s = check_launch()) != CSSM_OK) return s;
   }
 
@@ -416,10 +417,9 @@ int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weigh
   } else {
     // long thin planes whose DFT tables do not fit beside them
     const size_t smem = deltanet_smem_bytes(d->H, d->W);
-    cudaError_t e = cudaFuncSetAttribute(deltanet_spectral_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = func_smem(deltanet_spectral_kernel, smem);
     if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-    deltanet_spectral_kernel<<<d->B * C, GG_THREADS, smem, st>>>(sp);
+    launch_k(deltanet_spectral_kernel, d->B * C, GG_THREADS, smem, st, sp);
     if ((s = check_launch()) != CSSM_OK) return s;
   }
 

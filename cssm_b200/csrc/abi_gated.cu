@@ -1,6 +1,7 @@
 // extern "C" entry points of the gated (GatedCSSM) block and the shared error plumbing.
 #include <string.h>
 #include <stdio.h>
+#include <atomic>
 #include <cuda_bf16.h>
 #include "kernels.cuh"
 #include "gemm.cuh"
@@ -11,6 +12,40 @@ static thread_local char g_cuda_err[256] = "";
 
 void set_cuda_error(cudaError_t e) {
   snprintf(g_cuda_err, sizeof(g_cuda_err), "%s: %s", cudaGetErrorName(e), cudaGetErrorString(e));
+}
+
+thread_local int g_pdl = 0;
+
+// Open-addressed table keyed by the kernel's address; entries are only ever added, and a lost race at
+// worst repeats the call.
+cudaError_t func_smem_set(const void* kern, size_t bytes) {
+  constexpr int SLOTS = 512, DEVS = 16;
+  struct Entry { std::atomic<const void*> key; std::atomic<int> size[DEVS]; };
+  static Entry table[SLOTS];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  Entry* hit = nullptr;
+  size_t h = (reinterpret_cast<uintptr_t>(kern) >> 4) % SLOTS;
+  for (int i = 0; i < SLOTS && dev < DEVS; ++i, h = (h + 1) % SLOTS) {
+    const void* k = table[h].key.load(std::memory_order_acquire);
+    if (k == nullptr && table[h].key.compare_exchange_strong(k, kern)) k = kern;
+    if (k == kern) { hit = &table[h]; break; }
+  }
+  if (hit != nullptr && (size_t)hit->size[dev].load(std::memory_order_acquire) >= bytes && bytes > 0) return cudaSuccess;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess && hit != nullptr) hit->size[dev].store((int)bytes, std::memory_order_release);
+  return e;
+}
+
+int sm_count() {
+  static std::atomic<int> counts[16];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  if (dev < 16 && (n = counts[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+  if (dev < 16) counts[dev].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 int check_launch() {
@@ -252,6 +287,7 @@ namespace cssm {
 int gated_forward_internal(const cssm_gated_desc* d, const cssm_gated_weights* w,
                            const void* plan, const float* x, float* y, void* workspace,
                            size_t workspace_bytes, void* stream, int last_only, int x_bcast) {
+  PdlScope pdl(d != nullptr && (size_t)d->B * d->T * d->H * d->W * d->C * 4 <= PDL_MAX_BYTES);
   int s = validate(d);
   if (s != CSSM_OK) return s;
   s = validate_weights(d, w);
@@ -310,6 +346,7 @@ namespace cssm {
 // 8 elements per thread; n8 = number of 8-element groups, tail handled by the last threads
 __global__ void __launch_bounds__(256) bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ in,
                                                           float* __restrict__ out, size_t n) {
+  pdl_sync();
   const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 8;
   if (i + 8 <= n) {
     const uint4 v = *reinterpret_cast<const uint4*>(in + i);
@@ -328,6 +365,7 @@ __global__ void __launch_bounds__(256) bf16_to_f32_kernel(const __nv_bfloat16* _
 }
 __global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* __restrict__ in,
                                                           __nv_bfloat16* __restrict__ out, size_t n) {
+  pdl_sync();
   const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 8;
   if (i + 8 <= n) {
     const float4 a = *reinterpret_cast<const float4*>(in + i);
@@ -355,6 +393,7 @@ int cssm_gated_forward_bf16(const cssm_gated_desc* d, const cssm_gated_weights* 
                             const void* x_bf16, void* y, int32_t y_is_bf16, void* workspace,
                             size_t workspace_bytes, void* stream) {
   void* y_bf16 = y;
+  PdlScope pdl(d != nullptr && (size_t)d->B * d->T * d->H * d->W * d->C * 4 <= PDL_MAX_BYTES);
   const size_t base = cssm_gated_workspace_bytes(d);
   if (base == 0) return validate(d) != CSSM_OK ? validate(d) : CSSM_ERR_DIMS;
   if (!x_bf16 || !y || !workspace) return CSSM_ERR_NULL;
@@ -367,13 +406,13 @@ int cssm_gated_forward_bf16(const cssm_gated_desc* d, const cssm_gated_weights* 
   float* xf = (float*)(ws + base);
   float* yf = (float*)(ws + base + act);
   const unsigned grid = (unsigned)((n + 2047) / 2048);
-  bf16_to_f32_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)x_bf16, xf, n);
+  launch_k(bf16_to_f32_kernel, grid, 256, 0, st, (const __nv_bfloat16*)x_bf16, xf, n);
   int s = check_launch();
   if (s != CSSM_OK) return s;
   // float32 result (what Flax's promotion gives the reference) straight into y, or rounded to bf16
   s = gated_forward_internal(d, w, plan, xf, y_is_bf16 ? yf : (float*)y, workspace, base, stream, 0, 0);
   if (s != CSSM_OK || !y_is_bf16) return s;
-  f32_to_bf16_kernel<<<grid, 256, 0, st>>>(yf, (__nv_bfloat16*)y_bf16, n);
+  launch_k(f32_to_bf16_kernel, grid, 256, 0, st, yf, (__nv_bfloat16*)y_bf16, n);
   return check_launch();
 }
 

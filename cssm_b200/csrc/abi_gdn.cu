@@ -33,6 +33,7 @@ static GdnPlan gdn_plan_layout(const cssm_gdn_desc& d) {
 // (frames, 3C, HW) q/k/v buffer are multiplied by the 2C planes of the (frames, 2C, HW) gate buffer
 __global__ void __launch_bounds__(256) gdn_kv_gate_kernel(float* __restrict__ qkv, const float* __restrict__ gsp,
                                                           size_t per_frame4, size_t total4) {
+  pdl_sync();
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= total4) return;
   const size_t fr = i / per_frame4, r = i - fr * per_frame4;
@@ -184,6 +185,7 @@ int cssm_gdn_forward_timed(const cssm_gdn_desc* d, const cssm_gdn_weights* w, co
 int cssm::gdn_forward_internal(const cssm_gdn_desc* d, const cssm_gdn_weights* w, const void* plan,
                                const float* x, float* y, void* workspace, size_t workspace_bytes,
                                void* stream, int last_only, int x_bcast) {
+  PdlScope pdl(d != nullptr && (size_t)d->B * d->T * d->H * d->W * d->C * 4 <= PDL_MAX_BYTES);
   const int static_image = x_bcast == 2 ? 1 : 0;
   if (static_image) {
     x_bcast = 0;
@@ -329,7 +331,7 @@ int cssm::gdn_forward_internal(const cssm_gdn_desc* d, const cssm_gdn_weights* w
     if ((s = launch_gemm<false, true>(g, st)) != CSSM_OK) return s;
     if (((size_t)C * HW) % 8 != 0) return CSSM_ERR_UNSUPPORTED;
     const size_t per_frame4 = (size_t)2 * C * HW / 4, total4 = per_frame4 * BT;
-    gdn_kv_gate_kernel<<<(unsigned)((total4 + 255) / 256), 256, 0, st>>>(qkv, gsp, per_frame4, total4);
+    launch_k(gdn_kv_gate_kernel, (unsigned)((total4 + 255) / 256), 256, 0, st, qkv, gsp, per_frame4, total4);
     if ((s = check_launch()) != CSSM_OK) return s;
   }
 

@@ -11,6 +11,7 @@ namespace cssm {
 __global__ void __launch_bounds__(256) cl_to_planar_kernel(const float* __restrict__ x,
                                                            float* __restrict__ planar, int frames,
                                                            int HW, int C) {
+  pdl_sync();
   __shared__ float tile[32][33];
   const int ptiles = (HW + 31) / 32, ctiles = (C + 31) / 32;
   int bid = blockIdx.x;
@@ -78,6 +79,7 @@ int cssm_nogate_plan_init(const cssm_nogate_desc* d, const cssm_nogate_weights* 
 int cssm_nogate_forward(const cssm_nogate_desc* d, const cssm_nogate_weights* w, const void* plan,
                         const float* x, float* y, void* workspace, size_t workspace_bytes,
                         void* stream) {
+  PdlScope pdl(d != nullptr && (size_t)d->B * d->T * d->H * d->W * d->C * 4 <= PDL_MAX_BYTES);
   int s = nogate_validate(d);
   if (s != CSSM_OK) return s;
   if (!w || !w->out_proj_kernel || !w->out_proj_bias || !plan || !x || !y || !workspace) return CSSM_ERR_NULL;
@@ -88,7 +90,7 @@ int cssm_nogate_forward(const cssm_nogate_desc* d, const cssm_nogate_weights* w,
   const int frames = d->B * d->T, HW = d->H * d->W;
   const long long tiles = (long long)frames * ((HW + 31) / 32) * ((d->C + 31) / 32);
   if (tiles > 0x7fffffffLL) return CSSM_ERR_DIMS;
-  cl_to_planar_kernel<<<(unsigned)tiles, 256, 0, st>>>(x, planar, frames, HW, d->C);
+  launch_k(cl_to_planar_kernel, (unsigned)tiles, 256, 0, st, x, planar, frames, HW, d->C);
   if ((s = check_launch()) != CSSM_OK) return s;
   s = launch_spectral(d->B, d->T, d->H, d->W, d->C, (const cf*)plan, nullptr, planar, 0, 1, st);
   if (s != CSSM_OK) return s;

@@ -422,6 +422,7 @@ int cssm_shvit_block_plan_init(const cssm_shvit_block_desc* d, const cssm_shvit_
 int cssm_shvit_block_forward(const cssm_shvit_block_desc* d, const cssm_shvit_block_weights* w, const void* plan,
                              const void* x_bf16, void* y_bf16, void* workspace, size_t workspace_bytes,
                              void* stream) {
+  PdlScope pdl(true);
   int s = block_validate(d);
   if (s != CSSM_OK) return s;
   if (!w || !plan || !x_bf16 || !y_bf16 || !workspace) return CSSM_ERR_NULL;
@@ -478,6 +479,7 @@ int cssm_shvit_plan_init(const cssm_shvit_desc* d, const cssm_shvit_weights* w, 
 }
 int cssm_shvit_forward(const cssm_shvit_desc* d, const cssm_shvit_weights* w, const void* plan, const void* x_bf16,
                        float* logits, void* workspace, size_t workspace_bytes, void* stream) {
+  PdlScope pdl(true);
   int s = model_validate(d);
   if (s != CSSM_OK) return s;
   if (!w || !plan || !x_bf16 || !logits || !workspace) return CSSM_ERR_NULL;

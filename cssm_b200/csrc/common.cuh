@@ -77,6 +77,44 @@ struct FastDiv {
   }
 };
 
+// ---- launches ----
+// Programmatic dependent launch: inside a PdlScope every kernel but the first is launched so that its
+// CTAs may become resident while the one before still runs.  Each kernel waits (pdl_wait) before it
+// touches anything an earlier kernel writes or reads, and only then lets the next one start
+// (pdl_trigger), so at most two kernels of a chain overlap and what a kernel does ahead of its wait
+// (barriers, TMEM, tables, weights) may rely on everything before the chain's first kernel.
+// It pays where launches are short (CSSM-SHViT, one image: 630 -> 487 us); with activations of 1 GB, launches of
+// 0.5 ms and more, passes got 3 % slower, so the block drivers turn it on up to PDL_MAX_BYTES a tensor.
+extern thread_local int g_pdl;            // 0 off, 1 first launch of a scope pending, 2 on
+constexpr size_t PDL_MAX_BYTES = (size_t)256 << 20;
+struct PdlScope {
+  int prev;
+  explicit PdlScope(bool on) : prev(g_pdl) { if (g_pdl == 0 && on) g_pdl = 1; }
+  ~PdlScope() { g_pdl = prev; }
+};
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_sync() { pdl_wait(); pdl_trigger(); }
+
+template <class... P, class... A>
+inline void launch_k(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.attrs = at; cfg.numAttrs = g_pdl == 2 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);     // errors are read by check_launch
+  if (g_pdl == 1) g_pdl = 2;
+}
+// cudaFuncAttributeMaxDynamicSharedMemorySize, set once per kernel, device and size (the call costs as
+// much host time as a launch)
+cudaError_t func_smem_set(const void* kern, size_t bytes);
+template <class F> inline cudaError_t func_smem(F* kern, size_t bytes) {
+  return func_smem_set(reinterpret_cast<const void*>(kern), bytes);
+}
+int sm_count();                           // of the current device
+
 // Host-side record of the last CUDA error seen on this thread.
 void set_cuda_error(cudaError_t e);
 int check_launch();

@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) gdn_spectral_dft(const GdnSpectr
   const int Tdata = a.static_image ? 1 : a.T;           // frames of q, k, v per batch element
   dp_fill_table<NT>(TW, g.W, g.ldw);
   dp_fill_table<NT>(TH, g.H, g.ldh);
+  pdl_sync();
 
   for (int grp = blockIdx.x; grp < d.groups; grp += gridDim.x) {
     const int b = grp / d.hgroups, h0 = (grp - b * d.hgroups) * d.heads, nhd = min(d.heads, nh - h0), n = nhd * DK;
@@ -207,6 +208,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) deltanet_spectral_dft(const DnSp
   const bool chan = a.chan != nullptr;
   dp_fill_table<NT>(TW, g.W, g.ldw);
   dp_fill_table<NT>(TH, g.H, g.ldh);
+  pdl_sync();
 
   for (int grp = blockIdx.x; grp < d.groups; grp += gridDim.x) {
     const int b = grp / d.hgroups, c0 = (grp - b * d.hgroups) * d.heads, n = min(d.heads, a.C - c0);
@@ -293,10 +295,10 @@ static bool delta_dft_plan(int B, int T, int C, int H, int W, int dk, bool need_
 
 template <class Kern, class Args>
 static int delta_dft_launch(Kern kern, const Args& a, const DeltaDftArgs& d, const DpChoice& ch, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ch.smem);
+  cudaError_t e = func_smem(kern, ch.smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   const int slots = 148 * ch.ctas;
-  kern<<<d.groups < slots ? d.groups : slots, ch.threads, ch.smem, st>>>(a, d);
+  launch_k(kern, d.groups < slots ? d.groups : slots, ch.threads, ch.smem, st, a, d);
   return check_launch();
 }
 

@@ -23,6 +23,7 @@ constexpr int D32_SPEC_CF = 2 * 8 * D32_THREADS;       // [q, k][r][thread]
 constexpr int D32_SMEM_BYTES = (D32_EX_CF + D32_ZR_CF + D32_GB_CF + D32_SPEC_CF) * 8;
 
 __global__ void __launch_bounds__(D32_THREADS, 2) deltanet_spectral_r32(const DnSpectralArgs a) {
+  pdl_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cf* EX = reinterpret_cast<cf*>(smem_raw);
   cf* ZR = EX + D32_EX_CF;
@@ -210,10 +211,9 @@ __global__ void __launch_bounds__(D32_THREADS, 2) deltanet_spectral_r32(const Dn
 
 int launch_deltanet_spectral_r32(const DnSpectralArgs& a, cudaStream_t st) {
   if (a.H != 32 || a.W != 32 || a.C % 4 != 0) return CSSM_ERR_UNSUPPORTED;
-  cudaError_t e = cudaFuncSetAttribute(deltanet_spectral_r32,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, D32_SMEM_BYTES);
+  cudaError_t e = func_smem(deltanet_spectral_r32, D32_SMEM_BYTES);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  deltanet_spectral_r32<<<a.B * (a.C / 4), D32_THREADS, D32_SMEM_BYTES, st>>>(a);
+  launch_k(deltanet_spectral_r32, a.B * (a.C / 4), D32_THREADS, D32_SMEM_BYTES, st, a);
   return check_launch();
 }
 

@@ -16,6 +16,7 @@ namespace cssm {
 constexpr int DN64_SMEM_BYTES = (R64_EX_CF + R64_ZR_CF + R64_GB_CF + 2 * 8 * R64_NT) * (int)sizeof(cf);
 
 __global__ void __launch_bounds__(R64_NT, 2) deltanet_spectral_r64(const DnSpectralArgs a) {
+  pdl_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cf* EX = reinterpret_cast<cf*>(smem_raw);
   cf* SQ = EX + R64_EX_CF + R64_ZR_CF + R64_GB_CF;      // [8][288] q spectrum, lane-private slots
@@ -154,10 +155,9 @@ __global__ void __launch_bounds__(R64_NT, 2) deltanet_spectral_r64(const DnSpect
 
 int launch_deltanet_spectral_r64(const DnSpectralArgs& a, cudaStream_t st) {
   if (a.H != 64 || a.W != 64) return CSSM_ERR_UNSUPPORTED;
-  cudaError_t e = cudaFuncSetAttribute(deltanet_spectral_r64,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, DN64_SMEM_BYTES);
+  cudaError_t e = func_smem(deltanet_spectral_r64, DN64_SMEM_BYTES);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  deltanet_spectral_r64<<<a.B * a.C, R64_NT, DN64_SMEM_BYTES, st>>>(a);
+  launch_k(deltanet_spectral_r64, a.B * a.C, R64_NT, DN64_SMEM_BYTES, st, a);
   return check_launch();
 }
 

@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(R64_THREADS, 2)
 gated_spectral_r64(float* __restrict__ xz, const cf* __restrict__ khat,
                    const float4* __restrict__ gates, int T, int C,
                    const __grid_constant__ CUtensorMap pmap, const float* __restrict__ dchan) {
+  pdl_sync();
   constexpr int last_only = LAST ? 1 : 0;
   constexpr int PRS = 68;                                     // floats per staged row
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -205,6 +206,7 @@ __global__ void __launch_bounds__(GEN_THREADS)
 gated_spectral_generic(float* __restrict__ xz, const cf* __restrict__ khat,
                        const float4* __restrict__ gates, int T, int C, int H, int W, int last_only,
                        int nog, const float* __restrict__ dchan) {
+  pdl_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int Wf = W / 2 + 1, HW = H * W, NB = H * Wf;
   float* xs = reinterpret_cast<float*>(smem_raw);              // [H][W]
@@ -353,21 +355,18 @@ int launch_spectral(int B, int T, int H, int W, int C, const cf* khat, const flo
     if (nogate == 1) kern = last_only ? gated_spectral_r64<true, 1> : gated_spectral_r64<false, 1>;
     else if (nogate == 2) kern = last_only ? gated_spectral_r64<true, 2> : gated_spectral_r64<false, 2>;
     else if (nogate == 3) kern = last_only ? gated_spectral_r64<true, 3> : gated_spectral_r64<false, 3>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = func_smem(kern, smem);
     if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-    kern<<<grid, R64_THREADS, smem, st>>>(xz, khat, reinterpret_cast<const float4*>(gates), d.T,
+    launch_k(kern, grid, R64_THREADS, smem, st, xz, khat, reinterpret_cast<const float4*>(gates), d.T,
                                           d.C, pmap, dchan);
   } else if (gated_spectral_dft_fits(d.H, d.W, d.T)) {
     return launch_gated_spectral_dft(d.B, d.T, d.H, d.W, d.C, khat, gates, xz, last_only, nogate, st, dchan);
   } else {
     const size_t smem = generic_smem_bytes(d.H, d.W);
     if (smem > 200 * 1024) return CSSM_ERR_UNSUPPORTED;
-    cudaError_t e = cudaFuncSetAttribute(gated_spectral_generic,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = func_smem(gated_spectral_generic, smem);
     if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-    gated_spectral_generic<<<grid, GEN_THREADS, smem, st>>>(
-        xz, khat, reinterpret_cast<const float4*>(gates), d.T, d.C, d.H, d.W, last_only, nogate, dchan);
+    launch_k(gated_spectral_generic, grid, GEN_THREADS, smem, st, xz, khat, reinterpret_cast<const float4*>(gates), d.T, d.C, d.H, d.W, last_only, nogate, dchan);
   }
   return check_launch();
 }

@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
   const int HW = g.H * g.W, NB = g.H * g.Wp, ldx = a.ldx, ldc = a.ldc;
   dp_fill_table<NT>(TW, g.W, g.ldw);
   dp_fill_table<NT>(TH, g.H, g.ldh);
+  pdl_sync();
   const int cgroups = (a.C + a.P - 1) / a.P;
   const float invHW = 1.0f / (float)HW;
   const bool keep = a.T > 1;
@@ -163,10 +164,10 @@ int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat,
   a.ldx = dp_ld_rows(a.g, ch.P); a.ldc = dp_ld_cols(a.g, ch.P);
   auto kern = ch.threads == 256 ? (ch.wide ? gated_spectral_dft<2, 4, 256> : gated_spectral_dft<1, 2, 256>)
                                 : (ch.wide ? gated_spectral_dft<2, 4, 128> : gated_spectral_dft<1, 2, 128>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ch.smem);
+  cudaError_t e = func_smem(kern, ch.smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   const int slots = 148 * ch.ctas;
-  kern<<<a.groups < slots ? a.groups : slots, ch.threads, ch.smem, st>>>(a);
+  launch_k(kern, a.groups < slots ? a.groups : slots, ch.threads, ch.smem, st, a);
   return check_launch();
 }
 

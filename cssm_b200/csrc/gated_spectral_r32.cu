@@ -24,6 +24,7 @@ template <bool LAST, int MODE>
 __global__ void __launch_bounds__(R32_THREADS, 2)
 gated_spectral_r32(float* __restrict__ xz, const cf* __restrict__ khat,
                    const float4* __restrict__ gates, int T, int C, const float* __restrict__ dchan) {
+  pdl_sync();
   constexpr int last_only = LAST ? 1 : 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cf* EX = reinterpret_cast<cf*>(smem_raw);
@@ -169,11 +170,9 @@ int launch_gated_spectral_r32(float* xz, const cf* khat, const float* gates, int
   if (nogate == 1) kern = last_only ? gated_spectral_r32<true, 1> : gated_spectral_r32<false, 1>;
   if (nogate == 2) kern = last_only ? gated_spectral_r32<true, 2> : gated_spectral_r32<false, 2>;
   if (nogate == 3) kern = last_only ? gated_spectral_r32<true, 3> : gated_spectral_r32<false, 3>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       R32_SMEM_BYTES);
+  cudaError_t e = func_smem(kern, R32_SMEM_BYTES);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  kern<<<B * (C / 4), R32_THREADS, R32_SMEM_BYTES, st>>>(
-      xz, khat, reinterpret_cast<const float4*>(gates), T, C, dchan);
+  launch_k(kern, B * (C / 4), R32_THREADS, R32_SMEM_BYTES, st, xz, khat, reinterpret_cast<const float4*>(gates), T, C, dchan);
   return check_launch();
 }
 

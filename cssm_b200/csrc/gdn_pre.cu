@@ -2,6 +2,7 @@
 // per-row context sums, and the gate maps (alpha, beta per frequency bin; B_k, B_v per pixel).
 #include "kernels.cuh"
 #include "bf16_ops.cuh"
+#include "gates.cuh"
 
 namespace cssm {
 
@@ -24,6 +25,7 @@ __device__ __forceinline__ int dw_pos(int col, int c) {
 
 template <int K, int DW_CG>
 __global__ void __launch_bounds__(DW_THREADS, (K <= 5 ? 2 : 1)) rope_dwconv_cl_kernel(const GdnDwArgs a) {
+  pdl_sync();
   extern __shared__ __align__(16) float sm[];
   constexpr int LO = (K - 1) / 2, NR = DW_ROWS + K - 1;
   const int W = a.W, C = a.C, n2 = C / 2;
@@ -173,6 +175,7 @@ __global__ void __launch_bounds__(DW_THREADS, (K <= 5 ? 2 : 1)) rope_dwconv_cl_k
 // combined once per row, the w part comes from the table per element.
 constexpr int CTX_WARPS = 8;
 __global__ void __launch_bounds__(CTX_WARPS * 32) rope_ctx_rowsum_kernel(const GdnDwArgs a) {
+  pdl_sync();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long row = (long long)blockIdx.x * CTX_WARPS + warp;        // (frame, h)
   if (row >= (long long)a.BT * a.H) return;
@@ -206,11 +209,10 @@ template <int K, int DW_CG>
 static int launch_dw_cg(const GdnDwArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)(DW_ROWS + K - 1) * ((a.W + K - 1 + 1) & ~1) * DW_CG * sizeof(float);
   if (smem > 200 * 1024) return CSSM_ERR_UNSUPPORTED;
-  cudaError_t e = cudaFuncSetAttribute(rope_dwconv_cl_kernel<K, DW_CG>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = func_smem(rope_dwconv_cl_kernel<K, DW_CG>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   const int bands = (a.H + DW_ROWS - 1) / DW_ROWS;
-  rope_dwconv_cl_kernel<K, DW_CG><<<a.BT * bands * (a.C / DW_CG), DW_THREADS, smem, st>>>(a);
+  launch_k(rope_dwconv_cl_kernel<K, DW_CG>, a.BT * bands * (a.C / DW_CG), DW_THREADS, smem, st, a);
   return check_launch();
 }
 
@@ -225,7 +227,7 @@ int launch_rope_dwconv_cl(const GdnDwArgs& a, cudaStream_t st) {
   if (a.ksz <= 1 && a.out == nullptr) {
     if (a.ctx_part == nullptr) return CSSM_OK;
     const long long rows = (long long)a.BT * a.H;
-    rope_ctx_rowsum_kernel<<<(unsigned)((rows + CTX_WARPS - 1) / CTX_WARPS), CTX_WARPS * 32, 0, st>>>(a);
+    launch_k(rope_ctx_rowsum_kernel, (unsigned)((rows + CTX_WARPS - 1) / CTX_WARPS), CTX_WARPS * 32, 0, st, a);
     return check_launch();
   }
   switch (a.ksz > 1 ? a.ksz : 1) {
@@ -243,41 +245,28 @@ int launch_rope_dwconv_cl(const GdnDwArgs& a, cudaStream_t st) {
 // alpha = 0.1 + 0.89 * raw.  Stored as float2 {alpha, beta} at bin_index(path, kh, kw).
 // B_k / B_v: same over (h, w) pixels, float2 {B_k, B_v} at h*W + w.  cssm.py:4798-4848, 4864-4865.
 __global__ void __launch_bounds__(256) gdn_gates_kernel(const GdnGateArgs g) {
-  extern __shared__ float sh[];
+  extern __shared__ __align__(16) float sh[];
   const int Wf = g.W / 2 + 1, NB = g.H * Wf, HW = g.H * g.W;
   float* ctx = sh;                       // [C]
-  float* vec = sh + g.C;                 // factored: alpha_h, alpha_w, beta_h, beta_w, Bk_h, Bk_w, Bv_h, Bv_w
-  const int fr = blockIdx.x, tid = threadIdx.x, t = fr % g.T;
-  const float inv = 1.0f / (float)HW;
-  for (int c = tid; c < g.C; c += blockDim.x) {
-    float s = 0.f;
-    const int fsrc = g.ctx_per_clip ? fr / g.T : fr;
-    for (int h = 0; h < g.H; ++h) s += g.ctx_part[((size_t)fsrc * g.H + h) * g.C + c];
-    ctx[c] = s * inv + g.tcode[t * g.C + c];
-  }
-  __syncthreads();
+  float* scratch = sh + g.C;             // [256]
+  float* vec = scratch + 256;            // factored: alpha_h, alpha_w, beta_h, beta_w, Bk_h, Bk_w, Bv_h, Bv_w
+  const int fr = blockIdx.x, tid = threadIdx.x;
+  pdl_sync();
+  const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, g.ctx_per_clip, 1.0f / (float)HW};
+  gate_ctx(src, fr, 1, ctx, scratch);
   const int ngate = g.use_input_gates ? 4 : 2;
   if (g.gate_type == CSSM_GATE_FACTORED) {
     // segment offsets inside vec
     int off[9];
     off[0] = 0;
+#pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int wd = q < 2 ? Wf : g.W;
       off[2 * q + 1] = off[2 * q] + g.H;
       off[2 * q + 2] = off[2 * q + 1] + wd;
     }
-    const int total = off[2 * ngate];
-    for (int o = tid; o < total; o += blockDim.x) {
-      int seg = 0;
-      while (o >= off[seg + 1]) ++seg;
-      const int col = o - off[seg];
-      const int ncol = off[seg + 1] - off[seg];
-      const float* kk = g.gk[seg];
-      float acc = g.gb[seg][col];
-      for (int c = 0; c < g.C; ++c) acc = fmaf(ctx[c], kk[(size_t)c * ncol + col], acc);
-      vec[o] = acc;
-    }
-    __syncthreads();
+    if (g.use_input_gates) gate_vectors<8>(g.gk, g.gb, off, 8, ctx, g.C, vec, scratch);
+    else gate_vectors<8>(g.gk, g.gb, off, 4, ctx, g.C, vec, scratch);
     for (int bin = tid; bin < NB; bin += blockDim.x) {
       const int kh = bin / Wf, kw = bin % Wf;
       const float ra = sigmoid_f(vec[off[0] + kh] + vec[off[1] + kw]);
@@ -290,18 +279,15 @@ __global__ void __launch_bounds__(256) gdn_gates_kernel(const GdnGateArgs g) {
         g.bkv[(size_t)fr * HW + px] = make_float2(sigmoid_f(vec[off[4] + h] + vec[off[5] + w]),
                                                   sigmoid_f(vec[off[6] + h] + vec[off[7] + w]));
       }
-  } else if (g.gate_type == CSSM_GATE_SCALAR || g.gate_type == CSSM_GATE_CHANNEL) {
+  } else {
     // scalar: one value per frame and gate, Dense(1)(ctx) (cssm.py:4825-4833).  channel: alpha, beta
     // per head, Dense(n_h)(ctx) (cssm.py:4808-4810); its spatial gates are a 1x1 conv of the block
     // input and are applied elsewhere.  The maps are constant over the bins.
     const bool chan = g.gate_type == CSSM_GATE_CHANNEL;
     const int nout = chan ? g.nh : 1, nvec = chan ? 2 : ngate;
-    for (int o = tid; o < nvec * nout; o += blockDim.x) {
-      const int gi = o / nout, col = o - gi * nout;
-      float acc = g.gb[gi][col];
-      for (int c = 0; c < g.C; ++c) acc = fmaf(ctx[c], g.gk[gi][(size_t)c * nout + col], acc);
-      vec[o] = sigmoid_f(acc);
-    }
+    const int off[9] = {0, nout, 2 * nout, 3 * nout, 4 * nout, 0, 0, 0, 0};
+    gate_vectors<8>(g.gk, g.gb, off, nvec, ctx, g.C, vec, scratch);
+    for (int o = tid; o < nvec * nout; o += blockDim.x) vec[o] = sigmoid_f(vec[o]);
     __syncthreads();
     for (int i = tid; i < nout * NB; i += blockDim.x) {
       const int hh = i / NB;
@@ -309,32 +295,46 @@ __global__ void __launch_bounds__(256) gdn_gates_kernel(const GdnGateArgs g) {
     }
     if (!chan && g.use_input_gates)
       for (int px = tid; px < HW; px += blockDim.x) g.bkv[(size_t)fr * HW + px] = make_float2(vec[2], vec[3]);
-  } else {
-    for (int bin = tid; bin < NB; bin += blockDim.x) {
-      const int kh = bin / Wf, kw = bin % Wf;
-      float aa = g.gb[0][bin], bb = g.gb[1][bin];
-      for (int c = 0; c < g.C; ++c) {
-        aa = fmaf(ctx[c], g.gk[0][(size_t)c * NB + bin], aa);
-        bb = fmaf(ctx[c], g.gk[1][(size_t)c * NB + bin], bb);
-      }
-      g.ab[(size_t)fr * NB + bin_index(g.path, kh, kw, g.H, Wf)] =
-          make_float2(0.1f + 0.89f * sigmoid_f(aa), sigmoid_f(bb));
-    }
-    if (g.use_input_gates)
-      for (int px = tid; px < HW; px += blockDim.x) {
-        float aa = g.gb[2][px], bb = g.gb[3][px];
-        for (int c = 0; c < g.C; ++c) {
-          aa = fmaf(ctx[c], g.gk[2][(size_t)c * HW + px], aa);
-          bb = fmaf(ctx[c], g.gk[3][(size_t)c * HW + px], bb);
-        }
-        g.bkv[(size_t)fr * HW + px] = make_float2(sigmoid_f(aa), sigmoid_f(bb));
-      }
+  }
+}
+
+// Dense gates: a thread owns one bin (blockIdx.x < bin_chunks) or one pixel of G frames.
+template <int G>
+__global__ void __launch_bounds__(128) gdn_gates_dense_kernel(const GdnGateArgs g, int bin_chunks) {
+  extern __shared__ __align__(16) float sh[];
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, HW = g.H * g.W, f0 = blockIdx.y * G, nf = min(G, g.BT - f0);
+  pdl_sync();
+  const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, g.ctx_per_clip, 1.0f / (float)HW};
+  gate_ctx(src, f0, nf, sh, sh + G * g.C);
+  const bool bins = (int)blockIdx.x < bin_chunks;
+  const int i = (blockIdx.x - (bins ? 0 : bin_chunks)) * 128 + threadIdx.x, n = bins ? NB : HW;
+  if (i >= n) return;
+  float r[2][G];
+  gate_dense<2, G>(g.gk + (bins ? 0 : 2), g.gb + (bins ? 0 : 2), n, i, g.C, sh, r);
+  const int kh = i / Wf, o = bin_index(g.path, kh, i - kh * Wf, g.H, Wf);
+#pragma unroll
+  for (int f = 0; f < G; ++f) {
+    if (f >= nf) continue;
+    const float a = sigmoid_f(r[0][f]), b = sigmoid_f(r[1][f]);
+    if (bins) g.ab[(size_t)(f0 + f) * NB + o] = make_float2(0.1f + 0.89f * a, b);
+    else g.bkv[(size_t)(f0 + f) * HW + i] = make_float2(a, b);
   }
 }
 
 int launch_gdn_gates(const GdnGateArgs& g, cudaStream_t st) {
-  const size_t smem = (size_t)(g.C + 4 * g.H + 2 * (g.W / 2 + 1) + 2 * g.W + 2 * g.nh + 8) * sizeof(float);
-  gdn_gates_kernel<<<g.BT, 256, smem, st>>>(g);
+  const int Wf = g.W / 2 + 1;
+  if (g.gate_type == CSSM_GATE_DENSE) {
+    const int bc = (g.H * Wf + 127) / 128, chunks = bc + (g.use_input_gates ? (g.H * g.W + 127) / 128 : 0);
+    const int G = gate_dense_frames(g.BT, chunks);
+    const dim3 grid(chunks, (g.BT + G - 1) / G);
+    const size_t smem = (size_t)(G * g.C + 128) * sizeof(float);
+    if (G == 8) launch_k(gdn_gates_dense_kernel<8>, grid, 128, smem, st, g, bc);
+    else if (G == 4) launch_k(gdn_gates_dense_kernel<4>, grid, 128, smem, st, g, bc);
+    else launch_k(gdn_gates_dense_kernel<1>, grid, 128, smem, st, g, bc);
+    return check_launch();
+  }
+  const size_t smem = (size_t)(g.C + 256 + 4 * g.H + 2 * Wf + 2 * g.W + 4 * g.nh + 8) * sizeof(float);
+  launch_k(gdn_gates_kernel, g.BT, 256, smem, st, g);
   return check_launch();
 }
 

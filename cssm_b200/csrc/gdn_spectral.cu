@@ -29,6 +29,7 @@ __device__ __forceinline__ cf gdn_bin_update(cf* S, size_t ss, int dk, const cf*
 
 // ================================================================ generic planes ====
 __global__ void __launch_bounds__(GG_THREADS) gdn_spectral_generic(const GdnSpectralArgs a) {
+  pdl_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int H = a.H, W = a.W, dk = a.dk;
   const int Wf = W / 2 + 1, HW = H * W, NB = H * Wf;
@@ -171,10 +172,9 @@ int launch_gdn_spectral(const GdnSpectralArgs& a, cudaStream_t st) {
   // long thin planes whose DFT tables do not fit beside them
   const size_t smem = gdn_generic_smem_bytes(a.H, a.W, a.dk);
   if (smem > 220 * 1024) return CSSM_ERR_UNSUPPORTED;
-  cudaError_t e = cudaFuncSetAttribute(gdn_spectral_generic,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = func_smem(gdn_spectral_generic, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  gdn_spectral_generic<<<a.B * (a.C / a.dk), GG_THREADS, smem, st>>>(a);
+  launch_k(gdn_spectral_generic, a.B * (a.C / a.dk), GG_THREADS, smem, st, a);
   return check_launch();
 }
 

@@ -26,6 +26,7 @@ constexpr int G32_SMEM_BYTES = (G32_EX_CF + G32_ZR_CF + G32_GB_CF + G32_SPEC_CF 
 // STATIC: static-image fast path (one data frame per batch element, the T gate steps run per bin).
 template <bool LAST, bool STATIC>
 __global__ void __launch_bounds__(G32_THREADS, 1) gdn_spectral_r32(const GdnSpectralArgs a) {
+  pdl_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cf* EX = reinterpret_cast<cf*>(smem_raw);
   cf* ZR = EX + G32_EX_CF;
@@ -219,10 +220,9 @@ __global__ void __launch_bounds__(G32_THREADS, 1) gdn_spectral_r32(const GdnSpec
 int launch_gdn_spectral_r32(const GdnSpectralArgs& a, cudaStream_t st) {
   auto kern = a.static_image ? gdn_spectral_r32<false, true>
                              : (a.last_only ? gdn_spectral_r32<true, false> : gdn_spectral_r32<false, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       G32_SMEM_BYTES);
+  cudaError_t e = func_smem(kern, G32_SMEM_BYTES);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  kern<<<a.B * (a.C / 4), G32_THREADS, G32_SMEM_BYTES, st>>>(a);
+  launch_k(kern, a.B * (a.C / 4), G32_THREADS, G32_SMEM_BYTES, st, a);
   return check_launch();
 }
 

@@ -16,6 +16,7 @@ constexpr int G64_SMEM_CF = R64_EX_CF + R64_ZR_CF + R64_GB_CF + G64_SPEC_CF;
 // STATIC: static-image fast path (one data frame per batch element, the T gate steps run per bin).
 template <bool LAST, bool STATIC>
 __global__ void __launch_bounds__(R64_NT, 1) gdn_spectral_r64(const GdnSpectralArgs a) {
+  pdl_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cf* EX = reinterpret_cast<cf*>(smem_raw);
   cf* ZR = EX + R64_EX_CF;
@@ -208,9 +209,9 @@ int launch_gdn_spectral_r64(const GdnSpectralArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)G64_SMEM_CF * sizeof(cf);
   auto kern = a.static_image ? gdn_spectral_r64<false, true>
                              : (a.last_only ? gdn_spectral_r64<true, false> : gdn_spectral_r64<false, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  kern<<<a.B * (a.C / 4), R64_NT, smem, st>>>(a);
+  launch_k(kern, a.B * (a.C / 4), R64_NT, smem, st, a);
   return check_launch();
 }
 

@@ -120,10 +120,21 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
   if (warp == 0) {
     // ================================ TMA producer ================================
     if (lane == 0) {
+      // Weights do not depend on the kernel before this one: the resident ones, or the weight tiles of
+      // the first ring round, are on their way before the wait for it.
+      int npre = 0;
       if (wres) {
         tc::mbar_expect_tx(wfull, wres_bytes);
         for (int kb = 0; kb < kblocks; ++kb) tc::tma_load_2d(smem + (uint32_t)kb * BN * 128u, &bmap, kb * GB_BK, 0, wfull);
+      } else if (!IM2COL && blockIdx.x < num_tiles) {
+        const int n0 = (blockIdx.x % n_tiles) * g.BN;
+        const uint32_t a_bytes = g.conv_tma ? (uint32_t)(g.Wbox * g.Hbox * g.Bbox) * 128u : GB_A_BYTES;
+        for (; npre < NS && npre < kblocks; ++npre) {
+          tc::mbar_expect_tx(&full[npre], a_bytes + BN * 128u);
+          tc::tma_load_2d(ring + (uint32_t)npre * stage_bytes + GB_A_BYTES, &bmap, npre * GB_BK, n0, &full[npre]);
+        }
       }
+      pdl_sync();
       int it = 0;
       for (int tile = blockIdx.x; tile < num_tiles && !bad; tile += gridDim.x) {
         const int mt = tile / n_tiles;
@@ -142,7 +153,8 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
           if (!tc::mbar_wait(&empty[s], ((it / NS) & 1) ^ 1)) { atomicExch(&g_bf16_error, 5); bad = true; break; }
           unsigned char* a_s = ring + (uint32_t)s * stage_bytes;
           unsigned char* b_s = a_s + GB_A_BYTES;
-          tc::mbar_expect_tx(&full[s], (IM2COL ? 0u : a_bytes) + (wres ? 0u : BN * 128u));
+          const bool pre = it < npre;                       // its weight tile is already on the way
+          if (!pre) tc::mbar_expect_tx(&full[s], (IM2COL ? 0u : a_bytes) + (wres ? 0u : BN * 128u));
           if (g.conv_tma) {
             const int pos = kb / g.kb_per_tap, cb = kb - pos * g.kb_per_tap;
             const int pr = pos / g.pos_w, pc = pos - pr * g.pos_w;
@@ -150,7 +162,7 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
           } else if (!IM2COL) {
             tc::tma_load_2d(a_s, &amap, kb * GB_BK, m0, &full[s]);
           }
-          if (!wres) tc::tma_load_2d(b_s, &bmap, kb * GB_BK, n0, &full[s]);
+          if (!wres && !pre) tc::tma_load_2d(b_s, &bmap, kb * GB_BK, n0, &full[s]);
         }
       }
     }
@@ -197,6 +209,7 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
     const int half = (warp - 2) >> 2;
     const int row = q * 32 + lane;
     const uint32_t tlane = tmem_base + ((uint32_t)(q * 32) << 16);
+    pdl_wait();
     // bias, activation on 32 accumulator columns starting at tile column c0
     auto act32 = [&](const uint32_t (&r)[32], int n, float (&v)[32]) {
 #pragma unroll
@@ -397,6 +410,7 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
     }
   } else if (IM2COL) {
     // ================================ im2col producers ================================
+    pdl_wait();
     // lane = (row group rg, chunk c): the eight lanes of a group read the eight 16-byte chunks of one
     // output pixel's K block (contiguous channels of one or two taps); thread handles rows rg + 16 i.
     const int pt = tid - 10 * 32;                 // 0..127
@@ -628,10 +642,8 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
   }
   if (!make_kmajor_map(&bmap, g.Wt, (uint64_t)g.N, (uint64_t)g.Kpad, (uint64_t)g.ldw, (uint32_t)g.BN))
     return CSSM_ERR_CUDA;
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  const int sms = sm_count();
+  cudaError_t e;
   const int tiles = m_tiles * (g.N / g.BN);
   const int grid = tiles < sms ? tiles : sms;
   // Weights of at most 64 KB that form a single N tile stay resident in shared memory (a weight tile
@@ -659,9 +671,9 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
   auto kern = im2col ? (tma_out ? gemm_bf16_kernel<true, true, false> : gemm_bf16_kernel<true, false, false>)
                      : (tma_out ? (rtma ? gemm_bf16_kernel<false, true, true> : gemm_bf16_kernel<false, true, false>)
                                 : gemm_bf16_kernel<false, false, false>);
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  kern<<<grid, im2col ? GB_THREADS_CONV : GB_THREADS_PLAIN, smem, st>>>(g, amap, bmap, omap, rmap);
+  launch_k(kern, grid, im2col ? GB_THREADS_CONV : GB_THREADS_PLAIN, smem, st, g, amap, bmap, omap, rmap);
   return check_launch();
 }
 

@@ -161,6 +161,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_sync();
 
   if (warp < GS_MMA_WARP) {
     // ================================ producers ================================
@@ -545,10 +546,8 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
     nt = (g.N + most - 1) / most;
     q.BN = round32((g.N + nt - 1) / nt);
   }
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  const int sms = sm_count();
+  cudaError_t e;
   // few row tiles: narrower column tiles until two thirds of the SMs have one (each CTA then splits
   // fewer weights too; the row tile is split once more per column tile, which idle SMs do for free)
   for (int k = nt + 1; q.BN > 32 && q.m_tiles * ((g.N + q.BN - 1) / q.BN) * 3 < sms * 2; ++k)
@@ -581,9 +580,9 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   auto kern = a_planar ? (gate ? (res ? gemm_split_kernel<true, true, true> : gemm_split_kernel<true, false, true>)
                                : (res ? gemm_split_kernel<true, true, false> : gemm_split_kernel<true, false, false>))
                        : (res ? gemm_split_kernel<false, true, false> : gemm_split_kernel<false, false, false>);
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  kern<<<grid, GS_THREADS, smem, st>>>(g, q, map);
+  launch_k(kern, grid, GS_THREADS, smem, st, g, q, map);
   return check_launch();
 }
 

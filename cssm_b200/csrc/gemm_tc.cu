@@ -114,6 +114,7 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_sync();
 
   if (warp < 8 && tid < NPROD) {
     // ================================ producers ================================
@@ -475,16 +476,13 @@ static bool make_out_map(const GemmArgs& g, bool a_planar, CUtensorMap* map) {
 template <int N, bool A_PLANAR, bool STG, bool ZLAST = false>
 static int launch_tc_v(const GemmArgs& g, const CUtensorMap& map, cudaStream_t st) {
   const int num_tiles = g.M / TC_BM;
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  const int sms = sm_count();
+  cudaError_t e;
   const int grid = num_tiles < sms ? num_tiles : sms;
   const size_t smem = TcSmem<N, STG>::TOTAL + 1024;      // slack for the 1024-byte alignment
-  e = cudaFuncSetAttribute(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = func_smem(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  gemm_tc_kernel<N, A_PLANAR, STG, ZLAST><<<grid, TC_THREADS, smem, st>>>(g, num_tiles, map);
+  launch_k(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST>, grid, TC_THREADS, smem, st, g, num_tiles, map);
   return check_launch();
 }
 

@@ -102,6 +102,12 @@ mlp_fused_kernel(const MlpFusedArgs g, const __grid_constant__ CUtensorMap amap,
       tc::mbar_init(&stfull[h], 8);
     }
     tc::fence_mbar_init();
+    // the weights do not depend on the kernel before this one
+    tc::mbar_expect_tx(wfull, MF_W1_BYTES + MF_W2_BYTES);
+    tc::tma_load_2d(w1s, &w1map, 0, 0, wfull);
+    tc::tma_load_2d(w1s + 16384, &w1map, 0, 128, wfull);
+#pragma unroll
+    for (int kb = 0; kb < 4; ++kb) tc::tma_load_2d(w2s + kb * 8192, &w2map, kb * 64, 0, wfull);
   }
   for (int i = tid; i < MF_HD + MF_C; i += MF_THREADS) b1s[i] = i < MF_HD ? g.b1[i] : g.b2[i - MF_HD];
   if (warp == 1) {
@@ -113,15 +119,11 @@ mlp_fused_kernel(const MlpFusedArgs g, const __grid_constant__ CUtensorMap amap,
   tc::fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   bool bad = false;
+  pdl_sync();
 
   if (warp == 0) {
     // ================================ TMA producer ================================
     if (lane == 0) {
-      tc::mbar_expect_tx(wfull, MF_W1_BYTES + MF_W2_BYTES);
-      tc::tma_load_2d(w1s, &w1map, 0, 0, wfull);
-      tc::tma_load_2d(w1s + 16384, &w1map, 0, 128, wfull);
-#pragma unroll
-      for (int kb = 0; kb < 4; ++kb) tc::tma_load_2d(w2s + kb * 8192, &w2map, kb * 64, 0, wfull);
       int it = 0;
       for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++it) {
         const int s = it % MF_NS;
@@ -371,17 +373,14 @@ int launch_mlp_fused(const __nv_bfloat16* a, int M, const __nv_bfloat16* w1t, in
       !mf_map(&w2map, w2t, MF_C, MF_HD, (uint64_t)ld2, 64) || !mf_map(&rmap, res, (uint64_t)M, MF_C, MF_C, 128) ||
       !mf_map(&omap, out, (uint64_t)M, MF_C, MF_C, 128))
     return CSSM_ERR_CUDA;
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const size_t smem = MF_SMEM + 512 + (MF_HD + MF_C) * sizeof(float) + 1024;
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(mlp_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = func_smem(mlp_fused_kernel, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   const int tiles = (M + 127) / 128;
   MlpFusedArgs g;
   g.M = M; g.b1 = b1; g.b2 = b2;
-  mlp_fused_kernel<<<tiles < sms ? tiles : sms, MF_THREADS, smem, st>>>(g, amap, w1map, w2map, rmap, omap);
+  launch_k(mlp_fused_kernel, tiles < sms ? tiles : sms, MF_THREADS, smem, st, g, amap, w1map, w2map, rmap, omap);
   return check_launch();
 }
 

@@ -1,6 +1,7 @@
 // Weight-only precompute (kernel spectrum, RoPE tables), the per-plane short-conv stencil
 // with its plane sums, and the gate-map kernels.
 #include "kernels.cuh"
+#include "gates.cuh"
 
 namespace cssm {
 
@@ -51,7 +52,7 @@ __global__ void khat_kernel(const float* __restrict__ k, cf* __restrict__ out, i
 int launch_khat(const float* k, cf* out, int nch, int ks, int H, int W, float rho, int squash,
                 int floor_eps, int path, cudaStream_t st) {
   const int n = nch * H * (W / 2 + 1);
-  khat_kernel<<<(n + 127) / 128, 128, 0, st>>>(k, out, nch, ks, H, W, rho, squash, floor_eps, path);
+  launch_k(khat_kernel, (n + 127) / 128, 128, 0, st, k, out, nch, ks, H, W, rho, squash, floor_eps, path);
   return check_launch();
 }
 
@@ -109,7 +110,7 @@ __global__ void rope_table_kernel(float2* tt, float2* th, float2* tw, float* nz,
 int launch_rope_tables(float2* tt, float2* th, float2* tw, float* nz, int T, int H, int W, int C,
                        int mode, float base, cudaStream_t st) {
   const int total = (T + H + W) * (C / 2);
-  rope_table_kernel<<<(total + 127) / 128, 128, 0, st>>>(tt, th, tw, nz, T, H, W, C, mode, base);
+  launch_k(rope_table_kernel, (total + 127) / 128, 128, 0, st, tt, th, tw, nz, T, H, W, C, mode, base);
   return check_launch();
 }
 
@@ -124,7 +125,7 @@ __global__ void tcode_kernel(float* out, int T, int C, float base) {
 }
 
 int launch_tcode(float* out, int T, int C, float base, cudaStream_t st) {
-  tcode_kernel<<<(T * C + 127) / 128, 128, 0, st>>>(out, T, C, base);
+  launch_k(tcode_kernel, (T * C + 127) / 128, 128, 0, st, out, T, C, base);
   return check_launch();
 }
 
@@ -140,6 +141,7 @@ constexpr int ST_THREADS = 256;
 // KSP / KT >= 0 fix the tap counts at compile time (taps stay in registers); -1 = run time.
 template <int KSP, int KT>
 __global__ void __launch_bounds__(ST_THREADS) plane_stencil_kernel(const StencilArgs s) {
+  pdl_sync();
   extern __shared__ __align__(16) float sm[];
   const int HW = s.H * s.W;
   float* raw = sm;                       // [HW]
@@ -228,6 +230,7 @@ __global__ void __launch_bounds__(ST_THREADS) plane_stencil_kernel(const Stencil
 // NP = float4 groups per thread = H*W / 1024.
 template <int KSP, int KT, int NP>
 __global__ void __launch_bounds__(ST_THREADS) plane_stencil_fast_kernel(const StencilArgs s) {
+  pdl_sync();
   extern __shared__ __align__(16) float sm[];
   const int H = s.H, W = s.W, HW = H * W;
   const int RS = W + 8;                              // tile row stride (4-float pad each side)
@@ -382,10 +385,9 @@ template <int KSP, int KT, int NP>
 static int launch_stencil_fast(const StencilArgs& s, cudaStream_t st) {
   const size_t smem = ((KSP > 0 ? (size_t)(s.H + 2) * (s.W + 8) : 0) + (size_t)s.T * 8) * sizeof(float);
   if (smem > 200 * 1024) return CSSM_ERR_UNSUPPORTED;
-  cudaError_t e = cudaFuncSetAttribute(plane_stencil_fast_kernel<KSP, KT, NP>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = func_smem(plane_stencil_fast_kernel<KSP, KT, NP>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  plane_stencil_fast_kernel<KSP, KT, NP><<<s.B * s.C, ST_THREADS, smem, st>>>(s);
+  launch_k(plane_stencil_fast_kernel<KSP, KT, NP>, s.B * s.C, ST_THREADS, smem, st, s);
   return check_launch();
 }
 
@@ -413,10 +415,9 @@ int launch_plane_stencil(const StencilArgs& s, cudaStream_t st) {
   const size_t smem = (size_t)(1 + nh) * s.H * s.W * sizeof(float);
   if (smem > 200 * 1024) return CSSM_ERR_UNSUPPORTED;
   auto go = [&](auto kern) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = func_smem(kern, smem);
     if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-    kern<<<s.B * s.C, ST_THREADS, smem, st>>>(s);
+    launch_k(kern, s.B * s.C, ST_THREADS, smem, st, s);
     return check_launch();
   };
   if (s.ksp == 3 && s.kt == 4) return go(plane_stencil_kernel<3, 4>);
@@ -433,6 +434,7 @@ int launch_plane_stencil(const StencilArgs& s, cudaStream_t st) {
 // flight, so every plane is read once and written once at full occupancy.
 template <int KT>
 __global__ void __launch_bounds__(256) qkv_temporal_conv_kernel(const QkvTconvArgs a) {
+  pdl_sync();
   const int HW4 = a.HW >> 2;
   const long long gid = (long long)blockIdx.x * 256 + threadIdx.x;
   const long long total = (long long)a.B * 3 * a.C * HW4;
@@ -487,9 +489,9 @@ int launch_qkv_temporal_conv(const QkvTconvArgs& a, cudaStream_t st) {
   const long long total = (long long)a.B * 3 * a.C * (a.HW >> 2);
   const unsigned grid = (unsigned)((total + 255) / 256);
   switch (a.kt) {
-    case 2: qkv_temporal_conv_kernel<2><<<grid, 256, 0, st>>>(a); break;
-    case 3: qkv_temporal_conv_kernel<3><<<grid, 256, 0, st>>>(a); break;
-    case 4: qkv_temporal_conv_kernel<4><<<grid, 256, 0, st>>>(a); break;
+    case 2: launch_k(qkv_temporal_conv_kernel<2>, grid, 256, 0, st, a); break;
+    case 3: launch_k(qkv_temporal_conv_kernel<3>, grid, 256, 0, st, a); break;
+    case 4: launch_k(qkv_temporal_conv_kernel<4>, grid, 256, 0, st, a); break;
     default: return CSSM_ERR_UNSUPPORTED;
   }
   return check_launch();
@@ -505,55 +507,55 @@ __device__ __forceinline__ float gate_act(float x, int act) {
   return x > 20.f ? x : log1pf(expf(x));
 }
 
-__global__ void __launch_bounds__(256) gated_gates_kernel(const GatedGateArgs g) {
-  extern __shared__ float sh[];
-  const int Wf = g.W / 2 + 1, NB = g.H * Wf;
+__device__ __forceinline__ float4 gated_map(float rd, float rb, float rc, int act, float inv) {
+  const float D = gate_act(rd, act);
+  return make_float4(expf(-D), (D + 1e-8f) * rb, rc * inv, 1e-7f * (D + 1e-8f));
+}
+
+// Factored gates, one frame per CTA row; the bins of a frame are split over gridDim.y CTAs when there are
+// few frames.  (One thread per vector entry walking all C channels: 37 us for one 14 x 14 frame of 256.)
+constexpr int GF_THREADS = 512;
+__global__ void __launch_bounds__(GF_THREADS) gated_gates_factored_kernel(const GatedGateArgs g) {
+  extern __shared__ __align__(16) float sh[];
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, per = g.H + Wf;
   float* ctx = sh;                 // [C]
-  float* vec = sh + g.C;           // factored: 3 x (H + Wf)
-  const int bt = blockIdx.x, tid = threadIdx.x;
+  float* vec = sh + g.C;           // 3 x (H + Wf)
+  float* scratch = vec + 3 * per;  // [GF_THREADS]
   const float inv = 1.0f / (float)(g.H * g.W);
-  for (int i = tid; i < g.C; i += blockDim.x) ctx[i] = g.ctx_sum[(size_t)bt * g.C + i] * inv;
-  __syncthreads();
-  if (g.gate_type == CSSM_GATE_FACTORED) {
-    const int per = g.H + Wf;
-    for (int o = tid; o < 3 * per; o += blockDim.x) {
-      const int gi = o / per, r = o % per;
-      const bool isw = r >= g.H;
-      const int col = isw ? r - g.H : r, ncol = isw ? Wf : g.H;
-      const float* kk = g.gk[2 * gi + (isw ? 1 : 0)];
-      float acc = g.gb[2 * gi + (isw ? 1 : 0)][col];
-      for (int c = 0; c < g.C; ++c) acc = fmaf(ctx[c], kk[(size_t)c * ncol + col], acc);
-      vec[o] = acc;
-    }
-    __syncthreads();
-  }
-  // the bins of a frame are split over gridDim.y CTAs (few frames, many bins: dense gates)
+  pdl_sync();
+  const GateCtxSrc src = {g.ctx_sum, nullptr, nullptr, 1, g.C, g.H, 0, inv};
+  gate_ctx(src, blockIdx.x, 1, ctx, scratch);
+  const int off[7] = {0, g.H, per, per + g.H, 2 * per, 2 * per + g.H, 3 * per};
+  gate_vectors<6>(g.gk, g.gb, off, 6, ctx, g.C, vec, scratch);
   const int per_cta = (NB + gridDim.y - 1) / gridDim.y;
   const int bin_end = min(NB, (int)(blockIdx.y + 1) * per_cta);
-  for (int bin = blockIdx.y * per_cta + tid; bin < bin_end; bin += blockDim.x) {
-    const int kh = bin / Wf, kw = bin % Wf;
+  for (int bin = blockIdx.y * per_cta + threadIdx.x; bin < bin_end; bin += GF_THREADS) {
+    const int kh = bin / Wf, kw = bin - kh * Wf;
     float r[3];
-    if (g.gate_type == CSSM_GATE_FACTORED) {
-      const int per = g.H + Wf;
 #pragma unroll
-      for (int gi = 0; gi < 3; ++gi) r[gi] = vec[gi * per + kh] * vec[gi * per + g.H + kw];
-    } else {
-#pragma unroll
-      for (int gi = 0; gi < 3; ++gi) {
-        float acc = g.gb[gi][bin];
-        const float* kk = g.gk[gi];
-        for (int c = 0; c < g.C; ++c) acc = fmaf(ctx[c], kk[(size_t)c * NB + bin], acc);
-        r[gi] = acc;
-      }
-    }
-    const float D = gate_act(r[0], g.act);
-    float4 o;
-    o.x = expf(-D);
-    o.y = (D + 1e-8f) * r[1];
-    o.z = r[2] * inv;
-    o.w = 1e-7f * (D + 1e-8f);
-    g.maps[(size_t)bt * NB + bin_index(g.path, kh, kw, g.H, Wf)] = o;
+    for (int gi = 0; gi < 3; ++gi) r[gi] = vec[gi * per + kh] * vec[gi * per + g.H + kw];
+    g.maps[(size_t)blockIdx.x * NB + bin_index(g.path, kh, kw, g.H, Wf)] = gated_map(r[0], r[1], r[2], g.act, inv);
   }
+}
+
+// Dense gates: a thread owns one bin of G frames, so that a weight read serves all of them (one frame per
+// read moved 80 MB of weights through L2 for 128 frames of 56 x 56 x 32).
+template <int G>
+__global__ void __launch_bounds__(128) gated_gates_dense_kernel(const GatedGateArgs g) {
+  extern __shared__ __align__(16) float sh[];
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, f0 = blockIdx.y * G, nf = min(G, g.BT - f0);
+  const float inv = 1.0f / (float)(g.H * g.W);
+  pdl_sync();
+  const GateCtxSrc src = {g.ctx_sum, nullptr, nullptr, 1, g.C, g.H, 0, inv};
+  gate_ctx(src, f0, nf, sh, sh + G * g.C);
+  const int bin = blockIdx.x * 128 + threadIdx.x;
+  if (bin >= NB) return;
+  float r[3][G];
+  gate_dense<3, G>(g.gk, g.gb, NB, bin, g.C, sh, r);
+  const int kh = bin / Wf, o = bin_index(g.path, kh, bin - kh * Wf, g.H, Wf);
+#pragma unroll
+  for (int f = 0; f < G; ++f)
+    if (f < nf) g.maps[(size_t)(f0 + f) * NB + o] = gated_map(r[0][f], r[1][f], r[2][f], g.act, inv);
 }
 
 // Factored gates of many frames with small planes (the CSSM-SHViT stages: hundreds of frames of
@@ -564,6 +566,7 @@ __global__ void __launch_bounds__(256) gated_gates_kernel(const GatedGateArgs g)
 // written.
 constexpr int GB_FR = 4;
 __global__ void __launch_bounds__(256) gated_gates_batched_kernel(const GatedGateArgs g) {
+  pdl_sync();
   extern __shared__ __align__(16) float sh[];
   const int Wf = g.W / 2 + 1, NB = g.H * Wf, per = g.H + Wf;
   const int nH = g.C * g.H, nW = g.C * Wf;           // floats per matrix (multiples of 4: C % 4 == 0)
@@ -620,13 +623,7 @@ __global__ void __launch_bounds__(256) gated_gates_batched_kernel(const GatedGat
     float r[3];
 #pragma unroll
     for (int gi = 0; gi < 3; ++gi) r[gi] = v[gi * per + kh] * v[gi * per + g.H + kw];
-    const float D = gate_act(r[0], g.act);
-    float4 o;
-    o.x = expf(-D);
-    o.y = (D + 1e-8f) * r[1];
-    o.z = r[2] * inv;
-    o.w = 1e-7f * (D + 1e-8f);
-    g.maps[(size_t)(f0 + f) * NB + bin_index(g.path, kh, kw, g.H, Wf)] = o;
+    g.maps[(size_t)(f0 + f) * NB + bin_index(g.path, kh, kw, g.H, Wf)] = gated_map(r[0], r[1], r[2], g.act, inv);
   }
 }
 
@@ -638,23 +635,24 @@ int launch_gated_gates(const GatedGateArgs& g, cudaStream_t st) {
     bool al = g.C % 4 == 0;
     for (int i = 0; i < 6; ++i) al = al && aligned16(g.gk[i]);
     if (g.gate_type == CSSM_GATE_FACTORED && g.BT >= 64 && g.H * Wf <= 256 && bsm <= 160 * 1024 && al) {
-      cudaError_t e = cudaFuncSetAttribute(gated_gates_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)bsm);
+      cudaError_t e = func_smem(gated_gates_batched_kernel, bsm);
       if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-      gated_gates_batched_kernel<<<(g.BT + GB_FR - 1) / GB_FR, 256, bsm, st>>>(g);
+      launch_k(gated_gates_batched_kernel, (g.BT + GB_FR - 1) / GB_FR, 256, bsm, st, g);
       return check_launch();
     }
   }
-  const size_t smem = (size_t)(g.C + 3 * (g.H + Wf)) * sizeof(float);
-  // enough CTAs to cover the GPU when there are few frames: up to one CTA per 256 bins
   const int NB = g.H * Wf;
-  int chunks = 1;
-  if (g.BT < 296) {
-    chunks = (296 + g.BT - 1) / g.BT;
-    const int maxc = (NB + 255) / 256;
-    if (chunks > maxc) chunks = maxc;
+  if (g.gate_type == CSSM_GATE_FACTORED) {
+    const size_t smem = (size_t)(g.C + 3 * (g.H + Wf) + GF_THREADS) * sizeof(float);
+    launch_k(gated_gates_factored_kernel, dim3(g.BT, gate_chunks(g.BT, NB)), GF_THREADS, smem, st, g);
+    return check_launch();
   }
-  gated_gates_kernel<<<dim3(g.BT, chunks), 256, smem, st>>>(g);
+  const int chunks = (NB + 127) / 128, G = gate_dense_frames(g.BT, chunks);
+  const dim3 grid(chunks, (g.BT + G - 1) / G);
+  const size_t smem = (size_t)(G * g.C + 128) * sizeof(float);
+  if (G == 8) launch_k(gated_gates_dense_kernel<8>, grid, 128, smem, st, g);
+  else if (G == 4) launch_k(gated_gates_dense_kernel<4>, grid, 128, smem, st, g);
+  else launch_k(gated_gates_dense_kernel<1>, grid, 128, smem, st, g);
   return check_launch();
 }
 

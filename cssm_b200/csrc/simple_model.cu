@@ -57,6 +57,7 @@ struct StemArgs {
 // (a 64 -> 64 channel 3x3 layer: 147 KB), so that the one resident CTA still has 32 warps.
 template <int KS, int POOL, int CIN, bool FULLC, int NT>
 __global__ void __launch_bounds__(NT) stem_layer_kernel(const StemArgs a) {
+  pdl_sync();
   extern __shared__ __align__(16) float sm[];
   const int C = FULLC ? SM_MAXC : a.C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int Cin = CIN > 0 ? CIN : a.Cin;
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(NT) stem_layer_kernel(const StemArgs a) {
 constexpr int STEMW_THREADS = 512;
 template <int KS>
 __global__ void __launch_bounds__(STEMW_THREADS) stem_layer_wide_kernel(const StemArgs a) {
+  pdl_sync();
   extern __shared__ __align__(16) float sm[];
   const int C = a.C, Cin = a.Cin, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nw = KS * KS * Cin * C;
@@ -305,13 +307,12 @@ __global__ void __launch_bounds__(STEMW_THREADS) stem_layer_wide_kernel(const St
 template <int KS>
 static int launch_stem_layer_wide(StemArgs a, cudaStream_t st) {
   const size_t smem = ((size_t)KS * KS * a.Cin * a.C + 3 * (size_t)a.C) * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(stem_layer_wide_kernel<KS>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = func_smem(stem_layer_wide_kernel<KS>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   const long long total = (long long)a.N * a.Ho * a.Wo;
   const long long per_cta = (STEMW_THREADS / 32) * 8;
   const long long need = (total + per_cta - 1) / per_cta;
-  stem_layer_wide_kernel<KS><<<(unsigned)(need < 148 ? need : 148), STEMW_THREADS, smem, st>>>(a);
+  launch_k(stem_layer_wide_kernel<KS>, (unsigned)(need < 148 ? need : 148), STEMW_THREADS, smem, st, a);
   return check_launch();
 }
 
@@ -320,8 +321,7 @@ static int launch_stem_layer_v(StemArgs a, cudaStream_t st) {
   const size_t wbytes = (size_t)KS * KS * a.Cin * a.C * sizeof(float);
   a.w_in_smem = wbytes <= 160 * 1024 ? 1 : 0;
   const size_t smem = (a.w_in_smem ? wbytes : 0) + 3 * (size_t)a.C * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(stem_layer_kernel<KS, POOL, CIN, FULLC, NT>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = func_smem(stem_layer_kernel<KS, POOL, CIN, FULLC, NT>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   const long long total = (long long)a.N * a.Ho * a.Wo;
   const long long per_cta = (NT / 32) * (POOL == 2 ? 2 : 8);
@@ -329,7 +329,7 @@ static int launch_stem_layer_v(StemArgs a, cudaStream_t st) {
   // a few resident waves of CTAs that loop, so that the per-CTA weight staging is amortised
   const long long cap = NT == 1024 ? 148 : 148 * 16;
   const unsigned grid = (unsigned)(need < cap ? need : cap);
-  stem_layer_kernel<KS, POOL, CIN, FULLC, NT><<<grid, NT, smem, st>>>(a);
+  launch_k(stem_layer_kernel<KS, POOL, CIN, FULLC, NT>, grid, NT, smem, st, a);
   return check_launch();
 }
 
@@ -375,6 +375,7 @@ struct ReadoutArgs {
 // grid (bands, B): LayerNorm/softplus of (y + res) per pixel, pooled over the band's pixels.
 // Four lanes per pixel as in the stem (lane g owns float4 groups g + 4k); 8 pixels per warp.
 __global__ void __launch_bounds__(RO_THREADS) readout_pool_kernel(const ReadoutArgs a) {
+  pdl_sync();
   __shared__ float red[RO_THREADS / 32][SM_MAXC];
   __shared__ float vec[2 * SM_MAXC];
   const int C = a.C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -458,6 +459,7 @@ __global__ void __launch_bounds__(RO_THREADS) readout_pool_kernel(const ReadoutA
 
 // grid B, 64 threads: combine the band partials, LayerNorm (norm_post), Dense head
 __global__ void __launch_bounds__(SM_MAXC) readout_head_kernel(const ReadoutArgs a) {
+  pdl_sync();
   __shared__ float v[SM_MAXC];
   __shared__ float stats[2];
   const int C = a.C, tid = threadIdx.x, b = blockIdx.x;
@@ -538,6 +540,7 @@ static size_t block_ws_bytes(int block, const void* bd) {
 __global__ void __launch_bounds__(256) repeat_frames_kernel(const float4* __restrict__ in,
                                                             float4* __restrict__ out, size_t frame4,
                                                             int T, size_t total4) {
+  pdl_sync();
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= total4) return;
   const size_t fo = i / frame4, r = i - fo * frame4;
@@ -613,10 +616,10 @@ static int run_readout(const cssm_simple_desc* d, const cssm_simple_weights* w, 
   a.B = d->B; a.H = H; a.W = W; a.C = d->embed_dim; a.pool_max = d->pool_type;
   a.norm_post_order = d->readout_norm; a.ncls = d->num_classes;
   a.bands = (H + RO_ROWS - 1) / RO_ROWS;
-  readout_pool_kernel<<<dim3(a.bands, d->B), RO_THREADS, 0, st>>>(a);
+  launch_k(readout_pool_kernel, dim3(a.bands, d->B), RO_THREADS, 0, st, a);
   int s = check_launch();
   if (s != CSSM_OK) return s;
-  readout_head_kernel<<<d->B, SM_MAXC, 0, st>>>(a);
+  launch_k(readout_head_kernel, d->B, SM_MAXC, 0, st, a);
   return check_launch();
 }
 
@@ -678,6 +681,7 @@ int cssm_simple_forward(const cssm_simple_desc* d, const cssm_simple_weights* w,
   cudaStream_t st = (cudaStream_t)stream;
   char* ws = (char*)workspace;
   const SimpleDims o = stem_out_dims(*d);
+  PdlScope pdl((size_t)d->B * d->T * o.H * o.W * d->embed_dim * 4 <= PDL_MAX_BYTES);
   float* feat = (float*)(ws + l.feat);
   float* y = (float*)(ws + l.y);
   const size_t tmp_half = (l.y - l.tmp) / 2;
@@ -690,8 +694,7 @@ int cssm_simple_forward(const cssm_simple_desc* d, const cssm_simple_weights* w,
     const float* clips = feat;
     if (d->image_input) {
       const size_t frame4 = (size_t)o.H * o.W * d->embed_dim / 4, total4 = frame4 * d->B * d->T;
-      repeat_frames_kernel<<<(unsigned)((total4 + 255) / 256), 256, 0, st>>>(
-          (const float4*)feat, (float4*)(ws + l.rep), frame4, d->T, total4);
+      launch_k(repeat_frames_kernel, (unsigned)((total4 + 255) / 256), 256, 0, st, (const float4*)feat, (float4*)(ws + l.rep), frame4, d->T, total4);
       if ((s = check_launch()) != CSSM_OK) return s;
       clips = (const float*)(ws + l.rep);
     }

@@ -96,6 +96,7 @@ template <int N>
 __global__ void __launch_bounds__(SCL_TPB)
 gated_spectral_cl_kernel(const __nv_bfloat16* __restrict__ xz, int ld, int C,
                          const float4* __restrict__ gates, __nv_bfloat16* __restrict__ y, int ldy) {
+  pdl_sync();
   constexpr int Wf = N / 2 + 1, P = N * N, NB = N * Wf;
   constexpr int RH = (N + 1) / 2, KH = Wf / 2;       // rows / spectrum columns of the first thread of a plane
   constexpr float INV_N = 1.0f / (float)N;
@@ -287,13 +288,13 @@ int launch_gated_spectral_cl(const __nv_bfloat16* xz, int ld, int Nimg, int H, i
   const int grid = Nimg * (C / SCL_PL);
   cudaError_t e;
   if (H == 14) {
-    e = cudaFuncSetAttribute(gated_spectral_cl_kernel<14>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = func_smem(gated_spectral_cl_kernel<14>, smem);
     if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-    gated_spectral_cl_kernel<14><<<grid, SCL_TPB, smem, st>>>(xz, ld, C, reinterpret_cast<const float4*>(gates), y, ldy);
+    launch_k(gated_spectral_cl_kernel<14>, grid, SCL_TPB, smem, st, xz, ld, C, reinterpret_cast<const float4*>(gates), y, ldy);
   } else {
-    e = cudaFuncSetAttribute(gated_spectral_cl_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = func_smem(gated_spectral_cl_kernel<7>, smem);
     if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-    gated_spectral_cl_kernel<7><<<grid, SCL_TPB, smem, st>>>(xz, ld, C, reinterpret_cast<const float4*>(gates), y, ldy);
+    launch_k(gated_spectral_cl_kernel<7>, grid, SCL_TPB, smem, st, xz, ld, C, reinterpret_cast<const float4*>(gates), y, ldy);
   }
   return check_launch();
 }
