@@ -1,207 +1,232 @@
-// GDN fused spectral kernel for 64x64 planes, d_k = d_v = 4.  One CTA (288 threads) per
-// (batch, head).  Per step: the 8 q/k planes are transformed and their spectra parked in
-// shared memory in the column lanes' own bin order; the norms are applied in place; then each
-// of the 4 v planes is transformed, its state row updated and read out, and the output plane
-// inverse-transformed over the v plane.
+// GDN fused spectral kernel for 64x64 planes, d_k = d_v = 4.  A CTA runs one (batch, head) after another
+// with two groups of 288 threads, each with its own transform buffers: per step a group transforms
+// every other q / k plane into the shared spectra (shared memory, in the column lanes' own bin order),
+// the norms are applied there in place, and then each group takes every other v plane: transform,
+// update of its state row, readout, inverse transform over the v plane.
+//
+// Bound: the shared-memory pipe (80 % of its wavefronts, B = 16; DRAM 18 %, L2 23 %).  With one group (nine
+// warps) latency was the bound; the two groups fit next to the spectra because a group's inverse columns go
+// over its forward rows (one more barrier a v row) and the lanes without a column need no spectrum slot
+// and one exchange region.  The state of the running heads (270 KB each) stays in L2: scratch goes by CTA,
+// not by head, and the first step reads no state and the last one writes none.
+// 128 x 8 x 64 x 64 x 64: 4.61 -> 3.76 ms.
 #include "r64.cuh"
 #include "kernels.cuh"
 #include "gdn_common.cuh"
 
 namespace cssm {
 
-constexpr int G64_SPEC_CF = 8 * 8 * R64_NT;     // [plane 0..7][q 0..7][thread]
-constexpr int G64_SMEM_CF = R64_EX_CF + R64_ZR_CF + R64_GB_CF + G64_SPEC_CF;
+constexpr int G64_NT = 2 * R64_NT;
+constexpr int G64_COLS = 33 * 8;                       // lanes with a column
+constexpr int G64_EXG = 34;                            // exchange regions of a group
+constexpr int G64_SPEC_CF = 8 * 8 * G64_COLS;          // [plane 0..7][q 0..7][column lane]
+constexpr int G64_ZR_CF = R64_ZR_CF > R64_GB_CF ? R64_ZR_CF : R64_GB_CF;
+constexpr int G64_GRP_CF = G64_EXG * EX_GROUP_STRIDE + G64_ZR_CF;
+constexpr int G64_SMEM_CF = G64_SPEC_CF + 2 * G64_GRP_CF;
+static_assert(G64_SMEM_CF * sizeof(cf) <= 226 * 1024, "one CTA per SM");
+
+// r64_init for one group; the lanes without a column share the last exchange region
+__device__ __forceinline__ void g64_init(R64Ctx& c, cf* EX, cf* ZR, int tid) {
+  c.EX = EX; c.ZR = ZR; c.GB = ZR;
+  c.warp = tid >> 5; c.lane = tid & 31; c.sub = c.lane & 3; c.a = c.lane >> 2;
+  c.grp = c.warp * 4 + c.sub;
+  c.row_on = c.warp < 8; c.col_warp = true; c.col_on = c.grp <= 32;
+  c.exg = EX + min(c.grp, G64_EXG - 1) * EX_GROUP_STRIDE;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    float s, co;
+    sincospif(-(float)(c.a * k) / 32.0f, &s, &co);
+    c.tw[k] = mk(co, s);
+  }
+}
 
 // LAST: only the last step's output planes are produced (compile-time switch).
 // STATIC: static-image fast path (one data frame per batch element, the T gate steps run per bin).
 template <bool LAST, bool STATIC>
-__global__ void __launch_bounds__(R64_NT, 1) gdn_spectral_r64(const GdnSpectralArgs a) {
-  pdl_sync();
+__global__ void __launch_bounds__(G64_NT, 1) gdn_spectral_r64(const GdnSpectralArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cf* EX = reinterpret_cast<cf*>(smem_raw);
-  cf* ZR = EX + R64_EX_CF;
-  cf* GB = ZR + R64_ZR_CF;
-  cf* SPEC = GB + R64_GB_CF;
-  __shared__ float red[9][8];
+  __shared__ float red[2][9][4];
+  cf* SPEC = reinterpret_cast<cf*>(smem_raw);
+  const int half = threadIdx.x >= R64_NT ? 1 : 0, tid = threadIdx.x - half * R64_NT;
+  cf* own = SPEC + G64_SPEC_CF + half * G64_GRP_CF;
 
   R64Ctx c;
-  r64_init(c, EX, ZR, GB);
-  const int tid = threadIdx.x;
+  cf* ZR = own + G64_EXG * EX_GROUP_STRIDE;
+  g64_init(c, own, ZR, tid);
+  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(half + 1), "n"(R64_NT) : "memory"); };
   constexpr int HW = 4096, NB = 64 * 33, DK = 4;
-  const int nh = a.C / DK;
-  const int b = blockIdx.x / nh, hd = blockIdx.x % nh;
+  const int nh = a.C / DK, heads = a.B * nh;
   const int Tdata = STATIC ? 1 : a.T;          // frames of q, k, v per batch element
-
-  // state scratch: S[v][i][q][thread]; zero it (a thread only ever touches its own slots)
-  cf* S = a.state + (size_t)blockIdx.x * DK * DK * NB;   // 16 * 2112 = 16 * 8 * 264 slots
-  // lanes of column passes: slot index inside a (v,i) block is q*264 + (grp*8 + a), grp <= 32
-  const int cslot = c.grp * 8 + c.a;
-  if (c.col_on && !STATIC)
-    for (int vi = 0; vi < DK * DK; ++vi)
-#pragma unroll
-      for (int q = 0; q < 8; ++q) S[(size_t)vi * NB + q * 264 + cslot] = mk(0.f, 0.f);
-
-  cf wh[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q)
-    wh[q] = c.col_on ? a.what[(size_t)hd * NB + ((q * 33 + c.grp) << 3) + c.a] : mk(0.f, 0.f);
   const float invHW = 1.0f / (float)HW;
+  // slot of this lane in the spectra (warp 8 has one column: lanes 0, 4, 8, ...)
+  const int slot = c.warp < 8 ? tid : 256 + c.a;
+  // state scratch S[v][i][q][lane]; a thread only ever touches its own slots
+  cf* S = a.state + (size_t)blockIdx.x * DK * DK * NB + c.grp * 8 + c.a;
+  pdl_sync();
 
-  // plane idx 0..3 = q, 4..7 = k, 8..11 = v of step t; idx 12 = first plane of step t + 1
-  // last_only: steps before the last one skip the q planes (their sequence starts at idx 4)
-  auto first_of = [&](int t) -> int { return (LAST && t < Tdata - 1) ? 4 : 0; };
-  auto plane_of = [&](int t, int idx) -> float* {
-    if (idx >= 12) { ++t; idx = first_of(t); }
-    if (t >= Tdata) { t = Tdata - 1; idx = 0; }             // harmless re-read past the end
-    const size_t frame = (size_t)(b * Tdata + t);
-    return a.qkv + (frame * 3 * a.C + (size_t)(idx >> 2) * a.C + hd * DK + (idx & 3)) * HW;
+  // plane 2 i + half of step t: i = 0, 1 q, 2, 3 k, 4, 5 v; i = 6: the first of step t + 1 (of the
+  // next head).  last_only: steps before the last one skip the q planes.
+  auto first_of = [&](int t) -> int { return (LAST && t < Tdata - 1) ? 2 : 0; };
+  auto plane_of = [&](int bh, int t, int i) -> float* {
+    if (i >= 6) { ++t; if (t >= Tdata) { t = 0; bh += gridDim.x; } i = first_of(t); }
+    if (bh >= heads) bh = blockIdx.x;                       // harmless re-read past the end
+    const int b = bh / nh, hd = bh - b * nh, idx = 2 * i + half;
+    return a.qkv + ((size_t)(b * Tdata + t) * 3 * a.C + (size_t)(idx >> 2) * a.C + hd * DK + (idx & 3)) * HW;
   };
   cf nx[8];                                   // rows of the NEXT plane, fetched one pass ahead
-  r64_load_rows(c, plane_of(0, first_of(0)), nx);
+  r64_load_rows(c, plane_of(blockIdx.x, 0, first_of(0)), nx);
 
+  for (int bh = blockIdx.x; bh < heads; bh += gridDim.x) {
+  const int b = bh / nh, hd = bh - b * nh;
+  const cf* wh = a.what + (size_t)hd * NB + (c.grp << 3) + c.a;
   for (int t = 0; t < Tdata; ++t) {
-    const size_t frame = (size_t)(b * Tdata + t);
-    float* base = a.qkv + frame * 3 * a.C * HW;
     const bool emit = !LAST || t == Tdata - 1;       // same for the whole CTA
-    float ssq[8];
-#pragma unroll
-    for (int p = 0; p < 4; ++p) ssq[p] = 0.f;
-    // ---- q planes (p = 0..3) and k planes (p = 4..7) ----
+    // ---- q planes (i = 0, 1) and k planes (i = 2, 3) ----
 #pragma unroll 1
-    for (int p = first_of(t); p < 8; ++p) {
-      __syncthreads();                       // ZR free (previous column pass finished)
+    for (int i = first_of(t); i < 4; ++i) {
+      // own ZR free; at the first plane also: nobody reads the spectra of the step before any more
+      if (i == first_of(t)) __syncthreads(); else group_sync();
       {
         cf cur[8];
 #pragma unroll
         for (int m = 0; m < 8; ++m) cur[m] = nx[m];
-        r64_load_rows(c, plane_of(t, p + 1), nx);
+        r64_load_rows(c, plane_of(bh, t, i + 1), nx);
         r64_row_fwd_regs(c, cur);
       }
-      __syncthreads();
+      group_sync();
       float acc = 0.f;
-      if (c.col_warp) {
-        cf v[8];
-        r64_col_fwd(c, v);
+      cf v[8];
+      r64_col_fwd(c, v);
+      if (c.col_on) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          SPEC[(p * 8 + q) * R64_NT + tid] = v[q];
-          if (c.col_on) acc += v[q].x * v[q].x + v[q].y * v[q].y;
+          SPEC[((2 * i + half) * 8 + q) * G64_COLS + slot] = v[q];
+          acc += v[q].x * v[q].x + v[q].y * v[q].y;
         }
       }
       for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
-      // valid in lane 0 of each warp (ssq is indexed statically to stay in registers)
-#pragma unroll
-      for (int pp = 0; pp < 8; ++pp) if (pp == p) ssq[pp] = acc;
+      if (c.lane == 0) red[half][c.warp][i] = acc;
     }
     if (c.lane == 0)
-#pragma unroll
-      for (int p = 0; p < 8; ++p) red[c.warp][p] = ssq[p];
+      for (int i = 0; i < first_of(t); ++i) red[half][c.warp][i] = 0.f;
     __syncthreads();
-    float nrm[8];
+    // ---- normalise in place, the bins split between the groups:
+    //      q_hat = q*nq; k_hat = (k*nk) / sqrt(sum_i |.|^2 + 1e-6)
+    {
+      float mine = 0.f;                      // lanes 0..7: plane norms
+      if (c.lane < 8) {
 #pragma unroll
-    for (int p = 0; p < 8; ++p) {
-      float s = 0.f;
+        for (int w = 0; w < 9; ++w) mine += red[c.lane & 1][w][c.lane >> 1];
+        mine = a.use_l2 ? rsqrtf(mine + 1e-6f) : 1.f;
+      }
+      float nrm[8];
 #pragma unroll
-      for (int w = 0; w < 9; ++w) s += red[w][p];
-      nrm[p] = a.use_l2 ? rsqrtf(s + 1e-6f) : 1.f;
-    }
-    // ---- normalise own bins in place: q_hat = q*nq; k_hat = (k*nk) / sqrt(sum_i |.|^2 + 1e-6)
-    if (c.col_warp) {
+      for (int p = 0; p < 8; ++p) nrm[p] = __shfl_sync(0xffffffffu, mine, p);
+      if (c.col_on) {
+        cf* sp = SPEC + half * 4 * G64_COLS + slot;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        cf kv[4];
-        float ks = 0.f;
+        for (int q = 0; q < 4; ++q) {
+          cf kv[4];
+          float ks = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          cf z = SPEC[((4 + i) * 8 + q) * R64_NT + tid];
-          kv[i] = mk(z.x * nrm[4 + i], z.y * nrm[4 + i]);
-          ks += kv[i].x * kv[i].x + kv[i].y * kv[i].y;
-          if (emit) {
-            cf qq = SPEC[(i * 8 + q) * R64_NT + tid];
-            SPEC[(i * 8 + q) * R64_NT + tid] = mk(qq.x * nrm[i], qq.y * nrm[i]);
+          for (int i = 0; i < 4; ++i) {
+            const cf z = sp[((4 + i) * 8 + q) * G64_COLS];
+            kv[i] = mk(z.x * nrm[4 + i], z.y * nrm[4 + i]);
+            ks += kv[i].x * kv[i].x + kv[i].y * kv[i].y;
+            if (emit) {
+              const cf qq = sp[(i * 8 + q) * G64_COLS];
+              sp[(i * 8 + q) * G64_COLS] = mk(qq.x * nrm[i], qq.y * nrm[i]);
+            }
           }
-        }
-        const float kn = rsqrtf(ks + 1e-6f);
+          const float kn = rsqrtf(ks + 1e-6f);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          SPEC[((4 + i) * 8 + q) * R64_NT + tid] = mk(kv[i].x * kn, kv[i].y * kn);
+          for (int i = 0; i < 4; ++i) sp[((4 + i) * 8 + q) * G64_COLS] = mk(kv[i].x * kn, kv[i].y * kn);
+        }
       }
     }
+    __syncthreads();
     // gates: of this frame, or (static path) of step 0 of this batch element's T steps
+    const size_t frame = (size_t)(b * Tdata + t);
     const float2* abp = a.ab + ((STATIC ? (size_t)b * a.T : frame) * a.ab_heads + (a.ab_heads > 1 ? hd : 0)) * NB + (c.grp << 3) + c.a;
     // ---- v rows: transform, state update, readout, inverse transform over the v plane ----
 #pragma unroll 1
-    for (int vr = 0; vr < DK; ++vr) {
-      float* vplane = base + (size_t)(2 * a.C + hd * DK + vr) * HW;
-      __syncthreads();                       // ZR free; GB reads of the previous row finished
-      {
-        cf cur[8];
-#pragma unroll
-        for (int m = 0; m < 8; ++m) cur[m] = nx[m];
-        r64_load_rows(c, plane_of(t, 8 + vr + 1), nx);
-        r64_row_fwd_regs(c, cur);
-      }
-      __syncthreads();
-      if (c.col_warp) {
-        // the state row of all 8 bins is fetched before the transform (the scratch is only
-        // L2-resident) and written back after the last bin, so the loads are not pinned behind
-        // the stores of the previous bin
-        cf sreg[8][4];
-        float2 gab[8];
-        cf* srow = S + (size_t)(vr * DK) * NB + cslot;
-        if (!STATIC) {
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              sreg[q][i] = c.col_on ? srow[(size_t)i * NB + q * 264] : mk(0.f, 0.f);
-            gab[q] = c.col_on ? __ldg(abp + q * (33 * 8)) : make_float2(0.f, 0.f);
-          }
-        }
-        cf v[8];
+    for (int i = 4; i < 6; ++i) {
+      const int vr = 2 * (i - 4) + half;
+      if (i > 4) group_sync();               // ZR free: the row before has left it
+      r64_row_fwd_regs(c, nx);
+      group_sync();
+      cf v[8];
+      if (STATIC) {
         r64_col_fwd(c, v);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          cf kk[4], qq[4], o = mk(0.f, 0.f);
+          if (c.col_on) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              qq[j] = SPEC[(j * 8 + q) * G64_COLS + slot];
+              kk[j] = SPEC[((4 + j) * 8 + q) * G64_COLS + slot];
+            }
+            o = gdn_bin_static<4>(kk, qq, v[q], wh[q * 264], abp + q * 264, (size_t)a.ab_heads * NB, a.T);
+          }
+          v[q] = mk(o.x * invHW, o.y * invHW);
+        }
+      } else {
+        // a bin's state row and gates are requested two bins ahead (L2)
+        cf* srow = S + (size_t)(vr * DK) * NB;
+        cf sreg[2][4];
+        float2 gab[2], w[2];
+        auto fetch = [&](int q) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            sreg[q & 1][j] = (t > 0 && c.col_on) ? srow[(size_t)j * NB + q * 264] : mk(0.f, 0.f);
+          gab[q & 1] = c.col_on ? __ldg(abp + q * 264) : make_float2(0.f, 0.f);
+          w[q & 1] = c.col_on ? __ldg(reinterpret_cast<const float2*>(wh) + q * 264) : make_float2(0.f, 0.f);
+        };
+        fetch(0);
+        fetch(1);
+        r64_col_fwd(c, v);
+        const cf* sp = SPEC + (c.col_on ? slot : 0);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           cf kk[4], qq[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            qq[i] = SPEC[(i * 8 + q) * R64_NT + tid];
-            kk[i] = SPEC[((4 + i) * 8 + q) * R64_NT + tid];
+          for (int j = 0; j < 4; ++j) {
+            kk[j] = sp[((4 + j) * 8 + q) * G64_COLS];
+            qq[j] = emit ? sp[(j * 8 + q) * G64_COLS] : mk(0.f, 0.f);
           }
-          if (STATIC) {
-            cf o = mk(0.f, 0.f);
-            if (c.col_on) o = gdn_bin_static<4>(kk, qq, v[q], wh[q], abp + q * (33 * 8), (size_t)a.ab_heads * NB, a.T);
-            v[q] = mk(o.x * invHW, o.y * invHW);
-            continue;
-          }
-          const cf aw = mk(gab[q].x * wh[q].x, gab[q].x * wh[q].y);
-          if (emit) {
-            const cf o = gdn_bin_update_regs<4, true>(sreg[q], kk, qq, v[q], aw, gab[q].y);
-            v[q] = mk(o.x * invHW, o.y * invHW);
-          } else {
-            gdn_bin_update_regs<4, false>(sreg[q], kk, qq, v[q], aw, gab[q].y);
-          }
-        }
-        if (c.col_on && !STATIC) {
+          const cf aw = mk(gab[q & 1].x * w[q & 1].x, gab[q & 1].x * w[q & 1].y);
+          cf o = mk(0.f, 0.f);
+          if (emit) o = gdn_bin_update_regs<4, true>(sreg[q & 1], kk, qq, v[q], aw, gab[q & 1].y);
+          else gdn_bin_update_regs<4, false>(sreg[q & 1], kk, qq, v[q], aw, gab[q & 1].y);
+          v[q] = mk(o.x * invHW, o.y * invHW);
+          if (c.col_on && t + 1 < Tdata) {
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) srow[(size_t)i * NB + q * 264] = sreg[q][i];
+            for (int j = 0; j < 4; ++j) srow[(size_t)j * NB + q * 264] = sreg[q & 1][j];
+          }
+          if (q + 2 < 8) fetch(q + 2);
         }
-        if (emit) r64_col_inv(c, v);
       }
-      __syncthreads();
-      if (c.row_on && emit) {
-        cf v[8];
-        r64_row_inv(c, v);
-        float* y0 = vplane + (2 * c.grp) * 64 + c.a;
+      r64_load_rows(c, plane_of(bh, t, i + 1), nx);
+      if (emit) {
+        fft64_lane8<true>(v, c.tw, c.exg, c.a);
+        group_sync();                        // every column of ZR has been read: GB may go over it
 #pragma unroll
-        for (int n1 = 0; n1 < 8; ++n1) {
-          y0[8 * n1] = v[n1].x;
-          y0[64 + 8 * n1] = v[n1].y;
+        for (int n1 = 0; n1 < 8; ++n1)
+          if (c.col_on) c.GB[(c.a + 8 * n1) * R64_GBS + c.grp] = v[n1];
+        group_sync();
+        if (c.row_on) {
+          r64_row_inv(c, v);
+          float* y0 = a.qkv + (frame * 3 * a.C + 2 * a.C + hd * DK + vr) * HW + (2 * c.grp) * 64 + c.a;
+#pragma unroll
+          for (int n1 = 0; n1 < 8; ++n1) {
+            y0[8 * n1] = v[n1].x;
+            y0[64 + 8 * n1] = v[n1].y;
+          }
         }
       }
     }
+  }
   }
 }
 
@@ -211,7 +236,8 @@ int launch_gdn_spectral_r64(const GdnSpectralArgs& a, cudaStream_t st) {
                              : (a.last_only ? gdn_spectral_r64<true, false> : gdn_spectral_r64<false, false>);
   cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  launch_k(kern, a.B * (a.C / 4), R64_NT, smem, st, a);
+  const int heads = a.B * (a.C / 4), sms = sm_count();
+  launch_k(kern, heads < sms ? heads : sms, G64_NT, smem, st, a);
   return check_launch();
 }
 

@@ -169,3 +169,13 @@ def test_static_image_golden_fixture_on_gpu():
                             static_image_fast_path=True, num_timesteps=kw["num_timesteps"])
     y = mod.apply({"params": p}, torch.from_numpy(g["x"]).cuda()).cpu().numpy()
     assert orc.rel_l2(y, g["y"]) <= 2e-2
+
+
+@pytest.mark.parametrize("side,B,T", [(32, 20, 3), (64, 10, 3), (64, 10, 1)])
+def test_more_heads_than_resident_ctas(side, B, T):
+    """The 32x32 and 64x64 recurrence kernels walk the heads with as many CTAs as fit the chip, reusing a
+    CTA's state scratch from head to head: 320 heads of 32x32, 160 of 64x64.  float32 transforms, projections
+    and three steps: below 5e-6 of the 2-norm, checked at 1e-5."""
+    y, ref, last = _run(B, T, side, side, 64, 4, 5, "factored", "none", 4, 1, last=True)
+    assert orc.rel_l2(y, ref) <= 1e-5
+    assert orc.rel_l2(last, ref[:, -1]) <= 1e-5
