@@ -168,3 +168,22 @@ def test_streaming_host_entry_prefetches_the_next_batch():
         bound.forward_host_pipelined(xs[2], xs[2], lh, last_frame_only=True)
         assert orc.rel_l2(lh.numpy(), want[2].numpy()) <= 1e-5
         bound.close()
+
+
+@pytest.mark.parametrize("E,T,qkv,shape", [(16, 3, 3, (2, 26, 18, 1)), (16, 4, 3, (2, 26, 18, 1)), (32, 5, 5, (1, 34, 22, 1)),
+                                           (64, 4, 5, (1, 64, 64, 1)), (16, 6, 7, (1, 18, 70, 1)), (20, 4, 5, (1, 18, 20, 1))])
+@pytest.mark.parametrize("pos", ["none", "spatiotemporal", "mrope"])
+def test_repeated_image_qkv_conv(E, T, qkv, shape, pos):
+    """The qkv conv of one image repeated over T frames: one conv for all frames from four frames and 16
+    channels up, ragged bands and columns, against the oracle.  float32 through two projections, at most 49
+    taps and the recurrence: below 5e-6, checked at 1e-5."""
+    m = _model("gdn", E, 3, pos, "default", 1, "max", "pre", seq_len=T, delta_key_dim=4, qkv_conv_size=qkv)
+    x = np.random.default_rng(E + T).random(shape).astype(np.float32)
+    H, W = m.feature_hw(*shape[1:3])
+    bkw = _block_kwargs(m)
+    p = so.init_simple_params(5, cin=1, embed_dim=E, H=H, W=W, num_classes=m.num_classes, cssm_type="gdn",
+                              stem_mode="default", stem_layers=1, bias_scale=0.1, block_kwargs=bkw)
+    ref = so.simple_forward(p, x, cssm_type="gdn", seq_len=T, stem_mode="default", stem_layers=1, pool_type="max",
+                            readout_norm="pre", block_kwargs=bkw)
+    got = m.bind({"params": p})(torch.from_numpy(x).cuda()).cpu().numpy()
+    assert orc.rel_l2(got, ref) <= 1e-5
