@@ -381,6 +381,162 @@ __global__ void __launch_bounds__(ST_THREADS) plane_stencil_fast_kernel(const St
   }
 }
 
+// The plane stencil for planes of up to about 4096 pixels of any shape (3x3 or no spatial taps, four temporal
+// ones): what the walk above spends its time on is one load in flight per thread, divisions and edge
+// branches per tap and a history in shared memory.  Here a plane belongs to one warp (eight planes a CTA,
+// no CTA barrier) or to one CTA; a thread keeps J <= 8 pixels with their history in registers and
+// requests the next frame's pixels before it works on this one.  With 3x3 taps its pixels are a strip of a
+// column, so that a tile value read from shared memory serves up to three of them; the tile has a zero
+// halo and there are two in turn (one barrier per frame).
+// Bound: instruction issue and the shared-memory reads of the taps (floor 8 bytes a pixel: 24 us here).
+// 48 x 8 frames of 14x14x256, 3x3 and four taps: 365 us by the walk above, 121 with pixels dealt out a warp
+// wide, 73 as strips; 16 x 8 x 56x56 x 32: 100 -> 65 us.
+template <int KSP, int J, bool WARP>
+__global__ void __launch_bounds__(WARP ? 256 : 512, WARP ? 3 : 1) plane_stencil_small_kernel(const StencilArgs s) {
+  constexpr int KT = 4;
+  extern __shared__ __align__(16) float sm[];
+  const int W = s.W, HW = s.H * W, RS = W + 2, strips = (s.H + J - 1) / J, TS = (strips * J + 2) * RS;
+  const int nt = WARP ? 32 : blockDim.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int me = WARP ? lane : threadIdx.x, plane = WARP ? blockIdx.x * 8 + warp : blockIdx.x;
+  float* tile = KSP > 0 ? sm + (WARP ? warp * 2 * TS : 0) : nullptr;      // [2][TS]
+  float* red = sm + (KSP > 0 ? 2 * TS : 0);                               // [T][warps], CTA form only
+  auto sync = [&]() { if (WARP) __syncwarp(); else __syncthreads(); };
+  pdl_sync();
+  if (WARP && plane >= s.B * s.C) return;
+  const int b = plane / s.C, c = plane - b * s.C;
+
+  // pixels i0 + j * step, j < cnt
+  int i0 = me, step = nt, cnt = me < HW ? (HW - me + nt - 1) / nt : 0, toff = 0;
+  if (KSP > 0) {
+    const int st = me / W, w = me - st * W;
+    i0 = st * J * W + w; step = W;
+    cnt = min(J, s.H - st * J);                         // negative past the last strip
+    toff = (cnt > 0 ? st * J * RS : 0) + w;             // top left of the first pixel's window
+  }
+  float wsp[KSP > 0 ? KSP * KSP : 1], wt[KT];
+#pragma unroll
+  for (int i = 0; i < KSP * KSP; ++i) wsp[i] = __ldg(s.wsp + (size_t)i * s.C + c);
+  const float bsp = KSP > 0 ? __ldg(s.bsp + c) : 0.f;
+#pragma unroll
+  for (int j = 0; j < KT; ++j) wt[j] = __ldg(s.wt + (size_t)j * s.C + c);
+  const float btv = __ldg(s.bt + c);
+
+  const size_t pstride = (size_t)s.planes_per_frame * HW;
+  float* p = s.buf + ((size_t)(b * s.T) * s.planes_per_frame + s.plane0 + c) * HW + i0;
+  float cur[J], nxt[J], hist[J][KT - 1];      // hist[j][k] = s_{t-1-k}
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    cur[j] = j < cnt ? p[j * step] : 0.f;
+    nxt[j] = 0.f;
+#pragma unroll
+    for (int k = 0; k < KT - 1; ++k) hist[j][k] = 0.f;
+  }
+  if (KSP > 0) {
+    for (int i = me; i < 2 * TS; i += nt) tile[i] = 0.f;
+    sync();
+  }
+  for (int t = 0; t < s.T; ++t) {
+    if (t + 1 < s.T) {
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+        if (j < cnt) nxt[j] = p[pstride + j * step];
+    }
+    float v[J];
+    if (KSP > 0) {
+      float* tl = tile + (t & 1) * TS + toff;
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+        if (j < cnt) tl[(j + 1) * RS + 1] = cur[j];
+      sync();
+#pragma unroll
+      for (int j = 0; j < J; ++j) v[j] = bsp;
+#pragma unroll
+      for (int r = 0; r < J + 2; ++r) {
+        const float x0 = tl[r * RS], x1 = tl[r * RS + 1], x2 = tl[r * RS + 2];
+#pragma unroll
+        for (int di = 0; di < 3; ++di) {
+          const int j = r - di;
+          if (j < 0 || j >= J) continue;
+          v[j] = fmaf(wsp[KSP > 0 ? di * 3 : 0], x0, v[j]);
+          v[j] = fmaf(wsp[KSP > 0 ? di * 3 + 1 : 0], x1, v[j]);
+          v[j] = fmaf(wsp[KSP > 0 ? di * 3 + 2 : 0], x2, v[j]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < J; ++j) v[j] = cur[j];
+    }
+    const float* post = s.post ? s.post + ((size_t)(b * s.T + t) * HW + i0) * s.post_stride + s.post_off : nullptr;
+    float lsum = 0.f;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      float o = btv + wt[KT - 1] * v[j];
+#pragma unroll
+      for (int k = KT - 2; k >= 0; --k) o = fmaf(wt[KT - 2 - k], hist[j][k], o);
+#pragma unroll
+      for (int k = KT - 2; k > 0; --k) hist[j][k] = hist[j][k - 1];
+      hist[j][0] = v[j];
+      if (s.act) o = silu_f(o);
+      if (j < cnt) {
+        if (post) o *= __ldg(post + (size_t)(j * step) * s.post_stride);
+        p[j * step] = o;
+        lsum += o;
+      }
+      cur[j] = nxt[j];
+    }
+    p += pstride;
+    if (s.sums) {
+      for (int off = 16; off > 0; off >>= 1) lsum += __shfl_down_sync(0xffffffffu, lsum, off);
+      if (lane == 0) {
+        if (WARP) s.sums[(size_t)(b * s.T + t) * s.C + c] = lsum;
+        else red[t * (nt >> 5) + warp] = lsum;
+      }
+    }
+  }
+  if (!WARP && s.sums) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < s.T; t += nt) {
+      float tot = 0.f;
+      for (int w = 0; w < (nt >> 5); ++w) tot += red[t * (nt >> 5) + w];
+      s.sums[(size_t)(b * s.T + t) * s.C + c] = tot;
+    }
+  }
+}
+
+// the fewest threads (one warp, else a CTA) that hold the plane with at most eight pixels each
+template <int KSP>
+static int launch_stencil_small(const StencilArgs& s, cudaStream_t st, bool* handled) {
+  const int HW = s.H * s.W;
+  static const int sizes[4] = {32, 128, 256, 512}, js[4] = {2, 4, 7, 8};
+  int nt = 0, J = 0;
+  for (int k = 0; k < 4 && J == 0; ++k)
+    for (int i = 0; i < 4 && J == 0; ++i) {
+      const int j = js[i];
+      if (KSP > 0 ? (long long)s.W * ((s.H + j - 1) / j) <= sizes[k] : HW <= j * sizes[k]) { nt = sizes[k]; J = j; }
+    }
+  const bool warp = nt == 32;
+  const size_t tiles = KSP > 0 && J > 0 ? (size_t)2 * ((s.H + J - 1) / J * J + 2) * (s.W + 2) * (warp ? 8 : 1) : 0;
+  const size_t smem = (tiles + (warp ? 0 : (size_t)s.T * (nt / 32))) * sizeof(float);
+  *handled = J > 0 && smem <= 64 * 1024;
+  if (!*handled) return CSSM_OK;
+  auto go = [&](auto kern) -> int {
+    cudaError_t e = func_smem(kern, smem);
+    if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+    launch_k(kern, warp ? (s.B * s.C + 7) / 8 : s.B * s.C, warp ? 256 : nt, smem, st, s);
+    return check_launch();
+  };
+  if (warp) {
+    if (J == 2) return go(plane_stencil_small_kernel<KSP, 2, true>);
+    if (J == 4) return go(plane_stencil_small_kernel<KSP, 4, true>);
+    if (J == 7) return go(plane_stencil_small_kernel<KSP, 7, true>);
+    return go(plane_stencil_small_kernel<KSP, 8, true>);
+  }
+  if (J == 2) return go(plane_stencil_small_kernel<KSP, 2, false>);
+  if (J == 4) return go(plane_stencil_small_kernel<KSP, 4, false>);
+  if (J == 7) return go(plane_stencil_small_kernel<KSP, 7, false>);
+  return go(plane_stencil_small_kernel<KSP, 8, false>);
+}
+
 template <int KSP, int KT, int NP>
 static int launch_stencil_fast(const StencilArgs& s, cudaStream_t st) {
   const size_t smem = ((KSP > 0 ? (size_t)(s.H + 2) * (s.W + 8) : 0) + (size_t)s.T * 8) * sizeof(float);
@@ -409,6 +565,11 @@ int launch_plane_stencil(const StencilArgs& s, cudaStream_t st) {
     bool handled = false;
     const int rc = s.H * s.W == 4096 ? dispatch_stencil_fast<4>(s, st, &handled)
                                      : dispatch_stencil_fast<1>(s, st, &handled);
+    if (handled) return rc;
+  }
+  if (s.kt == 4 && (s.ksp == 0 || s.ksp == 3)) {
+    bool handled = false;
+    const int rc = s.ksp == 3 ? launch_stencil_small<3>(s, st, &handled) : launch_stencil_small<0>(s, st, &handled);
     if (handled) return rc;
   }
   const int nh = s.kt > 0 ? s.kt - 1 : 0;
