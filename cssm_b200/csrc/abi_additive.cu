@@ -27,13 +27,15 @@ __device__ __forceinline__ float add_sigmoid(float x) { return 1.0f / (1.0f + ex
 __device__ __forceinline__ float4 add_map(float rd, float rb, float rc, float inv, int floor) {
   return make_float4(0.1f + 0.89f * add_sigmoid(rd), add_sigmoid(rb), add_sigmoid(rc) * inv, floor ? 1e-7f : 0.f);
 }
-// factored: one frame per CTA row, its bins over gridDim.y CTAs
-__global__ void __launch_bounds__(256) additive_gates_factored_kernel(const AddGateArgs g) {
+// factored: one frame per CTA row, its bins over gridDim.y CTAs; 512 threads take the 3 (H + Wf) vector
+// entries of planes up to 64x64 in one pass
+constexpr int AF_THREADS = 512;
+__global__ void __launch_bounds__(AF_THREADS) additive_gates_factored_kernel(const AddGateArgs g) {
   extern __shared__ __align__(16) float sh[];
   const int Wf = g.W / 2 + 1, NB = g.H * Wf, per = g.H + Wf, fr = blockIdx.x;
   float* ctx = sh;                 // [C]
   float* vec = sh + g.C;           // 3 x (H + Wf)
-  float* scratch = vec + 3 * per;  // [256]
+  float* scratch = vec + 3 * per;  // [AF_THREADS]
   const float inv = 1.0f / (float)(g.H * g.W);
   pdl_sync();
   const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, 0, inv};
@@ -42,7 +44,7 @@ __global__ void __launch_bounds__(256) additive_gates_factored_kernel(const AddG
   gate_vectors<6>(g.gk, g.gb, off, 6, ctx, g.C, vec, scratch);
   const int per_cta = (NB + gridDim.y - 1) / gridDim.y;
   const int bin_end = min(NB, (int)(blockIdx.y + 1) * per_cta);
-  for (int bin = blockIdx.y * per_cta + threadIdx.x; bin < bin_end; bin += 256) {
+  for (int bin = blockIdx.y * per_cta + threadIdx.x; bin < bin_end; bin += AF_THREADS) {
     const int kh = bin / Wf, kw = bin - kh * Wf;
     float r[3];
 #pragma unroll
@@ -54,12 +56,12 @@ __global__ void __launch_bounds__(256) additive_gates_factored_kernel(const AddG
 template <int G>
 __global__ void __launch_bounds__(128) additive_gates_dense_kernel(const AddGateArgs g) {
   extern __shared__ __align__(16) float sh[];
-  const int Wf = g.W / 2 + 1, NB = g.H * Wf, f0 = blockIdx.y * G, nf = min(G, g.BT - f0);
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, f0 = blockIdx.x * G, nf = min(G, g.BT - f0);
   const float inv = 1.0f / (float)(g.H * g.W);
   pdl_sync();
   const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, 0, inv};
   gate_ctx(src, f0, nf, sh, sh + G * g.C);
-  const int bin = blockIdx.x * 128 + threadIdx.x;
+  const int bin = blockIdx.y * 128 + threadIdx.x;
   if (bin >= NB) return;
   float r[3][G];
   gate_dense<3, G>(g.gk, g.gb, NB, bin, g.C, sh, r);
@@ -114,12 +116,12 @@ __global__ void __launch_bounds__(256) additive_in_gate_kernel(float* __restrict
 static int launch_additive_gates(const AddGateArgs& g, cudaStream_t st) {
   const int Wf = g.W / 2 + 1, NB = g.H * Wf;
   if (g.gate_type == CSSM_GATE_FACTORED) {
-    const size_t smem = (size_t)(g.C + 3 * (g.H + Wf) + 256) * sizeof(float);
-    launch_k(additive_gates_factored_kernel, dim3(g.BT, gate_chunks(g.BT, NB)), 256, smem, st, g);
+    const size_t smem = (size_t)(g.C + 3 * (g.H + Wf) + AF_THREADS) * sizeof(float);
+    launch_k(additive_gates_factored_kernel, dim3(g.BT, gate_chunks(g.BT, NB)), AF_THREADS, smem, st, g);
     return check_launch();
   }
   const int chunks = (NB + 127) / 128, G = gate_dense_frames(g.BT, chunks);
-  const dim3 grid(chunks, (g.BT + G - 1) / G);
+  const dim3 grid((g.BT + G - 1) / G, chunks);
   const size_t smem = (size_t)(G * g.C + 128) * sizeof(float);
   if (G == 8) launch_k(additive_gates_dense_kernel<8>, grid, 128, smem, st, g);
   else if (G == 4) launch_k(additive_gates_dense_kernel<4>, grid, 128, smem, st, g);

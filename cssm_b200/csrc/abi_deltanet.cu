@@ -58,12 +58,12 @@ __global__ void __launch_bounds__(256) deltanet_gates_factored_kernel(const DnGa
 template <int G>
 __global__ void __launch_bounds__(128) deltanet_gates_dense_kernel(const DnGateArgs g) {
   extern __shared__ __align__(16) float sh[];
-  const int Wf = g.W / 2 + 1, NB = g.H * Wf, f0 = blockIdx.y * G, nf = min(G, g.BT - f0);
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, f0 = blockIdx.x * G, nf = min(G, g.BT - f0);
   const float inv = 1.0f / (float)(g.H * g.W);
   pdl_sync();
   const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, 0, inv};
   gate_ctx(src, f0, nf, sh, sh + G * g.C);
-  const int bin = blockIdx.x * 128 + threadIdx.x;
+  const int bin = blockIdx.y * 128 + threadIdx.x;
   if (bin >= NB) return;
   float r[5][G];
   gate_dense<5, G>(g.gk, g.gb, NB, bin, g.C, sh, r);
@@ -392,7 +392,7 @@ int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weigh
       launch_k(deltanet_gates_factored_kernel, dim3(BT, gate_chunks(BT, NB)), 256, smem, st, ga);
     } else {
       const int chunks = (NB + 127) / 128, G = gate_dense_frames(BT, chunks);
-      const dim3 grid(chunks, (BT + G - 1) / G);
+      const dim3 grid((BT + G - 1) / G, chunks);
       const size_t smem = (size_t)(G * C + 128) * sizeof(float);
       if (G == 8) launch_k(deltanet_gates_dense_kernel<8>, grid, 128, smem, st, ga);
       else if (G == 4) launch_k(deltanet_gates_dense_kernel<4>, grid, 128, smem, st, ga);

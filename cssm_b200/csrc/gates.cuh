@@ -6,10 +6,27 @@
 
 namespace cssm {
 
-// sum over c in [c0, c1) of ctx[c] * w[c * ld], 16 loads in flight
+// sum over c in [c0, c1) of ctx[c] * w[c * ld], 16 loads in flight; ctx is 16-byte aligned.  Whole blocks of
+// 16 run without predicates and with 16-byte reads of ctx: with one warp or two per scheduler the kernels
+// here are bound by the length of a thread's own instruction stream.
 __device__ __forceinline__ float gate_dot(const float* __restrict__ ctx, const float* __restrict__ w, int ld, int c0, int c1) {
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int c = c0; c < c1; c += 16) {
+  int c = c0;
+  if ((c0 & 3) == 0) {
+    const float* p = w + (size_t)c0 * ld;
+    for (; c + 16 <= c1; c += 16) {
+      float v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) { v[u] = __ldg(p); p += ld; }
+#pragma unroll
+      for (int u = 0; u < 16; u += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(ctx + c + u);
+        acc[0] = fmaf(x.x, v[u], acc[0]); acc[1] = fmaf(x.y, v[u + 1], acc[1]);
+        acc[2] = fmaf(x.z, v[u + 2], acc[2]); acc[3] = fmaf(x.w, v[u + 3], acc[3]);
+      }
+    }
+  }
+  for (; c < c1; c += 16) {
     float v[16];
 #pragma unroll
     for (int u = 0; u < 16; ++u) v[u] = c + u < c1 ? __ldg(w + (size_t)(c + u) * ld) : 0.f;

@@ -323,7 +323,7 @@ int launch_rope_dwconv_cl(const GdnDwArgs& a, cudaStream_t st) {
 // alpha/beta: sigmoid(row[h] + col[kw]) (factored) or sigmoid(Dense(H*Wf)) (dense);
 // alpha = 0.1 + 0.89 * raw.  Stored as float2 {alpha, beta} at bin_index(path, kh, kw).
 // B_k / B_v: same over (h, w) pixels, float2 {B_k, B_v} at h*W + w.  cssm.py:4798-4848, 4864-4865.
-__global__ void __launch_bounds__(256) gdn_gates_kernel(const GdnGateArgs g) {
+__global__ void __launch_bounds__(256, 5) gdn_gates_kernel(const GdnGateArgs g) {
   extern __shared__ __align__(16) float sh[];
   const int Wf = g.W / 2 + 1, NB = g.H * Wf, HW = g.H * g.W;
   float* ctx = sh;                       // [C]
@@ -377,16 +377,16 @@ __global__ void __launch_bounds__(256) gdn_gates_kernel(const GdnGateArgs g) {
   }
 }
 
-// Dense gates: a thread owns one bin (blockIdx.x < bin_chunks) or one pixel of G frames.
+// Dense gates: a thread owns one bin (blockIdx.y < bin_chunks) or one pixel of G frames.
 template <int G>
 __global__ void __launch_bounds__(128) gdn_gates_dense_kernel(const GdnGateArgs g, int bin_chunks) {
   extern __shared__ __align__(16) float sh[];
-  const int Wf = g.W / 2 + 1, NB = g.H * Wf, HW = g.H * g.W, f0 = blockIdx.y * G, nf = min(G, g.BT - f0);
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, HW = g.H * g.W, f0 = blockIdx.x * G, nf = min(G, g.BT - f0);
   pdl_sync();
   const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, g.ctx_per_clip, 1.0f / (float)HW};
   gate_ctx(src, f0, nf, sh, sh + G * g.C);
-  const bool bins = (int)blockIdx.x < bin_chunks;
-  const int i = (blockIdx.x - (bins ? 0 : bin_chunks)) * 128 + threadIdx.x, n = bins ? NB : HW;
+  const bool bins = (int)blockIdx.y < bin_chunks;
+  const int i = (blockIdx.y - (bins ? 0 : bin_chunks)) * 128 + threadIdx.x, n = bins ? NB : HW;
   if (i >= n) return;
   float r[2][G];
   gate_dense<2, G>(g.gk + (bins ? 0 : 2), g.gb + (bins ? 0 : 2), n, i, g.C, sh, r);
@@ -405,7 +405,7 @@ int launch_gdn_gates(const GdnGateArgs& g, cudaStream_t st) {
   if (g.gate_type == CSSM_GATE_DENSE) {
     const int bc = (g.H * Wf + 127) / 128, chunks = bc + (g.use_input_gates ? (g.H * g.W + 127) / 128 : 0);
     const int G = gate_dense_frames(g.BT, chunks);
-    const dim3 grid(chunks, (g.BT + G - 1) / G);
+    const dim3 grid((g.BT + G - 1) / G, chunks);
     const size_t smem = (size_t)(G * g.C + 128) * sizeof(float);
     if (G == 8) launch_k(gdn_gates_dense_kernel<8>, grid, 128, smem, st, g, bc);
     else if (G == 4) launch_k(gdn_gates_dense_kernel<4>, grid, 128, smem, st, g, bc);

@@ -704,12 +704,12 @@ __global__ void __launch_bounds__(GF_THREADS) gated_gates_factored_kernel(const 
 template <int G>
 __global__ void __launch_bounds__(128) gated_gates_dense_kernel(const GatedGateArgs g) {
   extern __shared__ __align__(16) float sh[];
-  const int Wf = g.W / 2 + 1, NB = g.H * Wf, f0 = blockIdx.y * G, nf = min(G, g.BT - f0);
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, f0 = blockIdx.x * G, nf = min(G, g.BT - f0);
   const float inv = 1.0f / (float)(g.H * g.W);
   pdl_sync();
   const GateCtxSrc src = {g.ctx_sum, nullptr, nullptr, 1, g.C, g.H, 0, inv};
   gate_ctx(src, f0, nf, sh, sh + G * g.C);
-  const int bin = blockIdx.x * 128 + threadIdx.x;
+  const int bin = blockIdx.y * 128 + threadIdx.x;
   if (bin >= NB) return;
   float r[3][G];
   gate_dense<3, G>(g.gk, g.gb, NB, bin, g.C, sh, r);
@@ -809,7 +809,7 @@ int launch_gated_gates(const GatedGateArgs& g, cudaStream_t st) {
     return check_launch();
   }
   const int chunks = (NB + 127) / 128, G = gate_dense_frames(g.BT, chunks);
-  const dim3 grid(chunks, (g.BT + G - 1) / G);
+  const dim3 grid((g.BT + G - 1) / G, chunks);
   const size_t smem = (size_t)(G * g.C + 128) * sizeof(float);
   if (G == 8) launch_k(gated_gates_dense_kernel<8>, grid, 128, smem, st, g);
   else if (G == 4) launch_k(gated_gates_dense_kernel<4>, grid, 128, smem, st, g);
