@@ -187,3 +187,19 @@ def test_repeated_image_qkv_conv(E, T, qkv, shape, pos):
                             readout_norm="pre", block_kwargs=bkw)
     got = m.bind({"params": p})(torch.from_numpy(x).cuda()).cpu().numpy()
     assert orc.rel_l2(got, ref) <= 1e-5
+
+
+@pytest.mark.parametrize("shape", [(1, 8, 8, 1), (1, 10, 6, 1), (2, 9, 13, 3), (1, 31, 44, 1), (8, 128, 128, 1), (3, 128, 126, 1)])
+def test_second_stem_layer_of_64_channels(shape):
+    """64 -> 64 channels, 3x3, pooled, on few images (two windows a warp): odd sides (padded pool windows, a
+    last window without a neighbour), one window, more windows than one round of warps, against the oracle.
+    float32 sums of 576 terms behind a LayerNorm: sqrt(576) * 2^-24 = 1.5e-6 of the 2-norm, checked at 5e-6."""
+    m = _model("gated", 64, 1, "none", "default", 2, "max", "pre", seq_len=1)
+    x = np.random.default_rng(shape[1]).random(shape).astype(np.float32)
+    H, W = m.feature_hw(*shape[1:3])
+    bkw = _block_kwargs(m)
+    p = so.init_simple_params(5, cin=shape[-1], embed_dim=64, H=H, W=W, num_classes=2, cssm_type="gated",
+                              stem_mode="default", stem_layers=2, bias_scale=0.1, block_kwargs=bkw)
+    ref = so.stem_forward(p, x.astype(np.float64), stem_mode="default", stem_layers=2)
+    got = m.bind({"params": p}).stem(torch.from_numpy(x).cuda()).cpu().numpy()
+    assert orc.rel_l2(got, ref) <= 5e-6
