@@ -305,9 +305,9 @@ __global__ void __launch_bounds__(STEMW_THREADS) stem_layer_wide_kernel(const St
   }
 }
 
-// Stem layer with many input channels and 64 output channels on few images.  The quad form above reads four
+// Stem layer with many input channels and 64 output channels.  The quad form above reads four
 // weight vectors per sixteen multiply-adds, the same 64 bytes for every pixel of the warp, and is bound by
-// those shared-memory reads; the window form needs more windows than a small batch has.  Here a lane owns two
+// those shared-memory reads, the window form still reads 64 bytes a time.  Here a lane owns two
 // channels (a weight read is 256 distinct bytes) of the eight pixels of two neighbouring pool windows; their
 // 4 x 6 input pixels are staged by the warp and read as broadcasts, LayerNorm sums cross the warp.
 // One CTA of twelve warps per SM (weights 147 KB + 6 KB a warp at 64 input channels).
@@ -440,19 +440,20 @@ static int launch_stem_layer_v(StemArgs a, cudaStream_t st) {
 
 template <int KS, int POOL, int CIN>
 static int launch_stem_layer_cin(const StemArgs& a, cudaStream_t st) {
-  // many input channels, pooled: the weight-reusing kernel (needs the weights in shared memory
-  // and float4 input reads)
   const size_t wbytes = (size_t)KS * KS * a.Cin * a.C * sizeof(float);
-  // it needs one full wave of windows to pay (measured at 64 -> 64 channels on 128x128 images:
-  // batch 8: 0.20 ms narrow vs 0.24 ms wide; batch 128: 2.67 vs 1.71 ms, both layers)
-  const long long windows = (long long)a.N * a.Ho * a.Wo;
-  if (CIN == 0 && POOL == 2 && a.Cin % 4 == 0 && a.Cin >= 16 && wbytes <= 200 * 1024 &&
-      windows >= 148LL * (STEMW_THREADS / 32) * 8)
-    return launch_stem_layer_wide<KS>(a, st);
+  // 64 output channels: two channels a lane, at every batch (both layers of 128x128 images, against the kernels
+  // below: batch 8 101 against 204 us, 19 196 / 468, 32 314 / 492, 128 1147 / 1718)
   const size_t pair_smem = wbytes + (3 * (size_t)a.C + STEMP_WARPS * 24 * (size_t)a.Cin) * sizeof(float);
   if (CIN == 0 && KS == 3 && POOL == 2 && a.C == SM_MAXC && a.Cin % 4 == 0 && wbytes > 64 * 1024 && pair_smem <= 227 * 1024 &&
       ((reinterpret_cast<uintptr_t>(a.wk) | reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.out)) & 15u) == 0)
     return launch_stem_layer_pair(a, pair_smem, st);
+  // many input channels, pooled: the weight-reusing kernel (needs the weights in shared memory
+  // and float4 input reads)
+  // it needs one full wave of windows to pay
+  const long long windows = (long long)a.N * a.Ho * a.Wo;
+  if (CIN == 0 && POOL == 2 && a.Cin % 4 == 0 && a.Cin >= 16 && wbytes <= 200 * 1024 &&
+      windows >= 148LL * (STEMW_THREADS / 32) * 8)
+    return launch_stem_layer_wide<KS>(a, st);
   // otherwise: weights beyond 64 KB leave room for one CTA per SM only, give that CTA 32 warps
   if (CIN == 0 && wbytes > 64 * 1024)
     return a.C == SM_MAXC ? launch_stem_layer_v<KS, POOL, 0, true, 1024>(a, st)
