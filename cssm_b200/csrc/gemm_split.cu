@@ -110,6 +110,8 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
   const uint32_t stage_bytes = GS_A_BYTES + (RES ? 0u : b_block);
   unsigned char* ring = smem + res_bytes;
   unsigned char* stg = ring + (uint32_t)NS * stage_bytes;         // 8 x 4 KB when the output is channels-last
+  // RES: bias of the CTA's N tile; else 32 floats per epilogue warp, filled for every 32-column chunk.
+  // (The bias itself is read by scalars: it may sit at any 4-byte offset of a parameter buffer.)
   float* bias_s = reinterpret_cast<float*>(stg + (A_PLANAR ? 8u * 4096u : 0u));
   float* ss_s = bias_s + 256;                                     // [GS_SS][2][128] row sums (RMS prologue)
   uint64_t* bars = reinterpret_cast<uint64_t*>(ss_s + (A_PLANAR ? GS_SS * 256 : 0));
@@ -409,6 +411,13 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
         if (n >= g.N) break;
         const bool zcols = n >= g.act_n0;               // all 32 columns are activated ones
         if (!A_PLANAR && zcols && g.z_last_only && !__any_sync(0xffffffffu, zrow)) continue;
+        const float* bias_c = bias_s + (RES ? cc * 32 : (warp - (GS_MMA_WARP + 1)) * 32);
+        if (!RES) {
+          const float b = (g.bias && n + lane < g.N) ? __ldg(g.bias + n + lane) : 0.f;
+          __syncwarp();                                 // the chunk before has been read
+          bias_s[(warp - (GS_MMA_WARP + 1)) * 32 + lane] = b;
+          __syncwarp();
+        }
         float v[32];
         {
           uint32_t r[32];
@@ -429,9 +438,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
         }
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
-          float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (RES) b = *reinterpret_cast<const float4*>(bias_s + cc * 32 + j);
-          else if (g.bias && n + j < g.N) b = __ldg(reinterpret_cast<const float4*>(g.bias + n + j));
+          const float4 b = *reinterpret_cast<const float4*>(bias_c + j);
           v[j] = fmaf(v[j], rinv, b.x);         v[j + 1] = fmaf(v[j + 1], rinv, b.y);
           v[j + 2] = fmaf(v[j + 2], rinv, b.z); v[j + 3] = fmaf(v[j + 3], rinv, b.w);
         }

@@ -48,3 +48,25 @@ def test_projections_against_float64(B, T, H, W, Cc):
     assert rel(y.double().reshape(ref.shape), ref) < 8e-7
     torch.cuda.synchronize()
     assert device_error() == 0
+
+
+@pytest.mark.parametrize("Cc", [64, 256, 384])
+def test_bias_at_a_four_byte_offset(Cc):
+    """Biases that are views into a flat parameter buffer, one float off any wider alignment: resident
+    weights (64, and in_proj at 256) and streamed ones (out_proj at 256, both at 384) give the bits of the
+    same call with aligned biases."""
+    mod = GatedCSSM(channels=Cc, kernel_size=1, gate_type="factored")
+    x = torch.randn((1, 2, 14, 13, Cc), device="cuda", generator=torch.Generator(device="cuda").manual_seed(Cc))
+    v = mod.init(5, tuple(x.shape), bias_scale=0.3)
+    want = mod.bind(v)(x).clone()
+    p = dict(v["params"])
+    for name in ("in_proj", "out_proj"):
+        b = torch.from_numpy(p[name]["bias"]).cuda()
+        flat = torch.zeros(b.numel() + 1, device="cuda")
+        flat[1:] = b
+        p[name] = {"kernel": p[name]["kernel"], "bias": flat[1:]}
+        assert flat[1:].data_ptr() % 16 == 4
+    got = mod.bind({"params": p})(x)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    assert device_error() == 0
