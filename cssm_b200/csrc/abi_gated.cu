@@ -5,6 +5,7 @@
 #include <cuda_bf16.h>
 #include "kernels.cuh"
 #include "gemm.cuh"
+#include "smem_limit.h"
 
 namespace cssm {
 
@@ -16,26 +17,20 @@ void set_cuda_error(cudaError_t e) {
 
 thread_local int g_pdl = 0;
 
-// Open-addressed table keyed by the kernel's address; entries are only ever added, and a lost race at
-// worst repeats the call.
 cudaError_t func_smem_set(const void* kern, size_t bytes) {
-  constexpr int SLOTS = 512, DEVS = 16;
-  struct Entry { std::atomic<const void*> key; std::atomic<int> size[DEVS]; };
-  static Entry table[SLOTS];
+  static SmemLimits limits;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  Entry* hit = nullptr;
-  size_t h = (reinterpret_cast<uintptr_t>(kern) >> 4) % SLOTS;
-  for (int i = 0; i < SLOTS && dev < DEVS; ++i, h = (h + 1) % SLOTS) {
-    const void* k = table[h].key.load(std::memory_order_acquire);
-    if (k == nullptr && table[h].key.compare_exchange_strong(k, kern)) k = kern;
-    if (k == kern) { hit = &table[h]; break; }
-  }
-  if (hit != nullptr && (size_t)hit->size[dev].load(std::memory_order_acquire) >= bytes && bytes > 0) return cudaSuccess;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess && hit != nullptr) hit->size[dev].store((int)bytes, std::memory_order_release);
-  return e;
+  return (cudaError_t)limits.raise(
+      kern, dev, bytes,
+      [&](size_t* now) {
+        cudaFuncAttributes at;
+        const cudaError_t r = cudaFuncGetAttributes(&at, kern);
+        *now = r == cudaSuccess ? (size_t)at.maxDynamicSharedSizeBytes : 0;
+        return (int)r;
+      },
+      [&](size_t n) { return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n); });
 }
 
 int sm_count() {

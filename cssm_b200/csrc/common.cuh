@@ -107,8 +107,8 @@ inline void launch_k(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cud
   cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);     // errors are read by check_launch
   if (g_pdl == 1) g_pdl = 2;
 }
-// cudaFuncAttributeMaxDynamicSharedMemorySize, set once per kernel, device and size (the call costs as
-// much host time as a launch)
+// cudaFuncAttributeMaxDynamicSharedMemorySize of the current device is at least `bytes` from here on: it only ever
+// rises (smem_limit.h)
 cudaError_t func_smem_set(const void* kern, size_t bytes);
 template <class F> inline cudaError_t func_smem(F* kern, size_t bytes) {
   return func_smem_set(reinterpret_cast<const void*>(kern), bytes);

@@ -1,0 +1,38 @@
+// Which limit of dynamic shared memory each kernel has been given, so that it is set when it has to rise and
+// not at every launch.  Host code only.
+#pragma once
+#include <cstddef>
+#include <map>
+#include <mutex>
+#include <utility>
+
+namespace cssm {
+
+// The limit is one attribute of a kernel that all threads share, and a launch reads it some time after
+// raise() has returned.  So it never falls (a smaller request of another thread must not undercut a launch
+// that is still to come), and check, call and record are one step under the lock: when raise() returns
+// success the limit holds `bytes` and keeps doing so.
+class SmemLimits {
+ public:
+  // get(&limit) reads the limit in force, set(bytes) changes it; both return 0 on success
+  template <class Get, class Set>
+  int raise(const void* kern, int device, std::size_t bytes, Get&& get, Set&& set) {
+    std::lock_guard<std::mutex> lock(mu_);
+    std::size_t& known = known_[{kern, device}];
+    if (known >= bytes && known > 0) return 0;
+    std::size_t now = 0;
+    int e = get(&now);
+    if (e == 0 && now < bytes) {
+      e = set(bytes);
+      now = bytes;
+    }
+    if (e == 0) known = now;
+    return e;
+  }
+
+ private:
+  std::mutex mu_;
+  std::map<std::pair<const void*, int>, std::size_t> known_;
+};
+
+}  // namespace cssm
