@@ -2,6 +2,7 @@
 #include <string.h>
 #include <stdio.h>
 #include <atomic>
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include "kernels.cuh"
 #include "gemm.cuh"
@@ -17,13 +18,24 @@ void set_cuda_error(cudaError_t e) {
 
 thread_local int g_pdl = 0;
 
+// Id of the calling thread's current context, 0 if it has none yet.  (10 ns; a launch takes 4 us.)
+static unsigned long long context_id() {
+  typedef CUresult (*GetId)(CUcontext, unsigned long long*);
+  static const GetId get = []() -> GetId {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+      return nullptr;
+    return reinterpret_cast<GetId>(p);
+  }();
+  unsigned long long id = 0;
+  return get != nullptr && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 cudaError_t func_smem_set(const void* kern, size_t bytes) {
   static SmemLimits limits;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
   return (cudaError_t)limits.raise(
-      kern, dev, bytes,
+      kern, context_id(), bytes,
       [&](size_t* now) {
         cudaFuncAttributes at;
         const cudaError_t r = cudaFuncGetAttributes(&at, kern);

@@ -12,27 +12,34 @@ namespace cssm {
 // raise() has returned.  So it never falls (a smaller request of another thread must not undercut a launch
 // that is still to come), and check, call and record are one step under the lock: when raise() returns
 // success the limit holds `bytes` and keeps doing so.
+//
+// The attribute lives as long as the context it was set in: `context` is an id that is never given twice, so
+// that after a cudaDeviceReset nothing is believed that was set before (0: unknown, nothing is remembered).
 class SmemLimits {
  public:
   // get(&limit) reads the limit in force, set(bytes) changes it; both return 0 on success
   template <class Get, class Set>
-  int raise(const void* kern, int device, std::size_t bytes, Get&& get, Set&& set) {
+  int raise(const void* kern, unsigned long long context, std::size_t bytes, Get&& get, Set&& set) {
     std::lock_guard<std::mutex> lock(mu_);
-    std::size_t& known = known_[{kern, device}];
-    if (known >= bytes && known > 0) return 0;
+    const auto it = known_.find({kern, context});
+    if (context != 0 && it != known_.end() && it->second >= bytes) return 0;
     std::size_t now = 0;
     int e = get(&now);
     if (e == 0 && now < bytes) {
       e = set(bytes);
       now = bytes;
     }
-    if (e == 0) known = now;
+    if (e == 0 && context != 0) {
+      if (known_.size() >= MAX_KNOWN) known_.clear();      // of dead contexts, mostly; the rest is read again
+      known_[{kern, context}] = now;
+    }
     return e;
   }
 
  private:
+  static constexpr std::size_t MAX_KNOWN = 4096;
   std::mutex mu_;
-  std::map<std::pair<const void*, int>, std::size_t> known_;
+  std::map<std::pair<const void*, unsigned long long>, std::size_t> known_;
 };
 
 }  // namespace cssm

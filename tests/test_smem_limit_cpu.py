@@ -28,7 +28,7 @@ int main() {
       for (int i = 0; i < 40; ++i) {
         const int k = r() % 2;
         const size_t bytes = 1000 * (1 + r() % 220);
-        const int e = limits.raise(&attr[k], 0, bytes, [&](size_t* n) { *n = attr[k].load(); return 0; },
+        const int e = limits.raise(&attr[k], 1, bytes, [&](size_t* n) { *n = attr[k].load(); return 0; },
                                    [&](size_t n) { nap(); attr[k].store(n); ++calls; nap(); return 0; });
         nap();                                          // the launch comes later
         if (e != 0 || attr[k].load() < bytes) ++short_of;
@@ -41,12 +41,17 @@ int main() {
     // a failing setter is reported and not remembered
     size_t now = 49152;
     auto get = [&](size_t* n) { *n = now; return 0; };
-    if (limits.raise(&now, 0, 60000, get, [](size_t) { return 7; }) != 7) ++bad;
-    if (limits.raise(&now, 0, 60000, get, [&](size_t n) { now = n; return 0; }) != 0 || now != 60000) ++bad;
-    // another device has a limit of its own
-    size_t other = 49152;
-    limits.raise(&now, 1, 60000, [&](size_t* n) { *n = other; return 0; }, [&](size_t n) { other = n; return 0; });
-    if (other != 60000) ++bad;
+    if (limits.raise(&now, 1, 60000, get, [](size_t) { return 7; }) != 7) ++bad;
+    if (limits.raise(&now, 1, 60000, get, [&](size_t n) { now = n; return 0; }) != 0 || now != 60000) ++bad;
+    // a new context starts over; an unknown one (0) is asked every time
+    for (unsigned long long context : {2ull, 0ull}) {
+      now = 49152;
+      limits.raise(&now, context, 60000, get, [&](size_t n) { now = n; return 0; });
+      if (now != 60000) ++bad;
+    }
+    now = 49152;
+    limits.raise(&now, 0, 60000, get, [&](size_t n) { now = n; return 0; });
+    if (now != 60000) ++bad;
   }
   std::printf("%d\n", bad);
   return bad != 0;
