@@ -117,16 +117,13 @@ static int launch_additive_gates(const AddGateArgs& g, cudaStream_t st) {
   const int Wf = g.W / 2 + 1, NB = g.H * Wf;
   if (g.gate_type == CSSM_GATE_FACTORED) {
     const size_t smem = (size_t)(g.C + 3 * (g.H + Wf) + AF_THREADS) * sizeof(float);
-    launch_k(additive_gates_factored_kernel, dim3(g.BT, gate_chunks(g.BT, NB)), AF_THREADS, smem, st, g);
-    return check_launch();
+    return launch_gates(additive_gates_factored_kernel, dim3(g.BT, gate_chunks(g.BT, NB)), AF_THREADS, smem, st, g);
   }
-  const int chunks = (NB + 127) / 128, G = gate_dense_frames(g.BT, chunks);
+  const int chunks = (NB + 127) / 128, G = gate_dense_frames(g.BT, chunks, g.C);
   const dim3 grid((g.BT + G - 1) / G, chunks);
   const size_t smem = (size_t)(G * g.C + 128) * sizeof(float);
-  if (G == 8) launch_k(additive_gates_dense_kernel<8>, grid, 128, smem, st, g);
-  else if (G == 4) launch_k(additive_gates_dense_kernel<4>, grid, 128, smem, st, g);
-  else launch_k(additive_gates_dense_kernel<1>, grid, 128, smem, st, g);
-  return check_launch();
+  return launch_gates(G == 8 ? additive_gates_dense_kernel<8> : G == 4 ? additive_gates_dense_kernel<4> : additive_gates_dense_kernel<1>,
+                      grid, 128, smem, st, g);
 }
 
 static int additive_validate(const cssm_additive_desc* d) {
@@ -296,8 +293,7 @@ int cssm_additive_forward(const cssm_additive_desc* d, const cssm_additive_weigh
     ca.BT = BT; ca.T = d->T; ca.C = C; ca.H = d->H; ca.W = d->W; ca.goom_floor = d->goom_floor;
     ca.dk = w->gate_kernel[0]; ca.db = w->gate_bias[0];
     ca.dchan = (float*)(ws + l.dchan); ca.maps = (float4*)(ws + l.maps);
-    launch_k(additive_chan_gates_kernel, BT, 256, (size_t)(2 * C + 256) * sizeof(float), st, ca);
-    if ((s = check_launch()) != CSSM_OK) return s;
+    if ((s = launch_gates(additive_chan_gates_kernel, BT, 256, (size_t)(2 * C + 256) * sizeof(float), st, ca)) != CSSM_OK) return s;
     // C_gate planes sigmoid(Conv1x1(rotated x))
     memset(&g, 0, sizeof(g));
     g.M = BT * HW; g.N = C; g.K = C; g.HW = HW;

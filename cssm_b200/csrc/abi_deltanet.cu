@@ -367,8 +367,7 @@ int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weigh
     ca.BT = BT; ca.T = d->T; ca.C = C; ca.H = d->H; ca.W = d->W;
     ca.ak = w->gate_kernel[0]; ca.ab = w->gate_bias[0]; ca.bk = w->gate_kernel[1]; ca.bb = w->gate_bias[1];
     ca.chan = (float2*)(ws + l.chan);
-    launch_k(deltanet_chan_gates_kernel, BT, 256, (size_t)(3 * C + 256) * sizeof(float), st, ca);
-    if ((s = check_launch()) != CSSM_OK) return s;
+    if ((s = launch_gates(deltanet_chan_gates_kernel, BT, 256, (size_t)(3 * C + 256) * sizeof(float), st, ca)) != CSSM_OK) return s;
     // spatial gates sigmoid(Conv1x1(rotated x)) -> planes (BT, 3C, H, W): B_k, B_v, C_gate
     float* gsp = (float*)(ws + l.gsp);
     memset(&g, 0, sizeof(g));
@@ -389,16 +388,15 @@ int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weigh
     const int Wf = d->W / 2 + 1, NB = d->H * Wf;
     if (d->gate_type == CSSM_GATE_FACTORED) {
       const size_t smem = (size_t)(C + 5 * (d->H + Wf) + 256) * sizeof(float);
-      launch_k(deltanet_gates_factored_kernel, dim3(BT, gate_chunks(BT, NB)), 256, smem, st, ga);
+      s = launch_gates(deltanet_gates_factored_kernel, dim3(BT, gate_chunks(BT, NB)), 256, smem, st, ga);
     } else {
-      const int chunks = (NB + 127) / 128, G = gate_dense_frames(BT, chunks);
+      const int chunks = (NB + 127) / 128, G = gate_dense_frames(BT, chunks, C);
       const dim3 grid((BT + G - 1) / G, chunks);
       const size_t smem = (size_t)(G * C + 128) * sizeof(float);
-      if (G == 8) launch_k(deltanet_gates_dense_kernel<8>, grid, 128, smem, st, ga);
-      else if (G == 4) launch_k(deltanet_gates_dense_kernel<4>, grid, 128, smem, st, ga);
-      else launch_k(deltanet_gates_dense_kernel<1>, grid, 128, smem, st, ga);
+      s = launch_gates(G == 8 ? deltanet_gates_dense_kernel<8> : G == 4 ? deltanet_gates_dense_kernel<4> : deltanet_gates_dense_kernel<1>,
+                       grid, 128, smem, st, ga);
     }
-    if ((s = check_launch()) != CSSM_OK) return s;
+    if (s != CSSM_OK) return s;
   }
 
   // 4. fused transforms + delta rule + output gate, output planes over the v planes

@@ -148,10 +148,10 @@ __device__ __forceinline__ void gate_dense(const float* const* gk, const float* 
 }
 
 // Frames per CTA of a dense-gate launch with `chunks` CTAs per frame group: a weight read serves that many
-// frames, as long as the SMs stay covered.
-inline int gate_dense_frames(int BT, int chunks) {
-  if ((long long)(BT / 8) * chunks >= 148) return 8;
-  if ((long long)(BT / 4) * chunks >= 148) return 4;
+// frames, as long as the SMs stay covered and two CTAs fit an SM with their contexts.
+inline int gate_dense_frames(int BT, int chunks, int C) {
+  for (int G : {8, 4})
+    if ((long long)(BT / G) * chunks >= 148 && (size_t)(G * C + 128) * sizeof(float) <= 100 * 1024) return G;
   return 1;
 }
 // CTAs per frame of a factored-gate launch: enough to cover the SMs, at most one per 256 bins
@@ -163,6 +163,18 @@ inline int gate_chunks(int BT, int NB) {
     if (chunks > maxc) chunks = maxc;
   }
   return chunks;
+}
+
+// Launch of a gate-map kernel: its contexts and vectors may need more than the 48 KB a launch has by default
+// (wide blocks, long planes).
+template <class... P, class... A>
+inline int launch_gates(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  if (smem > 48 * 1024) {
+    const cudaError_t e = func_smem(kern, smem);
+    if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  }
+  launch_k(kern, grid, dim3(threads), smem, st, args...);
+  return check_launch();
 }
 
 }  // namespace cssm

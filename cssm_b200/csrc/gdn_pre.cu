@@ -404,17 +404,14 @@ int launch_gdn_gates(const GdnGateArgs& g, cudaStream_t st) {
   const int Wf = g.W / 2 + 1;
   if (g.gate_type == CSSM_GATE_DENSE) {
     const int bc = (g.H * Wf + 127) / 128, chunks = bc + (g.use_input_gates ? (g.H * g.W + 127) / 128 : 0);
-    const int G = gate_dense_frames(g.BT, chunks);
+    const int G = gate_dense_frames(g.BT, chunks, g.C);
     const dim3 grid((g.BT + G - 1) / G, chunks);
     const size_t smem = (size_t)(G * g.C + 128) * sizeof(float);
-    if (G == 8) launch_k(gdn_gates_dense_kernel<8>, grid, 128, smem, st, g, bc);
-    else if (G == 4) launch_k(gdn_gates_dense_kernel<4>, grid, 128, smem, st, g, bc);
-    else launch_k(gdn_gates_dense_kernel<1>, grid, 128, smem, st, g, bc);
-    return check_launch();
+    return launch_gates(G == 8 ? gdn_gates_dense_kernel<8> : G == 4 ? gdn_gates_dense_kernel<4> : gdn_gates_dense_kernel<1>,
+                        grid, 128, smem, st, g, bc);
   }
   const size_t smem = (size_t)(g.C + 256 + 4 * g.H + 2 * Wf + 2 * g.W + 4 * g.nh + 8) * sizeof(float);
-  launch_k(gdn_gates_kernel, g.BT, 256, smem, st, g);
-  return check_launch();
+  return launch_gates(gdn_gates_kernel, g.BT, 256, smem, st, g);
 }
 
 }  // namespace cssm

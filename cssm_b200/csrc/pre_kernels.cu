@@ -805,16 +805,13 @@ int launch_gated_gates(const GatedGateArgs& g, cudaStream_t st) {
   const int NB = g.H * Wf;
   if (g.gate_type == CSSM_GATE_FACTORED) {
     const size_t smem = (size_t)(g.C + 3 * (g.H + Wf) + GF_THREADS) * sizeof(float);
-    launch_k(gated_gates_factored_kernel, dim3(g.BT, gate_chunks(g.BT, NB)), GF_THREADS, smem, st, g);
-    return check_launch();
+    return launch_gates(gated_gates_factored_kernel, dim3(g.BT, gate_chunks(g.BT, NB)), GF_THREADS, smem, st, g);
   }
-  const int chunks = (NB + 127) / 128, G = gate_dense_frames(g.BT, chunks);
+  const int chunks = (NB + 127) / 128, G = gate_dense_frames(g.BT, chunks, g.C);
   const dim3 grid((g.BT + G - 1) / G, chunks);
   const size_t smem = (size_t)(G * g.C + 128) * sizeof(float);
-  if (G == 8) launch_k(gated_gates_dense_kernel<8>, grid, 128, smem, st, g);
-  else if (G == 4) launch_k(gated_gates_dense_kernel<4>, grid, 128, smem, st, g);
-  else launch_k(gated_gates_dense_kernel<1>, grid, 128, smem, st, g);
-  return check_launch();
+  return launch_gates(G == 8 ? gated_gates_dense_kernel<8> : G == 4 ? gated_gates_dense_kernel<4> : gated_gates_dense_kernel<1>,
+                      grid, 128, smem, st, g);
 }
 
 }  // namespace cssm
