@@ -1044,9 +1044,13 @@ int launch_head(const float* pooled, const float* W, const float* b, float* logi
       return check_launch();
     }
   }
-  const int nx = (K + 31) / 32;
-  if (Nimg >= 8) launch_k(head_slice_kernel<8>, dim3(nx, (Nimg + 7) / 8), 256, (size_t)(8 * C + 8 * 8 * 32) * 4, st, pooled, W, b, logits, Nimg, C, K);
-  else launch_k(head_slice_kernel<1>, dim3(nx, Nimg), 256, (size_t)(C + 8 * 32) * 4, st, pooled, W, b, logits, Nimg, C, K);
+  // NS rows of C channels and the partial sums: above the 48 KB default from 1284 channels at NS = 8
+  const int nx = (K + 31) / 32, NS = Nimg >= 8 ? 8 : 1;
+  auto kern = NS == 8 ? head_slice_kernel<8> : head_slice_kernel<1>;
+  const size_t smem = (size_t)NS * (C + 8 * 32) * 4;
+  const cudaError_t e = func_smem(kern, smem);
+  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  launch_k(kern, dim3(nx, (Nimg + NS - 1) / NS), 256, smem, st, pooled, W, b, logits, Nimg, C, K);
   return check_launch();
 }
 

@@ -208,3 +208,15 @@ def test_cfg5_full_batch_picked_samples():
     ref = sv.shvit_forward(p, s, x[pick].float().numpy().astype(np.float64), **bench.shvit_model_kwargs("cfg5"))
     for i, b in enumerate(pick):
         assert orc.rel_l2(y[b], ref[i]) <= 2e-2, (b, orc.rel_l2(y[b], ref[i]))
+
+
+@pytest.mark.parametrize("C,B,classes", [(1280, 8, 10), (1344, 9, 10), (1536, 8, 6), (1536, 3, 10)])
+def test_head_of_wide_last_stages(C, B, classes):
+    """Around and above 1284 channels eight pooled rows and their partial sums leave the 48 KB of shared
+    memory that a launch has by default; logits against the oracle (bf16 model: 2e-2)."""
+    kw = dict(embed_dims=(32, 32, 64, C), depths=(1, 1, 1, 1), kernel_sizes=(1, 1, 1, 1), short_conv_spatial_size=0)
+    p, s = sv.init_shvit_params(11, (64, 64), num_classes=classes, **kw)
+    x = torch.randn((B, 64, 64, 3), generator=torch.Generator().manual_seed(C)).to(torch.bfloat16)
+    got = CSSMSHViT(num_classes=classes, num_timesteps=1, **kw).apply({"params": p, "batch_stats": s}, x.cuda())
+    want = sv.shvit_forward(p, s, x.float().numpy().astype(np.float64), num_timesteps=1, **kw)
+    assert orc.rel_l2(got.cpu().numpy(), want) <= 2e-2
