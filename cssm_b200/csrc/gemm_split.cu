@@ -5,8 +5,14 @@
 // whose weight reaches 2^-16 of the leading one (00, 01, 10, 11, 02, 20), accumulated in float32 in
 // TMEM.  What is dropped is below 2^-24 of |a||b|.  A bf16 MMA runs at twice the tf32 rate, so six of them
 // cost what three tf32 passes cost, in three quarters of the shared memory.  The accumulator truncates
-// at every MMA, so with more than one K block the 00 products have an accumulator of their own and the
-// five small ones another (24 truncations of the full sum at K = 384 instead of 144: relative error 2.2e-6 before).
+// at every MMA, so with more than one K block the 00 products have accumulators of their own and the five
+// small ones another (24 truncations of the full sum at K = 384 instead of 144: relative error 2.2e-6 before).
+// The truncations all go toward zero, so the error of one accumulator grows like the number of MMAs added to it
+// (0.56e-7 of the 2-norm for every K block of 64), that of float32 FMAs like its root (1.37e-7 sqrt(K blocks)).
+// Above six K blocks the 00 products are therefore dealt out to several accumulators (WIDE) of at most
+// 2 sqrt(K blocks) each, which the epilogue adds in registers, rounding to nearest.  Error against float64 (1e-7)
+// with one leading accumulator / so / with FMAs: K = 512 4.5 / 2.2 / 3.9, 1024 9.5 / 4.5 / 5.5, 2048 20 / 6.2 / 7.8,
+// 4096 42 / 9.6 / 11; it costs less than 1 % (96 x 14 x 14 x 1024, whole block: 1965 -> 1974 us).
 //
 // Persistent kernel, one CTA per SM, 544 threads, warp-specialised:
 //   warps 0-7  producers : 128-row x 64-k A blocks from global memory (channels-last rows with RoPE
@@ -30,6 +36,7 @@
 // out_proj 33 x 16^2, 256 -> 256: 121 -> 36 us; 16 x 8 x 56^2, 32 -> 64: 150 -> 67 us, 32 -> 32: 134 -> 37 us.
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <math.h>
 #include <string.h>
 #include "kernels.cuh"
 #include "gemm.cuh"
@@ -59,7 +66,10 @@ template <int V> struct Int { static constexpr int value = V; };
 
 struct SplitGeom {
   int BN, n_tiles, m_tiles, kblocks, stages;
-  int corr;                           // 1: separate accumulator for the small partial products
+  int nl;                             // leading accumulators beside that of the small partial products (0: one for all)
+  int lead;                           // WIDE: K blocks of one leading accumulator
+  int bufs;                           // WIDE: accumulator sets, 2 (the epilogue drains one while the MMAs fill the
+                                      // other) or 1; otherwise 2
   FastDiv hw, w, t, fdiv;             // divisions by HW, W, T and the source-frame divisor
 };
 
@@ -96,8 +106,8 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
 }
 
-// GATE: planar A times the gate planes.
-template <bool A_PLANAR, bool RES, bool GATE>
+// GATE: planar A times the gate planes.  WIDE: more than one leading accumulator (nl > 1).
+template <bool A_PLANAR, bool RES, bool GATE, bool WIDE>
 __global__ void __launch_bounds__(GS_THREADS, 1)
 gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ CUtensorMap omap) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -117,16 +127,17 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
   uint64_t* bars = reinterpret_cast<uint64_t*>(ss_s + (A_PLANAR ? GS_SS * 256 : 0));
   uint64_t* full = bars;           // [4] block written (8 producer warps)
   uint64_t* empty = bars + 4;      // [4] block consumed (tcgen05.commit)
-  uint64_t* accfull = bars + 8;    // [2] accumulator complete (tcgen05.commit)
-  uint64_t* accempty = bars + 10;  // [2] accumulator drained (8 epilogue warps)
+  uint64_t* accfull = bars + 8;    // [2] accumulator set complete (tcgen05.commit)
+  uint64_t* accempty = bars + 10;  // [2] accumulator set drained (8 epilogue warps)
   uint64_t* done = bars + 12;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int num_tiles = q.m_tiles * q.n_tiles;
-  const uint32_t acc_cols = q.corr ? 2u * BN : BN;                // TMEM columns of one accumulator (pair)
+  const int bufs = WIDE ? q.bufs : 2;
+  const uint32_t acc_cols = WIDE ? (1u + (uint32_t)q.nl) * BN : (q.nl ? 2u * BN : BN);      // of one set: [small | leading 0 | ...]
   uint32_t tmem_cols = 32;
-  while (tmem_cols < 2u * acc_cols) tmem_cols <<= 1;
+  while (tmem_cols < (uint32_t)bufs * acc_cols) tmem_cols <<= 1;
 
   if (tid == 0) {
     for (int s = 0; s < NS; ++s) { tc::mbar_init(&full[s], GS_PROD / 32); tc::mbar_init(&empty[s], 1); }
@@ -346,6 +357,8 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
       if (!tc::mbar_wait(&accempty[ac], aph)) { atomicExch(&g_split_error, 2); ok = false; break; }
       tc::fence_after_sync();
       const uint32_t d = tmem_base + (uint32_t)ac * acc_cols;
+      uint32_t d00 = WIDE || !q.nl ? d : d + BN;
+      int left = 0;                                     // WIDE: K blocks that still go to the leading accumulator d00
       for (int kb = 0; kb < kblocks; ++kb) {
         if (!tc::mbar_wait(&full[s], sph)) { atomicExch(&g_split_error, 2); ok = false; break; }
         tc::fence_after_sync();
@@ -354,7 +367,13 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
         const uint64_t ad0 = tc::make_desc_sw128(a_s), bd0 = tc::make_desc_sw128(b_s);
         const uint64_t bp = (uint64_t)(b_part >> 4);
         const uint64_t bd[3] = {bd0, bd0 + bp, bd0 + 2 * bp};
-        const uint32_t d00 = q.corr ? d + BN : d, first = kb == 0 ? 0u : 1u;
+        const uint32_t first = kb == 0 ? 0u : 1u;
+        uint32_t first00 = q.nl ? first : 1u;           // (one accumulator: the small products came before)
+        if (WIDE) {
+          first00 = left == 0 ? 0u : 1u;
+          if (left == 0) { d00 += BN; left = q.lead; }
+          --left;
+        }
         auto issue = [&](auto steps) {
           constexpr int KS = decltype(steps)::value;
 #pragma unroll
@@ -362,7 +381,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
 #pragma unroll
             for (int ks = 0; ks < KS; ++ks)
               mma_f16(p == 5 ? d00 : d, ad0 + PA[p] * (GS_A_PART >> 4) + ks * 2, bd[PB[p]] + ks * 2, idesc,
-                      p == 5 && ks == 0 ? (q.corr ? first : 1u) : (p | ks ? 1u : first), lead);
+                      p == 5 && ks == 0 ? first00 : (p | ks ? 1u : first), lead);
         };
         const int krem = g.K - kb * GS_BK;
         if (krem > 48) issue(Int<4>());
@@ -373,8 +392,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
         if (++s == NS) { s = 0; sph ^= 1; }
       }
       if (ok && lane == 0) tc::commit(&accfull[ac]);
-      if (ac == 1) aph ^= 1;
-      ac ^= 1;
+      if (++ac == bufs) { ac = 0; aph ^= 1; }
     }
     // nothing of lane 0's tensor work may be in flight when TMEM is freed
     if (lane == 0) tc::commit(done);
@@ -388,7 +406,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
     unsigned char* my_stg = stg + (uint32_t)(warp - (GS_MMA_WARP + 1)) * 4096u;
     int tcnt = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++tcnt) {
-      const int ac = tcnt & 1, ph = (tcnt >> 1) & 1;
+      const int ac = tcnt & (bufs - 1), ph = (tcnt >> (bufs - 1)) & 1;
       const int m0 = (tile / q.n_tiles) * GS_BM, n0 = (tile % q.n_tiles) * q.BN;
       const int m = m0 + row;
       int fr = 0, px = 0;
@@ -426,11 +444,11 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
         }
-        if (q.corr) {
+        for (int l = 1; l <= (WIDE ? q.nl : q.nl ? 1 : 0); ++l) {
 #pragma unroll
           for (int hf = 0; hf < 2; ++hf) {
             uint32_t r[16];
-            tc::ld_32x32b_x16(taddr + BN + cc * 32 + hf * 16, r);
+            tc::ld_32x32b_x16(taddr + l * BN + cc * 32 + hf * 16, r);
             tc::wait_ld();
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[hf * 16 + j] += __uint_as_float(r[j]);
@@ -543,13 +561,24 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   auto res_size = [&](int bn) { return (size_t)q.kblocks * 3 * bn * 128; };
   // Weights resident when a tile of at least 64 columns (or all of N) leaves room for two A stages:
   // every CTA then splits its weights once.  Otherwise 128-column tiles with the weights streamed.
-  q.corr = q.kblocks > 1 ? 1 : 0;
-  int nt = q.corr ? (g.N + 127) / 128 : (g.N + 255) / 256;
+  // The leading accumulators and the one of the small products of a tile share the 512 columns of TMEM.
+  q.nl = q.kblocks > 1 ? 1 : 0;
+  q.lead = q.kblocks;
+  if (q.kblocks > 6) {
+    const int most = (int)(2.0 * sqrt((double)q.kblocks)) > 6 ? (int)(2.0 * sqrt((double)q.kblocks)) : 6;
+    q.nl = (q.kblocks + most - 1) / most;
+    if (q.nl > 15) q.nl = 15;
+    q.lead = (q.kblocks + q.nl - 1) / q.nl;
+  }
+  const bool wide = q.nl > 1;
+  const int bn_tmem = 512 / (1 + q.nl) / 32 * 32;
+  int nt = q.nl > 0 ? (g.N + 127) / 128 : (g.N + 255) / 256;
   while (round32((g.N + nt - 1) / nt) > 32 && res_size(round32((g.N + nt - 1) / nt)) + 2 * GS_A_BYTES + fixed > LIMIT) ++nt;
   q.BN = round32((g.N + nt - 1) / nt);
-  const bool res = (q.BN >= 64 || nt == 1) && res_size(q.BN) + 2 * GS_A_BYTES + fixed <= LIMIT;
+  const bool res = !wide && (q.BN >= 64 || nt == 1) && res_size(q.BN) + 2 * GS_A_BYTES + fixed <= LIMIT;
   if (!res) {
-    const int most = a_planar ? 96 : 128;
+    int most = a_planar ? 96 : 128;
+    if (most > bn_tmem) most = bn_tmem;
     nt = (g.N + most - 1) / most;
     q.BN = round32((g.N + nt - 1) / nt);
   }
@@ -560,6 +589,7 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   for (int k = nt + 1; q.BN > 32 && q.m_tiles * ((g.N + q.BN - 1) / q.BN) * 3 < sms * 2; ++k)
     q.BN = round32((g.N + k - 1) / k);
   q.n_tiles = (g.N + q.BN - 1) / q.BN;
+  q.bufs = 2 * (1 + q.nl) * q.BN <= 512 ? 2 : 1;
   const size_t stage = GS_A_BYTES + (res ? 0 : (size_t)3 * q.BN * 128);
   const size_t base = (res ? res_size(q.BN) : 0) + fixed;
   q.stages = 4;
@@ -584,9 +614,12 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
       return CSSM_ERR_CUDA;
   }
   const bool gate = g.gate != nullptr;
-  auto kern = a_planar ? (gate ? (res ? gemm_split_kernel<true, true, true> : gemm_split_kernel<true, false, true>)
-                               : (res ? gemm_split_kernel<true, true, false> : gemm_split_kernel<true, false, false>))
-                       : (res ? gemm_split_kernel<false, true, false> : gemm_split_kernel<false, false, false>);
+  auto kern = a_planar ? (gate ? (res ? gemm_split_kernel<true, true, true, false> : gemm_split_kernel<true, false, true, false>)
+                               : (res ? gemm_split_kernel<true, true, false, false> : gemm_split_kernel<true, false, false, false>))
+                       : (res ? gemm_split_kernel<false, true, false, false> : gemm_split_kernel<false, false, false, false>);
+  if (wide)
+    kern = a_planar ? (gate ? gemm_split_kernel<true, false, true, true> : gemm_split_kernel<true, false, false, true>)
+                    : gemm_split_kernel<false, false, false, true>;
   e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   launch_k(kern, grid, GS_THREADS, smem, st, g, q, map);

@@ -4,9 +4,10 @@ around the 16 / 32 / 64 steps of the K loop and of the column tiles, resident an
 
 Tolerance: dropped partial products are below 2^-24 of |a||b|.  The accumulator is truncated (an error of
 half of 2^-23 of the running sum on average, always toward zero) at every MMA of 16 k: 6 * 4 times for
-K <= 64, K / 16 times for the leading products of larger K, at most 24 times either way.  The running sum
+K <= 64, K / 16 times for the leading products of K up to 384, at most 24 times either way.  The running sum
 averages about half of the final one, so the error is below 24 * 2^-24 * 0.5 + 2^-24 = 0.8e-6 of the
-result.  SiLU adds a few ulp."""
+result.  Larger K has several leading accumulators of at most 2 sqrt(K / 64) blocks of 64, four MMAs each; the
+parts are added with rounding to nearest.  SiLU adds a few ulp."""
 import ctypes as C
 
 import numpy as np
@@ -22,7 +23,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("B,T,H,W,Cc", [
     (1, 1, 3, 3, 4), (2, 3, 5, 7, 12), (1, 2, 11, 13, 16), (3, 2, 9, 14, 20), (1, 1, 16, 8, 32), (2, 2, 14, 14, 48),
     (1, 3, 10, 13, 64), (5, 4, 32, 32, 64), (1, 2, 12, 11, 68), (2, 1, 14, 14, 96), (1, 1, 7, 7, 128),
-    (3, 1, 14, 14, 256), (40, 2, 16, 16, 256), (2, 1, 7, 7, 384), (130, 1, 8, 8, 384)])
+    (3, 1, 14, 14, 256), (40, 2, 16, 16, 256), (2, 1, 7, 7, 384), (130, 1, 8, 8, 384),
+    (2, 1, 14, 14, 388), (1, 2, 9, 7, 448), (2, 1, 14, 14, 512), (1, 1, 14, 14, 772), (33, 1, 14, 14, 1024), (1, 1, 14, 14, 2048),
+    (1, 1, 5, 7, 6148)])
 def test_projections_against_float64(B, T, H, W, Cc):
     mod = GatedCSSM(channels=Cc, kernel_size=1, gate_type="factored")
     g = torch.Generator(device="cuda").manual_seed(B * 1000 + Cc)
@@ -36,8 +39,9 @@ def test_projections_against_float64(B, T, H, W, Cc):
     want = want.reshape(B * T, H, W, 2 * Cc).permute(0, 3, 1, 2)
     got = st["xz"].double()
     rel = lambda a, r: float((a - r).norm() / r.norm())
-    assert rel(got[:, :Cc], want[:, :Cc]) < 8e-7
-    assert rel(got[:, Cc:], torch.nn.functional.silu(want[:, Cc:])) < 1.2e-6
+    tol = 8e-7 if Cc <= 384 else (max(24, 4 * int(2 * (Cc / 64 + 1) ** 0.5)) * 0.5 + 1) * 2.0 ** -24
+    assert rel(got[:, :Cc], want[:, :Cc]) < tol
+    assert rel(got[:, Cc:], torch.nn.functional.silu(want[:, Cc:])) < 1.5 * tol
     # out_proj of these planes (planar in, channels-last out)
     d = b.desc(tuple(x.shape))
     lay = b.workspace_layout(d)
@@ -45,7 +49,7 @@ def test_projections_against_float64(B, T, H, W, Cc):
     check(b.L.cssm_gated_out_proj(C.byref(d), C.byref(b.w), b.buf.get("ws", lay.total).data_ptr() + lay.xz_planar,
                                   y.data_ptr(), torch.cuda.current_stream().cuda_stream), "out_proj")
     ref = got[:, :Cc].permute(0, 2, 3, 1) @ f64(p["out_proj"]["kernel"]) + f64(p["out_proj"]["bias"])
-    assert rel(y.double().reshape(ref.shape), ref) < 8e-7
+    assert rel(y.double().reshape(ref.shape), ref) < tol
     torch.cuda.synchronize()
     assert device_error() == 0
 
