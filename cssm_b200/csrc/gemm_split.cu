@@ -39,6 +39,7 @@
 #include <math.h>
 #include <string.h>
 #include "kernels.cuh"
+#include "bf16_ops.cuh"
 #include "gemm.cuh"
 #include "tc05.cuh"
 
@@ -73,6 +74,10 @@ struct SplitGeom {
   FastDiv hw, w, t, fdiv;             // divisions by HW, W, T and the source-frame divisor
 };
 
+// The arguments once more, for the path that takes their address: with the address of g and q themselves the
+// block 16 x 8 x 56 x 56 x 32 took 398 instead of 393 us.
+struct SplitArgs { GemmArgs g; SplitGeom q; };
+
 // x -> three bf16 parts for a pair of values, packed (low half = first value)
 __device__ __forceinline__ void split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p0) : "f"(y), "f"(x));
@@ -106,10 +111,61 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
 }
 
+// Columns [n, n + 32) of output row m once more, by float32 FMAs over k: for results that are not finite.  An
+// infinity, or a value above the largest bfloat16 (3.39e38), has no finite parts: the partial products give
+// inf - inf where the sum itself is infinite, or even finite.
+template <bool A_PLANAR>
+__device__ __noinline__ void split_row_fma(const SplitArgs& a, int m, int n, float rinv) {
+  const GemmArgs& g = a.g;
+  const SplitGeom& q = a.q;
+  const int fo = q.hw.div(m), px = m - fo * g.HW, tt = fo - q.t.div(fo) * g.T;
+  const int fr = (g.a_fmul != 0 || g.a_fadd != 0) ? q.fdiv.div(fo) * g.a_fmul + g.a_fadd : fo;
+#pragma unroll 1
+  for (const int end = min(n + 32, g.N); n < end; ++n) {
+    const float* w = g.Wk + n;
+    float v = 0.f;
+    if (A_PLANAR) {
+      const float* ap = g.A + ((size_t)fr * g.a_planes + g.a_plane0) * g.HW + px;
+      const float* gp = g.gate ? g.gate + ((size_t)(g.g_compact ? fo : fr) * g.g_planes + g.g_plane0) * g.HW + px : nullptr;
+      for (int k = 0; k < g.K; ++k) {
+        float x = ap[(size_t)k * g.HW];
+        if (g.rms_scale != nullptr) x *= rinv * g.rms_scale[k];
+        if (gp != nullptr) x *= gp[(size_t)k * g.HW];
+        v = fmaf(x, w[(size_t)k * g.N], v);
+      }
+    } else {
+      const float* ap = g.A + ((size_t)fr * g.HW + px) * g.K;
+      const int t = g.rope_tlast ? g.T - 1 : tt, h = q.w.div(px), wi = px - h * g.W, n2 = g.K >> 1;
+      for (int k = 0; k < g.K; k += 2) {
+        float x = ap[k], y = ap[k + 1];
+        if (g.rope_t != nullptr && (g.rope_nz == nullptr || g.rope_nz[k >> 1] != 0.f)) {
+          const float2 ct = g.rope_t[t * n2 + (k >> 1)], ch = g.rope_h[h * n2 + (k >> 1)], cw = g.rope_w[wi * n2 + (k >> 1)];
+          const float cx = ct.x * ch.x - ct.y * ch.y, sx = ct.x * ch.y + ct.y * ch.x;
+          const float c2 = cx * cw.x - sx * cw.y, s2 = cx * cw.y + sx * cw.x;
+          const float ne = x * c2 - y * s2;
+          y = x * s2 + y * c2;
+          x = ne;
+        }
+        v = fmaf(x, w[(size_t)k * g.N], v);
+        v = fmaf(y, w[(size_t)(k + 1) * g.N], v);
+      }
+    }
+    if (g.bias != nullptr) v += g.bias[n];
+    if (A_PLANAR) {
+      g.out[(size_t)m * g.N + n] = g.sub != nullptr ? v - g.sub[(size_t)m * g.N + n] : v;
+    } else {
+      if (n >= g.act_n0 && g.z_last_only && tt != g.T - 1) continue;
+      if (n >= g.act_n0 && g.out_act != 0) v = g.out_act == 1 ? silu_f(v) : sigmoid_f(v);
+      g.out[((size_t)fo * g.o_planes + g.o_plane0 + n) * g.HW + px] = v;
+    }
+  }
+}
+
 // GATE: planar A times the gate planes.  WIDE: more than one leading accumulator (nl > 1).
 template <bool A_PLANAR, bool RES, bool GATE, bool WIDE>
 __global__ void __launch_bounds__(GS_THREADS, 1)
-gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ CUtensorMap omap) {
+gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ CUtensorMap omap,
+                  const __grid_constant__ SplitArgs again) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // operand tiles need 1024-byte alignment (swizzle atoms); the launch adds 1024 bytes of slack
   unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -423,6 +479,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
         rinv = rsqrtf((sp[0] + sp[128]) / (float)g.K + 1e-6f);
       }
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)ac * acc_cols;
+      float odd = 0.f;                                  // NaN once a result of the row is not finite
 #pragma unroll 1
       for (int cc = half; cc * 32 < q.BN; cc += 2) {
         const int n = n0 + cc * 32;
@@ -454,6 +511,13 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
             for (int j = 0; j < 16; ++j) v[hf * 16 + j] += __uint_as_float(r[j]);
           }
         }
+        // (16 packed FMAs a thread and 32 columns: the same block 393 -> 395 us)
+        unsigned long long od[2] = {pk2(odd, 0.f), 0ull};
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) od[(j >> 1) & 1] = fma2(pk2(v[j], v[j + 1]), 0ull, od[(j >> 1) & 1]);
+        float o0, o1, o2, o3;
+        upk2(od[0], o0, o1); upk2(od[1], o2, o3);
+        odd = (o0 + o1) + (o2 + o3);
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
           const float4 b = *reinterpret_cast<const float4*>(bias_c + j);
@@ -518,6 +582,16 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
       tc::fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&accempty[ac]);
+      if (__any_sync(0xffffffffu, odd != odd)) {
+        if (A_PLANAR) {                                 // the TMA stores of this tile go first
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+          asm volatile("fence.proxy.async;" ::: "memory");
+          __syncwarp();
+        }
+        if (odd != odd && m < g.M)
+          for (int cc = half; cc * 32 < q.BN; cc += 2) split_row_fma<A_PLANAR>(again, m, n0 + cc * 32, rinv);
+        __syncwarp();
+      }
     }
     // shared memory must outlive the last TMA stores that read it
     if (A_PLANAR && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -622,7 +696,7 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
                     : gemm_split_kernel<false, false, false, true>;
   e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  launch_k(kern, grid, GS_THREADS, smem, st, g, q, map);
+  launch_k(kern, grid, GS_THREADS, smem, st, g, q, map, SplitArgs{g, q});
   return check_launch();
 }
 

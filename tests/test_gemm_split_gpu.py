@@ -74,3 +74,44 @@ def test_bias_at_a_four_byte_offset(Cc):
     torch.cuda.synchronize()
     assert torch.equal(got, want)
     assert device_error() == 0
+
+
+@pytest.mark.parametrize("Cc", [32, 48, 256, 512])
+def test_values_without_finite_parts(Cc):
+    """Infinities, NaN and finite values above the largest bfloat16 in a few pixels of either projection's
+    input: their rows are what float64 makes of them (rounded to float32), all other rows stay as they are."""
+    big = float(np.finfo(np.float32).max)
+    odd = {3: float("inf"), 40: -float("inf"), 41: big, 90: -big, 129: 3.395e38, 300: float("nan")}
+    mod = GatedCSSM(channels=Cc, kernel_size=1, gate_type="factored")
+    x = torch.randn((1, 2, 13, 15, Cc), device="cuda", generator=torch.Generator(device="cuda").manual_seed(Cc))
+    v = mod.init(5, tuple(x.shape), bias_scale=0.3)
+    b, p = mod.bind(v), v["params"]
+    f64 = lambda a: torch.from_numpy(np.asarray(a, np.float64)).cuda()
+    d = b.desc(tuple(x.shape))
+    lay = b.workspace_layout(d)
+
+    def same(got, want):
+        want32 = want.float()
+        assert torch.equal(got.isnan(), want32.isnan()) and torch.equal(got.isinf(), want32.isinf())
+        inf = want32.isinf()
+        assert torch.equal(got[inf], want32[inf])
+        rows = [r for r in range(got.shape[0]) if r not in odd]
+        assert float((got[rows].double() - want[rows]).norm() / want[rows].norm()) < 1.2e-6
+        for r in (41, 90, 129):
+            ok = want32[r].isfinite()
+            assert ok.any() and float((got[r][ok].double() / want[r][ok] - 1).abs().max()) < 1e-4
+
+    x.view(-1, Cc)[list(odd), Cc // 3] = torch.tensor(list(odd.values()), device="cuda")
+    xz = b.stages(x, upto="in_proj")["xz"]
+    same(xz[:, :Cc].permute(0, 2, 3, 1).reshape(-1, Cc),
+         x.double().view(-1, Cc) @ f64(p["in_proj"]["kernel"])[:, :Cc] + f64(p["in_proj"]["bias"])[:Cc])
+    planes = torch.randn((2, 2 * Cc, 13, 15), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    rows = planes[:, :Cc].permute(0, 2, 3, 1).reshape(-1, Cc)
+    rows[list(odd), Cc // 3] = torch.tensor(list(odd.values()), device="cuda")
+    planes[:, :Cc] = rows.view(2, 13, 15, Cc).permute(0, 3, 1, 2)
+    y = torch.empty_like(x)
+    check(b.L.cssm_gated_out_proj(C.byref(d), C.byref(b.w), planes.data_ptr(), y.data_ptr(),
+                                  torch.cuda.current_stream().cuda_stream), "out_proj")
+    same(y.view(-1, Cc), rows.double() @ f64(p["out_proj"]["kernel"]) + f64(p["out_proj"]["bias"]))
+    torch.cuda.synchronize()
+    assert device_error() == 0
