@@ -169,6 +169,8 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
     __syncwarp();
   } else if (warp == 1) {
     // ================================ MMA issuer ================================
+    // The limit of the waits below is for this kernel's own loads: they begin once the producer's wait is over.
+    pdl_wait();
     if (lane == 0) {
       const uint32_t idesc = make_idesc_bf16(GB_BM, BN);
       if (wres && !tc::mbar_wait(wfull, 0)) { atomicExch(&g_bf16_error, 6); bad = true; }
