@@ -414,7 +414,7 @@ int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weigh
     if (s != CSSM_OK) return s;
   } else {
     // long thin planes whose DFT tables do not fit beside them
-    const size_t smem = deltanet_smem_bytes(d->H, d->W);
+    const size_t smem = spread_smem(deltanet_smem_bytes(d->H, d->W), (long long)d->B * C);
     cudaError_t e = func_smem(deltanet_spectral_kernel, smem);
     if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
     launch_k(deltanet_spectral_kernel, d->B * C, GG_THREADS, smem, st, sp);

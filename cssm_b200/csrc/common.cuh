@@ -115,6 +115,19 @@ template <class F> inline cudaError_t func_smem(F* kern, size_t bytes) {
 }
 int sm_count();                           // of the current device
 
+// Shared memory to ask for where a kernel of `ctas` long CTAs (a recurrence over T) needs `smem`: in an overlapped
+// launch at least as much as keeps a CTA more than the even share off an SM.  Launched early such a kernel finds the
+// CTAs of the one before on most SMs and goes two or four at a time to the few with room, where it then stays for its whole run
+// while others are idle.  Block by block (packed, so): GDN 4 x 4 x 48 x 48 x 32 (32 CTAs) 1541, 942 us; gated 4 x 8 x
+// 60 x 60 x 32 226, 170; gated SimpleCSSM, 7 clips of 16 frames (112 CTAs) 216, 172.
+inline size_t spread_smem(size_t smem, long long ctas) {
+  constexpr size_t SM_BYTES = 228 * 1024, CTA_BYTES = 1024;         // of an SM; reserved by each CTA
+  const size_t share = (size_t)((ctas + sm_count() - 1) / sm_count());
+  if (g_pdl != 2 || share > 8) return smem;
+  const size_t least = SM_BYTES / (share + 1) - CTA_BYTES + 128;
+  return smem > least ? smem : least;
+}
+
 // Host-side record of the last CUDA error seen on this thread.
 void set_cuda_error(cudaError_t e);
 int check_launch();

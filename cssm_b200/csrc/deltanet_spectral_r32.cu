@@ -211,9 +211,10 @@ __global__ void __launch_bounds__(D32_THREADS, 2) deltanet_spectral_r32(const Dn
 
 int launch_deltanet_spectral_r32(const DnSpectralArgs& a, cudaStream_t st) {
   if (a.H != 32 || a.W != 32 || a.C % 4 != 0) return CSSM_ERR_UNSUPPORTED;
-  cudaError_t e = func_smem(deltanet_spectral_r32, D32_SMEM_BYTES);
+  const size_t smem = spread_smem(D32_SMEM_BYTES, (long long)a.B * (a.C / 4));
+  cudaError_t e = func_smem(deltanet_spectral_r32, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  launch_k(deltanet_spectral_r32, a.B * (a.C / 4), D32_THREADS, D32_SMEM_BYTES, st, a);
+  launch_k(deltanet_spectral_r32, a.B * (a.C / 4), D32_THREADS, smem, st, a);
   return check_launch();
 }
 

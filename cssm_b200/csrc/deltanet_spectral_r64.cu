@@ -155,9 +155,10 @@ __global__ void __launch_bounds__(R64_NT, 2) deltanet_spectral_r64(const DnSpect
 
 int launch_deltanet_spectral_r64(const DnSpectralArgs& a, cudaStream_t st) {
   if (a.H != 64 || a.W != 64) return CSSM_ERR_UNSUPPORTED;
-  cudaError_t e = func_smem(deltanet_spectral_r64, DN64_SMEM_BYTES);
+  const size_t smem = spread_smem(DN64_SMEM_BYTES, (long long)a.B * a.C);
+  cudaError_t e = func_smem(deltanet_spectral_r64, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  launch_k(deltanet_spectral_r64, a.B * a.C, R64_NT, DN64_SMEM_BYTES, st, a);
+  launch_k(deltanet_spectral_r64, a.B * a.C, R64_NT, smem, st, a);
   return check_launch();
 }
 

@@ -327,7 +327,7 @@ int launch_spectral(int B, int T, int H, int W, int C, const cf* khat, const flo
   const int grid = d.B * d.C;
   if (path == PATH_R32) return launch_gated_spectral_r32(xz, khat, gates, d.B, d.T, d.C, last_only, nogate, st, dchan);
   if (path == PATH_R64) {
-    const size_t smem = R64_SMEM_BYTES;
+    const size_t smem = spread_smem(R64_SMEM_BYTES, grid);
     // tensor map over the planar buffer as rows of 64 floats; box 68 x 64 (see the kernel)
     CUtensorMap pmap;
     memset(&pmap, 0, sizeof(pmap));
@@ -362,8 +362,8 @@ int launch_spectral(int B, int T, int H, int W, int C, const cf* khat, const flo
   } else if (gated_spectral_dft_fits(d.H, d.W, d.T)) {
     return launch_gated_spectral_dft(d.B, d.T, d.H, d.W, d.C, khat, gates, xz, last_only, nogate, st, dchan);
   } else {
-    const size_t smem = generic_smem_bytes(d.H, d.W);
-    if (smem > 200 * 1024) return CSSM_ERR_UNSUPPORTED;
+    if (generic_smem_bytes(d.H, d.W) > 200 * 1024) return CSSM_ERR_UNSUPPORTED;
+    const size_t smem = spread_smem(generic_smem_bytes(d.H, d.W), grid);
     cudaError_t e = func_smem(gated_spectral_generic, smem);
     if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
     launch_k(gated_spectral_generic, grid, GEN_THREADS, smem, st, xz, khat, reinterpret_cast<const float4*>(gates), d.T, d.C, d.H, d.W, last_only, nogate, dchan);

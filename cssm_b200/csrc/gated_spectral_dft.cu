@@ -164,10 +164,11 @@ int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat,
   a.ldx = dp_ld_rows(a.g, ch.P); a.ldc = dp_ld_cols(a.g, ch.P);
   auto kern = ch.threads == 256 ? (ch.wide ? gated_spectral_dft<2, 4, 256> : gated_spectral_dft<1, 2, 256>)
                                 : (ch.wide ? gated_spectral_dft<2, 4, 128> : gated_spectral_dft<1, 2, 128>);
-  cudaError_t e = func_smem(kern, ch.smem);
+  const int slots = 148 * ch.ctas, grid = a.groups < slots ? a.groups : slots;
+  const size_t smem = spread_smem(ch.smem, grid);
+  cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  const int slots = 148 * ch.ctas;
-  launch_k(kern, a.groups < slots ? a.groups : slots, ch.threads, ch.smem, st, a);
+  launch_k(kern, grid, ch.threads, smem, st, a);
   return check_launch();
 }
 

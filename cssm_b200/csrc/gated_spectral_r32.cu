@@ -170,9 +170,10 @@ int launch_gated_spectral_r32(float* xz, const cf* khat, const float* gates, int
   if (nogate == 1) kern = last_only ? gated_spectral_r32<true, 1> : gated_spectral_r32<false, 1>;
   if (nogate == 2) kern = last_only ? gated_spectral_r32<true, 2> : gated_spectral_r32<false, 2>;
   if (nogate == 3) kern = last_only ? gated_spectral_r32<true, 3> : gated_spectral_r32<false, 3>;
-  cudaError_t e = func_smem(kern, R32_SMEM_BYTES);
+  const size_t smem = spread_smem(R32_SMEM_BYTES, (long long)B * (C / 4));
+  cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  launch_k(kern, B * (C / 4), R32_THREADS, R32_SMEM_BYTES, st, xz, khat, reinterpret_cast<const float4*>(gates), T, C, dchan);
+  launch_k(kern, B * (C / 4), R32_THREADS, smem, st, xz, khat, reinterpret_cast<const float4*>(gates), T, C, dchan);
   return check_launch();
 }
 

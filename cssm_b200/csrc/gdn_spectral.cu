@@ -170,8 +170,8 @@ int launch_gdn_spectral(const GdnSpectralArgs& a, cudaStream_t st) {
   const int rc = launch_gdn_spectral_dft(a, st);
   if (rc != CSSM_ERR_UNSUPPORTED) return rc;
   // long thin planes whose DFT tables do not fit beside them
-  const size_t smem = gdn_generic_smem_bytes(a.H, a.W, a.dk);
-  if (smem > 220 * 1024) return CSSM_ERR_UNSUPPORTED;
+  if (gdn_generic_smem_bytes(a.H, a.W, a.dk) > 220 * 1024) return CSSM_ERR_UNSUPPORTED;
+  const size_t smem = spread_smem(gdn_generic_smem_bytes(a.H, a.W, a.dk), (long long)a.B * (a.C / a.dk));
   cudaError_t e = func_smem(gdn_spectral_generic, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   launch_k(gdn_spectral_generic, a.B * (a.C / a.dk), GG_THREADS, smem, st, a);
