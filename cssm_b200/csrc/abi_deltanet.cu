@@ -29,24 +29,44 @@ __device__ __forceinline__ void dn_write(const DnGateArgs& g, size_t oi, const f
   g.abkv[oi] = make_float4(0.1f + 0.89f * dn_sigmoid(r[0]), dn_sigmoid(r[1]), dn_sigmoid(r[2]), dn_sigmoid(r[3]));
   g.cg[oi] = dn_sigmoid(r[4]) * inv;
 }
-// factored: one frame per CTA row, its bins over gridDim.y CTAs
-__global__ void __launch_bounds__(256) deltanet_gates_factored_kernel(const DnGateArgs g) {
+// factored: one frame per CTA row, its bins over gridDim.y CTAs; 512 threads take the 5 (H + Wf) vector entries of
+// planes up to 64x64 in one pass.  (Entry and pointer by index: with gate_vectors' choice among ten pointers
+// the compiler issues the loads of a thread one after another, likewise with five dense gates in one call of
+// gate_dense.  28 frames of 64 x 64 x 64, factored, cold: 31 us that way, 12 so; 32 of 28 x 28 x 64, dense: 46 and 17 us.)
+constexpr int DF_THREADS = 512;
+__global__ void __launch_bounds__(DF_THREADS) deltanet_gates_factored_kernel(const DnGateArgs g) {
   extern __shared__ __align__(16) float sh[];
   const int Wf = g.W / 2 + 1, NB = g.H * Wf, per = g.H + Wf, fr = blockIdx.x;
   float* ctx = sh;                 // [C]
   float* vec = sh + g.C;           // 5 x (H + Wf)
-  float* scratch = vec + 5 * per;  // [256]
+  float* scratch = vec + 5 * per;  // [DF_THREADS]
   const float inv = 1.0f / (float)(g.H * g.W);
   pdl_sync();
   const GateCtxSrc src = {nullptr, g.ctx_part, g.tcode, g.T, g.C, g.H, 0, inv};
   gate_ctx(src, fr, 1, ctx, scratch);
-  int off[11];
-#pragma unroll
-  for (int q = 0; q <= 10; ++q) off[q] = (q >> 1) * per + ((q & 1) ? g.H : 0);
-  gate_vectors<10>(g.gk, g.gb, off, 10, ctx, g.C, vec, scratch);
+  auto entry = [&](int o, int sl, int S) {
+    const int gi = o / per, r = o - gi * per;
+    const bool isw = r >= g.H;
+    const int q = 2 * gi + (isw ? 1 : 0), col = isw ? r - g.H : r;
+    return gate_dot(ctx, g.gk[q] + col, isw ? Wf : g.H, sl * g.C / S, (sl + 1) * g.C / S) + (sl == 0 ? __ldg(g.gb[q] + col) : 0.f);
+  };
+  const int total = 5 * per, tid = threadIdx.x;
+  if (2 * total > DF_THREADS) {
+    for (int o = tid; o < total; o += DF_THREADS) vec[o] = entry(o, 0, 1);
+  } else {                         // the channels of an entry in slices
+    const int S = min(8, DF_THREADS / total), sl = tid / total;
+    if (sl < S) scratch[tid] = entry(tid - sl * total, sl, S);
+    __syncthreads();
+    if (tid < total) {
+      float v = scratch[tid];
+      for (int k = 1; k < S; ++k) v += scratch[k * total + tid];
+      vec[tid] = v;
+    }
+  }
+  __syncthreads();
   const int per_cta = (NB + gridDim.y - 1) / gridDim.y;
   const int bin_end = min(NB, (int)(blockIdx.y + 1) * per_cta);
-  for (int bin = blockIdx.y * per_cta + threadIdx.x; bin < bin_end; bin += 256) {
+  for (int bin = blockIdx.y * per_cta + threadIdx.x; bin < bin_end; bin += DF_THREADS) {
     const int kh = bin / Wf, kw = bin - kh * Wf;
     float r[5];
 #pragma unroll
@@ -65,13 +85,14 @@ __global__ void __launch_bounds__(128) deltanet_gates_dense_kernel(const DnGateA
   gate_ctx(src, f0, nf, sh, sh + G * g.C);
   const int bin = blockIdx.y * 128 + threadIdx.x;
   if (bin >= NB) return;
-  float r[5][G];
-  gate_dense<5, G>(g.gk, g.gb, NB, bin, g.C, sh, r);
+  float r[3][G], q[2][G];
+  gate_dense<3, G>(g.gk, g.gb, NB, bin, g.C, sh, r);
+  gate_dense<2, G>(g.gk + 3, g.gb + 3, NB, bin, g.C, sh, q);
   const int kh = bin / Wf, o = bin_index(g.path, kh, bin - kh * Wf, g.H, Wf);
 #pragma unroll
   for (int f = 0; f < G; ++f) {
     if (f >= nf) continue;
-    const float v[5] = {r[0][f], r[1][f], r[2][f], r[3][f], r[4][f]};
+    const float v[5] = {r[0][f], r[1][f], r[2][f], q[0][f], q[1][f]};
     dn_write(g, (size_t)(f0 + f) * NB + o, v, inv);
   }
 }
@@ -387,8 +408,8 @@ int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weigh
   } else {
     const int Wf = d->W / 2 + 1, NB = d->H * Wf;
     if (d->gate_type == CSSM_GATE_FACTORED) {
-      const size_t smem = (size_t)(C + 5 * (d->H + Wf) + 256) * sizeof(float);
-      s = launch_gates(deltanet_gates_factored_kernel, dim3(BT, gate_chunks(BT, NB)), 256, smem, st, ga);
+      const size_t smem = (size_t)(C + 5 * (d->H + Wf) + DF_THREADS) * sizeof(float);
+      s = launch_gates(deltanet_gates_factored_kernel, dim3(BT, gate_chunks(BT, NB)), DF_THREADS, smem, st, ga);
     } else {
       const int chunks = (NB + 127) / 128, G = gate_dense_frames(BT, chunks, C);
       const dim3 grid((BT + G - 1) / G, chunks);

@@ -51,6 +51,13 @@ def test_block_parity(case, gate_type, rope):
     assert _run(case, gate_type, rope) <= TOL
 
 
+@pytest.mark.parametrize("H,W,C", [(1, 1, 4), (2, 3, 4), (5, 8, 20), (26, 48, 8), (27, 48, 8), (51, 100, 4), (52, 100, 4)])
+def test_factored_gate_vectors(H, W, C):
+    """5 (H + W/2 + 1) vector entries around 256 and 512 (slices of the channels, fewer channels than slices, one
+    round of a CTA's threads, two).  float32 through two projections, transforms and two steps: 1e-5."""
+    assert _run((2, 2, H, W, C, 1), "factored", "none") <= 1e-5
+
+
 @pytest.mark.parametrize("scan_mode", ["ssd", "quadratic", "pallas"])
 def test_linear_scan_modes(scan_mode):
     assert _run((2, 6, 32, 32, 8, 5), "factored", "spatiotemporal", scan_mode=scan_mode) <= TOL
