@@ -9,7 +9,10 @@
 // Bound: the shared-memory pipe and the latency of the barriered passes.  With the state in shared memory
 // (70 KB per head) one CTA of nine warps fits an SM; the state of the running heads (20 MB) stays in L2
 // just as well: scratch goes by CTA, not by head, a bin's row is requested two bins ahead, the first step
-// reads none and the last one writes none.  128 x 32 x 32 x 32 x 64: 4.59 -> 3.85 ms.
+// reads none and the last one writes none.  128 x 32 x 32 x 32 x 64: 4.59 -> 3.85 ms.  Where every head has an SM of
+// its own (SMST) the state stays in shared memory, which is nearer: block 4 x 32 x 32 x 32 x 64 (64 heads) 743 us
+// from L2 (two CTAs on one SM at that), 536 so; 9 x 32 (144 heads) 905 and 695; 10 x 32 (160 heads) 933 from L2,
+// 1031 with one CTA per SM and its state in shared memory.
 #include "r32.cuh"
 #include "kernels.cuh"
 #include "gdn_common.cuh"
@@ -25,11 +28,14 @@ constexpr int G32_SPEC_CF = 8 * 8 * 17 * 4;            // [q planes 0-3, k plane
 constexpr int G32_COLS = 68 * 4;                        // lanes with a column
 constexpr int G32_SMEM_BYTES = (G32_EX_CF + G32_ZR_CF + G32_GB_CF + G32_SPEC_CF) * 8;
 static_assert(G32_SMEM_BYTES <= 112 * 1024, "two CTAs per SM");
+constexpr int G32_STATE_BYTES = 4 * 8 * G32_COLS * 8;   // [i][r][column lane]
+static_assert(G32_SMEM_BYTES + G32_STATE_BYTES <= 226 * 1024, "one CTA per SM");
 
 // LAST: only the last step's output planes are produced (compile-time switch).
 // STATIC: static-image fast path (one data frame per batch element, the T gate steps run per bin).
-template <bool LAST, bool STATIC>
-__global__ void __launch_bounds__(G32_THREADS, STATIC ? 1 : 2) gdn_spectral_r32(const GdnSpectralArgs a) {
+// SMST: state in shared memory, one CTA per SM.
+template <bool LAST, bool STATIC, bool SMST>
+__global__ void __launch_bounds__(G32_THREADS, STATIC || SMST ? 1 : 2) gdn_spectral_r32(const GdnSpectralArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cf* EX = reinterpret_cast<cf*>(smem_raw);
   cf* ZR = EX + G32_EX_CF;
@@ -59,8 +65,8 @@ __global__ void __launch_bounds__(G32_THREADS, STATIC ? 1 : 2) gdn_spectral_r32(
   const int kneg = (32 - kw) & 31;
   const int par = q & 1, ph = q >> 1;
 
-  // state scratch S[i][r][column lane]; a thread only ever touches its own slots
-  cf* S = a.state + (size_t)blockIdx.x * DK * DK * NB + tid;
+  // state S[i][r][column lane]; a thread only ever touches its own slots
+  cf* S = (SMST ? SPEC + G32_SPEC_CF : a.state + (size_t)blockIdx.x * DK * DK * NB) + tid;
   const float invHW = 1.0f / (float)HW;
 
   const int Tdata = STATIC ? 1 : a.T;          // frames of q, k, v per batch element
@@ -231,12 +237,15 @@ __global__ void __launch_bounds__(G32_THREADS, STATIC ? 1 : 2) gdn_spectral_r32(
 }
 
 int launch_gdn_spectral_r32(const GdnSpectralArgs& a, cudaStream_t st) {
-  auto kern = a.static_image ? gdn_spectral_r32<false, true>
-                             : (a.last_only ? gdn_spectral_r32<true, false> : gdn_spectral_r32<false, false>);
-  cudaError_t e = func_smem(kern, G32_SMEM_BYTES);
+  const int heads = a.B * (a.C / 4), sms = sm_count(), slots = (a.static_image ? 1 : 2) * sms;
+  const bool smst = heads <= sms && !a.static_image;
+  auto kern = a.static_image ? gdn_spectral_r32<false, true, false>
+              : smst ? (a.last_only ? gdn_spectral_r32<true, false, true> : gdn_spectral_r32<false, false, true>)
+                     : (a.last_only ? gdn_spectral_r32<true, false, false> : gdn_spectral_r32<false, false, false>);
+  const size_t smem = G32_SMEM_BYTES + (smst ? G32_STATE_BYTES : 0);
+  cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  const int heads = a.B * (a.C / 4), slots = (a.static_image ? 1 : 2) * sm_count();
-  launch_k(kern, heads < slots ? heads : slots, G32_THREADS, G32_SMEM_BYTES, st, a);
+  launch_k(kern, heads < slots ? heads : slots, G32_THREADS, smem, st, a);
   return check_launch();
 }
 
