@@ -62,7 +62,8 @@ __device__ __forceinline__ float rcp_fast(float d) {
 __device__ __forceinline__ float silu_f(float v) { return v * rcp_fast(1.0f + __expf(-v)); }
 __device__ __forceinline__ float sigmoid_f(float v) { return rcp_fast(1.0f + __expf(-v)); }
 
-// n / d for 0 <= n < 2^31 by one multiply-high: d's rounded-up reciprocal, 2^l >= d.
+// n / d for 0 <= n < 2^31 by one multiply-high with d's rounded-up reciprocal, 2^l >= d (division by invariant integers,
+// Granlund and Montgomery 1994).
 struct FastDiv {
   uint32_t mul, shift, one;
   FastDiv() = default;

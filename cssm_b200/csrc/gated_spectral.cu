@@ -331,18 +331,7 @@ int launch_spectral(int B, int T, int H, int W, int C, const cf* khat, const flo
     // tensor map over the planar buffer as rows of 64 floats; box 68 x 64 (see the kernel)
     CUtensorMap pmap;
     memset(&pmap, 0, sizeof(pmap));
-    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                 CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                 CUtensorMapFloatOOBfill);
-    static EncodeFn enc = []() -> EncodeFn {
-      void* p = nullptr;
-      cudaDriverEntryPointQueryResult q;
-      if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-          q != cudaDriverEntryPointSuccess)
-        return nullptr;
-      return reinterpret_cast<EncodeFn>(p);
-    }();
+    const tc::EncodeTiledFn enc = tc::encode_fn();
     const cuuint64_t dims[2] = {64, (cuuint64_t)d.B * d.T * 2 * d.C * 64};
     const cuuint64_t strides[1] = {256};
     const cuuint32_t box[2] = {68, 64}, es[2] = {1, 1};

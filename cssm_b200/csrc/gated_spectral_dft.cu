@@ -4,7 +4,7 @@
 // A CTA takes P consecutive channels of one batch element and walks t = 0 .. T-1 with their state in
 // shared memory; CTAs are persistent and loop over the channel groups, so the DFT tables are made once.
 // A thread always owns the same (column, row frequency pair) cells, so the state needs no barrier.
-// P is chosen by the launcher so that the register tiles of a pass fill the 256 threads.
+// P, the register tile and the number of threads (128 or 256) are chosen by the launcher (dp_choose).
 //
 // Bound: the packed FMAs of the four products and the shared-memory reads that feed them
 // (4 P Hp Wp (Hp + Wp) / 2 packed multiply-adds a step); below 20 x 20 pixels the loads and barriers.
@@ -109,12 +109,16 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
 // passes of a step (throughput of the SM, or the latency of a pass when its tiles do not fill the threads)
 // and a fixed part for the loads and barriers.  The constants were fitted to 19 shapes from 1 x 14 x 14 x 256
 // to 16 x 8 x 56 x 56 x 32 (some 40 choices each); the choice is within 5 % of the best of them everywhere.
-// The search is a few microseconds of host time, so each thread remembers its last few answers.
+// (Fitted on 148 SMs; another device's count takes the place of that number.)  The search is a few
+// microseconds of host time, so each thread remembers its last few answers: a pure function of the key.
 DpChoice dp_choose(int H, int W, int C, int B, int unit, size_t limit, size_t (*bytes)(const DpGeom&, int, int), int arg) {
-  struct Memo { int H, W, C, B, unit, arg; size_t (*bytes)(const DpGeom&, int, int); DpChoice c; };
+  struct Memo { int H, W, C, B, unit, arg, sms; size_t limit; size_t (*bytes)(const DpGeom&, int, int); DpChoice c; };
   static thread_local Memo memo[8] = {};
+  const int sms = sm_count();
   Memo& m = memo[(H * 31 + W * 17 + C + B * 7 + arg + unit) & 7];
-  if (m.bytes == bytes && m.H == H && m.W == W && m.C == C && m.B == B && m.unit == unit && m.arg == arg) return m.c;
+  if (m.bytes == bytes && m.H == H && m.W == W && m.C == C && m.B == B && m.unit == unit && m.arg == arg && m.sms == sms &&
+      m.limit == limit)
+    return m.c;
   const DpGeom g = dp_geom(H, W);
   DpChoice best;
   best.P = 0; best.cost = 1e30; best.wide = 0; best.ctas = 1; best.smem = 0;
@@ -134,13 +138,13 @@ DpChoice dp_choose(int H, int W, int C, int B, int unit, size_t limit, size_t (*
         const double thr = q * tiles * (n * per + 0.029 * RT * YT), ltn = ceil(tiles / nt) * (n * lat + epi);
         return thr > ltn ? thr : ltn;
       };
-      const double resident = groups < 148.0 * occ ? ceil(groups / 148) : occ;
+      const double resident = groups < (double)sms * occ ? ceil(groups / sms) : occ;
       const double step = 2 * pass(tr, g.Wp, resident) + 2 * pass(tc, g.Hp, resident) + 2930 + resident * P * H * W;
-      const double cost = ceil(groups / (148.0 * resident)) * step;
+      const double cost = ceil(groups / (sms * resident)) * step;
       if (cost < best.cost) { best.cost = cost; best.P = P; best.wide = wide; best.ctas = occ; best.threads = nt; best.smem = smem; }
     }
   }
-  m = Memo{H, W, C, B, unit, arg, bytes, best};
+  m = Memo{H, W, C, B, unit, arg, sms, limit, bytes, best};
   return best;
 }
 
@@ -164,7 +168,7 @@ int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat,
   a.ldx = dp_ld_rows(a.g, ch.P); a.ldc = dp_ld_cols(a.g, ch.P);
   auto kern = ch.threads == 256 ? (ch.wide ? gated_spectral_dft<2, 4, 256> : gated_spectral_dft<1, 2, 256>)
                                 : (ch.wide ? gated_spectral_dft<2, 4, 128> : gated_spectral_dft<1, 2, 128>);
-  const int slots = 148 * ch.ctas, grid = a.groups < slots ? a.groups : slots;
+  const int slots = sm_count() * ch.ctas, grid = a.groups < slots ? a.groups : slots;
   const size_t smem = spread_smem(ch.smem, grid);
   cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }

@@ -151,14 +151,15 @@ __device__ __forceinline__ void gate_dense(const float* const* gk, const float* 
 // frames, as long as the SMs stay covered and two CTAs fit an SM with their contexts.
 inline int gate_dense_frames(int BT, int chunks, int C) {
   for (int G : {8, 4})
-    if ((long long)(BT / G) * chunks >= 148 && (size_t)(G * C + 128) * sizeof(float) <= 100 * 1024) return G;
+    if ((long long)(BT / G) * chunks >= sm_count() && (size_t)(G * C + 128) * sizeof(float) <= 100 * 1024) return G;
   return 1;
 }
-// CTAs per frame of a factored-gate launch: enough to cover the SMs, at most one per 256 bins
+// CTAs per frame of a factored-gate launch: enough for two on every SM, at most one per 256 bins
 inline int gate_chunks(int BT, int NB) {
+  const int want = 2 * sm_count();
   int chunks = 1;
-  if (BT < 296) {
-    chunks = (296 + BT - 1) / BT;
+  if (BT < want) {
+    chunks = (want + BT - 1) / BT;
     const int maxc = (NB + 255) / 256;
     if (chunks > maxc) chunks = maxc;
   }

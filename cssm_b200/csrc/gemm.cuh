@@ -42,7 +42,6 @@ struct GemmArgs {
 bool gemm_tc_supported(const GemmArgs& g, bool a_planar);
 int launch_gemm_tc(const GemmArgs& g, bool a_planar, cudaStream_t st);
 int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st);
-int launch_gemm_any(const GemmArgs& g, bool a_planar, cudaStream_t st);
 int read_tc_error(int* out, int clear);
 int read_split_error(int* out, int clear);
 

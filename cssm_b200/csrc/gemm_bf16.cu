@@ -483,26 +483,10 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = []() -> EncodeTiledFn {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
 // K-major bf16 matrix [rows][kcols] (row stride ld elements) -> boxes of 64 k x box_rows rows
 static bool make_kmajor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t kcols,
                             uint64_t ld, uint32_t box_rows) {
-  EncodeTiledFn enc = encode_fn();
+  const tc::EncodeTiledFn enc = tc::encode_fn();
   if (!enc) return false;
   const cuuint64_t dims[2] = {kcols, rows};
   const cuuint64_t strides[1] = {ld * 2};
@@ -535,7 +519,7 @@ int gemm_bf16_pick_bn(int N) {
 
 // (rows x cols) bf16 output with row stride ld -> boxes of 64 columns x 128 rows for the TMA stores
 static bool make_out_map(CUtensorMap* map, void* base, uint64_t rows, uint64_t cols, uint64_t ld) {
-  EncodeTiledFn enc = encode_fn();
+  const tc::EncodeTiledFn enc = tc::encode_fn();
   if (!enc) return false;
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {ld * 2};
@@ -548,7 +532,7 @@ static bool make_out_map(CUtensorMap* map, void* base, uint64_t rows, uint64_t c
 // 4-D bf16 tensor (d0 innermost) with byte strides st[0..2] of dims 1..3, boxes and traversal strides
 static bool make_map_4d(CUtensorMap* map, const void* base, const uint64_t (&dims)[4], const uint64_t (&st)[3],
                         const uint32_t (&box)[4], const uint32_t (&es)[4]) {
-  EncodeTiledFn enc = encode_fn();
+  const tc::EncodeTiledFn enc = tc::encode_fn();
   if (!enc) return false;
   const cuuint64_t d[4] = {dims[0], dims[1], dims[2], dims[3]};
   const cuuint64_t s[3] = {st[0], st[1], st[2]};

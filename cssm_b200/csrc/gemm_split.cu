@@ -604,22 +604,6 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = []() -> EncodeTiledFn {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult qr;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qr) != cudaSuccess ||
-        qr != cudaDriverEntryPointSuccess)
-      return nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
 int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.HW <= 0) return CSSM_ERR_DIMS;
   if (g.K % 4 != 0 || g.N % 4 != 0) return CSSM_ERR_UNSUPPORTED;
@@ -679,7 +663,7 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
   if (a_planar) {
-    EncodeTiledFn enc = encode_fn();
+    const tc::EncodeTiledFn enc = tc::encode_fn();
     const cuuint64_t dims[2] = {(cuuint64_t)g.N, (cuuint64_t)g.M}, strides[1] = {(cuuint64_t)g.N * 4};
     const cuuint32_t box[2] = {32, 32}, es[2] = {1, 1};
     if (enc == nullptr ||

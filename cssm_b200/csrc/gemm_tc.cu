@@ -432,26 +432,9 @@ bool gemm_tc_supported(const GemmArgs& g, bool a_planar) {
   return true;
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = []() -> EncodeTiledFn {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
 // Tensor map of the GEMM output for the TMA-store epilogue: 16 KB boxes of 128 pixels x 32 columns.
 static bool make_out_map(const GemmArgs& g, bool a_planar, CUtensorMap* map) {
-  EncodeTiledFn enc = encode_fn();
+  const tc::EncodeTiledFn enc = tc::encode_fn();
   if (!enc) return false;
   const cuuint32_t es[3] = {1, 1, 1};
   CUresult r;

@@ -319,23 +319,9 @@ mlp_fused_kernel(const MlpFusedArgs g, const __grid_constant__ CUtensorMap amap,
   }
 }
 
-typedef CUresult (*MfEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static MfEncodeFn mf_encode_fn() {
-  static MfEncodeFn fn = []() -> MfEncodeFn {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return nullptr;
-    return reinterpret_cast<MfEncodeFn>(p);
-  }();
-  return fn;
-}
 // bf16 matrix [rows][cols] with row stride ld elements -> boxes of 64 columns x box_rows rows, 128-byte swizzle
 static bool mf_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
-  MfEncodeFn enc = mf_encode_fn();
+  const tc::EncodeTiledFn enc = tc::encode_fn();
   if (!enc) return false;
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {ld * 2};
