@@ -154,9 +154,10 @@ inline int gate_dense_frames(int BT, int chunks, int C) {
     if ((long long)(BT / G) * chunks >= sm_count() && (size_t)(G * C + 128) * sizeof(float) <= 100 * 1024) return G;
   return 1;
 }
-// CTAs per frame of a factored-gate launch: enough for two on every SM, at most one per 256 bins
+// CTAs per frame of a factored-gate launch (512 threads, and each makes all vectors of its frame): enough for every SM,
+// at most one per 256 bins
 inline int gate_chunks(int BT, int NB) {
-  const int want = 2 * sm_count();
+  const int want = sm_count();
   int chunks = 1;
   if (BT < want) {
     chunks = (want + BT - 1) / BT;
