@@ -409,7 +409,8 @@ int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weigh
     const int Wf = d->W / 2 + 1, NB = d->H * Wf;
     if (d->gate_type == CSSM_GATE_FACTORED) {
       const size_t smem = (size_t)(C + 5 * (d->H + Wf) + DF_THREADS) * sizeof(float);
-      s = launch_gates(deltanet_gates_factored_kernel, dim3(BT, gate_chunks(BT, NB)), DF_THREADS, smem, st, ga);
+      const int chunks = gate_chunks(BT, NB);
+      s = launch_gates(deltanet_gates_factored_kernel, dim3(BT, chunks), DF_THREADS, spread_smem(smem, (long long)BT * chunks), st, ga);
     } else {
       const int chunks = (NB + 127) / 128, G = gate_dense_frames(BT, chunks, C);
       const dim3 grid((BT + G - 1) / G, chunks);

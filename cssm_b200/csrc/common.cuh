@@ -85,7 +85,10 @@ struct FastDiv {
 // (pdl_trigger), so at most two kernels of a chain overlap and what a kernel does ahead of its wait
 // (barriers, TMEM, tables, weights) may rely on everything before the chain's first kernel.
 // It pays where launches are short (CSSM-SHViT, one image: 630 -> 487 us); with activations of 1 GB, launches of
-// 0.5 ms and more, passes got 3 % slower, so the block drivers turn it on up to PDL_MAX_BYTES a tensor.
+// 0.5 ms and more, passes got 3 % slower, so the block drivers turn it on up to PDL_MAX_BYTES a tensor.  The classifiers
+// keep it on at every size, for the mixer blocks in them too: it wins throughout (2 images 362 against 466 us without, 64
+// 821 / 941, 512 4054 / 4118, 768 5885 / 5925).  Exceptions within a scope: PdlOff, spread_smem.
+int sm_count();                           // of the current device
 extern thread_local int g_pdl;            // 0 off, 1 first launch of a scope pending, 2 on
 constexpr size_t PDL_MAX_BYTES = (size_t)256 << 20;
 struct PdlScope {
@@ -96,6 +99,23 @@ struct PdlScope {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_sync() { pdl_wait(); pdl_trigger(); }
+
+// A launch that waits for everything before it, also inside a scope, for persistent kernels of many rounds: in an overlapped
+// launch the CTAs take SMs in the order in which those come free, so neighbours in the grid, which work on neighbouring
+// tiles, sit far apart, and the CTAs that have a round more than others end up two on an SM (25 GDN clips of 12 frames,
+// 400 heads for 296 CTAs: the pass 809 us, 738 so).
+struct PdlOff {
+  int prev;
+  explicit PdlOff(bool off) : prev(g_pdl) { if (off && g_pdl == 2) g_pdl = 1; }
+  ~PdlOff() { if (prev == 2) g_pdl = 2; }
+};
+
+// Whether the CTAs that take one group more than others, `groups` dealt out to `occ` CTAs on every SM, would share SMs
+// with one another in an overlapped launch where they need not.
+inline bool uneven_rounds(long long groups, int occ) {
+  const long long sms = sm_count(), rest = groups % (sms * occ);
+  return groups > sms * occ && rest > 0 && (rest + sms - 1) / sms < occ;
+}
 
 template <class... P, class... A>
 inline void launch_k(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
@@ -114,8 +134,6 @@ cudaError_t func_smem_set(const void* kern, size_t bytes);
 template <class F> inline cudaError_t func_smem(F* kern, size_t bytes) {
   return func_smem_set(reinterpret_cast<const void*>(kern), bytes);
 }
-int sm_count();                           // of the current device
-
 // Shared memory to ask for where a kernel of `ctas` long CTAs (a recurrence over T) needs `smem`: in an overlapped
 // launch at least as much as keeps a CTA more than the even share off an SM.  Launched early such a kernel finds the
 // CTAs of the one before on most SMs and goes two or four at a time to the few with room, where it then stays for its whole run

@@ -296,6 +296,7 @@ static bool delta_dft_plan(int B, int T, int C, int H, int W, int dk, bool need_
 template <class Kern, class Args>
 static int delta_dft_launch(Kern kern, const Args& a, const DeltaDftArgs& d, const DpChoice& ch, cudaStream_t st) {
   const int slots = sm_count() * ch.ctas, grid = d.groups < slots ? d.groups : slots;
+  const PdlOff alone(uneven_rounds(d.groups, ch.ctas));
   const size_t smem = spread_smem(ch.smem, grid);
   cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }

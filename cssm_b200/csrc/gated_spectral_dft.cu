@@ -169,6 +169,7 @@ int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat,
   auto kern = ch.threads == 256 ? (ch.wide ? gated_spectral_dft<2, 4, 256> : gated_spectral_dft<1, 2, 256>)
                                 : (ch.wide ? gated_spectral_dft<2, 4, 128> : gated_spectral_dft<1, 2, 128>);
   const int slots = sm_count() * ch.ctas, grid = a.groups < slots ? a.groups : slots;
+  const PdlOff alone(uneven_rounds(a.groups, ch.ctas));
   const size_t smem = spread_smem(ch.smem, grid);
   cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }

@@ -245,6 +245,7 @@ int launch_gdn_spectral_r32(const GdnSpectralArgs& a, cudaStream_t st) {
   const size_t smem = G32_SMEM_BYTES + (smst ? G32_STATE_BYTES : 0);
   cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  const PdlOff alone(uneven_rounds(heads, a.static_image ? 1 : 2));
   launch_k(kern, heads < slots ? heads : slots, G32_THREADS, smem, st, a);
   return check_launch();
 }

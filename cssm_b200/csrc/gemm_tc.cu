@@ -465,6 +465,10 @@ static int launch_tc_v(const GemmArgs& g, const CUtensorMap& map, cudaStream_t s
   const size_t smem = TcSmem<N, STG>::TOTAL + 1024;      // slack for the 1024-byte alignment
   e = func_smem(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  // Planes of 64x64: the 64 planes of a tile lie 1 MB apart in all, which neighbouring SMs share (NoGate's output
+  // projection of 48 x 4 frames: 104 us in grid order, 139 with the CTAs where SMs came free); 8 x 4 frames and less, and
+  // smaller planes, gain more by the early start.  Channels-last input: the second projection of the same rows.
+  const PdlOff alone(N == 64 && num_tiles > 8 * sms && (!A_PLANAR || g.HW >= 4096));
   launch_k(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST>, grid, TC_THREADS, smem, st, g, num_tiles, map);
   return check_launch();
 }

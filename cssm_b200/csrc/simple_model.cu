@@ -730,7 +730,17 @@ static int run_readout(const cssm_simple_desc* d, const cssm_simple_weights* w, 
   a.B = d->B; a.H = H; a.W = W; a.C = d->embed_dim; a.pool_max = d->pool_type;
   a.norm_post_order = d->readout_norm; a.ncls = d->num_classes;
   a.bands = (H + RO_ROWS - 1) / RO_ROWS;
-  launch_k(readout_pool_kernel, dim3(a.bands, d->B), RO_THREADS, 0, st, a);
+  // Where a CTA reads 128 KB or more: no more than their even share of an SM, and none beside a CTA of the output projection
+  // (whose plane loads it would take the L1 while it waits).  8 x 4 frames of 64 x 64 x 64, the pass: 178 us packed, 169 so;
+  // for half of that, 4 clips of 32 x 32, an early start is worth more: 64 and 67 us.
+  size_t smem = 0;
+  if (g_pdl == 2 && (size_t)RO_ROWS * a.W * a.C * 4 >= 128 * 1024) {
+    smem = spread_smem(0, (long long)a.bands * d->B);
+    if (smem < 32 * 1024) smem = 32 * 1024;
+  }
+  const cudaError_t e = func_smem(readout_pool_kernel, smem);
+  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  launch_k(readout_pool_kernel, dim3(a.bands, d->B), RO_THREADS, smem, st, a);
   int s = check_launch();
   if (s != CSSM_OK) return s;
   launch_k(readout_head_kernel, d->B, SM_MAXC, 0, st, a);
