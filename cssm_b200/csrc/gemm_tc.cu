@@ -19,6 +19,7 @@
 #include "kernels.cuh"
 #include "gemm.cuh"
 #include "tc05.cuh"
+#include "stem.cuh"
 
 namespace cssm {
 
@@ -519,13 +520,16 @@ int cssm_device_error(int* out, int clear) {
   if (rc == CSSM_OK) rc = cssm::read_split_error(&a2, clear);
   if (rc != CSSM_OK) return rc;
   a |= a2;
+  rc = cssm::read_stem_error(&a2, clear);
+  if (rc != CSSM_OK) return rc;
+  a |= a2;
   rc = cssm::read_spec_error(&b, clear);
   if (rc != CSSM_OK) return rc;
   int c = 0, m = 0;
   rc = cssm::read_bf16_error(&c, clear);
   if (rc != CSSM_OK) return rc;
   rc = cssm::read_mlp_error(&m, clear);
-  // low byte: fp32 tensor-core GEMMs, next byte: fused spectral kernels, third: bf16 GEMM, fourth: fused MLP
+  // low byte: fp32 tensor-core GEMMs and stem, next byte: fused spectral kernels, third: bf16 GEMM, fourth: fused MLP
   *out = a | (b << 8) | (c << 16) | (m << 24);
   return rc;
 }

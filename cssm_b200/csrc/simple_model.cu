@@ -7,15 +7,12 @@
 #include <string.h>
 #include "kernels.cuh"
 #include "bf16_ops.cuh"
+#include "stem.cuh"
 
 namespace cssm {
 
 constexpr int SM_MAXC = 64;          // embed_dim limit (channel vectors live in registers)
 constexpr int STEM_THREADS = 256;
-
-__device__ __forceinline__ float softplus_f(float a) {
-  return fmaxf(a, 0.f) + __logf(1.0f + __expf(-fabsf(a)));
-}
 
 // LayerNorm over the C values of v (eps 1e-6, variance as E[d^2] - E[d]^2 of d = v - v[0]), in place.
 __device__ __forceinline__ void layer_norm_regs(float (&v)[SM_MAXC], int C, const float* __restrict__ scale,
@@ -35,14 +32,6 @@ __device__ __forceinline__ void layer_norm_regs(float (&v)[SM_MAXC], int C, cons
   for (int c = 0; c < SM_MAXC; ++c)
     if (c < C) v[c] = (v[c] - mean) * rinv * scale[c] + bias[c];
 }
-
-struct StemArgs {
-  const float* x; float* out;           // (N,Hin,Win,Cin) -> (N,Ho,Wo,C), channels-last
-  const float* wk; const float* bk;     // (KS,KS,Cin,C), (C)
-  const float* scale; const float* bias;
-  int N, Hin, Win, Cin, C, Ho, Wo;
-  int w_in_smem;                        // conv kernel staged in shared memory
-};
 
 // Four lanes share one pre-pool pixel: lane g of the quad owns the float4 channel groups
 // j = g + 4k (k = 0..3, j < C/4), i.e. channels 4j..4j+3.  LayerNorm sums cross the quad by two
@@ -305,107 +294,129 @@ __global__ void __launch_bounds__(STEMW_THREADS) stem_layer_wide_kernel(const St
   }
 }
 
-// Stem layer with many input channels and 64 output channels.  The quad form above reads four
-// weight vectors per sixteen multiply-adds, the same 64 bytes for every pixel of the warp, and is bound by
-// those shared-memory reads, the window form still reads 64 bytes a time.  Here a lane owns two
-// channels (a weight read is 256 distinct bytes) of the eight pixels of two neighbouring pool windows; their
-// 4 x 6 input pixels are staged by the warp and read as broadcasts, LayerNorm sums cross the warp.
-// One CTA of twelve warps per SM (weights 147 KB + 6 KB a warp at 64 input channels).
-// 8 images of 64x64x64: about 158 -> 55 us (the pass of a T = 1 SimpleCSSM 240 -> 138 us).
-constexpr int STEMP_WARPS = 12;
-__global__ void __launch_bounds__(STEMP_WARPS * 32) stem_layer_pair_kernel(const StemArgs a) {
-  extern __shared__ __align__(16) float sm[];
-  constexpr int C = SM_MAXC, NT = STEMP_WARPS * 32;
-  const int Cin = a.Cin, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c4 = Cin >> 2;
-  const int nw = 9 * Cin * C;
-  float* vec = sm + nw;                                       // bias, scale, lnbias
-  float4* patch = reinterpret_cast<float4*>(vec + 3 * C) + warp * 24 * c4;      // [4 rows][6 columns][Cin]
-  for (int i = tid; i < nw / 4; i += NT) reinterpret_cast<float4*>(sm)[i] = __ldg(reinterpret_cast<const float4*>(a.wk) + i);
-  for (int i = tid; i < C; i += NT) { vec[i] = a.bk[i]; vec[C + i] = a.scale[i]; vec[2 * C + i] = a.bias[i]; }
+// Stem layer of few input channels (images: 1, frames: 3), C = 16 * NG output channels.  Four lanes share four conv pixels, the
+// 2x2 window of a pooled layer or four neighbours in memory; lane g of the quad owns the float4 channel groups g + 4k of
+// all four.  A weight is read once for the four pixels and multiplied by packed FMAs (with one pixel a lane, the kernel
+// before, each weight vector was read for four multiply-adds and every value crossed the window by two shuffles); LayerNorm
+// sums cross the quad by two shuffles a pixel, and the window maximum stays in the lane.
+// Bound: the two special-function calls of softplus and about a dozen packed or scalar operations a conv output.
+// 128 images of 128x128: 265 -> 157 us; 128 clips of 32 frames of 32x32x3, pointwise: 301 -> 219 us (write floor 165).
+constexpr int STEMQ_THREADS = 256;
+template <int KS, int POOL, int CIN, int NG>
+__global__ void __launch_bounds__(STEMQ_THREADS, 2) stem_quad_kernel(const StemArgs a) {
+  constexpr int C = 16 * NG, NW = KS * KS * CIN * C, PS = POOL == 2 ? KS + 1 : 4, LO = (KS - 1) / 2;
+  constexpr int NX = POOL == 2 ? PS * PS : 4;                // input pixels of the four conv pixels
+  __shared__ __align__(16) float sm[NW + 3 * C];
+  float* vec = sm + NW;
+  const int tid = threadIdx.x, lane = tid & 31, g = lane & 3;
+  for (int i = tid; i < NW; i += STEMQ_THREADS) sm[i] = a.wk[i];
+  for (int i = tid; i < C; i += STEMQ_THREADS) { vec[i] = a.bk[i]; vec[C + i] = a.scale[i]; vec[2 * C + i] = a.bias[i]; }
   __syncthreads();
   pdl_sync();
-  const unsigned long long* w2 = reinterpret_cast<const unsigned long long*>(sm) + lane;      // [tap][ci][32 pairs]
-  const float2 bk = *reinterpret_cast<const float2*>(vec + 2 * lane);
-  const float2 sc = *reinterpret_cast<const float2*>(vec + C + 2 * lane), lb = *reinterpret_cast<const float2*>(vec + 2 * C + 2 * lane);
-  const int pairs = (a.Wo + 1) >> 1;
-  const long long total = (long long)a.N * a.Ho * pairs;
-  for (long long task = (long long)blockIdx.x * STEMP_WARPS + warp; task < total; task += (long long)gridDim.x * STEMP_WARPS) {
-    const int wo = 2 * (int)(task % pairs), ho = (int)((task / pairs) % a.Ho), n = (int)(task / ((long long)pairs * a.Ho));
-    const int h0 = 2 * ho, w0 = 2 * wo;
-    __syncwarp();                                             // the patch of the task before has been read
-    for (int i = lane; i < 24 * c4; i += 32) {
-      const int px = i / c4, k = i - px * c4, r = px / 6, hh = h0 - 1 + r, ww = w0 - 1 + px - 6 * r;
-      patch[i] = (hh >= 0 && hh < a.Hin && ww >= 0 && ww < a.Win)
-                     ? __ldg(reinterpret_cast<const float4*>(a.x + (((size_t)n * a.Hin + hh) * a.Win + ww) * Cin) + k)
-                     : make_float4(0.f, 0.f, 0.f, 0.f);
+  const unsigned total = (unsigned)a.N * a.Ho * a.Wo, units = POOL == 2 ? total : (total + 3) / 4;
+  const float4* w4 = reinterpret_cast<const float4*>(sm);
+  const float4* v4 = reinterpret_cast<const float4*>(vec);
+  for (unsigned u0 = (blockIdx.x * (STEMQ_THREADS / 32) + (tid >> 5)) * 8; u0 < units; u0 += gridDim.x * STEMQ_THREADS / 4) {
+    const unsigned u = u0 + (lane >> 2);
+    const bool valid = u < units;
+    const unsigned uc = valid ? u : 0;
+    int h0 = 0, w0 = 0;
+    float x[NX][CIN];
+    if (POOL == 2) {
+      const unsigned row = uc / (unsigned)a.Wo, n = row / (unsigned)a.Ho;
+      w0 = 2 * (int)(uc - row * a.Wo); h0 = 2 * (int)(row - n * a.Ho);
+      const float* xn = a.x + (size_t)n * a.Hin * a.Win * CIN;
+#pragma unroll
+      for (int i = 0; i < NX; ++i) {
+        const int hh = h0 - LO + i / PS, ww = w0 - LO + i % PS;
+        const bool ok = hh >= 0 && hh < a.Hin && ww >= 0 && ww < a.Win;
+        const float* xp = xn + ((size_t)(ok ? hh : 0) * a.Win + (ok ? ww : 0)) * CIN;
+#pragma unroll
+        for (int ci = 0; ci < CIN; ++ci) x[i][ci] = ok ? __ldg(xp + ci) : 0.f;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const size_t px = (size_t)uc * 4 + i;
+        const bool ok = px < total;
+#pragma unroll
+        for (int ci = 0; ci < CIN; ++ci) x[i][ci] = ok ? __ldg(a.x + px * CIN + ci) : 0.f;
+      }
     }
-    __syncwarp();
-    unsigned long long acc[2][4];
+    unsigned long long acc[4][2 * NG];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i >> 2][i & 3] = pk2(bk.x, bk.y);
-#pragma unroll 1
-    for (int k = 0; k < c4; ++k) {
+    for (int k = 0; k < NG; ++k) {
+      const float4 b = v4[g + 4 * k];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        float x[6][4];
+      for (int p = 0; p < 4; ++p) { acc[p][2 * k] = pk2(b.x, b.y); acc[p][2 * k + 1] = pk2(b.z, b.w); }
+    }
 #pragma unroll
-        for (int j = 0; j < 6; ++j) {
-          const float4 v = patch[(r * 6 + j) * c4 + k];
-          x[j][0] = v.x; x[j][1] = v.y; x[j][2] = v.z; x[j][3] = v.w;
-        }
+    for (int tap = 0; tap < KS * KS; ++tap)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          unsigned long long xx[6];
+      for (int ci = 0; ci < CIN; ++ci)
 #pragma unroll
-          for (int j = 0; j < 6; ++j) xx[j] = pk2(x[j][e], x[j][e]);
+        for (int k = 0; k < NG; ++k) {
+          const float4 w = w4[(tap * CIN + ci) * (C / 4) + g + 4 * k];
+          const unsigned long long wa = pk2(w.x, w.y), wb = pk2(w.z, w.w);
 #pragma unroll
-          for (int y = 0; y < 2; ++y) {
-            const int dy = r - y;                             // tap row that takes input row r to output row y
-            if (dy < 0 || dy > 2) continue;
-#pragma unroll
-            for (int dx = 0; dx < 3; ++dx) {
-              const unsigned long long w = w2[((dy * 3 + dx) * Cin + 4 * k + e) * 32];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) acc[y][j] = fma2(w, xx[j + dx], acc[y][j]);
-            }
+          for (int p = 0; p < 4; ++p) {
+            const float xv = POOL == 2 ? x[((p >> 1) + tap / KS) * PS + (p & 1) + tap % KS][ci] : x[p][ci];
+            const unsigned long long xx = pk2(xv, xv);
+            acc[p][2 * k] = fma2(xx, wa, acc[p][2 * k]);
+            acc[p][2 * k + 1] = fma2(xx, wb, acc[p][2 * k + 1]);
           }
         }
+    // softplus, LayerNorm over the quad's channels (moments of the values minus the pixel's first channel: layer_norm_regs)
+    float mx[NG][4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      float v[NG][4], s = 0.f, ss = 0.f;
+#pragma unroll
+      for (int k = 0; k < NG; ++k) {
+        upk2(acc[p][2 * k], v[k][0], v[k][1]);
+        upk2(acc[p][2 * k + 1], v[k][2], v[k][3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[k][e] = softplus_f(v[k][e]);
+      }
+      const float vref = __shfl_sync(0xffffffffu, v[0][0], lane & ~3);
+#pragma unroll
+      for (int k = 0; k < NG; ++k)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { v[k][e] -= vref; s += v[k][e]; ss = fmaf(v[k][e], v[k][e], ss); }
+      s += __shfl_xor_sync(0xffffffffu, s, 1);  ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);  ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+      const float mean = s / (float)C, rinv = rsqrtf(fmaxf(ss / (float)C - mean * mean, 0.f) + 1e-6f);
+      const bool inb = POOL == 1 || (h0 + (p >> 1) < a.Hin && w0 + (p & 1) < a.Win);      // else 'SAME' pool padding on odd sizes
+#pragma unroll
+      for (int k = 0; k < NG; ++k) {
+        const float4 sc = v4[C / 4 + g + 4 * k], lb = v4[C / 2 + g + 4 * k];
+        const float4 y = make_float4((v[k][0] - mean) * rinv * sc.x + lb.x, (v[k][1] - mean) * rinv * sc.y + lb.y,
+                                     (v[k][2] - mean) * rinv * sc.z + lb.z, (v[k][3] - mean) * rinv * sc.w + lb.w);
+        if (POOL == 1) {
+          const size_t px = (size_t)uc * 4 + p;
+          if (valid && px < total) *reinterpret_cast<float4*>(a.out + px * C + 4 * (g + 4 * k)) = y;
+        } else {
+          // fmaxf ignores a NaN: a window keeps its other pixels
+          mx[k][0] = fmaxf(p == 0 ? -INFINITY : mx[k][0], inb ? y.x : -INFINITY);
+          mx[k][1] = fmaxf(p == 0 ? -INFINITY : mx[k][1], inb ? y.y : -INFINITY);
+          mx[k][2] = fmaxf(p == 0 ? -INFINITY : mx[k][2], inb ? y.z : -INFINITY);
+          mx[k][3] = fmaxf(p == 0 ? -INFINITY : mx[k][3], inb ? y.w : -INFINITY);
+        }
       }
     }
-    // softplus, LayerNorm (moments of the values minus the pixel's first channel), 2x2 max
-    float2 mx[2] = {make_float2(-INFINITY, -INFINITY), make_float2(-INFINITY, -INFINITY)};
+    if (POOL == 2 && valid) {
+      float4* op = reinterpret_cast<float4*>(a.out + (size_t)uc * C);
 #pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float v0, v1;
-        upk2(acc[y][j], v0, v1);
-        v0 = softplus_f(v0); v1 = softplus_f(v1);
-        const float vref = __shfl_sync(0xffffffffu, v0, 0);
-        v0 -= vref; v1 -= vref;
-        float s = v0 + v1, ss = fmaf(v0, v0, v1 * v1);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          s += __shfl_xor_sync(0xffffffffu, s, off); ss += __shfl_xor_sync(0xffffffffu, ss, off);
-        }
-        const float mean = s / (float)C, rinv = rsqrtf(fmaxf(ss / (float)C - mean * mean, 0.f) + 1e-6f);
-        if (h0 + y < a.Hin && w0 + j < a.Win) {               // 'SAME' pool padding on odd sizes
-          mx[j >> 1].x = fmaxf(mx[j >> 1].x, (v0 - mean) * rinv * sc.x + lb.x);
-          mx[j >> 1].y = fmaxf(mx[j >> 1].y, (v1 - mean) * rinv * sc.y + lb.y);
-        }
-      }
-    float* o = a.out + (((size_t)n * a.Ho + ho) * a.Wo + wo) * C + 2 * lane;
-    *reinterpret_cast<float2*>(o) = mx[0];
-    if (wo + 1 < a.Wo) *reinterpret_cast<float2*>(o + C) = mx[1];
+      for (int k = 0; k < NG; ++k) op[g + 4 * k] = make_float4(mx[k][0], mx[k][1], mx[k][2], mx[k][3]);
+    }
   }
 }
 
-static int launch_stem_layer_pair(const StemArgs& a, size_t smem, cudaStream_t st) {
-  cudaError_t e = func_smem(stem_layer_pair_kernel, smem);
-  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  const long long need = ((long long)a.N * a.Ho * ((a.Wo + 1) / 2) + STEMP_WARPS - 1) / STEMP_WARPS;
-  const int sms = sm_count();
-  launch_k(stem_layer_pair_kernel, (unsigned)(need < sms ? need : sms), STEMP_WARPS * 32, smem, st, a);
+template <int KS, int POOL, int CIN, int NG>
+static int launch_stem_quad(const StemArgs& a, cudaStream_t st) {
+  const long long total = (long long)a.N * a.Ho * a.Wo, units = POOL == 2 ? total : (total + 3) / 4;
+  const long long need = (units + STEMQ_THREADS / 4 - 1) / (STEMQ_THREADS / 4), cap = 2LL * sm_count() * 8;
+  launch_k(stem_quad_kernel<KS, POOL, CIN, NG>, (unsigned)(need < cap ? need : cap), STEMQ_THREADS, 0, st, a);
   return check_launch();
 }
 
@@ -441,12 +452,10 @@ static int launch_stem_layer_v(StemArgs a, cudaStream_t st) {
 template <int KS, int POOL, int CIN>
 static int launch_stem_layer_cin(const StemArgs& a, cudaStream_t st) {
   const size_t wbytes = (size_t)KS * KS * a.Cin * a.C * sizeof(float);
-  // 64 output channels: two channels a lane, at every batch (both layers of 128x128 images, against the kernels
-  // below: batch 8 101 against 204 us, 19 196 / 468, 32 314 / 492, 128 1147 / 1718)
-  const size_t pair_smem = wbytes + (3 * (size_t)a.C + STEMP_WARPS * 24 * (size_t)a.Cin) * sizeof(float);
-  if (CIN == 0 && KS == 3 && POOL == 2 && a.C == SM_MAXC && a.Cin % 4 == 0 && wbytes > 64 * 1024 && pair_smem <= 227 * 1024 &&
-      ((reinterpret_cast<uintptr_t>(a.wk) | reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.out)) & 15u) == 0)
-    return launch_stem_layer_pair(a, pair_smem, st);
+  // 1 or 3 input channels to 32 or 64: four conv pixels a quad
+  if constexpr (CIN > 0)
+    if ((a.C == 32 || a.C == 64) && (long long)a.N * a.Ho * a.Wo < (1LL << 31))
+      return a.C == 64 ? launch_stem_quad<KS, POOL, CIN, 4>(a, st) : launch_stem_quad<KS, POOL, CIN, 2>(a, st);
   // many input channels, pooled: the weight-reusing kernel (needs the weights in shared memory
   // and float4 input reads)
   // it needs one full wave of windows to pay
@@ -458,8 +467,8 @@ static int launch_stem_layer_cin(const StemArgs& a, cudaStream_t st) {
   if (CIN == 0 && wbytes > 64 * 1024)
     return a.C == SM_MAXC ? launch_stem_layer_v<KS, POOL, 0, true, 1024>(a, st)
                           : launch_stem_layer_v<KS, POOL, 0, false, 1024>(a, st);
-  return a.C == SM_MAXC ? launch_stem_layer_v<KS, POOL, CIN, true, STEM_THREADS>(a, st)
-                        : launch_stem_layer_v<KS, POOL, CIN, false, STEM_THREADS>(a, st);
+  if (CIN == 0 && a.C == SM_MAXC) return launch_stem_layer_v<KS, POOL, 0, true, STEM_THREADS>(a, st);
+  return launch_stem_layer_v<KS, POOL, CIN, false, STEM_THREADS>(a, st);
 }
 
 template <int KS, int POOL>
@@ -661,7 +670,12 @@ __global__ void __launch_bounds__(256) repeat_frames_kernel(const float4* __rest
   for (int t = 0; t < T; ++t) o[t * frame4] = v;
 }
 
-struct SimpleWs { size_t feat, tmp, y, partial, rep, block, total; };
+// Split weights of a stem layer on the tensor cores (csrc/stem_tc.cu); one layer's at a time
+static size_t stem_split_bytes(const cssm_simple_desc& d) {
+  return d.stem_mode == 0 && d.stem_layers > 1 && (d.embed_dim == 32 || d.embed_dim == 64) ? round_up(stem_tc_scratch_bytes(d.embed_dim), 256) : 0;
+}
+
+struct SimpleWs { size_t feat, tmp, split, y, partial, rep, block, total; };
 static SimpleWs simple_ws_layout(const cssm_simple_desc& d, const void* bd) {
   SimpleWs l;
   const SimpleDims o = stem_out_dims(d);
@@ -674,6 +688,7 @@ static SimpleWs simple_ws_layout(const cssm_simple_desc& d, const void* bd) {
   if (d.stem_mode == 0 && d.stem_layers > 1)
     tmp = N * ((d.Hin + 1) / 2) * ((d.Win + 1) / 2) * C * sizeof(float);
   l.tmp = off; off += 2 * round_up(tmp, 256);
+  l.split = off; off += stem_split_bytes(d);
   l.y = off; off += round_up((size_t)d.B * d.T * o.H * o.W * C * sizeof(float), 256);
   l.partial = off; off += round_up((size_t)d.B * ((o.H + RO_ROWS - 1) / RO_ROWS) * C * sizeof(float), 256);
   // blocks 2..4 take clips only: an image batch's features are repeated over T for them
@@ -686,7 +701,7 @@ static SimpleWs simple_ws_layout(const cssm_simple_desc& d, const void* bd) {
 }
 
 static int run_stem(const cssm_simple_desc* d, const cssm_simple_weights* w, const float* x,
-                    float* feat, float* tmp0, float* tmp1, cudaStream_t st) {
+                    float* feat, float* tmp0, float* tmp1, void* split, cudaStream_t st) {
   StemArgs a;
   memset(&a, 0, sizeof(a));
   a.N = d->image_input ? d->B : d->B * d->T;
@@ -707,7 +722,13 @@ static int run_stem(const cssm_simple_desc* d, const cssm_simple_weights* w, con
     a.x = src; a.out = dst; a.wk = w->conv_kernel[i]; a.bk = w->conv_bias[i];
     a.scale = w->norm_scale[i]; a.bias = w->norm_bias[i];
     a.Hin = H; a.Win = W; a.Cin = Cin; a.Ho = (H + 1) / 2; a.Wo = (W + 1) / 2;
-    const int s = launch_stem_layer<3, 2>(a, st);
+    int s = CSSM_OK;
+    if (split != nullptr && stem_tc_supported(a)) {
+      s = launch_stem_split_weights(a.wk, split, a.C, st);
+      if (s == CSSM_OK) s = launch_stem_layer_tc(a, split, st);
+    } else {
+      s = launch_stem_layer<3, 2>(a, st);
+    }
     if (s != CSSM_OK) return s;
     src = dst; H = a.Ho; W = a.Wo; Cin = d->embed_dim;
   }
@@ -769,6 +790,7 @@ int cssm_simple_stem(const cssm_simple_desc* d, const cssm_simple_weights* w, co
   if (!aligned16(x) || !aligned16(feat)) return CSSM_ERR_ALIGN;
   float* t0 = nullptr;
   float* t1 = nullptr;
+  void* split = nullptr;
   if (d->stem_mode == 0 && d->stem_layers > 1) {
     const SimpleDims o = stem_out_dims(*d);
     const size_t tmp = round_up((size_t)o.N * ((d->Hin + 1) / 2) * ((d->Win + 1) / 2) * d->embed_dim * sizeof(float), 256);
@@ -776,8 +798,10 @@ int cssm_simple_stem(const cssm_simple_desc* d, const cssm_simple_weights* w, co
     if (!aligned16(workspace)) return CSSM_ERR_ALIGN;
     if (workspace_bytes < 2 * tmp) return CSSM_ERR_WORKSPACE;
     t0 = (float*)workspace; t1 = (float*)((char*)workspace + tmp);
+    const size_t sb = stem_split_bytes(*d);
+    if (sb > 0 && workspace_bytes >= 2 * tmp + sb) split = (char*)workspace + 2 * tmp;
   }
-  return run_stem(d, w, x, feat, t0, t1, (cudaStream_t)stream);
+  return run_stem(d, w, x, feat, t0, t1, split, (cudaStream_t)stream);
 }
 
 int cssm_simple_readout(const cssm_simple_desc* d, const cssm_simple_weights* w, int32_t H,
@@ -808,8 +832,8 @@ int cssm_simple_forward(const cssm_simple_desc* d, const cssm_simple_weights* w,
   PdlScope pdl((size_t)d->B * d->T * o.H * o.W * d->embed_dim * 4 <= PDL_MAX_BYTES);
   float* feat = (float*)(ws + l.feat);
   float* y = (float*)(ws + l.y);
-  const size_t tmp_half = (l.y - l.tmp) / 2;
-  s = run_stem(d, w, x, feat, (float*)(ws + l.tmp), (float*)(ws + l.tmp + tmp_half), st);
+  const size_t tmp_half = (l.split - l.tmp) / 2;
+  s = run_stem(d, w, x, feat, (float*)(ws + l.tmp), (float*)(ws + l.tmp + tmp_half), l.y > l.split ? ws + l.split : nullptr, st);
   if (s != CSSM_OK) return s;
   // the scalar-scan blocks have no last-frame-only entry point: they produce all T frames
   const int last_only = ((flags & CSSM_SIMPLE_LAST_FRAME_ONLY) && d->block < 2) ? 1 : 0;

@@ -261,7 +261,8 @@ class BoundSimple:
             feat = out
         frames = d.B if d.image_input else d.B * d.T
         half = frames * ((d.Hin + 1) // 2) * ((d.Win + 1) // 2) * d.embed_dim * 4
-        ws = self.buf.get("stem", 2 * ((half + 255) // 256 * 256))
+        split = 9 * d.embed_dim * d.embed_dim * 6 if d.embed_dim in (32, 64) else 0      # weights of the tensor-core layers
+        ws = self.buf.get("stem", 2 * ((half + 255) // 256 * 256) + split)
         check(self.L.cssm_simple_stem(C.byref(d), C.byref(self.w), x.data_ptr(), feat.data_ptr(),
                                       ws.data_ptr(), ws.numel(), _stream_ptr(self.device)),
               "cssm_simple_stem")

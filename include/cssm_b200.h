@@ -433,7 +433,9 @@ typedef struct cssm_simple_weights {
 size_t cssm_simple_workspace_bytes(const cssm_simple_desc* d, const void* block_desc);
 
 /* Stem alone: x frames -> features.  Image input: feat is (B,H,W,C) (the frame that the block
- * then reads for every t); clip input: (B,T,H,W,C).  Replaces simple_cssm.py:244-281. */
+ * then reads for every t); clip input: (B,T,H,W,C).  Replaces simple_cssm.py:244-281.
+ * workspace (several layers only): two buffers of frames * ceil(Hin/2) * ceil(Win/2) * embed_dim floats, each rounded up to
+ * 256 bytes; with 54 * embed_dim^2 bytes more, embed_dim 32 or 64, the later layers run on the tensor cores. */
 int cssm_simple_stem(const cssm_simple_desc* d, const cssm_simple_weights* w, const float* x,
                      float* feat, void* workspace, size_t workspace_bytes, void* stream);
 
