@@ -246,39 +246,71 @@ __global__ void __launch_bounds__(DW_THREADS, (K <= 5 ? 2 : 1)) rope_dwconv_cl_k
 }
 
 // ------------------------------------------- context row sums without a conv (K = 1) ----
-// ctx_part[(frame, h, c)] = sum over w of the rotated input.  One warp per image row: a lane
-// owns channel pairs lane, lane + 32, ... and walks the row, so every load is a coalesced
-// C*4-byte line and no cross-lane reduction is needed.  The t and h parts of the angle are
-// combined once per row, the w part comes from the table per element.
-constexpr int CTX_WARPS = 8;
+// ctx_part[(frame, h, c)] = sum over w of the rotated input.  One warp per image row of a source frame: a lane owns one
+// or more float4 channel groups, 32 / (C / 4) pixels side by side where C < 128, and walks the row eight 16-byte loads at a time.
+// Rotations commute, so the loop turns by the w part of the angle alone; the h and t parts turn the finished sums,
+// for every frame t of the clip where one source frame stands for all.
+// Bound: HBM (with 8-byte loads, four in flight, and the whole angle per element the kernel before ran at a quarter of its
+// rate): 128 x 32 frames of 32x32x64 316 -> 192 us (floor 165), 12 x 8 of 64x64x64 57 -> 27.
+constexpr int CTX_WARPS = 4;
 __global__ void __launch_bounds__(CTX_WARPS * 32) rope_ctx_rowsum_kernel(const GdnDwArgs a) {
   pdl_sync();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long row = (long long)blockIdx.x * CTX_WARPS + warp;        // (frame, h)
-  if (row >= (long long)a.BT * a.H) return;
+  const int copies = a.x_bcast ? a.T : 1, frames = a.BT / copies;
+  const long long row = (long long)blockIdx.x * CTX_WARPS + warp;        // (source frame, h)
+  if (row >= (long long)frames * a.H) return;
   const int fr = (int)(row / a.H), h = (int)(row % a.H);
-  const int t = fr % a.T, n2 = a.C / 2;
-  const int fsrc = a.x_bcast ? fr / a.T : fr;
-  const float* xr = a.x + ((size_t)fsrc * a.H + h) * a.W * a.C;
-  for (int pi = lane; pi < n2; pi += 32) {
-    float cth = 1.f, sth = 0.f;
-    if (a.rope_t != nullptr) {
-      const float2 ct = a.rope_t[t * n2 + pi], ch = a.rope_h[h * n2 + pi];
-      cth = ct.x * ch.x - ct.y * ch.y; sth = ct.x * ch.y + ct.y * ch.x;
-    }
-    float se = 0.f, so = 0.f;
-#pragma unroll 4
-    for (int w = 0; w < a.W; ++w) {
-      const float2 v = __ldg(reinterpret_cast<const float2*>(xr + (size_t)w * a.C + 2 * pi));
-      if (a.rope_t != nullptr) {
-        const float2 cw = __ldg(&a.rope_w[w * n2 + pi]);
-        const float c2 = cth * cw.x - sth * cw.y, s2 = cth * cw.y + sth * cw.x;
-        se += v.x * c2 - v.y * s2; so += v.x * s2 + v.y * c2;
-      } else {
-        se += v.x; so += v.y;
+  const int n2 = a.C / 2, c4 = a.C / 4, wide = c4 < 32 ? 32 / c4 : 1, sub = c4 < 32 ? lane / c4 : 0;
+  const bool rope = a.rope_t != nullptr;
+  const float4* xr = reinterpret_cast<const float4*>(a.x + (size_t)row * a.W * a.C);
+  for (int j0 = 0; j0 < c4; j0 += 32) {
+    const int j = j0 + (c4 < 32 ? lane - sub * c4 : lane);
+    const bool on = j < c4 && sub < wide;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (on) {
+      const float4* rw = reinterpret_cast<const float4*>(a.rope_w) + j;
+#pragma unroll 1
+      for (int w0 = sub; w0 < a.W; w0 += 8 * wide) {
+        float4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int w = w0 + u * wide;
+          v[u] = w < a.W ? __ldg(xr + (size_t)w * c4 + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int w = w0 + u * wide;
+          if (rope) {
+            const float4 c = __ldg(rw + (size_t)min(w, a.W - 1) * c4);
+            s.x = fmaf(v[u].x, c.x, fmaf(-v[u].y, c.y, s.x)); s.y = fmaf(v[u].x, c.y, fmaf(v[u].y, c.x, s.y));
+            s.z = fmaf(v[u].z, c.z, fmaf(-v[u].w, c.w, s.z)); s.w = fmaf(v[u].z, c.w, fmaf(v[u].w, c.z, s.w));
+          } else {
+            s.x += v[u].x; s.y += v[u].y; s.z += v[u].z; s.w += v[u].w;
+          }
+        }
       }
     }
-    *reinterpret_cast<float2*>(a.ctx_part + (size_t)row * a.C + 2 * pi) = make_float2(se, so);
+    for (int k = 1; k < wide; ++k) {                  // sums of the other pixels side by side
+      const int from = (lane + k * c4) & 31;
+      const float4 o = make_float4(__shfl_sync(0xffffffffu, s.x, from), __shfl_sync(0xffffffffu, s.y, from),
+                                   __shfl_sync(0xffffffffu, s.z, from), __shfl_sync(0xffffffffu, s.w, from));
+      if (sub == 0) { s.x += o.x; s.y += o.y; s.z += o.z; s.w += o.w; }
+    }
+    if (on && sub == 0) {
+      if (rope) {
+        const float4 c = __ldg(reinterpret_cast<const float4*>(a.rope_h + (size_t)h * n2) + j);
+        s = make_float4(s.x * c.x - s.y * c.y, s.x * c.y + s.y * c.x, s.z * c.z - s.w * c.w, s.z * c.w + s.w * c.z);
+      }
+      for (int k = 0; k < copies; ++k) {
+        float4 o = s;
+        if (rope) {
+          const int t = a.x_bcast ? k : fr % a.T;
+          const float4 c = __ldg(reinterpret_cast<const float4*>(a.rope_t + (size_t)t * n2) + j);
+          o = make_float4(s.x * c.x - s.y * c.y, s.x * c.y + s.y * c.x, s.z * c.z - s.w * c.w, s.z * c.w + s.w * c.z);
+        }
+        *reinterpret_cast<float4*>(a.ctx_part + (((size_t)fr * copies + k) * a.H + h) * a.C + 4 * j) = o;
+      }
+    }
   }
 }
 
@@ -305,7 +337,7 @@ int launch_rope_dwconv_cl(const GdnDwArgs& a, cudaStream_t st) {
   if (a.C % 4 != 0) return CSSM_ERR_UNSUPPORTED;
   if (a.ksz <= 1 && a.out == nullptr) {
     if (a.ctx_part == nullptr) return CSSM_OK;
-    const long long rows = (long long)a.BT * a.H;
+    const long long rows = (long long)(a.x_bcast ? a.BT / a.T : a.BT) * a.H;
     launch_k(rope_ctx_rowsum_kernel, (unsigned)((rows + CTX_WARPS - 1) / CTX_WARPS), CTX_WARPS * 32, 0, st, a);
     return check_launch();
   }
