@@ -115,21 +115,39 @@ static inline void trace(int kind, double bytes, cudaStream_t st) {
   ++t->count;
 }
 
+// whole: times M, the rows of the whole batch that these are a chunk of (Bf16GemmArgs::whole)
 static int gemm_plain(const __nv_bfloat16* A, int M, int K, const __nv_bfloat16* Wt, int N, const float* bias,
-                      int act, const __nv_bfloat16* res, __nv_bfloat16* out, cudaStream_t st) {
+                      int act, const __nv_bfloat16* res, __nv_bfloat16* out, cudaStream_t st, int whole = 1) {
   Bf16GemmArgs g;
   memset(&g, 0, sizeof(g));
-  g.A = A; g.M = M; g.N = N; g.K = K; g.lda = K;
+  g.A = A; g.M = M; g.N = N; g.K = K; g.lda = K; g.whole = whole;
   g.Wt = Wt; g.ldw = packed_ld(K); g.bias = bias; g.act = act;
   g.res = res; g.ldr = N; g.out = out; g.ldo = N;
   trace(CSSM_SHVIT_K_GEMM, 2.0 * ((double)M * K + (double)M * N * (res ? 2 : 1) + (double)N * K), st);
   return launch_gemm_bf16(g, st);
 }
 
+// The same with LayerNorm over K of the rows of A in the GEMM, where the few-row kernel takes it; else through T.
+static int layernorm_gemm(const __nv_bfloat16* A, const float* scale, const float* shift, __nv_bfloat16* T, int M, int K,
+                          const __nv_bfloat16* Wt, int N, const float* bias, int act, __nv_bfloat16* out, cudaStream_t st, int whole) {
+  if (gemm_small_ln_supported(M, N, K, whole, scale, shift)) {
+    Bf16GemmArgs g;
+    memset(&g, 0, sizeof(g));
+    g.A = A; g.M = M; g.N = N; g.K = K; g.lda = K;
+    g.Wt = Wt; g.ldw = packed_ld(K); g.bias = bias; g.act = act; g.out = out; g.ldo = N;
+    trace(CSSM_SHVIT_K_GEMM, 2.0 * ((double)M * K + (double)M * N + (double)N * K), st);
+    return launch_gemm_small(g, scale, shift, st);
+  }
+  trace(CSSM_SHVIT_K_LAYERNORM, 4.0 * M * K, st);
+  const int s = launch_layernorm_cl(A, scale, shift, T, M, K, st);
+  return s != CSSM_OK ? s : gemm_plain(T, M, K, Wt, N, bias, act, nullptr, out, st, whole);
+}
+
 static int conv_s2(const __nv_bfloat16* x, int B, int Hi, int Wi, int Cin, const __nv_bfloat16* Wt, int Cout,
-                   const float* bias, int act, __nv_bfloat16* out, cudaStream_t st) {
+                   const float* bias, int act, __nv_bfloat16* out, cudaStream_t st, int whole = 1) {
   Bf16GemmArgs g;
   memset(&g, 0, sizeof(g));
+  g.whole = whole;
   const int Ho = (Hi + 1) / 2, Wo = (Wi + 1) / 2;
   const int th = (Ho - 1) * 2 + 3 - Hi, tw = (Wo - 1) * 2 + 3 - Wi;
   g.A = x; g.M = B * Ho * Wo; g.N = Cout; g.K = 9 * Cin;
@@ -186,7 +204,7 @@ static int block_plan_init(const cssm_shvit_block_desc& d, const cssm_shvit_bloc
 }
 
 static int block_forward(const cssm_shvit_block_desc& d, const cssm_shvit_block_weights& w, const char* plan,
-                         const __nv_bfloat16* x, __nv_bfloat16* y, char* ws, cudaStream_t st) {
+                         const __nv_bfloat16* x, __nv_bfloat16* y, char* ws, cudaStream_t st, int whole = 1) {
   const BlockPlan p = block_plan_layout(d);
   const BlockWs l = block_ws_layout(d);
   const int M = d.B * d.H * d.W, C = d.C, Hd = d.hidden;
@@ -201,7 +219,7 @@ static int block_forward(const cssm_shvit_block_desc& d, const cssm_shvit_block_
     CSSM_RUN(launch_layernorm_cl(x, w.norm1_scale, w.norm1_bias, T, M, C, st));
     trace(CSSM_SHVIT_K_DWCONV7, 4.0 * M * C, st);
     CSSM_RUN(launch_dwconv_cl(T, w.dw_kernel, w.dw_bias, nullptr, nullptr, HB, nullptr, d.B, d.H, d.W, C, 7, 0, 1, st));
-    CSSM_RUN(gemm_plain(HB, M, C, (const __nv_bfloat16*)(plan + p.pw), C, w.pw_bias, 0, x, X1, st));
+    CSSM_RUN(gemm_plain(HB, M, C, (const __nv_bfloat16*)(plan + p.pw), C, w.pw_bias, 0, x, X1, st, whole));
   } else {
     float* na = (float*)(ws + l.na);
     float* nb = (float*)(ws + l.nb);
@@ -213,7 +231,7 @@ static int block_forward(const cssm_shvit_block_desc& d, const cssm_shvit_block_
       CSSM_RUN(launch_dwconv_cl(x, d.use_pos_conv ? w.dw_kernel : nullptr, w.dw_bias, na, nb, T, nullptr, d.B,
                                 d.H, d.W, C, 3, 1, 0, st));
       const float* inb = (const float*)(plan + p.inp_bias);
-      CSSM_RUN(gemm_plain(T, M, C, (const __nv_bfloat16*)(plan + p.inp), 2 * C, inb, 2, nullptr, HB, st));
+      CSSM_RUN(gemm_plain(T, M, C, (const __nv_bfloat16*)(plan + p.inp), 2 * C, inb, 2, nullptr, HB, st, whole));
       float* ctx = (float*)(ws + l.ctx);
       trace(CSSM_SHVIT_K_PLANE_SUM, 2.0 * M * C, st);
       CSSM_RUN(launch_plane_sum_cl(HB, 2 * C, d.B, d.H * d.W, C, ctx, st));
@@ -227,7 +245,7 @@ static int block_forward(const cssm_shvit_block_desc& d, const cssm_shvit_block_
       CSSM_RUN(launch_gated_gates(ga, st));
       trace(CSSM_SHVIT_K_SPECTRAL, 6.0 * M * C, st);          // x_main, z in; y out (bf16)
       CSSM_RUN(launch_gated_spectral_cl(HB, 2 * C, d.B, d.H, d.W, C, (const float*)(ws + l.maps), T, C, st));
-      CSSM_RUN(gemm_plain(T, M, C, (const __nv_bfloat16*)(plan + p.outp), C, w.cssm.out_proj_bias, 0, x, X1, st));
+      CSSM_RUN(gemm_plain(T, M, C, (const __nv_bfloat16*)(plan + p.outp), C, w.cssm.out_proj_bias, 0, x, X1, st, whole));
     } else {
       float* x32 = (float*)(ws + l.x32);
       float* y32 = (float*)(ws + l.y32);
@@ -242,14 +260,14 @@ static int block_forward(const cssm_shvit_block_desc& d, const cssm_shvit_block_
     }
   }
   // LN -> fc1 -> gelu -> [h + dw3x3(h)] -> fc2 + residual
-  trace(CSSM_SHVIT_K_LAYERNORM, 4.0 * M * C, st);
-  CSSM_RUN(launch_layernorm_cl(X1, w.norm2_scale, w.norm2_bias, T, M, C, st));
   if (!(d.is_cssm && d.use_dwconv) && mlp_fused_supported(C, Hd)) {
+    trace(CSSM_SHVIT_K_LAYERNORM, 4.0 * M * C, st);
+    CSSM_RUN(launch_layernorm_cl(X1, w.norm2_scale, w.norm2_bias, T, M, C, st));
     // fc1 + GELU + fc2 + residual in one kernel: the hidden tensor stays on chip
     trace(CSSM_SHVIT_K_MLP, 2.0 * (3.0 * M * C + 2.0 * C * Hd), st);
     return launch_mlp_fused(T, M, fc1, packed_ld(C), w.fc1_bias, fc2, packed_ld(Hd), w.fc2_bias, X1, y, st);
   }
-  CSSM_RUN(gemm_plain(T, M, C, fc1, Hd, w.fc1_bias, 1, nullptr, HB, st));
+  CSSM_RUN(layernorm_gemm(X1, w.norm2_scale, w.norm2_bias, T, M, C, fc1, Hd, w.fc1_bias, 1, HB, st, whole));
   const __nv_bfloat16* h = HB;
   if (d.is_cssm && d.use_dwconv) {
     __nv_bfloat16* H2 = (__nv_bfloat16*)(ws + l.hid2);
@@ -258,7 +276,7 @@ static int block_forward(const cssm_shvit_block_desc& d, const cssm_shvit_block_
                               3, 1, 0, st));
     h = H2;
   }
-  return gemm_plain(h, M, Hd, fc2, C, w.fc2_bias, 0, X1, y, st);
+  return gemm_plain(h, M, Hd, fc2, C, w.fc2_bias, 0, X1, y, st, whole);
 }
 
 // ---------------------------------------------------------------------------- model ----
@@ -357,7 +375,7 @@ static ModelWalk model_walk(const cssm_shvit_desc& d) {
 }
 
 static int model_forward(const cssm_shvit_desc& d, const cssm_shvit_weights& w, const char* plan,
-                         const __nv_bfloat16* x, float* logits, char* ws, cudaStream_t st) {
+                         const __nv_bfloat16* x, float* logits, char* ws, cudaStream_t st, int whole) {
   const ModelWalk m = model_walk(d);
   __nv_bfloat16* A = (__nv_bfloat16*)(ws + m.ws.a);
   __nv_bfloat16* B = (__nv_bfloat16*)(ws + m.ws.b);
@@ -368,7 +386,7 @@ static int model_forward(const cssm_shvit_desc& d, const cssm_shvit_weights& w, 
   CSSM_RUN(launch_stem_conv1(x, (const float*)(plan + m.plan.c1w), (const float*)(plan + m.plan.c1b), A, d.B, d.H,
                              d.W, d.Cin, E0 / 2, 1, st));
   CSSM_RUN(conv_s2(A, d.B, H1, W1, E0 / 2, (const __nv_bfloat16*)(plan + m.plan.c2w), E0,
-                   (const float*)(plan + m.plan.c2b), 0, B, st));
+                   (const float*)(plan + m.plan.c2b), 0, B, st, whole));
   __nv_bfloat16* cur = B;
   __nv_bfloat16* other = A;
   int bi = 0;
@@ -376,11 +394,11 @@ static int model_forward(const cssm_shvit_desc& d, const cssm_shvit_weights& w, 
     if (s > 0) {
       CSSM_RUN(conv_s2(cur, d.B, m.Hs[s - 1], m.Ws[s - 1], d.embed_dims[s - 1],
                        (const __nv_bfloat16*)(plan + m.plan.dsw[s - 1]), d.embed_dims[s],
-                       (const float*)(plan + m.plan.dsb[s - 1]), 0, other, st));
+                       (const float*)(plan + m.plan.dsb[s - 1]), 0, other, st, whole));
       __nv_bfloat16* t = cur; cur = other; other = t;
     }
     for (int b = 0; b < d.depths[s]; ++b, ++bi) {
-      CSSM_RUN(block_forward(m.bd[bi], w.blocks[bi], plan + m.plan.blocks[bi], cur, other, ws + m.ws.blk, st));
+      CSSM_RUN(block_forward(m.bd[bi], w.blocks[bi], plan + m.plan.blocks[bi], cur, other, ws + m.ws.blk, st, whole));
       __nv_bfloat16* t = cur; cur = other; other = t;
     }
   }
@@ -394,6 +412,21 @@ static int model_forward(const cssm_shvit_desc& d, const cssm_shvit_weights& w, 
   CSSM_RUN(launch_head(pooled, w.head_kernel, w.head_bias, logits, d.B, C3, d.num_classes, st));
   trace(CSSM_SHVIT_K_END, 0.0, st);
   return CSSM_OK;
+}
+
+// whole: d->B is one of `whole` chunks of a batch
+static int checked_forward(const cssm_shvit_desc* d, const cssm_shvit_weights* w, const void* plan, const void* x_bf16,
+                           float* logits, void* workspace, size_t workspace_bytes, void* stream, int whole) {
+  PdlScope pdl(true);
+  int s = model_validate(d);
+  if (s != CSSM_OK) return s;
+  if (!w || !plan || !x_bf16 || !logits || !workspace) return CSSM_ERR_NULL;
+  if (!aligned16(plan) || !aligned16(x_bf16) || !aligned16(logits) || !aligned16(workspace)) return CSSM_ERR_ALIGN;
+  const ModelWalk m = model_walk(*d);
+  if (m.status != CSSM_OK) return m.status;
+  if (workspace_bytes < m.ws.total) return CSSM_ERR_WORKSPACE;
+  return model_forward(*d, *w, (const char*)plan, (const __nv_bfloat16*)x_bf16, logits, (char*)workspace,
+                       (cudaStream_t)stream, whole);
 }
 
 }  // namespace cssm
@@ -479,16 +512,7 @@ int cssm_shvit_plan_init(const cssm_shvit_desc* d, const cssm_shvit_weights* w, 
 }
 int cssm_shvit_forward(const cssm_shvit_desc* d, const cssm_shvit_weights* w, const void* plan, const void* x_bf16,
                        float* logits, void* workspace, size_t workspace_bytes, void* stream) {
-  PdlScope pdl(true);
-  int s = model_validate(d);
-  if (s != CSSM_OK) return s;
-  if (!w || !plan || !x_bf16 || !logits || !workspace) return CSSM_ERR_NULL;
-  if (!aligned16(plan) || !aligned16(x_bf16) || !aligned16(logits) || !aligned16(workspace)) return CSSM_ERR_ALIGN;
-  const ModelWalk m = model_walk(*d);
-  if (m.status != CSSM_OK) return m.status;
-  if (workspace_bytes < m.ws.total) return CSSM_ERR_WORKSPACE;
-  return model_forward(*d, *w, (const char*)plan, (const __nv_bfloat16*)x_bf16, logits, (char*)workspace,
-                       (cudaStream_t)stream);
+  return checked_forward(d, w, plan, x_bf16, logits, workspace, workspace_bytes, stream, 1);
 }
 
 int cssm_shvit_forward_timed(const cssm_shvit_desc* d, const cssm_shvit_weights* w, const void* plan,
@@ -566,8 +590,8 @@ int cssm_shvit_forward_host(const cssm_shvit_desc* d, const cssm_shvit_weights* 
     CSSM_TRY(cudaEventRecord(ev_in[j], sc));
     CSSM_TRY(cudaStreamWaitEvent(st, ev_in[j], 0));
     if (rc == CSSM_OK)
-      rc = cssm_shvit_forward(&c, w, plan, ws + h.xbuf[j], ld + (size_t)k * h.chunk_b * d->num_classes,
-                              ws + h.model, h.model_bytes, stream);
+      rc = checked_forward(&c, w, plan, ws + h.xbuf[j], ld + (size_t)k * h.chunk_b * d->num_classes,
+                           ws + h.model, h.model_bytes, stream, nchunk);
     CSSM_TRY(cudaEventRecord(ev_comp[j], st));
   }
   CSSM_TRY(cudaMemcpyAsync(logits_host, ld, (size_t)d->B * d->num_classes * 4, cudaMemcpyDeviceToHost, st));

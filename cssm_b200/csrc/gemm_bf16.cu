@@ -573,6 +573,7 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
   } else if (g.K % 8 != 0 || g.lda % 8 != 0 || g.lda < g.K) {
     return CSSM_ERR_UNSUPPORTED;
   }
+  if (gemm_small_supported(g)) return launch_gemm_small(g, nullptr, nullptr, st);
   CUtensorMap amap, bmap, omap, rmap;
   memset(&amap, 0, sizeof(amap));
   memset(&bmap, 0, sizeof(bmap));

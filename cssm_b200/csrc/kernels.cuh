@@ -133,6 +133,8 @@ struct Bf16GemmArgs {
   int ldo;
   int Kpad, BN, stages;      // filled in by the launcher
   int nacc, ostg;            // TMEM accumulators; staging slots per epilogue half (launcher)
+  int whole;                 // the rows are one of `whole` chunks of a batch: few-row rules go by M * whole, so that
+                             // a chunked call takes the kernels, and gives the sums, of the whole one (0 as 1)
   int wres;                  // 1: the weights stay resident in shared memory (launcher)
   // conv mode through TMA (filled in by the launcher): an M tile is a patch of Bbox images x Hbox
   // output rows x Wbox output columns (at most 128 pixels); K block kb is `kb_ch` channels from
@@ -149,6 +151,10 @@ int conv3x3s2_weight_layout(int Cin, int Wi, int Cout);
 int conv3x3s2_packed_k(int Cin, int Wi, int Cout);
 int gemm_bf16_pick_bn(int N);
 int read_bf16_error(int* out, int clear);
+// few rows (csrc/gemm_small.cu); ln_scale, ln_bias: LayerNorm over K of the rows of A, or nullptr
+bool gemm_small_supported(const Bf16GemmArgs& g);
+bool gemm_small_ln_supported(int M, int N, int K, int whole, const float* scale, const float* bias);
+int launch_gemm_small(const Bf16GemmArgs& g, const float* ln_scale, const float* ln_bias, cudaStream_t st);
 
 // fused fc1 + GELU + fc2 + residual of the 64-channel ConvBlock (csrc/mlp_fused.cu)
 bool mlp_fused_supported(int C, int Hd);
