@@ -500,7 +500,6 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
                     const float* __restrict__ bias, const float* __restrict__ pre_a,
                     const float* __restrict__ pre_b, __nv_bfloat16* __restrict__ y, int H, int W, int C,
                     int add_centre, int gelu) {
-  pdl_sync();
   constexpr int CS = 64, P = (KS - 1) / 2, TW = CG * NC, PW = TW + KS - 1, PH = TH + KS - 1, NT = 32 * CG;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_raw);        // [PH][PW][CS]
@@ -510,6 +509,17 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
   const int tr = bid % (tiles_w * tiles_h), n = bid / (tiles_w * tiles_h);
   const int h0 = (tr / tiles_w) * TH, w0 = (tr % tiles_w) * TW, cs0 = sl * CS;
   const int cp = threadIdx.x & 31, cgp = threadIdx.x >> 5;                 // channel pair, column group
+  // (the weights do not depend on the kernel before)
+  unsigned long long wr[KS * KS];
+#pragma unroll
+  for (int t = 0; t < KS * KS; ++t) {
+    const float2 w2 = wk ? __ldg(reinterpret_cast<const float2*>(wk + (size_t)t * C + cs0) + cp) : make_float2(0.f, 0.f);
+    wr[t] = pk2(w2.x + ((add_centre && t == P * KS + P) ? 1.0f : 0.f),
+                w2.y + ((add_centre && t == P * KS + P) ? 1.0f : 0.f));     // x + conv(x)
+  }
+  const float2 b2 = (wk && bias) ? __ldg(reinterpret_cast<const float2*>(bias + cs0) + cp) : make_float2(0.f, 0.f);
+  const unsigned long long bz = pk2(b2.x, b2.y);
+  pdl_sync();
   // stage the patch (zeros outside the image): asynchronous 16-byte copies, all in flight at once
   // (with the LayerNorm affine the values pass through registers instead)
   constexpr int CH = CS / 8;                         // 16-byte chunks per pixel of the slice
@@ -573,15 +583,6 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
     }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
-  unsigned long long wr[KS * KS];
-#pragma unroll
-  for (int t = 0; t < KS * KS; ++t) {
-    const float2 w2 = wk ? __ldg(reinterpret_cast<const float2*>(wk + (size_t)t * C + cs0) + cp) : make_float2(0.f, 0.f);
-    wr[t] = pk2(w2.x + ((add_centre && t == P * KS + P) ? 1.0f : 0.f),
-                w2.y + ((add_centre && t == P * KS + P) ? 1.0f : 0.f));     // x + conv(x)
-  }
-  const float2 b2 = (wk && bias) ? __ldg(reinterpret_cast<const float2*>(bias + cs0) + cp) : make_float2(0.f, 0.f);
-  const unsigned long long bz = pk2(b2.x, b2.y);
   const uint32_t* tile32 = reinterpret_cast<const uint32_t*>(tile);        // [PH][PW][32 pairs]
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
@@ -641,6 +642,13 @@ int launch_dwconv_cl(const __nv_bfloat16* x, const float* wk, const float* bias,
   if (y_f32 == nullptr && C % 64 == 0 && (wk == nullptr || (aligned16(wk) && (bias == nullptr || aligned16(bias))))) {
 #define CSSM_DW(KS_, CG_, NC_, TH_) \
   return launch_dwconv_tiled<KS_, CG_, NC_, TH_>(x, wk, bias, pre_a, pre_b, y, Nimg, H, W, C, add_centre, gelu, st)
+    // Few images: tiles of 4 x 4 or 4 x 8 outputs while those of the large geometry leave SMs idle.
+    const long long large = (long long)Nimg * (C / 64) * (ks == 7 ? (long long)((H + 7) / 8) * ((W + 27) / 28)
+                                                                  : (long long)((H + 6) / 7) * ((W + 13) / 14));
+    if (large < sm_count()) {
+      if (ks == 7) CSSM_DW(7, 4, 1, 4);
+      CSSM_DW(3, 4, 1, 4);
+    }
     if (ks == 7) {
       if (W % 28 == 0 && H % 8 != 0 && H % 7 == 0) CSSM_DW(7, 4, 7, 7);      // 28 x 28 planes
       if (W % 28 == 0) CSSM_DW(7, 4, 7, 8);                                  // 56 x 56 planes
