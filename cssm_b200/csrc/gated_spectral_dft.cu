@@ -20,6 +20,7 @@ namespace cssm {
 struct GatedDftArgs {
   float* xz; const cf* khat; const float4* gates; const float* dchan;
   int B, T, C, P, groups, last_only, mode;        // mode: see launch_spectral
+  int reps, z_first;                              // recurrence steps of frame T - 1; 1: z planes in the first frame of a clip
   size_t region; int ldx, ldc;
   DpGeom g;
 };
@@ -60,18 +61,20 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
         const cf* kx = a.khat + (size_t)(c0 + pl) * NB + kw;
         float4 g0[YT], g1[YT];
         cf k0[YT], k1[YT];
+        const int reps = t == a.T - 1 ? a.reps : 1;
+        const bool need_k = t > 0 || reps > 1;
 #pragma unroll
         for (int e = 0; e < YT; ++e) {
           const int k = min(kr + e, g.Hp - 1), o0 = k * g.Wp, o1 = k == 0 ? 0 : (g.H - k) * g.Wp;
           g0[e] = g1[e] = make_float4(1.f, 1.f, invHW, 0.f);         // ungated: A = K_hat, U = X_hat
           if (a.mode != 1) { g0[e] = __ldg(gx + o0); g1[e] = __ldg(gx + o1); }
           k0[e] = k1[e] = mk(0.f, 0.f);
-          if (t > 0) {
+          if (need_k) {
             const float2 u0 = __ldg(reinterpret_cast<const float2*>(kx + o0)), u1 = __ldg(reinterpret_cast<const float2*>(kx + o1));
             k0[e] = mk(u0.x, u0.y); k1[e] = mk(u1.x, u1.y);
           }
         }
-        const float dc = (a.mode == 3 && t > 0) ? __ldg(a.dchan + frame * a.C + c0 + pl) : 1.f;
+        const float dc = (a.mode == 3 && need_k) ? __ldg(a.dchan + frame * a.C + c0 + pl) : 1.f;
         auto step = [](float4 gt, cf kh, cf f, cf h) {
           cf U = mk(gt.y * f.x, gt.y * f.y);
           if (U.x * U.x + U.y * U.y < gt.w * gt.w) U = mk(gt.w, 0.f);
@@ -86,7 +89,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
           float4 st = make_float4(0.f, 0.f, 0.f, 0.f);
           if (t > 0) st = ST[k * ldc + x];
           g0[e].x *= dc; g1[e].x *= dc;
-          const cf h0 = step(g0[e], k0[e], f0[e], mk(st.x, st.y)), h1 = step(g1[e], k1[e], f1[e], mk(st.z, st.w));
+          cf h0 = step(g0[e], k0[e], f0[e], mk(st.x, st.y)), h1 = step(g1[e], k1[e], f1[e], mk(st.z, st.w));
+          for (int r = 1; r < reps; ++r) { h0 = step(g0[e], k0[e], f0[e], h0); h1 = step(g1[e], k1[e], f1[e], h1); }
           if (keep) ST[k * ldc + x] = make_float4(h0.x, h0.y, h1.x, h1.y);
           if (emit)
             RA[k * ldc + x] = dp_fold_spec(k == 0 || 2 * k == g.H, mk(g0[e].z * h0.x, g0[e].z * h0.y),
@@ -100,7 +104,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
       float* out = reinterpret_cast<float*>(RA);
       dp_inv_rows<RT, YT, NT>(g, RB, ldx, TW, out, P);
       __syncthreads();
-      dp_store<NT>(g, out, xp, a.mode == 0 ? xp + (size_t)a.C * HW : nullptr, P);
+      const float* zp = (a.z_first ? a.xz + ((size_t)b * a.T * 2 * a.C + c0) * HW : xp) + (size_t)a.C * HW;
+      dp_store<NT>(g, out, xp, a.mode == 0 ? zp : nullptr, P);
     }
   }
 }
@@ -155,13 +160,14 @@ static size_t gated_dft_bytes(const DpGeom& g, int P, int T) {
 bool gated_spectral_dft_fits(int H, int W, int T) { return gated_dft_bytes(dp_geom(H, W), 1, T) <= 226 * 1024; }
 
 int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat, const float* gates, float* xz,
-                              int last_only, int mode, cudaStream_t st, const float* dchan) {
+                              int last_only, int mode, cudaStream_t st, const float* dchan, int reps, int z_first) {
   const DpChoice ch = dp_choose(H, W, C, B, 1, 226 * 1024, gated_dft_bytes, T);
   if (ch.P == 0) return CSSM_ERR_UNSUPPORTED;
   GatedDftArgs a;
   memset(&a, 0, sizeof(a));
   a.xz = xz; a.khat = khat; a.gates = reinterpret_cast<const float4*>(gates); a.dchan = dchan;
   a.B = B; a.T = T; a.C = C; a.P = ch.P; a.last_only = last_only; a.mode = mode;
+  a.reps = reps; a.z_first = z_first;
   a.g = dp_geom(H, W);
   a.groups = B * ((C + ch.P - 1) / ch.P);
   a.region = dp_region_bytes(a.g, ch.P);

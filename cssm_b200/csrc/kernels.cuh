@@ -23,6 +23,9 @@ struct StencilArgs {
   float* sums;                                   // (B*T, C) or nullptr
 };
 int launch_plane_stencil(const StencilArgs& s, cudaStream_t st);
+// The stencil of a clip of equal frames: reads the planes of the first frame of every clip, writes the T that differ
+// (T <= max(kt, 1)); post is not supported.  CSSM_ERR_UNSUPPORTED: planes that do not fit an SM.
+int launch_repeat_stencil(const StencilArgs& s, cudaStream_t st);
 
 // temporal conv + SiLU (+ input gates) on the q, k, v planes of the GDN block in one launch
 struct QkvTconvArgs {
@@ -52,8 +55,9 @@ int launch_spectral(int B, int T, int H, int W, int C, const cf* khat, const flo
 size_t generic_smem_bytes(int H, int W);
 // folded-DFT kernel for any plane size (csrc/gated_spectral_dft.cu); same arguments as launch_spectral
 bool gated_spectral_dft_fits(int H, int W, int T);
+// (reps: times the recurrence step of frame T - 1 is taken; z_first: the z planes are those of the first frame of a clip)
 int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat, const float* gates, float* xz,
-                              int last_only, int mode, cudaStream_t st, const float* dchan);
+                              int last_only, int mode, cudaStream_t st, const float* dchan, int reps = 1, int z_first = 0);
 int read_spec_error(int* out, int clear);
 
 // ---- DeltaNet block (scalar delta rule) ----

@@ -558,6 +558,121 @@ static int dispatch_stencil_fast(const StencilArgs& s, cudaStream_t st, bool* ha
   return CSSM_OK;
 }
 
+// One source frame for a whole clip: the spatial conv is the same for every frame, and frame f of the temporal one sees
+// f + 1 equal frames (after kt - 1 frames nothing changes any more: the caller asks for T <= kt).  So a plane is read and
+// convolved once, by G threads from a zero-bordered tile, and written for the T frames that differ (48 clips of 8 frames,
+// 14 x 14 x 256 twice and 7 x 7 x 384: three launches 184 us frame by frame, 56 so).
+// KSP, KT: tap counts, -1: at run time (up to 7 x 7 and 8).
+template <int G, int KSP, int KT>
+__global__ void __launch_bounds__(256) repeat_stencil_kernel(const StencilArgs s, FastDiv dw) {
+  extern __shared__ __align__(16) float sm[];
+  __shared__ float red[8][8];
+  constexpr int TF = KT > 0 ? KT : 8;                  // frames at most
+  const int ksp = KSP >= 0 ? KSP : s.ksp, kt = KT >= 0 ? KT : s.kt, lo = ksp > 0 ? (ksp - 1) / 2 : 0;
+  const int HW = s.H * s.W, pitch = s.W + (ksp > 0 ? ksp - 1 : 0), rows = s.H + (ksp > 0 ? ksp - 1 : 0);
+  const int lt = threadIdx.x % G, pl = threadIdx.x / G, lane = threadIdx.x & 31;
+  const int plane = blockIdx.x * (256 / G) + pl, total = s.B * s.C;
+  const bool on = plane < total;
+  const int b = on ? plane / s.C : 0, c = on ? plane - b * s.C : 0;
+  float* raw = sm + pl * pitch * rows;
+  const size_t fstride = (size_t)s.planes_per_frame * HW;
+  float* __restrict__ p = s.buf + ((size_t)b * s.T * s.planes_per_frame + s.plane0 + c) * HW;
+  float wsp[KSP > 0 ? KSP * KSP : 49], wt[TF];
+#pragma unroll
+  for (int i = 0; i < (KSP >= 0 ? KSP * KSP : 49); ++i) wsp[i] = i < ksp * ksp ? __ldg(s.wsp + (size_t)i * s.C + c) : 0.f;
+#pragma unroll
+  for (int j = 0; j < TF; ++j) wt[j] = j < kt ? __ldg(s.wt + (size_t)j * s.C + c) : 0.f;
+  const float bsp = ksp > 0 ? __ldg(s.bsp + c) : 0.f, bt = kt > 0 ? __ldg(s.bt + c) : 0.f;
+  for (int i = lt; i < pitch * rows; i += G) raw[i] = 0.f;
+  if (G == 32) __syncwarp(); else __syncthreads();
+  pdl_sync();
+  if (on)
+    for (int i0 = lt; i0 < HW; i0 += 8 * G) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = i0 + u * G < HW ? p[i0 + u * G] : 0.f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int i = i0 + u * G, h = dw.div(i);
+        if (i < HW) raw[(h + lo) * pitch + i - h * s.W + lo] = v[u];
+      }
+    }
+  if (G == 32) __syncwarp(); else __syncthreads();
+  float sum[TF];
+#pragma unroll
+  for (int f = 0; f < TF; ++f) sum[f] = 0.f;
+  if (on)
+    for (int i = lt; i < HW; i += G) {
+      const int h = dw.div(i), w = i - h * s.W;
+      const float* r = raw + h * pitch + w;
+      float v;
+      if (ksp > 0) {
+        v = bsp;
+        if constexpr (KSP >= 0) {
+#pragma unroll
+          for (int di = 0; di < KSP; ++di)
+#pragma unroll
+            for (int dj = 0; dj < KSP; ++dj) v = fmaf(wsp[di * KSP + dj], r[di * pitch + dj], v);
+        } else {
+          int q = 0;
+          for (int di = 0; di < ksp; ++di)
+            for (int dj = 0; dj < ksp; ++dj) v = fmaf(__ldg(s.wsp + (size_t)q++ * s.C + c), r[di * pitch + dj], v);
+        }
+      } else {
+        v = *r;
+      }
+#pragma unroll
+      for (int f = 0; f < TF; ++f) {
+        if (f >= s.T) continue;
+        float o = v;
+        if (kt > 0) {
+          // tap j reads frame f - (kt - 1) + j, the newest first
+          if constexpr (KT > 0) o = fmaf(wt[KT - 1], v, bt);
+          else {
+#pragma unroll
+            for (int j = 0; j < TF; ++j) if (j == kt - 1) o = fmaf(wt[j], v, bt);
+          }
+#pragma unroll
+          for (int j = 0; j < TF - 1; ++j) if (j < kt - 1 && j >= kt - 1 - f) o = fmaf(wt[j], v, o);
+        }
+        if (s.act) o = silu_f(o);
+        p[(size_t)f * fstride + i] = o;
+        sum[f] += o;
+      }
+    }
+  if (s.sums == nullptr) return;
+#pragma unroll
+  for (int f = 0; f < TF; ++f) {
+    if (f >= s.T) continue;
+    float t = sum[f];
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_down_sync(0xffffffffu, t, off);
+    if (G == 32) { if (lane == 0 && on) s.sums[((size_t)b * s.T + f) * s.C + c] = t; }
+    else if (lane == 0) red[f][threadIdx.x >> 5] = t;
+  }
+  if (G == 32) return;
+  __syncthreads();
+  if (on && lt < s.T) {
+    float t = 0.f;
+    for (int i = 0; i < 8; ++i) t += red[lt][i];
+    s.sums[((size_t)b * s.T + lt) * s.C + c] = t;
+  }
+}
+
+int launch_repeat_stencil(const StencilArgs& s, cudaStream_t st) {
+  const int halo = s.ksp > 0 ? s.ksp - 1 : 0;
+  const size_t plane = (size_t)(s.H + halo) * (s.W + halo) * sizeof(float);
+  if (s.T > 8 || s.kt > 8 || s.ksp > 7 || s.T > (s.kt > 1 ? s.kt : 1) || s.post != nullptr || plane > 200 * 1024) return CSSM_ERR_UNSUPPORTED;
+  const bool warp = 8 * plane <= 48 * 1024;            // a plane a warp up to 37 x 37 and a 3 x 3 conv, else a CTA
+  const size_t smem = warp ? 8 * plane : plane;
+  auto kern = s.ksp == 3 && s.kt == 4 ? (warp ? repeat_stencil_kernel<32, 3, 4> : repeat_stencil_kernel<256, 3, 4>)
+                                      : (warp ? repeat_stencil_kernel<32, -1, -1> : repeat_stencil_kernel<256, -1, -1>);
+  const cudaError_t e = func_smem(kern, smem);
+  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  const long long planes = (long long)s.B * s.C;
+  launch_k(kern, (unsigned)(warp ? (planes + 7) / 8 : planes), 256, smem, st, s, FastDiv(s.W));
+  return check_launch();
+}
+
 int launch_plane_stencil(const StencilArgs& s, cudaStream_t st) {
   if (s.ksp > 7 || s.kt > 8) return CSSM_ERR_UNSUPPORTED;
   if (s.W % 4 == 0 && (s.H * s.W == 4096 || s.H * s.W == 1024) &&
