@@ -114,6 +114,7 @@ struct GdnSpectralArgs {
                              // transforms, readout and inverse transforms of earlier steps are skipped)
 };
 int launch_gdn_spectral(const GdnSpectralArgs& a, cudaStream_t st);
+int read_p32_error(int* out, int clear);
 int launch_gdn_spectral_dft(const GdnSpectralArgs& a, cudaStream_t st);    // as launch_deltanet_spectral_dft
 size_t gdn_generic_smem_bytes(int H, int W, int dk);
 
