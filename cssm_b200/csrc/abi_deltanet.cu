@@ -431,7 +431,8 @@ int cssm_deltanet_forward(const cssm_deltanet_desc* d, const cssm_deltanet_weigh
   if (deltanet_path(*d) == PATH_R64) {
     if ((s = launch_deltanet_spectral_r64(sp, st)) != CSSM_OK) return s;
   } else if (deltanet_path(*d) == PATH_R32) {
-    if ((s = launch_deltanet_spectral_r32(sp, st)) != CSSM_OK) return s;
+    s = sp.chan != nullptr ? launch_deltanet_spectral_p32(sp, st) : launch_deltanet_spectral_r32(sp, st);
+    if (s != CSSM_OK) return s;
   } else if ((s = launch_deltanet_spectral_dft(sp, st)) != CSSM_ERR_UNSUPPORTED) {
     if (s != CSSM_OK) return s;
   } else {

@@ -1,4 +1,5 @@
-// Fused spectral kernel of the DeltaNetCSSM block for 32x32 planes.  One CTA of 288 threads per
+// Fused spectral kernel of the DeltaNetCSSM block for 32x32 planes with gate maps over the bins (per-channel gates:
+// csrc/gdn_spectral_p32.cu).  One CTA of 288 threads per
 // (batch, group of four channels) walks t = 0..T-1; the four q planes, the four k planes and the
 // four v planes of the group are each transformed side by side (r32.cuh geometry: plane = group / 17
 // in the column passes).  Per step:
@@ -57,8 +58,6 @@ __global__ void __launch_bounds__(D32_THREADS, 2) deltanet_spectral_r32(const Dn
   const int boff = (kw << 2) + q;                        // the lane's first bin; register r adds r * 68
   const cf* whp = a.what + (size_t)(c0 + cpl) * NB + boff;
   const float floor_mag = a.goom_floor ? 1e-7f : 0.f;
-  const bool chan = a.chan != nullptr;                   // same for the whole grid
-  const float invHW = 1.0f / (float)HW;
 
   cf hst[8];
 #pragma unroll
@@ -116,7 +115,7 @@ __global__ void __launch_bounds__(D32_THREADS, 2) deltanet_spectral_r32(const Dn
           for (int r = 0; r < 8; ++r) {
             cf z = v[r];
             if (pass == 1) {
-              const float bk = !col_on ? 0.f : (chan ? 1.f : __ldg(&a.abkv[gbase + r * 68].z));
+              const float bk = col_on ? __ldg(&a.abkv[gbase + r * 68].z) : 0.f;
               z = mk(z.x * bk, z.y * bk);
             }
             (pass == 0 ? SQ : SK)[r * D32_THREADS + tid] = z;
@@ -141,21 +140,14 @@ __global__ void __launch_bounds__(D32_THREADS, 2) deltanet_spectral_r32(const Dn
 #pragma unroll
       for (int w = 0; w < 9; ++w) { sq += red[w][cpl]; sk += red[w][4 + cpl]; }
       const float nq = rsqrtf(sq + 1e-6f), nk = rsqrtf(sk + 1e-6f);
-      float2 ab = make_float2(0.f, 0.f);
-      if (chan) ab = __ldg(&a.chan[frame * a.C + c0 + cpl]);
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
         float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
         float cgv = 0.f;
         cf w = mk(0.f, 0.f);
         if (col_on) {
-          if (chan) {
-            g = make_float4(ab.x, ab.y, 1.f, 1.f);
-            cgv = invHW;
-          } else {
-            g = __ldg(&a.abkv[gbase + r * 68]);
-            cgv = __ldg(&a.cg[gbase + r * 68]);
-          }
+          g = __ldg(&a.abkv[gbase + r * 68]);
+          cgv = __ldg(&a.cg[gbase + r * 68]);
           w = whp[r * 68];
         }
         const cf ks = SK[r * D32_THREADS + tid], qs = SQ[r * D32_THREADS + tid];
@@ -210,7 +202,7 @@ __global__ void __launch_bounds__(D32_THREADS, 2) deltanet_spectral_r32(const Dn
 }
 
 int launch_deltanet_spectral_r32(const DnSpectralArgs& a, cudaStream_t st) {
-  if (a.H != 32 || a.W != 32 || a.C % 4 != 0) return CSSM_ERR_UNSUPPORTED;
+  if (a.chan != nullptr || a.H != 32 || a.W != 32 || a.C % 4 != 0) return CSSM_ERR_UNSUPPORTED;
   const size_t smem = spread_smem(D32_SMEM_BYTES, (long long)a.B * (a.C / 4));
   cudaError_t e = func_smem(deltanet_spectral_r32, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }

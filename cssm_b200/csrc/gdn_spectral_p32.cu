@@ -13,6 +13,11 @@
 // was bound by the shared-memory pipe and its barriers: 128 x 32 x 32 x 32 x 64 3853 -> 2346 us.  Taken back: an inverse warp
 // beside six forward ones (2544: it sets the pace), one copy of the FFT per pass (2494), the inverse a step later (2449).
 // Every wait is bounded; on expiry the kernel records an error code (cssm_device_error) and winds down.
+//
+// The same stream serves the scalar delta rule of the DeltaNet block with per-channel gates (DN): a "head" is four channels, whose q,
+// k and v planes and outputs take the places of the four rows, and a bin's state is one number a channel.  24 x 12 x 32 x 32 x 64:
+// 337 -> 194 us.  (Gate maps over the bins scale k before its norm is taken, which the row pass here cannot see:
+// csrc/deltanet_spectral_r32.cu.)
 
 // Complex adds as scalar pairs: a lane's FFT is all register renaming then, where packed adds want their operands in aligned
 // register pairs and the moves for that cost more than the issue slots they save (2368 -> 2346 us).
@@ -37,9 +42,16 @@ constexpr uint32_t GP_BAR_OFF = GP_SPEC_OFF + 24u * P32_PLANE_CF * 8u;
 constexpr uint32_t GP_SMEM = GP_BAR_OFF + 256u;
 static_assert(GP_OUT_BYTES >= 2 * P32_PLANE_CF * 8 && GP_SMEM + 1024 <= 227 * 1024, "one CTA per SM");
 
+struct P32Args {
+  float* qkv; const cf* what;
+  const float2* ab; int ab_heads;              // GDN: gate maps
+  const float2* chan; float rho, floor_mag;    // DeltaNet: (BT, C) {alpha, beta}
+  int B, T, C, use_l2;
+};
+
 // LAST: only the last step's output planes are produced: the q planes, the readout and the inverse of earlier steps are skipped.
-template <bool LAST>
-__global__ void __launch_bounds__(GP_THREADS, 1) gdn_spectral_p32(const GdnSpectralArgs a, const __grid_constant__ CUtensorMap map) {
+template <bool LAST, bool DN>
+__global__ void __launch_bounds__(GP_THREADS, 1) gdn_spectral_p32(const P32Args a, const __grid_constant__ CUtensorMap map) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(smem + GP_BAR_OFF);     // [6]
@@ -202,12 +214,18 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gdn_spectral_p32(const GdnSpect
     typedef unsigned long long u64;
     u64 Sx[2][2][4], Sy[2][2][4];                                         // [bin][row pair][column of the state]
     float2 gn[2], wn[2];                                                  // gates and W_hat of the step to come
+    cf hs[2][4], wd[2][4];                                                // DN: states and W_hat of the head's channels
+    float2 cn = make_float2(0.f, 0.f);                                    // DN: gates of channel lane & 3 in the step to come
     auto fetch = [&](int head, int t) {
       const int b = head / nh, hd = head - b * nh;
-      const float2* ab = a.ab + ((size_t)(b * T + t) * a.ab_heads + (a.ab_heads > 1 ? hd : 0)) * NB;
-      const float2* wh = reinterpret_cast<const float2*>(a.what) + (size_t)hd * NB;
-      gn[0] = __ldg(ab + g0); gn[1] = __ldg(ab + g1);
-      wn[0] = __ldg(wh + g0); wn[1] = __ldg(wh + g1);
+      if constexpr (DN) {
+        cn = __ldg(a.chan + (size_t)(b * T + t) * a.C + hd * DK + (lane & 3));
+      } else {
+        const float2* ab = a.ab + ((size_t)(b * T + t) * a.ab_heads + (a.ab_heads > 1 ? hd : 0)) * NB;
+        const float2* wh = reinterpret_cast<const float2*>(a.what) + (size_t)hd * NB;
+        gn[0] = __ldg(ab + g0); gn[1] = __ldg(ab + g1);
+        wn[0] = __ldg(wh + g0); wn[1] = __ldg(wh + g1);
+      }
     };
     if (mine > 0) fetch(blockIdx.x, 0);
     int step = 0, emitted = 0;
@@ -217,13 +235,20 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gdn_spectral_p32(const GdnSpect
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int r = 0; r < 2; ++r)
+        for (int c = 0; c < 4; ++c) {
+          if constexpr (DN) {
+            const float2 u = __ldg(reinterpret_cast<const float2*>(a.what) + (size_t)((head % nh) * DK + c) * NB + (i ? g1 : g0));
+            wd[i][c] = mk(u.x, u.y);
+            hs[i][c] = mk(0.f, 0.f);
+          } else {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) Sx[i][r][c] = Sy[i][r][c] = 0ull;
+            for (int r = 0; r < 2; ++r) Sx[i][r][c] = Sy[i][r][c] = 0ull;
+          }
+        }
       for (int t = 0; t < T; ++t, ++step) {
         const int slot = step & 1;
         const bool emit = !LAST || t == T - 1;
-        const float2 gc[2] = {gn[0], gn[1]}, wc[2] = {wn[0], wn[1]};
+        const float2 gc[2] = {gn[0], gn[1]}, wc[2] = {wn[0], wn[1]}, cc = cn;
         if (t + 1 < T) fetch(head, t + 1);
         else if (h + 1 < mine) fetch(head + gridDim.x, 0);
         if (!(ok = wait(&spec_full[slot], (step >> 1) & 1, 3))) break;
@@ -234,65 +259,94 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gdn_spectral_p32(const GdnSpect
           nv[0] = n0.x; nv[1] = n0.y; nv[2] = n0.z; nv[3] = n0.w; nv[4] = n1.x; nv[5] = n1.y; nv[6] = n1.z; nv[7] = n1.w;
         }
         cf oo[2][4];
+        if constexpr (DN) {
+          // per channel: A = squash(alpha W_hat (1 - beta |k|^2)), h = A h + beta v conj(k), o = h q
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const float beta = gc[q].y;
-          u64 kx[4], ky[4], kyn[4];
-          {
-            cf kk[4];
-            float ks = 0.f;
+          for (int c = 0; c < 4; ++c) {
+            const float alpha = __shfl_sync(0xffffffffu, cc.x, c), beta = __shfl_sync(0xffffffffu, cc.y, c);
+            const float nq = nv[c] * (1.0f / 1024.0f), nk = nv[4 + c];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const cf k = p32_read1(sp + (4 + i) * P32_PLANE_CF, real, kw, kh, q);
-              kk[i] = mk(k.x * nv[4 + i], k.y * nv[4 + i]);
-              ks += kk[i].x * kk[i].x + kk[i].y * kk[i].y;
-            }
-            const float kn = rsqrtf(ks + 1e-6f);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float x = kk[i].x * kn, y = kk[i].y * kn;
-              kx[i] = pk2(x, x); ky[i] = pk2(y, y); kyn[i] = pk2(-y, -y);
-            }
-          }
-          const float awx = gc[q].x * wc[q].x, awy = gc[q].x * wc[q].y;
-          const u64 ax = pk2(awx, awx), ay = pk2(awy, awy), ayn = pk2(-awy, -awy), bn = pk2(-beta, -beta);
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const cf v0 = p32_read1(sp + (8 + 2 * r) * P32_PLANE_CF, real, kw, kh, q), v1 = p32_read1(sp + (9 + 2 * r) * P32_PLANE_CF, real, kw, kh, q);
-            // d = sum_j conj(k_j) S_j;  S_i <- aw (S_i - beta k_i d) + beta v conj(k_i)
-            u64 dr = 0ull, di = 0ull;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              dr = fma2(Sx[q][r][i], kx[i], dr); dr = fma2(Sy[q][r][i], ky[i], dr);
-              di = fma2(Sy[q][r][i], kx[i], di); di = fma2(Sx[q][r][i], kyn[i], di);
-            }
-            const u64 er = mul2(dr, bn), ei = mul2(di, bn);
-            const u64 bvx = pk2(beta * v0.x, beta * v1.x), bvy = pk2(beta * v0.y, beta * v1.y), bvxn = pk2(-beta * v0.x, -beta * v1.x);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const u64 ir = fma2(kyn[i], ei, fma2(kx[i], er, Sx[q][r][i])), ii = fma2(ky[i], er, fma2(kx[i], ei, Sy[q][r][i]));
-              Sx[q][r][i] = fma2(bvy, ky[i], fma2(bvx, kx[i], fma2(ayn, ii, mul2(ax, ir))));
-              Sy[q][r][i] = fma2(bvxn, ky[i], fma2(bvy, kx[i], fma2(ay, ir, mul2(ax, ii))));
-            }
-          }
-          if (emit) {
-            // o = sum_i S_i q_i
-            u64 orr[2] = {0ull, 0ull}, oi[2] = {0ull, 0ull};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const cf qv = p32_read1(sp + i * P32_PLANE_CF, real, kw, kh, q);
-              const float sc = nv[i] * (1.0f / 1024.0f), x = qv.x * sc, y = qv.y * sc;
-              const u64 qx = pk2(x, x), qy = pk2(y, y), qyn = pk2(-y, -y);
-#pragma unroll
-              for (int r = 0; r < 2; ++r) {
-                orr[r] = fma2(Sx[q][r][i], qx, orr[r]); orr[r] = fma2(Sy[q][r][i], qyn, orr[r]);
-                oi[r] = fma2(Sx[q][r][i], qy, oi[r]); oi[r] = fma2(Sy[q][r][i], qx, oi[r]);
+            for (int q = 0; q < 2; ++q) {
+              const cf ks = p32_read1(sp + (4 + c) * P32_PLANE_CF, real, kw, kh, q), v = p32_read1(sp + (8 + c) * P32_PLANE_CF, real, kw, kh, q);
+              const cf k = mk(ks.x * nk, ks.y * nk);
+              const float sc = alpha * (1.0f - beta * (k.x * k.x + k.y * k.y));
+              cf A = mk(wd[q][c].x * sc, wd[q][c].y * sc);
+              const float am = sqrtf(A.x * A.x + A.y * A.y), sq = a.rho / (1.0f + am);
+              A = mk(A.x * sq, A.y * sq);
+              if (am * sq < a.floor_mag) A = mk(a.floor_mag, 0.f);
+              cf U = cmulc(v, k);
+              U = mk(U.x * beta, U.y * beta);
+              if (U.x * U.x + U.y * U.y < a.floor_mag * a.floor_mag) U = mk(a.floor_mag, 0.f);
+              cf hn = cmul(A, hs[q][c]);
+              hn.x += U.x; hn.y += U.y;
+              hs[q][c] = hn;
+              if (emit) {
+                const cf qs = p32_read1(sp + c * P32_PLANE_CF, real, kw, kh, q);
+                oo[q][c] = cmul(hn, mk(qs.x * nq, qs.y * nq));
               }
             }
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const float beta = gc[q].y;
+            u64 kx[4], ky[4], kyn[4];
+            {
+              cf kk[4];
+              float ks = 0.f;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const cf k = p32_read1(sp + (4 + i) * P32_PLANE_CF, real, kw, kh, q);
+                kk[i] = mk(k.x * nv[4 + i], k.y * nv[4 + i]);
+                ks += kk[i].x * kk[i].x + kk[i].y * kk[i].y;
+              }
+              const float kn = rsqrtf(ks + 1e-6f);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float x = kk[i].x * kn, y = kk[i].y * kn;
+                kx[i] = pk2(x, x); ky[i] = pk2(y, y); kyn[i] = pk2(-y, -y);
+              }
+            }
+            const float awx = gc[q].x * wc[q].x, awy = gc[q].x * wc[q].y;
+            const u64 ax = pk2(awx, awx), ay = pk2(awy, awy), ayn = pk2(-awy, -awy), bn = pk2(-beta, -beta);
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-              upk2(orr[r], oo[q][2 * r].x, oo[q][2 * r + 1].x);
-              upk2(oi[r], oo[q][2 * r].y, oo[q][2 * r + 1].y);
+              const cf v0 = p32_read1(sp + (8 + 2 * r) * P32_PLANE_CF, real, kw, kh, q), v1 = p32_read1(sp + (9 + 2 * r) * P32_PLANE_CF, real, kw, kh, q);
+              // d = sum_j conj(k_j) S_j;  S_i <- aw (S_i - beta k_i d) + beta v conj(k_i)
+              u64 dr = 0ull, di = 0ull;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                dr = fma2(Sx[q][r][i], kx[i], dr); dr = fma2(Sy[q][r][i], ky[i], dr);
+                di = fma2(Sy[q][r][i], kx[i], di); di = fma2(Sx[q][r][i], kyn[i], di);
+              }
+              const u64 er = mul2(dr, bn), ei = mul2(di, bn);
+              const u64 bvx = pk2(beta * v0.x, beta * v1.x), bvy = pk2(beta * v0.y, beta * v1.y), bvxn = pk2(-beta * v0.x, -beta * v1.x);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const u64 ir = fma2(kyn[i], ei, fma2(kx[i], er, Sx[q][r][i])), ii = fma2(ky[i], er, fma2(kx[i], ei, Sy[q][r][i]));
+                Sx[q][r][i] = fma2(bvy, ky[i], fma2(bvx, kx[i], fma2(ayn, ii, mul2(ax, ir))));
+                Sy[q][r][i] = fma2(bvxn, ky[i], fma2(bvy, kx[i], fma2(ay, ir, mul2(ax, ii))));
+              }
+            }
+            if (emit) {
+              // o = sum_i S_i q_i
+              u64 orr[2] = {0ull, 0ull}, oi[2] = {0ull, 0ull};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const cf qv = p32_read1(sp + i * P32_PLANE_CF, real, kw, kh, q);
+                const float sc = nv[i] * (1.0f / 1024.0f), x = qv.x * sc, y = qv.y * sc;
+                const u64 qx = pk2(x, x), qy = pk2(y, y), qyn = pk2(-y, -y);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                  orr[r] = fma2(Sx[q][r][i], qx, orr[r]); orr[r] = fma2(Sy[q][r][i], qyn, orr[r]);
+                  oi[r] = fma2(Sx[q][r][i], qy, oi[r]); oi[r] = fma2(Sy[q][r][i], qx, oi[r]);
+                }
+              }
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                upk2(orr[r], oo[q][2 * r].x, oo[q][2 * r + 1].x);
+                upk2(oi[r], oo[q][2 * r].y, oo[q][2 * r + 1].y);
+              }
             }
           }
         }
@@ -333,19 +387,37 @@ static bool plane_map(CUtensorMap* map, float* base, uint64_t rows) {
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int launch_gdn_spectral_p32(const GdnSpectralArgs& a, cudaStream_t st) {
+static int launch_p32(const P32Args& a, bool last_only, bool dn, cudaStream_t st) {
   const long long rows = (long long)a.B * a.T * 3 * a.C * 32;
-  if (a.static_image || a.dk != 4 || a.H != 32 || a.W != 32 || rows >= (1LL << 31)) return CSSM_ERR_UNSUPPORTED;
+  if (rows >= (1LL << 31)) return CSSM_ERR_UNSUPPORTED;
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
   if (!plane_map(&map, a.qkv, (uint64_t)rows)) return CSSM_ERR_CUDA;
-  auto kern = a.last_only ? gdn_spectral_p32<true> : gdn_spectral_p32<false>;
+  auto kern = dn ? gdn_spectral_p32<false, true> : last_only ? gdn_spectral_p32<true, false> : gdn_spectral_p32<false, false>;
   const size_t smem = GP_SMEM + 1024;
   const cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   const int heads = a.B * (a.C / 4), sms = sm_count();
   launch_k(kern, heads < sms ? heads : sms, GP_THREADS, smem, st, a, map);
   return check_launch();
+}
+
+int launch_gdn_spectral_p32(const GdnSpectralArgs& g, cudaStream_t st) {
+  if (g.static_image || g.dk != 4 || g.H != 32 || g.W != 32) return CSSM_ERR_UNSUPPORTED;
+  P32Args a;
+  memset(&a, 0, sizeof(a));
+  a.qkv = g.qkv; a.what = g.what; a.ab = g.ab; a.ab_heads = g.ab_heads;
+  a.B = g.B; a.T = g.T; a.C = g.C; a.use_l2 = g.use_l2;
+  return launch_p32(a, g.last_only != 0, false, st);
+}
+
+int launch_deltanet_spectral_p32(const DnSpectralArgs& g, cudaStream_t st) {
+  if (g.chan == nullptr || g.H != 32 || g.W != 32 || g.C % 4 != 0) return CSSM_ERR_UNSUPPORTED;
+  P32Args a;
+  memset(&a, 0, sizeof(a));
+  a.qkv = g.qkv; a.what = g.what; a.chan = g.chan; a.rho = g.rho; a.floor_mag = g.goom_floor ? 1e-7f : 0.f;
+  a.B = g.B; a.T = g.T; a.C = g.C; a.use_l2 = 1;
+  return launch_p32(a, false, true, st);
 }
 
 int read_p32_error(int* out, int clear) {

@@ -73,7 +73,8 @@ struct DnSpectralArgs {
   int goom_floor;
 };
 int launch_deltanet_spectral_r64(const DnSpectralArgs& a, cudaStream_t st);
-int launch_deltanet_spectral_r32(const DnSpectralArgs& a, cudaStream_t st);
+int launch_deltanet_spectral_r32(const DnSpectralArgs& a, cudaStream_t st);      // gate maps; per-channel gates: _p32
+int launch_deltanet_spectral_p32(const DnSpectralArgs& a, cudaStream_t st);      // csrc/gdn_spectral_p32.cu
 // any plane size; CSSM_ERR_UNSUPPORTED when one channel does not fit an SM's shared memory
 int launch_deltanet_spectral_dft(const DnSpectralArgs& a, cudaStream_t st);
 

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from cssm_b200 import GatedDeltaNetCSSM, device_error
+from cssm_b200 import DeltaNetCSSM, GatedDeltaNetCSSM, device_error
 from oracle import cssm_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -47,3 +47,17 @@ def test_real_columns_alone(kind, l2):
     y, last, ref = _case(2, 3, 16, 3, edit, l2)
     assert orc.rel_l2(y, ref) <= 2e-5
     assert orc.rel_l2(last, ref[:, -1]) <= 2e-5
+
+
+@pytest.mark.parametrize("B,C", [(1, 4), (2, 12), (149, 4), (20, 64)])
+@pytest.mark.parametrize("T", [1, 2, 5])
+def test_deltanet_channel_gates(B, C, T):
+    kw = dict(kernel_size=3, rope_mode="none", gate_type="channel")
+    x = np.random.default_rng(T).standard_normal((B, T, 32, 32, C)).astype(np.float32)
+    m = DeltaNetCSSM(channels=C, **kw)
+    p = orc.init_deltanet_params(5, C, 32, 32, kernel_size=3, gate_type="channel", bias_scale=0.1)
+    p["output_proj"]["bias"][:] = 0                      # the block's signal is two orders below a 0.1-scale bias
+    ref = orc.deltanet_forward(p, x, **kw)
+    got = m.apply({"params": p}, torch.from_numpy(x).cuda()).cpu().numpy()
+    assert orc.rel_l2(got, ref) <= 1e-4
+    assert device_error() == 0
