@@ -494,15 +494,17 @@ dwconv_cl_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ 
 // Tile geometry as template parameters: CG column groups (32 * CG threads), NC columns per group, TH rows;
 // the launcher picks one that divides the plane (8 x 16 tiles on a 28 x 28 plane compute 31 % more
 // outputs than the plane has).
-template <int KS, int CG, int NC, int TH>
+// OUT: bfloat16 outputs, or float32 ones, whose staged patch is float32 too (the affine is not rounded).
+template <int KS, int CG, int NC, int TH, class OUT>
 __global__ void __launch_bounds__(32 * CG)
 dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ wk,
                     const float* __restrict__ bias, const float* __restrict__ pre_a,
-                    const float* __restrict__ pre_b, __nv_bfloat16* __restrict__ y, int H, int W, int C,
+                    const float* __restrict__ pre_b, OUT* __restrict__ y, int H, int W, int C,
                     int add_centre, int gelu) {
   constexpr int CS = 64, P = (KS - 1) / 2, TW = CG * NC, PW = TW + KS - 1, PH = TH + KS - 1, NT = 32 * CG;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_raw);        // [PH][PW][CS]
+  constexpr bool F32 = sizeof(OUT) == 4;
+  OUT* tile = reinterpret_cast<OUT*>(smem_raw);                            // [PH][PW][CS]
   const int tiles_w = (W + TW - 1) / TW, tiles_h = (H + TH - 1) / TH, slices = C / CS;
   int bid = blockIdx.x;
   const int sl = bid % slices; bid /= slices;
@@ -535,7 +537,7 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
     pav[0] = a0.x; pav[1] = a0.y; pav[2] = a0.z; pav[3] = a0.w; pav[4] = a1.x; pav[5] = a1.y; pav[6] = a1.z; pav[7] = a1.w;
     pbv[0] = b0.x; pbv[1] = b0.y; pbv[2] = b0.z; pbv[3] = b0.w; pbv[4] = b1.x; pbv[5] = b1.y; pbv[6] = b1.z; pbv[7] = b1.w;
   }
-  if (pre_a == nullptr) {
+  if (!F32 && pre_a == nullptr) {
     for (int pr = 0; pr < PH; ++pr) {
       const int hi = h0 + pr - P;
       const bool hin = hi >= 0 && hi < H;
@@ -543,7 +545,7 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
         const int ck = q & (CH - 1), pc = q / CH;
         const int wi = w0 + pc - P;
         const bool in = hin && wi >= 0 && wi < W;
-        __nv_bfloat16* dst = tile + ((size_t)pr * PW + pc) * CS + ck * 8;
+        OUT* dst = tile + ((size_t)pr * PW + pc) * CS + ck * 8;
         const __nv_bfloat16* src = xn + ((size_t)(in ? hi : 0) * W + (in ? wi : 0)) * C + ck * 8;
         // src-size 0 writes zeros
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
@@ -570,15 +572,19 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
       for (int u = 0; u < SBN; ++u) {
         const int i = base + u * NT;
         if (i >= TOT) continue;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (inb[u]) {
-          float f[8];
-          unpack8(raw[u], f);
+        float f[8];
+        unpack8(raw[u], f);
+        if (inb[u] && (!F32 || pre_a != nullptr)) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) f[j] = fmaf(pav[j], f[j], pbv[j]);
-          v = pack8(f);
         }
-        *reinterpret_cast<uint4*>(tile + (size_t)i * 8) = v;        // [pr][pc][ck] is the order of i
+        OUT* dst = tile + (size_t)i * 8;                            // [pr][pc][ck] is the order of i
+        if constexpr (F32) {
+          *reinterpret_cast<float4*>(dst) = make_float4(f[0], f[1], f[2], f[3]);
+          *reinterpret_cast<float4*>(dst + 4) = make_float4(f[4], f[5], f[6], f[7]);
+        } else {
+          *reinterpret_cast<uint4*>(dst) = pack8(f);
+        }
       }
     }
   }
@@ -598,8 +604,13 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
       unsigned long long xv[KS];
 #pragma unroll
       for (int tj = 0; tj < KS; ++tj) {
-        const uint32_t u = tile32[((size_t)ir * PW + wl + tj) * 32 + cp];
-        xv[tj] = pk2(__uint_as_float(u << 16), __uint_as_float(u & 0xFFFF0000u));
+        if constexpr (F32) {
+          const float2 u = *reinterpret_cast<const float2*>(tile + ((size_t)ir * PW + wl + tj) * CS + 2 * cp);
+          xv[tj] = pk2(u.x, u.y);
+        } else {
+          const uint32_t u = tile32[((size_t)ir * PW + wl + tj) * 32 + cp];
+          xv[tj] = pk2(__uint_as_float(u << 16), __uint_as_float(u & 0xFFFF0000u));
+        }
       }
 #pragma unroll
       for (int o = 0; o < TH; ++o) {
@@ -616,21 +627,23 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
       float va, vb;
       upk2(acc[o], va, vb);
       if (gelu) gelu_tanh_x2(va, vb);
-      *reinterpret_cast<uint32_t*>(y + (((size_t)n * H + h) * W + w0 + wl) * C + cs0 + 2 * cp) = float2_to_bf16x2(va, vb);
+      OUT* yo = y + (((size_t)n * H + h) * W + w0 + wl) * C + cs0 + 2 * cp;
+      if constexpr (F32) *reinterpret_cast<float2*>(yo) = make_float2(va, vb);
+      else *reinterpret_cast<uint32_t*>(yo) = float2_to_bf16x2(va, vb);
     }
   }
 }
 
-template <int KS, int CG, int NC, int TH>
+template <int KS, int CG, int NC, int TH, class OUT>
 static int launch_dwconv_tiled(const __nv_bfloat16* x, const float* wk, const float* bias, const float* pre_a,
-                               const float* pre_b, __nv_bfloat16* y, int Nimg, int H, int W, int C,
+                               const float* pre_b, OUT* y, int Nimg, int H, int W, int C,
                                int add_centre, int gelu, cudaStream_t st) {
   constexpr int TW = CG * NC;
-  const size_t smem = (size_t)(TH + KS - 1) * (TW + KS - 1) * 64 * 2;
-  cudaError_t e = func_smem(dwconv_tiled_kernel<KS, CG, NC, TH>, smem);
+  const size_t smem = (size_t)(TH + KS - 1) * (TW + KS - 1) * 64 * sizeof(OUT);
+  cudaError_t e = func_smem(dwconv_tiled_kernel<KS, CG, NC, TH, OUT>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   const long long grid = (long long)Nimg * ((H + TH - 1) / TH) * ((W + TW - 1) / TW) * (C / 64);
-  launch_k(dwconv_tiled_kernel<KS, CG, NC, TH>, (unsigned)grid, 32 * CG, smem, st, x, wk, bias, pre_a, pre_b, y, H, W, C,
+  launch_k(dwconv_tiled_kernel<KS, CG, NC, TH, OUT>, (unsigned)grid, 32 * CG, smem, st, x, wk, bias, pre_a, pre_b, y, H, W, C,
                                                                             add_centre, gelu);
   return check_launch();
 }
@@ -639,25 +652,30 @@ int launch_dwconv_cl(const __nv_bfloat16* x, const float* wk, const float* bias,
                      const float* pre_b, __nv_bfloat16* y, float* y_f32, int Nimg, int H, int W, int C,
                      int ks, int add_centre, int gelu, cudaStream_t st) {
   if (C % 8 != 0 || (ks != 3 && ks != 7)) return CSSM_ERR_UNSUPPORTED;
-  if (y_f32 == nullptr && C % 64 == 0 && (wk == nullptr || (aligned16(wk) && (bias == nullptr || aligned16(bias))))) {
+  // (float32 outputs, 33 images of 256 pixels: three launches 42 -> 21 us against dwconv_cl_kernel)
+  if ((y_f32 == nullptr || ks == 3) && C % 64 == 0 && (wk == nullptr || (aligned16(wk) && (bias == nullptr || aligned16(bias))))) {
 #define CSSM_DW(KS_, CG_, NC_, TH_) \
   return launch_dwconv_tiled<KS_, CG_, NC_, TH_>(x, wk, bias, pre_a, pre_b, y, Nimg, H, W, C, add_centre, gelu, st)
-    // Few images: tiles of 4 x 4 or 4 x 8 outputs while those of the large geometry leave SMs idle.
+#define CSSM_DW3(CG_, NC_, TH_) \
+  return y_f32 != nullptr ? launch_dwconv_tiled<3, CG_, NC_, TH_>(x, wk, bias, pre_a, pre_b, y_f32, Nimg, H, W, C, add_centre, gelu, st) \
+                          : launch_dwconv_tiled<3, CG_, NC_, TH_>(x, wk, bias, pre_a, pre_b, y, Nimg, H, W, C, add_centre, gelu, st)
+    // Few images: tiles of 4 x 4 outputs while those of the large geometry leave SMs idle.
     const long long large = (long long)Nimg * (C / 64) * (ks == 7 ? (long long)((H + 7) / 8) * ((W + 27) / 28)
                                                                   : (long long)((H + 6) / 7) * ((W + 13) / 14));
     if (large < sm_count()) {
       if (ks == 7) CSSM_DW(7, 4, 1, 4);
-      CSSM_DW(3, 4, 1, 4);
+      CSSM_DW3(4, 1, 4);
     }
     if (ks == 7) {
       if (W % 28 == 0 && H % 8 != 0 && H % 7 == 0) CSSM_DW(7, 4, 7, 7);      // 28 x 28 planes
       if (W % 28 == 0) CSSM_DW(7, 4, 7, 8);                                  // 56 x 56 planes
       CSSM_DW(7, 4, 4, 8);
     }
-    if (W == 14 && H == 14) CSSM_DW(3, 2, 7, 7);                             // two tiles per plane
-    if (W == 7 && H == 7) CSSM_DW(3, 1, 7, 7);
-    CSSM_DW(3, 4, 4, 8);
+    if (W == 14 && H == 14) CSSM_DW3(2, 7, 7);                               // two tiles per plane
+    if (W == 7 && H == 7) CSSM_DW3(1, 7, 7);
+    CSSM_DW3(4, 4, 8);
 #undef CSSM_DW
+#undef CSSM_DW3
   }
   constexpr int RH = 4;
   const size_t smem = (size_t)(ks * ks * C + C) * 4;
