@@ -34,6 +34,8 @@ struct GemmArgs {
   int g_compact;            // 1: the gate is indexed by the OUTPUT frame, 0: by the source frame
   int out_act;              // 0 none, 1 silu, 2 sigmoid; applied to output columns n >= act_n0
   int act_n0;
+  // planar output, gemm_tc only: columns n < mul_n multiply plane (frame*mul_planes + mul_plane0 + n) of mul in place and are not stored
+  float* mul; int mul_planes, mul_plane0, mul_n;
   int z_last_only;          // planar output: columns n >= act_n0 are only stored for frames with t == T-1
   const float* sub;         // channels-last output only: (M, N) tensor subtracted from the result, or nullptr
 };

@@ -606,7 +606,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
 
 int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.HW <= 0) return CSSM_ERR_DIMS;
-  if (g.K % 4 != 0 || g.N % 4 != 0) return CSSM_ERR_UNSUPPORTED;
+  if (g.K % 4 != 0 || g.N % 4 != 0 || g.mul != nullptr) return CSSM_ERR_UNSUPPORTED;
   SplitGeom q;
   memset(&q, 0, sizeof(q));
   q.kblocks = (g.K + GS_BK - 1) / GS_BK;

@@ -62,7 +62,8 @@ struct TcSmem {
 // ZLAST: the output columns from act_n0 on (the z half of the in_proj) are only produced for the
 // last frame of every clip (last-frame-only forward); a compile-time variant so that the default
 // kernel carries no extra test.
-template <int N, bool A_PLANAR, bool STG, bool ZLAST = false>
+// MUL: the first g.mul_n output columns multiply planes in place.
+template <int N, bool A_PLANAR, bool STG, bool ZLAST = false, bool MUL = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensorMap omap) {
   // tile schedule: round-robin over the CTAs
@@ -385,6 +386,14 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
 #pragma unroll
               for (int j = 0; j < 32; ++j) vals[j] = sigmoid_f(vals[j]);
             }
+            if (MUL && cc * 32 < g.mul_n) {
+              op = g.mul + ((size_t)fr * g.mul_planes + g.mul_plane0 + cc * 32) * g.HW + px;
+              float old[32];
+#pragma unroll
+              for (int j = 0; j < 32; ++j) old[j] = op[(size_t)j * g.HW];
+#pragma unroll
+              for (int j = 0; j < 32; ++j) vals[j] *= old[j];
+            }
 #pragma unroll
             for (int j = 0; j < 32; ++j) op[(size_t)j * g.HW] = vals[j];
           } else {
@@ -429,6 +438,7 @@ bool gemm_tc_supported(const GemmArgs& g, bool a_planar) {
   if (g.K != TC_K || (g.N != 64 && g.N != 128 && g.N != 192)) return false;
   if (g.HW % TC_BM != 0 || g.M % TC_BM != 0) return false;
   if (g.out_act != 0 && g.act_n0 % 32 != 0) return false;
+  if (g.mul != nullptr && (g.mul_n % 32 != 0 || g.N == 64)) return false;
   if (a_planar && g.N == 192) return false;
   return true;
 }
@@ -457,20 +467,20 @@ static bool make_out_map(const GemmArgs& g, bool a_planar, CUtensorMap* map) {
   return r == CUDA_SUCCESS;
 }
 
-template <int N, bool A_PLANAR, bool STG, bool ZLAST = false>
+template <int N, bool A_PLANAR, bool STG, bool ZLAST = false, bool MUL = false>
 static int launch_tc_v(const GemmArgs& g, const CUtensorMap& map, cudaStream_t st) {
   const int num_tiles = g.M / TC_BM;
   const int sms = sm_count();
   cudaError_t e;
   const int grid = num_tiles < sms ? num_tiles : sms;
   const size_t smem = TcSmem<N, STG>::TOTAL + 1024;      // slack for the 1024-byte alignment
-  e = func_smem(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST>, smem);
+  e = func_smem(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST, MUL>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   // Planes of 64x64: the 64 planes of a tile lie 1 MB apart in all, which neighbouring SMs share (NoGate's output
   // projection of 48 x 4 frames: 104 us in grid order, 139 with the CTAs where SMs came free); 8 x 4 frames and less, and
   // smaller planes, gain more by the early start.  Channels-last input: the second projection of the same rows.
   const PdlOff alone(N == 64 && num_tiles > 8 * sms && (!A_PLANAR || g.HW >= 4096));
-  launch_k(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST>, grid, TC_THREADS, smem, st, g, num_tiles, map);
+  launch_k(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST, MUL>, grid, TC_THREADS, smem, st, g, num_tiles, map);
   return check_launch();
 }
 
@@ -493,6 +503,11 @@ int launch_gemm_tc(const GemmArgs& g, bool a_planar, cudaStream_t st) {
     CUtensorMap map;
     memset(&map, 0, sizeof(map));
     return launch_tc_v<128, false, false, true>(g, map, st);
+  }
+  if (g.mul != nullptr && !a_planar) {
+    CUtensorMap map;
+    memset(&map, 0, sizeof(map));
+    return g.N == 192 ? launch_tc_v<192, false, false, false, true>(g, map, st) : launch_tc_v<128, false, false, false, true>(g, map, st);
   }
   if (!a_planar)
     return g.N == 192 ? launch_tc<192, false>(g, st)
