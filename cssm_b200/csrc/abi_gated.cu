@@ -189,7 +189,7 @@ int cssm_gated_plan_init(const cssm_gated_desc* d, const cssm_gated_weights* w, 
 
 static int gated_in_proj_impl(const cssm_gated_desc* d, const cssm_gated_weights* w,
                               const void* plan, const float* x, float* xz, void* stream,
-                              int x_bcast, int z_last_only = 0);
+                              int x_bcast, int z_last_only = 0, const void* wsplit = nullptr);
 
 int cssm_gated_in_proj(const cssm_gated_desc* d, const cssm_gated_weights* w, const void* plan,
                        const float* x, float* xz, void* stream) {
@@ -200,7 +200,7 @@ int cssm_gated_in_proj(const cssm_gated_desc* d, const cssm_gated_weights* w, co
 // z_last_only != 0: the silu(z) planes are only written for the last frame of every clip
 static int gated_in_proj_impl(const cssm_gated_desc* d, const cssm_gated_weights* w,
                               const void* plan, const float* x, float* xz, void* stream,
-                              int x_bcast, int z_last_only) {
+                              int x_bcast, int z_last_only, const void* wsplit) {
   int s = validate(d);
   if (s != CSSM_OK) return s;
   if (!w || !w->in_proj_kernel || !w->in_proj_bias || !plan || !x || !xz) return CSSM_ERR_NULL;
@@ -210,7 +210,7 @@ static int gated_in_proj_impl(const cssm_gated_desc* d, const cssm_gated_weights
   GemmArgs g;
   memset(&g, 0, sizeof(g));
   g.M = d->B * d->T * d->H * d->W; g.N = 2 * d->C; g.K = d->C; g.HW = d->H * d->W;
-  g.A = x; g.Wk = w->in_proj_kernel; g.bias = w->in_proj_bias;
+  g.A = x; g.Wk = w->in_proj_kernel; g.bias = w->in_proj_bias; g.wsplit = wsplit;
   g.out = xz; g.o_planes = 2 * d->C; g.o_plane0 = 0;
   g.out_act = 1; g.act_n0 = d->C;          // the z planes are stored as silu(z)
   if (d->rope_mode != CSSM_ROPE_NONE) {
@@ -303,11 +303,11 @@ static int distinct_frames(const cssm_gated_desc& d) {
 // Workspace frames: Td per image; x_main and z of the image in the first.  (48 images of 224 pixels, T = 8: the classifier's pass
 // 1702 -> 1044 us; projections 626 -> 213, short convs 184 -> 56, transforms 283 -> 180.)
 static int equal_frames_last(const cssm_gated_desc& d, const cssm_gated_weights& w, const void* plan, const float* x, float* y,
-                             float* xz, float* ctx, float* gm, int Td, cudaStream_t st) {
+                             float* xz, float* ctx, float* gm, int Td, const void* split_in, const void* split_out, cudaStream_t st) {
   GemmArgs g;
   memset(&g, 0, sizeof(g));
   g.M = d.B * d.H * d.W; g.N = 2 * d.C; g.K = d.C; g.HW = d.H * d.W;
-  g.A = x; g.Wk = w.in_proj_kernel; g.bias = w.in_proj_bias;
+  g.A = x; g.Wk = w.in_proj_kernel; g.bias = w.in_proj_bias; g.wsplit = split_in;
   g.out = xz; g.o_planes = Td * 2 * d.C; g.o_plane0 = 0;
   g.out_act = 1; g.act_n0 = d.C;
   g.T = 1; g.H = d.H; g.W = d.W;
@@ -332,10 +332,14 @@ static int equal_frames_last(const cssm_gated_desc& d, const cssm_gated_weights&
   g.M = d.B * d.H * d.W; g.N = d.C; g.K = d.C; g.HW = d.H * d.W;
   g.A = xz; g.a_planes = 2 * d.C; g.a_plane0 = 0;
   g.a_fmul = Td; g.a_fadd = Td - 1;
-  g.Wk = w.out_proj_kernel; g.bias = w.out_proj_bias;
+  g.Wk = w.out_proj_kernel; g.bias = w.out_proj_bias; g.wsplit = split_out;
   g.out = y;
   g.T = 1; g.H = d.H; g.W = d.W;
   return launch_gemm<true, false>(g, st);
+}
+
+size_t gated_split_bytes(const cssm_gated_desc& d) {
+  return round_up(split_weights_bytes(d.C, 2 * d.C), 256) + round_up(split_weights_bytes(d.C, d.C), 256);
 }
 
 int gated_forward_internal(const cssm_gated_desc* d, const cssm_gated_weights* w,
@@ -355,11 +359,20 @@ int gated_forward_internal(const cssm_gated_desc* d, const cssm_gated_weights* w
   float* xz = (float*)(ws + l.xz_planar);
   float* ctx = (float*)(ws + l.ctx_sum);
   float* gm = (float*)(ws + l.gate_maps);
+  // room behind the workspace: the projections' weights split once (the last frame's calls, whose projections are short)
+  const char *split_in = nullptr, *split_out = nullptr;
+  const size_t sb = gated_split_bytes(*d);
+  if (last_only && sb > 0 && workspace_bytes >= l.total + sb) {
+    char* out = ws + l.total;
+    split_in = out; split_out = out + round_up(split_weights_bytes(d->C, 2 * d->C), 256);
+    s = launch_split_weights(d->C, w->in_proj_kernel, 2 * d->C, out, w->out_proj_kernel, d->C, (char*)split_out, (cudaStream_t)stream);
+    if (s != CSSM_OK) return s;
+  }
   const int Td = distinct_frames(*d);
   if (x_bcast && last_only && d->T > 1 && d->rope_mode == CSSM_ROPE_NONE && spectral_path(d->H, d->W) == PATH_GENERIC &&
       gated_spectral_dft_fits(d->H, d->W, Td))
-    return equal_frames_last(*d, *w, plan, x, y, xz, ctx, gm, Td, (cudaStream_t)stream);
-  if ((s = gated_in_proj_impl(d, w, plan, x, xz, stream, x_bcast, last_only)) != CSSM_OK) return s;
+    return equal_frames_last(*d, *w, plan, x, y, xz, ctx, gm, Td, split_in, split_out, (cudaStream_t)stream);
+  if ((s = gated_in_proj_impl(d, w, plan, x, xz, stream, x_bcast, last_only, split_in)) != CSSM_OK) return s;
   if ((s = cssm_gated_short_conv(d, w, xz, ctx, stream)) != CSSM_OK) return s;
   if ((s = cssm_gated_gates(d, w, ctx, gm, stream)) != CSSM_OK) return s;
   if (!last_only) {
@@ -376,7 +389,7 @@ int gated_forward_internal(const cssm_gated_desc* d, const cssm_gated_weights* w
   g.M = d->B * d->H * d->W; g.N = d->C; g.K = d->C; g.HW = d->H * d->W;
   g.A = xz; g.a_planes = 2 * d->C; g.a_plane0 = 0;
   g.a_fmul = d->T; g.a_fadd = d->T - 1;
-  g.Wk = w->out_proj_kernel; g.bias = w->out_proj_bias;
+  g.Wk = w->out_proj_kernel; g.bias = w->out_proj_bias; g.wsplit = split_out;
   g.out = y;
   g.T = 1; g.H = d->H; g.W = d->W;
   return launch_gemm<true, false>(g, (cudaStream_t)stream);

@@ -94,7 +94,7 @@ static BlockWs block_ws_layout(const cssm_shvit_block_desc& d) {
       const cssm_gated_desc g = mixer_desc(d);
       l.x32 = take(M * C * 4);
       l.y32 = take(M * C * 4);
-      l.gws_bytes = cssm_gated_workspace_bytes(&g);
+      l.gws_bytes = cssm_gated_workspace_bytes(&g) + gated_split_bytes(g);
       l.gws = take(l.gws_bytes);
     }
   }

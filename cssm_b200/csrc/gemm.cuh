@@ -20,6 +20,7 @@ struct GemmArgs {
   int a_fdiv, a_fmul, a_fadd;
   int rope_tlast;         // 1: every output frame is rotated as t = T-1; 0: t = output frame % T
   const float* Wk;        // (K, N) row-major
+  const void* wsplit;       // Wk as launch_split_weights left it, or nullptr (gemm_split only; no RMS prologue)
   const float* bias;      // (N) or nullptr
   float* out;             // channels-last (M, N) or planar plane (frame*o_planes + o_plane0 + n)
   int o_planes, o_plane0;
@@ -44,6 +45,10 @@ struct GemmArgs {
 bool gemm_tc_supported(const GemmArgs& g, bool a_planar);
 int launch_gemm_tc(const GemmArgs& g, bool a_planar, cudaStream_t st);
 int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st);
+// The weights of up to two projections (K, N0), (K, N1) split once for all CTAs of their launches, in the layout of an operand
+// block; split_weights_bytes(K, N) each, 16-byte aligned.  0 bytes: K so short that every CTA keeps its share of the weights anyway.
+size_t split_weights_bytes(int K, int N);
+int launch_split_weights(int K, const float* w0, int N0, void* out0, const float* w1, int N1, void* out1, cudaStream_t st);
 int read_tc_error(int* out, int clear);
 int read_split_error(int* out, int clear);
 

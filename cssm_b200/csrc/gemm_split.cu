@@ -25,7 +25,9 @@
 //                          32-column chunks each), 1/rms, bias, activation; planar stores (coalesced
 //                          over pixels) or channels-last rows through a per-warp TMA tensor store.
 // RES: the whole (K, BN) weight tile is split once per CTA and stays in shared memory (the ring then
-// carries A only); without it the producers split the weight block of every stage again.
+// carries A only); without it the producers split the weight block of every stage again, unless the caller had the weights
+// split beforehand (wsplit): then bulk copies bring the blocks, which halves what the producers do (float32 mixers of the
+// classifier, 33 images of 256 pixels: a pass 823 -> 752 us).
 // Rows are flat pixels m = frame * HW + px, so a tile may cross frames and HW may be anything.
 // Every mbarrier wait is bounded; on expiry the kernel records an error code and winds down.
 //
@@ -161,6 +163,36 @@ __device__ __noinline__ void split_row_fma(const SplitArgs& a, int m, int n, flo
   }
 }
 
+// One 16-byte chunk per thread and part: rows n of 32-row groups, [group][K block][part][32 rows x 128 bytes], 128-byte swizzle
+__global__ void __launch_bounds__(256) split_weights_kernel(int K, const float* __restrict__ w0, int N0, unsigned char* __restrict__ out0,
+                                                            const float* __restrict__ w1, int N1, unsigned char* __restrict__ out1,
+                                                            int items0, int items) {
+  pdl_sync();
+  int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= items) return;
+  const bool second = i >= items0;
+  const float* w = second ? w1 : w0;
+  const int N = second ? N1 : N0;
+  unsigned char* out = second ? out1 : out0;
+  if (second) i -= items0;
+  const int kchunks = (K + GS_BK - 1) / GS_BK * 8, n = i % ((N + 31) / 32 * 32), ck = i / ((N + 31) / 32 * 32), kb = ck >> 3;
+  float v[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) v[e] = n < N && ck * 8 + e < K ? __ldg(w + (size_t)(ck * 8 + e) * N + n) : 0.f;
+  store_split8(out + ((size_t)(n >> 5) * (kchunks >> 3) + kb) * 3 * 4096, tc::sw128_offset(n & 31, ck & 7), 4096, v);
+}
+
+size_t split_weights_bytes(int K, int N) {
+  const int kblocks = (K + GS_BK - 1) / GS_BK;
+  return kblocks < 4 ? 0 : (size_t)((N + 31) / 32) * kblocks * 3 * 4096;
+}
+
+int launch_split_weights(int K, const float* w0, int N0, void* out0, const float* w1, int N1, void* out1, cudaStream_t st) {
+  const int kchunks = (K + GS_BK - 1) / GS_BK * 8, items0 = (N0 + 31) / 32 * 32 * kchunks, items = items0 + (N1 + 31) / 32 * 32 * kchunks;
+  launch_k(split_weights_kernel, (items + 255) / 256, 256, 0, st, K, w0, N0, (unsigned char*)out0, w1, N1, (unsigned char*)out1, items0, items);
+  return check_launch();
+}
+
 // GATE: planar A times the gate planes.  WIDE: more than one leading accumulator (nl > 1).
 template <bool A_PLANAR, bool RES, bool GATE, bool WIDE>
 __global__ void __launch_bounds__(GS_THREADS, 1)
@@ -180,7 +212,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
   // (The bias itself is read by scalars: it may sit at any 4-byte offset of a parameter buffer.)
   float* bias_s = reinterpret_cast<float*>(stg + (A_PLANAR ? 8u * 4096u : 0u));
   float* ss_s = bias_s + 256;                                     // [GS_SS][2][128] row sums (RMS prologue)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ss_s + (A_PLANAR ? GS_SS * 256 : 0));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ss_s + (A_PLANAR && g.rms_scale != nullptr ? GS_SS * 256 : 0));
   uint64_t* full = bars;           // [4] block written (8 producer warps)
   uint64_t* empty = bars + 4;      // [4] block consumed (tcgen05.commit)
   uint64_t* accfull = bars + 8;    // [2] accumulator set complete (tcgen05.commit)
@@ -196,7 +228,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
   while (tmem_cols < (uint32_t)bufs * acc_cols) tmem_cols <<= 1;
 
   if (tid == 0) {
-    for (int s = 0; s < NS; ++s) { tc::mbar_init(&full[s], GS_PROD / 32); tc::mbar_init(&empty[s], 1); }
+    for (int s = 0; s < NS; ++s) { tc::mbar_init(&full[s], GS_PROD / 32 + (!RES && g.wsplit != nullptr ? 1 : 0)); tc::mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; ++a) { tc::mbar_init(&accfull[a], 1); tc::mbar_init(&accempty[a], 8); }
     tc::mbar_init(done, 1);
     tc::fence_mbar_init();
@@ -382,7 +414,17 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
         if (g.rms_scale != nullptr && nkb == 0) { ss_s[((tcnt % GS_SS) * 2 + kh) * 128 + prow] = ss; ss = 0.f; }
         if (ntile < num_tiles) fetch(ntile, nkb);
       }
-      if (!RES) {
+      if (!RES && g.wsplit != nullptr) {
+        if (tid == 0) {                                 // (it has waited for the stage above)
+          unsigned char* b_s = a_s + GS_A_BYTES;
+          const int grp0 = (tile % q.n_tiles) * (q.BN >> 5), grps = min(q.BN >> 5, ((g.N + 31) >> 5) - grp0);
+          tc::mbar_expect_tx(&full[s], (uint32_t)grps * 3u * 4096u);
+          const unsigned char* src = static_cast<const unsigned char*>(g.wsplit) + ((size_t)grp0 * kblocks + kb) * 3 * 4096;
+          for (int i = 0; i < grps; ++i)
+            for (int p = 0; p < 3; ++p)
+              tc::bulk_g2s(b_s + p * b_part + i * 4096, src + ((size_t)i * kblocks * 3 + p) * 4096, 4096, &full[s]);
+        }
+      } else if (!RES) {
         unsigned char* b_s = a_s + GS_A_BYTES;
         const int n0 = (tile % q.n_tiles) * q.BN;
         for (int item = tid; item < q.BN * 8; item += GS_PROD) {
@@ -614,7 +656,8 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   q.hw = FastDiv(g.HW); q.w = FastDiv(g.W > 0 ? g.W : 1); q.t = FastDiv(g.T > 0 ? g.T : 1);
   q.fdiv = FastDiv(g.a_fdiv > 1 ? g.a_fdiv : 1);
   constexpr size_t LIMIT = 227 * 1024;
-  const size_t fixed = 1024 + 1024 + 128 + (a_planar ? 8 * 4096 + GS_SS * 1024 : 0);   // slack, bias, barriers, staging, sums
+  const size_t fixed = 1024 + 1024 + 128 + (a_planar ? 8 * 4096 + (g.rms_scale != nullptr ? GS_SS * 1024 : 0) : 0);   // slack, bias, barriers, staging, sums
+  if (g.wsplit != nullptr && (g.rms_scale != nullptr || !aligned16(g.wsplit))) return CSSM_ERR_UNSUPPORTED;
   auto round32 = [](int v) { return (v + 31) / 32 * 32; };
   auto res_size = [&](int bn) { return (size_t)q.kblocks * 3 * bn * 128; };
   // Weights resident when a tile of at least 64 columns (or all of N) leaves room for two A stages:
@@ -633,9 +676,9 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   int nt = q.nl > 0 ? (g.N + 127) / 128 : (g.N + 255) / 256;
   while (round32((g.N + nt - 1) / nt) > 32 && res_size(round32((g.N + nt - 1) / nt)) + 2 * GS_A_BYTES + fixed > LIMIT) ++nt;
   q.BN = round32((g.N + nt - 1) / nt);
-  const bool res = !wide && (q.BN >= 64 || nt == 1) && res_size(q.BN) + 2 * GS_A_BYTES + fixed <= LIMIT;
+  const bool res = !wide && g.wsplit == nullptr && (q.BN >= 64 || nt == 1) && res_size(q.BN) + 2 * GS_A_BYTES + fixed <= LIMIT;
   if (!res) {
-    int most = a_planar ? 96 : 128;
+    int most = g.rms_scale != nullptr ? 96 : 128;        // the row sums leave no room for two stages of 128 columns
     if (most > bn_tmem) most = bn_tmem;
     nt = (g.N + most - 1) / most;
     q.BN = round32((g.N + nt - 1) / nt);

@@ -200,6 +200,8 @@ int launch_gated_spectral_cl(const __nv_bfloat16* xz, int ld, int Nimg, int H, i
                              const float* gates, __nv_bfloat16* y, int ldy, cudaStream_t st);
 
 // ---- whole-block drivers shared by the C-ABI sources ----
+// bytes behind the workspace with which the last frame's calls have their projections' weights split once (0: no use)
+size_t gated_split_bytes(const cssm_gated_desc& d);
 // last_only: y is (B,H,W,C), the last output frame.  x_bcast: x is (B,H,W,C), one frame per
 // batch element standing for all T frames (an image repeated over the sequence).
 int gated_forward_internal(const cssm_gated_desc* d, const cssm_gated_weights* w, const void* plan,
