@@ -254,7 +254,10 @@ int cssm::gdn_forward_internal(const cssm_gdn_desc* d, const cssm_gdn_weights* w
     g.A = x; g.rope_t = rt; g.rope_h = rh; g.rope_w = rw; g.rope_nz = rnz;
     if (x_bcast) { g.a_fdiv = d->T; g.a_fmul = 1; g.a_fadd = 0; }
   }
-  if ((s = launch_gemm<false, true>(g, st)) != CSSM_OK) return s;
+  // with the temporal conv of stage 5 in the same launch it waits for the gate maps (B_k, B_v)
+  const bool with_conv = d->short_conv_size > 0 && gemm_qkv_tconv_supported(g, d->short_conv_size);
+  const GemmArgs qkv_proj = g;
+  if (!with_conv && (s = launch_gemm<false, true>(g, st)) != CSSM_OK) return s;
 
   // 3. output gate projection of the rotated input -> planar, through SiLU / sigmoid
   //    (last_only: rows of frame T-1 of every batch element -> planes (B, C, H, W))
@@ -290,15 +293,16 @@ int cssm::gdn_forward_internal(const cssm_gdn_desc* d, const cssm_gdn_weights* w
 
   // 5. causal temporal conv + SiLU on q, k, v planes, input gates on k and v
   mark(4, st);
-  bool tconv_done = false;
+  bool tconv_done = with_conv;
+  QkvTconvArgs ta;
+  memset(&ta, 0, sizeof(ta));
+  ta.buf = qkv; ta.B = d->B; ta.T = Tdata; ta.C = C; ta.HW = HW; ta.kt = d->short_conv_size;
+  for (int i = 0; i < 3; ++i) { ta.wt[i] = w->conv_t_kernel[i]; ta.bt[i] = w->conv_t_bias[i]; }
+  ta.bkv = (d->use_input_gates && !chan) ? (const float2*)(ws + l.bkv) : nullptr;
+  if (with_conv && (s = launch_gemm_qkv_tconv(qkv_proj, ta, st)) != CSSM_OK) return s;
   // one elementwise launch over q, k, v where it measured faster than three per-plane launches
   // (64x64 planes: 1.70 -> 1.36 ms on B=128, T=8; at 32x32 the per-plane kernel is ahead)
-  if (d->short_conv_size >= 2 && d->short_conv_size <= 4 && HW % 4 == 0 && HW != 1024) {
-    QkvTconvArgs ta;
-    memset(&ta, 0, sizeof(ta));
-    ta.buf = qkv; ta.B = d->B; ta.T = Tdata; ta.C = C; ta.HW = HW; ta.kt = d->short_conv_size;
-    for (int i = 0; i < 3; ++i) { ta.wt[i] = w->conv_t_kernel[i]; ta.bt[i] = w->conv_t_bias[i]; }
-    ta.bkv = (d->use_input_gates && !chan) ? (const float2*)(ws + l.bkv) : nullptr;
+  if (!tconv_done && d->short_conv_size >= 2 && d->short_conv_size <= 4 && HW % 4 == 0 && HW != 1024) {
     s = launch_qkv_temporal_conv(ta, st);
     if (s == CSSM_OK) tconv_done = true;
     else if (s != CSSM_ERR_UNSUPPORTED) return s;

@@ -535,6 +535,9 @@ int cssm_device_error(int* out, int clear) {
   if (rc == CSSM_OK) rc = cssm::read_split_error(&a2, clear);
   if (rc != CSSM_OK) return rc;
   a |= a2;
+  rc = cssm::read_qt_error(&a2, clear);
+  if (rc != CSSM_OK) return rc;
+  a |= a2;
   rc = cssm::read_stem_error(&a2, clear);
   if (rc != CSSM_OK) return rc;
   a |= a2;

@@ -34,6 +34,11 @@ struct QkvTconvArgs {
   const float* wt[3]; const float* bt[3];   // short_conv_q/k/v: (kt,1,C), (C)
   const float2* bkv;              // (B*T, H*W) {B_k, B_v} or nullptr (no input gates)
 };
+struct GemmArgs;
+// the projection that makes those planes and this conv in one launch (csrc/gemm_qkv_tconv.cu)
+bool gemm_qkv_tconv_supported(const GemmArgs& g, int kt);
+int launch_gemm_qkv_tconv(const GemmArgs& g, const QkvTconvArgs& a, cudaStream_t st);
+int read_qt_error(int* out, int clear);
 int launch_qkv_temporal_conv(const QkvTconvArgs& a, cudaStream_t st);   // CSSM_ERR_UNSUPPORTED: use the plane stencil
 
 struct GatedGateArgs {
