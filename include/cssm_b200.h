@@ -636,8 +636,9 @@ int cssm_bf16_conv3x3s2(const void* x, int32_t B, int32_t Hi, int32_t Wi, int32_
  * a code in a device word, stops storing results and winds down, and the forward call that
  * launched it has long since returned CSSM_OK (calls are asynchronous).  After synchronising the
  * stream, cssm_device_error copies that word to *out: 0 = no wait ever expired on the current
- * device since the last clear; low byte = fp32 tensor-core projection kernels (1 producer, 2 MMA
- * issuer, 3 drain, 4 epilogue), next byte = fused spectral kernels (1 input plane, 2 z plane),
+ * device since the last clear; low byte = fp32 tensor-core projection and stem kernels (1 producer, 2 MMA
+ * issuer, 3 drain, 4 epilogue), next byte = fused spectral kernels (1 input plane, 2 z plane, 1-6 also the
+ * hand-over of the 32x32 GDN kernel),
  * third byte = bf16 tensor-core GEMM (5 TMA producer, 6 MMA issuer, 7 drain, 8 epilogue, 9 im2col
  * producer), top byte = fused Mlp kernel (1 TMA producer, 2-6 MMA issuers, 8 drain, 9-13 epilogue).
  * A non-zero value means the outputs of the calls since the last clear are not to be trusted.
