@@ -37,13 +37,13 @@ __device__ __forceinline__ void delta_spectra(const DeltaDftArgs& d, const float
   __syncthreads();
   dp_rows<RT, YT, NT>(g, RA, d.ldx, TW, RB, d.ldc, P);
   __syncthreads();
-  dp_cols<RT, YT, NT>(g, RB, d.ldc, TH, P, [&](int x, const int* k, const bool* ok, const cf* f0, const cf* f1) {
+  dp_cols<RT, YT, NT>(g, RB, d.ldc, TH, P, [&](int x, int k0, int m, const cf* f0, const cf* f1) {
 #pragma unroll
     for (int e = 0; e < YT; ++e) {
-      if (!ok[e]) continue;
+      if (e >= m) continue;
       float s0 = 1.f, s1 = 1.f;
-      kgate(x, k[e], s0, s1);
-      RA[k[e] * d.ldc + x] = make_float4(s0 * f0[e].x, s0 * f0[e].y, s1 * f1[e].x, s1 * f1[e].y);
+      kgate(x, k0 + e, s0, s1);
+      RA[(k0 + e) * d.ldc + x] = make_float4(s0 * f0[e].x, s0 * f0[e].y, s1 * f1[e].x, s1 * f1[e].y);
     }
   });
   __syncthreads();

@@ -14,13 +14,7 @@
 //   inv. columns  column        row pair     row freq     (A.re, B.im) | (A.im, -B.re)    A, B = G_k +- G_{H-k}
 //   inv. rows     row pair      pixel pair   column k     f (Re, Im) of row p | of row H-p, f = 1 or 2
 // and what a thread finishes is already folded for the next pass, because its cell holds both members
-// of a pair.
-//
-// Along an axis of even N the outputs pair up too: with y' = N/2 - y,  cos(2 pi n y' / N) = (-1)^n cos(2 pi n y / N) and the sine
-// likewise with the other sign, so with E, O the sums over even and odd n,  acc[y] = E + O  and  acc[y'] = (E - O).(1, -1):  a
-// thread takes half of the y with two sums each, which halves the multiplications and spares a quarter of the reads
-// (16 x 8 x 56 x 56 x 32: 214 -> 203 us, GDN 12 x 8 x 28 x 28 x 64 with key dimension 2: 146 -> 144).
-// The products run from shared memory in register tiles of RT x YT cells; ldx is odd so that
+// of a pair.  The products run from shared memory in register tiles of RT x YT cells; ldx is odd so that
 // both the reads (consecutive lanes = consecutive x) and the transposed writes are free of bank conflicts.
 #pragma once
 #include "common.cuh"
@@ -36,7 +30,6 @@ __device__ __forceinline__ dp_u64 dp_fma2(dp_u64 a, dp_u64 b, dp_u64 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
-template <int V> struct DpInt { static constexpr int value = V; };
 __device__ __forceinline__ float2 dp_unpack(dp_u64 v) {
   float2 f;
   asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
@@ -55,19 +48,15 @@ __device__ inline void dp_fill_table(float2* tw, int N, int ld) {
   }
 }
 
-// One pass along an axis of N: op [Nred][ldx] 16-byte entries, tw [Nred][ldy] pairs, Nred = Y = N / 2 + 1.  epi(x, y, ok, lo, hi)
-// takes the YT cells (x, y[e]) of a tile row at once, those with ok[e], so that it can have their loads in flight together.
+// One pass: op [Nred][ldx] 16-byte entries, tw [Nred][ldy] pairs.  epi(x, y0, m, lo, hi) takes the first m of
+// the YT cells (x, y0 ..) of a tile row at once, so that it can have their loads in flight together.
 template <int RT, int YT, int NT, class Epi>
 __device__ __forceinline__ void dp_pass(const ulonglong2* __restrict__ op, int ldx, const dp_u64* __restrict__ tw,
-                                        int ldy, int N, int X, Epi&& epi) {
-  constexpr int YH = YT / 2;
-  const int Nred = N / 2 + 1, Y = Nred;
-  const bool even = (N & 1) == 0;                                    // same for the whole grid
-  const int base = even ? N / 4 + 1 : Y, wide = even ? YH : YT;      // y that a thread starts from
-  const int nx = (X + RT - 1) / RT, ny = (base + wide - 1) / wide;
+                                        int ldy, int Nred, int X, int Y, Epi&& epi) {
+  const int nx = (X + RT - 1) / RT, ny = (Y + YT - 1) / YT;
   for (int tile = threadIdx.x; tile < nx * ny; tile += NT) {
-    const int ty = tile / nx, tx = tile - ty * nx, y0 = ty * wide;
-    dp_u64 lo[RT][YT], hi[RT][YT];                                   // even: [0, YH) the sums over even n, [YH, YT) over odd n
+    const int ty = tile / nx, tx = tile - ty * nx;
+    dp_u64 lo[RT][YT], hi[RT][YT];
     const ulonglong2* po[RT];
 #pragma unroll
     for (int j = 0; j < RT; ++j) {
@@ -75,63 +64,30 @@ __device__ __forceinline__ void dp_pass(const ulonglong2* __restrict__ op, int l
 #pragma unroll
       for (int e = 0; e < YT; ++e) lo[j][e] = hi[j][e] = 0ull;
     }
-    const dp_u64* pt = tw + y0;
-    if (even) {
-      auto term = [&](auto odd) {
-        constexpr int O = decltype(odd)::value;
-        dp_u64 t[YH];
-        if constexpr (YH == 2) {
-          const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(pt);
-          t[0] = v.x; t[1] = v.y;
-        } else {
-          t[0] = *pt;
-        }
-        pt += ldy;
-#pragma unroll
-        for (int j = 0; j < RT; ++j) {
-          const ulonglong2 o = *po[j];
-          po[j] += ldx;
-#pragma unroll
-          for (int e = 0; e < YH; ++e) {
-            lo[j][O + e] = dp_fma2(o.x, t[e], lo[j][O + e]);
-            hi[j][O + e] = dp_fma2(o.y, t[e], hi[j][O + e]);
-          }
-        }
-      };
-      int n = 0;
+    const dp_u64* pt = tw + ty * YT;
 #pragma unroll 2
-      for (; n + 1 < Nred; n += 2) { term(DpInt<0>()); term(DpInt<YH>()); }
-      if (n < Nred) term(DpInt<0>());
-    } else {
-#pragma unroll 2
-      for (int n = 0; n < Nred; ++n) {
-        dp_u64 t[YT];
+    for (int n = 0; n < Nred; ++n) {
+      dp_u64 t[YT];
+      if constexpr (YT >= 2) {
 #pragma unroll
         for (int e = 0; e < YT; e += 2) {
           const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(pt + e);
           t[e] = v.x; t[e + 1] = v.y;
         }
-        pt += ldy;
+      } else {
+        t[0] = *pt;
+      }
+      pt += ldy;
 #pragma unroll
-        for (int j = 0; j < RT; ++j) {
-          const ulonglong2 o = *po[j];
-          po[j] += ldx;
+      for (int j = 0; j < RT; ++j) {
+        const ulonglong2 o = *po[j];
+        po[j] += ldx;
 #pragma unroll
-          for (int e = 0; e < YT; ++e) {
-            lo[j][e] = dp_fma2(o.x, t[e], lo[j][e]);
-            hi[j][e] = dp_fma2(o.y, t[e], hi[j][e]);
-          }
+        for (int e = 0; e < YT; ++e) {
+          lo[j][e] = dp_fma2(o.x, t[e], lo[j][e]);
+          hi[j][e] = dp_fma2(o.y, t[e], hi[j][e]);
         }
       }
-    }
-    int y[YT];
-    bool ok[YT];
-#pragma unroll
-    for (int e = 0; e < YT; ++e) {
-      const int k = y0 + (even && e >= YH ? e - YH : e);
-      y[e] = even && e >= YH ? N / 2 - k : k;
-      ok[e] = even ? k < base && (e < YH || 4 * k != N) : k < Y;
-      y[e] = ok[e] ? y[e] : 0;
     }
 #pragma unroll
     for (int j = 0; j < RT; ++j) {
@@ -140,15 +96,7 @@ __device__ __forceinline__ void dp_pass(const ulonglong2* __restrict__ op, int l
       float2 l[YT], h[YT];
 #pragma unroll
       for (int e = 0; e < YT; ++e) { l[e] = dp_unpack(lo[j][e]); h[e] = dp_unpack(hi[j][e]); }
-      if (even) {
-#pragma unroll
-        for (int e = 0; e < YH; ++e) {
-          const float2 le = l[e], lt = l[e + YH], he = h[e], ht = h[e + YH];
-          l[e] = make_float2(le.x + lt.x, le.y + lt.y); l[e + YH] = make_float2(le.x - lt.x, lt.y - le.y);
-          h[e] = make_float2(he.x + ht.x, he.y + ht.y); h[e + YH] = make_float2(he.x - ht.x, ht.y - he.y);
-        }
-      }
-      epi(x, y, ok, l, h);
+      epi(x, ty * YT, min(YT, Y - ty * YT), l, h);
     }
   }
 }
@@ -213,32 +161,32 @@ __device__ __forceinline__ void dp_load_fold(const DpGeom& g, const float* __res
 // rows: folded pixels -> folded column operand [row pair][plane * Wp + k]
 template <int RT, int YT, int NT>
 __device__ __forceinline__ void dp_rows(const DpGeom& g, const float4* S, int ldx, const float2* TW, float4* U, int ldc, int P) {
-  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(S), ldx, reinterpret_cast<const dp_u64*>(TW), g.ldw, g.W,
-                  P * g.Hp, [&](int x, const int* k, const bool* ok, const float2* y0, const float2* y1) {
+  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(S), ldx, reinterpret_cast<const dp_u64*>(TW), g.ldw, g.Wp,
+                  P * g.Hp, g.Wp, [&](int x, int k0, int m, const float2* y0, const float2* y1) {
     const int pl = g.dHp.div(x), p = x - pl * g.Hp;
     const bool self = p == 0 || 2 * p == g.H;
-    float4* dst = U + p * ldc + pl * g.Wp;
+    float4* dst = U + p * ldc + pl * g.Wp + k0;
 #pragma unroll
     for (int e = 0; e < YT; ++e)
-      if (ok[e])
-        dst[k[e]] = self ? make_float4(y0[e].x, 0.f, y0[e].y, 0.f)
+      if (e < m)
+        dst[e] = self ? make_float4(y0[e].x, 0.f, y0[e].y, 0.f)
                       : make_float4(y0[e].x + y1[e].x, y1[e].y - y0[e].y, y0[e].y + y1[e].y, y0[e].x - y1[e].x);
   });
 }
 
-// columns: epi(col, k, ok, F, G) with F[e] = F_{k[e]} and G[e] = F_{H-k[e]} of that column, k[e] in 0 .. H/2 where ok[e]
+// columns: epi(col, k0, m, F, G) with F[e] = F_{k0+e} and G[e] = F_{H-k0-e} of that column, k = 0 .. H/2
 // (G is meaningless for a self-paired k)
 template <int RT, int YT, int NT, class Epi>
 __device__ __forceinline__ void dp_cols(const DpGeom& g, const float4* U, int ldc, const float2* TH, int P, Epi&& epi) {
-  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(U), ldc, reinterpret_cast<const dp_u64*>(TH), g.ldh, g.H,
-                  P * g.Wp, [&](int x, const int* k, const bool* ok, const float2* lo, const float2* hi) {
+  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(U), ldc, reinterpret_cast<const dp_u64*>(TH), g.ldh, g.Hp,
+                  P * g.Wp, g.Hp, [&](int x, int k0, int m, const float2* lo, const float2* hi) {
     cf f0[YT], f1[YT];
 #pragma unroll
     for (int e = 0; e < YT; ++e) {
       f0[e] = mk(lo[e].x + lo[e].y, hi[e].x + hi[e].y);
       f1[e] = mk(lo[e].x - lo[e].y, hi[e].x - hi[e].y);
     }
-    epi(x, k, ok, f0, f1);
+    epi(x, k0, m, f0, f1);
   });
 }
 
@@ -251,15 +199,15 @@ __device__ __forceinline__ float4 dp_fold_spec(bool self, cf g0, cf g1) {
 // inverse columns: [k][col] -> inverse row operand [column k][row pair]
 template <int RT, int YT, int NT>
 __device__ __forceinline__ void dp_inv_cols(const DpGeom& g, const float4* V, int ldc, const float2* TH, float4* R, int ldx, int P) {
-  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(V), ldc, reinterpret_cast<const dp_u64*>(TH), g.ldh, g.H,
-                  P * g.Wp, [&](int x, const int* p, const bool* ok, const float2* lo, const float2* hi) {
+  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(V), ldc, reinterpret_cast<const dp_u64*>(TH), g.ldh, g.Hp,
+                  P * g.Wp, g.Hp, [&](int x, int p0, int m, const float2* lo, const float2* hi) {
     const int pl = g.dWp.div(x), k = x - pl * g.Wp;
     const float f = (k == 0 || 2 * k == g.W) ? 1.f : 2.f;
-    float4* dst = R + k * ldx + pl * g.Hp;
+    float4* dst = R + k * ldx + pl * g.Hp + p0;
 #pragma unroll
     for (int e = 0; e < YT; ++e)
-      if (ok[e])
-        dst[p[e]] = make_float4(f * (lo[e].x + lo[e].y), f * (hi[e].x + hi[e].y), f * (lo[e].x - lo[e].y), f * (hi[e].x - hi[e].y));
+      if (e < m)
+        dst[e] = make_float4(f * (lo[e].x + lo[e].y), f * (hi[e].x + hi[e].y), f * (lo[e].x - lo[e].y), f * (hi[e].x - hi[e].y));
   });
 }
 
@@ -268,16 +216,16 @@ __device__ __forceinline__ void dp_inv_cols(const DpGeom& g, const float4* V, in
 template <int RT, int YT, int NT>
 __device__ __forceinline__ void dp_inv_rows(const DpGeom& g, const float4* R, int ldx, const float2* TW, float* out, int P) {
   const int pitch = g.W | 1;
-  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(R), ldx, reinterpret_cast<const dp_u64*>(TW), g.ldw, g.W,
-                  P * g.Hp, [&](int x, const int* ws, const bool* ok, const float2* lo, const float2* hi) {
+  dp_pass<RT, YT, NT>(reinterpret_cast<const ulonglong2*>(R), ldx, reinterpret_cast<const dp_u64*>(TW), g.ldw, g.Wp,
+                  P * g.Hp, g.Wp, [&](int x, int w0, int m, const float2* lo, const float2* hi) {
     const int pl = g.dHp.div(x), p = x - pl * g.Hp;
     float* r0 = out + (pl * g.H + p) * pitch;
     float* r1 = r0 + (g.H - 2 * p) * pitch;
     const bool two = p != 0 && 2 * p != g.H;
 #pragma unroll
     for (int e = 0; e < YT; ++e) {
-      const int w = ws[e];
-      if (!ok[e]) continue;
+      const int w = w0 + e;
+      if (e >= m) continue;
       const bool self_w = w == 0 || 2 * w == g.W;
       r0[w] = lo[e].x + lo[e].y;
       if (!self_w) r0[g.W - w] = lo[e].x - lo[e].y;

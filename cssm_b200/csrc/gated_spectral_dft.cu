@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
       dp_rows<RT, YT, NT>(g, RA, ldx, TW, RB, ldc, P);
       __syncthreads();
       const float4* gp = a.gates + frame * NB;
-      dp_cols<RT, YT, NT>(g, RB, ldc, TH, P, [&](int x, const int* kr, const bool* ok, const cf* f0, const cf* f1) {
+      dp_cols<RT, YT, NT>(g, RB, ldc, TH, P, [&](int x, int kr, int m, const cf* f0, const cf* f1) {
         const int pl = g.dWp.div(x), kw = x - pl * g.Wp;
         const float4* gx = gp + kw;
         const cf* kx = a.khat + (size_t)(c0 + pl) * NB + kw;
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
         const bool need_k = t > 0 || reps > 1;
 #pragma unroll
         for (int e = 0; e < YT; ++e) {
-          const int k = kr[e], o0 = k * g.Wp, o1 = k == 0 ? 0 : (g.H - k) * g.Wp;
+          const int k = min(kr + e, g.Hp - 1), o0 = k * g.Wp, o1 = k == 0 ? 0 : (g.H - k) * g.Wp;
           g0[e] = g1[e] = make_float4(1.f, 1.f, invHW, 0.f);         // ungated: A = K_hat, U = X_hat
           if (a.mode != 1) { g0[e] = __ldg(gx + o0); g1[e] = __ldg(gx + o1); }
           k0[e] = k1[e] = mk(0.f, 0.f);
@@ -84,8 +84,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
         };
 #pragma unroll
         for (int e = 0; e < YT; ++e) {
-          if (!ok[e]) continue;
-          const int k = kr[e];
+          if (e >= m) continue;
+          const int k = kr + e;
           float4 st = make_float4(0.f, 0.f, 0.f, 0.f);
           if (t > 0) st = ST[k * ldc + x];
           g0[e].x *= dc; g1[e].x *= dc;
