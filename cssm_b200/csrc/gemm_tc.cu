@@ -1,15 +1,15 @@
 // tcgen05 / TMEM GEMM for the K = 64 channel projections in fp32-equivalent precision
 // (3 x TF32: A_hi*B_hi + A_lo*B_hi + A_hi*B_lo, accumulated in fp32 in TMEM).
 //
-// Persistent kernel, one CTA per SM, 544 threads, warp-specialised:
-//   warps 0-7  producers : read a 128-pixel A tile from global memory (channels-last rows with
+// Persistent kernel, one CTA per SM, warp-specialised (16 or 8 producer warps first):
+//   producers            : read a 128-pixel A tile from global memory (channels-last rows with
 //                          RoPE fused, loaded one tile ahead into registers so a whole tile is
 //                          in flight per SM; or planar planes times gate planes), split every value into tf32 hi + remainder, and
 //                          write both into the 128-byte-swizzled K-major operand layout of a
 //                          2-stage ring;
-//   warp  8    MMA issuer: one lane issues 24 tcgen05.mma (M128 x N x K8) per tile into one of
+//   MMA issuer, 1 warp   : one lane issues 24 tcgen05.mma (M128 x N x K8) per tile into one of
 //                          two TMEM accumulators and commits to mbarriers;
-//   warps 9-16 epilogue  : tcgen05.ld the accumulator (lane = pixel; two warps per TMEM lane
+//   epilogue, 8 warps    : tcgen05.ld the accumulator (lane = pixel; two warps per TMEM lane
 //                          quadrant, half of the columns each), add bias / activation, store
 //                          planar (coalesced over pixels) or channels-last rows.
 // The weight tile (both halves of the split) is prepared once per CTA and stays in shared memory.
@@ -37,8 +37,12 @@ __device__ inline size_t gemm_src_row(const GemmArgs& g, int m) {
   return (size_t)gemm_src_frame(g, fo) * g.HW + (m - fo * g.HW);
 }
 
-constexpr int TC_THREADS = 544;      // 8 producer warps, 1 MMA warp, 8 epilogue warps
-constexpr int TC_MMA_WARP = 8;
+// Producer warps.  Sixteen have twice the loads and table reads of eight in flight in half the registers a thread (72 against 96, the
+// epilogue's too): additive block 12 x 8 x 64 x 64 x 64 283 -> 267 us a pass, SimpleCSSM gated 128 x 128^2, T = 8 3087 -> 3060.  The stores
+// that multiply planes in place need those registers (DeltaNet 24 x 12 x 32 x 32 x 64: 474 -> 496 with 16, 470 with 8), and so do
+// the ones that skip frames (gated, last frame only: 1 % slower with 16).
+template <bool ZLAST, bool MUL> constexpr int tc_prod_warps = ZLAST || MUL ? 8 : 16;
+template <bool ZLAST, bool MUL> constexpr int tc_threads = (tc_prod_warps<ZLAST, MUL> + 9) * 32;      // + MMA warp, 8 epilogue warps
 constexpr int TC_BM = 128;
 constexpr int TC_K = 64;
 constexpr uint32_t TC_A_HALF = 2u * TC_BM * 128u;      // one of hi / lo: 2 K-blocks x 128 rows x 128 B
@@ -64,7 +68,7 @@ struct TcSmem {
 // kernel carries no extra test.
 // MUL: the first g.mul_n output columns multiply planes in place.
 template <int N, bool A_PLANAR, bool STG, bool ZLAST = false, bool MUL = false>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__((tc_threads<ZLAST, MUL>), 1)
 gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensorMap omap) {
   // tile schedule: round-robin over the CTAs
   const int t_first = blockIdx.x, t_step = gridDim.x, t_end = num_tiles;
@@ -76,7 +80,7 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
   const uint32_t sbase = tc::smem_u32(smem);
   float* bias_s = reinterpret_cast<float*>(smem + L::BIAS_OFF);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-  uint64_t* full = bars;          // [2] A stage written (128 producer arrivals)
+  uint64_t* full = bars;          // [2] A stage written (an arrival a producer warp)
   uint64_t* empty = bars + 2;     // [2] A stage consumed (tcgen05.commit)
   uint64_t* accfull = bars + 4;   // [2] accumulator complete (tcgen05.commit)
   uint64_t* accempty = bars + 6;  // [2] accumulator drained (128 epilogue arrivals)
@@ -84,7 +88,10 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr int NPROD = 256;                        // producer threads that arrive on `full`
+  constexpr int TC_MMA_WARP = tc_prod_warps<ZLAST, MUL>, TC_THREADS = (tc_threads<ZLAST, MUL>);
+  constexpr int NPROD = TC_MMA_WARP * 32;            // producer threads; a lane of each warp arrives on `full`
+  constexpr int TC_ROWS = NPROD / 8;                 // channels-last A: rows of a tile that one round of 16-byte chunks covers
+  constexpr int TC_ITEMS = 2 * TC_BM / TC_ROWS;      // 16-byte chunks of a thread
   constexpr uint32_t TMEM_COLS = (2 * N <= 32) ? 32 : (2 * N <= 64) ? 64 : (2 * N <= 128) ? 128
                                  : (2 * N <= 256) ? 256 : 512;
 
@@ -118,15 +125,15 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
   const uint32_t tmem_base = *tmem_slot;
   pdl_sync();
 
-  if (warp < 8 && tid < NPROD) {
+  if (warp < TC_MMA_WARP) {
     // ================================ producers ================================
     int it = 0;
-    // channels-last mode: the 128 x 16 float4 chunks of a tile are walked in two halves of four
-    // iterations: iteration r covers chunk (tid & 7) + 8*(r >> 2) of row (tid >> 3) + 32*(r & 3),
+    // channels-last mode: the 128 x 16 float4 chunks of a tile are walked in two halves of
+    // TC_ITEMS / 2 iterations: chunk tid & 7 (+ 8 in the second) of rows tid >> 3, + TC_ROWS, ...,
     // so a warp load touches four rows x 128 contiguous bytes.  RoPE only rotates the low channel
     // pairs in most modes: a lane rotates in the half whose chunk holds a rotated pair, which
-    // spreads the rotation evenly over all eight warps.  `pre` always holds the NEXT tile.
-    float4 pre[8];
+    // spreads the rotation evenly over the producer warps.  `pre` always holds the NEXT tile.
+    float4 pre[TC_ITEMS];
     const int chunk_lo = tid & 7, rsub = tid >> 3;
     bool rot[2] = {false, false};
     if (!A_PLANAR) {
@@ -135,9 +142,9 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
       const int m0 = t_first * TC_BM;
       const float* a0 = g.A + gemm_src_row(g, m0 < g.M ? m0 : 0) * TC_K;
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int row = rsub + 32 * (r & 3);
-        const int chunk = chunk_lo + 8 * (r >> 2);
+      for (int r = 0; r < TC_ITEMS; ++r) {
+        const int row = rsub + TC_ROWS * (r % (TC_ITEMS / 2));
+        const int chunk = chunk_lo + 8 * (r / (TC_ITEMS / 2));
         pre[r] = (t_first < t_end && m0 + row < g.M)
                      ? __ldg(reinterpret_cast<const float4*>(a0 + (size_t)row * TC_K + chunk * 4))
                      : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -154,17 +161,17 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
     for (int tile = t_first; tile < t_end; tile += t_step, ++it) {
       const int s = it % NSTAGE;
       const int m0 = tile * TC_BM;
-      float4 cur[8];
+      float4 cur[TC_ITEMS];
       if (!A_PLANAR) {
 #pragma unroll
-        for (int r = 0; r < 8; ++r) cur[r] = pre[r];
+        for (int r = 0; r < TC_ITEMS; ++r) cur[r] = pre[r];
         const int nt = tile + t_step;
         if (nt < t_end) {
           const float* a0 = g.A + gemm_src_row(g, nt * TC_BM) * TC_K;
 #pragma unroll
-          for (int r = 0; r < 8; ++r) {
-            const int row = rsub + 32 * (r & 3);
-            const int chunk = chunk_lo + 8 * (r >> 2);
+          for (int r = 0; r < TC_ITEMS; ++r) {
+            const int row = rsub + TC_ROWS * (r % (TC_ITEMS / 2));
+            const int chunk = chunk_lo + 8 * (r / (TC_ITEMS / 2));
             pre[r] = (nt * TC_BM + row < g.M)
                          ? __ldg(reinterpret_cast<const float4*>(a0 + (size_t)row * TC_K + chunk * 4))
                          : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -183,11 +190,11 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
           t = gemm_rope_t(g, fr);
         }
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          const int row = rsub + 32 * (r & 3);
-          const int chunk = chunk_lo + 8 * (r >> 2);
+        for (int r = 0; r < TC_ITEMS; ++r) {
+          const int row = rsub + TC_ROWS * (r % (TC_ITEMS / 2));
+          const int chunk = chunk_lo + 8 * (r / (TC_ITEMS / 2));
           float4 v = cur[r];
-          if (rot[r >> 2]) {
+          if (rot[r / (TC_ITEMS / 2)]) {
             const int px = px0 + row;
             const int h = (int)(((float)px + 0.5f) * invW);     // exact for px < 2^22
             const int w = px - h * g.W;
@@ -212,31 +219,33 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
           *reinterpret_cast<float4*>(a_lo + off) = l4;
         }
       } else {
-        // thread = (pixel row, K half); planes are contiguous over pixels, so each k is a
+        // thread = (pixel row, part of K); planes are contiguous over pixels, so each k is a
         // coalesced read across the lanes of a warp
         const int row = tid & 127, kh = tid >> 7, m = m0 + row;
-        float v[32];
+        constexpr int KP = TC_K * 128 / NPROD;
+        float v[KP];
         if (m < g.M) {
           const int fo = m / g.HW, px = m - fo * g.HW;
           const int fr = gemm_src_frame(g, fo);
-          const float* ap = g.A + ((size_t)fr * g.a_planes + g.a_plane0 + kh * 32) * g.HW + px;
+          const float* ap = g.A + ((size_t)fr * g.a_planes + g.a_plane0 + kh * KP) * g.HW + px;
 #pragma unroll
-          for (int k = 0; k < 32; ++k) v[k] = __ldg(ap + (size_t)k * g.HW);
+          for (int k = 0; k < KP; ++k) v[k] = __ldg(ap + (size_t)k * g.HW);
           if (g.gate != nullptr) {
-            const float* gp = g.gate + ((size_t)(g.g_compact ? fo : fr) * g.g_planes + g.g_plane0 + kh * 32) * g.HW + px;
+            const float* gp = g.gate + ((size_t)(g.g_compact ? fo : fr) * g.g_planes + g.g_plane0 + kh * KP) * g.HW + px;
 #pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] *= __ldg(gp + (size_t)k * g.HW);
+            for (int k = 0; k < KP; ++k) v[k] *= __ldg(gp + (size_t)k * g.HW);
           }
         } else {
 #pragma unroll
-          for (int k = 0; k < 32; ++k) v[k] = 0.f;
+          for (int k = 0; k < KP; ++k) v[k] = 0.f;
         }
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < KP / 4; ++c) {
           float4 h4, l4;
           tc::split_tf32(v[4 * c + 0], h4.x, l4.x); tc::split_tf32(v[4 * c + 1], h4.y, l4.y);
           tc::split_tf32(v[4 * c + 2], h4.z, l4.z); tc::split_tf32(v[4 * c + 3], h4.w, l4.w);
-          const uint32_t off = (uint32_t)kh * (TC_BM * 128u) + tc::sw128_offset(row, c);
+          const int cg = kh * (KP / 4) + c;
+          const uint32_t off = (uint32_t)(cg >> 3) * (TC_BM * 128u) + tc::sw128_offset(row, cg & 7);
           *reinterpret_cast<float4*>(a_hi + off) = h4;
           *reinterpret_cast<float4*>(a_lo + off) = l4;
         }
@@ -480,7 +489,7 @@ static int launch_tc_v(const GemmArgs& g, const CUtensorMap& map, cudaStream_t s
   // projection of 48 x 4 frames: 104 us in grid order, 139 with the CTAs where SMs came free); 8 x 4 frames and less, and
   // smaller planes, gain more by the early start.  Channels-last input: the second projection of the same rows.
   const PdlOff alone(N == 64 && num_tiles > 8 * sms && (!A_PLANAR || g.HW >= 4096));
-  launch_k(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST, MUL>, grid, TC_THREADS, smem, st, g, num_tiles, map);
+  launch_k(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST, MUL>, grid, (tc_threads<ZLAST, MUL>), smem, st, g, num_tiles, map);
   return check_launch();
 }
 
