@@ -420,6 +420,112 @@ static int launch_stem_quad(const StemArgs& a, cudaStream_t st) {
   return check_launch();
 }
 
+// Stem layer with many input channels and 64 output channels.  The quad form above reads four
+// weight vectors per sixteen multiply-adds, the same 64 bytes for every pixel of the warp, and is bound by
+// those shared-memory reads, the window form still reads 64 bytes a time.  Here a lane owns two
+// channels (a weight read is 256 distinct bytes) of the eight pixels of two neighbouring pool windows; their
+// 4 x 6 input pixels are staged by the warp and read as broadcasts, LayerNorm sums cross the warp.
+// One CTA of twelve warps per SM (weights 147 KB + 6 KB a warp at 64 input channels).
+// For the layers that csrc/stem_tc.cu does not take: a first layer of many input channels, and later ones of callers without
+// room for its split weights.  us a call, the forms below / this one: 8 images of 64x64x64, one layer 184 / 84, 3 of 33x33x48
+// 130 / 23; two layers of 128x128 images, 1 image 189 / 42, 8 200 / 108, 128 1615 / 1158.
+constexpr int STEMP_WARPS = 12;
+__global__ void __launch_bounds__(STEMP_WARPS * 32) stem_layer_pair_kernel(const StemArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int C = SM_MAXC, NT = STEMP_WARPS * 32;
+  const int Cin = a.Cin, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c4 = Cin >> 2;
+  const int nw = 9 * Cin * C;
+  float* vec = sm + nw;                                       // bias, scale, lnbias
+  float4* patch = reinterpret_cast<float4*>(vec + 3 * C) + warp * 24 * c4;      // [4 rows][6 columns][Cin]
+  for (int i = tid; i < nw / 4; i += NT) reinterpret_cast<float4*>(sm)[i] = __ldg(reinterpret_cast<const float4*>(a.wk) + i);
+  for (int i = tid; i < C; i += NT) { vec[i] = a.bk[i]; vec[C + i] = a.scale[i]; vec[2 * C + i] = a.bias[i]; }
+  __syncthreads();
+  pdl_sync();
+  const unsigned long long* w2 = reinterpret_cast<const unsigned long long*>(sm) + lane;      // [tap][ci][32 pairs]
+  const float2 bk = *reinterpret_cast<const float2*>(vec + 2 * lane);
+  const float2 sc = *reinterpret_cast<const float2*>(vec + C + 2 * lane), lb = *reinterpret_cast<const float2*>(vec + 2 * C + 2 * lane);
+  const int pairs = (a.Wo + 1) >> 1;
+  const long long total = (long long)a.N * a.Ho * pairs;
+  for (long long task = (long long)blockIdx.x * STEMP_WARPS + warp; task < total; task += (long long)gridDim.x * STEMP_WARPS) {
+    const int wo = 2 * (int)(task % pairs), ho = (int)((task / pairs) % a.Ho), n = (int)(task / ((long long)pairs * a.Ho));
+    const int h0 = 2 * ho, w0 = 2 * wo;
+    __syncwarp();                                             // the patch of the task before has been read
+    for (int i = lane; i < 24 * c4; i += 32) {
+      const int px = i / c4, k = i - px * c4, r = px / 6, hh = h0 - 1 + r, ww = w0 - 1 + px - 6 * r;
+      patch[i] = (hh >= 0 && hh < a.Hin && ww >= 0 && ww < a.Win)
+                     ? __ldg(reinterpret_cast<const float4*>(a.x + (((size_t)n * a.Hin + hh) * a.Win + ww) * Cin) + k)
+                     : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncwarp();
+    unsigned long long acc[2][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i >> 2][i & 3] = pk2(bk.x, bk.y);
+#pragma unroll 1
+    for (int k = 0; k < c4; ++k) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        float x[6][4];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+          const float4 v = patch[(r * 6 + j) * c4 + k];
+          x[j][0] = v.x; x[j][1] = v.y; x[j][2] = v.z; x[j][3] = v.w;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          unsigned long long xx[6];
+#pragma unroll
+          for (int j = 0; j < 6; ++j) xx[j] = pk2(x[j][e], x[j][e]);
+#pragma unroll
+          for (int y = 0; y < 2; ++y) {
+            const int dy = r - y;                             // tap row that takes input row r to output row y
+            if (dy < 0 || dy > 2) continue;
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+              const unsigned long long w = w2[((dy * 3 + dx) * Cin + 4 * k + e) * 32];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) acc[y][j] = fma2(w, xx[j + dx], acc[y][j]);
+            }
+          }
+        }
+      }
+    }
+    // softplus, LayerNorm (moments of the values minus the pixel's first channel), 2x2 max
+    float2 mx[2] = {make_float2(-INFINITY, -INFINITY), make_float2(-INFINITY, -INFINITY)};
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float v0, v1;
+        upk2(acc[y][j], v0, v1);
+        v0 = softplus_f(v0); v1 = softplus_f(v1);
+        const float vref = __shfl_sync(0xffffffffu, v0, 0);
+        v0 -= vref; v1 -= vref;
+        float s = v0 + v1, ss = fmaf(v0, v0, v1 * v1);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+          s += __shfl_xor_sync(0xffffffffu, s, off); ss += __shfl_xor_sync(0xffffffffu, ss, off);
+        }
+        const float mean = s / (float)C, rinv = rsqrtf(fmaxf(ss / (float)C - mean * mean, 0.f) + 1e-6f);
+        if (h0 + y < a.Hin && w0 + j < a.Win) {               // 'SAME' pool padding on odd sizes
+          mx[j >> 1].x = fmaxf(mx[j >> 1].x, (v0 - mean) * rinv * sc.x + lb.x);
+          mx[j >> 1].y = fmaxf(mx[j >> 1].y, (v1 - mean) * rinv * sc.y + lb.y);
+        }
+      }
+    float* o = a.out + (((size_t)n * a.Ho + ho) * a.Wo + wo) * C + 2 * lane;
+    *reinterpret_cast<float2*>(o) = mx[0];
+    if (wo + 1 < a.Wo) *reinterpret_cast<float2*>(o + C) = mx[1];
+  }
+}
+
+static int launch_stem_layer_pair(const StemArgs& a, size_t smem, cudaStream_t st) {
+  cudaError_t e = func_smem(stem_layer_pair_kernel, smem);
+  if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  const long long need = ((long long)a.N * a.Ho * ((a.Wo + 1) / 2) + STEMP_WARPS - 1) / STEMP_WARPS;
+  const int sms = sm_count();
+  launch_k(stem_layer_pair_kernel, (unsigned)(need < sms ? need : sms), STEMP_WARPS * 32, smem, st, a);
+  return check_launch();
+}
+
 template <int KS>
 static int launch_stem_layer_wide(StemArgs a, cudaStream_t st) {
   const size_t smem = ((size_t)KS * KS * a.Cin * a.C + 3 * (size_t)a.C) * sizeof(float);
@@ -456,6 +562,11 @@ static int launch_stem_layer_cin(const StemArgs& a, cudaStream_t st) {
   if constexpr (CIN > 0)
     if ((a.C == 32 || a.C == 64) && (long long)a.N * a.Ho * a.Wo < (1LL << 31))
       return a.C == 64 ? launch_stem_quad<KS, POOL, CIN, 4>(a, st) : launch_stem_quad<KS, POOL, CIN, 2>(a, st);
+  // many input channels to 64: two channels a lane
+  const size_t pair_smem = wbytes + (3 * (size_t)a.C + STEMP_WARPS * 24 * (size_t)a.Cin) * sizeof(float);
+  if (CIN == 0 && KS == 3 && POOL == 2 && a.C == SM_MAXC && a.Cin % 4 == 0 && wbytes > 64 * 1024 && pair_smem <= 227 * 1024 &&
+      ((reinterpret_cast<uintptr_t>(a.wk) | reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.out)) & 15u) == 0)
+    return launch_stem_layer_pair(a, pair_smem, st);
   // many input channels, pooled: the weight-reusing kernel (needs the weights in shared memory
   // and float4 input reads)
   // it needs one full wave of windows to pay
