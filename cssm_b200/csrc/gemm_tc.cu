@@ -37,12 +37,17 @@ __device__ inline size_t gemm_src_row(const GemmArgs& g, int m) {
   return (size_t)gemm_src_frame(g, fo) * g.HW + (m - fo * g.HW);
 }
 
+// Forms of the epilogue: plain; ZLAST: the output columns from act_n0 on (the z half of the in_proj) are only produced for the
+// last frame of every clip (last-frame-only forward); MUL: the first g.mul_n output columns multiply planes in place; SUB: the
+// channels-last tensor g.sub is subtracted from the rows.  Compile-time variants, so that the plain one carries no extra test.
+enum TcForm { TC_PLAIN, TC_ZLAST, TC_MUL, TC_SUB };
 // Producer warps.  Sixteen have twice the loads and table reads of eight in flight in half the registers a thread (72 against 96, the
 // epilogue's too): additive block 12 x 8 x 64 x 64 x 64 283 -> 267 us a pass, SimpleCSSM gated 128 x 128^2, T = 8 3087 -> 3060.  The stores
 // that multiply planes in place need those registers (DeltaNet 24 x 12 x 32 x 32 x 64: 474 -> 496 with 16, 470 with 8), and so do
-// the ones that skip frames (gated, last frame only: 1 % slower with 16).
-template <bool ZLAST, bool MUL> constexpr int tc_prod_warps = ZLAST || MUL ? 8 : 16;
-template <bool ZLAST, bool MUL> constexpr int tc_threads = (tc_prod_warps<ZLAST, MUL> + 9) * 32;      // + MMA warp, 8 epilogue warps
+// the ones that skip frames (gated, last frame only: 1 % slower with 16) and the rows with a tensor to subtract, whose loads are in
+// flight together (NoGate, with 16 / 8: 60 x 8 x 32 x 32 x 64 300 / 285, 12 x 8 x 64 x 64 x 64 221 / 210, 2 x 8 x 32 x 32 36.0 / 35.5).
+template <TcForm FORM> constexpr int tc_prod_warps = FORM == TC_PLAIN ? 16 : 8;
+template <TcForm FORM> constexpr int tc_threads = (tc_prod_warps<FORM> + 9) * 32;      // + MMA warp, 8 epilogue warps
 constexpr int TC_BM = 128;
 constexpr int TC_K = 64;
 constexpr uint32_t TC_A_HALF = 2u * TC_BM * 128u;      // one of hi / lo: 2 K-blocks x 128 rows x 128 B
@@ -63,12 +68,8 @@ struct TcSmem {
   static constexpr uint32_t TOTAL = BAR_OFF + 128u;
 };
 
-// ZLAST: the output columns from act_n0 on (the z half of the in_proj) are only produced for the
-// last frame of every clip (last-frame-only forward); a compile-time variant so that the default
-// kernel carries no extra test.
-// MUL: the first g.mul_n output columns multiply planes in place.
-template <int N, bool A_PLANAR, bool STG, bool ZLAST = false, bool MUL = false>
-__global__ void __launch_bounds__((tc_threads<ZLAST, MUL>), 1)
+template <int N, bool A_PLANAR, bool STG, TcForm FORM = TC_PLAIN>
+__global__ void __launch_bounds__(tc_threads<FORM>, 1)
 gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensorMap omap) {
   // tile schedule: round-robin over the CTAs
   const int t_first = blockIdx.x, t_step = gridDim.x, t_end = num_tiles;
@@ -88,7 +89,7 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr int TC_MMA_WARP = tc_prod_warps<ZLAST, MUL>, TC_THREADS = (tc_threads<ZLAST, MUL>);
+  constexpr int TC_MMA_WARP = tc_prod_warps<FORM>, TC_THREADS = tc_threads<FORM>;
   constexpr int NPROD = TC_MMA_WARP * 32;            // producer threads; a lane of each warp arrives on `full`
   constexpr int TC_ROWS = NPROD / 8;                 // channels-last A: rows of a tile that one round of 16-byte chunks covers
   constexpr int TC_ITEMS = 2 * TC_BM / TC_ROWS;      // 16-byte chunks of a thread
@@ -320,7 +321,7 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)s * N;
 #pragma unroll 1
       for (int cc = half * (N / 64); cc < (half + 1) * (N / 64); ++cc) {
-        if (ZLAST && cc * 32 >= g.act_n0 && (m / g.HW) % g.T != g.T - 1) continue;   // tile-uniform
+        if (FORM == TC_ZLAST && cc * 32 >= g.act_n0 && (m / g.HW) % g.T != g.T - 1) continue;   // tile-uniform
         uint32_t r[32];
         tc::ld_32x32b_x32(taddr + cc * 32, r);
         tc::wait_ld();
@@ -349,7 +350,7 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
             float vals[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) vals[j] = __uint_as_float(r[j]) + bs[j];
-            if (g.sub != nullptr) {
+            if (FORM == TC_SUB) {
               const float4* sp = reinterpret_cast<const float4*>(g.sub + (size_t)m * g.N + cc * 32);
 #pragma unroll
               for (int j = 0; j < 32; j += 4) {
@@ -395,7 +396,7 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
 #pragma unroll
               for (int j = 0; j < 32; ++j) vals[j] = sigmoid_f(vals[j]);
             }
-            if (MUL && cc * 32 < g.mul_n) {
+            if (FORM == TC_MUL && cc * 32 < g.mul_n) {
               op = g.mul + ((size_t)fr * g.mul_planes + g.mul_plane0 + cc * 32) * g.HW + px;
               float old[32];
 #pragma unroll
@@ -414,7 +415,7 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
               v.y = __uint_as_float(r[j + 1]) + bias_s[cc * 32 + j + 1];
               v.z = __uint_as_float(r[j + 2]) + bias_s[cc * 32 + j + 2];
               v.w = __uint_as_float(r[j + 3]) + bias_s[cc * 32 + j + 3];
-              if (g.sub != nullptr) {
+              if (FORM == TC_SUB) {
                 const float4 sv = __ldg(reinterpret_cast<const float4*>(g.sub + (size_t)m * g.N + cc * 32 + j));
                 v.x -= sv.x; v.y -= sv.y; v.z -= sv.z; v.w -= sv.w;
               }
@@ -448,7 +449,7 @@ bool gemm_tc_supported(const GemmArgs& g, bool a_planar) {
   if (g.HW % TC_BM != 0 || g.M % TC_BM != 0) return false;
   if (g.out_act != 0 && g.act_n0 % 32 != 0) return false;
   if (g.mul != nullptr && (g.mul_n % 32 != 0 || g.N == 64)) return false;
-  if (a_planar && g.N == 192) return false;
+  if (a_planar && (g.N == 192 || (g.sub != nullptr && g.N != 64))) return false;
   return true;
 }
 
@@ -476,24 +477,24 @@ static bool make_out_map(const GemmArgs& g, bool a_planar, CUtensorMap* map) {
   return r == CUDA_SUCCESS;
 }
 
-template <int N, bool A_PLANAR, bool STG, bool ZLAST = false, bool MUL = false>
+template <int N, bool A_PLANAR, bool STG, TcForm FORM>
 static int launch_tc_v(const GemmArgs& g, const CUtensorMap& map, cudaStream_t st) {
   const int num_tiles = g.M / TC_BM;
   const int sms = sm_count();
   cudaError_t e;
   const int grid = num_tiles < sms ? num_tiles : sms;
   const size_t smem = TcSmem<N, STG>::TOTAL + 1024;      // slack for the 1024-byte alignment
-  e = func_smem(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST, MUL>, smem);
+  e = func_smem(gemm_tc_kernel<N, A_PLANAR, STG, FORM>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   // Planes of 64x64: the 64 planes of a tile lie 1 MB apart in all, which neighbouring SMs share (NoGate's output
   // projection of 48 x 4 frames: 104 us in grid order, 139 with the CTAs where SMs came free); 8 x 4 frames and less, and
   // smaller planes, gain more by the early start.  Channels-last input: the second projection of the same rows.
   const PdlOff alone(N == 64 && num_tiles > 8 * sms && (!A_PLANAR || g.HW >= 4096));
-  launch_k(gemm_tc_kernel<N, A_PLANAR, STG, ZLAST, MUL>, grid, (tc_threads<ZLAST, MUL>), smem, st, g, num_tiles, map);
+  launch_k(gemm_tc_kernel<N, A_PLANAR, STG, FORM>, grid, tc_threads<FORM>, smem, st, g, num_tiles, map);
   return check_launch();
 }
 
-template <int N, bool A_PLANAR>
+template <int N, bool A_PLANAR, TcForm FORM = TC_PLAIN>
 static int launch_tc(const GemmArgs& g, cudaStream_t st) {
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
@@ -502,26 +503,17 @@ static int launch_tc(const GemmArgs& g, cudaStream_t st) {
   // the in_proj of cfg2), so that direction keeps direct stores.
   const bool stg = A_PLANAR && N <= 128 && (reinterpret_cast<uintptr_t>(g.out) & 15u) == 0 &&
                    make_out_map(g, A_PLANAR, &map);
-  if (N <= 128 && stg) return launch_tc_v<N, A_PLANAR, (N <= 128)>(g, map, st);
-  return launch_tc_v<N, A_PLANAR, false>(g, map, st);
+  if (N <= 128 && stg) return launch_tc_v<N, A_PLANAR, A_PLANAR && (N <= 128), FORM>(g, map, st);
+  return launch_tc_v<N, A_PLANAR, false, FORM>(g, map, st);
 }
 
 int launch_gemm_tc(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   if (!gemm_tc_supported(g, a_planar)) return CSSM_ERR_UNSUPPORTED;
-  if (g.z_last_only && !a_planar && g.N == 128) {
-    CUtensorMap map;
-    memset(&map, 0, sizeof(map));
-    return launch_tc_v<128, false, false, true>(g, map, st);
-  }
-  if (g.mul != nullptr && !a_planar) {
-    CUtensorMap map;
-    memset(&map, 0, sizeof(map));
-    return g.N == 192 ? launch_tc_v<192, false, false, false, true>(g, map, st) : launch_tc_v<128, false, false, false, true>(g, map, st);
-  }
-  if (!a_planar)
-    return g.N == 192 ? launch_tc<192, false>(g, st)
-                      : g.N == 128 ? launch_tc<128, false>(g, st) : launch_tc<64, false>(g, st);
-  return g.N == 128 ? launch_tc<128, true>(g, st) : launch_tc<64, true>(g, st);
+  if (a_planar)
+    return g.N == 128 ? launch_tc<128, true>(g, st) : g.sub != nullptr ? launch_tc<64, true, TC_SUB>(g, st) : launch_tc<64, true>(g, st);
+  if (g.z_last_only && g.N == 128) return launch_tc<128, false, TC_ZLAST>(g, st);
+  if (g.mul != nullptr) return g.N == 192 ? launch_tc<192, false, TC_MUL>(g, st) : launch_tc<128, false, TC_MUL>(g, st);
+  return g.N == 192 ? launch_tc<192, false>(g, st) : g.N == 128 ? launch_tc<128, false>(g, st) : launch_tc<64, false>(g, st);
 }
 
 int read_tc_error(int* out, int clear) {
