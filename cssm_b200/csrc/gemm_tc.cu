@@ -350,7 +350,7 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
             float vals[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) vals[j] = __uint_as_float(r[j]) + bs[j];
-            if (FORM == TC_SUB) {
+            if (FORM == TC_SUB && g.sub != nullptr) {
               const float4* sp = reinterpret_cast<const float4*>(g.sub + (size_t)m * g.N + cc * 32);
 #pragma unroll
               for (int j = 0; j < 32; j += 4) {
@@ -415,7 +415,7 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
               v.y = __uint_as_float(r[j + 1]) + bias_s[cc * 32 + j + 1];
               v.z = __uint_as_float(r[j + 2]) + bias_s[cc * 32 + j + 2];
               v.w = __uint_as_float(r[j + 3]) + bias_s[cc * 32 + j + 3];
-              if (FORM == TC_SUB) {
+              if (FORM == TC_SUB && g.sub != nullptr) {
                 const float4 sv = __ldg(reinterpret_cast<const float4*>(g.sub + (size_t)m * g.N + cc * 32 + j));
                 v.x -= sv.x; v.y -= sv.y; v.z -= sv.z; v.w -= sv.w;
               }
