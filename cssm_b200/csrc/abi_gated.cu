@@ -326,7 +326,7 @@ static int equal_frames_last(const cssm_gated_desc& d, const cssm_gated_weights&
   if ((s = cssm_gated_gates(&dd, &w, ctx, gm, st)) != CSSM_OK) return s;
   const GatedPlan p = gated_plan_layout(d);
   s = launch_gated_spectral_dft(d.B, Td, d.H, d.W, d.C, (const cf*)((const char*)plan + p.khat), gm, xz, 1, 0, st, nullptr,
-                                d.T - Td + 1, 1);
+                                d.T - Td + 1);
   if (s != CSSM_OK) return s;
   memset(&g, 0, sizeof(g));
   g.M = d.B * d.H * d.W; g.N = d.C; g.K = d.C; g.HW = d.H * d.W;

@@ -20,12 +20,15 @@ namespace cssm {
 struct GatedDftArgs {
   float* xz; const cf* khat; const float4* gates; const float* dchan;
   int B, T, C, P, groups, last_only, mode;        // mode: see launch_spectral
-  int reps, z_first;                              // recurrence steps of frame T - 1; 1: z planes in the first frame of a clip
+  int reps;                                       // EQUAL: recurrence steps of frame T - 1
   size_t region; int ldx, ldc;
   DpGeom g;
 };
 
-template <int RT, int YT, int NT>
+// EQUAL: clips of equal frames, of which the T first are there (launch_gated_spectral_dft).  A variant of its own: the tests and the
+// loop of steps took 0.5 to 5 % of the other blocks' passes (NoGate 367 x 5 x 8 x 8 x 32 88.2 us with, 84.5 without; 22 x 8 x 37 x 16 x 64
+// 121.7, 119.4; gated 16 x 8 x 14 x 14 x 64 86.7, 84.9).
+template <int RT, int YT, int NT, bool EQUAL>
 __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDftArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DpGeom& g = a.g;
@@ -61,8 +64,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
         const cf* kx = a.khat + (size_t)(c0 + pl) * NB + kw;
         float4 g0[YT], g1[YT];
         cf k0[YT], k1[YT];
-        const int reps = t == a.T - 1 ? a.reps : 1;
-        const bool need_k = t > 0 || reps > 1;
+        const int reps = EQUAL && t == a.T - 1 ? a.reps : 1;
+        const bool need_k = t > 0 || (EQUAL && reps > 1);
 #pragma unroll
         for (int e = 0; e < YT; ++e) {
           const int k = min(kr + e, g.Hp - 1), o0 = k * g.Wp, o1 = k == 0 ? 0 : (g.H - k) * g.Wp;
@@ -90,7 +93,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
           if (t > 0) st = ST[k * ldc + x];
           g0[e].x *= dc; g1[e].x *= dc;
           cf h0 = step(g0[e], k0[e], f0[e], mk(st.x, st.y)), h1 = step(g1[e], k1[e], f1[e], mk(st.z, st.w));
-          for (int r = 1; r < reps; ++r) { h0 = step(g0[e], k0[e], f0[e], h0); h1 = step(g1[e], k1[e], f1[e], h1); }
+          if (EQUAL) for (int r = 1; r < reps; ++r) { h0 = step(g0[e], k0[e], f0[e], h0); h1 = step(g1[e], k1[e], f1[e], h1); }
           if (keep) ST[k * ldc + x] = make_float4(h0.x, h0.y, h1.x, h1.y);
           if (emit)
             RA[k * ldc + x] = dp_fold_spec(k == 0 || 2 * k == g.H, mk(g0[e].z * h0.x, g0[e].z * h0.y),
@@ -104,7 +107,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
       float* out = reinterpret_cast<float*>(RA);
       dp_inv_rows<RT, YT, NT>(g, RB, ldx, TW, out, P);
       __syncthreads();
-      const float* zp = (a.z_first ? a.xz + ((size_t)b * a.T * 2 * a.C + c0) * HW : xp) + (size_t)a.C * HW;
+      const float* zp = (EQUAL ? a.xz + ((size_t)b * a.T * 2 * a.C + c0) * HW : xp) + (size_t)a.C * HW;
       dp_store<NT>(g, out, xp, a.mode == 0 ? zp : nullptr, P);
     }
   }
@@ -159,21 +162,26 @@ static size_t gated_dft_bytes(const DpGeom& g, int P, int T) {
 
 bool gated_spectral_dft_fits(int H, int W, int T) { return gated_dft_bytes(dp_geom(H, W), 1, T) <= 226 * 1024; }
 
+template <bool EQUAL>
+static auto pick_kernel(const DpChoice& ch) {
+  return ch.threads == 256 ? (ch.wide ? gated_spectral_dft<2, 4, 256, EQUAL> : gated_spectral_dft<1, 2, 256, EQUAL>)
+                           : (ch.wide ? gated_spectral_dft<2, 4, 128, EQUAL> : gated_spectral_dft<1, 2, 128, EQUAL>);
+}
+
 int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat, const float* gates, float* xz,
-                              int last_only, int mode, cudaStream_t st, const float* dchan, int reps, int z_first) {
+                              int last_only, int mode, cudaStream_t st, const float* dchan, int equal_steps) {
   const DpChoice ch = dp_choose(H, W, C, B, 1, 226 * 1024, gated_dft_bytes, T);
   if (ch.P == 0) return CSSM_ERR_UNSUPPORTED;
   GatedDftArgs a;
   memset(&a, 0, sizeof(a));
   a.xz = xz; a.khat = khat; a.gates = reinterpret_cast<const float4*>(gates); a.dchan = dchan;
   a.B = B; a.T = T; a.C = C; a.P = ch.P; a.last_only = last_only; a.mode = mode;
-  a.reps = reps; a.z_first = z_first;
+  a.reps = equal_steps;
   a.g = dp_geom(H, W);
   a.groups = B * ((C + ch.P - 1) / ch.P);
   a.region = dp_region_bytes(a.g, ch.P);
   a.ldx = dp_ld_rows(a.g, ch.P); a.ldc = dp_ld_cols(a.g, ch.P);
-  auto kern = ch.threads == 256 ? (ch.wide ? gated_spectral_dft<2, 4, 256> : gated_spectral_dft<1, 2, 256>)
-                                : (ch.wide ? gated_spectral_dft<2, 4, 128> : gated_spectral_dft<1, 2, 128>);
+  auto kern = equal_steps > 0 ? pick_kernel<true>(ch) : pick_kernel<false>(ch);
   const int slots = sm_count() * ch.ctas, grid = a.groups < slots ? a.groups : slots;
   const PdlOff alone(uneven_rounds(a.groups, ch.ctas));
   const size_t smem = spread_smem(ch.smem, grid);

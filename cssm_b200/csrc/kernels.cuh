@@ -60,9 +60,10 @@ int launch_spectral(int B, int T, int H, int W, int C, const cf* khat, const flo
 size_t generic_smem_bytes(int H, int W);
 // folded-DFT kernel for any plane size (csrc/gated_spectral_dft.cu); same arguments as launch_spectral
 bool gated_spectral_dft_fits(int H, int W, int T);
-// (reps: times the recurrence step of frame T - 1 is taken; z_first: the z planes are those of the first frame of a clip)
+// (equal_steps > 0: clips of equal frames, of which the T first are there; the recurrence step of frame T - 1 is taken equal_steps
+// times, and the z planes are those of the first frame of a clip)
 int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat, const float* gates, float* xz,
-                              int last_only, int mode, cudaStream_t st, const float* dchan, int reps = 1, int z_first = 0);
+                              int last_only, int mode, cudaStream_t st, const float* dchan, int equal_steps = 0);
 int read_spec_error(int* out, int clear);
 
 // ---- DeltaNet block (scalar delta rule) ----
