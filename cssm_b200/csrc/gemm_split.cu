@@ -211,8 +211,10 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
   // RES: bias of the CTA's N tile; else 32 floats per epilogue warp, filled for every 32-column chunk.
   // (The bias itself is read by scalars: it may sit at any 4-byte offset of a parameter buffer.)
   float* bias_s = reinterpret_cast<float*>(stg + (A_PLANAR ? 8u * 4096u : 0u));
-  float* ss_s = bias_s + 256;                                     // [GS_SS][2][128] row sums (RMS prologue)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ss_s + (A_PLANAR && g.rms_scale != nullptr ? GS_SS * 256 : 0));
+  // (barriers before the row sums, which not every launch has: with their address depending on that, the short launches of 392 to
+  // 5880 rows and 288 to 512 channels took 2 to 5 % of the ungated block's pass longer)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(bias_s + 256);
+  float* ss_s = bias_s + 256 + 32;                                // [GS_SS][2][128] row sums (RMS prologue alone has room for them)
   uint64_t* full = bars;           // [4] block written (8 producer warps)
   uint64_t* empty = bars + 4;      // [4] block consumed (tcgen05.commit)
   uint64_t* accfull = bars + 8;    // [2] accumulator set complete (tcgen05.commit)
