@@ -675,17 +675,26 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   }
   const bool wide = q.nl > 1;
   const int bn_tmem = 512 / (1 + q.nl) / 32 * 32;
+  // Planar A, weights split by the producers: tiles of 96 or 128 columns, by rounds over the SMs, a tile of bn columns taking as long
+  // as bn + 30 of them.  us a pass of the ungated block, K = N, 96- / 128-column tiles: 384 channels, 5880 rows 83 / 64, 13916
+  // 135 / 151, 29988 313 / 295; 448 channels, 20972 288 / 300, 55860 689 / 697; 512 channels, 5880 105 / 119, 13916 245 / 206.
+  const int sms = sm_count();
+  auto rounds = [&](int bn) { return (((long long)q.m_tiles * ((g.N + bn - 1) / bn) + sms - 1) / sms) * (bn + 30); };
   int nt = q.nl > 0 ? (g.N + 127) / 128 : (g.N + 255) / 256;
   while (round32((g.N + nt - 1) / nt) > 32 && res_size(round32((g.N + nt - 1) / nt)) + 2 * GS_A_BYTES + fixed > LIMIT) ++nt;
   q.BN = round32((g.N + nt - 1) / nt);
   const bool res = !wide && g.wsplit == nullptr && (q.BN >= 64 || nt == 1) && res_size(q.BN) + 2 * GS_A_BYTES + fixed <= LIMIT;
   if (!res) {
-    int most = g.rms_scale != nullptr ? 96 : 128;        // the row sums leave no room for two stages of 128 columns
-    if (most > bn_tmem) most = bn_tmem;
-    nt = (g.N + most - 1) / most;
-    q.BN = round32((g.N + nt - 1) / nt);
+    // (the row sums of the RMS prologue leave no room for two stages of 128 columns)
+    auto width = [&](int most) {
+      most = most < bn_tmem ? most : bn_tmem;
+      const int n = (g.N + most - 1) / most;
+      return round32((g.N + n - 1) / n);
+    };
+    q.BN = width(g.rms_scale != nullptr ? 96 : 128);
+    if (a_planar && g.wsplit == nullptr && rounds(width(96)) < rounds(q.BN)) q.BN = width(96);
+    nt = (g.N + q.BN - 1) / q.BN;
   }
-  const int sms = sm_count();
   cudaError_t e;
   // few row tiles: narrower column tiles until two thirds of the SMs have one (each CTA then splits
   // fewer weights too; the row tile is split once more per column tile, which idle SMs do for free)
