@@ -558,10 +558,15 @@ static int launch_stem_layer_v(StemArgs a, cudaStream_t st) {
 template <int KS, int POOL, int CIN>
 static int launch_stem_layer_cin(const StemArgs& a, cudaStream_t st) {
   const size_t wbytes = (size_t)KS * KS * a.Cin * a.C * sizeof(float);
-  // 1 or 3 input channels to 32 or 64: four conv pixels a quad
-  if constexpr (CIN > 0)
-    if ((a.C == 32 || a.C == 64) && (long long)a.N * a.Ho * a.Wo < (1LL << 31))
+  // 1 or 3 input channels to 32 or 64: four conv pixels a quad.  At 64 channels a quad's four pixels are a longer chain than the one of
+  // the kernel below: only where three SMs in four get a CTA of 256 pixels.  us a launch here / below, 64 channels: clips of
+  // 32x32x3, pointwise, 8 frames 6.2 / 4.2, 16 6.2 / 5.3, 32 6.2 / 6.2, 8 of 128x128x3 12.4 / 14.5; images of 128x128x1, 3x3, one
+  // 7.2 / 6.3, two 7.3 / 10.3, of 32x32x3, 8 images 10.4 / 8.3, 32 images 10.4 / 16.5.  At 32 channels never behind.
+  if constexpr (CIN > 0) {
+    const long long outs = (long long)a.N * a.Ho * a.Wo, ctas = (outs * (POOL == 2 ? 4 : 1) + 255) / 256;
+    if (outs < (1LL << 31) && (a.C == 32 || (a.C == 64 && 4 * ctas >= 3LL * sm_count())))
       return a.C == 64 ? launch_stem_quad<KS, POOL, CIN, 4>(a, st) : launch_stem_quad<KS, POOL, CIN, 2>(a, st);
+  }
   // many input channels to 64: two channels a lane
   const size_t pair_smem = wbytes + (3 * (size_t)a.C + STEMP_WARPS * 24 * (size_t)a.Cin) * sizeof(float);
   if (CIN == 0 && KS == 3 && POOL == 2 && a.C == SM_MAXC && a.Cin % 4 == 0 && wbytes > 64 * 1024 && pair_smem <= 227 * 1024 &&
@@ -578,8 +583,8 @@ static int launch_stem_layer_cin(const StemArgs& a, cudaStream_t st) {
   if (CIN == 0 && wbytes > 64 * 1024)
     return a.C == SM_MAXC ? launch_stem_layer_v<KS, POOL, 0, true, 1024>(a, st)
                           : launch_stem_layer_v<KS, POOL, 0, false, 1024>(a, st);
-  if (CIN == 0 && a.C == SM_MAXC) return launch_stem_layer_v<KS, POOL, 0, true, STEM_THREADS>(a, st);
-  return launch_stem_layer_v<KS, POOL, CIN, false, STEM_THREADS>(a, st);
+  return a.C == SM_MAXC ? launch_stem_layer_v<KS, POOL, CIN, true, STEM_THREADS>(a, st)
+                        : launch_stem_layer_v<KS, POOL, CIN, false, STEM_THREADS>(a, st);
 }
 
 template <int KS, int POOL>

@@ -50,3 +50,20 @@ def test_first_layer_of_many_channels(E, shape):
     x = np.random.default_rng(shape[3]).standard_normal(shape).astype(np.float32)
     ref = np.asarray(so.stem_forward(p, x.astype(np.float64), stem_mode="default", stem_layers=1))
     assert orc.rel_l2(b.stem(torch.from_numpy(x).cuda()).cpu().numpy().reshape(ref.shape), ref) <= 5e-6
+
+
+# three quarters of 148 SMs with a CTA of 256 pixels: 111 CTAs (the first of each pair has 108)
+@pytest.mark.parametrize("stem,shape", [("default", (3, 96, 96, 1)), ("default", (3, 96, 98, 1)), ("default", (3, 96, 98, 3)), ("default", (1, 9, 7, 3)),
+                                        ("pathtracker", (1, 27, 32, 32, 3)), ("pathtracker", (1, 28, 32, 32, 3)), ("pathtracker", (2, 1, 5, 3, 1))])
+def test_first_layer_of_few_and_many_pixels(stem, shape):
+    clip = stem == "pathtracker"
+    m = SimpleCSSM(cssm_type="gated", embed_dim=64, kernel_size=1, pos_embed="none", seq_len=shape[1] if clip else 1, stem_mode=stem,
+                   stem_layers=1, gate_type="factored", pool_type="max")
+    H, W = m.feature_hw(*shape[-3:-1])
+    bkw = dict(kernel_size=1, rope_mode="none", gate_type="factored", short_conv_size=4, short_conv_spatial_size=3)
+    p = so.init_simple_params(3, cin=shape[-1], embed_dim=64, H=H, W=W, num_classes=2, cssm_type="gated", stem_mode=stem, stem_layers=1,
+                              bias_scale=0.1, block_kwargs=bkw)
+    x = np.random.default_rng(shape[-2]).random(shape).astype(np.float32)
+    got = m.bind({"params": p}).stem(torch.from_numpy(x).cuda()).cpu().numpy()
+    ref = np.asarray(so.stem_forward(p, x.reshape(-1, *shape[-3:]).astype(np.float64), stem_mode=stem, stem_layers=1)).reshape(got.shape)
+    assert orc.rel_l2(got, ref) <= 5e-6
