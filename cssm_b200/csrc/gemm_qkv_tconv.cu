@@ -204,7 +204,8 @@ __global__ void __launch_bounds__(QT_THREADS, 1) gemm_qkv_tconv_kernel(const __g
         const float2 gv = a.bkv != nullptr ? __ldg(a.bkv + frame * g.HW + px) : make_float2(1.f, 1.f);
         if (__any_sync(0xffffffffu, !tc::mbar_wait(&accfull[n & 1], (n >> 1) & 1))) { atomicExch(&g_qt_error, 4); ok = false; break; }
         tc::fence_after_sync();
-        const int back = t < 3 ? t : 3;                                     // earlier frames of this clip that count
+        // earlier frames of this clip under the taps (frames further back may hold anything: no product with a zero tap)
+        const int back = t < a.kt - 1 ? t : a.kt - 1;
         uint32_t sl[4];                                                     // ring slots of t, t - 1, t - 2, t - 3
 #pragma unroll
         for (int d = 0; d < 4; ++d) sl[d] = (uint32_t)(slot >= d ? slot - d : slot - d + QT_RING) * QT_N;

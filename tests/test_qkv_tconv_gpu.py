@@ -67,3 +67,28 @@ def test_image_held_for_several_frames():
     ref = so.simple_forward(p, x[:2], cssm_type="gdn", seq_len=5, stem_mode="default", stem_layers=1, pool_type="max", block_kwargs=bkw)
     assert orc.rel_l2(got, few) <= 1e-5
     assert orc.rel_l2(got[:2], ref) <= 1e-4
+
+
+@pytest.mark.parametrize("kt", [1, 2, 3])
+def test_frames_behind_the_taps(kt):
+    """A channel that q alone reads overflows in frame 0: q of frames 0 .. kt - 1 is not finite, and from frame kt on nothing may remember it."""
+    kw = dict(delta_key_dim=4, kernel_size=3, gate_type="factored", short_conv_size=kt)
+    B, T, c = 37, 6, 5
+    x = np.random.default_rng(kt).standard_normal((B, T, 32, 32, 64)).astype(np.float32)
+    p = orc.init_gdn_params(kt, 64, 32, 32, bias_scale=0.1, **kw)
+    for name, leaf in p.items():
+        if isinstance(leaf, dict) and "kernel" in leaf and leaf["kernel"].ndim == 2 and leaf["kernel"].shape[0] == 64 and name != "output_proj":
+            w = np.array(leaf["kernel"])
+            w[c] = 0
+            if name == "qkv_proj":
+                w[c, :64] = 100
+            leaf["kernel"] = w
+    x[:, 0, :, :, c] = 0
+    m = GatedDeltaNetCSSM(channels=64, rope_mode="none", qkv_conv_size=1, **kw).bind({"params": p})
+    want = m(torch.from_numpy(x).cuda()).clone()
+    x[:, 0, 3, 7, c] = 1e38
+    got = m(torch.from_numpy(x).cuda())
+    assert bool(want.isfinite().all())
+    assert not bool(got[:, 0].isfinite().all())
+    assert torch.equal(got[:, kt:], want[:, kt:])
+    assert device_error() == 0
