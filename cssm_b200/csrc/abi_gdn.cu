@@ -44,6 +44,11 @@ __global__ void __launch_bounds__(256) gdn_kv_gate_kernel(float* __restrict__ qk
   *d = v;
 }
 
+// Channel gates: k and v multiplied where they lie by the projection that makes the gates.  At 64 channels and planes of whole tiles
+// that is gemm_tc's store (DeltaNet 24 x 12 x 32 x 32 x 64: 34 us less than with a launch that reads and writes k, v and the gates
+// again); in gemm_split_kernel the loads of k and v sit on the epilogue's chain (12 x 8 x 28 x 28 x 64: 273 against 267 us a pass).
+static bool kv_gates_in_place(const cssm_gdn_desc& d) { return gemm_tc_in_place(d.C, 2 * d.C, d.H * d.W, 2 * d.C); }
+
 struct GdnWs { size_t xdw, qkv, gate, ctx_part, ab, bkv, gsp, state, total; };
 static GdnWs gdn_ws_layout(const cssm_gdn_desc& d) {
   GdnWs l;
@@ -58,8 +63,9 @@ static GdnWs gdn_ws_layout(const cssm_gdn_desc& d) {
   const bool chan = d.gate_type == CSSM_GATE_CHANNEL;
   l.ab = off;       off += round_up(BT * (chan ? nh : 1) * NB * sizeof(float2), 256);
   l.bkv = off;      off += round_up(BT * HW * sizeof(float2), 256);
-  l.gsp = off;      off += (chan && d.use_input_gates) ? round_up(BT * 2 * d.C * HW * sizeof(float), 256) : 0;
-  l.state = off;    off += round_up((size_t)d.B * nh * dk * dk * NB * sizeof(cf), 256);
+  l.gsp = off;      off += (chan && d.use_input_gates && !kv_gates_in_place(d)) ? round_up(BT * 2 * d.C * HW * sizeof(float), 256) : 0;
+  // (the 32x32 kernels keep the states in registers)
+  l.state = off;    off += gdn_path(d) == PATH_R32 ? 0 : round_up((size_t)d.B * nh * dk * dk * NB * sizeof(cf), 256);
   l.total = off;
   return l;
 }
@@ -333,15 +339,11 @@ int cssm::gdn_forward_internal(const cssm_gdn_desc* d, const cssm_gdn_weights* w
     g.T = Tdata; g.H = d->H; g.W = d->W;
     g.out_act = 2; g.act_n0 = 0;
     if (((size_t)C * HW) % 8 != 0) return CSSM_ERR_UNSUPPORTED;
-    // Multiplied in the projection's store where gemm_tc takes it (DeltaNet 24 x 12 x 32 x 32 x 64: 34 us less than with a launch
-    // that reads and writes k, v and the gates again); in gemm_split_kernel the loads of k and v sit on the epilogue's
-    // chain (12 x 8 x 28 x 28 x 64: 273 against 267 us a pass).
-    g.mul = qkv; g.mul_planes = 3 * C; g.mul_plane0 = C; g.mul_n = 2 * C;
-    const bool in_store = gemm_tc_supported(g, false);
-    if (!in_store) g.mul = nullptr;
+    const bool in_place = kv_gates_in_place(*d);      // (no gate planes then: gsp has no room)
+    if (in_place) { g.mul = qkv; g.mul_planes = 3 * C; g.mul_plane0 = C; g.mul_n = 2 * C; }
     if ((s = launch_gemm<false, true>(g, st)) != CSSM_OK) return s;
     const size_t per_frame4 = (size_t)2 * C * HW / 4, total4 = per_frame4 * BT;
-    if (!in_store) {
+    if (!in_place) {
       launch_k(gdn_kv_gate_kernel, (unsigned)((total4 + 255) / 256), 256, 0, st, qkv, gsp, per_frame4, total4);
       if ((s = check_launch()) != CSSM_OK) return s;
     }

@@ -43,6 +43,8 @@ struct GemmArgs {
 
 // Two tf32 parts, K = 64 only; three bf16 parts, any size.
 bool gemm_tc_supported(const GemmArgs& g, bool a_planar);
+// whether gemm_tc takes a channels-last (M, K) by (K, N) projection of frames of HW pixels that multiplies planes in place (mul)
+bool gemm_tc_in_place(int K, int N, int HW, int mul_n);
 int launch_gemm_tc(const GemmArgs& g, bool a_planar, cudaStream_t st);
 int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st);
 // The weights of up to two projections (K, N0), (K, N1) split once for all CTAs of their launches, in the layout of an operand

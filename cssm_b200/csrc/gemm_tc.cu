@@ -439,6 +439,10 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
   }
 }
 
+bool gemm_tc_in_place(int K, int N, int HW, int mul_n) {
+  return K == TC_K && (N == 128 || N == 192) && HW % TC_BM == 0 && mul_n % 32 == 0;
+}
+
 // Whether this kernel takes the problem (else gemm_split_kernel, csrc/gemm_split.cu): 64 channels, tiles
 // inside one frame, no RMS prologue.  Splitting into two tf32 parts costs the producers half of what
 // three bf16 parts do, and at K = 64 the producers set the pace: in_proj of 4.2 M rows 649 against
@@ -448,7 +452,7 @@ bool gemm_tc_supported(const GemmArgs& g, bool a_planar) {
   if (g.K != TC_K || (g.N != 64 && g.N != 128 && g.N != 192)) return false;
   if (g.HW % TC_BM != 0 || g.M % TC_BM != 0) return false;
   if (g.out_act != 0 && g.act_n0 % 32 != 0) return false;
-  if (g.mul != nullptr && (g.mul_n % 32 != 0 || g.N == 64)) return false;
+  if (g.mul != nullptr && !gemm_tc_in_place(g.K, g.N, g.HW, g.mul_n)) return false;
   if (a_planar && (g.N == 192 || (g.sub != nullptr && g.N != 64))) return false;
   return true;
 }
