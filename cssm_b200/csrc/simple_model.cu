@@ -534,7 +534,8 @@ static int launch_stem_layer_wide(StemArgs a, cudaStream_t st) {
   const long long total = (long long)a.N * a.Ho * a.Wo;
   const long long per_cta = (STEMW_THREADS / 32) * 8;
   const long long need = (total + per_cta - 1) / per_cta;
-  launch_k(stem_layer_wide_kernel<KS>, (unsigned)(need < 148 ? need : 148), STEMW_THREADS, smem, st, a);
+  const int sms = sm_count();
+  launch_k(stem_layer_wide_kernel<KS>, (unsigned)(need < sms ? need : sms), STEMW_THREADS, smem, st, a);
   return check_launch();
 }
 
@@ -549,7 +550,7 @@ static int launch_stem_layer_v(StemArgs a, cudaStream_t st) {
   const long long per_cta = (NT / 32) * (POOL == 2 ? 2 : 8);
   const long long need = (total + per_cta - 1) / per_cta;
   // a few resident waves of CTAs that loop, so that the per-CTA weight staging is amortised
-  const long long cap = NT == 1024 ? 148 : 148 * 16;
+  const long long cap = sm_count() * (NT == 1024 ? 1LL : 16LL);
   const unsigned grid = (unsigned)(need < cap ? need : cap);
   launch_k(stem_layer_kernel<KS, POOL, CIN, FULLC, NT>, grid, NT, smem, st, a);
   return check_launch();
@@ -577,7 +578,7 @@ static int launch_stem_layer_cin(const StemArgs& a, cudaStream_t st) {
   // it needs one full wave of windows to pay
   const long long windows = (long long)a.N * a.Ho * a.Wo;
   if (CIN == 0 && POOL == 2 && a.Cin % 4 == 0 && a.Cin >= 16 && wbytes <= 200 * 1024 &&
-      windows >= 148LL * (STEMW_THREADS / 32) * 8)
+      windows >= (long long)sm_count() * (STEMW_THREADS / 32) * 8)
     return launch_stem_layer_wide<KS>(a, st);
   // otherwise: weights beyond 64 KB leave room for one CTA per SM only, give that CTA 32 warps
   if (CIN == 0 && wbytes > 64 * 1024)
