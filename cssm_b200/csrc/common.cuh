@@ -102,8 +102,8 @@ __device__ __forceinline__ void pdl_sync() { pdl_wait(); pdl_trigger(); }
 
 // A launch that waits for everything before it, also inside a scope, for persistent kernels of many rounds: in an overlapped
 // launch the CTAs take SMs in the order in which those come free, so neighbours in the grid, which work on neighbouring
-// tiles, sit far apart, and the CTAs that have a round more than others end up two on an SM (25 GDN clips of 12 frames,
-// 400 heads for 296 CTAs: the pass 809 us, 738 so).
+// tiles, sit far apart, and the CTAs that have a round more than others end up two on an SM (24 DeltaNet clips of 8 frames of
+// 28x28x64: the pass 451 us, 429 so; 10 of 40x40x64: 463, 447).
 struct PdlOff {
   int prev;
   explicit PdlOff(bool off) : prev(g_pdl) { if (off && g_pdl == 2) g_pdl = 1; }

@@ -190,7 +190,6 @@ int launch_gdn_spectral_r32(const GdnSpectralArgs& a, cudaStream_t st) {
   const int heads = a.B * (a.C / 4), sms = sm_count();
   const cudaError_t e = func_smem(gdn_spectral_r32, G32_SMEM_BYTES);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  const PdlOff alone(uneven_rounds(heads, 1));
   launch_k(gdn_spectral_r32, heads < sms ? heads : sms, G32_THREADS, G32_SMEM_BYTES, st, a);
   return check_launch();
 }
