@@ -649,7 +649,9 @@ int cssm_device_error(int* out, int clear);
 /* cssm_gdn_forward with per-stage timing: `stage_events` is an array of 8 cudaEvent_t created by
  * the caller; events[i] is recorded on `stream` before stage i (0 dwconv+ctx, 1 qkv_proj,
  * 2 gate_proj, 3 gates, 4 short convs, 5 fused spectral kernel, 6 norm+gate+output_proj) and
- * events[7] at the end.  Nothing is kept after the call returns. */
+ * events[7] at the end.  Where the projection and the temporal conv are one launch (64 channels, 1 to 4 taps, H*W a
+ * multiple of 128, B*H*W / 64 at least twice the SM count), stage 1 is empty and
+ * stage 4 holds both.  Nothing is kept after the call returns. */
 int cssm_gdn_forward_timed(const cssm_gdn_desc* d, const cssm_gdn_weights* w, const void* plan,
                            const float* x, float* y, void* workspace, size_t workspace_bytes,
                            void* stream, void** stage_events);
