@@ -269,7 +269,10 @@ bool gemm_qkv_tconv_supported(const GemmArgs& g, int kt) {
   if (g.K != 64 || g.N != 192 || g.HW % QT_BM != 0 || g.T <= 0 || g.M % g.HW != 0 || g.M / g.HW % g.T != 0 || kt < 1 || kt > 4 ||
       g.bias == nullptr || g.o_planes != 192 || g.o_plane0 != 0)
     return false;
-  // a sequence of T steps is the unit of work: with fewer than two for every SM the tiles of two launches spread better
+  // A sequence of T steps is the unit of work and cannot be split.  From two for every SM on the joined launch is ahead wherever the
+  // last round ends (three rounds for the work of 2.05 included).  GDN block, us a pass, two launches / this one: 32x32, T = 8, 19
+  // clips (304 sequences) 306 / 288, 20 310 / 294, 23 331 / 310, 27 380 / 331, 28 412 / 382, 38 533 / 478, 120 1463 / 1263; T = 1, 19
+  // clips 82.8 / 71.7; T = 32, 19 1046 / 1001; 64x64, T = 8, 5 clips (320) 460 / 439, 10 874 / 816; 16x16, T = 4, 80 clips (320) 260 / 248.
   return sequences(g) >= 2 * sm_count() && sequences(g) < (1LL << 31) && sm_count() > 1;
 }
 
