@@ -115,10 +115,11 @@ int cssm_gated_forward(const cssm_gated_desc* d, const cssm_gated_weights* w,
  * src/models/cssm_shvit.py:214).  The recurrence still runs over all T steps; the inverse
  * transforms, the SiLU(z) gate, the stores and the out_proj of the earlier frames are skipped.
  * Same plan and workspace as cssm_gated_forward.  C > 192: with
- * 12288 * ceil(C / 64) * (ceil(2 C / 32) + ceil(C / 32)) bytes more in workspace_bytes (16-byte
- * aligned like the rest), the weights of the two projections are split once into that room instead of by every
- * CTA (14 x 14 planes, T = 4: 12 clips of 384 channels 134 -> 107 us, 100 of 512 1366 -> 979);
- * results differ from those of a call without it by float32 rounding (bound tested: 4e-6 of the 2-norm).  A caller that compares calls bit by bit gives all of them the same workspace_bytes. */
+ * 12288 * ceil(C / 64) * (ceil(2 C / 32) + ceil(C / 32)) bytes more in workspace_bytes, the
+ * weights of the two projections are split once into that room instead of by every CTA (14 x 14
+ * planes, T = 4: 12 clips of 384 channels 134 -> 107 us, 100 of 512 1366 -> 979);
+ * results differ from those of a call without it by float32 rounding (bound tested: 4e-6 of the
+ * 2-norm).  A caller that compares calls bit by bit gives all of them the same workspace_bytes. */
 int cssm_gated_forward_last(const cssm_gated_desc* d, const cssm_gated_weights* w,
                             const void* plan, const float* x, float* y_last,
                             void* workspace, size_t workspace_bytes, void* stream);
