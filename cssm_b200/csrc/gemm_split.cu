@@ -194,7 +194,10 @@ int launch_split_weights(int K, const float* w0, int N0, void* out0, const float
 }
 
 // GATE: planar A times the gate planes.  WIDE: more than one leading accumulator (nl > 1).
-template <bool A_PLANAR, bool RES, bool GATE, bool WIDE>
+// PRE (channels-last A): weights split beforehand.  Planar A without gate planes tests wsplit at run time, with gate planes there never is
+// one: where the test is not needed it costs (GDN 100 x 2 x 14 x 14 x 384 1577 us a pass with it in the gated form, 1556 without;
+// gated 1 x 2 x 14 x 14 x 384 62.1 / 60.7 in the channels-last one), and planar A is not better off with a variant of its own.
+template <bool A_PLANAR, bool RES, bool GATE, bool WIDE, bool PRE = false>
 __global__ void __launch_bounds__(GS_THREADS, 1)
 gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ CUtensorMap omap,
                   const __grid_constant__ SplitArgs again) {
@@ -204,6 +207,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
   const uint32_t sbase = tc::smem_u32(smem);
   const uint32_t BN = (uint32_t)q.BN, b_part = BN * 128u, b_block = 3u * b_part;
   const int NS = q.stages, kblocks = q.kblocks;
+  const bool pre_split = (PRE || (A_PLANAR && !RES && !GATE)) && g.wsplit != nullptr;
   const uint32_t res_bytes = RES ? (uint32_t)kblocks * b_block : 0u;
   const uint32_t stage_bytes = GS_A_BYTES + (RES ? 0u : b_block);
   unsigned char* ring = smem + res_bytes;
@@ -230,7 +234,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
   while (tmem_cols < (uint32_t)bufs * acc_cols) tmem_cols <<= 1;
 
   if (tid == 0) {
-    for (int s = 0; s < NS; ++s) { tc::mbar_init(&full[s], GS_PROD / 32 + (!RES && g.wsplit != nullptr ? 1 : 0)); tc::mbar_init(&empty[s], 1); }
+    for (int s = 0; s < NS; ++s) { tc::mbar_init(&full[s], GS_PROD / 32 + (pre_split ? 1 : 0)); tc::mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; ++a) { tc::mbar_init(&accfull[a], 1); tc::mbar_init(&accempty[a], 8); }
     tc::mbar_init(done, 1);
     tc::fence_mbar_init();
@@ -416,7 +420,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
         if (g.rms_scale != nullptr && nkb == 0) { ss_s[((tcnt % GS_SS) * 2 + kh) * 128 + prow] = ss; ss = 0.f; }
         if (ntile < num_tiles) fetch(ntile, nkb);
       }
-      if (!RES && g.wsplit != nullptr) {
+      if (pre_split) {
         if (tid == 0) {                                 // (it has waited for the stage above)
           unsigned char* b_s = a_s + GS_A_BYTES;
           const int grp0 = (tile % q.n_tiles) * (q.BN >> 5), grps = min(q.BN >> 5, ((g.N + 31) >> 5) - grp0);
@@ -659,7 +663,7 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   q.fdiv = FastDiv(g.a_fdiv > 1 ? g.a_fdiv : 1);
   constexpr size_t LIMIT = 227 * 1024;
   const size_t fixed = 1024 + 1024 + 128 + (a_planar ? 8 * 4096 + (g.rms_scale != nullptr ? GS_SS * 1024 : 0) : 0);   // slack, bias, barriers, staging, sums
-  if (g.wsplit != nullptr && (g.rms_scale != nullptr || !aligned16(g.wsplit))) return CSSM_ERR_UNSUPPORTED;
+  if (g.wsplit != nullptr && (g.rms_scale != nullptr || g.gate != nullptr || !aligned16(g.wsplit))) return CSSM_ERR_UNSUPPORTED;
   auto round32 = [](int v) { return (v + 31) / 32 * 32; };
   auto res_size = [&](int bn) { return (size_t)q.kblocks * 3 * bn * 128; };
   // Weights resident when a tile of at least 64 columns (or all of N) leaves room for two A stages:
@@ -732,6 +736,8 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   if (wide)
     kern = a_planar ? (gate ? gemm_split_kernel<true, false, true, true> : gemm_split_kernel<true, false, false, true>)
                     : gemm_split_kernel<false, false, false, true>;
+  if (g.wsplit != nullptr && !a_planar)
+    kern = wide ? gemm_split_kernel<false, false, false, true, true> : gemm_split_kernel<false, false, false, false, true>;
   e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   launch_k(kern, grid, GS_THREADS, smem, st, g, q, map, SplitArgs{g, q});

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 # steps below, at and above the number of temporal taps; no temporal conv; spatial conv of 0, 3 and 5 taps; a plane a warp and a CTA
 @pytest.mark.parametrize("T", [2, 3, 4, 5, 9])
-@pytest.mark.parametrize("kt,ksp,side", [(4, 3, (22, 34)), (0, 3, (22, 34)), (1, 0, (20, 20)), (2, 3, (20, 20)), (3, 3, (90, 88))])
+@pytest.mark.parametrize("kt,ksp,side", [(4, 3, (22, 34)), (0, 3, (22, 34)), (1, 0, (20, 20)), (2, 3, (20, 20)), (3, 3, (90, 88)), (5, 5, (20, 24))])
 @pytest.mark.parametrize("gate", ["factored", "dense"])
 def test_last_frame_of_a_repeated_image(T, kt, ksp, side, gate):
     E = 16

@@ -58,7 +58,8 @@ def test_small_conv(B, Hi, Wi, Cin, Cout):
 
 @pytest.mark.parametrize("C,side", [(64, 9), (96, 5), (128, 28), (256, 6), (384, 7), (512, 3)])
 def test_fc1_with_its_layernorm(C, side):
-    """A ConvBlock of one image: LayerNorm inside the GEMM for every number of steps a warp takes, against the oracle."""
+    """A ConvBlock of one image against the oracle: LayerNorm inside the GEMM (128 and 256 channels: one step of K for each of four and
+    eight warps), in a launch of its own (96, 384 and 512), and the fused Mlp (64)."""
     from cssm_b200.shvit import CSSMSHViT
     from oracle import shvit_oracle as sv
     rng = np.random.default_rng(C)
@@ -70,4 +71,19 @@ def test_fc1_with_its_layernorm(C, side):
     net = CSSMSHViT(num_classes=10, num_timesteps=1, short_conv_spatial_size=0, **kw)
     got = net.apply({"params": p, "batch_stats": s}, x.cuda()).float().cpu().numpy()
     want = sv.shvit_forward(p, s, x.float().numpy().astype(np.float64), num_timesteps=1, **kw)
+    assert float(np.abs(got - want).max() / max(np.abs(want - want.mean()).max(), 1e-30)) <= 2e-2
+
+
+@pytest.mark.parametrize("side", [3, 9])
+def test_fc1_with_its_layernorm_two_warps_a_tile(side):
+    """64 channels in a mixer block, whose Mlp has a depthwise conv in it and so does not run in the fused kernel."""
+    from cssm_b200.shvit import CSSMSHViT
+    from oracle import shvit_oracle as sv
+    kw = dict(embed_dims=(64,) * 4, depths=(1, 1, 1, 1), kernel_sizes=(1, 1, 1, 1), use_cssm_stages=(True,) * 4)
+    hw = (4 * side, 4 * side)
+    p, s = sv.init_shvit_params(5, hw, num_classes=10, short_conv_spatial_size=0, **kw)
+    x = torch.from_numpy(np.random.default_rng(side).standard_normal((1, *hw, 3)).astype(np.float32)).to(torch.bfloat16)
+    net = CSSMSHViT(num_classes=10, num_timesteps=1, short_conv_spatial_size=0, **kw)
+    got = net.apply({"params": p, "batch_stats": s}, x.cuda()).float().cpu().numpy()
+    want = sv.shvit_forward(p, s, x.float().numpy().astype(np.float64), num_timesteps=1, short_conv_spatial_size=0, **kw)
     assert float(np.abs(got - want).max() / max(np.abs(want - want.mean()).max(), 1e-30)) <= 2e-2
