@@ -20,9 +20,9 @@ namespace cssm {
 struct GatedDftArgs {
   float* xz; const cf* khat; const float4* gates; const float* dchan;
   int B, T, C, P, groups, last_only, mode;        // mode: see launch_spectral
-  int reps;                                       // EQUAL: recurrence steps of frame T - 1
   size_t region; int ldx, ldc;
   DpGeom g;
+  int reps;                                       // EQUAL: recurrence steps of frame T - 1
 };
 
 // EQUAL: clips of equal frames, of which the T first are there (launch_gated_spectral_dft).  A variant of its own: the tests and the
@@ -107,8 +107,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
       float* out = reinterpret_cast<float*>(RA);
       dp_inv_rows<RT, YT, NT>(g, RB, ldx, TW, out, P);
       __syncthreads();
-      const float* zp = (EQUAL ? a.xz + ((size_t)b * a.T * 2 * a.C + c0) * HW : xp) + (size_t)a.C * HW;
-      dp_store<NT>(g, out, xp, a.mode == 0 ? zp : nullptr, P);
+      if constexpr (EQUAL) dp_store<NT>(g, out, xp, a.xz + (((size_t)b * a.T * 2 + 1) * a.C + c0) * HW, P);      // (mode 0)
+      else dp_store<NT>(g, out, xp, a.mode == 0 ? xp + (size_t)a.C * HW : nullptr, P);
     }
   }
 }
@@ -171,7 +171,7 @@ static auto pick_kernel(const DpChoice& ch) {
 int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat, const float* gates, float* xz,
                               int last_only, int mode, cudaStream_t st, const float* dchan, int equal_steps) {
   const DpChoice ch = dp_choose(H, W, C, B, 1, 226 * 1024, gated_dft_bytes, T);
-  if (ch.P == 0) return CSSM_ERR_UNSUPPORTED;
+  if (ch.P == 0 || (equal_steps > 0 && mode != 0)) return CSSM_ERR_UNSUPPORTED;
   GatedDftArgs a;
   memset(&a, 0, sizeof(a));
   a.xz = xz; a.khat = khat; a.gates = reinterpret_cast<const float4*>(gates); a.dchan = dchan;
