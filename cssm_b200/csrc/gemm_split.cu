@@ -662,7 +662,11 @@ int launch_gemm_split(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   q.hw = FastDiv(g.HW); q.w = FastDiv(g.W > 0 ? g.W : 1); q.t = FastDiv(g.T > 0 ? g.T : 1);
   q.fdiv = FastDiv(g.a_fdiv > 1 ? g.a_fdiv : 1);
   constexpr size_t LIMIT = 227 * 1024;
-  const size_t fixed = 1024 + 1024 + 128 + (a_planar ? 8 * 4096 + (g.rms_scale != nullptr ? GS_SS * 1024 : 0) : 0);   // slack, bias, barriers, staging, sums
+  // The RMS prologue's row sums; two and three K blocks ask for their room in any case: 8 KB less and the CTAs of an overlapped launch
+  // find room beside those of the transforms on some SMs, and 128-column tiles of 128 channels fit (ungated block, us a pass without / with:
+  // 54 x 14 x 14 x 96 32.2 / 31.1, 40 x 14 x 14 x 128 30.2 / 28.9, 120 53.3 / 51.7; one block gains without: 10 x 14 x 14 x 32 15.5 / 16.5).
+  const bool sums = g.rms_scale != nullptr || q.kblocks == 2 || q.kblocks == 3;
+  const size_t fixed = 1024 + 1024 + 128 + (a_planar ? 8 * 4096 + (sums ? GS_SS * 1024 : 0) : 0);   // slack, bias, barriers, staging, sums
   if (g.wsplit != nullptr && (g.rms_scale != nullptr || g.gate != nullptr || !aligned16(g.wsplit))) return CSSM_ERR_UNSUPPORTED;
   auto round32 = [](int v) { return (v + 31) / 32 * 32; };
   auto res_size = [&](int bn) { return (size_t)q.kblocks * 3 * bn * 128; };
