@@ -157,39 +157,37 @@ __global__ void __launch_bounds__(QT_THREADS, 1) gemm_qkv_tconv_kernel(const __g
     }
   } else if (warp == QT_MMA_WARP) {
     // ================================ MMA issuer ================================
-    if (lane == 0) {
-      const uint32_t idesc = tc::make_idesc_tf32(QT_BM, QT_N);
-      const int mine = a.seqs > (int)blockIdx.x ? (a.seqs - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * T : 0;
-      bool ok = true;
-      int slot = 0;
-      for (int n = 0; n < mine; ++n) {
-        // the accumulator of step n - 5 was last read by the epilogue of step n - 2
-        if (!tc::mbar_wait(&accempty[n & 1], ((n >> 1) & 1) ^ 1) || !tc::mbar_wait(&full[n & 1], (n >> 1) & 1)) {
-          atomicExch(&g_qt_error, 2); ok = false; break;
-        }
-        tc::fence_after_sync();
-        const uint32_t a_hi = sbase + QT_A_OFF + (uint32_t)(n & 1) * 2u * QT_A_HALF, a_lo = a_hi + QT_A_HALF;
-        const uint32_t d = tmem_base + (uint32_t)slot * QT_N;
-        if (++slot == QT_RING) slot = 0;
-        uint32_t acc = 0;
+    // The whole warp walks the loop, one lane issues (elect_one).
+    const uint32_t idesc = tc::make_idesc_tf32(QT_BM, QT_N);
+    const int mine = a.seqs > (int)blockIdx.x ? (a.seqs - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * T : 0;
+    bool ok = true;
+    int slot = 0;
+    for (int n = 0; n < mine; ++n) {
+      // the accumulator of step n - 5 was last read by the epilogue of step n - 2
+      if (__any_sync(0xffffffffu, !tc::mbar_wait(&accempty[n & 1], ((n >> 1) & 1) ^ 1) || !tc::mbar_wait(&full[n & 1], (n >> 1) & 1))) {
+        atomicExch(&g_qt_error, 2); ok = false; break;
+      }
+      tc::fence_after_sync();
+      const uint32_t a_hi = sbase + QT_A_OFF + (uint32_t)(n & 1) * 2u * QT_A_HALF, a_lo = a_hi + QT_A_HALF;
+      const uint32_t d = tmem_base + (uint32_t)slot * QT_N;
+      if (++slot == QT_RING) slot = 0;
+      if (tc::elect_one()) {
 #pragma unroll
         for (int pass = 0; pass < 3; ++pass) {
-          const uint32_t ab = pass == 1 ? a_lo : a_hi, bb = pass == 2 ? sbase + QT_B_HALF : sbase;
+          const uint64_t ad = tc::make_desc_sw128(pass == 1 ? a_lo : a_hi), bd = tc::make_desc_sw128(pass == 2 ? sbase + QT_B_HALF : sbase);
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint32_t koff = (uint32_t)(ks & 3) * 32u;
-            tc::mma_tf32(d, tc::make_desc_sw128(ab + (uint32_t)(ks >> 2) * (QT_BM * 128u) + koff),
-                         tc::make_desc_sw128(bb + (uint32_t)(ks >> 2) * (QT_N * 128u) + koff), idesc, acc);
-            acc = 1;
-          }
+          for (int ks = 0; ks < 8; ++ks)
+            tc::mma_tf32(d, ad + (ks >> 2) * (QT_BM * 128u >> 4) + (ks & 3) * 2, bd + (ks >> 2) * (QT_N * 128u >> 4) + (ks & 3) * 2, idesc, (pass | ks) ? 1u : 0u);
         }
         tc::commit(&empty[n & 1]);
         tc::commit(&accfull[n & 1]);
       }
-      // nothing of this thread's tensor work may be in flight when TMEM is freed
-      tc::commit(done);
-      if (!tc::mbar_wait(done, 0) && ok) atomicExch(&g_qt_error, 3);
+      __syncwarp();
     }
+    // nothing of this warp's tensor work may be in flight when TMEM is freed
+    if (tc::elect_one()) tc::commit(done);
+    __syncwarp();
+    if (!tc::mbar_wait(done, 0) && ok) atomicExch(&g_qt_error, 3);
     __syncwarp();
   } else {
     // ================================ epilogue ================================

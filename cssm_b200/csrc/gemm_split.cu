@@ -102,15 +102,13 @@ __device__ __forceinline__ void store_split8(unsigned char* base, uint32_t off, 
 __device__ __forceinline__ uint32_t idesc_bf16_f32(uint32_t M, uint32_t N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
-// issued by the lanes with lead != 0 (one of the warp)
 __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate, uint32_t lead) {
+                                        uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, l;\n\t"
+      "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 l, %5, 0;\n\t"
-      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
 // Columns [n, n + 32) of output row m once more, by float32 FMAs over k: for results that are not finite.  An
@@ -448,23 +446,20 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
     }
   } else if (warp == GS_MMA_WARP) {
     // ================================ MMA issuer ================================
-    // The whole warp walks the loop and only the instruction itself is predicated on lane 0: in a
-    // one-lane branch the compiler has to move every descriptor into uniform registers again, and that
-    // set the pace (about 125 clocks an MMA).
+    // The whole warp walks the loop, one lane issues (elect_one).
     const uint32_t idesc = idesc_bf16_f32(GS_BM, BN);
-    const uint32_t lead = lane == 0 ? 1u : 0u;
     // (A part, B part) of the six partial products, smallest first
     constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
     int s = 0, sph = 0, ac = 0, aph = 1;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-      if (!tc::mbar_wait(&accempty[ac], aph)) { atomicExch(&g_split_error, 2); ok = false; break; }
+      if (__any_sync(0xffffffffu, !tc::mbar_wait(&accempty[ac], aph))) { atomicExch(&g_split_error, 2); ok = false; break; }
       tc::fence_after_sync();
       const uint32_t d = tmem_base + (uint32_t)ac * acc_cols;
       uint32_t d00 = WIDE || !q.nl ? d : d + BN;
       int left = 0;                                     // WIDE: K blocks that still go to the leading accumulator d00
       for (int kb = 0; kb < kblocks; ++kb) {
-        if (!tc::mbar_wait(&full[s], sph)) { atomicExch(&g_split_error, 2); ok = false; break; }
+        if (__any_sync(0xffffffffu, !tc::mbar_wait(&full[s], sph))) { atomicExch(&g_split_error, 2); ok = false; break; }
         tc::fence_after_sync();
         const uint32_t a_s = sbase + res_bytes + (uint32_t)s * stage_bytes;
         const uint32_t b_s = RES ? sbase + (uint32_t)kb * b_block : a_s + GS_A_BYTES;
@@ -485,21 +480,26 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
 #pragma unroll
             for (int ks = 0; ks < KS; ++ks)
               mma_f16(p == 5 ? d00 : d, ad0 + PA[p] * (GS_A_PART >> 4) + ks * 2, bd[PB[p]] + ks * 2, idesc,
-                      p == 5 && ks == 0 ? first00 : (p | ks ? 1u : first), lead);
+                      p == 5 && ks == 0 ? first00 : (p | ks ? 1u : first));
         };
         const int krem = g.K - kb * GS_BK;
-        if (krem > 48) issue(Int<4>());
-        else if (krem > 32) issue(Int<3>());
-        else if (krem > 16) issue(Int<2>());
-        else issue(Int<1>());
-        if (lane == 0) tc::commit(&empty[s]);
+        if (tc::elect_one()) {
+          if (krem > 48) issue(Int<4>());
+          else if (krem > 32) issue(Int<3>());
+          else if (krem > 16) issue(Int<2>());
+          else issue(Int<1>());
+          tc::commit(&empty[s]);
+        }
+        __syncwarp();
         if (++s == NS) { s = 0; sph ^= 1; }
       }
-      if (ok && lane == 0) tc::commit(&accfull[ac]);
+      if (ok && tc::elect_one()) tc::commit(&accfull[ac]);
+      __syncwarp();
       if (++ac == bufs) { ac = 0; aph ^= 1; }
     }
-    // nothing of lane 0's tensor work may be in flight when TMEM is freed
-    if (lane == 0) tc::commit(done);
+    // nothing of this warp's tensor work may be in flight when TMEM is freed
+    if (tc::elect_one()) tc::commit(done);
+    __syncwarp();
     if (!tc::mbar_wait(done, 0) && ok) atomicExch(&g_split_error, 3);
     __syncwarp();
   } else {

@@ -135,54 +135,60 @@ mlp_fused_kernel(const MlpFusedArgs g, const __grid_constant__ CUtensorMap amap,
     __syncwarp();
   } else if (warp < 3) {
     // ================================ MMA issuers ================================
+    // Whole warps walk the loop, one lane issues (elect_one).
     const int half = warp - 1;
-    if (lane == 0) {
-      const uint32_t acc1 = tmem_base + (uint32_t)half * 192u, acc2 = acc1 + 128u;   // acc1: two 64-column buffers
-      const uint32_t id = mf_idesc(128, 64);
-      const uint32_t hs_a = sbase + (uint32_t)(hs - smem) + (uint32_t)half * MF_HS_BYTES;
-      const uint32_t w1_a = sbase + (uint32_t)(w1s - smem), w2_a = sbase + (uint32_t)(w2s - smem);
-      if (!tc::mbar_wait(wfull, 0)) { atomicExch(&g_mlp_error, 2); bad = true; }
-      int it = 0, j = 0;                               // it: CTA-local tile index; j: tiles of this half
-      // fc2 over hidden chunk ch (64 columns = one K block) of the half's j-th tile
-      auto fc2_chunk = [&](int ch) -> bool {
-        const int b = ch & 1, nb = (4 * j + ch) >> 1;          // nb-th use of hidden buffer b
-        if (ch == 0 && !tc::mbar_wait(&acc2empty[half], (j & 1) ^ 1)) { atomicExch(&g_mlp_error, 5); return false; }
-        if (!tc::mbar_wait(&hsfull[2 * half + b], nb & 1)) { atomicExch(&g_mlp_error, 6); return false; }
+    auto wok = [](bool ok) { return !__any_sync(0xffffffffu, !ok); };       // all lanes agree
+    const uint32_t acc1 = tmem_base + (uint32_t)half * 192u, acc2 = acc1 + 128u;   // acc1: two 64-column buffers
+    const uint32_t id = mf_idesc(128, 64);
+    const uint32_t hs_a = sbase + (uint32_t)(hs - smem) + (uint32_t)half * MF_HS_BYTES;
+    const uint32_t w1_a = sbase + (uint32_t)(w1s - smem), w2_a = sbase + (uint32_t)(w2s - smem);
+    if (!wok(tc::mbar_wait(wfull, 0))) { atomicExch(&g_mlp_error, 2); bad = true; }
+    int it = 0, j = 0;                               // it: CTA-local tile index; j: tiles of this half
+    // fc2 over hidden chunk ch (64 columns = one K block) of the half's j-th tile
+    auto fc2_chunk = [&](int ch) -> bool {
+      const int b = ch & 1, nb = (4 * j + ch) >> 1;          // nb-th use of hidden buffer b
+      if (ch == 0 && !wok(tc::mbar_wait(&acc2empty[half], (j & 1) ^ 1))) { atomicExch(&g_mlp_error, 5); return false; }
+      if (!wok(tc::mbar_wait(&hsfull[2 * half + b], nb & 1))) { atomicExch(&g_mlp_error, 6); return false; }
+      tc::fence_after_sync();
+      const uint64_t ad = tc::make_desc_sw128(hs_a + b * 16384u), bd = tc::make_desc_sw128(w2_a + ch * 8192u);
+      if (tc::elect_one()) {
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) mf_mma(acc2, ad + ks * 2, bd + ks * 2, id, (ch | ks) ? 1u : 0u);
+      }
+      __syncwarp();
+      return true;
+    };
+    for (int tile = blockIdx.x; tile < num_tiles && !bad; tile += gridDim.x, ++it) {
+      if ((it & 1) != half) continue;
+      const int s = it % MF_NS;
+      const uint32_t t_a = sbase + (uint32_t)(ts - smem) + (uint32_t)s * MF_T_BYTES;
+      if (!wok(tc::mbar_wait(&tfull[s], (it / MF_NS) & 1))) { atomicExch(&g_mlp_error, 3); bad = true; break; }
+      // fc1 in four chunks of 64 hidden columns through two accumulators; the fc2 of a chunk is
+      // issued one chunk later, while the epilogue works on the next accumulator
+      for (int ch = 0; ch < 4 && !bad; ++ch) {
+        const int b = ch & 1, nb = (4 * j + ch) >> 1;
+        if (!wok(tc::mbar_wait(&acc1empty[2 * half + b], (nb & 1) ^ 1))) { atomicExch(&g_mlp_error, 4); bad = true; break; }
         tc::fence_after_sync();
+        const uint64_t ad = tc::make_desc_sw128(t_a), bd = tc::make_desc_sw128(w1_a + ch * 8192u);
+        if (tc::elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          mf_mma(acc2, tc::make_desc_sw128(hs_a + b * 16384u + ks * 32u),
-                 tc::make_desc_sw128(w2_a + ch * 8192u + ks * 32u), id, (ch | ks) ? 1u : 0u);
-        return true;
-      };
-      for (int tile = blockIdx.x; tile < num_tiles && !bad; tile += gridDim.x, ++it) {
-        if ((it & 1) != half) continue;
-        const int s = it % MF_NS;
-        const uint32_t t_a = sbase + (uint32_t)(ts - smem) + (uint32_t)s * MF_T_BYTES;
-        if (!tc::mbar_wait(&tfull[s], (it / MF_NS) & 1)) { atomicExch(&g_mlp_error, 3); bad = true; break; }
-        // fc1 in four chunks of 64 hidden columns through two accumulators; the fc2 of a chunk is
-        // issued one chunk later, while the epilogue works on the next accumulator
-        for (int ch = 0; ch < 4 && !bad; ++ch) {
-          const int b = ch & 1, nb = (4 * j + ch) >> 1;
-          if (!tc::mbar_wait(&acc1empty[2 * half + b], (nb & 1) ^ 1)) { atomicExch(&g_mlp_error, 4); bad = true; break; }
-          tc::fence_after_sync();
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            mf_mma(acc1 + b * 64u, tc::make_desc_sw128(t_a + ks * 32u),
-                   tc::make_desc_sw128(w1_a + ch * 8192u + ks * 32u), id, ks ? 1u : 0u);
+          for (int ks = 0; ks < 4; ++ks) mf_mma(acc1 + b * 64u, ad + ks * 2, bd + ks * 2, id, ks ? 1u : 0u);
           tc::commit(&acc1full[2 * half + b]);
           if (ch == 3) tc::commit(&tempty[s]);         // the input tile has been read by all chunks
-          if (ch > 0 && !fc2_chunk(ch - 1)) { bad = true; break; }
         }
-        if (bad) break;
-        if (!fc2_chunk(3)) { bad = true; break; }
-        tc::commit(&acc2full[half]);
-        ++j;
+        __syncwarp();
+        if (ch > 0 && !fc2_chunk(ch - 1)) { bad = true; break; }
       }
-      // nothing of this thread's tensor work may be in flight when TMEM is freed
-      tc::commit(&done[half]);
-      if (!tc::mbar_wait(&done[half], 0) && !bad) atomicExch(&g_mlp_error, 8);
+      if (bad) break;
+      if (!fc2_chunk(3)) { bad = true; break; }
+      if (tc::elect_one()) tc::commit(&acc2full[half]);
+      __syncwarp();
+      ++j;
     }
+    // nothing of this thread's tensor work may be in flight when TMEM is freed
+    if (tc::elect_one()) tc::commit(&done[half]);
+    __syncwarp();
+    if (!tc::mbar_wait(&done[half], 0) && !bad) atomicExch(&g_mlp_error, 8);
     __syncwarp();
   } else {
     // ================================ epilogue ================================

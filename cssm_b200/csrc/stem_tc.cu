@@ -171,30 +171,35 @@ stem_layer_tc_kernel(const __grid_constant__ StemArgs a, const unsigned char* __
       load_stage(st);
     }
   }
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
+    // the whole warp walks the loop, one lane issues (elect_one)
     constexpr uint32_t ALBO = ST_PIX * 16u, ASBO = ST_PW * 16u, BLBO = 3u * C * 16u;
     const uint32_t id1 = stem_idesc(128, C), id2 = stem_idesc(128, 2 * C);
     for (int st = 0; st < L::STAGES; ++st) {
-      if (!tc::mbar_wait_spin(&full[st % ST_RING], (st / ST_RING) & 1)) { atomicExch(&g_stem_error, 2); s_bad = 1; break; }
+      if (__any_sync(0xffffffffu, !tc::mbar_wait_spin(&full[st % ST_RING], (st / ST_RING) & 1))) { atomicExch(&g_stem_error, 2); s_bad = 1; break; }
       tc::fence_after_sync();
       const int tap = st / (C / 32), half = st % (C / 32);
       const uint32_t bs = sbase + L::RING_OFF + (st % ST_RING) * L::STAGE_BYTES;
       const uint32_t as = sbase + L::A_OFF + (uint32_t)(half * 4 * ST_PIX + (tap / 3) * ST_PW + tap % 3) * 16u;
       const uint32_t lead = tmem + (tap < 5 ? 0u : (uint32_t)C), small = tmem + 2u * C;
       const bool first_lead = half == 0 && (tap == 0 || tap == 5);
+      if (tc::elect_one()) {
 #pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
-        const uint32_t ak = as + 2u * ks * ALBO, bk = bs + 2u * ks * BLBO;
-        const uint64_t a0 = desc_k(ak, ALBO, ASBO), a1 = desc_k(ak + L::PART, ALBO, ASBO), a2 = desc_k(ak + 2 * L::PART, ALBO, ASBO);
-        const uint64_t b0 = desc_k(bk, BLBO, 128), b1 = desc_k(bk + C * 16u, BLBO, 128);
-        stem_mma(lead, a0, b0, id1, !(first_lead && ks == 0));
-        stem_mma(small, a0, b1, id2, !(st == 0 && ks == 0));       // [01 02]
-        stem_mma(small, a1, b0, id2, 1);                           // [10 11]
-        stem_mma(small, a2, b0, id1, 1);                           // [20]
+        for (int ks = 0; ks < 2; ++ks) {
+          const uint32_t ak = as + 2u * ks * ALBO, bk = bs + 2u * ks * BLBO;
+          const uint64_t a0 = desc_k(ak, ALBO, ASBO), a1 = desc_k(ak + L::PART, ALBO, ASBO), a2 = desc_k(ak + 2 * L::PART, ALBO, ASBO);
+          const uint64_t b0 = desc_k(bk, BLBO, 128), b1 = desc_k(bk + C * 16u, BLBO, 128);
+          stem_mma(lead, a0, b0, id1, !(first_lead && ks == 0));
+          stem_mma(small, a0, b1, id2, !(st == 0 && ks == 0));       // [01 02]
+          stem_mma(small, a1, b0, id2, 1);                           // [10 11]
+          stem_mma(small, a2, b0, id1, 1);                           // [20]
+        }
+        tc::commit(&empty[st % ST_RING]);
       }
-      tc::commit(&empty[st % ST_RING]);
+      __syncwarp();
     }
-    tc::commit(accfull);
+    if (tc::elect_one()) tc::commit(accfull);
+    __syncwarp();
   }
   __syncwarp();
 
