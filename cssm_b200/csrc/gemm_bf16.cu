@@ -3,23 +3,29 @@
 //
 //   out[m, n] = act( sum_k A[m, k] * Wt[n, k] + bias[n] ) (+ res[m, n]),  bf16 in, fp32 accumulate.
 //
-// Persistent kernel, one CTA per SM, 320 threads (448 in conv mode), warp-specialised:
+// Persistent kernel, one CTA per SM, 18 warps (14 in the im2col form), warp-specialised:
 //   warp 0     TMA producer: one lane issues cp.async.bulk.tensor loads of the A tile (128 rows x
 //              64 k, plain mode) and the weight tile (BN rows x 64 k) of every K block into a
 //              4-stage ring of 128-byte-swizzled K-major operand tiles;
 //   warp 1     MMA issuer: one lane issues 4 tcgen05.mma.kind::f16 (M128 x BN x K16) per K block
 //              into one of four TMEM accumulators (BN <= 128; two for wider single tiles);
 //              tcgen05.commit frees the stage / publishes the accumulator;
-//   warps 2-9  epilogue, two warps per TMEM lane quadrant: tcgen05.ld (lane = output row), bias,
-//              GELU / SiLU, residual; each half (one warp per quadrant) owns every other tile and two
-//              of the accumulators, stages boxes of 128 rows x 64 bf16 columns in the 128-byte
-//              swizzle in a ring of three or four slots and writes them with TMA tensor stores; the
-//              residual box is fetched by TMA into the slot it will be staged in, two boxes ahead,
-//              and added in place (N a multiple of 64; otherwise direct 16-byte loads and stores);
-//   warps 10-13 im2col producers (conv mode only): eight consecutive lanes fetch the eight 16-byte
+//   warps 2-17 epilogue, four warps per TMEM lane quadrant: tcgen05.ld (lane = output row), bias (from shared
+//              memory), GELU / SiLU, residual; each half (two warps per quadrant) owns every other tile and half of the
+//              accumulators.  Without a residual by TMA a warp has its 32 rows of every other box of 64 columns, a 4 KB
+//              staging slot in the 128-byte swizzle and TMA tensor stores of its own and waits for no other warp.  With
+//              one, and in conv mode, the half shares boxes of 128 rows x 64 columns in a ring of two to four slots
+//              (a warp 32 of the columns) with a barrier before the store; the residual box is fetched by TMA into the
+//              slot it will be staged in, two boxes ahead, and added in place (N a multiple of 64; otherwise direct
+//              16-byte loads and stores).  The im2col form has eight epilogue warps;
+//   4 more     im2col producers (conv mode only): eight consecutive lanes fetch the eight 16-byte
 //              channel chunks of one output pixel's K block from the channels-last input (zero
 //              outside the image), four pixels per warp instruction, and write them in the same
 //              swizzled layout; the loads of the next two K blocks are in flight meanwhile.
+// With eight warps, a barrier a box and the bias read from global memory behind every accumulator load the epilogue was a chain of
+// waits (GELU, 128 x 256 tiles: issue slots 40 % busy, special-function pipe 37 %, most stalls on loads and barriers).  M x K -> N, us:
+// 401408 x 128 -> 512 GELU 152 -> 107, 100352 x 256 -> 1024 GELU 94 -> 75, 100352 x 256 -> 512 SiLU 55 -> 45, 25088 x 384 -> 1536 GELU
+// 49 -> 41, 25088 x 1536 -> 384 + residual 50 -> 47; sixteen warps alone 148, 90, 53, 47, 48.
 // Every mbarrier wait is bounded; on expiry the kernel records an error code (cssm_device_error)
 // and winds down.  No multicast, no cluster: each CTA loads its own tiles.
 #include <cuda.h>
@@ -33,7 +39,9 @@ namespace cssm {
 
 __device__ int g_bf16_error = 0;
 
-constexpr int GB_THREADS_PLAIN = 320, GB_THREADS_CONV = 448;
+// Epilogue warps: sixteen; eight beside the gathering warps of the im2col form, which need the registers.
+template <bool IM2COL> constexpr int gb_epi_warps = IM2COL ? 8 : 16;
+template <bool IM2COL> constexpr int gb_threads = (2 + gb_epi_warps<IM2COL> + (IM2COL ? 4 : 0)) * 32;
 constexpr int GB_BM = 128, GB_BK = 64, GB_MAX_STAGES = 4;
 constexpr uint32_t GB_A_BYTES = GB_BM * 128u;            // one A stage: 128 rows x 128 bytes
 
@@ -56,8 +64,9 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
 }
 
 // RTMA (with TMA_OUT): the residual boxes come by TMA into the staging slots.
-template <bool IM2COL, bool TMA_OUT, bool RTMA>
-__global__ void __launch_bounds__(IM2COL ? GB_THREADS_CONV : GB_THREADS_PLAIN, 1)
+// ROWS (with TMA_OUT, plain GEMMs): every epilogue warp stages and stores boxes of its own 32 rows.
+template <bool IM2COL, bool TMA_OUT, bool RTMA, bool ROWS = false>
+__global__ void __launch_bounds__(gb_threads<IM2COL>, 1)
 gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
                  const __grid_constant__ CUtensorMap bmap, const __grid_constant__ CUtensorMap omap,
                  const __grid_constant__ CUtensorMap rmap) {
@@ -82,8 +91,10 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
   uint64_t* done = resfull + 8;
   uint64_t* wfull = done + 1;                   // resident weights landed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wfull + 1);
+  float* bias_s = reinterpret_cast<float*>(bars + 32);      // the bias, where it fits (g.bias_n values)
   const int NACC = g.nacc;                                  // TMEM accumulators: 4 of BN <= 128 columns, else 2
 
+  constexpr int EW = gb_epi_warps<IM2COL>, HALF_THREADS = EW * 16, CW = EW / 8;      // CW: warps of a half and lane quadrant
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tiles = g.N / g.BN;
   const int m_tiles = g.conv_tma ? g.tiles_w * g.tiles_h * ((g.Bimg + g.Bbox - 1) / g.Bbox) : (g.M + GB_BM - 1) / GB_BM;
@@ -100,13 +111,14 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
     for (int a = 0; a < 4; ++a) {
       tc::mbar_init(&accfull[a], 1);
       // one lane per warp of the half that drains the accumulator
-      tc::mbar_init(&accempty[a], 4);
+      tc::mbar_init(&accempty[a], EW / 2);
     }
     for (int a = 0; a < 8; ++a) tc::mbar_init(&resfull[a], 1);
     tc::mbar_init(done, 1);
     tc::mbar_init(wfull, 1);
     tc::fence_mbar_init();
   }
+  for (int i = tid; i < g.bias_n; i += gb_threads<IM2COL>) bias_s[i] = __ldg(g.bias + i);      // (as the weights: no wait)
   if (warp == 1) {
     tc::tmem_alloc(tmem_slot, tmem_cols);
     tc::tmem_relinquish();
@@ -170,45 +182,47 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
   } else if (warp == 1) {
     // ================================ MMA issuer ================================
     // The limit of the waits below is for this kernel's own loads: they begin once the producer's wait is over.
+    // The whole warp walks the loop, one lane issues (elect_one).
     pdl_wait();
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc_bf16(GB_BM, BN);
-      if (wres && !tc::mbar_wait(wfull, 0)) { atomicExch(&g_bf16_error, 6); bad = true; }
-      int it = 0, tcnt = 0;
-      for (int tile = blockIdx.x; tile < num_tiles && !bad; tile += gridDim.x, ++tcnt) {
-        const int ac = tcnt % NACC, aph = (tcnt / NACC) & 1;
-        if (!tc::mbar_wait(&accempty[ac], aph ^ 1)) { atomicExch(&g_bf16_error, 6); bad = true; break; }
+    const uint32_t idesc = make_idesc_bf16(GB_BM, BN);
+    if (wres && !tc::mbar_wait(wfull, 0)) { atomicExch(&g_bf16_error, 6); bad = true; }
+    bad = __any_sync(0xffffffffu, bad);
+    int s = 0, sph = 0, ac = 0, aph = 1;
+    for (int tile = blockIdx.x; tile < num_tiles && !bad; tile += gridDim.x) {
+      if (__any_sync(0xffffffffu, !tc::mbar_wait(&accempty[ac], aph))) { atomicExch(&g_bf16_error, 6); bad = true; break; }
+      tc::fence_after_sync();
+      const uint32_t d = tmem_base + (uint32_t)ac * BN;
+      for (int kb = 0; kb < kblocks; ++kb) {
+        if (__any_sync(0xffffffffu, !tc::mbar_wait(&full[s], sph))) { atomicExch(&g_bf16_error, 6); bad = true; break; }
         tc::fence_after_sync();
-        const uint32_t d = tmem_base + (uint32_t)ac * BN;
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % NS;
-          if (!tc::mbar_wait(&full[s], (it / NS) & 1)) { atomicExch(&g_bf16_error, 6); bad = true; break; }
-          tc::fence_after_sync();
-          const uint32_t a_s = sbase + wres_bytes + (uint32_t)s * stage_bytes;
-          const uint32_t b_s = wres ? sbase + (uint32_t)kb * BN * 128u : a_s + GB_A_BYTES;
+        const uint32_t a_s = sbase + wres_bytes + (uint32_t)s * stage_bytes;
+        const uint64_t ad = tc::make_desc_sw128(a_s), bd = tc::make_desc_sw128(wres ? sbase + (uint32_t)kb * BN * 128u : a_s + GB_A_BYTES);
+        if (tc::elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) {
-            const uint64_t ad = tc::make_desc_sw128(a_s + (uint32_t)ks * 32u);
-            const uint64_t bd = tc::make_desc_sw128(b_s + (uint32_t)ks * 32u);
-            mma_bf16(d, ad, bd, idesc, (kb | ks) ? 1u : 0u);
-          }
+          for (int ks = 0; ks < 4; ++ks) mma_bf16(d, ad + ks * 2, bd + ks * 2, idesc, (kb | ks) ? 1u : 0u);
           tc::commit(&empty[s]);
         }
-        if (bad) break;
-        tc::commit(&accfull[ac]);
+        __syncwarp();
+        if (++s == NS) { s = 0; sph ^= 1; }
       }
-      // nothing of this thread's tensor work may be in flight when TMEM is freed
-      tc::commit(done);
-      if (!tc::mbar_wait(done, 0) && !bad) atomicExch(&g_bf16_error, 7);
+      if (bad) break;
+      if (tc::elect_one()) tc::commit(&accfull[ac]);
+      __syncwarp();
+      if (++ac == NACC) { ac = 0; aph ^= 1; }
     }
+    // nothing of this warp's tensor work may be in flight when TMEM is freed
+    if (tc::elect_one()) tc::commit(done);
     __syncwarp();
-  } else if (warp < 10) {
+    if (!tc::mbar_wait(done, 0) && !bad) atomicExch(&g_bf16_error, 7);
+    __syncwarp();
+  } else if (warp < 2 + EW) {
     // ================================ epilogue ================================
     // Two halves of four warps (one per TMEM lane quadrant).  Half h owns the tiles of its CTA with
     // tile count parity h; accumulator = tile count mod NACC, so a half drains one accumulator while
     // the MMA warp fills its other one.
     const int q = warp & 3;                       // TMEM lane quadrant this warp may read
-    const int half = (warp - 2) >> 2;
+    const int half = (warp - 2) / (EW / 2);
+    const int sub = CW == 1 ? 0 : ((warp - 2) >> 2) & 1;      // CW = 2: which 32 columns of every 64 are this warp's
     const int row = q * 32 + lane;
     const uint32_t tlane = tmem_base + ((uint32_t)(q * 32) << 16);
     pdl_wait();
@@ -216,7 +230,14 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
     auto act32 = [&](const uint32_t (&r)[32], int n, float (&v)[32]) {
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-      if (g.bias != nullptr) {
+      if (g.bias_n != 0) {
+        const float4* bp = reinterpret_cast<const float4*>(bias_s + n);
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          const float4 b4 = bp[j >> 2];
+          v[j] += b4.x; v[j + 1] += b4.y; v[j + 2] += b4.z; v[j + 3] += b4.w;
+        }
+      } else if (g.bias != nullptr) {
         const float4* bp = reinterpret_cast<const float4*>(g.bias + n);
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
@@ -232,14 +253,79 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
         for (int j = 0; j < 32; j += 2) silu_tanh_x2(v[j], v[j + 1]);
       }
     };
-    if constexpr (TMA_OUT) {
+    if constexpr (ROWS) {
+      // A warp has 32 rows of every other box of 64 columns: it stages them in a 4 KB slot of its own and writes them with a
+      // TMA store of its own, so it waits for nobody but the accumulator.
+      unsigned char* stg = out_s + (uint32_t)(warp - 2) * 4096u;
+      const int nb = g.BN / 64;
+      for (int tcnt = half;; tcnt += 2) {
+        const int tile = blockIdx.x + tcnt * (int)gridDim.x;
+        if (tile >= num_tiles) break;
+        const int m0 = (tile / n_tiles) * GB_BM, n0 = (tile % n_tiles) * g.BN;
+        const int ac = tcnt % NACC, aph = (tcnt / NACC) & 1;
+        const bool has_res = g.res != nullptr && m0 + row < g.M;
+        const uint4* rrow = reinterpret_cast<const uint4*>(g.res + (has_res ? (size_t)(m0 + row) * g.ldr + n0 : 0));
+        uint4 rs[4];                              // residual of the warp's next 32 columns
+        auto fetch_res = [&](int c) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) rs[j] = has_res && c < 2 * nb ? __ldg(rrow + c * 4 + j) : make_uint4(0u, 0u, 0u, 0u);
+        };
+        const int s0 = (sub + (tcnt >> 1)) & (CW - 1);      // (an odd number of boxes: the two warps take the extra one in turn)
+        if (g.res != nullptr) fetch_res(2 * s0);
+        if (__any_sync(0xffffffffu, !tc::mbar_wait(&accfull[ac], aph))) { atomicExch(&g_bf16_error, 8); break; }
+        tc::fence_after_sync();
+        const uint32_t taddr = tlane + (uint32_t)ac * BN;
+        for (int box = s0; box < nb; box += CW) {
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            uint32_t ra[32];
+            float v[32];
+            tc::ld_32x32b_x32(taddr + box * 64 + hh * 32, ra);
+            tc::wait_ld();
+            act32(ra, n0 + box * 64 + hh * 32, v);
+            if (g.res != nullptr) {
+#pragma unroll
+              for (int j4 = 0; j4 < 4; ++j4) {
+                float f[8];
+                unpack8(rs[j4], f);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[j4 * 8 + e] += f[e];
+              }
+              fetch_res(hh == 0 ? 2 * box + 1 : 2 * (box + CW));
+            }
+            if (hh == 0) {
+              // the store before has read the slot
+              if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+              __syncwarp();
+            }
+#pragma unroll
+            for (int j4 = 0; j4 < 4; ++j4) {
+              const float f[8] = {v[j4 * 8], v[j4 * 8 + 1], v[j4 * 8 + 2], v[j4 * 8 + 3],
+                                  v[j4 * 8 + 4], v[j4 * 8 + 5], v[j4 * 8 + 6], v[j4 * 8 + 7]};
+              *reinterpret_cast<uint4*>(stg + tc::sw128_offset(lane, hh * 4 + j4)) = pack8(f);
+            }
+          }
+          tc::fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            tc::tma_store_2d(&omap, stg, n0 + box * 64, m0 + q * 32);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        }
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&accempty[ac]);
+      }
+      // the slot must outlive the last TMA store that reads it
+      if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    } else if constexpr (TMA_OUT) {
       // Output boxes of 128 rows x 64 bf16 columns are staged in the 128-byte swizzle in a ring of D
       // slots per half and written by TMA tensor stores.  A residual is fetched by TMA into the
       // very slot its box will be staged in, D - 2 boxes ahead (the wait before a slot is reused
       // leaves only the most recent store pending), and is added in place.
       // (Both halves draining every tile of a two-accumulator configuration, each every other box,
       // measured slower than whole tiles in turn: 232 against 197 us for M = 1.6 M, K = 64, N = 256.)
-      const bool issuer = q == 0 && lane == 0;    // issues this half's TMA loads and stores
+      const bool issuer = q == 0 && sub == 0 && lane == 0;    // issues this half's TMA loads and stores
       const int D = g.ostg, nb = g.BN / 64;
       constexpr int b0 = 0, bstep = 1, tstep = 2;
       const int t0 = half;
@@ -261,15 +347,15 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
       };
       if (rtma && issuer)
         for (int k = 0; k < D - 2; ++k) pf_issue();
-      // all 128 threads of the half agree on `ok` (and meet, as a barrier)
+      // all threads of the half agree on `ok` (and meet, as a barrier)
       auto all_ok = [&](bool ok) {
         uint32_t r;
         asm volatile(
             "{\n\t.reg .pred p, q;\n\t"
             "setp.ne.u32 p, %1, 0;\n\t"
-            "bar.red.and.pred q, %2, 128, p;\n\t"
+            "bar.red.and.pred q, %2, %3, p;\n\t"
             "selp.u32 %0, 1, 0, q;\n\t}"
-            : "=r"(r) : "r"((uint32_t)ok), "r"(1 + half) : "memory");
+            : "=r"(r) : "r"((uint32_t)ok), "r"(1 + half), "n"(HALF_THREADS) : "memory");
         return r != 0;
       };
       int bq = 0;                                 // boxes staged by this half so far
@@ -281,10 +367,10 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
         const int ac = tcnt % NACC, aph = (tcnt / NACC) & 1;
         const bool has_res = rreg && m0 + row < g.M;
         const uint4* rrow = reinterpret_cast<const uint4*>(g.res + (has_res ? (size_t)(m0 + row) * g.ldr + n0 : 0));
-        uint4 rs[8];                              // rreg: residual of the next 64 columns
+        uint4 rs[8 / CW];                         // rreg: residual of this warp's part of the next 64 columns
         auto fetch_res = [&](int c0) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) rs[j] = has_res ? __ldg(rrow + (c0 >> 3) + j) : make_uint4(0u, 0u, 0u, 0u);
+          for (int j = 0; j < 8 / CW; ++j) rs[j] = has_res ? __ldg(rrow + (c0 >> 3) + sub * 4 + j) : make_uint4(0u, 0u, 0u, 0u);
         };
         if (rreg) fetch_res(0);
         if (!all_ok(tc::mbar_wait(&accfull[ac], aph))) { atomicExch(&g_bf16_error, 8); break; }
@@ -300,9 +386,10 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
           // accumulator -> bias, activation, residual -> eight packed 16-byte chunks.  Nothing here
           // writes the slot, so it runs while the earlier stores drain.  (Keeping the TMEM load of the
           // next 32 columns in flight during the arithmetic measured slower.)
-          uint4 pk[8];
+          uint4 pk[8 / CW];
 #pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
+          for (int i = 0; i < 2 / CW; ++i) {
+            const int hh = CW == 1 ? i : sub;
             float v[32];
             tc::ld_32x32b_x32(taddr + box * 64 + hh * 32, ra);
             tc::wait_ld();
@@ -312,7 +399,7 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
               for (int j4 = 0; j4 < 4; ++j4) {
                 float f[8];
                 unpack8(rtma ? *reinterpret_cast<const uint4*>(stg + tc::sw128_offset(row, hh * 4 + j4))
-                             : rs[hh * 4 + j4], f);
+                             : rs[i * 4 + j4], f);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[j4 * 8 + e] += f[e];
               }
@@ -321,7 +408,7 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
             for (int j4 = 0; j4 < 4; ++j4) {
               const float f[8] = {v[j4 * 8], v[j4 * 8 + 1], v[j4 * 8 + 2], v[j4 * 8 + 3],
                                   v[j4 * 8 + 4], v[j4 * 8 + 5], v[j4 * 8 + 6], v[j4 * 8 + 7]};
-              pk[hh * 4 + j4] = pack8(f);
+              pk[i * 4 + j4] = pack8(f);
             }
           }
           if (issuer) {
@@ -334,13 +421,13 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
           }
           // without the TMA residual the slot's last reader is only known to the issuer; with it
           // every thread rewrites just its own row of the box it has read
-          if (!rtma) asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+          if (!rtma) asm volatile("bar.sync %0, %1;" ::"r"(1 + half), "n"(HALF_THREADS) : "memory");
           if (rreg && box + 1 < nb) fetch_res((box + 1) * 64);
 #pragma unroll
-          for (int c = 0; c < 8; ++c)
-            *reinterpret_cast<uint4*>(stg + tc::sw128_offset(row, c)) = pk[c];
+          for (int c = 0; c < 8 / CW; ++c)
+            *reinterpret_cast<uint4*>(stg + tc::sw128_offset(row, sub * 4 + c)) = pk[c];
           tc::fence_proxy_async();
-          asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+          asm volatile("bar.sync %0, %1;" ::"r"(1 + half), "n"(HALF_THREADS) : "memory");
           if (issuer) {
             if (g.conv_tma) {
               const int mt = tile / n_tiles;
@@ -373,12 +460,12 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
         const uint4* rrow = reinterpret_cast<const uint4*>(g.res + (has_res ? (size_t)m * g.ldr + n0 : 0));
         uint4 rs[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) rs[j] = has_res ? __ldg(rrow + j) : make_uint4(0u, 0u, 0u, 0u);
+        for (int j = 0; j < 4; ++j) rs[j] = has_res && sub * 32 < g.BN ? __ldg(rrow + sub * 4 + j) : make_uint4(0u, 0u, 0u, 0u);
         if (__any_sync(0xffffffffu, !tc::mbar_wait(&accfull[ac], aph))) { atomicExch(&g_bf16_error, 8); break; }
         tc::fence_after_sync();
         const uint32_t taddr = tlane + (uint32_t)ac * BN;
         uint32_t ra[32];
-        for (int c0 = 0; c0 < g.BN; c0 += 32) {
+        for (int c0 = sub * 32; c0 < g.BN; c0 += 32 * CW) {
           float v[32];
           tc::ld_32x32b_x32(taddr + c0, ra);
           tc::wait_ld();
@@ -390,10 +477,10 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
 #pragma unroll
             for (int e = 0; e < 8; ++e) v[j4 * 8 + e] += f[e];
           }
-          if (c0 + 32 < g.BN) {
+          if (c0 + 32 * CW < g.BN) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-              rs[j] = has_res ? __ldg(rrow + ((c0 + 32) >> 3) + j) : make_uint4(0u, 0u, 0u, 0u);
+              rs[j] = has_res ? __ldg(rrow + ((c0 + 32 * CW) >> 3) + j) : make_uint4(0u, 0u, 0u, 0u);
           }
           if (m < g.M) {
             uint4* op = reinterpret_cast<uint4*>(g.out + (size_t)m * g.ldo + n0 + c0);
@@ -415,7 +502,7 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
     pdl_wait();
     // lane = (row group rg, chunk c): the eight lanes of a group read the eight 16-byte chunks of one
     // output pixel's K block (contiguous channels of one or two taps); thread handles rows rg + 16 i.
-    const int pt = tid - 10 * 32;                 // 0..127
+    const int pt = tid - (2 + EW) * 32;           // 0..127
     const int c = pt & 7, rg = pt >> 3;
     const int HWo = g.Ho * g.Wo;
     int it = 0;
@@ -518,12 +605,12 @@ int gemm_bf16_pick_bn(int N) {
 }
 
 // (rows x cols) bf16 output with row stride ld -> boxes of 64 columns x 128 rows for the TMA stores
-static bool make_out_map(CUtensorMap* map, void* base, uint64_t rows, uint64_t cols, uint64_t ld) {
+static bool make_out_map(CUtensorMap* map, void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows = 128) {
   const tc::EncodeTiledFn enc = tc::encode_fn();
   if (!enc) return false;
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {ld * 2};
-  const cuuint32_t box[2] = {64, 128}, es[2] = {1, 1};
+  const cuuint32_t box[2] = {64, box_rows}, es[2] = {1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, es,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
              CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -633,7 +720,9 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
     // A: out-of-range k columns (K < Kpad) and rows (M not a multiple of 128) arrive as zeros
     if (!im2col && !make_kmajor_map(&amap, g.A, (uint64_t)g.M, (uint64_t)g.K, (uint64_t)g.lda, GB_BM))
       return CSSM_ERR_CUDA;
-    tma_out = tma_out && make_out_map(&omap, g.out, (uint64_t)g.M, (uint64_t)g.N, (uint64_t)g.ldo);
+    // (boxes of 32 rows: see ROWS)
+    const bool boxes128 = im2col || (g.res != nullptr && g.BN <= 128);
+    tma_out = tma_out && make_out_map(&omap, g.out, (uint64_t)g.M, (uint64_t)g.N, (uint64_t)g.ldo, boxes128 ? 128 : 32);
     if (tma_out && g.res != nullptr && g.BN <= 128)
       tma_out = make_out_map(&rmap, const_cast<__nv_bfloat16*>(g.res), (uint64_t)g.M, (uint64_t)g.N, (uint64_t)g.ldr);
   }
@@ -647,7 +736,8 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
   const size_t wres_bytes = (size_t)g.Kpad * g.BN * 2;
   g.wres = (!im2col && g.N == g.BN && wres_bytes <= 64 * 1024) ? 1 : 0;
   const size_t stage = GB_A_BYTES + (g.wres ? 0 : (size_t)g.BN * 128u);
-  const size_t budget = 227 * 1024 - (g.wres ? wres_bytes : 0), fixed = 256 + 1024;
+  g.bias_n = g.bias != nullptr && g.N <= 2048 ? g.N : 0;
+  const size_t budget = 227 * 1024 - (g.wres ? wres_bytes : 0), fixed = 256 + 1024 + (size_t)g.bias_n * 4;
   // Residual by TMA (plain GEMMs with tiles of at most 128 columns): four accumulators and three or
   // four staging slots per epilogue half.  Everything else: two accumulators, two slots, residual
   // rows (if any) by plain loads -- the configuration that measured best without a residual.
@@ -656,7 +746,7 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
   g.stages = GB_MAX_STAGES;
   g.ostg = 0;
   if (tma_out) {
-    while (g.stages > 2 && g.stages * stage + 4 * 16384 + fixed > budget) --g.stages;
+    while (g.stages > 2 && g.stages * stage + 4 * 16384 + fixed > budget) --g.stages;      // (ROWS: sixteen slots of 4 KB)
     g.ostg = rtma ? (int)((budget - fixed - g.stages * stage) / (2 * 16384)) : 2;
     if (g.ostg > 4) g.ostg = 4;
     if (g.ostg < (rtma ? 3 : 2)) return CSSM_ERR_UNSUPPORTED;
@@ -665,11 +755,11 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
   }
   const size_t smem = (g.wres ? wres_bytes : 0) + g.stages * stage + (size_t)g.ostg * 2 * 16384 + fixed;
   auto kern = im2col ? (tma_out ? gemm_bf16_kernel<true, true, false> : gemm_bf16_kernel<true, false, false>)
-                     : (tma_out ? (rtma ? gemm_bf16_kernel<false, true, true> : gemm_bf16_kernel<false, true, false>)
+                     : (tma_out ? (rtma ? gemm_bf16_kernel<false, true, true> : conv ? gemm_bf16_kernel<false, true, false> : gemm_bf16_kernel<false, true, false, true>)
                                 : gemm_bf16_kernel<false, false, false>);
   e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  launch_k(kern, grid, im2col ? GB_THREADS_CONV : GB_THREADS_PLAIN, smem, st, g, amap, bmap, omap, rmap);
+  launch_k(kern, grid, im2col ? gb_threads<true> : gb_threads<false>, smem, st, g, amap, bmap, omap, rmap);
   return check_launch();
 }
 

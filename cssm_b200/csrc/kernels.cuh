@@ -148,6 +148,7 @@ struct Bf16GemmArgs {
   int whole;                 // the rows are one of `whole` chunks of a batch: few-row rules go by M * whole, so that
                              // a chunked call takes the kernels, and gives the sums, of the whole one (0 as 1)
   int wres;                  // 1: the weights stay resident in shared memory (launcher)
+  int bias_n;                // bias values kept in shared memory, 0: none (launcher)
   // conv mode through TMA (filled in by the launcher): an M tile is a patch of Bbox images x Hbox
   // output rows x Wbox output columns (at most 128 pixels); K block kb is `kb_ch` channels from
   // channel (kb % kb_per_tap) * kb_ch of window position kb / kb_per_tap (row = pos / pos_w,
