@@ -483,24 +483,30 @@ dwconv_cl_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ 
 }
 
 // Depthwise KS x KS 'SAME' conv, tiled through shared memory (the path of every bf16 output).
-// A CTA of 128 threads owns a tile of 8 output rows x 16 columns x 64 channels of one image and one
+// A CTA of 32 CG threads owns a tile of TH output rows x CG NC columns x 64 channels of one image and one
 // channel slice; the bf16 input patch with its halo is staged with 16-byte loads as it lies in
 // memory ([row][column][channel]; the per-sample LayerNorm affine, when given, is applied while
 // staging and the result rounded to bf16, zeros stay zeros outside the image).  Thread = one PAIR of
 // channels of one column group (a warp = the 32 channel pairs of the slice), its KS*KS weight pairs in
-// registers; for each of its four columns it walks the input rows of the window once: KS four-byte
-// shared-memory loads per row (conflict-free: the lanes of a warp are consecutive pairs), each value
-// pair feeds the output rows it belongs to with packed f32x2 FMAs (two channels per instruction).
+// registers; it computes blocks of R x Q outputs, for which every input of the block's window is read once (four-byte
+// shared-memory loads, conflict-free: the lanes of a warp are consecutive pairs) and feeds up to R Q of the taps with packed f32x2
+// FMAs (two channels per instruction).  The sums run over the window's rows and columns in order whatever the block.
+// 7 x 7: the issue slots bound it, so the block has to save loads and conversions: 2 x 7 outputs take 104 loads and as
+// many pairs of conversions for 686 FMAs, a column of 8 rows 98 for 392 (FMA pipe 41 -> 53 % busy; three CTAs an SM at 168 registers):
+// 512 x 56 x 56 x 64 362 -> 317 us, 33 x 64 x 64 x 64 45 -> 41 with 4 x 4, 512 x 28 x 28 x 128 190 -> 184; 4 x 7 blocks spill (329).
+// 3 x 3 is bound by memory: bigger blocks only lost warps (512 x 14 x 14 x 1024 111 -> 117), but for the float32 patch of
+// 14 x 14 planes (48 x 256 channels 16.4 -> 12.3).
 // Tile geometry as template parameters: CG column groups (32 * CG threads), NC columns per group, TH rows;
 // the launcher picks one that divides the plane (8 x 16 tiles on a 28 x 28 plane compute 31 % more
 // outputs than the plane has).
 // OUT: bfloat16 outputs, or float32 ones, whose staged patch is float32 too (the affine is not rounded).
-template <int KS, int CG, int NC, int TH, class OUT>
-__global__ void __launch_bounds__(32 * CG)
+template <int KS, int CG, int NC, int TH, int R, int Q, class OUT>
+__global__ void __launch_bounds__(32 * CG, KS == 7 ? 12 / CG : 1)
 dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ wk,
                     const float* __restrict__ bias, const float* __restrict__ pre_a,
                     const float* __restrict__ pre_b, OUT* __restrict__ y, int H, int W, int C,
                     int add_centre, int gelu) {
+  static_assert(TH % R == 0 && NC % Q == 0, "whole blocks of outputs");
   constexpr int CS = 64, P = (KS - 1) / 2, TW = CG * NC, PW = TW + KS - 1, PH = TH + KS - 1, NT = 32 * CG;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr bool F32 = sizeof(OUT) == 4;
@@ -589,61 +595,76 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
     }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
-  const uint32_t* tile32 = reinterpret_cast<const uint32_t*>(tile);        // [PH][PW][32 pairs]
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
 #pragma unroll 1
-  for (int cc = 0; cc < NC; ++cc) {
-    const int wl = cgp * NC + cc;                    // column inside the tile
-    if (w0 + wl >= W) break;
-    unsigned long long acc[TH];
+  for (int blk = 0; blk < (TH / R) * (NC / Q); ++blk) {
+    const int rl = blk / (NC / Q) * R, wl = cgp * NC + blk % (NC / Q) * Q;       // first row and column inside the tile
+    if (w0 + wl >= W) continue;
+    unsigned long long acc[R][Q];
 #pragma unroll
-    for (int o = 0; o < TH; ++o) acc[o] = bz;
+    for (int o = 0; o < R; ++o)
 #pragma unroll
-    for (int ir = 0; ir < PH; ++ir) {
-      unsigned long long xv[KS];
+      for (int q = 0; q < Q; ++q) acc[o][q] = bz;
+    const OUT* src = tile + ((size_t)rl * PW + wl) * CS + 2 * cp;
 #pragma unroll
-      for (int tj = 0; tj < KS; ++tj) {
-        if constexpr (F32) {
-          const float2 u = *reinterpret_cast<const float2*>(tile + ((size_t)ir * PW + wl + tj) * CS + 2 * cp);
-          xv[tj] = pk2(u.x, u.y);
-        } else {
-          const uint32_t u = tile32[((size_t)ir * PW + wl + tj) * 32 + cp];
-          xv[tj] = pk2(__uint_as_float(u << 16), __uint_as_float(u & 0xFFFF0000u));
+    for (int ir = 0; ir < R + KS - 1; ++ir) {
+      constexpr int NL = KS == 3 ? Q + KS - 1 : 1;                               // values read together
+#pragma unroll
+      for (int j0 = 0; j0 < Q + KS - 1; j0 += NL) {
+        unsigned long long xv[NL];
+#pragma unroll
+        for (int i = 0; i < NL; ++i) {
+          if constexpr (F32) {
+            const float2 u = *reinterpret_cast<const float2*>(src + (ir * PW + j0 + i) * CS);
+            xv[i] = pk2(u.x, u.y);
+          } else {
+            const uint32_t u = *reinterpret_cast<const uint32_t*>(src + (ir * PW + j0 + i) * CS);
+            xv[i] = pk2(__uint_as_float(u << 16), __uint_as_float(u & 0xFFFF0000u));
+          }
         }
-      }
 #pragma unroll
-      for (int o = 0; o < TH; ++o) {
-        const int ti = ir - o;
-        if (ti < 0 || ti >= KS) continue;
+        for (int o = 0; o < R; ++o) {
+          const int ti = ir - o;
+          if (ti < 0 || ti >= KS) continue;
 #pragma unroll
-        for (int tj = 0; tj < KS; ++tj) acc[o] = fma2(xv[tj], wr[ti * KS + tj], acc[o]);
+          for (int i = 0; i < NL; ++i)
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+              const int tj = j0 + i - q;
+              if (tj >= 0 && tj < KS) acc[o][q] = fma2(xv[i], wr[ti * KS + tj], acc[o][q]);
+            }
+        }
       }
     }
 #pragma unroll
-    for (int o = 0; o < TH; ++o) {
-      const int h = h0 + o;
-      if (h >= H) continue;
-      float va, vb;
-      upk2(acc[o], va, vb);
-      if (gelu) gelu_tanh_x2(va, vb);
+    for (int o = 0; o < R; ++o) {
+      const int h = h0 + rl + o;
+      if (h >= H) break;
       OUT* yo = y + (((size_t)n * H + h) * W + w0 + wl) * C + cs0 + 2 * cp;
-      if constexpr (F32) *reinterpret_cast<float2*>(yo) = make_float2(va, vb);
-      else *reinterpret_cast<uint32_t*>(yo) = float2_to_bf16x2(va, vb);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if (w0 + wl + q >= W) break;
+        float va, vb;
+        upk2(acc[o][q], va, vb);
+        if (gelu) gelu_tanh_x2(va, vb);
+        if constexpr (F32) *reinterpret_cast<float2*>(yo + (size_t)q * C) = make_float2(va, vb);
+        else *reinterpret_cast<uint32_t*>(yo + (size_t)q * C) = float2_to_bf16x2(va, vb);
+      }
     }
   }
 }
 
-template <int KS, int CG, int NC, int TH, class OUT>
+template <int KS, int CG, int NC, int TH, int R, int Q, class OUT>
 static int launch_dwconv_tiled(const __nv_bfloat16* x, const float* wk, const float* bias, const float* pre_a,
                                const float* pre_b, OUT* y, int Nimg, int H, int W, int C,
                                int add_centre, int gelu, cudaStream_t st) {
   constexpr int TW = CG * NC;
   const size_t smem = (size_t)(TH + KS - 1) * (TW + KS - 1) * 64 * sizeof(OUT);
-  cudaError_t e = func_smem(dwconv_tiled_kernel<KS, CG, NC, TH, OUT>, smem);
+  cudaError_t e = func_smem(dwconv_tiled_kernel<KS, CG, NC, TH, R, Q, OUT>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   const long long grid = (long long)Nimg * ((H + TH - 1) / TH) * ((W + TW - 1) / TW) * (C / 64);
-  launch_k(dwconv_tiled_kernel<KS, CG, NC, TH, OUT>, (unsigned)grid, 32 * CG, smem, st, x, wk, bias, pre_a, pre_b, y, H, W, C,
+  launch_k(dwconv_tiled_kernel<KS, CG, NC, TH, R, Q, OUT>, (unsigned)grid, 32 * CG, smem, st, x, wk, bias, pre_a, pre_b, y, H, W, C,
                                                                             add_centre, gelu);
   return check_launch();
 }
@@ -654,26 +675,27 @@ int launch_dwconv_cl(const __nv_bfloat16* x, const float* wk, const float* bias,
   if (C % 8 != 0 || (ks != 3 && ks != 7)) return CSSM_ERR_UNSUPPORTED;
   // (float32 outputs, 33 images of 256 pixels: three launches 42 -> 21 us against dwconv_cl_kernel)
   if ((y_f32 == nullptr || ks == 3) && C % 64 == 0 && (wk == nullptr || (aligned16(wk) && (bias == nullptr || aligned16(bias))))) {
-#define CSSM_DW(KS_, CG_, NC_, TH_) \
-  return launch_dwconv_tiled<KS_, CG_, NC_, TH_>(x, wk, bias, pre_a, pre_b, y, Nimg, H, W, C, add_centre, gelu, st)
-#define CSSM_DW3(CG_, NC_, TH_) \
-  return y_f32 != nullptr ? launch_dwconv_tiled<3, CG_, NC_, TH_>(x, wk, bias, pre_a, pre_b, y_f32, Nimg, H, W, C, add_centre, gelu, st) \
-                          : launch_dwconv_tiled<3, CG_, NC_, TH_>(x, wk, bias, pre_a, pre_b, y, Nimg, H, W, C, add_centre, gelu, st)
+#define CSSM_DW(KS_, CG_, NC_, TH_, R_, Q_) \
+  return launch_dwconv_tiled<KS_, CG_, NC_, TH_, R_, Q_>(x, wk, bias, pre_a, pre_b, y, Nimg, H, W, C, add_centre, gelu, st)
+#define CSSM_DW3(CG_, NC_, TH_, R_, QF_, Q_) \
+  return y_f32 != nullptr ? launch_dwconv_tiled<3, CG_, NC_, TH_, R_, QF_>(x, wk, bias, pre_a, pre_b, y_f32, Nimg, H, W, C, add_centre, gelu, st) \
+                          : launch_dwconv_tiled<3, CG_, NC_, TH_, R_, Q_>(x, wk, bias, pre_a, pre_b, y, Nimg, H, W, C, add_centre, gelu, st)
     // Few images: tiles of 4 x 4 outputs while those of the large geometry leave SMs idle.
     const long long large = (long long)Nimg * (C / 64) * (ks == 7 ? (long long)((H + 7) / 8) * ((W + 27) / 28)
                                                                   : (long long)((H + 6) / 7) * ((W + 13) / 14));
     if (large < sm_count()) {
-      if (ks == 7) CSSM_DW(7, 4, 1, 4);
-      CSSM_DW3(4, 1, 4);
+      if (ks == 7) CSSM_DW(7, 4, 1, 4, 4, 1);
+      CSSM_DW3(4, 1, 4, 4, 1, 1);
     }
     if (ks == 7) {
-      if (W % 28 == 0 && H % 8 != 0 && H % 7 == 0) CSSM_DW(7, 4, 7, 7);      // 28 x 28 planes
-      if (W % 28 == 0) CSSM_DW(7, 4, 7, 8);                                  // 56 x 56 planes
-      CSSM_DW(7, 4, 4, 8);
+      // (rows of four where eight would compute an eighth or more in vain: 28 x 28 planes)
+      if (W % 28 == 0 && H < 32 && H % 8 >= 1 && H % 8 <= 4) CSSM_DW(7, 4, 7, 4, 2, 7);
+      if (W % 28 == 0) CSSM_DW(7, 4, 7, 8, 2, 7);                               // 56 x 56 planes
+      CSSM_DW(7, 4, 4, 8, 4, 4);
     }
-    if (W == 14 && H == 14) CSSM_DW3(2, 7, 7);                               // two tiles per plane
-    if (W == 7 && H == 7) CSSM_DW3(1, 7, 7);
-    CSSM_DW3(4, 4, 8);
+    if (W == 14 && H == 14) CSSM_DW3(2, 7, 7, 7, 7, 1);                          // two tiles per plane
+    if (W == 7 && H == 7) CSSM_DW3(1, 7, 7, 7, 1, 1);
+    CSSM_DW3(4, 4, 8, 8, 1, 1);
 #undef CSSM_DW
 #undef CSSM_DW3
   }
