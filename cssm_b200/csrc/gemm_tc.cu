@@ -1,18 +1,21 @@
 // tcgen05 / TMEM GEMM for the K = 64 channel projections in fp32-equivalent precision
 // (3 x TF32: A_hi*B_hi + A_lo*B_hi + A_hi*B_lo, accumulated in fp32 in TMEM).
 //
-// Persistent kernel, one CTA per SM, warp-specialised (16 or 8 producer warps first):
-//   producers            : read a 128-pixel A tile from global memory (channels-last rows with
-//                          RoPE fused, loaded one tile ahead into registers so a whole tile is
-//                          in flight per SM; or planar planes times gate planes), split every value into tf32 hi + remainder, and
-//                          write both into the 128-byte-swizzled K-major operand layout of a
-//                          2-stage ring;
-//   MMA issuer, 1 warp   : one lane issues 24 tcgen05.mma (M128 x N x K8) per tile into one of
-//                          two TMEM accumulators and commits to mbarriers;
+// Persistent kernel, one CTA per SM, 26 warps:
+//   loader, 1 warp       : TMA copies of 128-pixel A tiles as they lie in memory (channels-last rows, or planar planes and
+//                          their gate planes) into a ring of raw tiles;
+//   converters, 16 warps : lane = pixel, 16 of the 64 channels a warp: read the raw tile, apply RoPE or the gate, split every
+//                          value into tf32 hi + remainder and write both to TMEM (tcgen05.st), where the MMAs read their A operand;
+//                          a stage is half of the channels;
+//   MMA issuer, 1 warp   : 24 tcgen05.mma (M128 x N x K8, A in TMEM, B in shared memory) per tile into one of two TMEM
+//                          accumulators, commits to mbarriers;
 //   epilogue, 8 warps    : tcgen05.ld the accumulator (lane = pixel; two warps per TMEM lane
 //                          quadrant, half of the columns each), add bias / activation, store
 //                          planar (coalesced over pixels) or channels-last rows.
 // The weight tile (both halves of the split) is prepared once per CTA and stays in shared memory.
+// With A in shared memory the MMAs' operand reads (6 to 8 KB an instruction) and the converters' stores shared its one port, and the
+// converters, which loaded A through the L1 as well and so kept the rotation tables out of it, set the pace: a clock trace had them
+// at 2000 clocks a tile without RoPE and 2800 to 3700 with it, of 3700 to 5000 in all.
 // Every mbarrier wait is bounded; on expiry the kernel records an error code and winds down.
 #include <cuda.h>
 #include <string.h>
@@ -25,87 +28,76 @@ namespace cssm {
 
 __device__ int g_tc_error = 0;
 
-__device__ inline int gemm_src_frame(const GemmArgs& g, int f) {
-  if (g.a_fmul == 0 && g.a_fadd == 0) return f;
-  return (g.a_fdiv > 1 ? f / g.a_fdiv : f) * g.a_fmul + g.a_fadd;
-}
-__device__ inline int gemm_rope_t(const GemmArgs& g, int f) { return g.rope_tlast ? g.T - 1 : f % g.T; }
-// channels-last A: source row of output row m
-__device__ inline size_t gemm_src_row(const GemmArgs& g, int m) {
-  if (g.a_fmul == 0 && g.a_fadd == 0) return (size_t)m;
-  const int fo = m / g.HW;
-  return (size_t)gemm_src_frame(g, fo) * g.HW + (m - fo * g.HW);
-}
-
 // Forms of the epilogue: plain; ZLAST: the output columns from act_n0 on (the z half of the in_proj) are only produced for the
 // last frame of every clip (last-frame-only forward); MUL: the first g.mul_n output columns multiply planes in place; SUB: the
 // channels-last tensor g.sub is subtracted from the rows.  Compile-time variants, so that the plain one carries no extra test.
 enum TcForm { TC_PLAIN, TC_ZLAST, TC_MUL, TC_SUB };
-// Producer warps.  Sixteen have twice the loads and table reads of eight in flight in half the registers a thread (72 against 96, the
-// epilogue's too): additive block 12 x 8 x 64 x 64 x 64 283 -> 267 us a pass, SimpleCSSM gated 128 x 128^2, T = 8 3087 -> 3060.  The stores
-// that multiply planes in place need those registers (DeltaNet 24 x 12 x 32 x 32 x 64: 474 -> 496 with 16, 470 with 8), and so do
-// the ones that skip frames (gated, last frame only: 1 % slower with 16) and the rows with a tensor to subtract, whose loads are in
-// flight together (NoGate, with 16 / 8: 60 x 8 x 32 x 32 x 64 300 / 285, 12 x 8 x 64 x 64 x 64 221 / 210, 2 x 8 x 32 x 32 36.0 / 35.5).
-template <TcForm FORM> constexpr int tc_prod_warps = FORM == TC_PLAIN ? 16 : 8;
-template <TcForm FORM> constexpr int tc_threads = (tc_prod_warps<FORM> + 9) * 32;      // + MMA warp, 8 epilogue warps
+constexpr int TC_CONV = 16;                                              // converter warps
+constexpr int TC_MMA_WARP = TC_CONV, TC_LOAD_WARP = TC_CONV + 1, TC_EPI_WARP = TC_CONV + 2, TC_THREADS = (TC_CONV + 10) * 32;
 constexpr int TC_BM = 128;
 constexpr int TC_K = 64;
-constexpr uint32_t TC_A_HALF = 2u * TC_BM * 128u;      // one of hi / lo: 2 K-blocks x 128 rows x 128 B
+constexpr uint32_t TC_RAW = TC_BM * TC_K * 4;                            // one raw tile
+constexpr uint32_t TC_ANG = 8 * 32 * 8;                                 // angles of up to eight image rows
+// Divisions by HW, T and the source-frame divisor.
+struct TcGeom { FastDiv hw, t, fdiv; };
 
-// STG = false: the epilogue warps store straight from registers.
-// STG = true : the epilogue stages 16 KB chunks (128 pixels x 32 output columns) in shared memory,
-//              one chunk buffer per half of the epilogue warps, and writes each chunk with one TMA
-//              tensor store (N <= 128: two A stages + two chunk buffers fit in 227 KB).
-template <int N, bool STG>
+// STG = true: the epilogue stages 16 KB chunks (128 pixels x 32 output columns) in shared memory, one chunk buffer per half of the
+// epilogue warps, and writes each chunk with one TMA tensor store (channels-last output, N <= 128); else it stores from registers.
+template <int N, bool GATE, bool STG>
 struct TcSmem {
-  static constexpr uint32_t NSTAGE = 2u;
+  static constexpr int NT = N == 192 ? 1 : 2;                            // tiles of A in TMEM, two stages of 64 columns each
+  static constexpr int NRAW = GATE ? 2 : N == 192 ? 3 : 4;                              // raw tiles in flight
+  static constexpr uint32_t RAW_BYTES = GATE ? 2u * TC_RAW : TC_RAW;
   static constexpr uint32_t B_HALF = 2u * N * 128u;
   static constexpr uint32_t B_OFF = 0;
-  static constexpr uint32_t A_OFF = 2u * B_HALF;                 // after B_hi, B_lo
-  static constexpr uint32_t OUT_OFF = A_OFF + NSTAGE * 2u * TC_A_HALF;   // 2 x 16 KB when STG
+  static constexpr uint32_t RAW_OFF = 2u * B_HALF;                       // after B_hi, B_lo
+  static constexpr uint32_t OUT_OFF = RAW_OFF + NRAW * RAW_BYTES;        // 2 x 16 KB when STG
   static constexpr uint32_t BIAS_OFF = OUT_OFF + (STG ? 2u * 16384u : 0u);
-  static constexpr uint32_t BAR_OFF = BIAS_OFF + N * 4u;
-  static constexpr uint32_t TOTAL = BAR_OFF + 128u;
+  static constexpr uint32_t ANG_OFF = BIAS_OFF + N * 4u;                 // angles of a raw tile's rows: [NRAW][8 rows][32 pairs]
+  static constexpr uint32_t BAR_OFF = ANG_OFF + (STG ? 0u : NRAW * TC_ANG);
+  static constexpr uint32_t TOTAL = BAR_OFF + 256u;
+  static_assert(TOTAL + 1024u <= 227u * 1024u, "one CTA per SM");
 };
 
-template <int N, bool A_PLANAR, bool STG, TcForm FORM = TC_PLAIN>
-__global__ void __launch_bounds__(tc_threads<FORM>, 1)
-gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensorMap omap) {
+template <int N, bool A_PLANAR, bool GATE, bool STG, TcForm FORM = TC_PLAIN>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+gemm_tc_kernel(const GemmArgs g, const TcGeom dv, int num_tiles, const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap gmap,
+               const __grid_constant__ CUtensorMap omap) {
   // tile schedule: round-robin over the CTAs
   const int t_first = blockIdx.x, t_step = gridDim.x, t_end = num_tiles;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // operand tiles need 1024-byte alignment (swizzle atoms); the launch adds 1024 bytes of slack
   unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
-  using L = TcSmem<N, STG>;
-  constexpr int NSTAGE = L::NSTAGE;
+  using L = TcSmem<N, GATE, STG>;
+  constexpr int NT = L::NT, NST = 2 * NT, NRAW = L::NRAW;
   const uint32_t sbase = tc::smem_u32(smem);
   float* bias_s = reinterpret_cast<float*>(smem + L::BIAS_OFF);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-  uint64_t* full = bars;          // [2] A stage written (an arrival a producer warp)
-  uint64_t* empty = bars + 2;     // [2] A stage consumed (tcgen05.commit)
-  uint64_t* accfull = bars + 4;   // [2] accumulator complete (tcgen05.commit)
-  uint64_t* accempty = bars + 6;  // [2] accumulator drained (128 epilogue arrivals)
-  uint64_t* done = bars + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+  uint64_t* raw_full = bars;           // [4] raw tile landed
+  uint64_t* raw_empty = bars + 4;      // [4] and read (16 converter warps)
+  uint64_t* full = bars + 8;           // [4] A stage written (8 converter warps)
+  uint64_t* empty = bars + 12;         // [4] A stage consumed (tcgen05.commit)
+  uint64_t* accfull = bars + 16;       // [2] accumulator complete (tcgen05.commit)
+  uint64_t* accempty = bars + 18;      // [2] accumulator drained (8 epilogue warps)
+  uint64_t* done = bars + 20;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
+  __shared__ int s_bad;                // a bounded wait expired
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr int TC_MMA_WARP = tc_prod_warps<FORM>, TC_THREADS = tc_threads<FORM>;
-  constexpr int NPROD = TC_MMA_WARP * 32;            // producer threads; a lane of each warp arrives on `full`
-  constexpr int TC_ROWS = NPROD / 8;                 // channels-last A: rows of a tile that one round of 16-byte chunks covers
-  constexpr int TC_ITEMS = 2 * TC_BM / TC_ROWS;      // 16-byte chunks of a thread
-  constexpr uint32_t TMEM_COLS = (2 * N <= 32) ? 32 : (2 * N <= 64) ? 64 : (2 * N <= 128) ? 128
-                                 : (2 * N <= 256) ? 256 : 512;
 
+  // RoPE where tiles are whole image rows of 16 pixels or more: a lane's column w is the same in every tile, so its angles stay in
+  // registers, and the loader adds up those of the frame and of the tile's rows for all lanes.
+  const bool one_w = !A_PLANAR && g.rope_t != nullptr && TC_BM % g.W == 0 && g.W >= 16;
   if (tid == 0) {
-    tc::mbar_init(&full[0], NPROD / 32); tc::mbar_init(&full[1], NPROD / 32);      // one lane per producer warp
-    tc::mbar_init(&empty[0], 1); tc::mbar_init(&empty[1], 1);
-    tc::mbar_init(&accfull[0], 1); tc::mbar_init(&accfull[1], 1);
-    tc::mbar_init(&accempty[0], 8); tc::mbar_init(&accempty[1], 8);                  // one lane per epilogue warp
+    for (int i = 0; i < NRAW; ++i) { tc::mbar_init(&raw_full[i], one_w ? 2 : 1); tc::mbar_init(&raw_empty[i], TC_CONV); }
+    for (int i = 0; i < NST; ++i) { tc::mbar_init(&full[i], TC_CONV / 2); tc::mbar_init(&empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { tc::mbar_init(&accfull[i], 1); tc::mbar_init(&accempty[i], 8); }
     tc::mbar_init(done, 1);
     tc::fence_mbar_init();
+    s_bad = 0;
   }
   if (warp == TC_MMA_WARP) {
-    tc::tmem_alloc(tmem_slot, TMEM_COLS);
+    tc::tmem_alloc(tmem_slot, 512);
     tc::tmem_relinquish();
   }
   // ---- weights: W[k][n] -> B_hi / B_lo rows n, K-major swizzled ----
@@ -124,179 +116,183 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_a = tmem_base + 2u * N;            // stages of 64 columns: 32 channels hi, 32 lo
   pdl_sync();
+  // all lanes of a warp agree; a wait that expires is recorded
+  auto wait = [&](uint64_t* bar, uint32_t phase, int code) {
+    const bool ok = !__any_sync(0xffffffffu, !tc::mbar_wait(bar, phase));
+    if (!ok) { if (lane == 0) atomicExch(&g_tc_error, code); s_bad = 1; }
+    return ok;
+  };
 
-  if (warp < TC_MMA_WARP) {
-    // ================================ producers ================================
-    int it = 0;
-    // channels-last mode: the 128 x 16 float4 chunks of a tile are walked in two halves of
-    // TC_ITEMS / 2 iterations: chunk tid & 7 (+ 8 in the second) of rows tid >> 3, + TC_ROWS, ...,
-    // so a warp load touches four rows x 128 contiguous bytes.  RoPE only rotates the low channel
-    // pairs in most modes: a lane rotates in the half whose chunk holds a rotated pair, which
-    // spreads the rotation evenly over the producer warps.  `pre` always holds the NEXT tile.
-    float4 pre[TC_ITEMS];
-    const int chunk_lo = tid & 7, rsub = tid >> 3;
-    bool rot[2] = {false, false};
-    if (!A_PLANAR) {
-      // a tile never crosses a frame (H*W is a multiple of the tile height), so the source-frame
-      // remap is one row offset per tile
-      const int m0 = t_first * TC_BM;
-      const float* a0 = g.A + gemm_src_row(g, m0 < g.M ? m0 : 0) * TC_K;
+  if (warp < TC_CONV) {
+    // ================================ converters ================================
+    const int q = warp & 3, grp = warp >> 2, hf = grp >> 1, sl = grp & 1;     // lane quadrant; 16 channels from 32 hf + 16 sl on
+    const int row = q * 32 + lane, k0 = hf * 32 + sl * 16;
+    const uint32_t tdst = tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)(hf * 64 + sl * 16);
+    bool rot[4] = {false, false, false, false};
+    float4 wang[4];
+    if (!A_PLANAR && g.rope_t != nullptr) {
 #pragma unroll
-      for (int r = 0; r < TC_ITEMS; ++r) {
-        const int row = rsub + TC_ROWS * (r % (TC_ITEMS / 2));
-        const int chunk = chunk_lo + 8 * (r / (TC_ITEMS / 2));
-        pre[r] = (t_first < t_end && m0 + row < g.M)
-                     ? __ldg(reinterpret_cast<const float4*>(a0 + (size_t)row * TC_K + chunk * 4))
-                     : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      if (g.rope_t != nullptr) {
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          const int pi = 2 * (chunk_lo + 8 * hf);
-          rot[hf] = g.rope_nz == nullptr || g.rope_nz[pi] != 0.f || g.rope_nz[pi + 1] != 0.f;
-        }
+      for (int c = 0; c < 4; ++c) {
+        const int pi = (k0 >> 1) + 2 * c;
+        rot[c] = g.rope_nz == nullptr || g.rope_nz[pi] != 0.f || g.rope_nz[pi + 1] != 0.f;
+        wang[c] = one_w && rot[c] ? __ldg(reinterpret_cast<const float4*>(g.rope_w + (row & (g.W - 1)) * 32 + pi)) : make_float4(1.f, 0.f, 1.f, 0.f);
       }
     }
     const float invW = 1.0f / (float)g.W;
+    const int wshift = 31 - __clz(g.W);                       // (one_w)
+    int it = 0;
     for (int tile = t_first; tile < t_end; tile += t_step, ++it) {
-      const int s = it % NSTAGE;
-      const int m0 = tile * TC_BM;
-      float4 cur[TC_ITEMS];
-      if (!A_PLANAR) {
+      const int rs = it % NRAW;
+      float4 th[4];                                          // (cos, sin) of the frame's and the row's angle together, two pairs
+      if (!one_w && (rot[0] || rot[1] || rot[2] || rot[3])) {
+        const int m0 = tile * TC_BM, fr = dv.hw.div(m0), px = m0 - fr * g.HW + row, t = g.rope_tlast ? g.T - 1 : fr - dv.t.div(fr) * g.T;
+        const int h = (int)(((float)px + 0.5f) * invW);     // exact for px < 2^22
 #pragma unroll
-        for (int r = 0; r < TC_ITEMS; ++r) cur[r] = pre[r];
-        const int nt = tile + t_step;
-        if (nt < t_end) {
-          const float* a0 = g.A + gemm_src_row(g, nt * TC_BM) * TC_K;
-#pragma unroll
-          for (int r = 0; r < TC_ITEMS; ++r) {
-            const int row = rsub + TC_ROWS * (r % (TC_ITEMS / 2));
-            const int chunk = chunk_lo + 8 * (r / (TC_ITEMS / 2));
-            pre[r] = (nt * TC_BM + row < g.M)
-                         ? __ldg(reinterpret_cast<const float4*>(a0 + (size_t)row * TC_K + chunk * 4))
-                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int c = 0; c < 4; ++c)
+          if (rot[c]) {
+            const int pi = (k0 >> 1) + 2 * c;
+            const float4 a = __ldg(reinterpret_cast<const float4*>(g.rope_t + t * 32 + pi));
+            const float4 b = __ldg(reinterpret_cast<const float4*>(g.rope_h + h * 32 + pi));
+            th[c] = make_float4(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x, a.z * b.z - a.w * b.w, a.z * b.w + a.w * b.z);
+            wang[c] = __ldg(reinterpret_cast<const float4*>(g.rope_w + (px - h * g.W) * 32 + pi));
           }
-        }
       }
-      // warp-uniform exit: the lanes of a warp meet again at the __syncwarp before the arrive
-      if (__any_sync(0xffffffffu, !tc::mbar_wait(&empty[s], ((it / NSTAGE) & 1) ^ 1))) { atomicExch(&g_tc_error, 1); break; }
-      unsigned char* a_hi = smem + L::A_OFF + (uint32_t)s * 2u * TC_A_HALF;
-      unsigned char* a_lo = a_hi + TC_A_HALF;
+      if (!wait(&raw_full[rs], (it / NRAW) & 1, 1)) break;
+      const unsigned char* raw = smem + L::RAW_OFF + rs * L::RAW_BYTES;
+      float v[16];
       if (!A_PLANAR) {
-        int px0 = 0, t = 0;
-        if (rot[0] || rot[1]) {
-          const int fr = m0 / g.HW;
-          px0 = m0 - fr * g.HW;
-          t = gemm_rope_t(g, fr);
-        }
+        const unsigned char* rp = raw + hf * (TC_BM * 128);
 #pragma unroll
-        for (int r = 0; r < TC_ITEMS; ++r) {
-          const int row = rsub + TC_ROWS * (r % (TC_ITEMS / 2));
-          const int chunk = chunk_lo + 8 * (r / (TC_ITEMS / 2));
-          float4 v = cur[r];
-          if (rot[r / (TC_ITEMS / 2)]) {
-            const int px = px0 + row;
-            const int h = (int)(((float)px + 0.5f) * invW);     // exact for px < 2^22
-            const int w = px - h * g.W;
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const float2 ct = __ldg(&g.rope_t[t * 32 + chunk * 2 + e]);
-              const float2 ch = __ldg(&g.rope_h[h * 32 + chunk * 2 + e]);
-              const float2 cw = __ldg(&g.rope_w[w * 32 + chunk * 2 + e]);
-              const float cx = ct.x * ch.x - ct.y * ch.y, sx = ct.x * ch.y + ct.y * ch.x;
-              const float c2 = cx * cw.x - sx * cw.y, s2 = cx * cw.y + sx * cw.x;
-              float& xe = e ? v.z : v.x;
-              float& xo = e ? v.w : v.y;
-              const float ne = xe * c2 - xo * s2, no = xe * s2 + xo * c2;
-              xe = ne; xo = no;
-            }
-          }
-          float4 h4, l4;
-          tc::split_tf32(v.x, h4.x, l4.x); tc::split_tf32(v.y, h4.y, l4.y);
-          tc::split_tf32(v.z, h4.z, l4.z); tc::split_tf32(v.w, h4.w, l4.w);
-          const uint32_t off = (uint32_t)(chunk >> 3) * (TC_BM * 128u) + tc::sw128_offset(row, chunk & 7);
-          *reinterpret_cast<float4*>(a_hi + off) = h4;
-          *reinterpret_cast<float4*>(a_lo + off) = l4;
+        for (int c = 0; c < 4; ++c) {
+          const float4 x = *reinterpret_cast<const float4*>(rp + tc::sw128_offset(row, sl * 4 + c));
+          v[4 * c] = x.x; v[4 * c + 1] = x.y; v[4 * c + 2] = x.z; v[4 * c + 3] = x.w;
         }
       } else {
-        // thread = (pixel row, part of K); planes are contiguous over pixels, so each k is a
-        // coalesced read across the lanes of a warp
-        const int row = tid & 127, kh = tid >> 7, m = m0 + row;
-        constexpr int KP = TC_K * 128 / NPROD;
-        float v[KP];
-        if (m < g.M) {
-          const int fo = m / g.HW, px = m - fo * g.HW;
-          const int fr = gemm_src_frame(g, fo);
-          const float* ap = g.A + ((size_t)fr * g.a_planes + g.a_plane0 + kh * KP) * g.HW + px;
+        const float* rp = reinterpret_cast<const float*>(raw) + k0 * TC_BM + row;
 #pragma unroll
-          for (int k = 0; k < KP; ++k) v[k] = __ldg(ap + (size_t)k * g.HW);
-          if (g.gate != nullptr) {
-            const float* gp = g.gate + ((size_t)(g.g_compact ? fo : fr) * g.g_planes + g.g_plane0 + kh * KP) * g.HW + px;
+        for (int j = 0; j < 16; ++j) v[j] = rp[j * TC_BM];
+        if (GATE) {
 #pragma unroll
-            for (int k = 0; k < KP; ++k) v[k] *= __ldg(gp + (size_t)k * g.HW);
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < KP; ++k) v[k] = 0.f;
-        }
-#pragma unroll
-        for (int c = 0; c < KP / 4; ++c) {
-          float4 h4, l4;
-          tc::split_tf32(v[4 * c + 0], h4.x, l4.x); tc::split_tf32(v[4 * c + 1], h4.y, l4.y);
-          tc::split_tf32(v[4 * c + 2], h4.z, l4.z); tc::split_tf32(v[4 * c + 3], h4.w, l4.w);
-          const int cg = kh * (KP / 4) + c;
-          const uint32_t off = (uint32_t)(cg >> 3) * (TC_BM * 128u) + tc::sw128_offset(row, cg & 7);
-          *reinterpret_cast<float4*>(a_hi + off) = h4;
-          *reinterpret_cast<float4*>(a_lo + off) = l4;
+          for (int j = 0; j < 16; ++j) v[j] *= rp[(TC_K + j) * TC_BM];
         }
       }
-      tc::fence_proxy_async();
+      if (!A_PLANAR && one_w) {
+        const float4* an = reinterpret_cast<const float4*>(smem + L::ANG_OFF + rs * TC_ANG) + (row >> wshift) * 16 + (k0 >> 2);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (rot[c]) th[c] = an[c];
+      }
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&raw_empty[rs]);
+      const int s = (it % NT) * 2 + hf;
+      if (!wait(&empty[s], ((it / NT) & 1) ^ 1, 1)) break;
+      tc::fence_after_sync();
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {                          // eight channels at a time: registers
+        float* x = v + 8 * p;
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+          if (rot[2 * p + c]) {
+            auto turn = [](float tx, float ty, float wx, float wy, float& x, float& y) {
+              const float c2 = tx * wx - ty * wy, s2 = tx * wy + ty * wx;
+              const float ne = x * c2 - y * s2, no = x * s2 + y * c2;
+              x = ne; y = no;
+            };
+            const float4 a = th[2 * p + c], w = wang[2 * p + c];
+            turn(a.x, a.y, w.x, w.y, x[4 * c], x[4 * c + 1]);
+            turn(a.z, a.w, w.z, w.w, x[4 * c + 2], x[4 * c + 3]);
+          }
+        uint32_t hi[8], lo[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float h, l;
+          tc::split_tf32(x[j], h, l);
+          hi[j] = __float_as_uint(h); lo[j] = __float_as_uint(l);
+        }
+        tc::st_32x32b_x8(tdst + (uint32_t)(it % NT) * 128u + p * 8u, hi);
+        tc::st_32x32b_x8(tdst + (uint32_t)(it % NT) * 128u + 32u + p * 8u, lo);
+      }
+      tc::wait_st();
+      tc::fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&full[s]);
     }
+  } else if (warp == TC_LOAD_WARP) {
+    // ================================ loader ================================
+    const int nrow = one_w ? TC_BM / g.W : 0;
+    int it = 0;
+    for (int tile = t_first; tile < t_end; tile += t_step, ++it) {
+      const int rs = it % NRAW;
+      const int m0 = tile * TC_BM, fo = dv.hw.div(m0), px0 = m0 - fo * g.HW;
+      const int fr = (g.a_fmul == 0 && g.a_fadd == 0) ? fo : dv.fdiv.div(fo) * g.a_fmul + g.a_fadd;
+      if (!wait(&raw_empty[rs], ((it / NRAW) & 1) ^ 1, 5)) break;
+      if (tc::elect_one()) {
+        unsigned char* raw = smem + L::RAW_OFF + rs * L::RAW_BYTES;
+        tc::mbar_expect_tx(&raw_full[rs], L::RAW_BYTES);
+        if (!A_PLANAR) {
+          tc::tma_load_2d(raw, &amap, 0, fr * g.HW + px0, &raw_full[rs]);
+          tc::tma_load_2d(raw + TC_BM * 128, &amap, 32, fr * g.HW + px0, &raw_full[rs]);
+        } else {
+          tc::tma_load_3d(raw, &amap, px0, g.a_plane0, fr, &raw_full[rs]);
+          if (GATE) tc::tma_load_3d(raw + TC_RAW, &gmap, px0, g.g_plane0, g.g_compact ? fo : fr, &raw_full[rs]);
+        }
+      }
+      __syncwarp();
+      if (!A_PLANAR && one_w) {
+        const int t = g.rope_tlast ? g.T - 1 : fo - dv.t.div(fo) * g.T, h0 = px0 >> (31 - __clz(g.W));
+        const float2 a = __ldg(g.rope_t + t * 32 + lane);
+        float2* an = reinterpret_cast<float2*>(smem + L::ANG_OFF + rs * TC_ANG) + lane;
+        for (int r = 0; r < nrow; ++r) {
+          const float2 b = __ldg(g.rope_h + (h0 + r) * 32 + lane);
+          an[r * 32] = make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&raw_full[rs]);
+      }
+    }
   } else if (warp == TC_MMA_WARP) {
     // ================================ MMA issuer ================================
-    if (lane == 0) {
-      const uint32_t idesc = tc::make_idesc_tf32(TC_BM, N);
-      const uint32_t b_hi = sbase + L::B_OFF, b_lo = b_hi + L::B_HALF;
-      int it = 0;
-      bool ok = true;
-      for (int tile = t_first; tile < t_end; tile += t_step, ++it) {
-        const int s = it % NSTAGE, sph = (it / NSTAGE) & 1;    // A stage and its phase
-        const int ac = it & 1, ph = (it >> 1) & 1;              // accumulator and its phase
-        if (!tc::mbar_wait(&accempty[ac], ph ^ 1) || !tc::mbar_wait(&full[s], sph)) {
-          atomicExch(&g_tc_error, 2); ok = false; break;
-        }
+    // The whole warp walks the loop, one lane issues (elect_one).
+    const uint32_t idesc = tc::make_idesc_tf32(TC_BM, N);
+    const uint64_t b_hi = tc::make_desc_sw128(sbase + L::B_OFF), b_lo = tc::make_desc_sw128(sbase + L::B_OFF + L::B_HALF);
+    int it = 0;
+    bool ok = true;
+    for (int tile = t_first; tile < t_end && ok; tile += t_step, ++it) {
+      const int ac = it & 1, ph = (it >> 1) & 1;              // accumulator and its phase
+      if (!(ok = wait(&accempty[ac], ph ^ 1, 2))) break;
+      const uint32_t d = tmem_base + (uint32_t)ac * N;
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const int s = (it % NT) * 2 + hf;
+        if (!(ok = wait(&full[s], (it / NT) & 1, 2))) break;
         tc::fence_after_sync();
-        const uint32_t a_hi = sbase + L::A_OFF + (uint32_t)s * 2u * TC_A_HALF, a_lo = a_hi + TC_A_HALF;
-        const uint32_t d = tmem_base + (uint32_t)ac * N;
-        uint32_t acc = 0;
+        const uint32_t a = tmem_a + (uint32_t)s * 64u;
+        if (tc::elect_one()) {
 #pragma unroll
-        for (int pass = 0; pass < 3; ++pass) {
-          const uint32_t ab = pass == 1 ? a_lo : a_hi;
-          const uint32_t bb = pass == 2 ? b_lo : b_hi;
+          for (int pass = 0; pass < 3; ++pass) {
+            const uint32_t ab = pass == 1 ? a + 32u : a;
+            const uint64_t bb = (pass == 2 ? b_lo : b_hi) + (uint64_t)(hf * (N * 128u >> 4));
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint32_t koff = (uint32_t)(ks & 3) * 32u;
-            const uint64_t ad = tc::make_desc_sw128(ab + (uint32_t)(ks >> 2) * (TC_BM * 128u) + koff);
-            const uint64_t bd = tc::make_desc_sw128(bb + (uint32_t)(ks >> 2) * (N * 128u) + koff);
-            tc::mma_tf32(d, ad, bd, idesc, acc);
-            acc = 1;
+            for (int ks = 0; ks < 4; ++ks) tc::mma_tf32_ts(d, ab + ks * 8u, bb + ks * 2, idesc, (hf | pass | ks) ? 1u : 0u);
           }
+          tc::commit(&empty[s]);
         }
-        tc::commit(&empty[s]);
-        tc::commit(&accfull[ac]);
+        __syncwarp();
       }
-      // nothing of this thread's tensor work may be in flight when TMEM is freed
-      tc::commit(done);
-      if (!tc::mbar_wait(done, 0) && ok) atomicExch(&g_tc_error, 3);
+      if (ok && tc::elect_one()) tc::commit(&accfull[ac]);
+      __syncwarp();
     }
+    // nothing of this warp's tensor work may be in flight when TMEM is freed
+    if (tc::elect_one()) tc::commit(done);
     __syncwarp();
-  } else if (warp > TC_MMA_WARP) {
+    if (!tc::mbar_wait(done, 0) && ok) atomicExch(&g_tc_error, 3);
+    __syncwarp();
+  } else {
     // ================================ epilogue ================================
     const int q = warp & 3;                 // TMEM lane quadrant this warp may read
-    const int half = (warp - (TC_MMA_WARP + 1)) >> 2;   // which half of the N columns
+    const int half = (warp - TC_EPI_WARP) >> 2;   // which half of the N columns
     const int row = q * 32 + lane;
     int it = 0;
     for (int tile = t_first; tile < t_end; tile += t_step, ++it) {
@@ -315,19 +311,19 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
       } else {
         ok = !__any_sync(0xffffffffu, !ok);
       }
-      if (!ok) { atomicExch(&g_tc_error, 4); break; }
+      if (!ok) { atomicExch(&g_tc_error, 4); s_bad = 1; break; }
       tc::fence_after_sync();
-      const int m = tile * TC_BM + row;
+      const int m = tile * TC_BM + row, fr = dv.hw.div(tile * TC_BM), px = m - fr * g.HW;
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)s * N;
 #pragma unroll 1
       for (int cc = half * (N / 64); cc < (half + 1) * (N / 64); ++cc) {
-        if (FORM == TC_ZLAST && cc * 32 >= g.act_n0 && (m / g.HW) % g.T != g.T - 1) continue;   // tile-uniform
+        if (FORM == TC_ZLAST && cc * 32 >= g.act_n0 && fr - dv.t.div(fr) * g.T != g.T - 1) continue;   // tile-uniform
         uint32_t r[32];
         tc::ld_32x32b_x32(taddr + cc * 32, r);
         tc::wait_ld();
         if (STG) {
           // this half's 128 threads share two 16 KB staging chunks and named barrier 1 + half
-          const int grp_tid = tid - (TC_MMA_WARP + 1 + 4 * half) * 32;      // 0..127
+          const int grp_tid = tid - (TC_EPI_WARP + 4 * half) * 32;      // 0..127
           float* stg = reinterpret_cast<float*>(smem + L::OUT_OFF) + half * 4096;
           // the TMA store that last read this chunk buffer must have drained it
           if (grp_tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -369,8 +365,7 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
           if (grp_tid == 0) {
             const int m0 = tile * TC_BM;
             if (!A_PLANAR) {
-              const int fr = m0 / g.HW, px0 = m0 - fr * g.HW;
-              tc::tma_store_3d(&omap, stg, px0, g.o_plane0 + cc * 32, fr);
+              tc::tma_store_3d(&omap, stg, px - row, g.o_plane0 + cc * 32, fr);
             } else {
               tc::tma_store_2d(&omap, stg, cc * 32, m0);
             }
@@ -383,7 +378,6 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
             // planar output: lanes = consecutive pixels -> 128-byte coalesced stores per column.
             // All 32 values are finished in registers before the first store: the stores go
             // through a generic pointer, so bias loads placed between them could not be hoisted.
-            const int fr = m / g.HW, px = m - fr * g.HW;
             float* op = g.out + ((size_t)fr * g.o_planes + g.o_plane0 + cc * 32) * g.HW + px;
             const float* bs = bias_s + cc * 32;
             float vals[32];
@@ -433,9 +427,12 @@ gemm_tc_kernel(const GemmArgs g, int num_tiles, const __grid_constant__ CUtensor
   }
   tc::fence_before_sync();
   __syncthreads();
+  // error path only: give copies that may still be in flight a bounded time (~1 ms) to land
+  if (s_bad)
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   if (warp == TC_MMA_WARP) {
     tc::fence_after_sync();
-    tc::tmem_dealloc(tmem_base, TMEM_COLS);
+    tc::tmem_dealloc(tmem_base, 512);
   }
 }
 
@@ -481,20 +478,54 @@ static bool make_out_map(const GemmArgs& g, bool a_planar, CUtensorMap* map) {
   return r == CUDA_SUCCESS;
 }
 
-template <int N, bool A_PLANAR, bool STG, TcForm FORM>
-static int launch_tc_v(const GemmArgs& g, const CUtensorMap& map, cudaStream_t st) {
+// Tensor maps of A (and of the gate planes): boxes of 128 rows x 32 channels, 128-byte swizzle, or of 128 pixels x 64 planes.
+// The rows of a channels-last A are those of its source frames, which may be fewer or more than the output's: the map covers
+// all that the tiles name.
+static bool make_in_map(const GemmArgs& g, bool a_planar, bool gate, CUtensorMap* map) {
+  const tc::EncodeTiledFn enc = tc::encode_fn();
+  if (!enc) return false;
+  const int fo = g.M / g.HW;                                       // output frames; their last source frame
+  const bool remap = (g.a_fmul != 0 || g.a_fadd != 0) && !(gate && g.g_compact);
+  const cuuint64_t frames = remap ? (cuuint64_t)((g.a_fdiv > 1 ? (fo - 1) / g.a_fdiv : fo - 1) * (long long)g.a_fmul + g.a_fadd + 1) : (cuuint64_t)fo;
+  const cuuint32_t es[3] = {1, 1, 1};
+  CUresult r;
+  if (!a_planar) {
+    const cuuint64_t dims[2] = {TC_K, frames * g.HW};
+    const cuuint64_t strides[1] = {TC_K * 4};
+    const cuuint32_t box[2] = {32, TC_BM};
+    r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(g.A), dims, strides, box, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  } else {
+    const int planes = gate ? g.g_planes : g.a_planes;
+    const cuuint64_t dims[3] = {(cuuint64_t)g.HW, (cuuint64_t)planes, frames};
+    const cuuint64_t strides[2] = {(cuuint64_t)g.HW * 4, (cuuint64_t)planes * g.HW * 4};
+    const cuuint32_t box[3] = {TC_BM, TC_K, 1};
+    r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(gate ? g.gate : g.A), dims, strides, box, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  }
+  return r == CUDA_SUCCESS;
+}
+
+template <int N, bool A_PLANAR, bool GATE, bool STG, TcForm FORM>
+static int launch_tc_v(const GemmArgs& g, const CUtensorMap& omap, cudaStream_t st) {
   const int num_tiles = g.M / TC_BM;
   const int sms = sm_count();
   cudaError_t e;
   const int grid = num_tiles < sms ? num_tiles : sms;
-  const size_t smem = TcSmem<N, STG>::TOTAL + 1024;      // slack for the 1024-byte alignment
-  e = func_smem(gemm_tc_kernel<N, A_PLANAR, STG, FORM>, smem);
+  const size_t smem = TcSmem<N, GATE, STG>::TOTAL + 1024;      // slack for the 1024-byte alignment
+  e = func_smem(gemm_tc_kernel<N, A_PLANAR, GATE, STG, FORM>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
+  CUtensorMap amap, gmap;
+  memset(&gmap, 0, sizeof(gmap));
+  if (!make_in_map(g, A_PLANAR, false, &amap) || (GATE && !make_in_map(g, true, true, &gmap))) return CSSM_ERR_CUDA;
   // Planes of 64x64: the 64 planes of a tile lie 1 MB apart in all, which neighbouring SMs share (NoGate's output
   // projection of 48 x 4 frames: 104 us in grid order, 139 with the CTAs where SMs came free); 8 x 4 frames and less, and
   // smaller planes, gain more by the early start.  Channels-last input: the second projection of the same rows.
   const PdlOff alone(N == 64 && num_tiles > 8 * sms && (!A_PLANAR || g.HW >= 4096));
-  launch_k(gemm_tc_kernel<N, A_PLANAR, STG, FORM>, grid, tc_threads<FORM>, smem, st, g, num_tiles, map);
+  const TcGeom dv = {FastDiv(g.HW), FastDiv(g.T > 0 ? g.T : 1), FastDiv(g.a_fdiv > 1 ? g.a_fdiv : 1)};
+  launch_k(gemm_tc_kernel<N, A_PLANAR, GATE, STG, FORM>, grid, TC_THREADS, smem, st, g, dv, num_tiles, amap, gmap, omap);
   return check_launch();
 }
 
@@ -502,13 +533,13 @@ template <int N, bool A_PLANAR, TcForm FORM = TC_PLAIN>
 static int launch_tc(const GemmArgs& g, cudaStream_t st) {
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
-  // TMA-store epilogue for the channels-last output (planar A) unless the driver entry point is
-  // missing.  For the planar output it measured slower than direct stores (2.1 ms vs 1.44 ms on
-  // the in_proj of cfg2), so that direction keeps direct stores.
-  const bool stg = A_PLANAR && N <= 128 && (reinterpret_cast<uintptr_t>(g.out) & 15u) == 0 &&
-                   make_out_map(g, A_PLANAR, &map);
-  if (N <= 128 && stg) return launch_tc_v<N, A_PLANAR, A_PLANAR && (N <= 128), FORM>(g, map, st);
-  return launch_tc_v<N, A_PLANAR, false, FORM>(g, map, st);
+  if constexpr (!A_PLANAR) {
+    // (planar output: TMA stores measured slower than direct ones, 2.1 against 1.44 ms on an in_proj of 4.2 M rows)
+    return launch_tc_v<N, false, false, false, FORM>(g, map, st);
+  } else {
+    if (!make_out_map(g, true, &map)) return CSSM_ERR_CUDA;
+    return g.gate != nullptr ? launch_tc_v<N, true, true, true, FORM>(g, map, st) : launch_tc_v<N, true, false, true, FORM>(g, map, st);
+  }
 }
 
 int launch_gemm_tc(const GemmArgs& g, bool a_planar, cudaStream_t st) {
