@@ -70,6 +70,16 @@ __device__ __forceinline__ float tanh_approx(float u) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
   return t;
 }
+// 1 / (1 + e^-x) of a pair: e^-x as 2^(-x log2 e), two special functions a value and packed arithmetic around them (half the
+// instructions of the scalar form, whose exponential also scales denormal results; here they are zero beside the 1)
+__device__ __forceinline__ unsigned long long sigmoid_x2(unsigned long long x) {
+  float a, b, c, d;
+  upk2(mul2(x, pk2(-1.4426950408889634f, -1.4426950408889634f)), a, b);
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(c) : "f"(a));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(d) : "f"(b));
+  upk2(add2(pk2(c, d), pk2(1.0f, 1.0f)), a, b);
+  return pk2(rcp_fast(a), rcp_fast(b));
+}
 // gelu (tanh form) of a and b in place
 __device__ __forceinline__ void gelu_tanh_x2(float& a, float& b) {
   const unsigned long long x = pk2(a, b);

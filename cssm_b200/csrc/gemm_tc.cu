@@ -1,27 +1,30 @@
 // tcgen05 / TMEM GEMM for the K = 64 channel projections in fp32-equivalent precision
-// (3 x TF32: A_hi*B_hi + A_lo*B_hi + A_hi*B_lo, accumulated in fp32 in TMEM).
+// (3 x TF32: A_lo*B_hi + A_hi*B_lo + A_hi*B_hi, accumulated in fp32 in TMEM).
 //
 // Persistent kernel, one CTA per SM, 26 warps:
 //   loader, 1 warp       : TMA copies of 128-pixel A tiles as they lie in memory (channels-last rows, or planar planes and
-//                          their gate planes) into a ring of raw tiles;
-//   converters, 16 warps : lane = pixel, 16 of the 64 channels a warp: read the raw tile, apply RoPE or the gate, split every
+//                          their gate planes) into a ring of raw tiles, and the angles of the tile's frame and rows;
+//   converters, 16 or 8  : lane = pixel, 16 of the 64 channels at a time: read the raw tile, apply RoPE or the gate, split every
 //                          value into tf32 hi + remainder and write both to TMEM (tcgen05.st), where the MMAs read their A operand;
 //                          a stage is half of the channels;
 //   MMA issuer, 1 warp   : 24 tcgen05.mma (M128 x N x K8, A in TMEM, B in shared memory) per tile into one of two TMEM
 //                          accumulators, commits to mbarriers;
-//   epilogue, 8 warps    : tcgen05.ld the accumulator (lane = pixel; two warps per TMEM lane
-//                          quadrant, half of the columns each), add bias / activation, store
+//   epilogue, 8 or 16    : tcgen05.ld the accumulator (lane = pixel; two or four warps per TMEM lane
+//                          quadrant, a share of the columns each), add bias / activation, store
 //                          planar (coalesced over pixels) or channels-last rows.
 // The weight tile (both halves of the split) is prepared once per CTA and stays in shared memory.
 // With A in shared memory the MMAs' operand reads (6 to 8 KB an instruction) and the converters' stores shared its one port, and the
 // converters, which loaded A through the L1 as well and so kept the rotation tables out of it, set the pace: a clock trace had them
-// at 2000 clocks a tile without RoPE and 2800 to 3700 with it, of 3700 to 5000 in all.
+// at 2000 clocks a tile without RoPE and 2800 to 3700 with it, of 3700 to 5000 in all.  4.2 M rows, us: 64 -> 128 columns 631 -> 429, planes
+// -> 64 435 -> 359, 64 -> 64 with sigmoid 472 -> 330 (rows of repeated frames 619 -> 345), planes under RMS and gate 706 (gemm_split) ->
+// 507; HBM's copy rate allows 493, 328, 328 (164) and 493.  98 K rows of 64 -> 128 + 64 in place 137 -> 110.
+// Bound now: HBM for the planes, issue slots (65 to 70 % busy) where little is read.
 // Every mbarrier wait is bounded; on expiry the kernel records an error code and winds down.
 #include <cuda.h>
 #include <string.h>
 #include "kernels.cuh"
-#include "gemm.cuh"
-#include "tc05.cuh"
+#include "gemm_tc.cuh"
+#include "bf16_ops.cuh"
 #include "stem.cuh"
 
 namespace cssm {
@@ -31,22 +34,34 @@ __device__ int g_tc_error = 0;
 // Forms of the epilogue: plain; ZLAST: the output columns from act_n0 on (the z half of the in_proj) are only produced for the
 // last frame of every clip (last-frame-only forward); MUL: the first g.mul_n output columns multiply planes in place; SUB: the
 // channels-last tensor g.sub is subtracted from the rows.  Compile-time variants, so that the plain one carries no extra test.
-enum TcForm { TC_PLAIN, TC_ZLAST, TC_MUL, TC_SUB };
-constexpr int TC_CONV = 16;                                              // converter warps
-constexpr int TC_MMA_WARP = TC_CONV, TC_LOAD_WARP = TC_CONV + 1, TC_EPI_WARP = TC_CONV + 2, TC_THREADS = (TC_CONV + 10) * 32;
-constexpr int TC_BM = 128;
-constexpr int TC_K = 64;
-constexpr uint32_t TC_RAW = TC_BM * TC_K * 4;                            // one raw tile
-constexpr uint32_t TC_ANG = 8 * 32 * 8;                                 // angles of up to eight image rows
-// Divisions by HW, T and the source-frame divisor.
-struct TcGeom { FastDiv hw, t, fdiv; };
+// RMS (planar A, 64 columns): a <- a * rsqrt(mean_k a^2 + eps) * scale[k]; the scale goes into the weights, the row factor to the accumulator.
+enum TcForm { TC_PLAIN, TC_ZLAST, TC_MUL, TC_SUB, TC_RMS };
+// Warps: converters, MMA issuer, loader, epilogue.  A wide planar output has more to store than to convert (with sixteen converters and
+// eight epilogue warps: 4.2 M rows to 128 columns 491 us, 429 so; DeltaNet 32x32, whose 192 columns multiply planes, 462 and 415 a pass).
+template <int N, bool A_PLANAR> constexpr int tc_conv = (!A_PLANAR && N > 64) ? 8 : 16;
+constexpr int TC_THREADS = 26 * 32;
+
+// One output of a planar A under the RMS prologue by float32 FMAs over k: for results that are not finite (the products are taken
+// before the row factor, and an infinity has no finite parts).
+__device__ __noinline__ float tc_planar_fma(const GemmArgs& g, const TcGeom& dv, int m, int n, float rinv) {
+  const int fo = dv.hw.div(m), px = m - fo * g.HW, fr = tc_src_frame(g, dv, fo);
+  const float* ap = g.A + ((size_t)fr * g.a_planes + g.a_plane0) * g.HW + px;
+  const float* gp = g.gate ? g.gate + ((size_t)(g.g_compact ? fo : fr) * g.g_planes + g.g_plane0) * g.HW + px : nullptr;
+  float v = 0.f;
+  for (int k = 0; k < TC_K; ++k) {
+    float x = ap[(size_t)k * g.HW] * (rinv * g.rms_scale[k]);
+    if (gp != nullptr) x *= gp[(size_t)k * g.HW];
+    v = fmaf(x, g.Wk[(size_t)k * g.N + n], v);
+  }
+  return g.bias != nullptr ? v + g.bias[n] : v;
+}
 
 // STG = true: the epilogue stages 16 KB chunks (128 pixels x 32 output columns) in shared memory, one chunk buffer per half of the
 // epilogue warps, and writes each chunk with one TMA tensor store (channels-last output, N <= 128); else it stores from registers.
-template <int N, bool GATE, bool STG>
+template <int N, bool GATE, bool STG, bool RMS = false>
 struct TcSmem {
   static constexpr int NT = N == 192 ? 1 : 2;                            // tiles of A in TMEM, two stages of 64 columns each
-  static constexpr int NRAW = GATE ? 2 : N == 192 ? 3 : 4;                              // raw tiles in flight
+  static constexpr int NRAW = GATE ? 2 : N == 192 ? 3 : 4;          // raw tiles in flight
   static constexpr uint32_t RAW_BYTES = GATE ? 2u * TC_RAW : TC_RAW;
   static constexpr uint32_t B_HALF = 2u * N * 128u;
   static constexpr uint32_t B_OFF = 0;
@@ -54,21 +69,25 @@ struct TcSmem {
   static constexpr uint32_t OUT_OFF = RAW_OFF + NRAW * RAW_BYTES;        // 2 x 16 KB when STG
   static constexpr uint32_t BIAS_OFF = OUT_OFF + (STG ? 2u * 16384u : 0u);
   static constexpr uint32_t ANG_OFF = BIAS_OFF + N * 4u;                 // angles of a raw tile's rows: [NRAW][8 rows][32 pairs]
-  static constexpr uint32_t BAR_OFF = ANG_OFF + (STG ? 0u : NRAW * TC_ANG);
-  static constexpr uint32_t TOTAL = BAR_OFF + 256u;
+  static constexpr uint32_t WANG_OFF = ANG_OFF + (STG ? 0u : NRAW * TC_ANG);
+  static constexpr uint32_t BAR_OFF = WANG_OFF + (STG ? 0u : TC_WANG);
+  static constexpr uint32_t SS_OFF = BAR_OFF + 256u;                     // RMS: [4 tiles][4 parts of the channels][128] sums of squares
+  static constexpr uint32_t TOTAL = SS_OFF + (RMS ? 4u * 4u * 128u * 4u : 0u);
   static_assert(TOTAL + 1024u <= 227u * 1024u, "one CTA per SM");
 };
 
 template <int N, bool A_PLANAR, bool GATE, bool STG, TcForm FORM = TC_PLAIN>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-gemm_tc_kernel(const GemmArgs g, const TcGeom dv, int num_tiles, const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap gmap,
+gemm_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ TcGeom dv, int num_tiles, const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap gmap,
                const __grid_constant__ CUtensorMap omap) {
   // tile schedule: round-robin over the CTAs
   const int t_first = blockIdx.x, t_step = gridDim.x, t_end = num_tiles;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // operand tiles need 1024-byte alignment (swizzle atoms); the launch adds 1024 bytes of slack
   unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
-  using L = TcSmem<N, GATE, STG>;
+  using L = TcSmem<N, GATE, STG, FORM == TC_RMS>;
+  constexpr int CONV = tc_conv<N, A_PLANAR>, EPI = 24 - CONV;
+  constexpr int MMA_WARP = CONV, LOAD_WARP = CONV + 1, EPI_WARP = CONV + 2;
   constexpr int NT = L::NT, NST = 2 * NT, NRAW = L::NRAW;
   const uint32_t sbase = tc::smem_u32(smem);
   float* bias_s = reinterpret_cast<float*>(smem + L::BIAS_OFF);
@@ -85,31 +104,21 @@ gemm_tc_kernel(const GemmArgs g, const TcGeom dv, int num_tiles, const __grid_co
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  // RoPE where tiles are whole image rows of 16 pixels or more: a lane's column w is the same in every tile, so its angles stay in
-  // registers, and the loader adds up those of the frame and of the tile's rows for all lanes.
-  const bool one_w = !A_PLANAR && g.rope_t != nullptr && TC_BM % g.W == 0 && g.W >= 16;
+  const bool rope_s = !A_PLANAR && tc_rope_shared(g);
   if (tid == 0) {
-    for (int i = 0; i < NRAW; ++i) { tc::mbar_init(&raw_full[i], one_w ? 2 : 1); tc::mbar_init(&raw_empty[i], TC_CONV); }
-    for (int i = 0; i < NST; ++i) { tc::mbar_init(&full[i], TC_CONV / 2); tc::mbar_init(&empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { tc::mbar_init(&accfull[i], 1); tc::mbar_init(&accempty[i], 8); }
+    for (int i = 0; i < NRAW; ++i) { tc::mbar_init(&raw_full[i], rope_s ? 2 : 1); tc::mbar_init(&raw_empty[i], CONV); }
+    for (int i = 0; i < NST; ++i) { tc::mbar_init(&full[i], CONV / 2); tc::mbar_init(&empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { tc::mbar_init(&accfull[i], 1); tc::mbar_init(&accempty[i], EPI); }
     tc::mbar_init(done, 1);
     tc::fence_mbar_init();
     s_bad = 0;
   }
-  if (warp == TC_MMA_WARP) {
+  if (warp == MMA_WARP) {
     tc::tmem_alloc(tmem_slot, 512);
     tc::tmem_relinquish();
   }
-  // ---- weights: W[k][n] -> B_hi / B_lo rows n, K-major swizzled ----
-  for (int item = tid; item < N * 16; item += TC_THREADS) {
-    const int n = item % N, c = item / N;               // c: 16-byte chunk of 4 k values
-    float hi[4], lo[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) tc::split_tf32(g.Wk[(size_t)(4 * c + e) * g.N + n], hi[e], lo[e]);
-    const uint32_t off = (uint32_t)(c >> 3) * (N * 128u) + tc::sw128_offset(n, c & 7);
-    *reinterpret_cast<float4*>(smem + L::B_OFF + off) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-    *reinterpret_cast<float4*>(smem + L::B_OFF + L::B_HALF + off) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-  }
+  tc_split_weights<N, FORM == TC_RMS>(g.Wk, g.N, 0, smem + L::B_OFF, smem + L::B_OFF + L::B_HALF, tid, TC_THREADS, g.rms_scale);
+  if (rope_s) tc_rope_columns(g, smem + L::WANG_OFF, tid, TC_THREADS);
   for (int n = tid; n < N; n += TC_THREADS) bias_s[n] = g.bias ? g.bias[n] : 0.f;
   tc::fence_proxy_async();
   tc::fence_before_sync();
@@ -125,108 +134,61 @@ gemm_tc_kernel(const GemmArgs g, const TcGeom dv, int num_tiles, const __grid_co
     return ok;
   };
 
-  if (warp < TC_CONV) {
+  if (warp < CONV) {
     // ================================ converters ================================
-    const int q = warp & 3, grp = warp >> 2, hf = grp >> 1, sl = grp & 1;     // lane quadrant; 16 channels from 32 hf + 16 sl on
-    const int row = q * 32 + lane, k0 = hf * 32 + sl * 16;
-    const uint32_t tdst = tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)(hf * 64 + sl * 16);
-    bool rot[4] = {false, false, false, false};
-    float4 wang[4];
-    if (!A_PLANAR && g.rope_t != nullptr) {
+    // channels 32 hf + 16 sl .. + 15 of the quadrant's pixels; of eight warps each has both sl
+    const int q = warp & 3, grp = warp >> 2, hf = CONV == 16 ? grp >> 1 : grp, sl0 = CONV == 16 ? grp & 1 : 0;
+    const int row = q * 32 + lane;
+    const uint32_t tdst = tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)(hf * 64);
+    uint32_t rot[16 / CONV];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int pi = (k0 >> 1) + 2 * c;
-        rot[c] = g.rope_nz == nullptr || g.rope_nz[pi] != 0.f || g.rope_nz[pi + 1] != 0.f;
-        wang[c] = one_w && rot[c] ? __ldg(reinterpret_cast<const float4*>(g.rope_w + (row & (g.W - 1)) * 32 + pi)) : make_float4(1.f, 0.f, 1.f, 0.f);
-      }
-    }
-    const float invW = 1.0f / (float)g.W;
-    const int wshift = 31 - __clz(g.W);                       // (one_w)
+    for (int i = 0; i < 16 / CONV; ++i) rot[i] = A_PLANAR ? 0u : tc_rotated(g, hf * 32 + (sl0 + i) * 16);
     int it = 0;
     for (int tile = t_first; tile < t_end; tile += t_step, ++it) {
-      const int rs = it % NRAW;
-      float4 th[4];                                          // (cos, sin) of the frame's and the row's angle together, two pairs
-      if (!one_w && (rot[0] || rot[1] || rot[2] || rot[3])) {
-        const int m0 = tile * TC_BM, fr = dv.hw.div(m0), px = m0 - fr * g.HW + row, t = g.rope_tlast ? g.T - 1 : fr - dv.t.div(fr) * g.T;
-        const int h = (int)(((float)px + 0.5f) * invW);     // exact for px < 2^22
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (rot[c]) {
-            const int pi = (k0 >> 1) + 2 * c;
-            const float4 a = __ldg(reinterpret_cast<const float4*>(g.rope_t + t * 32 + pi));
-            const float4 b = __ldg(reinterpret_cast<const float4*>(g.rope_h + h * 32 + pi));
-            th[c] = make_float4(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x, a.z * b.z - a.w * b.w, a.z * b.w + a.w * b.z);
-            wang[c] = __ldg(reinterpret_cast<const float4*>(g.rope_w + (px - h * g.W) * 32 + pi));
-          }
+      const int rs = it % NRAW, s = (it % NT) * 2 + hf;
+      const unsigned char* raw = smem + L::RAW_OFF + rs * L::RAW_BYTES;
+      int t = 0, px = 0;
+      if (!A_PLANAR && !rope_s && g.rope_t != nullptr) {
+        const int m0 = tile * TC_BM, fr = dv.hw.div(m0);
+        px = m0 - fr * g.HW + row;
+        t = tc_rope_t(g, dv, fr);
       }
       if (!wait(&raw_full[rs], (it / NRAW) & 1, 1)) break;
-      const unsigned char* raw = smem + L::RAW_OFF + rs * L::RAW_BYTES;
-      float v[16];
-      if (!A_PLANAR) {
-        const unsigned char* rp = raw + hf * (TC_BM * 128);
+      bool ok = true;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float4 x = *reinterpret_cast<const float4*>(rp + tc::sw128_offset(row, sl * 4 + c));
-          v[4 * c] = x.x; v[4 * c + 1] = x.y; v[4 * c + 2] = x.z; v[4 * c + 3] = x.w;
+      for (int i = 0; i < 16 / CONV; ++i) {
+        const int sl = sl0 + i, k0 = hf * 32 + sl * 16;
+        float v[16], ss = 0.f;
+        if (!A_PLANAR) {
+          tc_read16_rows(raw, row, k0, v);
+          tc_rotate16(g, rope_s, rot[i], smem + L::ANG_OFF + rs * TC_ANG, smem + L::WANG_OFF, row, t, px, k0, v);
+        } else {
+          ss = tc_read16_planes<GATE, FORM == TC_RMS>(raw, row, k0, v);
         }
-      } else {
-        const float* rp = reinterpret_cast<const float*>(raw) + k0 * TC_BM + row;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = rp[j * TC_BM];
-        if (GATE) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] *= rp[(TC_K + j) * TC_BM];
+        if (i == 16 / CONV - 1) {
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&raw_empty[rs]);
         }
-      }
-      if (!A_PLANAR && one_w) {
-        const float4* an = reinterpret_cast<const float4*>(smem + L::ANG_OFF + rs * TC_ANG) + (row >> wshift) * 16 + (k0 >> 2);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (rot[c]) th[c] = an[c];
-      }
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&raw_empty[rs]);
-      const int s = (it % NT) * 2 + hf;
-      if (!wait(&empty[s], ((it / NT) & 1) ^ 1, 1)) break;
-      tc::fence_after_sync();
-#pragma unroll
-      for (int p = 0; p < 2; ++p) {                          // eight channels at a time: registers
-        float* x = v + 8 * p;
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-          if (rot[2 * p + c]) {
-            auto turn = [](float tx, float ty, float wx, float wy, float& x, float& y) {
-              const float c2 = tx * wx - ty * wy, s2 = tx * wy + ty * wx;
-              const float ne = x * c2 - y * s2, no = x * s2 + y * c2;
-              x = ne; y = no;
-            };
-            const float4 a = th[2 * p + c], w = wang[2 * p + c];
-            turn(a.x, a.y, w.x, w.y, x[4 * c], x[4 * c + 1]);
-            turn(a.z, a.w, w.z, w.w, x[4 * c + 2], x[4 * c + 3]);
-          }
-        uint32_t hi[8], lo[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          float h, l;
-          tc::split_tf32(x[j], h, l);
-          hi[j] = __float_as_uint(h); lo[j] = __float_as_uint(l);
+        if (i == 0) {
+          if (!(ok = wait(&empty[s], ((it / NT) & 1) ^ 1, 1))) break;
+          tc::fence_after_sync();
+          // (the epilogue of the tile four back is through: the MMAs of the one two back, which this stage waited for, began after it)
+          if (FORM == TC_RMS) reinterpret_cast<float*>(smem + L::SS_OFF)[((it & 3) * 4 + grp) * 128 + row] = ss;
         }
-        tc::st_32x32b_x8(tdst + (uint32_t)(it % NT) * 128u + p * 8u, hi);
-        tc::st_32x32b_x8(tdst + (uint32_t)(it % NT) * 128u + 32u + p * 8u, lo);
+        tc_split_store16(tdst + (uint32_t)(it % NT) * 128u + sl * 16u, v);
       }
+      if (!ok) break;
       tc::wait_st();
       tc::fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&full[s]);
     }
-  } else if (warp == TC_LOAD_WARP) {
+  } else if (warp == LOAD_WARP) {
     // ================================ loader ================================
-    const int nrow = one_w ? TC_BM / g.W : 0;
     int it = 0;
     for (int tile = t_first; tile < t_end; tile += t_step, ++it) {
       const int rs = it % NRAW;
-      const int m0 = tile * TC_BM, fo = dv.hw.div(m0), px0 = m0 - fo * g.HW;
-      const int fr = (g.a_fmul == 0 && g.a_fadd == 0) ? fo : dv.fdiv.div(fo) * g.a_fmul + g.a_fadd;
+      const int m0 = tile * TC_BM, fo = dv.hw.div(m0), px0 = m0 - fo * g.HW, fr = tc_src_frame(g, dv, fo);
       if (!wait(&raw_empty[rs], ((it / NRAW) & 1) ^ 1, 5)) break;
       if (tc::elect_one()) {
         unsigned char* raw = smem + L::RAW_OFF + rs * L::RAW_BYTES;
@@ -240,19 +202,13 @@ gemm_tc_kernel(const GemmArgs g, const TcGeom dv, int num_tiles, const __grid_co
         }
       }
       __syncwarp();
-      if (!A_PLANAR && one_w) {
-        const int t = g.rope_tlast ? g.T - 1 : fo - dv.t.div(fo) * g.T, h0 = px0 >> (31 - __clz(g.W));
-        const float2 a = __ldg(g.rope_t + t * 32 + lane);
-        float2* an = reinterpret_cast<float2*>(smem + L::ANG_OFF + rs * TC_ANG) + lane;
-        for (int r = 0; r < nrow; ++r) {
-          const float2 b = __ldg(g.rope_h + (h0 + r) * 32 + lane);
-          an[r * 32] = make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-        }
+      if (rope_s) {
+        tc_rope_rows(g, smem + L::ANG_OFF + rs * TC_ANG, tc_rope_t(g, dv, fo), px0, lane);
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&raw_full[rs]);
       }
     }
-  } else if (warp == TC_MMA_WARP) {
+  } else if (warp == MMA_WARP) {
     // ================================ MMA issuer ================================
     // The whole warp walks the loop, one lane issues (elect_one).
     const uint32_t idesc = tc::make_idesc_tf32(TC_BM, N);
@@ -263,25 +219,22 @@ gemm_tc_kernel(const GemmArgs g, const TcGeom dv, int num_tiles, const __grid_co
       const int ac = it & 1, ph = (it >> 1) & 1;              // accumulator and its phase
       if (!(ok = wait(&accempty[ac], ph ^ 1, 2))) break;
       const uint32_t d = tmem_base + (uint32_t)ac * N;
+      const int s = (it % NT) * 2;
+      const uint32_t a = tmem_a + (uint32_t)s * 64u;
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
-        const int s = (it % NT) * 2 + hf;
-        if (!(ok = wait(&full[s], (it / NT) & 1, 2))) break;
+        if (!(ok = wait(&full[s + hf], (it / NT) & 1, 2))) break;
         tc::fence_after_sync();
-        const uint32_t a = tmem_a + (uint32_t)s * 64u;
-        if (tc::elect_one()) {
-#pragma unroll
-          for (int pass = 0; pass < 3; ++pass) {
-            const uint32_t ab = pass == 1 ? a + 32u : a;
-            const uint64_t bb = (pass == 2 ? b_lo : b_hi) + (uint64_t)(hf * (N * 128u >> 4));
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) tc::mma_tf32_ts(d, ab + ks * 8u, bb + ks * 2, idesc, (hf | pass | ks) ? 1u : 0u);
-          }
-          tc::commit(&empty[s]);
-        }
+        if (tc::elect_one()) tc_mma_small<N>(d, a + hf * 64u, b_hi, b_lo, hf, idesc);
         __syncwarp();
       }
-      if (ok && tc::elect_one()) tc::commit(&accfull[ac]);
+      if (ok && tc::elect_one()) {
+        tc_mma_lead<N>(d, a, b_hi, 0, idesc);
+        tc::commit(&empty[s]);
+        tc_mma_lead<N>(d, a + 64u, b_hi, 1, idesc);
+        tc::commit(&empty[s + 1]);
+        tc::commit(&accfull[ac]);
+      }
       __syncwarp();
     }
     // nothing of this warp's tensor work may be in flight when TMEM is freed
@@ -292,7 +245,10 @@ gemm_tc_kernel(const GemmArgs g, const TcGeom dv, int num_tiles, const __grid_co
   } else {
     // ================================ epilogue ================================
     const int q = warp & 3;                 // TMEM lane quadrant this warp may read
-    const int half = (warp - TC_EPI_WARP) >> 2;   // which half of the N columns
+    // (Two groups of warps with an accumulator and every other tile each, as in gemm_qkv_tconv_kernel, were no faster here: DeltaNet 32x32
+    // 415 -> 427 us a pass, the gate projection of 64x64 GDN 347 -> 397.)
+    const int half = (warp - EPI_WARP) >> 2;      // which half (of eight warps) or quarter (of sixteen) of the N columns
+    constexpr int CH = EPI == 16 ? 16 : 32, COLS = N / (EPI / 4);
     const int row = q * 32 + lane;
     int it = 0;
     for (int tile = t_first; tile < t_end; tile += t_step, ++it) {
@@ -315,39 +271,33 @@ gemm_tc_kernel(const GemmArgs g, const TcGeom dv, int num_tiles, const __grid_co
       tc::fence_after_sync();
       const int m = tile * TC_BM + row, fr = dv.hw.div(tile * TC_BM), px = m - fr * g.HW;
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)s * N;
+      float rinv = 1.f;
+      if (FORM == TC_RMS) {
+        const float* sp = reinterpret_cast<const float*>(smem + L::SS_OFF) + (it & 3) * 512 + row;
+        rinv = rsqrtf(((sp[0] + sp[128]) + (sp[256] + sp[384])) * (1.0f / TC_K) + 1e-6f);
+      }
 #pragma unroll 1
-      for (int cc = half * (N / 64); cc < (half + 1) * (N / 64); ++cc) {
-        if (FORM == TC_ZLAST && cc * 32 >= g.act_n0 && fr - dv.t.div(fr) * g.T != g.T - 1) continue;   // tile-uniform
-        uint32_t r[32];
-        tc::ld_32x32b_x32(taddr + cc * 32, r);
+      for (int c0 = half * COLS; c0 < (half + 1) * COLS; c0 += CH) {
+        if (FORM == TC_ZLAST && c0 >= g.act_n0 && fr - dv.t.div(fr) * g.T != g.T - 1) continue;   // tile-uniform
+        uint32_t r[CH];
+        if constexpr (CH == 32) tc::ld_32x32b_x32(taddr + c0, r);
+        else tc::ld_32x32b_x16(taddr + c0, r);
         tc::wait_ld();
         if (STG) {
           // this half's 128 threads share two 16 KB staging chunks and named barrier 1 + half
-          const int grp_tid = tid - (TC_EPI_WARP + 4 * half) * 32;      // 0..127
+          const int grp_tid = tid - (EPI_WARP + 4 * half) * 32;      // 0..127
           float* stg = reinterpret_cast<float*>(smem + L::OUT_OFF) + half * 4096;
           // the TMA store that last read this chunk buffer must have drained it
           if (grp_tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
-          const float* bs = bias_s + cc * 32;
-          const int act = (g.out_act != 0 && cc * 32 >= g.act_n0) ? g.out_act : 0;
-          if (!A_PLANAR) {
-            // chunk layout [column j][pixel]: lanes write consecutive pixels (conflict-free)
-            float vals[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              float v = __uint_as_float(r[j]) + bs[j];
-              if (act == 1) v = silu_f(v); else if (act == 2) v = sigmoid_f(v);
-              vals[j] = v;
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) stg[j * 128 + row] = vals[j];
-          } else {
+          const float* bs = bias_s + c0;
+          {
             // chunk layout [pixel][32 columns] in the 128-byte swizzle the tensor map expects
             float vals[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) vals[j] = __uint_as_float(r[j]) + bs[j];
+            for (int j = 0; j < 32; ++j) vals[j] = FORM == TC_RMS ? fmaf(__uint_as_float(r[j]), rinv, bs[j]) : __uint_as_float(r[j]) + bs[j];
             if (FORM == TC_SUB && g.sub != nullptr) {
-              const float4* sp = reinterpret_cast<const float4*>(g.sub + (size_t)m * g.N + cc * 32);
+              const float4* sp = reinterpret_cast<const float4*>(g.sub + (size_t)m * g.N + c0);
 #pragma unroll
               for (int j = 0; j < 32; j += 4) {
                 const float4 sv = __ldg(sp + (j >> 2));
@@ -359,64 +309,52 @@ gemm_tc_kernel(const GemmArgs g, const TcGeom dv, int num_tiles, const __grid_co
               *reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(stg) +
                                          tc::sw128_offset(row, j >> 2)) =
                   make_float4(vals[j], vals[j + 1], vals[j + 2], vals[j + 3]);
+            if (FORM == TC_RMS) {
+              // not finite, though the normalised row may be: again by FMAs
+              float odd = 0.f;
+#pragma unroll
+              for (int j = 0; j < 32; ++j) odd = fmaf(vals[j], 0.f, odd);
+              if (odd != 0.f)
+                for (int j = 0; j < 32; ++j)
+                  *reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(stg) + tc::sw128_offset(row, j >> 2) + (j & 3) * 4) =
+                      tc_planar_fma(g, dv, m, c0 + j, rinv);
+            }
           }
           tc::fence_proxy_async();
           asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
           if (grp_tid == 0) {
-            const int m0 = tile * TC_BM;
-            if (!A_PLANAR) {
-              tc::tma_store_3d(&omap, stg, px - row, g.o_plane0 + cc * 32, fr);
-            } else {
-              tc::tma_store_2d(&omap, stg, cc * 32, m0);
-            }
+            tc::tma_store_2d(&omap, stg, c0, tile * TC_BM);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
           continue;
         }
-        if (m < g.M) {
-          if (!A_PLANAR) {
-            // planar output: lanes = consecutive pixels -> 128-byte coalesced stores per column.
-            // All 32 values are finished in registers before the first store: the stores go
-            // through a generic pointer, so bias loads placed between them could not be hoisted.
-            float* op = g.out + ((size_t)fr * g.o_planes + g.o_plane0 + cc * 32) * g.HW + px;
-            const float* bs = bias_s + cc * 32;
-            float vals[32];
+        // planar output: lanes = consecutive pixels -> 128-byte coalesced stores per column.
+        // All values are finished in registers before the first store: the stores go
+        // through a generic pointer, so bias loads placed between them could not be hoisted.
+        float* op = g.out + ((size_t)fr * g.o_planes + g.o_plane0 + c0) * g.HW + px;
+        float vals[CH];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) vals[j] = __uint_as_float(r[j]) + bs[j];
-            if (g.out_act == 1 && cc * 32 >= g.act_n0) {
+        for (int j = 0; j < CH; ++j) vals[j] = __uint_as_float(r[j]) + bias_s[c0 + j];
+        if (g.out_act == 1 && c0 >= g.act_n0) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) vals[j] = silu_f(vals[j]);
-            } else if (g.out_act == 2 && cc * 32 >= g.act_n0) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) vals[j] = sigmoid_f(vals[j]);
-            }
-            if (FORM == TC_MUL && cc * 32 < g.mul_n) {
-              op = g.mul + ((size_t)fr * g.mul_planes + g.mul_plane0 + cc * 32) * g.HW + px;
-              float old[32];
-#pragma unroll
-              for (int j = 0; j < 32; ++j) old[j] = op[(size_t)j * g.HW];
-#pragma unroll
-              for (int j = 0; j < 32; ++j) vals[j] *= old[j];
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) op[(size_t)j * g.HW] = vals[j];
-          } else {
-            float* op = g.out + (size_t)m * g.N + cc * 32;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              float4 v;
-              v.x = __uint_as_float(r[j + 0]) + bias_s[cc * 32 + j + 0];
-              v.y = __uint_as_float(r[j + 1]) + bias_s[cc * 32 + j + 1];
-              v.z = __uint_as_float(r[j + 2]) + bias_s[cc * 32 + j + 2];
-              v.w = __uint_as_float(r[j + 3]) + bias_s[cc * 32 + j + 3];
-              if (FORM == TC_SUB && g.sub != nullptr) {
-                const float4 sv = __ldg(reinterpret_cast<const float4*>(g.sub + (size_t)m * g.N + cc * 32 + j));
-                v.x -= sv.x; v.y -= sv.y; v.z -= sv.z; v.w -= sv.w;
-              }
-              *reinterpret_cast<float4*>(op + j) = v;
-            }
+          for (int j = 0; j < CH; j += 2) {
+            const unsigned long long x = pk2(vals[j], vals[j + 1]);
+            upk2(mul2(x, sigmoid_x2(x)), vals[j], vals[j + 1]);
           }
+        } else if (g.out_act == 2 && c0 >= g.act_n0) {
+#pragma unroll
+          for (int j = 0; j < CH; j += 2) upk2(sigmoid_x2(pk2(vals[j], vals[j + 1])), vals[j], vals[j + 1]);
         }
+        if (FORM == TC_MUL && c0 < g.mul_n) {
+          op = g.mul + ((size_t)fr * g.mul_planes + g.mul_plane0 + c0) * g.HW + px;
+          float old[CH];
+#pragma unroll
+          for (int j = 0; j < CH; ++j) old[j] = op[(size_t)j * g.HW];
+#pragma unroll
+          for (int j = 0; j < CH; ++j) vals[j] *= old[j];
+        }
+#pragma unroll
+        for (int j = 0; j < CH; ++j) op[(size_t)j * g.HW] = vals[j];
       }
       tc::fence_before_sync();
       __syncwarp();
@@ -430,7 +368,7 @@ gemm_tc_kernel(const GemmArgs g, const TcGeom dv, int num_tiles, const __grid_co
   // error path only: give copies that may still be in flight a bounded time (~1 ms) to land
   if (s_bad)
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
-  if (warp == TC_MMA_WARP) {
+  if (warp == MMA_WARP) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem_base, 512);
   }
@@ -440,48 +378,34 @@ bool gemm_tc_in_place(int K, int N, int HW, int mul_n) {
   return K == TC_K && (N == 128 || N == 192) && HW % TC_BM == 0 && mul_n % 32 == 0;
 }
 
-// Whether this kernel takes the problem (else gemm_split_kernel, csrc/gemm_split.cu): 64 channels, tiles
-// inside one frame, no RMS prologue.  Splitting into two tf32 parts costs the producers half of what
-// three bf16 parts do, and at K = 64 the producers set the pace: in_proj of 4.2 M rows 649 against
-// 788 us.  With the RMS prologue (row sums over K) the other kernel is ahead, 683 against 847 us.
+// Whether this kernel takes the problem (else gemm_split_kernel, csrc/gemm_split.cu): 64 channels, tiles inside one frame, 16-byte
+// aligned tensors; the RMS prologue for 64 columns.
 bool gemm_tc_supported(const GemmArgs& g, bool a_planar) {
-  if (g.rms_scale != nullptr) return false;
+  if (g.rms_scale != nullptr && !(a_planar && g.N == 64 && g.sub == nullptr)) return false;
   if (g.K != TC_K || (g.N != 64 && g.N != 128 && g.N != 192)) return false;
   if (g.HW % TC_BM != 0 || g.M % TC_BM != 0) return false;
   if (g.out_act != 0 && g.act_n0 % 32 != 0) return false;
   if (g.mul != nullptr && !gemm_tc_in_place(g.K, g.N, g.HW, g.mul_n)) return false;
   if (a_planar && (g.N == 192 || (g.sub != nullptr && g.N != 64))) return false;
+  if (!aligned16(g.A) || (a_planar && (!aligned16(g.out) || (g.gate != nullptr && !aligned16(g.gate))))) return false;      // TMA
   return true;
 }
 
-// Tensor map of the GEMM output for the TMA-store epilogue: 16 KB boxes of 128 pixels x 32 columns.
-static bool make_out_map(const GemmArgs& g, bool a_planar, CUtensorMap* map) {
+// Tensor map of the channels-last output for the TMA stores: 16 KB boxes of 128 pixels x 32 columns.
+static bool make_out_map(const GemmArgs& g, CUtensorMap* map) {
   const tc::EncodeTiledFn enc = tc::encode_fn();
   if (!enc) return false;
-  const cuuint32_t es[3] = {1, 1, 1};
-  CUresult r;
-  if (!a_planar) {
-    const cuuint64_t dims[3] = {(cuuint64_t)g.HW, (cuuint64_t)g.o_planes, (cuuint64_t)(g.M / g.HW)};
-    const cuuint64_t strides[2] = {(cuuint64_t)g.HW * 4, (cuuint64_t)g.o_planes * g.HW * 4};
-    const cuuint32_t box[3] = {128, 32, 1};
-    r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, g.out, dims, strides, box, es,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-            CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  } else {
-    const cuuint64_t dims[2] = {(cuuint64_t)g.N, (cuuint64_t)g.M};
-    const cuuint64_t strides[1] = {(cuuint64_t)g.N * 4};
-    const cuuint32_t box[2] = {32, 128};
-    r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, g.out, dims, strides, box, es,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-            CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  }
-  return r == CUDA_SUCCESS;
+  const cuuint32_t es[2] = {1, 1};
+  const cuuint64_t dims[2] = {(cuuint64_t)g.N, (cuuint64_t)g.M};
+  const cuuint64_t strides[1] = {(cuuint64_t)g.N * 4};
+  const cuuint32_t box[2] = {32, 128};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, g.out, dims, strides, box, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+             CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Tensor maps of A (and of the gate planes): boxes of 128 rows x 32 channels, 128-byte swizzle, or of 128 pixels x 64 planes.
-// The rows of a channels-last A are those of its source frames, which may be fewer or more than the output's: the map covers
-// all that the tiles name.
-static bool make_in_map(const GemmArgs& g, bool a_planar, bool gate, CUtensorMap* map) {
+// (the rows of a channels-last A are those of its source frames, which may be fewer or more than the output's)
+bool tc_input_map(const GemmArgs& g, bool a_planar, bool gate, CUtensorMap* map) {
   const tc::EncodeTiledFn enc = tc::encode_fn();
   if (!enc) return false;
   const int fo = g.M / g.HW;                                       // output frames; their last source frame
@@ -514,17 +438,17 @@ static int launch_tc_v(const GemmArgs& g, const CUtensorMap& omap, cudaStream_t 
   const int sms = sm_count();
   cudaError_t e;
   const int grid = num_tiles < sms ? num_tiles : sms;
-  const size_t smem = TcSmem<N, GATE, STG>::TOTAL + 1024;      // slack for the 1024-byte alignment
+  const size_t smem = TcSmem<N, GATE, STG, FORM == TC_RMS>::TOTAL + 1024;      // slack for the 1024-byte alignment
   e = func_smem(gemm_tc_kernel<N, A_PLANAR, GATE, STG, FORM>, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   CUtensorMap amap, gmap;
   memset(&gmap, 0, sizeof(gmap));
-  if (!make_in_map(g, A_PLANAR, false, &amap) || (GATE && !make_in_map(g, true, true, &gmap))) return CSSM_ERR_CUDA;
+  if (!tc_input_map(g, A_PLANAR, false, &amap) || (GATE && !tc_input_map(g, true, true, &gmap))) return CSSM_ERR_CUDA;
   // Planes of 64x64: the 64 planes of a tile lie 1 MB apart in all, which neighbouring SMs share (NoGate's output
   // projection of 48 x 4 frames: 104 us in grid order, 139 with the CTAs where SMs came free); 8 x 4 frames and less, and
   // smaller planes, gain more by the early start.  Channels-last input: the second projection of the same rows.
   const PdlOff alone(N == 64 && num_tiles > 8 * sms && (!A_PLANAR || g.HW >= 4096));
-  const TcGeom dv = {FastDiv(g.HW), FastDiv(g.T > 0 ? g.T : 1), FastDiv(g.a_fdiv > 1 ? g.a_fdiv : 1)};
+  const TcGeom dv(g);
   launch_k(gemm_tc_kernel<N, A_PLANAR, GATE, STG, FORM>, grid, TC_THREADS, smem, st, g, dv, num_tiles, amap, gmap, omap);
   return check_launch();
 }
@@ -537,7 +461,7 @@ static int launch_tc(const GemmArgs& g, cudaStream_t st) {
     // (planar output: TMA stores measured slower than direct ones, 2.1 against 1.44 ms on an in_proj of 4.2 M rows)
     return launch_tc_v<N, false, false, false, FORM>(g, map, st);
   } else {
-    if (!make_out_map(g, true, &map)) return CSSM_ERR_CUDA;
+    if (!make_out_map(g, &map)) return CSSM_ERR_CUDA;
     return g.gate != nullptr ? launch_tc_v<N, true, true, true, FORM>(g, map, st) : launch_tc_v<N, true, false, true, FORM>(g, map, st);
   }
 }
@@ -545,7 +469,8 @@ static int launch_tc(const GemmArgs& g, cudaStream_t st) {
 int launch_gemm_tc(const GemmArgs& g, bool a_planar, cudaStream_t st) {
   if (!gemm_tc_supported(g, a_planar)) return CSSM_ERR_UNSUPPORTED;
   if (a_planar)
-    return g.N == 128 ? launch_tc<128, true>(g, st) : g.sub != nullptr ? launch_tc<64, true, TC_SUB>(g, st) : launch_tc<64, true>(g, st);
+    return g.N == 128 ? launch_tc<128, true>(g, st) : g.sub != nullptr ? launch_tc<64, true, TC_SUB>(g, st)
+                          : g.rms_scale != nullptr ? launch_tc<64, true, TC_RMS>(g, st) : launch_tc<64, true>(g, st);
   if (g.z_last_only && g.N == 128) return launch_tc<128, false, TC_ZLAST>(g, st);
   if (g.mul != nullptr) return g.N == 192 ? launch_tc<192, false, TC_MUL>(g, st) : launch_tc<128, false, TC_MUL>(g, st);
   return g.N == 192 ? launch_tc<192, false>(g, st) : g.N == 128 ? launch_tc<128, false>(g, st) : launch_tc<64, false>(g, st);
