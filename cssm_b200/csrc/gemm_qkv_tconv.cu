@@ -3,33 +3,43 @@
 //
 //   out[b, t, n, px] = silu(b_t[n] + sum_j w_j[n] s[b, t - 3 + j, n, px]) * gate,   s = A W + bias (frames before 0: nothing)
 //
-// The tcgen05 GEMM of csrc/gemm_tc.cu (3 x TF32, producers / MMA warp / epilogue) with another order of the tiles: a CTA takes 128
-// pixels and half of the 192 columns through t = 0 .. T - 1.  Its accumulators, 96 columns each, are a ring of five in
-// TMEM: the epilogue of step t reads those of t - 3 .. t, while the MMAs of t + 1 fill the fifth.  So the projected planes
-// never go to memory and back for the conv (6.4 GB of 128 x 8 x 64 x 64 x 64).  The price is that each tile of A is split
-// twice, once for either half of the columns (all 192 would need 768 columns of TMEM for the history).
+// The tcgen05 GEMM of csrc/gemm_tc.cu (3 x TF32, raw tiles by TMA, A in TMEM) with another order of the tiles: a CTA takes 128
+// pixels and one of q, k and v (64 columns) through t = 0 .. T - 1.  Its accumulators, 64 columns each, are a ring of five in
+// TMEM: the epilogue of step t reads those of t - 3 .. t, while the MMAs of t + 1 fill the fifth; the other 128 columns are the A operand.
+// So the projected planes never go to memory and back for the conv (6.4 GB of 128 x 8 x 64 x 64 x 64).  The price is that each tile
+// of A is split three times, once for each of q, k and v (all 192 columns would need 768 of TMEM for the history); the CTAs of the three
+// run side by side, so HBM sees it once.
+// Bound: the epilogue's issue slots and special functions.  With halves of 96 columns, A in shared memory and eight epilogue warps the epilogue's reads
+// of the taps waited for the MMAs' reads of A, and two warps a scheduler could not hide the special functions behind them.
 #include "kernels.cuh"
-#include "gemm.cuh"
-#include "tc05.cuh"
+#include "gemm_tc.cuh"
+#include "bf16_ops.cuh"
 
 namespace cssm {
 
 __device__ int g_qt_error = 0;
 
-constexpr int QT_THREADS = 544, QT_MMA_WARP = 8, QT_N = 96, QT_RING = 5, QT_BM = 128;
-constexpr uint32_t QT_A_HALF = 2u * QT_BM * 128u, QT_B_HALF = 2u * QT_N * 128u;
-constexpr uint32_t QT_A_OFF = 2u * QT_B_HALF, QT_TAB_OFF = QT_A_OFF + 4u * QT_A_HALF;      // two stages of hi, lo
-constexpr uint32_t QT_BAR_OFF = QT_TAB_OFF + 8u * QT_N * 4u, QT_SMEM = QT_BAR_OFF + 128u;   // tables: w[4][96], constants[4][96]
+constexpr int QT_CONV = 8, QT_EPI = 16;                           // converter and epilogue warps
+constexpr int QT_MMA_WARP = QT_CONV, QT_LOAD_WARP = QT_CONV + 1, QT_EPI_WARP = QT_CONV + 2, QT_THREADS = (QT_CONV + 2 + QT_EPI) * 32;
+constexpr int QT_N = 64, QT_RING = 5, QT_NRAW = 3;
+constexpr uint32_t QT_B_HALF = 2u * QT_N * 128u;
+constexpr uint32_t QT_RAW_OFF = 2u * QT_B_HALF, QT_TAB_OFF = QT_RAW_OFF + QT_NRAW * TC_RAW;
+constexpr uint32_t QT_ANG_OFF = QT_TAB_OFF + 8u * QT_N * 4u, QT_WANG_OFF = QT_ANG_OFF + QT_NRAW * TC_ANG;      // tables: w[4][64], constants[4][64]
+constexpr uint32_t QT_BAR_OFF = QT_WANG_OFF + TC_WANG, QT_SMEM = QT_BAR_OFF + 256u;
 static_assert(QT_SMEM + 1024 <= 227 * 1024, "one CTA per SM");
 
 struct QkvTconvGemmArgs {
   GemmArgs g;                                   // M, HW, A, source frames, RoPE, Wk (64, 192), bias, out (3C planes a frame), T
   const float* wt[3]; const float* bt[3]; int kt;
   const float2* bkv;                            // (frames, HW) {B_k, B_v} or nullptr
-  int seqs;                                     // 2 * clips * HW / 128
+  int seqs;                                     // 3 * clips * HW / 128
+  FastDiv blocks;                               // by the pixel blocks of a frame
 };
 
-__global__ void __launch_bounds__(QT_THREADS, 1) gemm_qkv_tconv_kernel(const __grid_constant__ QkvTconvGemmArgs a) {
+template <int V> struct QtInt { static constexpr int value = V; };
+
+__global__ void __launch_bounds__(QT_THREADS, 1) gemm_qkv_tconv_kernel(const __grid_constant__ QkvTconvGemmArgs a, const TcGeom dv,
+                                                                       const __grid_constant__ CUtensorMap amap) {
   const GemmArgs& g = a.g;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -37,44 +47,42 @@ __global__ void __launch_bounds__(QT_THREADS, 1) gemm_qkv_tconv_kernel(const __g
   float* wtab = reinterpret_cast<float*>(smem + QT_TAB_OFF);      // [tap][column], tap 3 = the current frame
   float* ctab = wtab + 4 * QT_N;                                  // [min(t, 3)][column]: b_t + bias * sum of the taps in use
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + QT_BAR_OFF);
-  uint64_t* full = bars;          // [2] A stage written (8 warps)
-  uint64_t* empty = bars + 2;     // [2] A stage consumed
-  uint64_t* accfull = bars + 4;   // [2] accumulator of step n, n & 1
-  uint64_t* accempty = bars + 6;  // [2] epilogue of step n is through (8 warps)
-  uint64_t* done = bars + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+  uint64_t* raw_full = bars;       // [3] raw tile landed
+  uint64_t* raw_empty = bars + 3;  // [3] and read (8 converter warps)
+  uint64_t* full = bars + 6;       // [2] A stage (half of the channels) written (4 warps)
+  uint64_t* empty = bars + 8;      // [2] A stage consumed
+  uint64_t* accfull = bars + 10;   // [2] accumulator of step n, n & 1
+  uint64_t* accempty = bars + 12;  // [2] epilogue of step n is through (8 warps)
+  uint64_t* done = bars + 14;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  __shared__ int s_bad;            // a bounded wait expired
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int half = blockIdx.x & 1, n0 = half * QT_N;              // the grid is even: a CTA keeps its half of the columns
+  const int part3 = blockIdx.x % 3;                               // q, k or v: the grid is a multiple of three, a CTA keeps its own
+  const bool rope_s = tc_rope_shared(g);
 
   if (tid == 0) {
+    for (int i = 0; i < QT_NRAW; ++i) { tc::mbar_init(&raw_full[i], rope_s ? 2 : 1); tc::mbar_init(&raw_empty[i], QT_CONV); }
     for (int i = 0; i < 2; ++i) {
-      tc::mbar_init(&full[i], 8); tc::mbar_init(&empty[i], 1);
-      tc::mbar_init(&accfull[i], 1); tc::mbar_init(&accempty[i], 8);
+      tc::mbar_init(&full[i], QT_CONV / 2); tc::mbar_init(&empty[i], 1);
+      tc::mbar_init(&accfull[i], 1); tc::mbar_init(&accempty[i], QT_EPI / 2);
     }
     tc::mbar_init(done, 1);
     tc::fence_mbar_init();
+    s_bad = 0;
   }
   if (warp == QT_MMA_WARP) {
     tc::tmem_alloc(tmem_slot, 512);
     tc::tmem_relinquish();
   }
-  for (int item = tid; item < QT_N * 16; item += QT_THREADS) {
-    const int n = item % QT_N, c = item / QT_N;                   // c: 16-byte chunk of 4 k values
-    float hi[4], lo[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) tc::split_tf32(g.Wk[(size_t)(4 * c + e) * 192 + n0 + n], hi[e], lo[e]);
-    const uint32_t off = (uint32_t)(c >> 3) * (QT_N * 128u) + tc::sw128_offset(n, c & 7);
-    *reinterpret_cast<float4*>(smem + off) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-    *reinterpret_cast<float4*>(smem + QT_B_HALF + off) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-  }
+  tc_split_weights<QT_N>(g.Wk, 192, part3 * QT_N, smem, smem + QT_B_HALF, tid, QT_THREADS);
+  if (rope_s) tc_rope_columns(g, smem + QT_WANG_OFF, tid, QT_THREADS);
   for (int n = tid; n < QT_N; n += QT_THREADS) {
-    const int grp = (n0 + n) >> 6, c = (n0 + n) & 63;
-    const float* wp = grp == 0 ? a.wt[0] : grp == 1 ? a.wt[1] : a.wt[2];
-    const float bt = (grp == 0 ? a.bt[0] : grp == 1 ? a.bt[1] : a.bt[2])[c], b = g.bias[n0 + n];
+    const float* wp = part3 == 0 ? a.wt[0] : part3 == 1 ? a.wt[1] : a.wt[2];
+    const float bt = (part3 == 0 ? a.bt[0] : part3 == 1 ? a.bt[1] : a.bt[2])[n], b = g.bias[part3 * QT_N + n];
     float sum = 0.f;
     for (int j = 3; j >= 0; --j) {                                // newest first; fewer taps than four: zeros before them
       const int i = j - (4 - a.kt);
-      const float w = i >= 0 ? wp[(size_t)i * 64 + c] : 0.f;
+      const float w = i >= 0 ? wp[(size_t)i * 64 + n] : 0.f;
       wtab[j * QT_N + n] = w;
       sum += w;
       ctab[(3 - j) * QT_N + n] = fmaf(b, sum, bt);
@@ -84,102 +92,111 @@ __global__ void __launch_bounds__(QT_THREADS, 1) gemm_qkv_tconv_kernel(const __g
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + QT_RING * QT_N;
   pdl_sync();
+  // all lanes of a warp agree; a wait that expires is recorded
+  auto wait = [&](uint64_t* bar, uint32_t phase, int code) {
+    const bool ok = !__any_sync(0xffffffffu, !tc::mbar_wait(bar, phase));
+    if (!ok) { if (lane == 0) atomicExch(&g_qt_error, code); s_bad = 1; }
+    return ok;
+  };
 
-  const int blocks = g.HW / QT_BM, T = g.T;                       // pixel blocks of a frame
-  // source frame of frame f, pixel block of sequence s
-  auto src_frame = [&](int f) { return g.a_fmul == 0 && g.a_fadd == 0 ? f : (g.a_fdiv > 1 ? f / g.a_fdiv : f) * g.a_fmul + g.a_fadd; };
+  const int T = g.T;
+  // sequence s: q, k or v s % 3 of pixel block s / 3 of the clips
+  auto clip_of = [&](int s, int& px0) {
+    const int pb = s / 3, b = a.blocks.div(pb);
+    px0 = (pb - b * (g.HW / TC_BM)) * TC_BM;
+    return b;
+  };
 
-  if (warp < 8) {
-    // ================================ producers ================================
-    // item r: chunk (tid & 7) + 8 (r >> 2) of row (tid >> 3) + 32 (r & 3), as in gemm_tc_kernel; `pre` holds the next step's tile
-    float4 pre[8];
-    const int chunk = tid & 7, rsub = tid >> 3;
-    const uint32_t dst0 = tc::sw128_offset(rsub, chunk);
-    bool rot[2] = {false, false};
-    if (g.rope_t != nullptr)
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        const int pi = 2 * (chunk + 8 * hf);
-        rot[hf] = g.rope_nz == nullptr || g.rope_nz[pi] != 0.f || g.rope_nz[pi + 1] != 0.f;
-      }
-    const float invW = 1.0f / (float)g.W;
-    auto fetch = [&](int s, int t) {
-      const int pb = s >> 1, b = pb / blocks, px0 = (pb - b * blocks) * QT_BM;
-      const float* a0 = g.A + ((size_t)src_frame(b * T + t) * g.HW + px0 + rsub) * 64 + chunk * 4;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) pre[r] = __ldg(reinterpret_cast<const float4*>(a0 + (size_t)(r & 3) * 32 * 64 + (r >> 2) * 32));
-    };
-    int it = 0;
+  if (warp < QT_CONV) {
+    // ================================ converters ================================
+    const int q = warp & 3, hf = warp >> 2, row = q * 32 + lane;             // lane quadrant, half of the channels
+    const uint32_t tdst = tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)(hf * 64);
+    const uint32_t rot[2] = {tc_rotated(g, hf * 32), tc_rotated(g, hf * 32 + 16)};
+    int n = 0, rs = 0;
+    uint32_t rph = 0;
     bool ok = true;
-    if ((int)blockIdx.x < a.seqs) fetch(blockIdx.x, 0);
     for (int s = blockIdx.x; s < a.seqs && ok; s += gridDim.x) {
-      const int pb = s >> 1, px0 = (pb - pb / blocks * blocks) * QT_BM;
-      for (int t = 0; t < T; ++t, ++it) {
-        const int st = it & 1;
-        float4 cur[8];
+      int px0;
+      clip_of(s, px0);
+      for (int t = 0; t < T; ++t, ++n) {
+        const unsigned char* raw = smem + QT_RAW_OFF + rs * TC_RAW;
+        if (!(ok = wait(&raw_full[rs], rph, 1))) break;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) cur[r] = pre[r];
-        if (t + 1 < T) fetch(s, t + 1);
-        else if (s + (int)gridDim.x < a.seqs) fetch(s + gridDim.x, 0);
-        if (__any_sync(0xffffffffu, !tc::mbar_wait(&empty[st], ((it >> 1) & 1) ^ 1))) { atomicExch(&g_qt_error, 1); ok = false; break; }
-        unsigned char* a_hi = smem + QT_A_OFF + (uint32_t)st * 2u * QT_A_HALF + dst0;
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          float4 v = cur[r];
-          if (rot[r >> 2]) {
-            const int px = px0 + rsub + 32 * (r & 3), pi = 2 * (chunk + 8 * (r >> 2));
-            const int h = (int)(((float)px + 0.5f) * invW), w = px - h * g.W;             // exact for px < 2^22
-            const float4 ct = __ldg(reinterpret_cast<const float4*>(g.rope_t + t * 32 + pi));
-            const float4 ch = __ldg(reinterpret_cast<const float4*>(g.rope_h + h * 32 + pi));
-            const float4 cw = __ldg(reinterpret_cast<const float4*>(g.rope_w + w * 32 + pi));
-            auto turn = [](float tx, float ty, float hx, float hy, float wx, float wy, float& x, float& y) {
-              const float cx = tx * hx - ty * hy, sx = tx * hy + ty * hx;
-              const float c2 = cx * wx - sx * wy, s2 = cx * wy + sx * wx;
-              const float ne = x * c2 - y * s2, no = x * s2 + y * c2;
-              x = ne; y = no;
-            };
-            turn(ct.x, ct.y, ch.x, ch.y, cw.x, cw.y, v.x, v.y);
-            turn(ct.z, ct.w, ch.z, ch.w, cw.z, cw.w, v.z, v.w);
+        for (int sl = 0; sl < 2; ++sl) {
+          const int k0 = hf * 32 + sl * 16;
+          float v[16];
+          tc_read16_rows(raw, row, k0, v);
+          tc_rotate16(g, rope_s, rot[sl], smem + QT_ANG_OFF + rs * TC_ANG, smem + QT_WANG_OFF, row, t, px0 + row, k0, v);
+          if (sl == 1) {
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&raw_empty[rs]);
+          } else {
+            if (!(ok = wait(&empty[hf], (n & 1) ^ 1, 1))) break;
+            tc::fence_after_sync();
           }
-          float4 h4, l4;
-          tc::split_tf32(v.x, h4.x, l4.x); tc::split_tf32(v.y, h4.y, l4.y);
-          tc::split_tf32(v.z, h4.z, l4.z); tc::split_tf32(v.w, h4.w, l4.w);
-          unsigned char* d = a_hi + (r & 3) * 4096 + (r >> 2) * (QT_BM * 128);            // 32 rows = 4096 bytes on
-          *reinterpret_cast<float4*>(d) = h4;
-          *reinterpret_cast<float4*>(d + QT_A_HALF) = l4;
+          tc_split_store16(tdst + sl * 16u, v);
         }
-        tc::fence_proxy_async();
+        if (!ok) break;
+        tc::wait_st();
+        tc::fence_before_sync();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&full[st]);
+        if (lane == 0) tc::mbar_arrive(&full[hf]);
+        if (++rs == QT_NRAW) { rs = 0; rph ^= 1; }
+      }
+    }
+  } else if (warp == QT_LOAD_WARP) {
+    // ================================ loader ================================
+    int rs = 0;
+    uint32_t rph = 0;
+    bool ok = true;
+    for (int s = blockIdx.x; s < a.seqs && ok; s += gridDim.x) {
+      int px0;
+      const int b = clip_of(s, px0);
+      for (int t = 0; t < T; ++t) {
+        const int r0 = tc_src_frame(g, dv, b * T + t) * g.HW + px0;
+        if (!(ok = wait(&raw_empty[rs], rph ^ 1, 5))) break;
+        if (tc::elect_one()) {
+          unsigned char* raw = smem + QT_RAW_OFF + rs * TC_RAW;
+          tc::mbar_expect_tx(&raw_full[rs], TC_RAW);
+          tc::tma_load_2d(raw, &amap, 0, r0, &raw_full[rs]);
+          tc::tma_load_2d(raw + TC_BM * 128, &amap, 32, r0, &raw_full[rs]);
+        }
+        __syncwarp();
+        if (rope_s) {
+          tc_rope_rows(g, smem + QT_ANG_OFF + rs * TC_ANG, t, px0, lane);
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&raw_full[rs]);
+        }
+        if (++rs == QT_NRAW) { rs = 0; rph ^= 1; }
       }
     }
   } else if (warp == QT_MMA_WARP) {
     // ================================ MMA issuer ================================
     // The whole warp walks the loop, one lane issues (elect_one).
-    const uint32_t idesc = tc::make_idesc_tf32(QT_BM, QT_N);
+    const uint32_t idesc = tc::make_idesc_tf32(TC_BM, QT_N);
+    const uint64_t b_hi = tc::make_desc_sw128(sbase), b_lo = tc::make_desc_sw128(sbase + QT_B_HALF);
     const int mine = a.seqs > (int)blockIdx.x ? (a.seqs - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * T : 0;
     bool ok = true;
     int slot = 0;
-    for (int n = 0; n < mine; ++n) {
+    for (int n = 0; n < mine && ok; ++n) {
       // the accumulator of step n - 5 was last read by the epilogue of step n - 2
-      if (__any_sync(0xffffffffu, !tc::mbar_wait(&accempty[n & 1], ((n >> 1) & 1) ^ 1) || !tc::mbar_wait(&full[n & 1], (n >> 1) & 1))) {
-        atomicExch(&g_qt_error, 2); ok = false; break;
-      }
-      tc::fence_after_sync();
-      const uint32_t a_hi = sbase + QT_A_OFF + (uint32_t)(n & 1) * 2u * QT_A_HALF, a_lo = a_hi + QT_A_HALF;
+      if (!(ok = wait(&accempty[n & 1], ((n >> 1) & 1) ^ 1, 2))) break;
       const uint32_t d = tmem_base + (uint32_t)slot * QT_N;
       if (++slot == QT_RING) slot = 0;
-      if (tc::elect_one()) {
 #pragma unroll
-        for (int pass = 0; pass < 3; ++pass) {
-          const uint64_t ad = tc::make_desc_sw128(pass == 1 ? a_lo : a_hi), bd = tc::make_desc_sw128(pass == 2 ? sbase + QT_B_HALF : sbase);
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks)
-            tc::mma_tf32(d, ad + (ks >> 2) * (QT_BM * 128u >> 4) + (ks & 3) * 2, bd + (ks >> 2) * (QT_N * 128u >> 4) + (ks & 3) * 2, idesc, (pass | ks) ? 1u : 0u);
-        }
-        tc::commit(&empty[n & 1]);
+      for (int hf = 0; hf < 2; ++hf) {
+        if (!(ok = wait(&full[hf], n & 1, 2))) break;
+        tc::fence_after_sync();
+        if (tc::elect_one()) tc_mma_small<QT_N>(d, tmem_a + hf * 64u, b_hi, b_lo, hf, idesc);
+        __syncwarp();
+      }
+      if (ok && tc::elect_one()) {
+        tc_mma_lead<QT_N>(d, tmem_a, b_hi, 0, idesc);
+        tc::commit(&empty[0]);
+        tc_mma_lead<QT_N>(d, tmem_a + 64u, b_hi, 1, idesc);
+        tc::commit(&empty[1]);
         tc::commit(&accfull[n & 1]);
       }
       __syncwarp();
@@ -191,87 +208,103 @@ __global__ void __launch_bounds__(QT_THREADS, 1) gemm_qkv_tconv_kernel(const __g
     __syncwarp();
   } else {
     // ================================ epilogue ================================
-    const int q = warp & 3, part = (warp - (QT_MMA_WARP + 1)) >> 2;          // TMEM lane quadrant; 48 of the 96 columns
-    const uint32_t tlane = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)part * 48u;
-    int n = 0, slot = 0;
+    // Two groups of eight warps take every other step, so that one loads while the other is at its special functions.  Half of the columns
+    // a warp, eight at a time: the frames under the four taps are requested together, one wait.
+    constexpr int PART = QT_N / 2;
+    const int q = warp & 3, grp = (warp - QT_EPI_WARP) >> 3, part = ((warp - QT_EPI_WARP) >> 2) & 1;      // q: TMEM lane quadrant
+    const uint32_t tlane = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * PART);
+    int n = grp, slot = grp, t = grp, s = blockIdx.x;
     bool ok = true;
-    for (int s = blockIdx.x; s < a.seqs && ok; s += gridDim.x) {
-      const int pb = s >> 1, b = pb / blocks, px = (pb - b * blocks) * QT_BM + q * 32 + lane;
-      for (int t = 0; t < T; ++t, ++n) {
+    while (ok) {
+      while (t >= T && s < a.seqs) { t -= T; s += gridDim.x; }
+      if (s >= a.seqs) break;
+      int px;
+      const int b = clip_of(s, px);
+      px += q * 32 + lane;
+      {
         const size_t frame = (size_t)b * T + t;
-        const float2 gv = a.bkv != nullptr ? __ldg(a.bkv + frame * g.HW + px) : make_float2(1.f, 1.f);
-        if (__any_sync(0xffffffffu, !tc::mbar_wait(&accfull[n & 1], (n >> 1) & 1))) { atomicExch(&g_qt_error, 4); ok = false; break; }
+        const float2 gv = a.bkv != nullptr && part3 != 0 ? __ldg(a.bkv + frame * g.HW + px) : make_float2(1.f, 1.f);
+        if (!(ok = wait(&accfull[n & 1], (n >> 1) & 1, 4))) break;
         tc::fence_after_sync();
         // earlier frames of this clip under the taps (frames further back may hold anything: no product with a zero tap)
         const int back = t < a.kt - 1 ? t : a.kt - 1;
         uint32_t sl[4];                                                     // ring slots of t, t - 1, t - 2, t - 3
 #pragma unroll
         for (int d = 0; d < 4; ++d) sl[d] = (uint32_t)(slot >= d ? slot - d : slot - d + QT_RING) * QT_N;
-        if (++slot == QT_RING) slot = 0;
-#pragma unroll 1
-        for (int pc = 0; pc < 3; ++pc) {
-          const int c0 = part * 48 + pc * 16;
-          float v[16];
+        const float gate = part3 == 0 ? 1.f : part3 == 1 ? gv.x : gv.y;
+        float* op = g.out + (frame * 192 + part3 * QT_N + part * PART) * g.HW + px;
+        // eight columns from pc on: taps of frames t - BACK .. t
+        auto chunk = [&](auto BACK, int pc) {
+          constexpr int NB = decltype(BACK)::value;
+          const int c0 = part * PART + pc;
+          uint32_t r[NB + 1][8];
 #pragma unroll
-          for (int j = 0; j < 16; j += 4) {
-            const float4 c = *reinterpret_cast<const float4*>(ctab + back * QT_N + c0 + j);
-            v[j] = c.x; v[j + 1] = c.y; v[j + 2] = c.z; v[j + 3] = c.w;
+          for (int d = 0; d <= NB; ++d) tc::ld_32x32b_x8(tlane + sl[d] + pc, r[d]);
+          typedef unsigned long long u64;
+          u64 v[4];
+#pragma unroll
+          for (int j = 0; j < 4; j += 2) {
+            const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(ctab + NB * QT_N + c0 + 2 * j);
+            v[j] = c.x; v[j + 1] = c.y;
           }
-          auto tap = [&](const uint32_t (&r)[16], int d) {
-#pragma unroll
-            for (int j = 0; j < 16; j += 4) {
-              const float4 w = *reinterpret_cast<const float4*>(wtab + (3 - d) * QT_N + c0 + j);
-              v[j] = fmaf(w.x, __uint_as_float(r[j]), v[j]);             v[j + 1] = fmaf(w.y, __uint_as_float(r[j + 1]), v[j + 1]);
-              v[j + 2] = fmaf(w.z, __uint_as_float(r[j + 2]), v[j + 2]); v[j + 3] = fmaf(w.w, __uint_as_float(r[j + 3]), v[j + 3]);
-            }
-          };
-          uint32_t r0[16], r1[16];
-          tc::ld_32x32b_x16(tlane + sl[0] + pc * 16, r0);
-          if (back >= 1) tc::ld_32x32b_x16(tlane + sl[1] + pc * 16, r1);
           tc::wait_ld();
-          tap(r0, 0);
-          if (back >= 1) tap(r1, 1);
-          if (back >= 2) {
-            tc::ld_32x32b_x16(tlane + sl[2] + pc * 16, r0);
-            if (back >= 3) tc::ld_32x32b_x16(tlane + sl[3] + pc * 16, r1);
-            tc::wait_ld();
-            tap(r0, 2);
-            if (back >= 3) tap(r1, 3);
-          }
-          const int col = n0 + c0;
-          const float gate = col < 64 ? 1.f : col < 128 ? gv.x : gv.y;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = silu_f(v[j]) * gate;
-          float* op = g.out + (frame * 192 + col) * g.HW + px;
+          for (int d = 0; d <= NB; ++d)
 #pragma unroll
-          for (int j = 0; j < 16; ++j) op[(size_t)j * g.HW] = v[j];
+            for (int j = 0; j < 4; j += 2) {
+              const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(wtab + (3 - d) * QT_N + c0 + 2 * j);
+              v[j] = fma2(w.x, pk2(__uint_as_float(r[d][2 * j]), __uint_as_float(r[d][2 * j + 1])), v[j]);
+              v[j + 1] = fma2(w.y, pk2(__uint_as_float(r[d][2 * j + 2]), __uint_as_float(r[d][2 * j + 3])), v[j + 1]);
+            }
+          const u64 g2 = pk2(gate, gate);
+          float o[8];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) upk2(mul2(mul2(v[j], sigmoid_x2(v[j])), g2), o[2 * j], o[2 * j + 1]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) op[(size_t)j * g.HW] = o[j];
+          op += (size_t)8 * g.HW;
+        };
+#pragma unroll 1
+        for (int pc = 0; pc < PART; pc += 8) {
+          if (back == 3) chunk(QtInt<3>(), pc);
+          else if (back == 0) chunk(QtInt<0>(), pc);
+          else if (back == 1) chunk(QtInt<1>(), pc);
+          else chunk(QtInt<2>(), pc);
         }
         tc::fence_before_sync();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&accempty[n & 1]);
       }
+      n += 2; t += 2;
+      slot += 2;
+      if (slot >= QT_RING) slot -= QT_RING;
     }
   }
   tc::fence_before_sync();
   __syncthreads();
+  // error path only: give copies that may still be in flight a bounded time (~1 ms) to land
+  if (s_bad)
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   if (warp == QT_MMA_WARP) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem_base, 512);
   }
 }
 
-static long long sequences(const GemmArgs& g) { return 2LL * (g.M / g.HW / g.T) * (g.HW / QT_BM); }
+static long long sequences(const GemmArgs& g) { return 3LL * (g.M / g.HW / g.T) * (g.HW / TC_BM); }
 
 // g: the projection as launch_gemm takes it; kt: taps of the conv on its output
 bool gemm_qkv_tconv_supported(const GemmArgs& g, int kt) {
-  if (g.K != 64 || g.N != 192 || g.HW % QT_BM != 0 || g.T <= 0 || g.M % g.HW != 0 || g.M / g.HW % g.T != 0 || kt < 1 || kt > 4 ||
-      g.bias == nullptr || g.o_planes != 192 || g.o_plane0 != 0)
+  if (g.K != 64 || g.N != 192 || g.HW % TC_BM != 0 || g.T <= 0 || g.M % g.HW != 0 || g.M / g.HW % g.T != 0 || kt < 1 || kt > 4 ||
+      g.bias == nullptr || g.o_planes != 192 || g.o_plane0 != 0 || !aligned16(g.A))
     return false;
-  // A sequence of T steps is the unit of work and cannot be split.  From two for every SM on the joined launch is ahead wherever the
-  // last round ends (three rounds for the work of 2.05 included).  GDN block, us a pass, two launches / this one: 32x32, T = 8, 19
-  // clips (304 sequences) 306 / 288, 20 310 / 294, 23 331 / 310, 27 380 / 331, 28 412 / 382, 38 533 / 478, 120 1463 / 1263; T = 1, 19
-  // clips 82.8 / 71.7; T = 32, 19 1046 / 1001; 64x64, T = 8, 5 clips (320) 460 / 439, 10 874 / 816; 16x16, T = 4, 80 clips (320) 260 / 248.
-  return sequences(g) >= 2 * sm_count() && sequences(g) < (1LL << 31) && sm_count() > 1;
+  // A sequence of T steps is the unit of work and cannot be split: with few of them most SMs are idle for T steps.  The joined launch is
+  // ahead from two sequences for three SMs on, and at up to four steps always (one launch less).  GDN block, us a pass, two launches / this
+  // one: 32x32, T = 8, 4 clips (96 sequences) 112 / 98, 19 271 / 249, 62 734 / 620; T = 32, 4 312 / 287, 19 972 / 867; T = 1, 19 79 / 68; 64x64,
+  // T = 8, 2 clips (192) 343 / 336, T = 32 1273 / 1250; 16x16, T = 32, 16 clips (96) 546 / 529; below: 16x16, T = 8, 4 clips 122 / 123, T =
+  // 32, 12 clips 501 / 512, T = 4, one clip 78.8 / 78.5; 32x32, T = 32, one clip 236 / 238.  With halves of 96 columns 32x32, T = 8, 19
+  // clips took 288, 62 694.
+  return (g.T <= 4 || 3 * sequences(g) >= 2 * (sm_count() / 3 * 3)) && sequences(g) < (1LL << 31) && sm_count() > 2;
 }
 
 int launch_gemm_qkv_tconv(const GemmArgs& g, const QkvTconvArgs& t, cudaStream_t st) {
@@ -280,11 +313,14 @@ int launch_gemm_qkv_tconv(const GemmArgs& g, const QkvTconvArgs& t, cudaStream_t
   a.g = g;
   for (int i = 0; i < 3; ++i) { a.wt[i] = t.wt[i]; a.bt[i] = t.bt[i]; }
   a.kt = t.kt; a.bkv = t.bkv;
-  const int sms = sm_count() & ~1;
   a.seqs = (int)sequences(g);
+  const int sms = sm_count() / 3 * 3, grid = a.seqs < sms ? a.seqs : sms;       // multiples of three
+  a.blocks = FastDiv(g.HW / TC_BM);
+  CUtensorMap amap;
+  if (!tc_input_map(g, false, false, &amap)) return CSSM_ERR_CUDA;
   const cudaError_t e = func_smem(gemm_qkv_tconv_kernel, QT_SMEM + 1024);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  launch_k(gemm_qkv_tconv_kernel, sms, QT_THREADS, QT_SMEM + 1024, st, a);
+  launch_k(gemm_qkv_tconv_kernel, grid, QT_THREADS, QT_SMEM + 1024, st, a, TcGeom(g), amap);
   return check_launch();
 }
 

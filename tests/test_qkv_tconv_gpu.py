@@ -1,5 +1,6 @@
-"""q, k, v projection and temporal conv in one launch (csrc/gemm_qkv_tconv.cu: 64 channels, planes of whole 128-pixel tiles, at least two
-sequences an SM) against the block on fewer clips, which goes through the two launches, and against the oracle."""
+"""q, k, v projection and temporal conv in one launch (csrc/gemm_qkv_tconv.cu: 64 channels, planes of whole 128-pixel tiles, two
+sequences for three SMs and more or up to four steps) against the block on fewer clips, which from five steps on goes through the two
+launches, and against the oracle."""
 import numpy as np
 import pytest
 import torch
