@@ -6,7 +6,7 @@
 // Persistent kernel, one CTA per SM, 18 warps (14 in the im2col form), warp-specialised:
 //   warp 0     TMA producer: one lane issues cp.async.bulk.tensor loads of the A tile (128 rows x
 //              64 k, plain mode) and the weight tile (BN rows x 64 k) of every K block into a
-//              4-stage ring of 128-byte-swizzled K-major operand tiles;
+//              ring of 128-byte-swizzled K-major operand tiles (as many stages as there is room for, at most eight);
 //   warp 1     MMA issuer: one lane issues 4 tcgen05.mma.kind::f16 (M128 x BN x K16) per K block
 //              into one of four TMEM accumulators (BN <= 128; two for wider single tiles);
 //              tcgen05.commit frees the stage / publishes the accumulator;
@@ -42,7 +42,8 @@ __device__ int g_bf16_error = 0;
 // Epilogue warps: sixteen; eight beside the gathering warps of the im2col form, which need the registers.
 template <bool IM2COL> constexpr int gb_epi_warps = IM2COL ? 8 : 16;
 template <bool IM2COL> constexpr int gb_threads = (2 + gb_epi_warps<IM2COL> + (IM2COL ? 4 : 0)) * 32;
-constexpr int GB_BM = 128, GB_BK = 64, GB_MAX_STAGES = 4;
+constexpr int GB_BM = 128, GB_BK = 64, GB_MAX_STAGES = 8;
+constexpr uint32_t GB_BAR_BYTES = 320;                   // barriers and the TMEM slot
 constexpr uint32_t GB_A_BYTES = GB_BM * 128u;            // one A stage: 128 rows x 128 bytes
 
 __device__ __forceinline__ uint32_t make_idesc_bf16(uint32_t M, uint32_t N) {
@@ -83,15 +84,15 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
   unsigned char* ring = smem + wres_bytes;
   unsigned char* out_s = ring + (uint32_t)NS * stage_bytes; // TMA_OUT: 2 x ostg staging boxes of 16 KB
   uint64_t* bars = reinterpret_cast<uint64_t*>(out_s + (TMA_OUT ? (uint32_t)(2 * g.ostg) * 16384u : 0u));
-  uint64_t* full = bars;                        // [4] operands landed
-  uint64_t* empty = bars + GB_MAX_STAGES;       // [4] stage consumed
+  uint64_t* full = bars;                        // [8] operands landed
+  uint64_t* empty = bars + GB_MAX_STAGES;       // [8] stage consumed
   uint64_t* accfull = bars + 2 * GB_MAX_STAGES; // [4] accumulator complete
   uint64_t* accempty = accfull + 4;             // [4] accumulator drained
   uint64_t* resfull = accempty + 4;             // [2][4] residual box landed in its staging slot
   uint64_t* done = resfull + 8;
   uint64_t* wfull = done + 1;                   // resident weights landed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wfull + 1);
-  float* bias_s = reinterpret_cast<float*>(bars + 32);      // the bias, where it fits (g.bias_n values)
+  float* bias_s = reinterpret_cast<float*>(bars + GB_BAR_BYTES / 8);      // the bias, where it fits (g.bias_n values)
   const int NACC = g.nacc;                                  // TMEM accumulators: 4 of BN <= 128 columns, else 2
 
   constexpr int EW = gb_epi_warps<IM2COL>, HALF_THREADS = EW * 16, CW = EW / 8;      // CW: warps of a half and lane quadrant
@@ -131,54 +132,61 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
 
   if (warp == 0) {
     // ================================ TMA producer ================================
-    if (lane == 0) {
-      // Weights do not depend on the kernel before this one: the resident ones, or the weight tiles of
-      // the first ring round, are on their way before the wait for it.
-      int npre = 0;
-      if (wres) {
+    // The whole warp walks the loop with counters in place of divisions, one lane issues (elect_one): a lane that divided its way to every box
+    // was itself what the 3x3 convs waited for (780 of 980 clocks a K block).
+    // Weights do not depend on the kernel before this one: the resident ones, or the weight tiles of
+    // the first ring round, are on their way before the wait for it.
+    const uint32_t a_bytes = g.conv_tma ? (uint32_t)(g.Wbox * g.Hbox * g.Bbox) * 128u : GB_A_BYTES;
+    int npre = 0;
+    if (wres) {
+      if (tc::elect_one()) {
         tc::mbar_expect_tx(wfull, wres_bytes);
         for (int kb = 0; kb < kblocks; ++kb) tc::tma_load_2d(smem + (uint32_t)kb * BN * 128u, &bmap, kb * GB_BK, 0, wfull);
-      } else if (!IM2COL && blockIdx.x < num_tiles) {
-        const int n0 = (blockIdx.x % n_tiles) * g.BN;
-        const uint32_t a_bytes = g.conv_tma ? (uint32_t)(g.Wbox * g.Hbox * g.Bbox) * 128u : GB_A_BYTES;
-        for (; npre < NS && npre < kblocks; ++npre) {
-          tc::mbar_expect_tx(&full[npre], a_bytes + BN * 128u);
-          tc::tma_load_2d(ring + (uint32_t)npre * stage_bytes + GB_A_BYTES, &bmap, npre * GB_BK, n0, &full[npre]);
-        }
       }
-      pdl_sync();
-      int it = 0;
-      for (int tile = blockIdx.x; tile < num_tiles && !bad; tile += gridDim.x) {
-        const int mt = tile / n_tiles;
-        const int m0 = mt * GB_BM, n0 = (tile % n_tiles) * g.BN;
-        // conv through TMA: the tile's patch origin (input coordinates of window position (0,0))
-        int cw0 = 0, ch0 = 0, cb0 = 0;
-        if (g.conv_tma) {
-          const int tw = mt % g.tiles_w, th = (mt / g.tiles_w) % g.tiles_h;
-          cb0 = (mt / (g.tiles_w * g.tiles_h)) * g.Bbox;
-          cw0 = tw * g.Wbox * (g.conv_tma == 2 ? 1 : g.stride) - (g.conv_tma == 2 ? 0 : g.pad_w);
-          ch0 = th * g.Hbox * g.stride - g.pad_h;
+      __syncwarp();
+    } else if (!IM2COL && blockIdx.x < num_tiles) {
+      const int n0 = (blockIdx.x % n_tiles) * g.BN;
+      npre = NS < kblocks ? NS : kblocks;
+      if (tc::elect_one())
+        for (int i = 0; i < npre; ++i) {
+          tc::mbar_expect_tx(&full[i], a_bytes + BN * 128u);
+          tc::tma_load_2d(ring + (uint32_t)i * stage_bytes + GB_A_BYTES, &bmap, i * GB_BK, n0, &full[i]);
         }
-        const uint32_t a_bytes = g.conv_tma ? (uint32_t)(g.Wbox * g.Hbox * g.Bbox) * 128u : GB_A_BYTES;
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % NS;
-          if (!tc::mbar_wait(&empty[s], ((it / NS) & 1) ^ 1)) { atomicExch(&g_bf16_error, 5); bad = true; break; }
-          unsigned char* a_s = ring + (uint32_t)s * stage_bytes;
-          unsigned char* b_s = a_s + GB_A_BYTES;
-          const bool pre = it < npre;                       // its weight tile is already on the way
+      __syncwarp();
+    }
+    pdl_sync();
+    int s = 0;
+    uint32_t sph = 0;
+    for (int tile = blockIdx.x; tile < num_tiles && !bad; tile += gridDim.x) {
+      const int mt = tile / n_tiles;
+      const int m0 = mt * GB_BM, n0 = (tile - mt * n_tiles) * g.BN;
+      // conv through TMA: the tile's patch origin (input coordinates of window position (0,0))
+      int cw0 = 0, ch0 = 0, cb0 = 0, pr = 0, pc = 0, cb = 0;
+      if (g.conv_tma) {
+        const int r = mt / g.tiles_w, tw = mt - r * g.tiles_w, b = r / g.tiles_h, th = r - b * g.tiles_h;
+        cb0 = b * g.Bbox;
+        cw0 = tw * g.Wbox * (g.conv_tma == 2 ? 1 : g.stride) - (g.conv_tma == 2 ? 0 : g.pad_w);
+        ch0 = th * g.Hbox * g.stride - g.pad_h;
+      }
+      for (int kb = 0; kb < kblocks; ++kb) {
+        if (__any_sync(0xffffffffu, !tc::mbar_wait(&empty[s], sph ^ 1))) { atomicExch(&g_bf16_error, 5); bad = true; break; }
+        unsigned char* a_s = ring + (uint32_t)s * stage_bytes;
+        const bool pre = npre > 0;                        // its weight tile is already on the way
+        if (tc::elect_one()) {
           if (!pre) tc::mbar_expect_tx(&full[s], (IM2COL ? 0u : a_bytes) + (wres ? 0u : BN * 128u));
-          if (g.conv_tma) {
-            const int pos = kb / g.kb_per_tap, cb = kb - pos * g.kb_per_tap;
-            const int pr = pos / g.pos_w, pc = pos - pr * g.pos_w;
-            tc::tma_load_4d(a_s, &amap, cb * GB_BK, cw0 + pc, ch0 + pr, cb0, &full[s]);
-          } else if (!IM2COL) {
-            tc::tma_load_2d(a_s, &amap, kb * GB_BK, m0, &full[s]);
-          }
-          if (!wres && !pre) tc::tma_load_2d(b_s, &bmap, kb * GB_BK, n0, &full[s]);
+          if (g.conv_tma) tc::tma_load_4d(a_s, &amap, cb * GB_BK, cw0 + pc, ch0 + pr, cb0, &full[s]);
+          else if (!IM2COL) tc::tma_load_2d(a_s, &amap, kb * GB_BK, m0, &full[s]);
+          if (!wres && !pre) tc::tma_load_2d(a_s + GB_A_BYTES, &bmap, kb * GB_BK, n0, &full[s]);
         }
+        __syncwarp();
+        if (pre) --npre;
+        if (g.conv_tma && ++cb == g.kb_per_tap) {
+          cb = 0;
+          if (++pc == g.pos_w) { pc = 0; ++pr; }
+        }
+        if (++s == NS) { s = 0; sph ^= 1; }
       }
     }
-    __syncwarp();
   } else if (warp == 1) {
     // ================================ MMA issuer ================================
     // The limit of the waits below is for this kernel's own loads: they begin once the producer's wait is over.
@@ -737,13 +745,13 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
   g.wres = (!im2col && g.N == g.BN && wres_bytes <= 64 * 1024) ? 1 : 0;
   const size_t stage = GB_A_BYTES + (g.wres ? 0 : (size_t)g.BN * 128u);
   g.bias_n = g.bias != nullptr && g.N <= 2048 ? g.N : 0;
-  const size_t budget = 227 * 1024 - (g.wres ? wres_bytes : 0), fixed = 256 + 1024 + (size_t)g.bias_n * 4;
+  const size_t budget = 227 * 1024 - (g.wres ? wres_bytes : 0), fixed = GB_BAR_BYTES + 1024 + (size_t)g.bias_n * 4;
   // Residual by TMA (plain GEMMs with tiles of at most 128 columns): four accumulators and three or
   // four staging slots per epilogue half.  Everything else: two accumulators, two slots, residual
   // rows (if any) by plain loads -- the configuration that measured best without a residual.
   const bool rtma = tma_out && g.res != nullptr && !conv && g.BN <= 128;
   g.nacc = rtma ? 4 : 2;
-  g.stages = GB_MAX_STAGES;
+  g.stages = rtma ? 4 : GB_MAX_STAGES;                     // (with residuals by TMA the room goes to the staging slots)
   g.ostg = 0;
   if (tma_out) {
     while (g.stages > 2 && g.stages * stage + 4 * 16384 + fixed > budget) --g.stages;      // (ROWS: sixteen slots of 4 KB)
