@@ -10,7 +10,7 @@
 //
 // Bound: the packed FMAs of the products, 4 planes' worth per head and key dimension (the direct DFTs that
 // ran here before did four to eight times the multiplications).  GDN 12 x 8 x 28 x 28 x 64, key dimension 2:
-// 667 -> 146 us.
+// 667 -> 146 us; 16 x 8 x 28 x 28 x 64 238 -> 212 with a pair of register tiles (dp_pick) instead of one for all passes.
 #include <math.h>
 #include <string.h>
 #include "kernels.cuh"
@@ -26,7 +26,7 @@ struct DeltaDftArgs {
 };
 
 // planes [k | v | q] of n planes each (q only when the step is read out) -> spectra in RA[k][col]
-template <int RT, int YT, int NT, class KGate>
+template <class TL, int NT, class KGate>
 __device__ __forceinline__ void delta_spectra(const DeltaDftArgs& d, const float* base, size_t seg, int n, bool emit,
                                               float4* RA, float4* RB, const float2* TW, const float2* TH, KGate&& kgate) {
   const DpGeom& g = d.g;
@@ -35,11 +35,11 @@ __device__ __forceinline__ void delta_spectra(const DeltaDftArgs& d, const float
   if (emit) dp_load_fold<NT>(g, base, RA + 2 * n * g.Hp, d.ldx, n);              // q
   const int P = emit ? 3 * n : 2 * n;
   __syncthreads();
-  dp_rows<RT, YT, NT>(g, RA, d.ldx, TW, RB, d.ldc, P);
+  dp_rows<TL::RL, TL::YL, NT>(g, RA, d.ldx, TW, RB, d.ldc, P);
   __syncthreads();
-  dp_cols<RT, YT, NT>(g, RB, d.ldc, TH, P, [&](int x, int k0, int m, const cf* f0, const cf* f1) {
+  dp_cols<TL::RT, TL::YT, NT>(g, RB, d.ldc, TH, P, [&](int x, int k0, int m, const cf* f0, const cf* f1) {
 #pragma unroll
-    for (int e = 0; e < YT; ++e) {
+    for (int e = 0; e < TL::YT; ++e) {
       if (e >= m) continue;
       float s0 = 1.f, s1 = 1.f;
       kgate(x, k0 + e, s0, s1);
@@ -71,24 +71,24 @@ __device__ __forceinline__ void delta_norms(const DeltaDftArgs& d, const float4*
 }
 
 // folded output spectra RB[k][col of n planes] -> real planes at dst
-template <int RT, int YT, int NT>
+template <class TL, int NT>
 __device__ __forceinline__ void delta_output(const DeltaDftArgs& d, float4* RA, float4* RB, const float2* TW, const float2* TH,
                                              float* dst, int n) {
   __syncthreads();
-  dp_inv_cols<RT, YT, NT>(d.g, RB, d.ldc, TH, RA, d.ldx, n);
+  dp_inv_cols<TL::RL, TL::YL, NT>(d.g, RB, d.ldc, TH, RA, d.ldx, n);
   __syncthreads();
-  dp_inv_rows<RT, YT, NT>(d.g, RA, d.ldx, TW, reinterpret_cast<float*>(RB), n);
+  dp_inv_rows<TL::RL, TL::YL, NT>(d.g, RA, d.ldx, TW, reinterpret_cast<float*>(RB), n);
   __syncthreads();
   dp_store<NT>(d.g, reinterpret_cast<const float*>(RB), dst, nullptr, n);
 }
 
-template <int RT, int YT, int NT, int DK>
+template <class TL, int NT, int DK>
 __global__ void __launch_bounds__(NT, 512 / NT) gdn_spectral_dft(const GdnSpectralArgs a, const DeltaDftArgs d) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DpGeom& g = d.g;
   float2* TW = reinterpret_cast<float2*>(smem_raw);
   float2* TH = TW + g.Wp * g.ldw;
-  unsigned char* base = reinterpret_cast<unsigned char*>(TH + g.Hp * g.ldh);
+  unsigned char* base = reinterpret_cast<unsigned char*>(TW + dp_table_pairs(g));
   float4* RA = reinterpret_cast<float4*>(base);
   float4* RB = reinterpret_cast<float4*>(base + d.region);
   float* nrm = reinterpret_cast<float*>(base + 2 * d.region);
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) gdn_spectral_dft(const GdnSpectr
       const size_t seg = (size_t)a.C * HW;
       const bool emit = !a.last_only || t == Tdata - 1;               // same for the whole CTA
       __syncthreads();                                                // tables written; RA, RB free again
-      delta_spectra<RT, YT, NT>(d, fp, seg, n, emit, RA, RB, TW, TH, [](int, int, float&, float&) {});
+      delta_spectra<TL, NT>(d, fp, seg, n, emit, RA, RB, TW, TH, [](int, int, float&, float&) {});
       delta_norms<NT>(d, RA, nrm, n, emit, a.use_l2 != 0);
       const float2* abf = a.ab + (a.static_image ? (size_t)b * a.T : frame) * a.ab_heads * NB;
       for (int i = threadIdx.x; i < nhd * cells; i += NT) {
@@ -187,18 +187,18 @@ __global__ void __launch_bounds__(NT, 512 / NT) gdn_spectral_dft(const GdnSpectr
                                                                mk(o[1].x * invHW, o[1].y * invHW));
         }
       }
-      if (emit) delta_output<RT, YT, NT>(d, RA, RB, TW, TH, fp + 2 * seg, n);
+      if (emit) delta_output<TL, NT>(d, RA, RB, TW, TH, fp + 2 * seg, n);
     }
   }
 }
 
-template <int RT, int YT, int NT>
+template <class TL, int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) deltanet_spectral_dft(const DnSpectralArgs a, const DeltaDftArgs d) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DpGeom& g = d.g;
   float2* TW = reinterpret_cast<float2*>(smem_raw);
   float2* TH = TW + g.Wp * g.ldw;
-  unsigned char* base = reinterpret_cast<unsigned char*>(TH + g.Hp * g.ldh);
+  unsigned char* base = reinterpret_cast<unsigned char*>(TW + dp_table_pairs(g));
   float4* RA = reinterpret_cast<float4*>(base);
   float4* RB = reinterpret_cast<float4*>(base + d.region);
   float* nrm = reinterpret_cast<float*>(base + 2 * d.region);
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) deltanet_spectral_dft(const DnSp
       const float4* gm = a.abkv + frame * NB;
       const float* cg = a.cg + frame * NB;
       __syncthreads();                                                // tables written; RA, RB free again
-      delta_spectra<RT, YT, NT>(d, fp, seg, n, true, RA, RB, TW, TH, [&](int x, int k, float& s0, float& s1) {
+      delta_spectra<TL, NT>(d, fp, seg, n, true, RA, RB, TW, TH, [&](int x, int k, float& s0, float& s1) {
         if (chan || x >= n * g.Wp) return;                            // B_k scales the key spectra
         const int kw = x - g.dWp.div(x) * g.Wp;
         s0 = __ldg(&gm[k * g.Wp + kw].z);
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) deltanet_spectral_dft(const DnSp
         *ss = make_float4(h[0].x, h[0].y, h[1].x, h[1].y);
         RB[k * d.ldc + cl * g.Wp + kw] = dp_fold_spec(self, o[0], o[1]);
       }
-      delta_output<RT, YT, NT>(d, RA, RB, TW, TH, fp + 2 * seg, n);
+      delta_output<TL, NT>(d, RA, RB, TW, TH, fp + 2 * seg, n);
     }
   }
 }
@@ -278,7 +278,7 @@ static size_t delta_dft_bytes(const DpGeom& g, int P, int arg) {
 static bool delta_dft_plan(int B, int T, int C, int H, int W, int dk, bool need_smem_state, DeltaDftArgs* d, DpChoice* ch) {
   memset(d, 0, sizeof(*d));
   for (int st = 1; st >= (need_smem_state ? 1 : 0); --st) {
-    *ch = dp_choose(H, W, 3 * C, B, 3 * dk, 226 * 1024, delta_dft_bytes, 2 * dk + st);
+    *ch = dp_choose(H, W, 3 * C, B, 3 * dk, 3, 226 * 1024, delta_dft_bytes, 2 * dk + st);
     if (ch->P == 0) continue;
     d->smem_state = st;
     d->B = B; d->T = T; d->C = C;
@@ -306,11 +306,10 @@ static int delta_dft_launch(Kern kern, const Args& a, const DeltaDftArgs& d, con
 
 template <int DK>
 static int gdn_dft_dk(const GdnSpectralArgs& a, const DeltaDftArgs& d, const DpChoice& ch, cudaStream_t st) {
-  if (ch.threads == 256)
-    return ch.wide ? delta_dft_launch(gdn_spectral_dft<2, 4, 256, DK>, a, d, ch, st)
-                   : delta_dft_launch(gdn_spectral_dft<1, 2, 256, DK>, a, d, ch, st);
-  return ch.wide ? delta_dft_launch(gdn_spectral_dft<2, 4, 128, DK>, a, d, ch, st)
-                 : delta_dft_launch(gdn_spectral_dft<1, 2, 128, DK>, a, d, ch, st);
+  return dp_pick(ch.tiles, [&](auto tl) {
+    using TL = decltype(tl);
+    return ch.threads == 256 ? delta_dft_launch(gdn_spectral_dft<TL, 256, DK>, a, d, ch, st) : delta_dft_launch(gdn_spectral_dft<TL, 128, DK>, a, d, ch, st);
+  });
 }
 
 int launch_gdn_spectral_dft(const GdnSpectralArgs& a, cudaStream_t st) {
@@ -329,11 +328,10 @@ int launch_deltanet_spectral_dft(const DnSpectralArgs& a, cudaStream_t st) {
   DeltaDftArgs d;
   DpChoice ch;
   if (!delta_dft_plan(a.B, a.T, a.C, a.H, a.W, 1, true, &d, &ch)) return CSSM_ERR_UNSUPPORTED;
-  if (ch.threads == 256)
-    return ch.wide ? delta_dft_launch(deltanet_spectral_dft<2, 4, 256>, a, d, ch, st)
-                   : delta_dft_launch(deltanet_spectral_dft<1, 2, 256>, a, d, ch, st);
-  return ch.wide ? delta_dft_launch(deltanet_spectral_dft<2, 4, 128>, a, d, ch, st)
-                 : delta_dft_launch(deltanet_spectral_dft<1, 2, 128>, a, d, ch, st);
+  return dp_pick(ch.tiles, [&](auto tl) {
+    using TL = decltype(tl);
+    return ch.threads == 256 ? delta_dft_launch(deltanet_spectral_dft<TL, 256>, a, d, ch, st) : delta_dft_launch(deltanet_spectral_dft<TL, 128>, a, d, ch, st);
+  });
 }
 
 }  // namespace cssm

@@ -123,9 +123,9 @@ inline size_t dp_region_bytes(const DpGeom& g, int P) {
   m = m > plane ? m : plane;
   return m * 16;
 }
-inline size_t dp_table_bytes(const DpGeom& g) {
-  return ((size_t)g.Wp * g.ldw + (size_t)g.Hp * g.ldh) * 8;
-}
+// Both tables and four pairs more: a tile of eight cells may read that far past the last row (cells it throws away).
+__host__ __device__ inline int dp_table_pairs(const DpGeom& g) { return g.Wp * g.ldw + g.Hp * g.ldh + 4; }
+inline size_t dp_table_bytes(const DpGeom& g) { return (size_t)dp_table_pairs(g) * 8; }
 
 // P planes from global memory (consecutive, HW apart) -> folded row operand [pixel pair][row pair].
 // Four entries (16 loads) in flight per thread.
@@ -259,9 +259,27 @@ __device__ __forceinline__ void dp_store(const DpGeom& g, const float* out, floa
   }
 }
 
-// Launch choice of the plane-group kernels: P planes per CTA (a multiple of `unit`), wide = 2 x 4 register
-// tiles instead of 1 x 2, CTAs per SM, threads, dynamic shared memory.  bytes(g, P, arg): shared memory of P planes.
-struct DpChoice { int P, wide, ctas, threads; size_t smem; double cost; };
-DpChoice dp_choose(int H, int W, int C, int B, int unit, size_t limit, size_t (*bytes)(const DpGeom&, int, int), int arg);
+// Register tiles of a kernel: RT x YT cells in the forward columns, whose epilogue holds the recurrence, and RL x YL in the
+// other three passes.  A pass reads 16 (RT + YT / 2) bytes of shared memory for its 2 RT YT packed multiply-adds, so that a
+// lane's 16-byte operand (four wavefronts a warp) is what the light passes wait for: eight cells a lane (1 x 8, one operand
+// and four broadcast reads of the table) take 8 wavefronts for 16 of them where 2 x 4 takes 10 and 1 x 2 takes 20.  The forward columns have no
+// registers left for it, and planes that leave lanes idle want the smaller tiles.  (2 x 8: best for none of 40 shapes.)
+template <int RT_, int YT_, int RL_, int YL_> struct DpTiles { static constexpr int RT = RT_, YT = YT_, RL = RL_, YL = YL_; };
+
+// Launch choice of the plane-group kernels: P planes per CTA (a multiple of `unit`; one of `back` is transformed back), the pair of register tiles (dp_pick),
+// CTAs per SM, threads, dynamic shared memory.  bytes(g, P, arg): shared memory of P planes.
+struct DpChoice { int P, tiles, ctas, threads; size_t smem; double cost; };
+DpChoice dp_choose(int H, int W, int C, int B, int unit, int back, size_t limit, size_t (*bytes)(const DpGeom&, int, int), int arg);
+
+constexpr int DP_TILES = 5;
+template <class F> auto dp_pick(int tiles, F&& f) {
+  switch (tiles) {
+    case 0: return f(DpTiles<1, 2, 1, 2>{});
+    case 1: return f(DpTiles<1, 2, 1, 4>{});
+    case 2: return f(DpTiles<2, 4, 1, 4>{});
+    case 3: return f(DpTiles<2, 4, 2, 4>{});
+    default: return f(DpTiles<2, 4, 1, 8>{});
+  }
+}
 
 }  // namespace cssm

@@ -8,7 +8,8 @@
 //
 // Bound: the packed FMAs of the four products and the shared-memory reads that feed them
 // (4 P Hp Wp (Hp + Wp) / 2 packed multiply-adds a step); below 20 x 20 pixels the loads and barriers.
-// 16 x 8 x 56 x 56 x 32: 1074 (direct DFTs, one thread per output) -> 210 us; 48 x 8 x 14 x 14 x 256 and
+// 16 x 8 x 56 x 56 x 32: 1074 (direct DFTs, one thread per output) -> 223 -> 197 us (1 x 8 cells a lane in three passes instead
+// of 2 x 4); 12 x 8 x 28 x 28 x 64 82 -> 74, 2 x 4 x 72 x 72 x 32 92 -> 72, 512 x 1 x 7 x 7 x 384 84 -> 72; 48 x 8 x 14 x 14 x 256 and
 // 7 x 7 x 384, last frame only: 676 -> 283 us for the three launches of a forward.
 #include <math.h>
 #include <string.h>
@@ -28,13 +29,14 @@ struct GatedDftArgs {
 // EQUAL: clips of equal frames, of which the T first are there (launch_gated_spectral_dft).  A variant of its own: the tests and the
 // loop of steps took 0.5 to 5 % of the other blocks' passes (NoGate 367 x 5 x 8 x 8 x 32 88.2 us with, 84.5 without; 22 x 8 x 37 x 16 x 64
 // 121.7, 119.4; gated 16 x 8 x 14 x 14 x 64 86.7, 84.9).
-template <int RT, int YT, int NT, bool EQUAL>
+template <class TL, int NT, bool EQUAL>
 __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDftArgs a) {
+  constexpr int RT = TL::RT, YT = TL::YT, RL = TL::RL, YL = TL::YL;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DpGeom& g = a.g;
   float2* TW = reinterpret_cast<float2*>(smem_raw);
   float2* TH = TW + g.Wp * g.ldw;
-  unsigned char* base = reinterpret_cast<unsigned char*>(TH + g.Hp * g.ldh);
+  unsigned char* base = reinterpret_cast<unsigned char*>(TW + dp_table_pairs(g));
   float4* RA = reinterpret_cast<float4*>(base);
   float4* RB = reinterpret_cast<float4*>(base + a.region);
   float4* ST = reinterpret_cast<float4*>(base + 2 * a.region);       // [k][col] {h_k, h_{H-k}}
@@ -55,7 +57,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
       __syncthreads();                                               // tables written; RA free again
       dp_load_fold<NT>(g, xp, RA, ldx, P);
       __syncthreads();
-      dp_rows<RT, YT, NT>(g, RA, ldx, TW, RB, ldc, P);
+      dp_rows<RL, YL, NT>(g, RA, ldx, TW, RB, ldc, P);
       __syncthreads();
       const float4* gp = a.gates + frame * NB;
       dp_cols<RT, YT, NT>(g, RB, ldc, TH, P, [&](int x, int kr, int m, const cf* f0, const cf* f1) {
@@ -102,10 +104,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
       });
       if (!emit) continue;
       __syncthreads();
-      dp_inv_cols<RT, YT, NT>(g, RA, ldc, TH, RB, ldx, P);
+      dp_inv_cols<RL, YL, NT>(g, RA, ldc, TH, RB, ldx, P);
       __syncthreads();
       float* out = reinterpret_cast<float*>(RA);
-      dp_inv_rows<RT, YT, NT>(g, RB, ldx, TW, out, P);
+      dp_inv_rows<RL, YL, NT>(g, RB, ldx, TW, out, P);
       __syncthreads();
       if constexpr (EQUAL) dp_store<NT>(g, out, xp, a.xz + (((size_t)b * a.T * 2 + 1) * a.C + c0) * HW, P);      // (mode 0)
       else dp_store<NT>(g, out, xp, a.mode == 0 ? xp + (size_t)a.C * HW : nullptr, P);
@@ -113,46 +115,52 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
   }
 }
 
-// Planes per CTA, register tile and threads: the estimate adds up, for a wave of CTAs, the time of the four
+// Planes per CTA, register tiles and threads: the estimate adds up, for a wave of CTAs, the time of the four
 // passes of a step (throughput of the SM, or the latency of a pass when its tiles do not fill the threads)
-// and a fixed part for the loads and barriers.  The constants were fitted to 19 shapes from 1 x 14 x 14 x 256
-// to 16 x 8 x 56 x 56 x 32 (some 40 choices each); the choice is within 5 % of the best of them everywhere.
+// and a fixed part for the loads and barriers.  The constants were fitted to 40 shapes of the gated kernel and 19 of the
+// gated DeltaNet's, 1 x 14 x 14 to 16 x 8 x 56 x 56 (100 to 170 choices each): the times that it picks are 1.6 % above the best
+// of all choices in the mean and 5.4 % below those with one register tile for all passes; two of the 59 are above them, by a microsecond or two.
 // (Fitted on 148 SMs; another device's count takes the place of that number.)  The search is a few
 // microseconds of host time, so each thread remembers its last few answers: a pure function of the key.
-DpChoice dp_choose(int H, int W, int C, int B, int unit, size_t limit, size_t (*bytes)(const DpGeom&, int, int), int arg) {
-  struct Memo { int H, W, C, B, unit, arg, sms; size_t limit; size_t (*bytes)(const DpGeom&, int, int); DpChoice c; };
+DpChoice dp_choose(int H, int W, int C, int B, int unit, int back, size_t limit, size_t (*bytes)(const DpGeom&, int, int), int arg) {
+  struct Memo { int H, W, C, B, unit, back, arg, sms; size_t limit; size_t (*bytes)(const DpGeom&, int, int); DpChoice c; };
   static thread_local Memo memo[8] = {};
   const int sms = sm_count();
   Memo& m = memo[(H * 31 + W * 17 + C + B * 7 + arg + unit) & 7];
-  if (m.bytes == bytes && m.H == H && m.W == W && m.C == C && m.B == B && m.unit == unit && m.arg == arg && m.sms == sms &&
+  if (m.bytes == bytes && m.H == H && m.W == W && m.C == C && m.B == B && m.unit == unit && m.back == back && m.arg == arg && m.sms == sms &&
       m.limit == limit)
     return m.c;
   const DpGeom g = dp_geom(H, W);
   DpChoice best;
-  best.P = 0; best.cost = 1e30; best.wide = 0; best.ctas = 1; best.smem = 0;
+  best.P = 0; best.cost = 1e30; best.tiles = 0; best.ctas = 1; best.smem = 0;
   for (int P = unit; P <= C && P <= 128 * unit; P += unit) {
     const size_t smem = bytes(g, P, arg);
     if (smem > limit) break;
     const double groups = (double)B * ((C + P - 1) / P);
-    for (int v = 0; v < 4; ++v) {
-      const int wide = v & 1, nt = v & 2 ? 256 : 128;
+    for (int v = 0; v < 2 * DP_TILES; ++v) {
+      const int tiles = v >> 1, nt = v & 1 ? 256 : 128;
       const int fit = (int)((227 * 1024) / (smem + 1024)), most = 512 / nt, occ = fit > most ? most : (fit < 1 ? 1 : fit);
-      const int RT = wide ? 2 : 1, YT = wide ? 4 : 2;
-      auto up = [](int a, int b) { return (a + b - 1) / b; };
-      const double tr = (double)up(P * g.Hp, RT) * up(g.Wp, YT), tc = (double)up(P * g.Wp, RT) * up(g.Hp, YT);
       // clocks: SM time of a tile and reduction step, latency of a step, of an epilogue
-      const double per = wide ? 0.094 : 0.163, lat = wide ? 129 : 30, epi = wide ? 180 : 320;
-      auto pass = [&](double tiles, int n, double q) {
-        const double thr = q * tiles * (n * per + 0.029 * RT * YT), ltn = ceil(tiles / nt) * (n * lat + epi);
+      struct Tile { int r, y; double per, lat, epi; };
+      static constexpr Tile HEAVY[2] = {{1, 2, 0.11, 34.7, 198}, {2, 4, 0.0501, 39, 954}};
+      static constexpr Tile LIGHT[4] = {{1, 2, 0.082, 36, 216}, {1, 4, 0.123, 37.9, 304}, {2, 4, 0.272, 78.5, 478}, {1, 8, 0.224, 77.2, 427}};
+      const Tile h = HEAVY[tiles >= 2], l = LIGHT[tiles >= 2 ? tiles - 1 : tiles];
+      auto up = [](int a, int b) { return (a + b - 1) / b; };
+      auto pass = [&](const Tile& t, int X, int Y, double q) {
+        const int nx = up(X, t.r);                 // (a warp on the border of two rows of tiles reads two table entries)
+        const double n = (double)nx * up(Y, t.y);
+        const double thr = q * n * (Y * t.per * (1 + 0.185 * 32 / nx) + 0.0108 * t.r * t.y), ltn = ceil(n / nt) * (Y * t.lat + t.epi);
         return thr > ltn ? thr : ltn;
       };
       const double resident = groups < (double)sms * occ ? ceil(groups / sms) : occ;
-      const double step = 2 * pass(tr, g.Wp, resident) + 2 * pass(tc, g.Hp, resident) + 2930 + resident * P * H * W;
-      const double cost = ceil(groups / (sms * resident)) * step;
-      if (cost < best.cost) { best.cost = cost; best.P = P; best.wide = wide; best.ctas = occ; best.threads = nt; best.smem = smem; }
+      const int Q = P / back;
+      const double step = pass(l, P * g.Hp, g.Wp, resident) + pass(h, P * g.Wp, g.Hp, resident) + pass(l, Q * g.Wp, g.Hp, resident) +
+                          pass(l, Q * g.Hp, g.Wp, resident) + 455 + 0.252 * resident * P * H * W;
+      const double cost = ceil(groups / (sms * resident)) * step * (nt > 128 ? 1.03 : 1.0);
+      if (cost < best.cost) { best.cost = cost; best.P = P; best.tiles = tiles; best.ctas = occ; best.threads = nt; best.smem = smem; }
     }
   }
-  m = Memo{H, W, C, B, unit, arg, sms, limit, bytes, best};
+  m = Memo{H, W, C, B, unit, back, arg, sms, limit, bytes, best};
   return best;
 }
 
@@ -164,13 +172,15 @@ bool gated_spectral_dft_fits(int H, int W, int T) { return gated_dft_bytes(dp_ge
 
 template <bool EQUAL>
 static auto pick_kernel(const DpChoice& ch) {
-  return ch.threads == 256 ? (ch.wide ? gated_spectral_dft<2, 4, 256, EQUAL> : gated_spectral_dft<1, 2, 256, EQUAL>)
-                           : (ch.wide ? gated_spectral_dft<2, 4, 128, EQUAL> : gated_spectral_dft<1, 2, 128, EQUAL>);
+  return dp_pick(ch.tiles, [&](auto tl) {
+    using TL = decltype(tl);
+    return ch.threads == 256 ? gated_spectral_dft<TL, 256, EQUAL> : gated_spectral_dft<TL, 128, EQUAL>;
+  });
 }
 
 int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat, const float* gates, float* xz,
                               int last_only, int mode, cudaStream_t st, const float* dchan, int equal_steps) {
-  const DpChoice ch = dp_choose(H, W, C, B, 1, 226 * 1024, gated_dft_bytes, T);
+  const DpChoice ch = dp_choose(H, W, C, B, 1, 1, 226 * 1024, gated_dft_bytes, T);
   if (ch.P == 0 || (equal_steps > 0 && mode != 0)) return CSSM_ERR_UNSUPPORTED;
   GatedDftArgs a;
   memset(&a, 0, sizeof(a));

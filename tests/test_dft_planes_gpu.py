@@ -59,3 +59,22 @@ def test_delta_rules(B, T, H, W, C, dk):
         kw = dict(kernel_size=1, rope_mode="none", gate_type="dense" if H % 2 else "channel")
         p = orc.init_deltanet_params(3, C, H, W, kernel_size=1, gate_type=kw["gate_type"], bias_scale=0.1)
         _check(DeltaNetCSSM(channels=C, **kw).apply({"params": p}, xd), orc.deltanet_forward(p, x, **kw))
+
+
+# Batches that fill the GPU, where the passes take the larger register tiles (1 x 4, 2 x 4 and 1 x 8 cells): two clips over and
+# over, so that the oracle has two to do and every plane group of the batch has to repeat them.
+@pytest.mark.parametrize("kind,B,T,H,W,C", [("gated", 16, 2, 56, 56, 32), ("gated", 33, 1, 16, 16, 256), ("gated", 40, 2, 24, 24, 64),
+                                            ("gated", 12, 2, 28, 28, 64), ("gated", 9, 1, 51, 43, 64), ("delta", 16, 2, 28, 28, 64),
+                                            ("delta", 9, 2, 47, 45, 32), ("delta", 33, 1, 14, 14, 64)])
+def test_full_batches(kind, B, T, H, W, C):
+    x = np.random.default_rng(H + W + C).standard_normal((2, T, H, W, C)).astype(np.float32)
+    idx = np.arange(B) % 2
+    xd = torch.from_numpy(x[idx]).cuda()
+    kw = dict(kernel_size=1, rope_mode="none", gate_type="factored")
+    if kind == "gated":
+        p = orc.init_gated_params(1, C, H, W, bias_scale=0.1, kernel_size=1, gate_type="factored")
+        _check(GatedCSSM(channels=C, **kw).apply({"params": p}, xd), orc.gated_forward(p, x, **kw)[idx])
+    else:
+        p = orc.init_gdn_params(1, C, H, W, bias_scale=0.1, perturb_rms=True, delta_key_dim=2, kernel_size=1, gate_type="factored")
+        _check(GatedDeltaNetCSSM(channels=C, delta_key_dim=2, **kw).apply({"params": p}, xd),
+               orc.gdn_forward(p, x, delta_key_dim=2, **kw)[idx])
