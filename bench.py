@@ -84,7 +84,7 @@ GDN_JOINED = {"qkv_proj": "qkv_proj_short_convs", "short_convs": "qkv_proj_short
 def spectral_kernel(gdn, H):
     """Kernel of the recurrence on H x H planes (GDN: key dim 4)."""
     if gdn:
-        return {64: "gdn_spectral_r64", 32: "gdn_spectral_p32"}.get(H, "gdn_spectral_dft")
+        return {64: "gdn_spectral_p64", 32: "gdn_spectral_p32"}.get(H, "gdn_spectral_dft")
     return {64: "gated_spectral_r64", 32: "gated_spectral_r32"}.get(H, "gated_spectral_dft")
 
 

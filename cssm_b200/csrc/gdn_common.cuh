@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_bf16.h>
 #include "common.cuh"
+#include "bf16_ops.cuh"
 
 namespace cssm {
 
@@ -63,6 +64,55 @@ __device__ __forceinline__ cf gdn_bin_update_regs(cf (&s)[DK], const cf* kk, con
     }
   }
   return o;
+}
+
+// The same update for all four rows of a 4 x 4 state, packed over pairs of rows: S?[r][i] = {row 2 r, row 2 r + 1} of column i, x real
+// and y imaginary parts; bv: beta times the rows' values.
+__device__ __forceinline__ void gdn_rows_update(unsigned long long (&Sx)[2][4], unsigned long long (&Sy)[2][4], const cf (&kk)[4],
+                                                const cf (&bv)[4], cf aw, float beta) {
+  typedef unsigned long long u64;
+  u64 kx[4], ky[4], kyn[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { kx[i] = pk2(kk[i].x, kk[i].x); ky[i] = pk2(kk[i].y, kk[i].y); kyn[i] = pk2(-kk[i].y, -kk[i].y); }
+  const u64 ax = pk2(aw.x, aw.x), ay = pk2(aw.y, aw.y), ayn = pk2(-aw.y, -aw.y), bn = pk2(-beta, -beta);
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    // d = sum_j conj(k_j) S_j;  S_i <- aw (S_i - beta k_i d) + beta v conj(k_i)
+    u64 dr = 0ull, di = 0ull;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      dr = fma2(Sx[r][i], kx[i], dr); dr = fma2(Sy[r][i], ky[i], dr);
+      di = fma2(Sy[r][i], kx[i], di); di = fma2(Sx[r][i], kyn[i], di);
+    }
+    const u64 er = mul2(dr, bn), ei = mul2(di, bn);
+    const cf v0 = bv[2 * r], v1 = bv[2 * r + 1];
+    const u64 bvx = pk2(v0.x, v1.x), bvy = pk2(v0.y, v1.y), bvxn = pk2(-v0.x, -v1.x);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const u64 ir = fma2(kyn[i], ei, fma2(kx[i], er, Sx[r][i])), ii = fma2(ky[i], er, fma2(kx[i], ei, Sy[r][i]));
+      Sx[r][i] = fma2(bvy, ky[i], fma2(bvx, kx[i], fma2(ayn, ii, mul2(ax, ir))));
+      Sy[r][i] = fma2(bvxn, ky[i], fma2(bvy, kx[i], fma2(ay, ir, mul2(ax, ii))));
+    }
+  }
+}
+// o = sum_i S_i q_i
+__device__ __forceinline__ void gdn_rows_read(const unsigned long long (&Sx)[2][4], const unsigned long long (&Sy)[2][4], const cf (&qq)[4], cf (&o)[4]) {
+  typedef unsigned long long u64;
+  u64 orr[2] = {0ull, 0ull}, oi[2] = {0ull, 0ull};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const u64 qx = pk2(qq[i].x, qq[i].x), qy = pk2(qq[i].y, qq[i].y), qyn = pk2(-qq[i].y, -qq[i].y);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      orr[r] = fma2(Sx[r][i], qx, orr[r]); orr[r] = fma2(Sy[r][i], qyn, orr[r]);
+      oi[r] = fma2(Sx[r][i], qy, oi[r]); oi[r] = fma2(Sy[r][i], qx, oi[r]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    upk2(orr[r], o[2 * r].x, o[2 * r + 1].x);
+    upk2(oi[r], o[2 * r].y, o[2 * r + 1].y);
+  }
 }
 
 __device__ __forceinline__ float bf16r(float x) {

@@ -163,10 +163,11 @@ size_t gdn_generic_smem_bytes(int H, int W, int dk) {
 int launch_gdn_spectral_r64(const GdnSpectralArgs& a, cudaStream_t st);
 int launch_gdn_spectral_r32(const GdnSpectralArgs& a, cudaStream_t st);
 int launch_gdn_spectral_p32(const GdnSpectralArgs& a, cudaStream_t st);
+int launch_gdn_spectral_p64(const GdnSpectralArgs& a, cudaStream_t st);
 
 int launch_gdn_spectral(const GdnSpectralArgs& a, cudaStream_t st) {
   if (a.dk < 1 || a.dk > GDN_MAXDK || a.C % a.dk != 0) return CSSM_ERR_UNSUPPORTED;
-  if (spectral_path(a.H, a.W) == PATH_R64 && a.dk == 4) return launch_gdn_spectral_r64(a, st);
+  if (spectral_path(a.H, a.W) == PATH_R64 && a.dk == 4) return a.static_image ? launch_gdn_spectral_r64(a, st) : launch_gdn_spectral_p64(a, st);
   if (spectral_path(a.H, a.W) == PATH_R32 && a.dk == 4) return a.static_image ? launch_gdn_spectral_r32(a, st) : launch_gdn_spectral_p32(a, st);
   const int rc = launch_gdn_spectral_dft(a, st);
   if (rc != CSSM_ERR_UNSUPPORTED) return rc;

@@ -1,15 +1,13 @@
-// GDN fused spectral kernel for 64x64 planes, d_k = d_v = 4.  A CTA runs one (batch, head) after another
-// with two groups of 288 threads, each with its own transform buffers: per step a group transforms
+// GDN fused spectral kernel for 64x64 planes, d_k = d_v = 4, static images (one frame of q, k, v per batch element, the T gate steps
+// run per bin; frames of their own: csrc/gdn_spectral_p64.cu).  A CTA runs one (batch, head) after another
+// with two groups of 288 threads, each with its own transform buffers: a group transforms
 // every other q / k plane into the shared spectra (shared memory, in the column lanes' own bin order),
 // the norms are applied there in place, and then each group takes every other v plane: transform,
-// update of its state row, readout, inverse transform over the v plane.
+// all steps of its state row, readout, inverse transform over the v plane.
 //
-// Bound: the shared-memory pipe (80 % of its wavefronts, B = 16; DRAM 18 %, L2 23 %).  With one group (nine
-// warps) latency was the bound; the two groups fit next to the spectra because a group's inverse columns go
-// over its forward rows (one more barrier a v row) and the lanes without a column need no spectrum slot
-// and one exchange region.  The state of the running heads (270 KB each) stays in L2: scratch goes by CTA,
-// not by head, and the first step reads no state and the last one writes none.
-// 128 x 8 x 64 x 64 x 64: 4.61 -> 3.76 ms.
+// Bound: the T steps of a bin, four rows of sixteen complex products rounded to bfloat16.  The two groups fit next to the spectra because a
+// group's inverse columns go over its forward rows (one more barrier a v row) and the lanes without a column need no spectrum slot
+// and one exchange region.
 #include "r64.cuh"
 #include "kernels.cuh"
 #include "gdn_common.cuh"
@@ -40,9 +38,6 @@ __device__ __forceinline__ void g64_init(R64Ctx& c, cf* EX, cf* ZR, int tid) {
   }
 }
 
-// LAST: only the last step's output planes are produced (compile-time switch).
-// STATIC: static-image fast path (one data frame per batch element, the T gate steps run per bin).
-template <bool LAST, bool STATIC>
 __global__ void __launch_bounds__(G64_NT, 1) gdn_spectral_r64(const GdnSpectralArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float red[2][9][4];
@@ -56,41 +51,34 @@ __global__ void __launch_bounds__(G64_NT, 1) gdn_spectral_r64(const GdnSpectralA
   auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(half + 1), "n"(R64_NT) : "memory"); };
   constexpr int HW = 4096, NB = 64 * 33, DK = 4;
   const int nh = a.C / DK, heads = a.B * nh;
-  const int Tdata = STATIC ? 1 : a.T;          // frames of q, k, v per batch element
   const float invHW = 1.0f / (float)HW;
   // slot of this lane in the spectra (warp 8 has one column: lanes 0, 4, 8, ...)
   const int slot = c.warp < 8 ? tid : 256 + c.a;
-  // state scratch S[v][i][q][lane]; a thread only ever touches its own slots
-  cf* S = a.state + (size_t)blockIdx.x * DK * DK * NB + c.grp * 8 + c.a;
   pdl_sync();
 
-  // plane 2 i + half of step t: i = 0, 1 q, 2, 3 k, 4, 5 v; i = 6: the first of step t + 1 (of the
-  // next head).  last_only: steps before the last one skip the q planes.
-  auto first_of = [&](int t) -> int { return (LAST && t < Tdata - 1) ? 2 : 0; };
-  auto plane_of = [&](int bh, int t, int i) -> float* {
-    if (i >= 6) { ++t; if (t >= Tdata) { t = 0; bh += gridDim.x; } i = first_of(t); }
+  // plane 2 i + half: i = 0, 1 q, 2, 3 k, 4, 5 v; i = 6: the first of the next head
+  auto plane_of = [&](int bh, int i) -> float* {
+    if (i >= 6) { bh += gridDim.x; i = 0; }
     if (bh >= heads) bh = blockIdx.x;                       // harmless re-read past the end
     const int b = bh / nh, hd = bh - b * nh, idx = 2 * i + half;
-    return a.qkv + ((size_t)(b * Tdata + t) * 3 * a.C + (size_t)(idx >> 2) * a.C + hd * DK + (idx & 3)) * HW;
+    return a.qkv + ((size_t)b * 3 * a.C + (size_t)(idx >> 2) * a.C + hd * DK + (idx & 3)) * HW;
   };
   cf nx[8];                                   // rows of the NEXT plane, fetched one pass ahead
-  r64_load_rows(c, plane_of(blockIdx.x, 0, first_of(0)), nx);
+  r64_load_rows(c, plane_of(blockIdx.x, 0), nx);
 
   for (int bh = blockIdx.x; bh < heads; bh += gridDim.x) {
-  const int b = bh / nh, hd = bh - b * nh;
-  const cf* wh = a.what + (size_t)hd * NB + (c.grp << 3) + c.a;
-  for (int t = 0; t < Tdata; ++t) {
-    const bool emit = !LAST || t == Tdata - 1;       // same for the whole CTA
+    const int b = bh / nh, hd = bh - b * nh;
+    const cf* wh = a.what + (size_t)hd * NB + (c.grp << 3) + c.a;
     // ---- q planes (i = 0, 1) and k planes (i = 2, 3) ----
 #pragma unroll 1
-    for (int i = first_of(t); i < 4; ++i) {
-      // own ZR free; at the first plane also: nobody reads the spectra of the step before any more
-      if (i == first_of(t)) __syncthreads(); else group_sync();
+    for (int i = 0; i < 4; ++i) {
+      // own ZR free; at the first plane also: nobody reads the spectra of the head before any more
+      if (i == 0) __syncthreads(); else group_sync();
       {
         cf cur[8];
 #pragma unroll
         for (int m = 0; m < 8; ++m) cur[m] = nx[m];
-        r64_load_rows(c, plane_of(bh, t, i + 1), nx);
+        r64_load_rows(c, plane_of(bh, i + 1), nx);
         r64_row_fwd_regs(c, cur);
       }
       group_sync();
@@ -107,8 +95,6 @@ __global__ void __launch_bounds__(G64_NT, 1) gdn_spectral_r64(const GdnSpectralA
       for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
       if (c.lane == 0) red[half][c.warp][i] = acc;
     }
-    if (c.lane == 0)
-      for (int i = 0; i < first_of(t); ++i) red[half][c.warp][i] = 0.f;
     __syncthreads();
     // ---- normalise in place, the bins split between the groups:
     //      q_hat = q*nq; k_hat = (k*nk) / sqrt(sum_i |.|^2 + 1e-6)
@@ -133,10 +119,8 @@ __global__ void __launch_bounds__(G64_NT, 1) gdn_spectral_r64(const GdnSpectralA
             const cf z = sp[((4 + i) * 8 + q) * G64_COLS];
             kv[i] = mk(z.x * nrm[4 + i], z.y * nrm[4 + i]);
             ks += kv[i].x * kv[i].x + kv[i].y * kv[i].y;
-            if (emit) {
-              const cf qq = sp[(i * 8 + q) * G64_COLS];
-              sp[(i * 8 + q) * G64_COLS] = mk(qq.x * nrm[i], qq.y * nrm[i]);
-            }
+            const cf qq = sp[(i * 8 + q) * G64_COLS];
+            sp[(i * 8 + q) * G64_COLS] = mk(qq.x * nrm[i], qq.y * nrm[i]);
           }
           const float kn = rsqrtf(ks + 1e-6f);
 #pragma unroll
@@ -145,9 +129,8 @@ __global__ void __launch_bounds__(G64_NT, 1) gdn_spectral_r64(const GdnSpectralA
       }
     }
     __syncthreads();
-    // gates: of this frame, or (static path) of step 0 of this batch element's T steps
-    const size_t frame = (size_t)(b * Tdata + t);
-    const float2* abp = a.ab + ((STATIC ? (size_t)b * a.T : frame) * a.ab_heads + (a.ab_heads > 1 ? hd : 0)) * NB + (c.grp << 3) + c.a;
+    // gates of step 0 of this batch element's T steps
+    const float2* abp = a.ab + ((size_t)b * a.T * a.ab_heads + (a.ab_heads > 1 ? hd : 0)) * NB + (c.grp << 3) + c.a;
     // ---- v rows: transform, state update, readout, inverse transform over the v plane ----
 #pragma unroll 1
     for (int i = 4; i < 6; ++i) {
@@ -156,88 +139,47 @@ __global__ void __launch_bounds__(G64_NT, 1) gdn_spectral_r64(const GdnSpectralA
       r64_row_fwd_regs(c, nx);
       group_sync();
       cf v[8];
-      if (STATIC) {
-        r64_col_fwd(c, v);
+      r64_col_fwd(c, v);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          cf kk[4], qq[4], o = mk(0.f, 0.f);
-          if (c.col_on) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              qq[j] = SPEC[(j * 8 + q) * G64_COLS + slot];
-              kk[j] = SPEC[((4 + j) * 8 + q) * G64_COLS + slot];
-            }
-            o = gdn_bin_static<4>(kk, qq, v[q], wh[q * 264], abp + q * 264, (size_t)a.ab_heads * NB, a.T);
-          }
-          v[q] = mk(o.x * invHW, o.y * invHW);
-        }
-      } else {
-        // a bin's state row and gates are requested two bins ahead (L2)
-        cf* srow = S + (size_t)(vr * DK) * NB;
-        cf sreg[2][4];
-        float2 gab[2], w[2];
-        auto fetch = [&](int q) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            sreg[q & 1][j] = (t > 0 && c.col_on) ? srow[(size_t)j * NB + q * 264] : mk(0.f, 0.f);
-          gab[q & 1] = c.col_on ? __ldg(abp + q * 264) : make_float2(0.f, 0.f);
-          w[q & 1] = c.col_on ? __ldg(reinterpret_cast<const float2*>(wh) + q * 264) : make_float2(0.f, 0.f);
-        };
-        fetch(0);
-        fetch(1);
-        r64_col_fwd(c, v);
-        const cf* sp = SPEC + (c.col_on ? slot : 0);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          cf kk[4], qq[4];
+      for (int q = 0; q < 8; ++q) {
+        cf kk[4], qq[4], o = mk(0.f, 0.f);
+        if (c.col_on) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            kk[j] = sp[((4 + j) * 8 + q) * G64_COLS];
-            qq[j] = emit ? sp[(j * 8 + q) * G64_COLS] : mk(0.f, 0.f);
+            qq[j] = SPEC[(j * 8 + q) * G64_COLS + slot];
+            kk[j] = SPEC[((4 + j) * 8 + q) * G64_COLS + slot];
           }
-          const cf aw = mk(gab[q & 1].x * w[q & 1].x, gab[q & 1].x * w[q & 1].y);
-          cf o = mk(0.f, 0.f);
-          if (emit) o = gdn_bin_update_regs<4, true>(sreg[q & 1], kk, qq, v[q], aw, gab[q & 1].y);
-          else gdn_bin_update_regs<4, false>(sreg[q & 1], kk, qq, v[q], aw, gab[q & 1].y);
-          v[q] = mk(o.x * invHW, o.y * invHW);
-          if (c.col_on && t + 1 < Tdata) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) srow[(size_t)j * NB + q * 264] = sreg[q & 1][j];
-          }
-          if (q + 2 < 8) fetch(q + 2);
+          o = gdn_bin_static<4>(kk, qq, v[q], wh[q * 264], abp + q * 264, (size_t)a.ab_heads * NB, a.T);
         }
+        v[q] = mk(o.x * invHW, o.y * invHW);
       }
-      r64_load_rows(c, plane_of(bh, t, i + 1), nx);
-      if (emit) {
-        fft64_lane8<true>(v, c.tw, c.exg, c.a);
-        group_sync();                        // every column of ZR has been read: GB may go over it
+      r64_load_rows(c, plane_of(bh, i + 1), nx);
+      fft64_lane8<true>(v, c.tw, c.exg, c.a);
+      group_sync();                          // every column of ZR has been read: GB may go over it
 #pragma unroll
-        for (int n1 = 0; n1 < 8; ++n1)
-          if (c.col_on) c.GB[(c.a + 8 * n1) * R64_GBS + c.grp] = v[n1];
-        group_sync();
-        if (c.row_on) {
-          r64_row_inv(c, v);
-          float* y0 = a.qkv + (frame * 3 * a.C + 2 * a.C + hd * DK + vr) * HW + (2 * c.grp) * 64 + c.a;
+      for (int n1 = 0; n1 < 8; ++n1)
+        if (c.col_on) c.GB[(c.a + 8 * n1) * R64_GBS + c.grp] = v[n1];
+      group_sync();
+      if (c.row_on) {
+        r64_row_inv(c, v);
+        float* y0 = a.qkv + ((size_t)b * 3 * a.C + 2 * a.C + hd * DK + vr) * HW + (2 * c.grp) * 64 + c.a;
 #pragma unroll
-          for (int n1 = 0; n1 < 8; ++n1) {
-            y0[8 * n1] = v[n1].x;
-            y0[64 + 8 * n1] = v[n1].y;
-          }
+        for (int n1 = 0; n1 < 8; ++n1) {
+          y0[8 * n1] = v[n1].x;
+          y0[64 + 8 * n1] = v[n1].y;
         }
       }
     }
   }
-  }
 }
 
 int launch_gdn_spectral_r64(const GdnSpectralArgs& a, cudaStream_t st) {
+  if (!a.static_image) return CSSM_ERR_UNSUPPORTED;
   const size_t smem = (size_t)G64_SMEM_CF * sizeof(cf);
-  auto kern = a.static_image ? gdn_spectral_r64<false, true>
-                             : (a.last_only ? gdn_spectral_r64<true, false> : gdn_spectral_r64<false, false>);
-  cudaError_t e = func_smem(kern, smem);
+  cudaError_t e = func_smem(gdn_spectral_r64, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   const int heads = a.B * (a.C / 4), sms = sm_count();
-  launch_k(kern, heads < sms ? heads : sms, G64_NT, smem, st, a);
+  launch_k(gdn_spectral_r64, heads < sms ? heads : sms, G64_NT, smem, st, a);
   return check_launch();
 }
 

@@ -508,6 +508,9 @@ int cssm_device_error(int* out, int clear) {
   rc = cssm::read_p32_error(&b2, clear);
   if (rc != CSSM_OK) return rc;
   b |= b2;
+  rc = cssm::read_p64_error(&b2, clear);
+  if (rc != CSSM_OK) return rc;
+  b |= b2;
   int c = 0, m = 0;
   rc = cssm::read_bf16_error(&c, clear);
   if (rc != CSSM_OK) return rc;

@@ -122,6 +122,7 @@ struct GdnSpectralArgs {
 };
 int launch_gdn_spectral(const GdnSpectralArgs& a, cudaStream_t st);
 int read_p32_error(int* out, int clear);
+int read_p64_error(int* out, int clear);
 int launch_gdn_spectral_dft(const GdnSpectralArgs& a, cudaStream_t st);    // as launch_deltanet_spectral_dft
 size_t gdn_generic_smem_bytes(int H, int W, int dk);
 
