@@ -1,7 +1,7 @@
 // tcgen05 / TMEM GEMM for the K = 64 channel projections in fp32-equivalent precision
 // (3 x TF32: A_lo*B_hi + A_hi*B_lo + A_hi*B_hi, accumulated in fp32 in TMEM).
 //
-// Persistent kernel, one CTA per SM, 26 warps:
+// Persistent kernel, one CTA per SM, 26 warps (18 where a second tensor is subtracted):
 //   loader, 1 warp       : TMA copies of 128-pixel A tiles as they lie in memory (channels-last rows, or planar planes and
 //                          their gate planes) into a ring of raw tiles, and the angles of the tile's frame and rows;
 //   converters, 16 or 8  : lane = pixel, 16 of the 64 channels at a time: read the raw tile, apply RoPE or the gate, split every
@@ -38,8 +38,11 @@ __device__ int g_tc_error = 0;
 enum TcForm { TC_PLAIN, TC_ZLAST, TC_MUL, TC_SUB, TC_RMS };
 // Warps: converters, MMA issuer, loader, epilogue.  A wide planar output has more to store than to convert (with sixteen converters and
 // eight epilogue warps: 4.2 M rows to 128 columns 491 us, 429 so; DeltaNet 32x32, whose 192 columns multiply planes, 462 and 415 a pass).
-template <int N, bool A_PLANAR> constexpr int tc_conv = (!A_PLANAR && N > 64) ? 8 : 16;
-constexpr int TC_THREADS = 26 * 32;
+// SUB reads a second tensor behind the accumulator: eight of each, whose registers hold the row to come (26 warps cannot: 12 x 8 x 64 x 64
+// NoGate 218 us a pass, 128 x 8 x 32 x 32 600; so 205 and 562).
+template <int N, bool A_PLANAR, TcForm FORM> constexpr int tc_conv = (FORM == TC_SUB || (!A_PLANAR && N > 64)) ? 8 : 16;
+template <int N, bool A_PLANAR, TcForm FORM> constexpr int tc_epi = FORM == TC_SUB ? 8 : 24 - tc_conv<N, A_PLANAR, FORM>;
+template <int N, bool A_PLANAR, TcForm FORM> constexpr int tc_threads = (tc_conv<N, A_PLANAR, FORM> + tc_epi<N, A_PLANAR, FORM> + 2) * 32;
 
 // One output of a planar A under the RMS prologue by float32 FMAs over k: for results that are not finite (the products are taken
 // before the row factor, and an infinity has no finite parts).
@@ -77,7 +80,7 @@ struct TcSmem {
 };
 
 template <int N, bool A_PLANAR, bool GATE, bool STG, TcForm FORM = TC_PLAIN>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__((tc_threads<N, A_PLANAR, FORM>), 1)
 gemm_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ TcGeom dv, int num_tiles, const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap gmap,
                const __grid_constant__ CUtensorMap omap) {
   // tile schedule: round-robin over the CTAs
@@ -86,7 +89,7 @@ gemm_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ TcGeo
   // operand tiles need 1024-byte alignment (swizzle atoms); the launch adds 1024 bytes of slack
   unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   using L = TcSmem<N, GATE, STG, FORM == TC_RMS>;
-  constexpr int CONV = tc_conv<N, A_PLANAR>, EPI = 24 - CONV;
+  constexpr int CONV = tc_conv<N, A_PLANAR, FORM>, EPI = tc_epi<N, A_PLANAR, FORM>, THREADS = tc_threads<N, A_PLANAR, FORM>;
   constexpr int MMA_WARP = CONV, LOAD_WARP = CONV + 1, EPI_WARP = CONV + 2;
   constexpr int NT = L::NT, NST = 2 * NT, NRAW = L::NRAW;
   const uint32_t sbase = tc::smem_u32(smem);
@@ -117,9 +120,9 @@ gemm_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ TcGeo
     tc::tmem_alloc(tmem_slot, 512);
     tc::tmem_relinquish();
   }
-  tc_split_weights<N, FORM == TC_RMS>(g.Wk, g.N, 0, smem + L::B_OFF, smem + L::B_OFF + L::B_HALF, tid, TC_THREADS, g.rms_scale);
-  if (rope_s) tc_rope_columns(g, smem + L::WANG_OFF, tid, TC_THREADS);
-  for (int n = tid; n < N; n += TC_THREADS) bias_s[n] = g.bias ? g.bias[n] : 0.f;
+  tc_split_weights<N, FORM == TC_RMS>(g.Wk, g.N, 0, smem + L::B_OFF, smem + L::B_OFF + L::B_HALF, tid, THREADS, g.rms_scale);
+  if (rope_s) tc_rope_columns(g, smem + L::WANG_OFF, tid, THREADS);
+  for (int n = tid; n < N; n += THREADS) bias_s[n] = g.bias ? g.bias[n] : 0.f;
   tc::fence_proxy_async();
   tc::fence_before_sync();
   __syncthreads();
@@ -253,6 +256,14 @@ gemm_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ TcGeo
     int it = 0;
     for (int tile = t_first; tile < t_end; tile += t_step, ++it) {
       const int s = it & 1, ph = (it >> 1) & 1;
+      // SUB (one chunk a half): the row to subtract is in flight while the accumulator is waited for
+      float4 sv[FORM == TC_SUB ? CH / 4 : 1];
+      if constexpr (FORM == TC_SUB) {
+        static_assert(COLS == CH && STG, "one chunk");
+        const float4* sp = reinterpret_cast<const float4*>(g.sub + (size_t)(tile * TC_BM + row) * g.N + half * COLS);
+#pragma unroll
+        for (int j = 0; j < CH / 4; ++j) sv[j] = __ldg(sp + j);
+      }
       bool ok = tc::mbar_wait(&accfull[s], ph);
       if (STG) {
         // the named barriers below need all 128 threads of the half: make the exit uniform
@@ -296,12 +307,11 @@ gemm_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ TcGeo
             float vals[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) vals[j] = FORM == TC_RMS ? fmaf(__uint_as_float(r[j]), rinv, bs[j]) : __uint_as_float(r[j]) + bs[j];
-            if (FORM == TC_SUB && g.sub != nullptr) {
-              const float4* sp = reinterpret_cast<const float4*>(g.sub + (size_t)m * g.N + c0);
+            if (FORM == TC_SUB) {
 #pragma unroll
               for (int j = 0; j < 32; j += 4) {
-                const float4 sv = __ldg(sp + (j >> 2));
-                vals[j] -= sv.x; vals[j + 1] -= sv.y; vals[j + 2] -= sv.z; vals[j + 3] -= sv.w;
+                const float4 u = sv[j >> 2];
+                vals[j] -= u.x; vals[j + 1] -= u.y; vals[j + 2] -= u.z; vals[j + 3] -= u.w;
               }
             }
 #pragma unroll
@@ -449,7 +459,7 @@ static int launch_tc_v(const GemmArgs& g, const CUtensorMap& omap, cudaStream_t 
   // smaller planes, gain more by the early start.  Channels-last input: the second projection of the same rows.
   const PdlOff alone(N == 64 && num_tiles > 8 * sms && (!A_PLANAR || g.HW >= 4096));
   const TcGeom dv(g);
-  launch_k(gemm_tc_kernel<N, A_PLANAR, GATE, STG, FORM>, grid, TC_THREADS, smem, st, g, dv, num_tiles, amap, gmap, omap);
+  launch_k(gemm_tc_kernel<N, A_PLANAR, GATE, STG, FORM>, grid, tc_threads<N, A_PLANAR, FORM>, smem, st, g, dv, num_tiles, amap, gmap, omap);
   return check_launch();
 }
 
