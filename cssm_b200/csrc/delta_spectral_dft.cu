@@ -278,7 +278,7 @@ static size_t delta_dft_bytes(const DpGeom& g, int P, int arg) {
 static bool delta_dft_plan(int B, int T, int C, int H, int W, int dk, bool need_smem_state, DeltaDftArgs* d, DpChoice* ch) {
   memset(d, 0, sizeof(*d));
   for (int st = 1; st >= (need_smem_state ? 1 : 0); --st) {
-    *ch = dp_choose(H, W, 3 * C, B, 3 * dk, 3, 226 * 1024, delta_dft_bytes, 2 * dk + st);
+    *ch = dp_choose(H, W, 3 * C, B, 3 * dk, 3, DP_SMEM_LIMIT, delta_dft_bytes, 2 * dk + st);
     if (ch->P == 0) continue;
     d->smem_state = st;
     d->B = B; d->T = T; d->C = C;

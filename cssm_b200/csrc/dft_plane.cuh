@@ -125,6 +125,7 @@ inline size_t dp_region_bytes(const DpGeom& g, int P) {
 }
 // Both tables and four pairs more: a tile of eight cells may read that far past the last row (cells it throws away).
 __host__ __device__ inline int dp_table_pairs(const DpGeom& g) { return g.Wp * g.ldw + g.Hp * g.ldh + 4; }
+constexpr size_t DP_SMEM_LIMIT = 226 * 1024 + 32;        // (the four pairs refuse no plane that fitted without them)
 inline size_t dp_table_bytes(const DpGeom& g) { return (size_t)dp_table_pairs(g) * 8; }
 
 // P planes from global memory (consecutive, HW apart) -> folded row operand [pixel pair][row pair].

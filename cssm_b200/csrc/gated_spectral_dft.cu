@@ -168,7 +168,7 @@ static size_t gated_dft_bytes(const DpGeom& g, int P, int T) {
   return dp_table_bytes(g) + 2 * dp_region_bytes(g, P) + (T > 1 ? (size_t)g.Hp * dp_ld_cols(g, P) * 16 : 0);
 }
 
-bool gated_spectral_dft_fits(int H, int W, int T) { return gated_dft_bytes(dp_geom(H, W), 1, T) <= 226 * 1024; }
+bool gated_spectral_dft_fits(int H, int W, int T) { return gated_dft_bytes(dp_geom(H, W), 1, T) <= DP_SMEM_LIMIT; }
 
 template <bool EQUAL>
 static auto pick_kernel(const DpChoice& ch) {
@@ -180,7 +180,7 @@ static auto pick_kernel(const DpChoice& ch) {
 
 int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat, const float* gates, float* xz,
                               int last_only, int mode, cudaStream_t st, const float* dchan, int equal_steps) {
-  const DpChoice ch = dp_choose(H, W, C, B, 1, 1, 226 * 1024, gated_dft_bytes, T);
+  const DpChoice ch = dp_choose(H, W, C, B, 1, 1, DP_SMEM_LIMIT, gated_dft_bytes, T);
   if (ch.P == 0 || (equal_steps > 0 && mode != 0)) return CSSM_ERR_UNSUPPORTED;
   GatedDftArgs a;
   memset(&a, 0, sizeof(a));
