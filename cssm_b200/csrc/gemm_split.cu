@@ -489,12 +489,11 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
           else if (krem > 16) issue(Int<2>());
           else issue(Int<1>());
           tc::commit(&empty[s]);
+          if (kb + 1 == kblocks) tc::commit(&accfull[ac]);
         }
         __syncwarp();
         if (++s == NS) { s = 0; sph ^= 1; }
       }
-      if (ok && tc::elect_one()) tc::commit(&accfull[ac]);
-      __syncwarp();
       if (++ac == bufs) { ac = 0; aph ^= 1; }
     }
     // nothing of this warp's tensor work may be in flight when TMEM is freed
