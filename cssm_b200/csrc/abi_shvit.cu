@@ -3,6 +3,7 @@
 #include <string.h>
 #include <new>
 #include "kernels.cuh"
+#include "gemm_bf16_room.h"
 
 namespace cssm {
 
@@ -25,15 +26,15 @@ static cssm_gated_desc mixer_desc(const cssm_shvit_block_desc& d) {
 // RoPE, 14x14 or 7x7 planes.  Everything else runs the float32 block.
 static bool mixer_fast(const cssm_shvit_block_desc& d) {
   return d.is_cssm && d.short_conv_spatial_size == 0 && d.rope_mode == CSSM_ROPE_NONE &&
-         spectral_cl_supported(d.H, d.W, d.C, d.num_timesteps) && gemm_bf16_pick_bn(2 * d.C) != 0 &&
-         gemm_bf16_pick_bn(d.C) != 0 && d.C % 64 == 0;
+         spectral_cl_supported(d.H, d.W, d.C, d.num_timesteps) && gb_columns(2 * d.C) != 0 &&
+         gb_columns(d.C) != 0 && d.C % 64 == 0;
 }
 
 static int block_validate(const cssm_shvit_block_desc* d) {
   if (!d) return CSSM_ERR_NULL;
   if (d->B <= 0 || d->H <= 0 || d->W <= 0 || d->C <= 0 || d->hidden <= 0) return CSSM_ERR_DIMS;
   if (d->C % 8 != 0 || d->hidden % 8 != 0) return CSSM_ERR_UNSUPPORTED;
-  if (gemm_bf16_pick_bn(d->C) == 0 || gemm_bf16_pick_bn(d->hidden) == 0) return CSSM_ERR_UNSUPPORTED;
+  if (gb_columns(d->C) == 0 || gb_columns(d->hidden) == 0) return CSSM_ERR_UNSUPPORTED;
   if (d->is_cssm) {
     if (d->num_timesteps <= 0) return CSSM_ERR_DIMS;
     if (!mixer_fast(*d)) {

@@ -34,6 +34,7 @@
 #include "kernels.cuh"
 #include "tc05.cuh"
 #include "bf16_ops.cuh"
+#include "gemm_bf16_room.h"
 
 namespace cssm {
 
@@ -42,9 +43,6 @@ __device__ int g_bf16_error = 0;
 // Epilogue warps: sixteen; eight beside the gathering warps of the im2col form, which need the registers.
 template <bool IM2COL> constexpr int gb_epi_warps = IM2COL ? 8 : 16;
 template <bool IM2COL> constexpr int gb_threads = (2 + gb_epi_warps<IM2COL> + (IM2COL ? 4 : 0)) * 32;
-constexpr int GB_BM = 128, GB_BK = 64, GB_MAX_STAGES = 8;
-constexpr uint32_t GB_BAR_BYTES = 320;                   // barriers and the TMEM slot
-constexpr uint32_t GB_A_BYTES = GB_BM * 128u;            // one A stage: 128 rows x 128 bytes
 
 __device__ __forceinline__ uint32_t make_idesc_bf16(uint32_t M, uint32_t N) {
   uint32_t d = 0;
@@ -601,17 +599,6 @@ int read_bf16_error(int* out, int clear) {
   return CSSM_OK;
 }
 
-// Tile width: 256, 192, 128 or 64 columns with the TMA-store epilogue;
-// other multiples of 32 up to 256 as one tile with direct stores.
-int gemm_bf16_pick_bn(int N) {
-  if (N % 256 == 0) return 256;
-  if (N % 192 == 0) return 192;
-  if (N % 128 == 0) return 128;
-  if (N % 64 == 0) return 64;
-  if (N <= 256 && N % 32 == 0) return N;
-  return 0;
-}
-
 // (rows x cols) bf16 output with row stride ld -> boxes of 64 columns x 128 rows for the TMA stores
 static bool make_out_map(CUtensorMap* map, void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows = 128) {
   const tc::EncodeTiledFn enc = tc::encode_fn();
@@ -651,10 +638,7 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
     g.conv_tma = wide ? 2 : 1;
   const int Kw = conv ? conv3x3s2_packed_k(g.Cin, g.Wi, g.N) : g.K;      // K as the packed weights lay it out
   g.Kpad = (Kw + GB_BK - 1) / GB_BK * GB_BK;
-  g.BN = gemm_bf16_pick_bn(g.N);
-  // a residual with a short K loop gains more from the TMA residual prefetch (three staging slots,
-  // BN <= 128) than it loses in operand traffic: 37 against 47 us for M = 100 K, K = 256, N = 256
-  if (g.BN == 256 && g.res != nullptr && g.K < 512) g.BN = 128;
+  g.BN = gb_columns(g.N, g.K, g.res != nullptr);
   if (g.BN == 0 || g.ldw < g.Kpad || (g.ldw % 8) != 0) return CSSM_ERR_UNSUPPORTED;
   if (g.ldo % 8 != 0 || (g.res != nullptr && g.ldr % 8 != 0)) return CSSM_ERR_UNSUPPORTED;
   if (!aligned16(g.A) || !aligned16(g.Wt) || (g.out && !aligned16(g.out)) ||
@@ -677,13 +661,6 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
   bool tma_out = g.BN % 64 == 0;
   int m_tiles = (g.M + GB_BM - 1) / GB_BM;
   const int sms = sm_count();
-  // Few row tiles: narrower column tiles while every tile still gets an SM of its own, so that a CTA has
-  // less of an epilogue and fewer weights to wait for.  One 224-pixel image: the 23 launches 258 -> 199 us,
-  // the pass 405 -> 351 us; 33 images of 256 pixels 866 -> 842 us.
-  auto narrow = [&]() {
-    for (int bn = 128; bn >= 64; bn /= 2)
-      if (g.BN > bn && g.N % bn == 0 && (long long)m_tiles * (g.N / bn) <= sms) g.BN = bn;
-  };
   if (g.conv_tma) {
     // M tile = Bbox images x Hbox output rows x Wbox output columns, at most 128 pixels
     g.Bimg = g.M / (g.Ho * g.Wo);
@@ -696,7 +673,7 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
     if (g.Bbox > g.Bimg) g.Bbox = g.Bimg;
     if (g.Bbox < 1) g.Bbox = 1;
     m_tiles = g.tiles_w * g.tiles_h * ((g.Bimg + g.Bbox - 1) / g.Bbox);
-    narrow();
+    g.BN = gb_narrow(g.BN, g.N, m_tiles, sms);
     const uint64_t C = (uint64_t)g.Cin;
     bool ok;
     if (g.conv_tma == 2) {
@@ -724,7 +701,7 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
     ok = ok && make_map_4d(&omap, g.out, odims, ost, obox, oes);
     if (!ok) return CSSM_ERR_CUDA;
   } else {
-    narrow();
+    g.BN = gb_narrow(g.BN, g.N, m_tiles, sms);
     // A: out-of-range k columns (K < Kpad) and rows (M not a multiple of 128) arrive as zeros
     if (!im2col && !make_kmajor_map(&amap, g.A, (uint64_t)g.M, (uint64_t)g.K, (uint64_t)g.lda, GB_BM))
       return CSSM_ERR_CUDA;
@@ -739,29 +716,15 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
   cudaError_t e;
   const int tiles = m_tiles * (g.N / g.BN);
   const int grid = tiles < sms ? tiles : sms;
-  // Weights of at most 64 KB that form a single N tile stay resident in shared memory (a weight tile
-  // re-read from L2 for every M tile costs as much operand traffic as the A tile itself).
-  const size_t wres_bytes = (size_t)g.Kpad * g.BN * 2;
-  g.wres = (!im2col && g.N == g.BN && wres_bytes <= 64 * 1024) ? 1 : 0;
-  const size_t stage = GB_A_BYTES + (g.wres ? 0 : (size_t)g.BN * 128u);
-  g.bias_n = g.bias != nullptr && g.N <= 2048 ? g.N : 0;
-  const size_t budget = 227 * 1024 - (g.wres ? wres_bytes : 0), fixed = GB_BAR_BYTES + 1024 + (size_t)g.bias_n * 4;
-  // Residual by TMA (plain GEMMs with tiles of at most 128 columns): four accumulators and three or
-  // four staging slots per epilogue half.  Everything else: two accumulators, two slots, residual
-  // rows (if any) by plain loads -- the configuration that measured best without a residual.
   const bool rtma = tma_out && g.res != nullptr && !conv && g.BN <= 128;
+  const Bf16Room room = gb_room(g.N, g.BN, g.Kpad, im2col, tma_out, rtma, g.bias != nullptr, aligned16(g.bias));
+  if (room.bytes == 0) return CSSM_ERR_UNSUPPORTED;
+  if (g.bias != nullptr && room.bias_n == 0 && !aligned16(g.bias)) return CSSM_ERR_ALIGN;
+  g.wres = room.wres; g.stages = room.stages; g.ostg = room.ostg; g.bias_n = room.bias_n;
+  // Residual by TMA (plain GEMMs with tiles of at most 128 columns): four accumulators.  Everything else: two, residual rows (if any)
+  // by plain loads -- the configuration that measured best without a residual.
   g.nacc = rtma ? 4 : 2;
-  g.stages = rtma ? 4 : GB_MAX_STAGES;                     // (with residuals by TMA the room goes to the staging slots)
-  g.ostg = 0;
-  if (tma_out) {
-    while (g.stages > 2 && g.stages * stage + 4 * 16384 + fixed > budget) --g.stages;      // (ROWS: sixteen slots of 4 KB)
-    g.ostg = rtma ? (int)((budget - fixed - g.stages * stage) / (2 * 16384)) : 2;
-    if (g.ostg > 4) g.ostg = 4;
-    if (g.ostg < (rtma ? 3 : 2)) return CSSM_ERR_UNSUPPORTED;
-  } else {
-    while (g.stages > 2 && g.stages * stage + fixed > budget) --g.stages;
-  }
-  const size_t smem = (g.wres ? wres_bytes : 0) + g.stages * stage + (size_t)g.ostg * 2 * 16384 + fixed;
+  const size_t smem = room.bytes;
   auto kern = im2col ? (tma_out ? gemm_bf16_kernel<true, true, false> : gemm_bf16_kernel<true, false, false>)
                      : (tma_out ? (rtma ? gemm_bf16_kernel<false, true, true> : conv ? gemm_bf16_kernel<false, true, false> : gemm_bf16_kernel<false, true, false, true>)
                                 : gemm_bf16_kernel<false, false, false>);

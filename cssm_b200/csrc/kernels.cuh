@@ -163,7 +163,6 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st);
 // [column 2 | zeros], so that every K block is one 128-byte pair of adjacent input pixels.
 int conv3x3s2_weight_layout(int Cin, int Wi, int Cout);
 int conv3x3s2_packed_k(int Cin, int Wi, int Cout);
-int gemm_bf16_pick_bn(int N);
 int read_bf16_error(int* out, int clear);
 // few rows (csrc/gemm_small.cu); ln_scale, ln_bias: LayerNorm over K of the rows of A, or nullptr
 bool gemm_small_supported(const Bf16GemmArgs& g);
