@@ -15,6 +15,14 @@ __device__ __forceinline__ uint32_t float2_to_bf16x2(float lo, float hi) {
 }
 __device__ __forceinline__ float bf16_to_float(__nv_bfloat16 v) { return __bfloat162float(v); }
 
+// x -> three bf16 parts for a pair of values, packed (low half = first value)
+__device__ __forceinline__ void split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p0) : "f"(y), "f"(x));
+  const cf r = mk(x, y) - mk(__uint_as_float(p0 << 16), __uint_as_float(p0 & 0xffff0000u));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1) : "f"(r.y), "f"(r.x));
+  const cf u = r - mk(__uint_as_float(p1 << 16), __uint_as_float(p1 & 0xffff0000u));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p2) : "f"(u.y), "f"(u.x));
+}
 // 8 consecutive bf16 (16 bytes) <-> 8 floats
 __device__ __forceinline__ void unpack8(const uint4 u, float (&f)[8]) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};

@@ -41,7 +41,7 @@ struct GemmArgs {
   const float* sub;         // channels-last output only: (M, N) tensor subtracted from the result, or nullptr
 };
 
-// Two tf32 parts, K = 64 only; three bf16 parts, any size.
+// Two tf32 parts (three bf16 ones under the RMS prologue), K = 64 only; three bf16 parts, any size.
 bool gemm_tc_supported(const GemmArgs& g, bool a_planar);
 // whether gemm_tc takes a channels-last (M, K) by (K, N) projection of frames of HW pixels that multiplies planes in place (mul)
 bool gemm_tc_in_place(int K, int N, int HW, int mul_n);

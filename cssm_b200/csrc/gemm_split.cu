@@ -80,14 +80,6 @@ struct SplitGeom {
 // block 16 x 8 x 56 x 56 x 32 took 398 instead of 393 us.
 struct SplitArgs { GemmArgs g; SplitGeom q; };
 
-// x -> three bf16 parts for a pair of values, packed (low half = first value)
-__device__ __forceinline__ void split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p0) : "f"(y), "f"(x));
-  const cf r = mk(x, y) - mk(__uint_as_float(p0 << 16), __uint_as_float(p0 & 0xffff0000u));
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1) : "f"(r.y), "f"(r.x));
-  const cf u = r - mk(__uint_as_float(p1 << 16), __uint_as_float(p1 & 0xffff0000u));
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p2) : "f"(u.y), "f"(u.x));
-}
 // eight consecutive k values -> one 16-byte chunk in each of the three parts
 __device__ __forceinline__ void store_split8(unsigned char* base, uint32_t off, uint32_t part, const float (&v)[8]) {
   uint4 a, b, c;
@@ -98,9 +90,6 @@ __device__ __forceinline__ void store_split8(unsigned char* base, uint32_t off, 
   *reinterpret_cast<uint4*>(base + off) = a;
   *reinterpret_cast<uint4*>(base + part + off) = b;
   *reinterpret_cast<uint4*>(base + 2 * part + off) = c;
-}
-__device__ __forceinline__ uint32_t idesc_bf16_f32(uint32_t M, uint32_t N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                         uint32_t accumulate) {
@@ -447,7 +436,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
   } else if (warp == GS_MMA_WARP) {
     // ================================ MMA issuer ================================
     // The whole warp walks the loop, one lane issues (elect_one).
-    const uint32_t idesc = idesc_bf16_f32(GS_BM, BN);
+    const uint32_t idesc = tc::make_idesc_bf16(GS_BM, BN);
     // (A part, B part) of the six partial products, smallest first
     constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
     int s = 0, sph = 0, ac = 0, aph = 1;

@@ -1,5 +1,5 @@
 // tcgen05 / TMEM GEMM for the K = 64 channel projections in fp32-equivalent precision
-// (3 x TF32: A_lo*B_hi + A_hi*B_lo + A_hi*B_hi, accumulated in fp32 in TMEM).
+// (3 x TF32: A_lo*B_hi + A_hi*B_lo + A_hi*B_hi, accumulated in fp32 in TMEM; with the RMS prologue six products of three bf16 parts).
 //
 // Persistent kernel, one CTA per SM, 26 warps (18 where a second tensor is subtracted):
 //   loader, 1 warp       : TMA copies of 128-pixel A tiles as they lie in memory (channels-last rows, or planar planes and
@@ -7,7 +7,7 @@
 //   converters, 16 or 8  : lane = pixel, 16 of the 64 channels at a time: read the raw tile, apply RoPE or the gate, split every
 //                          value into tf32 hi + remainder and write both to TMEM (tcgen05.st), where the MMAs read their A operand;
 //                          a stage is half of the channels;
-//   MMA issuer, 1 warp   : 24 tcgen05.mma (M128 x N x K8, A in TMEM, B in shared memory) per tile into one of two TMEM
+//   MMA issuer, 1 warp   : 24 tcgen05.mma (M128 x N x K8, bf16 K16; A in TMEM, B in shared memory) per tile into one of two TMEM
 //                          accumulators, commits to mbarriers;
 //   epilogue, 8 or 16    : tcgen05.ld the accumulator (lane = pixel; two or four warps per TMEM lane
 //                          quadrant, a share of the columns each), add bias / activation, store
@@ -35,6 +35,9 @@ __device__ int g_tc_error = 0;
 // last frame of every clip (last-frame-only forward); MUL: the first g.mul_n output columns multiply planes in place; SUB: the
 // channels-last tensor g.sub is subtracted from the rows.  Compile-time variants, so that the plain one carries no extra test.
 // RMS (planar A, 64 columns): a <- a * rsqrt(mean_k a^2 + eps) * scale[k]; the scale goes into the weights, the row factor to the accumulator.
+// Its operands are three bf16 parts, all 24 bits of a float32, as gemm_split_kernel has them (two tf32 parts hold 22): error of the launch
+// against float64 1.1e-7 of the 2-norm, 2.0e-7 with two tf32 parts, at the same time (4.2 M rows 507 us, 1 M 135); gemm_split_kernel 1.2e-7,
+// 701.
 enum TcForm { TC_PLAIN, TC_ZLAST, TC_MUL, TC_SUB, TC_RMS };
 // Warps: converters, MMA issuer, loader, epilogue.  A wide planar output has more to store than to convert (with sixteen converters and
 // eight epilogue warps: 4.2 M rows to 128 columns 491 us, 429 so; DeltaNet 32x32, whose 192 columns multiply planes, 462 and 415 a pass).
@@ -120,7 +123,8 @@ gemm_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ TcGeo
     tc::tmem_alloc(tmem_slot, 512);
     tc::tmem_relinquish();
   }
-  tc_split_weights<N, FORM == TC_RMS>(g.Wk, g.N, 0, smem + L::B_OFF, smem + L::B_OFF + L::B_HALF, tid, THREADS, g.rms_scale);
+  if constexpr (FORM == TC_RMS) tc_split3_weights<N>(g.Wk, g.rms_scale, smem + L::B_OFF, tid, THREADS);
+  else tc_split_weights<N>(g.Wk, g.N, 0, smem + L::B_OFF, smem + L::B_OFF + L::B_HALF, tid, THREADS);
   if (rope_s) tc_rope_columns(g, smem + L::WANG_OFF, tid, THREADS);
   for (int n = tid; n < N; n += THREADS) bias_s[n] = g.bias ? g.bias[n] : 0.f;
   tc::fence_proxy_async();
@@ -178,7 +182,8 @@ gemm_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ TcGeo
           // (the epilogue of the tile four back is through: the MMAs of the one two back, which this stage waited for, began after it)
           if (FORM == TC_RMS) reinterpret_cast<float*>(smem + L::SS_OFF)[((it & 3) * 4 + grp) * 128 + row] = ss;
         }
-        tc_split_store16(tdst + (uint32_t)(it % NT) * 128u + sl * 16u, v);
+        if constexpr (FORM == TC_RMS) tc_split3_store16(tdst + (uint32_t)(it % NT) * 128u + sl * 8u, v);
+        else tc_split_store16(tdst + (uint32_t)(it % NT) * 128u + sl * 16u, v);
       }
       if (!ok) break;
       tc::wait_st();
@@ -214,7 +219,7 @@ gemm_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ TcGeo
   } else if (warp == MMA_WARP) {
     // ================================ MMA issuer ================================
     // The whole warp walks the loop, one lane issues (elect_one).
-    const uint32_t idesc = tc::make_idesc_tf32(TC_BM, N);
+    const uint32_t idesc = FORM == TC_RMS ? tc::make_idesc_bf16(TC_BM, N) : tc::make_idesc_tf32(TC_BM, N);
     const uint64_t b_hi = tc::make_desc_sw128(sbase + L::B_OFF), b_lo = tc::make_desc_sw128(sbase + L::B_OFF + L::B_HALF);
     int it = 0;
     bool ok = true;
@@ -228,14 +233,19 @@ gemm_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ TcGeo
       for (int hf = 0; hf < 2; ++hf) {
         if (!(ok = wait(&full[s + hf], (it / NT) & 1, 2))) break;
         tc::fence_after_sync();
-        if (tc::elect_one()) tc_mma_small<N>(d, a + hf * 64u, b_hi, b_lo, hf, idesc);
+        if (tc::elect_one()) {
+          if constexpr (FORM == TC_RMS) tc_mma3_small<N>(d, a + hf * 64u, b_hi, hf, idesc);
+          else tc_mma_small<N>(d, a + hf * 64u, b_hi, b_lo, hf, idesc);
+        }
         __syncwarp();
       }
       if (ok && tc::elect_one()) {
-        tc_mma_lead<N>(d, a, b_hi, 0, idesc);
-        tc::commit(&empty[s]);
-        tc_mma_lead<N>(d, a + 64u, b_hi, 1, idesc);
-        tc::commit(&empty[s + 1]);
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          if constexpr (FORM == TC_RMS) tc_mma3<N>(d, a + hf * 64u, b_hi, 0, 0, hf, idesc, false);
+          else tc_mma_lead<N>(d, a + hf * 64u, b_hi, hf, idesc);
+          tc::commit(&empty[s + hf]);
+        }
         tc::commit(&accfull[ac]);
       }
       __syncwarp();

@@ -4,6 +4,7 @@
 #include <cuda.h>
 #include "gemm.cuh"
 #include "tc05.cuh"
+#include "bf16_ops.cuh"
 
 namespace cssm {
 
@@ -144,18 +145,56 @@ __device__ __forceinline__ void tc_mma_lead(uint32_t d, uint32_t a, uint64_t b_h
 #pragma unroll
   for (int ks = 0; ks < 4; ++ks) tc::mma_tf32_ts(d, a + ks * 8u, b_hi + (uint64_t)(hf * (N * 128u >> 4)) + ks * 2, idesc, 1u);
 }
-// Weights W[k][n0 + n] of a (64, ldn) matrix (times scale[k]) -> B_hi / B_lo rows n, K-major swizzled
-template <int N, bool SCALE = false>
-__device__ __forceinline__ void tc_split_weights(const float* Wk, int ldn, int n0, unsigned char* b_hi, unsigned char* b_lo, int tid, int threads,
-                                                 const float* scale = nullptr) {
+// Weights W[k][n0 + n] of a (64, ldn) matrix -> B_hi / B_lo rows n, K-major swizzled
+template <int N>
+__device__ __forceinline__ void tc_split_weights(const float* Wk, int ldn, int n0, unsigned char* b_hi, unsigned char* b_lo, int tid, int threads) {
   for (int item = tid; item < N * 16; item += threads) {
     const int n = item % N, c = item / N;               // c: 16-byte chunk of 4 k values
     float hi[4], lo[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) tc::split_tf32(Wk[(size_t)(4 * c + e) * ldn + n0 + n] * (SCALE ? scale[4 * c + e] : 1.f), hi[e], lo[e]);
+    for (int e = 0; e < 4; ++e) tc::split_tf32(Wk[(size_t)(4 * c + e) * ldn + n0 + n], hi[e], lo[e]);
     const uint32_t off = (uint32_t)(c >> 3) * (N * 128u) + tc::sw128_offset(n, c & 7);
     *reinterpret_cast<float4*>(b_hi + off) = make_float4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<float4*>(b_lo + off) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+  }
+}
+
+// The same for three bf16 parts (split3: 24 bits, where two tf32 parts hold 22) and their six products down to 2^-16 of the leading
+// one: sixteen channels are eight columns of a part, the parts of a stage sixteen columns apart.
+__device__ __forceinline__ void tc_split3_store16(uint32_t taddr, const float (&v)[16]) {
+  uint32_t p[3][8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) split3(v[2 * j], v[2 * j + 1], p[0][j], p[1][j], p[2][j]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) tc::st_32x32b_x8(taddr + 16u * i, p[i]);
+}
+// b: the first part of B; the others follow N rows on each
+template <int N>
+__device__ __forceinline__ void tc_mma3(uint32_t d, uint32_t a, uint64_t b, int pa, int pb, int hf, uint32_t idesc, bool first) {
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks)
+    tc::mma_bf16_ts(d, a + pa * 16u + ks * 8u, b + (uint64_t)(pb * (N * 128 >> 4) + (hf * 2 + ks) * 2), idesc, first && ks == 0 ? 0u : 1u);
+}
+template <int N>
+__device__ __forceinline__ void tc_mma3_small(uint32_t d, uint32_t a, uint64_t b, int hf, uint32_t idesc) {
+  constexpr int PA[5] = {2, 0, 1, 1, 0}, PB[5] = {0, 2, 1, 0, 1};
+#pragma unroll
+  for (int p = 0; p < 5; ++p) tc_mma3<N>(d, a, b, PA[p], PB[p], hf, idesc, (hf | p) == 0);
+}
+// Weights W[k][n] of a (64, N) matrix times scale[k] -> three parts of N rows, K-major swizzled
+template <int N>
+__device__ __forceinline__ void tc_split3_weights(const float* Wk, const float* scale, unsigned char* b, int tid, int threads) {
+  for (int item = tid; item < N * 8; item += threads) {
+    const int n = item % N, c = item / N;               // c: 16-byte chunk of 8 k values
+    uint32_t p[3][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int k = 8 * c + 2 * e;
+      split3(Wk[(size_t)k * N + n] * scale[k], Wk[(size_t)(k + 1) * N + n] * scale[k + 1], p[0][e], p[1][e], p[2][e]);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      *reinterpret_cast<uint4*>(b + (uint32_t)i * (N * 128u) + tc::sw128_offset(n, c)) = make_uint4(p[i][0], p[i][1], p[i][2], p[i][3]);
   }
 }
 

@@ -160,6 +160,15 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, ui
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// bf16 x bf16 -> fp32 with A in TMEM (lane = row, a 32-bit column two elements of K, the first in its low half).
+__device__ __forceinline__ void mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
 // 32 lanes x 8 consecutive 32-bit columns: thread i of the warp writes lane (base_lane + i).
 __device__ __forceinline__ void st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8]) {
   asm volatile(
@@ -244,6 +253,11 @@ __device__ __forceinline__ uint32_t make_idesc_tf32(uint32_t M, uint32_t N) {
   d |= (N >> 3) << 17;     // N / 8
   d |= (M >> 4) << 24;     // M / 16
   return d;
+}
+
+// kind::f16 with bf16 operands, f32 accumulate
+__device__ __forceinline__ uint32_t make_idesc_bf16(uint32_t M, uint32_t N) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
 // round-to-nearest tf32 part and the exact remainder: x = hi + lo
