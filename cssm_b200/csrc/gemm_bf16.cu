@@ -717,7 +717,8 @@ int launch_gemm_bf16(Bf16GemmArgs g, cudaStream_t st) {
   const int tiles = m_tiles * (g.N / g.BN);
   const int grid = tiles < sms ? tiles : sms;
   const bool rtma = tma_out && g.res != nullptr && !conv && g.BN <= 128;
-  const Bf16Room room = gb_room(g.N, g.BN, g.Kpad, im2col, tma_out, rtma, g.bias != nullptr, aligned16(g.bias));
+  const Bf16Room room = gb_room({g.N, g.BN, g.Kpad, tiles / grid, im2col, tma_out, g.res != nullptr, rtma, g.act != 0, g.bias != nullptr,
+                                 aligned16(g.bias)});
   if (room.bytes == 0) return CSSM_ERR_UNSUPPORTED;
   if (g.bias != nullptr && room.bias_n == 0 && !aligned16(g.bias)) return CSSM_ERR_ALIGN;
   g.wres = room.wres; g.stages = room.stages; g.ostg = room.ostg; g.bias_n = room.bias_n;

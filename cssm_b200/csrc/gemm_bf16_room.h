@@ -41,39 +41,54 @@ struct Bf16Room {
   size_t bytes;              // dynamic shared memory; 0: does not fit
 };
 
-// staged: output through staging slots and TMA stores; rtma (with staged): residual boxes by TMA into those slots.
-inline Bf16Room gb_room(int N, int BN, int Kpad, bool im2col, bool staged, bool rtma, bool bias, bool bias_aligned) {
+struct Bf16Form {
+  int N, BN, Kpad;
+  int rounds;                // tiles a CTA takes
+  bool im2col;
+  bool staged;               // output through staging slots and TMA stores
+  bool res, rtma;            // a residual; its boxes by TMA into the slots (with staged)
+  bool act;                  // GELU or SiLU
+  bool bias, bias_aligned;   // a bias; it starts on 16 bytes
+};
+
+inline Bf16Room gb_room(const Bf16Form& f) {
   Bf16Room r = {};
   // Weights of at most 64 KB that form a single N tile stay resident (a weight tile re-read from L2 for every M tile costs as
   // much operand traffic as the A tile itself).
-  const size_t weights = (size_t)Kpad * BN * 2;
-  r.wres = !im2col && N == BN && weights <= 64 * 1024 ? 1 : 0;
-  const size_t stage = GB_A_BYTES + (r.wres ? 0 : (size_t)BN * 128), held = r.wres ? weights : 0;
+  const size_t weights = (size_t)f.Kpad * f.BN * 2;
+  r.wres = !f.im2col && f.N == f.BN && weights <= 64 * 1024 ? 1 : 0;
+  const size_t stage = GB_A_BYTES + (r.wres ? 0 : (size_t)f.BN * 128), held = r.wres ? weights : 0;
   // Residual by TMA: four stages, the rest goes to three or four staging slots a half.  Everything else: as many stages as there
   // is room for beside two slots (sixteen of 4 KB where every warp has its own).
   auto fit = [&](int bias_n, int stages) {
     const size_t fixed = GB_BAR_BYTES + 1024 + (size_t)bias_n * 4, room = GB_SMEM - held;      // 1024: alignment
     r.bias_n = bias_n;
     r.stages = stages;
-    while (r.stages > 2 && r.stages * stage + (staged ? 4 * GB_BOX : 0) + fixed > room) --r.stages;
+    while (r.stages > 2 && r.stages * stage + (f.staged ? 4 * GB_BOX : 0) + fixed > room) --r.stages;
     const size_t used = r.stages * stage + fixed;
-    r.ostg = !staged ? 0 : !rtma ? 2 : used > room ? 0 : (int)((room - used) / (2 * GB_BOX));
+    r.ostg = !f.staged ? 0 : !f.rtma ? 2 : used > room ? 0 : (int)((room - used) / (2 * GB_BOX));
     if (r.ostg > 4) r.ostg = 4;
-    r.bytes = r.ostg < (rtma ? 3 : staged ? 2 : 0) ? 0 : held + used + r.ostg * 2 * GB_BOX;
+    r.bytes = r.ostg < (f.rtma ? 3 : f.staged ? 2 : 0) ? 0 : held + used + r.ostg * 2 * GB_BOX;
     if (r.bytes > GB_SMEM) r.bytes = 0;
   };
-  const int most = rtma ? 4 : GB_MAX_STAGES;
+  const int most = f.rtma ? 4 : GB_MAX_STAGES;
   fit(0, most);
-  if (!bias || N > GB_BIAS_MAX) return r;
+  if (!f.bias || f.N > GB_BIAS_MAX) return r;
+  const Bf16Room without = r;
+  fit(f.N, most);
   // The bias takes no staging slot away: four stages of 128 columns and three slots leave room for 432 values, so that a longer one
   // is read from global memory there (100000 x 64 -> 448 + residual in 64-column tiles: 51 us with the bias copied and three slots, 43
   // with four).  One that starts off 16 bytes can only be copied: a stage less then.
-  const Bf16Room without = r;
-  fit(N, most);
-  if (rtma && r.ostg < without.ostg) {
-    if (bias_aligned) return without;
-    fit(N, 3);
+  if (f.rtma && r.ostg < without.ostg) {
+    if (f.bias_aligned) return without;
+    fit(f.N, 3);
   }
+  // Nor the fourth stage of 192-column tiles (room for 432 values beside it, too), where long K loops of many tiles need it.  us a
+  // launch, bias in global memory and four stages / copied and three: 100352 rows, 576 -> 1152 142 / 162, 384 -> 576 56 / 62, 192 -> 576
+  // 42 / 42, 64 -> 576 31 / 28; 576 -> 576 + residual 95 / 90, 768 -> 576 104 / 110; 25088 rows, 384 -> 1344 GELU 40 / 38, 576 -> 1344 48 /
+  // 51, 384 -> 960 (six rounds) 28 / 27; 5000 rows 3 % to 20 % the other way at every depth.
+  const int deep = f.res ? 12 : f.act ? 9 : 6;
+  if (!f.rtma && f.bias_aligned && r.stages < 4 && without.stages >= 4 && f.rounds >= 7 && f.Kpad >= deep * GB_BK) return without;
   return r;
 }
 

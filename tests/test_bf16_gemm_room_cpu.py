@@ -1,6 +1,6 @@
 """Tiles and shared memory of the bf16 GEMM (csrc/gemm_bf16_room.h), walked over widths, depths, row tiles and forms in a small host
 program: every width that has a tile fits, a residual by TMA has its three staging slots, and a bias in shared memory takes none of
-the slots that the form has without one."""
+the slots that the form has without one, nor a long K loop's fourth stage."""
 import os
 import shutil
 import subprocess
@@ -21,8 +21,8 @@ int main() {
   for (int N = 32; N <= 4096; N += 32)
     for (int K : {32, 64, 96, 128, 192, 256, 320, 448, 512, 640, 1024, 2048, 4096})
       for (int mt : {1, 2, 9, 18, 19, 24, 37, 74, 100, 148, 149, 1000})
-        for (int form = 0; form < 16; ++form) {
-          const bool res = form & 1, bias = form & 2, aligned = !(form & 4), im2col = form & 8;
+        for (int form = 0; form < 32; ++form) {
+          const bool res = form & 1, bias = form & 2, aligned = !(form & 4), im2col = form & 8, act = form & 16;
           if (im2col && res) continue;
           const int Kpad = (K + GB_BK - 1) / GB_BK * GB_BK;
           int BN = gb_columns(N, K, res);
@@ -32,8 +32,9 @@ int main() {
           }
           BN = gb_narrow(BN, N, mt, 148);
           const bool staged = BN % 64 == 0, rtma = staged && res && BN <= 128;
-          const Bf16Room r = gb_room(N, BN, Kpad, im2col, staged, rtma, bias, aligned);
-          const Bf16Room plain = gb_room(N, BN, Kpad, im2col, staged, rtma, false, true);
+          const int rounds = (mt * (N / BN) + 147) / 148;
+          const Bf16Room r = gb_room({N, BN, Kpad, rounds, im2col, staged, res, rtma, act, bias, aligned});
+          const Bf16Room plain = gb_room({N, BN, Kpad, rounds, im2col, staged, res, rtma, act, false, true});
           ++seen;
           if (N % BN != 0) report("not whole tiles", N, K, mt, BN, r);
           if (r.bytes == 0 || r.bytes > 227 * 1024) report("refused", N, K, mt, BN, r);
@@ -41,6 +42,8 @@ int main() {
           if (staged && r.ostg < (rtma ? 3 : 2)) report("slots", N, K, mt, BN, r);
           if (aligned && r.ostg < plain.ostg) report("fewer slots", N, K, mt, BN, r);
           if (aligned && rtma && r.stages < plain.stages) report("fewer stages", N, K, mt, BN, r);
+          // long K loops of many tiles keep the fourth stage
+          if (aligned && rounds >= 7 && Kpad >= 12 * GB_BK && plain.stages >= 4 && r.stages < 4) report("fourth stage", N, K, mt, BN, r);
           if (r.bias_n != 0 && (!bias || r.bias_n != N)) report("bias", N, K, mt, BN, r);
           // what the kernel lays out: weights, ring, two halves of staging slots, barriers, bias, 1024 bytes of alignment
           const size_t need = (r.wres ? (size_t)Kpad * BN * 2 : 0) + (size_t)r.stages * (GB_A_BYTES + (r.wres ? 0 : BN * 128)) +
