@@ -69,3 +69,11 @@ def test_default_widths():
     bound.forward_host(xh, lh)
     assert np.array_equal(lh[:64].numpy(), y)
     assert device_error() == 0
+
+
+@pytest.mark.parametrize("M,K,N,act", [(60001, 64, 64, 0), (40001, 64, 192, 2), (100003, 256, 512, 1), (30011, 384, 576, 0), (25001, 576, 1344, 1),
+                                       (9001, 128, 2304, 2), (20001, 96, 160, 0), (50001, 448, 320, 1)])
+def test_several_tiles_a_cta(M, K, N, act):
+    """No residual, more tiles than SMs: accumulators, ring and slots come round; an odd number of 64-column boxes, which the two warps of a
+    quadrant take in turn; a bias from global memory; direct stores (160 columns)."""
+    _gemm(M, K, N, act, False)

@@ -34,6 +34,42 @@ def test_joined_launch(kt, T, gate, inputs, B, H, W):
     assert device_error() == 0
 
 
+@pytest.mark.parametrize("kt", [1, 2, 3])
+@pytest.mark.parametrize("T", [5, 7])
+def test_fewer_taps_above_four_steps(kt, T):
+    """Each tap count against the two launches (up to four steps the joined one takes any number of clips)."""
+    kw = dict(delta_key_dim=4, kernel_size=3, gate_type="factored", short_conv_size=kt)
+    x = torch.from_numpy(np.random.default_rng(T + kt).standard_normal((20, T, 32, 32, 64)).astype(np.float32)).cuda()
+    m = GatedDeltaNetCSSM(channels=64, rope_mode="mrope", qkv_conv_size=1, **kw).bind({"params": orc.init_gdn_params(kt, 64, 32, 32, bias_scale=0.1, **kw)})
+    got = m(x).clone()
+    few = torch.cat([m(x[i:i + 1].contiguous()).clone() for i in range(20)])
+    assert orc.rel_l2(got.cpu().numpy(), few.cpu().numpy()) <= 5e-6
+    assert device_error() == 0
+
+
+@pytest.mark.parametrize("kt,T", [(4, 1), (4, 2), (4, 3), (4, 4), (3, 4), (2, 4), (1, 3), (3, 2), (2, 1)])
+@pytest.mark.parametrize("B,H,W", [(1, 8, 16), (30, 16, 16)])
+def test_few_steps_against_float64(kt, T, B, H, W):
+    """Up to four steps: the q and k planes that the launch leaves.  Products off by 2^-22 at most and the accumulator's eight truncations
+    (3.3e-7 together, tests/test_tc_projections_gpu.py), SiLU and four taps of float32 FMAs."""
+    m = GatedDeltaNetCSSM(channels=64, delta_key_dim=4, kernel_size=3, rope_mode="none", qkv_conv_size=1, gate_type="factored",
+                          short_conv_size=kt, use_input_gates=False)
+    x = torch.randn((B, T, H, W, 64), device="cuda", generator=torch.Generator(device="cuda").manual_seed(T + kt))
+    v = m.init(3, tuple(x.shape), bias_scale=0.3)
+    b, p = m.bind(v), v["params"]
+    b(x)
+    f64 = lambda a: torch.from_numpy(np.asarray(a, np.float64)).cuda()
+    qkv = b.buf.get("ws", 0).view(torch.float32)[:3 * x.numel()].view(B, T, 192, H, W)
+    s = x.double() @ f64(p["qkv_proj"]["kernel"]) + f64(p["qkv_proj"]["bias"])
+    for i, name in enumerate("qk"):
+        c = p[f"short_conv_{name}"]
+        k = f64(c["kernel"]).reshape(kt, 64)
+        past = torch.nn.functional.pad(s[..., i * 64:(i + 1) * 64], (0, 0) * 3 + (kt - 1, 0))
+        want = torch.nn.functional.silu(sum(past[:, j:j + T] * k[j] for j in range(kt)) + f64(c["bias"])).permute(0, 1, 4, 2, 3)
+        assert float((qkv[:, :, i * 64:(i + 1) * 64].double() - want).norm() / want.norm()) < 5e-7
+    assert device_error() == 0
+
+
 @pytest.mark.parametrize("rope", ["none", "spatiotemporal"])
 @pytest.mark.parametrize("conv", [1, 3])
 def test_input_forms(rope, conv):
