@@ -30,9 +30,8 @@ __device__ __forceinline__ void dn_write(const DnGateArgs& g, size_t oi, const f
   g.cg[oi] = dn_sigmoid(r[4]) * inv;
 }
 // factored: one frame per CTA row, its bins over gridDim.y CTAs; 512 threads take the 5 (H + Wf) vector entries of
-// planes up to 64x64 in one pass.  (Entry and pointer by index: with gate_vectors' choice among ten pointers
-// the compiler issues the loads of a thread one after another, likewise with five dense gates in one call of
-// gate_dense.  28 frames of 64 x 64 x 64, factored, cold: 31 us that way, 12 so; 32 of 28 x 28 x 64, dense: 46 and 17 us.)
+// planes up to 64x64 in one pass.  (Entry and pointer by index, instead of gate_vectors' choice among ten pointers and five dense
+// gates in one call of gate_dense: 28 frames of 64 x 64 x 64, factored, cold 31 -> 12 us; 32 of 28 x 28 x 64, dense 46 -> 17.)
 constexpr int DF_THREADS = 512;
 __global__ void __launch_bounds__(DF_THREADS) deltanet_gates_factored_kernel(const DnGateArgs g) {
   extern __shared__ __align__(16) float sh[];

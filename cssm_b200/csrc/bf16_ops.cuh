@@ -78,8 +78,8 @@ __device__ __forceinline__ float tanh_approx(float u) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
   return t;
 }
-// 1 / (1 + e^-x) of a pair: e^-x as 2^(-x log2 e), two special functions a value and packed arithmetic around them (half the
-// instructions of the scalar form, whose exponential also scales denormal results; here they are zero beside the 1)
+// 1 / (1 + e^-x) of a pair: e^-x = 2^(-x log2 e), two special functions a value and packed arithmetic around them.  (A result of ex2 below
+// the smallest normal number may be zero: beside the 1 it is.)
 __device__ __forceinline__ unsigned long long sigmoid_x2(unsigned long long x) {
   float a, b, c, d;
   upk2(mul2(x, pk2(-1.4426950408889634f, -1.4426950408889634f)), a, b);

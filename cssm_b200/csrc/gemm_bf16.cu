@@ -223,7 +223,7 @@ gemm_bf16_kernel(const Bf16GemmArgs g, const __grid_constant__ CUtensorMap amap,
     __syncwarp();
   } else if (warp < 2 + EW) {
     // ================================ epilogue ================================
-    // Two halves of four warps (one per TMEM lane quadrant).  Half h owns the tiles of its CTA with
+    // Two halves of eight warps, two per TMEM lane quadrant (im2col: of four).  Half h owns the tiles of its CTA with
     // tile count parity h; accumulator = tile count mod NACC, so a half drains one accumulator while
     // the MMA warp fills its other one.
     const int q = warp & 3;                       // TMEM lane quadrant this warp may read

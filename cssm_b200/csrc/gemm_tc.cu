@@ -99,11 +99,11 @@ gemm_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ TcGeo
   float* bias_s = reinterpret_cast<float*>(smem + L::BIAS_OFF);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   uint64_t* raw_full = bars;           // [4] raw tile landed
-  uint64_t* raw_empty = bars + 4;      // [4] and read (16 converter warps)
-  uint64_t* full = bars + 8;           // [4] A stage written (8 converter warps)
+  uint64_t* raw_empty = bars + 4;      // [4] and read (all converter warps)
+  uint64_t* full = bars + 8;           // [4] A stage written (half of the converter warps)
   uint64_t* empty = bars + 12;         // [4] A stage consumed (tcgen05.commit)
   uint64_t* accfull = bars + 16;       // [2] accumulator complete (tcgen05.commit)
-  uint64_t* accempty = bars + 18;      // [2] accumulator drained (8 epilogue warps)
+  uint64_t* accempty = bars + 18;      // [2] accumulator drained (all epilogue warps)
   uint64_t* done = bars + 20;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
   __shared__ int s_bad;                // a bounded wait expired

@@ -110,12 +110,6 @@ __device__ __forceinline__ void tma_store_2d(const void* map, const void* smem_s
                ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
                : "memory");
 }
-__device__ __forceinline__ void tma_store_3d(const void* map, const void* smem_src, int c0, int c1,
-                                             int c2) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1),
-                 "r"(c2) : "memory");
-}
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -142,16 +136,7 @@ __device__ __forceinline__ void fence_after_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem], kind::tf32, one CTA.
-__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
-                                         uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// The same with A in TMEM (lane = row, a 32-bit column an element of K).
+// D[tmem] (+)= A[tmem] * B[smem], kind::tf32, one CTA; A: lane = row, a 32-bit column an element of K.
 __device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {
   asm volatile(
@@ -218,10 +203,9 @@ __device__ __forceinline__ void wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// True in one lane of the (converged) warp.  The way into every issue of tcgen05.mma: behind `lane == 0`, or predicated on a lane, the
-// compiler moves each operand into uniform registers again before every instruction, and a warp that shares its scheduler with busy ones
-// gets to issue an MMA every few hundred clocks; behind elect.sync it knows that one thread runs and keeps them there.  M128 N64 K8,
-// clocks an MMA, alone / beside six warps of FMAs: lane == 0 50 / 819, predicated 72 / 998, this 50 / 67.
+// True in one lane of the (converged) warp.  The way into every issue of tcgen05.mma: behind `lane == 0`, or predicated on a lane, a warp that
+// shares its scheduler with busy ones gets to issue an MMA every few hundred clocks only.  M128 N64 K8, clocks an MMA, alone / beside six
+// warps of FMAs: lane == 0 50 / 819, predicated 72 / 998, this 50 / 67.
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
