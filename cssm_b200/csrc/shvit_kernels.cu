@@ -495,13 +495,14 @@ dwconv_cl_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ 
 // many pairs of conversions for 686 FMAs, a column of 8 rows 98 for 392 (FMA pipe 41 -> 53 % busy; three CTAs an SM at 168 registers):
 // 512 x 56 x 56 x 64 362 -> 317 us, 33 x 64 x 64 x 64 45 -> 41 with 4 x 4, 512 x 28 x 28 x 128 190 -> 184; 4 x 7 blocks spill (329).
 // 3 x 3 is bound by memory: bigger blocks only lost warps (512 x 14 x 14 x 1024 111 -> 117), but for the float32 patch of
-// 14 x 14 planes (48 x 256 channels 16.4 -> 12.3).
+// 14 x 14 planes (48 x 256 channels 16.4 -> 12.3).  Its launch bounds name no number of CTAs: one cost up to ten registers a thread, and rows
+// past the plane are passed over, not left by (24 x 13 x 13 x 1024 12.3 -> 10.3, float32 outputs 10 x 69 x 69 x 64 10.1 -> 8.6).
 // Tile geometry as template parameters: CG column groups (32 * CG threads), NC columns per group, TH rows;
 // the launcher picks one that divides the plane (8 x 16 tiles on a 28 x 28 plane compute 31 % more
 // outputs than the plane has).
 // OUT: bfloat16 outputs, or float32 ones, whose staged patch is float32 too (the affine is not rounded).
 template <int KS, int CG, int NC, int TH, int R, int Q, class OUT>
-__global__ void __launch_bounds__(32 * CG, KS == 7 ? 12 / CG : 1)
+__global__ void __launch_bounds__(32 * CG, KS == 7 ? 12 / CG : 0)
 dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ wk,
                     const float* __restrict__ bias, const float* __restrict__ pre_a,
                     const float* __restrict__ pre_b, OUT* __restrict__ y, int H, int W, int C,
@@ -600,7 +601,7 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
 #pragma unroll 1
   for (int blk = 0; blk < (TH / R) * (NC / Q); ++blk) {
     const int rl = blk / (NC / Q) * R, wl = cgp * NC + blk % (NC / Q) * Q;       // first row and column inside the tile
-    if (w0 + wl >= W) continue;
+    if (w0 + wl >= W || (TH > R && h0 + rl >= H)) continue;
     unsigned long long acc[R][Q];
 #pragma unroll
     for (int o = 0; o < R; ++o)
@@ -609,7 +610,7 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
     const OUT* src = tile + ((size_t)rl * PW + wl) * CS + 2 * cp;
 #pragma unroll
     for (int ir = 0; ir < R + KS - 1; ++ir) {
-      constexpr int NL = KS == 3 ? Q + KS - 1 : 1;                               // values read together
+      constexpr int NL = KS == 3 || Q == 1 ? Q + KS - 1 : 1;                               // values read together
 #pragma unroll
       for (int j0 = 0; j0 < Q + KS - 1; j0 += NL) {
         unsigned long long xv[NL];
@@ -640,11 +641,13 @@ dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
 #pragma unroll
     for (int o = 0; o < R; ++o) {
       const int h = h0 + rl + o;
-      if (h >= H) break;
+      if (h >= H) {
+        if constexpr (KS == 7) break; else continue;
+      }
       OUT* yo = y + (((size_t)n * H + h) * W + w0 + wl) * C + cs0 + 2 * cp;
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
-        if (w0 + wl + q >= W) break;
+        if (Q > 1 && w0 + wl + q >= W) break;
         float va, vb;
         upk2(acc[o][q], va, vb);
         if (gelu) gelu_tanh_x2(va, vb);
