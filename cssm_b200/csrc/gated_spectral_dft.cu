@@ -115,13 +115,22 @@ __global__ void __launch_bounds__(NT, 512 / NT) gated_spectral_dft(const GatedDf
   }
 }
 
-// Planes per CTA, register tiles and threads: the estimate adds up, for a wave of CTAs, the time of the four
-// passes of a step (throughput of the SM, or the latency of a pass when its tiles do not fill the threads)
-// and a fixed part for the loads and barriers.  The constants were fitted to 40 shapes of the gated kernel and 19 of the
-// gated DeltaNet's, 1 x 14 x 14 to 16 x 8 x 56 x 56 (100 to 170 choices each): the times that it picks are 1.6 % above the best
-// of all choices in the mean and 5.4 % below those with one register tile for all passes; two of the 59 are above them, by a microsecond or two.
-// (Fitted on 148 SMs; another device's count takes the place of that number.)  The search is a few
-// microseconds of host time, so each thread remembers its last few answers: a pure function of the key.
+// Planes per CTA, register tiles and threads: the estimate adds up, for a wave of CTAs, the time of the four passes of a step (from the
+// throughput of the SM and the latency of a pass when its tiles do not fill the threads) and a fixed part for the loads and barriers.
+// The constants were fitted to measured times of all choices (on 148 SMs; another device's count takes the place of that number): 40
+// shapes of the gated kernel and 19 of the gated DeltaNet's for DP_FEW; 750 of the delta rules for DP_MANY, which has the groups of nine
+// planes and more (key dimension 3 and 4).  Those often leave one CTA of eight warps an SM, where throughput and latency both count
+// (the root of their squares); with the larger of the two 1 x 4 cells were taken there, 3 % behind 2 x 4 or 1 x 8 (31 x 8 x 39 x 39 x 32,
+// dk = 4: 466 us, now 450).  307 other shapes of dk 3 and 4: 0.991 of the times with DP_FEW; of key dimension 1 and 2 as many lose as gain.
+struct DpTileCost { int r, y; double per, lat, epi; };      // cells; clocks: SM time of a tile and step, latency of a step, of an epilogue
+struct DpModel { DpTileCost heavy[2], light[4]; double border, cell, step, plane, wide; bool both; };
+static constexpr DpModel DP_FEW = {{{1, 2, 0.11, 34.7, 198}, {2, 4, 0.0501, 39, 954}},
+                                   {{1, 2, 0.082, 36, 216}, {1, 4, 0.123, 37.9, 304}, {2, 4, 0.272, 78.5, 478}, {1, 8, 0.224, 77.2, 427}},
+                                   0.185, 0.0108, 455, 0.252, 1.03, false};
+static constexpr DpModel DP_MANY = {{{1, 2, 0.0235, 29.8, 219}, {2, 4, 0.00509, 18.6, 171}},
+                                    {{1, 2, 0.0474, 38.9, 130}, {1, 4, 0.0791, 48.7, 352}, {2, 4, 0.268, 44.6, 955}, {1, 8, 0.295, 60.5, 518}},
+                                    0.65, 0.0104, 1890, 0.181, 1.038, true};
+// The search is a few microseconds of host time, so each thread remembers its last few answers: a pure function of the key.
 DpChoice dp_choose(int H, int W, int C, int B, int unit, int back, size_t limit, size_t (*bytes)(const DpGeom&, int, int), int arg) {
   struct Memo { int H, W, C, B, unit, back, arg, sms; size_t limit; size_t (*bytes)(const DpGeom&, int, int); DpChoice c; };
   static thread_local Memo memo[8] = {};
@@ -131,6 +140,7 @@ DpChoice dp_choose(int H, int W, int C, int B, int unit, int back, size_t limit,
       m.limit == limit)
     return m.c;
   const DpGeom g = dp_geom(H, W);
+  const DpModel& dm = unit < 9 ? DP_FEW : DP_MANY;
   DpChoice best;
   best.P = 0; best.cost = 1e30; best.tiles = 0; best.ctas = 1; best.smem = 0;
   for (int P = unit; P <= C && P <= 128 * unit; P += unit) {
@@ -140,23 +150,19 @@ DpChoice dp_choose(int H, int W, int C, int B, int unit, int back, size_t limit,
     for (int v = 0; v < 2 * DP_TILES; ++v) {
       const int tiles = v >> 1, nt = v & 1 ? 256 : 128;
       const int fit = (int)((227 * 1024) / (smem + 1024)), most = 512 / nt, occ = fit > most ? most : (fit < 1 ? 1 : fit);
-      // clocks: SM time of a tile and reduction step, latency of a step, of an epilogue
-      struct Tile { int r, y; double per, lat, epi; };
-      static constexpr Tile HEAVY[2] = {{1, 2, 0.11, 34.7, 198}, {2, 4, 0.0501, 39, 954}};
-      static constexpr Tile LIGHT[4] = {{1, 2, 0.082, 36, 216}, {1, 4, 0.123, 37.9, 304}, {2, 4, 0.272, 78.5, 478}, {1, 8, 0.224, 77.2, 427}};
-      const Tile h = HEAVY[tiles >= 2], l = LIGHT[tiles >= 2 ? tiles - 1 : tiles];
+      const DpTileCost &h = dm.heavy[tiles >= 2], &l = dm.light[tiles >= 2 ? tiles - 1 : tiles];
       auto up = [](int a, int b) { return (a + b - 1) / b; };
-      auto pass = [&](const Tile& t, int X, int Y, double q) {
+      auto pass = [&](const DpTileCost& t, int X, int Y, double q) {
         const int nx = up(X, t.r);                 // (a warp on the border of two rows of tiles reads two table entries)
         const double n = (double)nx * up(Y, t.y);
-        const double thr = q * n * (Y * t.per * (1 + 0.185 * 32 / nx) + 0.0108 * t.r * t.y), ltn = ceil(n / nt) * (Y * t.lat + t.epi);
-        return thr > ltn ? thr : ltn;
+        const double thr = q * n * (Y * t.per * (1 + dm.border * 32 / nx) + dm.cell * t.r * t.y), ltn = ceil(n / nt) * (Y * t.lat + t.epi);
+        return dm.both ? sqrt(thr * thr + ltn * ltn) : thr > ltn ? thr : ltn;
       };
       const double resident = groups < (double)sms * occ ? ceil(groups / sms) : occ;
       const int Q = P / back;
       const double step = pass(l, P * g.Hp, g.Wp, resident) + pass(h, P * g.Wp, g.Hp, resident) + pass(l, Q * g.Wp, g.Hp, resident) +
-                          pass(l, Q * g.Hp, g.Wp, resident) + 455 + 0.252 * resident * P * H * W;
-      const double cost = ceil(groups / (sms * resident)) * step * (nt > 128 ? 1.03 : 1.0);
+                          pass(l, Q * g.Hp, g.Wp, resident) + dm.step + dm.plane * resident * P * H * W;
+      const double cost = ceil(groups / (sms * resident)) * step * (nt > 128 ? dm.wide : 1.0);
       if (cost < best.cost) { best.cost = cost; best.P = P; best.tiles = tiles; best.ctas = occ; best.threads = nt; best.smem = smem; }
     }
   }
