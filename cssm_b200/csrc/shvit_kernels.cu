@@ -496,13 +496,14 @@ dwconv_cl_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ 
 // 512 x 56 x 56 x 64 362 -> 317 us, 33 x 64 x 64 x 64 45 -> 41 with 4 x 4, 512 x 28 x 28 x 128 190 -> 184; 4 x 7 blocks spill (329).
 // 3 x 3 is bound by memory: bigger blocks only lost warps (512 x 14 x 14 x 1024 111 -> 117), but for the float32 patch of
 // 14 x 14 planes (48 x 256 channels 16.4 -> 12.3).  Its launch bounds name no number of CTAs: one cost up to ten registers a thread, and rows
-// past the plane are passed over, not left by (24 x 13 x 13 x 1024 12.3 -> 10.3, float32 outputs 10 x 69 x 69 x 64 10.1 -> 8.6).
+// past the plane are passed over, not left by (24 x 13 x 13 x 1024 12.3 -> 10.3, float32 outputs 10 x 69 x 69 x 64 10.1 -> 8.6).  The 4 x 4 tiles of
+// few images, of which an SM has few anyway, do better with the registers (pass of one 224-pixel image 208.2 -> 207.2).
 // Tile geometry as template parameters: CG column groups (32 * CG threads), NC columns per group, TH rows;
 // the launcher picks one that divides the plane (8 x 16 tiles on a 28 x 28 plane compute 31 % more
 // outputs than the plane has).
 // OUT: bfloat16 outputs, or float32 ones, whose staged patch is float32 too (the affine is not rounded).
 template <int KS, int CG, int NC, int TH, int R, int Q, class OUT>
-__global__ void __launch_bounds__(32 * CG, KS == 7 ? 12 / CG : 0)
+__global__ void __launch_bounds__(32 * CG, KS == 7 ? 12 / CG : TH == 4 ? 1 : 0)
 dwconv_tiled_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ wk,
                     const float* __restrict__ bias, const float* __restrict__ pre_a,
                     const float* __restrict__ pre_b, OUT* __restrict__ y, int H, int W, int C,
