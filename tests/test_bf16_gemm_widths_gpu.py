@@ -5,7 +5,7 @@ import pytest
 import torch
 import torch.nn.functional as F
 
-from cssm_b200 import CSSMSHViT, device_error, lib
+from cssm_b200 import CSSMSHViT, CssmError, device_error, lib
 from cssm_b200._lib import check
 from oracle import cssm_oracle as orc
 from oracle import shvit_oracle as sv
@@ -53,6 +53,12 @@ def test_long_bias_off_sixteen_bytes():
     """Copied to shared memory whatever its alignment, at the cost of a stage."""
     _gemm(5000, 640, 640, 0, True, bias_offset=1)
     _gemm(2400, 2048, 512, 0, True, bias_offset=3)
+
+
+def test_long_bias_read_in_place_has_to_be_aligned():
+    """Beyond 2048 columns the bias is read from global memory, sixteen bytes at a time: refused on the host otherwise."""
+    with pytest.raises(CssmError):
+        _gemm(5000, 64, 2304, 0, False, bias_offset=1)
 
 
 def test_default_widths():
