@@ -184,17 +184,17 @@ __device__ __forceinline__ void tc_mma3_small(uint32_t d, uint32_t a, uint64_t b
 // Weights W[k][n] of a (64, N) matrix times scale[k] -> three parts of N rows, K-major swizzled
 template <int N>
 __device__ __forceinline__ void tc_split3_weights(const float* Wk, const float* scale, unsigned char* b, int tid, int threads) {
-  for (int item = tid; item < N * 8; item += threads) {
-    const int n = item % N, c = item / N;               // c: 16-byte chunk of 8 k values
-    uint32_t p[3][4];
+  for (int item = tid; item < N * 16; item += threads) {
+    const int n = item % N, c = item / N;               // c: half of a 16-byte chunk, 4 k values
+    float w[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int k = 8 * c + 2 * e;
-      split3(Wk[(size_t)k * N + n] * scale[k], Wk[(size_t)(k + 1) * N + n] * scale[k + 1], p[0][e], p[1][e], p[2][e]);
-    }
+    for (int e = 0; e < 4; ++e) w[e] = Wk[(size_t)(4 * c + e) * N + n] * scale[4 * c + e];
+    uint32_t p[3][2];
+    split3(w[0], w[1], p[0][0], p[1][0], p[2][0]);
+    split3(w[2], w[3], p[0][1], p[1][1], p[2][1]);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
-      *reinterpret_cast<uint4*>(b + (uint32_t)i * (N * 128u) + tc::sw128_offset(n, c)) = make_uint4(p[i][0], p[i][1], p[i][2], p[i][3]);
+      *reinterpret_cast<uint2*>(b + (uint32_t)i * (N * 128u) + tc::sw128_offset(n, c >> 1) + (c & 1) * 8u) = make_uint2(p[i][0], p[i][1]);
   }
 }
 
