@@ -611,7 +611,8 @@ int cssm_simple_forward_host_pipelined(const cssm_simple_desc* d, const cssm_sim
  * shvit.py:165-180; cssm.py:481, 584 inside a bf16 model):
  *   out (M,N) bf16 = act(A (M,K) bf16 @ kernel (K,N) + bias) [+ res (M,N) bf16]
  * `wt` is the kernel packed by cssm_bf16_pack_weight: (N, ldw) bf16, ldw = cssm_bf16_packed_ld(K).
- * act: 0 none, 1 gelu (tanh form, jax.nn.gelu's default), 2 silu.  K and N multiples of 32. */
+ * act: 0 none, 1 gelu (tanh form, jax.nn.gelu's default), 2 silu.  K and N multiples of 32.  `bias` may be NULL;
+ * more than 2048 values have to start on 16 bytes (CSSM_ERR_ALIGN). */
 int32_t cssm_bf16_packed_ld(int32_t K);
 int cssm_bf16_pack_weight(const float* kernel, int32_t K, int32_t N, const float* col_scale,
                           void* wt, void* stream);

@@ -83,3 +83,25 @@ def test_several_tiles_a_cta(M, K, N, act):
     """No residual, more tiles than SMs: accumulators, ring and slots come round; an odd number of 64-column boxes, which the two warps of a
     quadrant take in turn; a bias from global memory; direct stores (160 columns)."""
     _gemm(M, K, N, act, False)
+
+
+@pytest.mark.parametrize("B,H,Cin,Cout,act", [(256, 28, 64, 576, 0), (260, 27, 64, 576, 1), (20, 28, 128, 960, 0)])
+def test_conv_of_192_column_tiles(B, H, Cin, Cout, act):
+    """The strided conv at widths of 192-column tiles whose bias would take the fourth stage: seven tiles a CTA, and fewer."""
+    L = lib()
+    st = torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(B + Cout)
+    x = torch.randn((B, H, H, Cin), device="cuda", generator=g).to(torch.bfloat16)
+    W = torch.randn((3, 3, Cin, Cout), device="cuda", generator=g) / (9 * Cin) ** 0.5
+    b = torch.randn((Cout,), device="cuda", generator=g)
+    wt = torch.empty((Cout, L.cssm_bf16_conv3x3s2_packed_ld(Cin, H, Cout)), dtype=torch.bfloat16, device="cuda")
+    check(L.cssm_bf16_pack_conv3x3s2_weight(W.data_ptr(), Cin, Cout, H, None, wt.data_ptr(), st), "pack")
+    Ho = (H + 1) // 2
+    out = torch.full((B, Ho, Ho, Cout), float("nan"), dtype=torch.bfloat16, device="cuda")
+    check(L.cssm_bf16_conv3x3s2(x.data_ptr(), B, H, H, Cin, wt.data_ptr(), Cout, b.data_ptr(), act, out.data_ptr(), st), "conv")
+    # 'SAME' of stride 2: one row and column of zeros behind an even plane, one on each side of an odd one
+    xp = F.pad(x.double().permute(0, 3, 1, 2), (0, 1, 0, 1) if H % 2 == 0 else (1, 1, 1, 1))
+    ref = F.conv2d(xp, W.to(torch.bfloat16).double().permute(3, 2, 0, 1), b.double(), stride=2).permute(0, 2, 3, 1)
+    ref = F.gelu(ref, approximate="tanh") if act else ref
+    assert device_error() == 0
+    assert float((out.double() - ref).norm() / ref.norm()) < 3e-3

@@ -78,3 +78,13 @@ def test_full_batches(kind, B, T, H, W, C):
         p = orc.init_gdn_params(1, C, H, W, bias_scale=0.1, perturb_rms=True, delta_key_dim=2, kernel_size=1, gate_type="factored")
         _check(GatedDeltaNetCSSM(channels=C, delta_key_dim=2, **kw).apply({"params": p}, xd),
                orc.gdn_forward(p, x, delta_key_dim=2, **kw)[idx])
+
+
+@pytest.mark.parametrize("B,T,H,W,C,dk", [(31, 2, 39, 39, 32, 4), (9, 1, 28, 28, 48, 3), (40, 2, 16, 8, 64, 4), (7, 3, 47, 22, 24, 3), (2, 2, 58, 34, 64, 4)])
+def test_full_batches_of_long_keys(B, T, H, W, C, dk):
+    """Key dimension 3 and 4, whose tiles have an estimate of their own: one CTA of eight warps an SM, and several."""
+    x = np.random.default_rng(H + W + C).standard_normal((min(B, 2), T, H, W, C)).astype(np.float32)
+    idx = np.arange(B) % len(x)
+    kw = dict(kernel_size=1, rope_mode="none", gate_type="factored", delta_key_dim=dk)
+    p = orc.init_gdn_params(1, C, H, W, bias_scale=0.1, perturb_rms=True, kernel_size=1, gate_type="factored", delta_key_dim=dk)
+    _check(GatedDeltaNetCSSM(channels=C, **kw).apply({"params": p}, torch.from_numpy(x[idx]).cuda()), orc.gdn_forward(p, x, **kw)[idx])
