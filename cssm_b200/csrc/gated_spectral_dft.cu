@@ -1,4 +1,4 @@
-// Fused spectral kernel of the gated block for planes of any size (64x64 and 32x32 have their own):
+// Fused spectral kernel of the gated block for planes of any size (64x64, 32x32 and most square ones have their own):
 // rfft2 -> gated recurrence over T -> irfft2 -> * silu(z), on the folded-DFT products of dft_plane.cuh.
 //
 // A CTA takes P consecutive channels of one batch element and walks t = 0 .. T-1 with their state in
@@ -186,8 +186,10 @@ static auto pick_kernel(const DpChoice& ch) {
 
 int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat, const float* gates, float* xz,
                               int last_only, int mode, cudaStream_t st, const float* dchan, int equal_steps) {
+  if (equal_steps > 0 && mode != 0) return CSSM_ERR_UNSUPPORTED;
+  if (gated_spectral_fft_takes(B, T, H, W, C)) return launch_gated_spectral_fft(B, T, H, C, khat, gates, xz, last_only, mode, st, dchan, equal_steps);
   const DpChoice ch = dp_choose(H, W, C, B, 1, 1, DP_SMEM_LIMIT, gated_dft_bytes, T);
-  if (ch.P == 0 || (equal_steps > 0 && mode != 0)) return CSSM_ERR_UNSUPPORTED;
+  if (ch.P == 0) return CSSM_ERR_UNSUPPORTED;
   GatedDftArgs a;
   memset(&a, 0, sizeof(a));
   a.xz = xz; a.khat = khat; a.gates = reinterpret_cast<const float4*>(gates); a.dchan = dchan;

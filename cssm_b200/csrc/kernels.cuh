@@ -64,6 +64,10 @@ bool gated_spectral_dft_fits(int H, int W, int T);
 // times, and the z planes are those of the first frame of a clip)
 int launch_gated_spectral_dft(int B, int T, int H, int W, int C, const cf* khat, const float* gates, float* xz,
                               int last_only, int mode, cudaStream_t st, const float* dchan, int equal_steps = 0);
+// square planes with whole FFTs in a lane's registers (csrc/gated_spectral_fft.cu); called by launch_gated_spectral_dft
+bool gated_spectral_fft_takes(int B, int T, int H, int W, int C);
+int launch_gated_spectral_fft(int B, int T, int H, int C, const cf* khat, const float* gates, float* xz, int last_only, int mode,
+                              cudaStream_t st, const float* dchan, int equal_steps);
 int read_spec_error(int* out, int clear);
 
 // ---- DeltaNet block (scalar delta rule) ----
