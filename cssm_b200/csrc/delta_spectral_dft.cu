@@ -1,6 +1,7 @@
 // Fused spectral kernels of the two delta-rule blocks (GatedDeltaNetCSSM, DeltaNetCSSM) for planes of any
 // size and key dimensions 1 .. 4, on the folded-DFT products of dft_plane.cuh (64x64 and 32x32 planes
-// with key dimension 4, and DeltaNet's, have kernels of their own).
+// with key dimension 4, and DeltaNet's, have kernels of their own, and so have most square planes with key dimensions 2 and 4,
+// and DeltaNet's: csrc/delta_spectral_fft.cuh).
 //
 // A CTA takes `heads` consecutive heads of one batch element (DeltaNet: channels, key dimension 1): the
 // k, v and q planes of the heads are transformed side by side, their spectra stay in shared memory as
@@ -315,6 +316,10 @@ static int gdn_dft_dk(const GdnSpectralArgs& a, const DeltaDftArgs& d, const DpC
 int launch_gdn_spectral_dft(const GdnSpectralArgs& a, cudaStream_t st) {
   DeltaDftArgs d;
   DpChoice ch;
+  if (a.H == a.W && !a.static_image && (a.dk == 2 || a.dk == 4)) {
+    const int rc = a.dk == 2 ? launch_gdn_spectral_fft2(a, st) : launch_gdn_spectral_fft4(a, st);
+    if (rc != CSSM_ERR_UNSUPPORTED) return rc;
+  }
   if (!delta_dft_plan(a.B, a.T, a.C, a.H, a.W, a.dk, false, &d, &ch)) return CSSM_ERR_UNSUPPORTED;
   switch (a.dk) {
     case 1: return gdn_dft_dk<1>(a, d, ch, st);
@@ -327,6 +332,10 @@ int launch_gdn_spectral_dft(const GdnSpectralArgs& a, cudaStream_t st) {
 int launch_deltanet_spectral_dft(const DnSpectralArgs& a, cudaStream_t st) {
   DeltaDftArgs d;
   DpChoice ch;
+  if (a.H == a.W) {
+    const int rc = launch_deltanet_spectral_fft(a, st);
+    if (rc != CSSM_ERR_UNSUPPORTED) return rc;
+  }
   if (!delta_dft_plan(a.B, a.T, a.C, a.H, a.W, 1, true, &d, &ch)) return CSSM_ERR_UNSUPPORTED;
   return dp_pick(ch.tiles, [&](auto tl) {
     using TL = decltype(tl);

@@ -127,6 +127,10 @@ struct GdnSpectralArgs {
 int launch_gdn_spectral(const GdnSpectralArgs& a, cudaStream_t st);
 int read_p32_error(int* out, int clear);
 int read_p64_error(int* out, int clear);
+// square planes with whole FFTs in a lane's registers (csrc/gdn_spectral_fft.cuh, csrc/deltanet_spectral_fft.cu); called by launch_*_spectral_dft
+int launch_gdn_spectral_fft2(const GdnSpectralArgs& a, cudaStream_t st);
+int launch_gdn_spectral_fft4(const GdnSpectralArgs& a, cudaStream_t st);
+int launch_deltanet_spectral_fft(const DnSpectralArgs& a, cudaStream_t st);
 int launch_gdn_spectral_dft(const GdnSpectralArgs& a, cudaStream_t st);    // as launch_deltanet_spectral_dft
 size_t gdn_generic_smem_bytes(int H, int W, int dk);
 
