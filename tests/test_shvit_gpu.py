@@ -210,6 +210,20 @@ def test_cfg5_full_batch_picked_samples():
         assert orc.rel_l2(y[b], ref[i]) <= 2e-2, (b, orc.rel_l2(y[b], ref[i]))
 
 
+def test_few_and_many_images():
+    """76 images take the kernels of many (64 channels a CTA in the mixers' spectral kernel, ...), the same images by twos those of few.  Each is
+    some 5.5e-3 from a float64 forward (bf16 roundings that fall the other way), so below sqrt(2) times that of one another."""
+    m = CSSMSHViT(embed_dims=(64, 128, 256, 384), depths=(1, 1, 1, 1), num_classes=10, num_timesteps=1, kernel_sizes=(1, 1, 1, 1),
+                  short_conv_spatial_size=0)
+    p, s = sv.init_shvit_params(3, (224, 224), num_classes=10, short_conv_spatial_size=0, embed_dims=m.embed_dims, depths=m.depths,
+                                kernel_sizes=m.kernel_sizes)
+    b = m.bind({"params": p, "batch_stats": s})
+    x = torch.randn(76, 224, 224, 3, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).cuda()
+    many = b(x).cpu().numpy()
+    few = np.concatenate([b(x[i:i + 2].contiguous()).cpu().numpy() for i in (0, 38, 74)])
+    assert orc.rel_l2(few, many[[0, 1, 38, 39, 74, 75]]) <= 8e-3
+
+
 @pytest.mark.parametrize("C,B,classes", [(1280, 8, 10), (1344, 9, 10), (1536, 8, 6), (1536, 3, 10)])
 def test_head_of_wide_last_stages(C, B, classes):
     """Around and above 1284 channels eight pooled rows and their partial sums leave the 48 KB of shared
