@@ -788,29 +788,108 @@ __device__ __forceinline__ float4 gated_map(float rd, float rb, float rc, int ac
   return make_float4(expf(-D), (D + 1e-8f) * rb, rc * inv, 1e-7f * (D + 1e-8f));
 }
 
-// Factored gates, one frame per CTA row; the bins of a frame are split over gridDim.y CTAs when there are
-// few frames.  (One thread per vector entry walking all C channels: 37 us for one 14 x 14 frame of 256.)
-constexpr int GF_THREADS = 512;
-__global__ void __launch_bounds__(GF_THREADS) gated_gates_factored_kernel(const GatedGateArgs g) {
+// Factored gates of FR frames a CTA (the bins of a frame are split over gridDim.y CTAs when there are few frames).  The entries of the six
+// vectors go to the lanes, four a lane, the channels in S slices to the warps, so that a weight read serves FR frames and a warp's weights are
+// some 16 loads a lane and entry: those of the first 16 channels are on their way before the kernel waits for the one before it (weights are
+// older than the chain).  Then the slices' sums meet in shared memory and all threads write the maps.
+// (Before: one frame a CTA with all loads behind the wait, 12 us of a pass with 33 frames of 16 x 16 x 256, now 5.5; four frames with the
+// matrices copied to shared memory first, 18 us a launch for 192 frames of 14 x 14 x 256, now 6.4.)
+constexpr int GF_THREADS = 512, GF_E = 4, GF_U = 16;
+struct GateSplit { int S, EC; };           // slices of the channels, chunks of 32 * GF_E entries
+template <int FR>
+__global__ void __launch_bounds__(GF_THREADS) gated_gates_factored_kernel(const GatedGateArgs g, const GateSplit q) {
   extern __shared__ __align__(16) float sh[];
-  const int Wf = g.W / 2 + 1, NB = g.H * Wf, per = g.H + Wf;
-  float* ctx = sh;                 // [C]
-  float* vec = sh + g.C;           // 3 x (H + Wf)
-  float* scratch = vec + 3 * per;  // [GF_THREADS]
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf, per = g.H + Wf, E = 3 * per, C = g.C;
+  float* ctx = sh;                          // [C][FR]
+  float* part = sh + C * FR;                // [S][E][FR]
+  float* vec = part + q.S * E * FR;         // [E][FR]
   const float inv = 1.0f / (float)(g.H * g.W);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, f0 = blockIdx.x * FR, nf = min(FR, g.BT - f0);
+  const int step = (GF_THREADS / 32) / q.S, sl = warp % q.S, c0 = sl * C / q.S, c1 = (sl + 1) * C / q.S;
+  auto column = [&](int e, const float*& w, int& ld, const float*& bias) {
+    const int m = e / per, r = e - m * per, h = r < g.H ? 0 : 1, col = h ? r - g.H : r;
+    const float* k = g.gk[0];
+    const float* bp = g.gb[0];
+#pragma unroll
+    for (int i = 1; i < 6; ++i)
+      if (i == 2 * m + h) { k = g.gk[i]; bp = g.gb[i]; }
+    w = k + col; bias = bp + col; ld = h ? Wf : g.H;
+  };
+  const float* wp[GF_E];
+  int ld[GF_E];
+  float w[GF_E][GF_U];
+  auto point = [&](int ec) {
+#pragma unroll
+    for (int i = 0; i < GF_E; ++i) {
+      const float* b;
+      column(min((ec * GF_E + i) * 32 + lane, E - 1), wp[i], ld[i], b);
+    }
+  };
+  auto fetch = [&](int c) {
+#pragma unroll
+    for (int u = 0; u < GF_U; ++u)
+#pragma unroll
+      for (int i = 0; i < GF_E; ++i) w[i][u] = __ldg(wp[i] + (size_t)min(c + u, C - 1) * ld[i]);
+  };
+  int ec = warp / q.S;
+  const bool busy = ec < step && ec < q.EC;
+  point(min(ec, q.EC - 1));
+  fetch(c0);
   pdl_sync();
-  const GateCtxSrc src = {g.ctx_sum, nullptr, nullptr, 1, g.C, g.H, 0, inv};
-  gate_ctx(src, blockIdx.x, 1, ctx, scratch);
-  const int off[7] = {0, g.H, per, per + g.H, 2 * per, 2 * per + g.H, 3 * per};
-  gate_vectors<6>(g.gk, g.gb, off, 6, ctx, g.C, vec, scratch);
-  const int per_cta = (NB + gridDim.y - 1) / gridDim.y;
-  const int bin_end = min(NB, (int)(blockIdx.y + 1) * per_cta);
-  for (int bin = blockIdx.y * per_cta + threadIdx.x; bin < bin_end; bin += GF_THREADS) {
-    const int kh = bin / Wf, kw = bin - kh * Wf;
+  for (int i = tid; i < C * FR; i += GF_THREADS) {
+    const int f = i / C, c = i - f * C;
+    ctx[c * FR + f] = f < nf ? __ldg(g.ctx_sum + (size_t)(f0 + f) * C + c) * inv : 0.f;
+  }
+  __syncthreads();
+  if (busy) {
+    for (bool first = true; ec < q.EC; ec += step, first = false) {
+      if (!first) { point(ec); fetch(c0); }
+      float acc[GF_E][FR];
+#pragma unroll
+      for (int i = 0; i < GF_E; ++i)
+#pragma unroll
+        for (int f = 0; f < FR; ++f) acc[i][f] = 0.f;
+      for (int c = c0; c < c1; c += GF_U) {
+        if (c > c0) fetch(c);
+#pragma unroll
+        for (int u = 0; u < GF_U; ++u) {
+          if (c + u >= c1) break;
+#pragma unroll
+          for (int f = 0; f < FR; ++f) {
+            const float x = ctx[(c + u) * FR + f];
+#pragma unroll
+            for (int i = 0; i < GF_E; ++i) acc[i][f] = fmaf(x, w[i][u], acc[i][f]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < GF_E; ++i) {
+        const int e = (ec * GF_E + i) * 32 + lane;
+        if (e < E) {
+#pragma unroll
+          for (int f = 0; f < FR; ++f) part[(sl * E + e) * FR + f] = acc[i][f];
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < E * FR; i += GF_THREADS) {
+    const int e = i / FR;
+    const float *k, *b;
+    int l;
+    column(e, k, l, b);
+    float v = __ldg(b);
+    for (int t = 0; t < q.S; ++t) v += part[t * E * FR + i];
+    vec[i] = v;
+  }
+  __syncthreads();
+  const int per_cta = (NB + gridDim.y - 1) / gridDim.y, b0 = blockIdx.y * per_cta, nb = min(per_cta, NB - b0);
+  for (int i = tid; i < nf * nb; i += GF_THREADS) {
+    const int f = i / nb, bin = b0 + i - f * nb, kh = bin / Wf, kw = bin - kh * Wf;
     float r[3];
 #pragma unroll
-    for (int gi = 0; gi < 3; ++gi) r[gi] = vec[gi * per + kh] * vec[gi * per + g.H + kw];
-    g.maps[(size_t)blockIdx.x * NB + bin_index(g.path, kh, kw, g.H, Wf)] = gated_map(r[0], r[1], r[2], g.act, inv);
+    for (int gi = 0; gi < 3; ++gi) r[gi] = vec[(gi * per + kh) * FR + f] * vec[(gi * per + g.H + kw) * FR + f];
+    g.maps[(size_t)(f0 + f) * NB + bin_index(g.path, kh, kw, g.H, Wf)] = gated_map(r[0], r[1], r[2], g.act, inv);
   }
 }
 
@@ -834,93 +913,20 @@ __global__ void __launch_bounds__(128) gated_gates_dense_kernel(const GatedGateA
     if (f < nf) g.maps[(size_t)(f0 + f) * NB + o] = gated_map(r[0][f], r[1][f], r[2][f], g.act, inv);
 }
 
-// Factored gates of many frames with small planes (the CSSM-SHViT stages: hundreds of frames of
-// 14x14 / 7x7).  A CTA takes GB_FR frames.  It first copies the six gate matrices (C x H and C x Wf
-// each, at most ~100 KB) to shared memory with every thread's 16-byte loads all in flight at once (a
-// walk through them with a few loads per thread in flight is a chain of cold misses: 31 us); then a
-// thread computes whole gate-vector entries (one dot product over the C channels) and the bins are
-// written.
-constexpr int GB_FR = 4;
-__global__ void __launch_bounds__(256) gated_gates_batched_kernel(const GatedGateArgs g) {
-  pdl_sync();
-  extern __shared__ __align__(16) float sh[];
-  const int Wf = g.W / 2 + 1, NB = g.H * Wf, per = g.H + Wf;
-  const int nH = g.C * g.H, nW = g.C * Wf;           // floats per matrix (multiples of 4: C % 4 == 0)
-  float* wsm = sh;                         // six matrices as they lie in memory: [gate][H part | Wf part]
-  float* ctx = wsm + 3 * (nH + nW);        // [GB_FR][C]
-  float* vec = ctx + GB_FR * g.C;          // [GB_FR][3][per]: the H then the Wf entries of each gate
-  const int tid = threadIdx.x;
-  const int f0 = blockIdx.x * GB_FR;
-  const int nf = g.BT - f0 < GB_FR ? g.BT - f0 : GB_FR;
-  const float inv = 1.0f / (float)(g.H * g.W);
-  {
-    const int q4H = nH / 4, q4W = nW / 4, tot4 = 3 * (q4H + q4W);
-    for (int i0 = tid; i0 < tot4; i0 += 16 * 256) {
-      float4 v[16];
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int i = i0 + u * 256;
-        if (i < tot4) {
-          const int gi = i / (q4H + q4W), r = i - gi * (q4H + q4W);
-          v[u] = r < q4H ? __ldg(reinterpret_cast<const float4*>(g.gk[2 * gi]) + r)
-                         : __ldg(reinterpret_cast<const float4*>(g.gk[2 * gi + 1]) + (r - q4H));
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int i = i0 + u * 256;
-        if (i < tot4) reinterpret_cast<float4*>(wsm)[i] = v[u];
-      }
-    }
-  }
-  for (int i = tid; i < nf * g.C; i += blockDim.x) ctx[i] = g.ctx_sum[(size_t)f0 * g.C + i] * inv;
-  __syncthreads();
-  for (int idx = tid; idx < nf * 3 * per; idx += blockDim.x) {
-    const int f = idx / (3 * per), o = idx - f * 3 * per;
-    const int gi = o / per, col = o - gi * per;
-    const bool wpart = col >= g.H;
-    const int cc = wpart ? col - g.H : col, ncol = wpart ? Wf : g.H;
-    const float* src = wsm + gi * (nH + nW) + (wpart ? nH : 0) + cc;
-    const float* cx = ctx + f * g.C;
-    float acc[4] = {g.gb[2 * gi + (wpart ? 1 : 0)][cc], 0.f, 0.f, 0.f};
-    int c = 0;
-    for (; c + 4 <= g.C; c += 4) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) acc[u] = fmaf(cx[c + u], src[(c + u) * ncol], acc[u]);
-    }
-    for (; c < g.C; ++c) acc[0] = fmaf(cx[c], src[c * ncol], acc[0]);
-    vec[idx] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-  }
-  __syncthreads();
-  for (int idx = tid; idx < nf * NB; idx += blockDim.x) {
-    const int f = idx / NB, bin = idx - f * NB;
-    const int kh = bin / Wf, kw = bin - kh * Wf;
-    const float* v = vec + f * 3 * per;
-    float r[3];
-#pragma unroll
-    for (int gi = 0; gi < 3; ++gi) r[gi] = v[gi * per + kh] * v[gi * per + g.H + kw];
-    g.maps[(size_t)(f0 + f) * NB + bin_index(g.path, kh, kw, g.H, Wf)] = gated_map(r[0], r[1], r[2], g.act, inv);
-  }
-}
-
 int launch_gated_gates(const GatedGateArgs& g, cudaStream_t st) {
-  const int Wf = g.W / 2 + 1;
-  {
-    const size_t per = (size_t)g.H + Wf;
-    const size_t bsm = ((size_t)3 * g.C * per + (size_t)GB_FR * (g.C + 3 * per)) * sizeof(float);
-    bool al = g.C % 4 == 0;
-    for (int i = 0; i < 6; ++i) al = al && aligned16(g.gk[i]);
-    if (g.gate_type == CSSM_GATE_FACTORED && g.BT >= 64 && g.H * Wf <= 256 && bsm <= 160 * 1024 && al) {
-      cudaError_t e = func_smem(gated_gates_batched_kernel, bsm);
-      if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-      launch_k(gated_gates_batched_kernel, (g.BT + GB_FR - 1) / GB_FR, 256, bsm, st, g);
-      return check_launch();
-    }
-  }
-  const int NB = g.H * Wf;
+  const int Wf = g.W / 2 + 1, NB = g.H * Wf;
   if (g.gate_type == CSSM_GATE_FACTORED) {
-    const size_t smem = (size_t)(g.C + 3 * (g.H + Wf) + GF_THREADS) * sizeof(float);
-    return launch_gates(gated_gates_factored_kernel, dim3(g.BT, gate_chunks(g.BT, NB)), GF_THREADS, smem, st, g);
+    const int E = 3 * (g.H + Wf), sms = sm_count();
+    GateSplit q;
+    q.EC = (E + 32 * GF_E - 1) / (32 * GF_E);
+    q.S = q.EC < GF_THREADS / 32 ? GF_THREADS / 32 / q.EC : 1;
+    // Frames a CTA: the classifier's pass with 1, 2, 4: 32 images 488, 490, 492 us; 48 images of T = 8 (192 frames) 774, 762, 765; 256
+    // images 1922, 1911, 1912; 512 3590, 3565, 3552.
+    const int FR = g.BT >= 3 * sms ? 4 : g.BT >= sms ? 2 : 1;
+    const size_t smem = (size_t)FR * (g.C + (q.S + 1) * E) * sizeof(float);
+    const dim3 grid((g.BT + FR - 1) / FR, gate_chunks((g.BT + FR - 1) / FR, NB));
+    return launch_gates(FR == 4 ? gated_gates_factored_kernel<4> : FR == 2 ? gated_gates_factored_kernel<2> : gated_gates_factored_kernel<1>, grid,
+                        GF_THREADS, smem, st, g, q);
   }
   const int chunks = (NB + 127) / 128, G = gate_dense_frames(g.BT, chunks, g.C);
   const dim3 grid((g.BT + G - 1) / G, chunks);

@@ -869,99 +869,126 @@ int launch_layernorm_cl(const __nv_bfloat16* x, const float* scale, const float*
 }
 
 // ------------------------------------------------------------------ LayerNorm over a sample ----
-// Moments over all H*W*C values of each sample (two passes over the L2-resident sample), written as
-// the per-(sample, channel) affine the consumer applies on load:
+// Moments over all H*W*C values of each sample, written as the per-(sample, channel) affine the consumer applies on load:
 //   a[n, c] = rstd_n * scale[c],  b[n, c] = bias[c] - mean_n * rstd_n * scale[c].
-__global__ void __launch_bounds__(512)
+// A thread holds its first SN_U chunks of eight values in registers, all of their loads in flight at once (one at a time and read twice
+// by 512 threads before: 33 samples of 16 x 16 x 256 8.5 -> 5.4 us of a pass); what is beyond them is read a second time for the squares
+// about the mean.
+constexpr int SN_U = 8, SN_THREADS = 1024;
+__global__ void __launch_bounds__(SN_THREADS)
 sample_norm_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ scale,
                    const float* __restrict__ bias, float* __restrict__ a, float* __restrict__ b, int per,
                    int C) {
   pdl_sync();
-  __shared__ float red[16];
-  __shared__ float bc;
-  const int n = blockIdx.x;
+  __shared__ float red[2][32];
+  const int n = blockIdx.x, tid = threadIdx.x;
   const uint4* xs = reinterpret_cast<const uint4*>(x + (size_t)n * per);
   const int chunks = per / 8;
-  auto block_sum = [&](float s) {
+  auto block_sum = [&](float s, int k) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((tid & 31) == 0) red[k][tid >> 5] = s;
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float t = 0.f;
-      for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[i];
-      bc = t;
-    }
-    __syncthreads();
-    return bc;
+    float t = (tid & 31) < SN_THREADS / 32 ? red[k][tid & 31] : 0.f;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
   };
+  uint4 r[SN_U];
+#pragma unroll
+  for (int u = 0; u < SN_U; ++u) r[u] = __ldg(xs + min(tid + u * SN_THREADS, chunks - 1));
   float s = 0.f;
-  for (int i = threadIdx.x; i < chunks; i += blockDim.x) {
+#pragma unroll
+  for (int u = 0; u < SN_U; ++u) {
+    if (tid + u * SN_THREADS >= chunks) break;
+    float v[8];
+    unpack8(r[u], v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += v[j];
+  }
+#pragma unroll 4
+  for (int i = tid + SN_U * SN_THREADS; i < chunks; i += SN_THREADS) {
     float v[8];
     unpack8(__ldg(xs + i), v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) s += v[j];
   }
-  const float mean = block_sum(s) / (float)per;
+  const float mean = block_sum(s, 0) / (float)per;
   float q = 0.f;
-  for (int i = threadIdx.x; i < chunks; i += blockDim.x) {
+#pragma unroll
+  for (int u = 0; u < SN_U; ++u) {
+    if (tid + u * SN_THREADS >= chunks) break;
+    float v[8];
+    unpack8(r[u], v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { const float d = v[j] - mean; q = fmaf(d, d, q); }
+  }
+#pragma unroll 4
+  for (int i = tid + SN_U * SN_THREADS; i < chunks; i += SN_THREADS) {
     float v[8];
     unpack8(__ldg(xs + i), v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) { const float d = v[j] - mean; q = fmaf(d, d, q); }
   }
-  const float rstd = rsqrtf(block_sum(q) / (float)per + 1e-6f);
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    const float sc = rstd * scale[c];
+  const float rstd = rsqrtf(block_sum(q, 1) / (float)per + 1e-6f);
+  for (int c = tid; c < C; c += SN_THREADS) {
+    const float sc = rstd * __ldg(scale + c);
     a[(size_t)n * C + c] = sc;
-    b[(size_t)n * C + c] = bias[c] - mean * sc;
+    b[(size_t)n * C + c] = __ldg(bias + c) - mean * sc;
   }
 }
 int launch_sample_norm(const __nv_bfloat16* x, const float* scale, const float* bias, float* a, float* b,
                        int Nimg, int per, int C, cudaStream_t st) {
   if (per % 8 != 0) return CSSM_ERR_UNSUPPORTED;
-  launch_k(sample_norm_kernel, Nimg, 512, 0, st, x, scale, bias, a, b, per, C);
+  launch_k(sample_norm_kernel, Nimg, SN_THREADS, 0, st, x, scale, bias, a, b, per, C);
   return check_launch();
 }
 
 // ------------------------------------------------------------------ plane sums ----
 // sums[n, c] = sum over the P pixels of x[n, p, c] (x has row stride ld): thread = 8 channels of a
-// slice of the pixels; deterministic order.
-__global__ void __launch_bounds__(256)
+// slice of the pixels, four loads in flight; deterministic order.  (32 slices: with eight one to 16 images are 2 % of a pass slower.)
+constexpr int PS_SLICES = 32;
+__global__ void __launch_bounds__(32 * PS_SLICES)
 plane_sum_cl_kernel(const __nv_bfloat16* __restrict__ x, int ld, int P, int C, float* __restrict__ sums) {
   pdl_sync();
-  __shared__ float part[8][33][8];
-  const int chunks = C / 8;                          // blockDim.x = 32 chunk lanes, blockDim.y = 8 pixel slices
+  __shared__ float part[PS_SLICES][32][8];
+  const int chunks = C / 8;                          // blockDim.x = 32 chunk lanes, blockDim.y = PS_SLICES pixel slices
   const int n = blockIdx.y, ck = blockIdx.x * 32 + threadIdx.x;
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
   if (ck < chunks) {
     const __nv_bfloat16* xp = x + (size_t)n * P * ld + ck * 8;
-    for (int p = threadIdx.y; p < P; p += 8) {
-      float v[8];
-      unpack8(__ldg(reinterpret_cast<const uint4*>(xp + (size_t)p * ld)), v);
+    for (int p = threadIdx.y; p < P; p += 4 * PS_SLICES) {
+      uint4 r[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += v[j];
+      for (int u = 0; u < 4; ++u) r[u] = __ldg(reinterpret_cast<const uint4*>(xp + (size_t)min(p + u * PS_SLICES, P - 1) * ld));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (p + u * PS_SLICES >= P) break;
+        float v[8];
+        unpack8(r[u], v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += v[j];
+      }
     }
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) part[threadIdx.y][threadIdx.x][j] = acc[j];
   __syncthreads();
-  if (threadIdx.y == 0 && ck < chunks) {
+  // 256 values of PS_SLICES partial sums
+  const int t = threadIdx.y * 32 + threadIdx.x;
+  if (t < 256 && blockIdx.x * 32 + t / 8 < chunks) {
+    float v = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float t = 0.f;
-      for (int s = 0; s < 8; ++s) t += part[s][threadIdx.x][j];
-      sums[(size_t)n * C + ck * 8 + j] = t;
-    }
+    for (int s = 0; s < PS_SLICES; ++s) v += part[s][t / 8][t % 8];
+    sums[(size_t)n * C + (blockIdx.x * 32) * 8 + t] = v;
   }
 }
 int launch_plane_sum_cl(const __nv_bfloat16* x, int ld, int Nimg, int P, int C, float* sums, cudaStream_t st) {
   if (C % 8 != 0 || ld % 8 != 0) return CSSM_ERR_UNSUPPORTED;
-  dim3 grid((C / 8 + 31) / 32, Nimg), block(32, 8);
-  launch_k(plane_sum_cl_kernel, grid, block, 0, st, x, ld, P, C, sums);
+  const dim3 grid((C / 8 + 31) / 32, Nimg);
+  launch_k(plane_sum_cl_kernel, grid, dim3(32, PS_SLICES), 0, st, x, ld, P, C, sums);
   return check_launch();
 }
 
@@ -995,20 +1022,24 @@ __global__ void __launch_bounds__(256)
 head_slice_kernel(const float* __restrict__ pooled, const float* __restrict__ W, const float* __restrict__ b,
                   float* __restrict__ logits, int Nimg, int C, int K) {
   extern __shared__ __align__(16) float ps[];        // [NS][C], then [8][NS][32] partial sums
-  pdl_sync();
   const int n0 = blockIdx.y * NS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < NS * C; i += 256) ps[i] = n0 + i / C < Nimg ? __ldg(pooled + (size_t)n0 * C + i) : 0.f;
-  float* part = ps + NS * C;
   const int k = blockIdx.x * 32 + lane, kc = min(k, K - 1);
   const int per = ((C + 7) / 8 + 3) / 4 * 4, c0 = warp * per, c1 = min(C, c0 + per);      // C % 4 == 0
+  float w[16];
+  auto fetch = [&](int c) {
+#pragma unroll
+    for (int u = 0; u < 16; ++u) w[u] = c + u < c1 ? __ldg(W + (size_t)(c + u) * K + kc) : 0.f;
+  };
+  fetch(c0);                                         // (weights are older than the chain of launches)
+  pdl_sync();
+  for (int i = threadIdx.x; i < NS * C; i += 256) ps[i] = n0 + i / C < Nimg ? __ldg(pooled + (size_t)n0 * C + i) : 0.f;
+  float* part = ps + NS * C;
   float acc[NS];
 #pragma unroll
   for (int j = 0; j < NS; ++j) acc[j] = 0.f;
   __syncthreads();
   for (int c = c0; c < c1; c += 16) {
-    float w[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) w[u] = c + u < c1 ? __ldg(W + (size_t)(c + u) * K + kc) : 0.f;
+    if (c > c0) fetch(c);
 #pragma unroll
     for (int u = 0; u < 16; u += 4) {
       if (c + u >= c1) continue;
