@@ -58,8 +58,20 @@ __device__ __forceinline__ float rcp_fast(float d) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
   return r;
 }
-__device__ __forceinline__ float silu_f(float v) { return v * rcp_fast(1.0f + __expf(-v)); }
-__device__ __forceinline__ float sigmoid_f(float v) { return rcp_fast(1.0f + __expf(-v)); }
+// e^v and log v without the scaling of subnormal results and arguments that the intrinsics wrap around the same instructions (three more
+// each): for sums 1 + e^v, which subnormals do not change, and logarithms of at least 1.
+__device__ __forceinline__ float exp_ftz(float v) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v * 1.44269504088896340736f));
+  return r;
+}
+__device__ __forceinline__ float log_ftz(float v) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r * 0.69314718055994530942f;
+}
+__device__ __forceinline__ float silu_f(float v) { return v * rcp_fast(1.0f + exp_ftz(-v)); }
+__device__ __forceinline__ float sigmoid_f(float v) { return rcp_fast(1.0f + exp_ftz(-v)); }
 
 // n / d for 0 <= n < 2^31 by one multiply-high with d's rounded-up reciprocal, 2^l >= d (division by invariant integers,
 // Granlund and Montgomery 1994).

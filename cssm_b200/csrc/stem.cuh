@@ -5,7 +5,7 @@
 namespace cssm {
 
 __device__ __forceinline__ float softplus_f(float a) {
-  return fmaxf(a, 0.f) + __logf(1.0f + __expf(-fabsf(a)));
+  return fmaxf(a, 0.f) + log_ftz(1.0f + exp_ftz(-fabsf(a)));
 }
 
 struct StemArgs {
