@@ -300,7 +300,8 @@ __global__ void __launch_bounds__(STEMW_THREADS) stem_layer_wide_kernel(const St
 // before, each weight vector was read for four multiply-adds and every value crossed the window by two shuffles); LayerNorm
 // sums cross the quad by two shuffles a pixel, and the window maximum stays in the lane.
 // Bound: the two special-function calls of softplus and about a dozen packed or scalar operations a conv output.
-// 128 images of 128x128: 265 -> 157 us; 128 clips of 32 frames of 32x32x3, pointwise: 301 -> 219 us (write floor 165).
+// 128 images of 128x128: 265 -> 157 us; 128 clips of 32 frames of 32x32x3, pointwise: 301 -> 219 us (write floor 165).  Softplus without the
+// intrinsics' subnormal scaling, sums and normalisation packed, the window's maximum before scale and bias: 156 -> 140, 217 -> 206.
 constexpr int STEMQ_THREADS = 256;
 template <int KS, int POOL, int CIN, int NG>
 __global__ void __launch_bounds__(STEMQ_THREADS, 2) stem_quad_kernel(const StemArgs a) {
@@ -316,6 +317,9 @@ __global__ void __launch_bounds__(STEMQ_THREADS, 2) stem_quad_kernel(const StemA
   const unsigned total = (unsigned)a.N * a.Ho * a.Wo, units = POOL == 2 ? total : (total + 3) / 4;
   const float4* w4 = reinterpret_cast<const float4*>(sm);
   const float4* v4 = reinterpret_cast<const float4*>(vec);
+  bool negative = false;                                     // a scale of this CTA's channels, the same for all its threads
+  if (POOL == 2)
+    for (int c = 0; c < C; ++c) negative = negative || vec[C + c] < 0.f;
   for (unsigned u0 = (blockIdx.x * (STEMQ_THREADS / 32) + (tid >> 5)) * 8; u0 < units; u0 += gridDim.x * STEMQ_THREADS / 4) {
     const unsigned u = u0 + (lane >> 2);
     const bool valid = u < units;
@@ -367,47 +371,71 @@ __global__ void __launch_bounds__(STEMQ_THREADS, 2) stem_quad_kernel(const StemA
           }
         }
     // softplus, LayerNorm over the quad's channels (moments of the values minus the pixel's first channel: layer_norm_regs)
-    float mx[NG][4];
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      float v[NG][4], s = 0.f, ss = 0.f;
-#pragma unroll
-      for (int k = 0; k < NG; ++k) {
-        upk2(acc[p][2 * k], v[k][0], v[k][1]);
-        upk2(acc[p][2 * k + 1], v[k][2], v[k][3]);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) v[k][e] = softplus_f(v[k][e]);
-      }
-      const float vref = __shfl_sync(0xffffffffu, v[0][0], lane & ~3);
+    float mx[NG][4], mn[NG][4];                              // of the normalised values before scale and bias
+    if (POOL == 2) {
 #pragma unroll
       for (int k = 0; k < NG; ++k)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) { v[k][e] -= vref; s += v[k][e]; ss = fmaf(v[k][e], v[k][e], ss); }
+        for (int e = 0; e < 4; ++e) { mx[k][e] = -INFINITY; mn[k][e] = INFINITY; }
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      float v0 = 0.f;
+#pragma unroll
+      for (int k = 0; k < 2 * NG; ++k) {
+        float x0, x1;
+        upk2(acc[p][k], x0, x1);
+        x0 = softplus_f(x0); x1 = softplus_f(x1);
+        if (k == 0) v0 = x0;
+        acc[p][k] = pk2(x0, x1);
+      }
+      const float vref = -__shfl_sync(0xffffffffu, v0, lane & ~3);
+      const unsigned long long ref2 = pk2(vref, vref);
+      unsigned long long s2 = 0ull, ss2 = 0ull;
+#pragma unroll
+      for (int k = 0; k < 2 * NG; ++k) {
+        acc[p][k] = add2(acc[p][k], ref2);
+        s2 = add2(s2, acc[p][k]);
+        ss2 = fma2(acc[p][k], acc[p][k], ss2);
+      }
+      float s, ss, sb, ssb;
+      upk2(s2, s, sb); upk2(ss2, ss, ssb);
+      s += sb; ss += ssb;
       s += __shfl_xor_sync(0xffffffffu, s, 1);  ss += __shfl_xor_sync(0xffffffffu, ss, 1);
       s += __shfl_xor_sync(0xffffffffu, s, 2);  ss += __shfl_xor_sync(0xffffffffu, ss, 2);
       const float mean = s / (float)C, rinv = rsqrtf(fmaxf(ss / (float)C - mean * mean, 0.f) + 1e-6f);
-      const bool inb = POOL == 1 || (h0 + (p >> 1) < a.Hin && w0 + (p & 1) < a.Win);      // else 'SAME' pool padding on odd sizes
+      const unsigned long long r2 = pk2(rinv, rinv), m2 = pk2(-mean, -mean);
+      if (POOL == 1) {
+        const size_t px = (size_t)uc * 4 + p;
 #pragma unroll
-      for (int k = 0; k < NG; ++k) {
-        const float4 sc = v4[C / 4 + g + 4 * k], lb = v4[C / 2 + g + 4 * k];
-        const float4 y = make_float4((v[k][0] - mean) * rinv * sc.x + lb.x, (v[k][1] - mean) * rinv * sc.y + lb.y,
-                                     (v[k][2] - mean) * rinv * sc.z + lb.z, (v[k][3] - mean) * rinv * sc.w + lb.w);
-        if (POOL == 1) {
-          const size_t px = (size_t)uc * 4 + p;
+        for (int k = 0; k < NG; ++k) {
+          const float4 sc = v4[C / 4 + g + 4 * k], lb = v4[C / 2 + g + 4 * k];
+          float4 y;
+          upk2(fma2(mul2(add2(acc[p][2 * k], m2), r2), pk2(sc.x, sc.y), pk2(lb.x, lb.y)), y.x, y.y);
+          upk2(fma2(mul2(add2(acc[p][2 * k + 1], m2), r2), pk2(sc.z, sc.w), pk2(lb.z, lb.w)), y.z, y.w);
           if (valid && px < total) *reinterpret_cast<float4*>(a.out + px * C + 4 * (g + 4 * k)) = y;
-        } else {
-          // fmaxf ignores a NaN: a window keeps its other pixels
-          mx[k][0] = fmaxf(p == 0 ? -INFINITY : mx[k][0], inb ? y.x : -INFINITY);
-          mx[k][1] = fmaxf(p == 0 ? -INFINITY : mx[k][1], inb ? y.y : -INFINITY);
-          mx[k][2] = fmaxf(p == 0 ? -INFINITY : mx[k][2], inb ? y.z : -INFINITY);
-          mx[k][3] = fmaxf(p == 0 ? -INFINITY : mx[k][3], inb ? y.w : -INFINITY);
+        }
+      } else if (h0 + (p >> 1) < a.Hin && w0 + (p & 1) < a.Win) {      // else 'SAME' pool padding on odd sizes
+        // (fmaxf and fminf ignore a NaN: a window keeps its other pixels)
+#pragma unroll
+        for (int k = 0; k < 2 * NG; ++k) {
+          float t0, t1;
+          upk2(mul2(add2(acc[p][k], m2), r2), t0, t1);
+          float &a0 = mx[k >> 1][2 * (k & 1)], &a1 = mx[k >> 1][2 * (k & 1) + 1], &b0 = mn[k >> 1][2 * (k & 1)], &b1 = mn[k >> 1][2 * (k & 1) + 1];
+          a0 = fmaxf(a0, t0); a1 = fmaxf(a1, t1);
+          if (negative) { b0 = fminf(b0, t0); b1 = fminf(b1, t1); }
         }
       }
     }
     if (POOL == 2 && valid) {
+      // the largest of scale * t + bias over the window is at the largest t, or the smallest where the scale is negative
       float4* op = reinterpret_cast<float4*>(a.out + (size_t)uc * C);
 #pragma unroll
-      for (int k = 0; k < NG; ++k) op[g + 4 * k] = make_float4(mx[k][0], mx[k][1], mx[k][2], mx[k][3]);
+      for (int k = 0; k < NG; ++k) {
+        const float4 sc = v4[C / 4 + g + 4 * k], lb = v4[C / 2 + g + 4 * k];
+        auto pick = [&](float f, float b, int e) { return f == 0.f ? b : fmaf(f < 0.f ? mn[k][e] : mx[k][e], f, b); };
+        op[g + 4 * k] = make_float4(pick(sc.x, lb.x, 0), pick(sc.y, lb.y, 1), pick(sc.z, lb.z, 2), pick(sc.w, lb.w, 3));
+      }
     }
   }
 }
@@ -609,43 +637,49 @@ struct ReadoutArgs {
 };
 
 // grid (bands, B): LayerNorm/softplus of (y + res) per pixel, pooled over the band's pixels.
-// Four lanes per pixel as in the stem (lane g owns float4 groups g + 4k); 8 pixels per warp.
-__global__ void __launch_bounds__(RO_THREADS) readout_pool_kernel(const ReadoutArgs a) {
+// Four lanes per pixel as in the stem (lane g owns float4 groups g + 4k); 8 pixels per warp, the loads of the next eight on their way.
+// Few CTAs have 32 warps, so that a band of 8 x 32 pixels is one step (8 images of 32 x 32 10.3 -> 6.0 us of a pass).
+template <int NT>
+__global__ void __launch_bounds__(NT) readout_pool_kernel(const ReadoutArgs a) {
   pdl_sync();
-  __shared__ float red[RO_THREADS / 32][SM_MAXC];
+  __shared__ float red[NT / 32][SM_MAXC];
   __shared__ float vec[2 * SM_MAXC];
   const int C = a.C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int band = blockIdx.x, b = blockIdx.y;
-  for (int i = tid; i < C; i += RO_THREADS) { vec[i] = a.pre_scale[i]; vec[SM_MAXC + i] = a.pre_bias[i]; }
-  __syncthreads();
   const int g = lane & 3, ps = lane >> 2, ngrp = C >> 2;
   const int h0 = band * RO_ROWS, rows = min(RO_ROWS, a.H - h0);
   const int npx = rows * a.W;
+  float4 yv[4], rv[4];
+  auto fetch = [&](int p0) {                        // (past the end the last pixel again)
+    const size_t px = (size_t)h0 * a.W + min(p0 + ps, npx - 1);
+    const float4* yp = reinterpret_cast<const float4*>(a.y + (size_t)b * a.y_stride + px * C);
+    const float4* rp = reinterpret_cast<const float4*>(a.res + (size_t)b * a.res_stride + px * C);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int j = min(g + 4 * k, ngrp - 1);
+      yv[k] = __ldg(yp + j); rv[k] = __ldg(rp + j);
+    }
+  };
+  fetch(warp * 8);
+  for (int i = tid; i < C; i += NT) { vec[i] = a.pre_scale[i]; vec[SM_MAXC + i] = a.pre_bias[i]; }
+  __syncthreads();
   const float init = a.pool_max ? -INFINITY : 0.f;
   float pool[4][4];
 #pragma unroll
   for (int k = 0; k < 4; ++k)
 #pragma unroll
     for (int e = 0; e < 4; ++e) pool[k][e] = init;
-  for (int p0 = warp * 8; p0 < npx; p0 += (RO_THREADS / 32) * 8) {      // uniform per warp
-    const int p = p0 + ps;
-    const bool on = p < npx;
-    const size_t px = (size_t)h0 * a.W + (on ? p : 0);
-    const float4* yp = reinterpret_cast<const float4*>(a.y + (size_t)b * a.y_stride + px * C);
-    const float4* rp = reinterpret_cast<const float4*>(a.res + (size_t)b * a.res_stride + px * C);
+  for (int p0 = warp * 8; p0 < npx; p0 += (NT / 32) * 8) {      // uniform per warp
+    const bool on = p0 + ps < npx;
     float v[4][4];
     float s = 0.f, ss = 0.f;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int j = g + 4 * k;
-      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (j < ngrp) {
-        const float4 yv = __ldg(yp + j), rv = __ldg(rp + j);
-        t = make_float4(yv.x + rv.x, yv.y + rv.y, yv.z + rv.z, yv.w + rv.w);
-        if (a.norm_post_order) t = make_float4(softplus_f(t.x), softplus_f(t.y), softplus_f(t.z), softplus_f(t.w));
-      }
+      float4 t = make_float4(yv[k].x + rv[k].x, yv[k].y + rv[k].y, yv[k].z + rv[k].z, yv[k].w + rv[k].w);
+      if (a.norm_post_order) t = make_float4(softplus_f(t.x), softplus_f(t.y), softplus_f(t.z), softplus_f(t.w));
       v[k][0] = t.x; v[k][1] = t.y; v[k][2] = t.z; v[k][3] = t.w;
     }
+    fetch(p0 + (NT / 32) * 8);
     // moments of the values minus the pixel's first channel (see layer_norm_regs)
     const float vref = __shfl_sync(0xffffffffu, v[0][0], lane & ~3);
 #pragma unroll
@@ -688,42 +722,52 @@ __global__ void __launch_bounds__(RO_THREADS) readout_pool_kernel(const ReadoutA
   __syncthreads();
   if (tid < C) {
     float r = red[0][tid];
-    for (int w = 1; w < RO_THREADS / 32; ++w) r = a.pool_max ? fmaxf(r, red[w][tid]) : r + red[w][tid];
+#pragma unroll
+    for (int w = 1; w < NT / 32; ++w) r = a.pool_max ? fmaxf(r, red[w][tid]) : r + red[w][tid];
     a.partial[((size_t)b * a.bands + band) * C + tid] = r;
   }
 }
 
-// grid B, 64 threads: combine the band partials, LayerNorm (norm_post), Dense head
+// grid B, 64 threads: combine the band partials, LayerNorm (norm_post), Dense head.  The head's weights of a class are on their way before
+// the wait for the pooling (they are older than the chain of launches).
 __global__ void __launch_bounds__(SM_MAXC) readout_head_kernel(const ReadoutArgs a) {
-  pdl_sync();
   __shared__ float v[SM_MAXC];
-  __shared__ float stats[2];
-  const int C = a.C, tid = threadIdx.x, b = blockIdx.x;
-  float r = 0.f;
-  if (tid < C) {
-    r = a.partial[(size_t)b * a.bands * C + tid];
-    for (int k = 1; k < a.bands; ++k) {
-      const float o = a.partial[((size_t)b * a.bands + k) * C + tid];
-      r = a.pool_max ? fmaxf(r, o) : r + o;
-    }
-    if (!a.pool_max) r /= (float)(a.H * a.W);
-    v[tid] = r;
+  __shared__ float part[2][2];
+  const int C = a.C, tid = threadIdx.x, b = blockIdx.x, cls = min(tid, a.ncls - 1), ct = min(tid, C - 1);
+  float hk[SM_MAXC];
+#pragma unroll
+  for (int c = 0; c < SM_MAXC; ++c) hk[c] = c < C ? __ldg(a.head_k + (size_t)c * a.ncls + cls) : 0.f;
+  const float hb = __ldg(a.head_b + cls), sc = __ldg(a.post_scale + ct), bi = __ldg(a.post_bias + ct);
+  pdl_sync();
+  const float* pp = a.partial + (size_t)b * a.bands * C + ct;
+  float r = pp[0];
+  for (int k0 = 1; k0 < a.bands; k0 += 8) {
+    float o[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) o[u] = pp[(size_t)min(k0 + u, a.bands - 1) * C];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (k0 + u < a.bands) r = a.pool_max ? fmaxf(r, o[u]) : r + o[u];
   }
+  if (!a.pool_max) r /= (float)(a.H * a.W);
+  v[tid] = r;
   __syncthreads();
-  if (tid == 0) {
-    float s = 0.f, ss = 0.f;
-    const float vref = v[0];
-    for (int c = 0; c < C; ++c) { const float d = v[c] - vref; s += d; ss = fmaf(d, d, ss); }
-    const float mean = s / (float)C;
-    stats[0] = mean + vref;
-    stats[1] = rsqrtf(fmaxf(ss / (float)C - mean * mean, 0.f) + 1e-6f);
-  }
+  // moments of the values minus the first one (see layer_norm_regs)
+  const float vref = v[0], d = tid < C ? r - vref : 0.f;
+  float s = d, ss = d * d;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) { s += __shfl_xor_sync(0xffffffffu, s, o); ss += __shfl_xor_sync(0xffffffffu, ss, o); }
+  if ((tid & 31) == 0) { part[0][tid >> 5] = s; part[1][tid >> 5] = ss; }
   __syncthreads();
-  if (tid < C) v[tid] = (v[tid] - stats[0]) * stats[1] * a.post_scale[tid] + a.post_bias[tid];
+  s = part[0][0] + part[0][1]; ss = part[1][0] + part[1][1];
+  const float mean = s / (float)C, rinv = rsqrtf(fmaxf(ss / (float)C - mean * mean, 0.f) + 1e-6f);
+  v[tid] = (r - (mean + vref)) * rinv * sc + bi;
   __syncthreads();
   if (tid < a.ncls) {
-    float acc = a.head_b[tid];
-    for (int c = 0; c < C; ++c) acc = fmaf(v[c], a.head_k[(size_t)c * a.ncls + tid], acc);
+    float acc = hb;
+#pragma unroll
+    for (int c = 0; c < SM_MAXC; ++c)
+      if (c < C) acc = fmaf(v[c], hk[c], acc);
     a.logits[(size_t)b * a.ncls + tid] = acc;
   }
 }
@@ -876,9 +920,11 @@ static int run_readout(const cssm_simple_desc* d, const cssm_simple_weights* w, 
     smem = spread_smem(0, (long long)a.bands * d->B);
     if (smem < 32 * 1024) smem = 32 * 1024;
   }
-  const cudaError_t e = func_smem(readout_pool_kernel, smem);
+  const bool few = (long long)a.bands * d->B <= sm_count();
+  auto kern = few ? readout_pool_kernel<1024> : readout_pool_kernel<RO_THREADS>;
+  const cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  launch_k(readout_pool_kernel, dim3(a.bands, d->B), RO_THREADS, smem, st, a);
+  launch_k(kern, dim3(a.bands, d->B), few ? 1024 : RO_THREADS, smem, st, a);
   int s = check_launch();
   if (s != CSSM_OK) return s;
   launch_k(readout_head_kernel, d->B, SM_MAXC, 0, st, a);

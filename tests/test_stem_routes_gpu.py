@@ -67,3 +67,17 @@ def test_first_layer_of_few_and_many_pixels(stem, shape):
     got = m.bind({"params": p}).stem(torch.from_numpy(x).cuda()).cpu().numpy()
     ref = np.asarray(so.stem_forward(p, x.reshape(-1, *shape[-3:]).astype(np.float64), stem_mode=stem, stem_layers=1)).reshape(got.shape)
     assert orc.rel_l2(got, ref) <= 5e-6
+
+
+# a window's largest value is at the smallest normalised one where a channel's scale is negative, and its bias where it is zero
+@pytest.mark.parametrize("E", [32, 64])
+@pytest.mark.parametrize("shape", [(2, 17, 24, 1), (1, 16, 15, 3), (4, 96, 98, 1)])
+def test_scales_of_any_sign(E, shape):
+    _, p, _ = _model(E, 1, shape)
+    rng = np.random.default_rng(shape[1])
+    p["norm1"]["scale"] = (rng.standard_normal(E) * (np.arange(E) % 7 != 3)).astype(np.float32)
+    b = SimpleCSSM(cssm_type="gated", embed_dim=E, kernel_size=1, pos_embed="none", seq_len=1, stem_layers=1, gate_type="factored",
+                   pool_type="max").bind({"params": p})
+    x = rng.standard_normal(shape).astype(np.float32)
+    ref = np.asarray(so.stem_forward(p, x.astype(np.float64), stem_mode="default", stem_layers=1))
+    assert orc.rel_l2(b.stem(torch.from_numpy(x).cuda()).cpu().numpy().reshape(ref.shape), ref) <= 5e-6
