@@ -224,18 +224,18 @@ __global__ void __launch_bounds__(ST_THREADS) plane_stencil_kernel(const Stencil
   }
 }
 
-// Fast path of the plane stencil for 64x64 and 32x32 planes: float4 loads with the next
+// Fast path of the plane stencil for rows of whole float4 groups: float4 loads with the next
 // step's plane prefetched into registers, the temporal history in registers, the spatial
 // conv from a zero-haloed shared tile, per-step sums reduced once at the end.
-// NP = float4 groups per thread = H*W / 1024.
-template <int KSP, int KT, int NP>
-__global__ void __launch_bounds__(ST_THREADS) plane_stencil_fast_kernel(const StencilArgs s) {
+// NP = float4 groups per thread = H*W / 1024; ANY: planes of any size with W % 4 == 0, blockDim.x threads and groups past the end of the plane.
+template <int KSP, int KT, int NP, bool ANY>
+__global__ void __launch_bounds__(ANY ? 512 : ST_THREADS) plane_stencil_fast_kernel(const StencilArgs s) {
   pdl_sync();
   extern __shared__ __align__(16) float sm[];
-  const int H = s.H, W = s.W, HW = H * W;
+  const int H = s.H, W = s.W, HW = H * W, nt = ANY ? blockDim.x : ST_THREADS, nw = nt >> 5, groups = HW >> 2;
   const int RS = W + 8;                              // tile row stride (4-float pad each side)
   float* tile = sm;                                  // [(H+2)][RS], used when KSP > 0
-  float* red = sm + (KSP > 0 ? (H + 2) * RS : 0);    // [T][8] per-warp partial sums
+  float* red = sm + (KSP > 0 ? (H + 2) * RS : 0);    // [T][warps] per-warp partial sums
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int b = blockIdx.x / s.C, c = blockIdx.x % s.C;
   constexpr int NHIST = KT > 0 ? KT - 1 : 0;
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(ST_THREADS) plane_stencil_fast_kernel(const St
   }
   const float btv = KT > 0 ? s.bt[c] : 0.f;
   if (KSP > 0) {
-    for (int i = tid; i < (H + 2) * RS; i += ST_THREADS) tile[i] = 0.f;
+    for (int i = tid; i < (H + 2) * RS; i += nt) tile[i] = 0.f;
   }
   float4 hist[NP][NHIST > 0 ? NHIST : 1];
 #pragma unroll
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(ST_THREADS) plane_stencil_fast_kernel(const St
   bool left_edge[NP], right_edge[NP];
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
-    const int g4 = tid + j * ST_THREADS;
+    const int g4 = ANY ? min(tid + j * nt, groups - 1) : tid + j * nt;
     cur[j] = reinterpret_cast<const float4*>(p0)[g4];
     const int h = g4 / gpr, gc = g4 - h * gpr;
     toff[j] = (h + 1) * RS + 4 + gc * 4;
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(ST_THREADS) plane_stencil_fast_kernel(const St
     if (t + 1 < s.T) {
 #pragma unroll
       for (int j = 0; j < NP; ++j)
-        nxt[j] = reinterpret_cast<const float4*>(p + pstride)[tid + j * ST_THREADS];
+        nxt[j] = reinterpret_cast<const float4*>(p + pstride)[ANY ? min(tid + j * nt, groups - 1) : tid + j * nt];
     }
     if (KSP > 0) {
 #pragma unroll
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(ST_THREADS) plane_stencil_fast_kernel(const St
     float4 outv[NP];
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
-      const int g4 = tid + j * ST_THREADS;
+      const int g4 = tid + j * nt;
       float4 v = cur[j];
       if (KSP == 3) {
         // 3x3: the row's float4 from the tile, its left / right neighbours from the adjacent
@@ -352,19 +352,20 @@ __global__ void __launch_bounds__(ST_THREADS) plane_stencil_fast_kernel(const St
       }
       if (s.act) { o.x = silu_f(o.x); o.y = silu_f(o.y); o.z = silu_f(o.z); o.w = silu_f(o.w); }
       if (s.post) {
-        const float* pp = s.post + ((size_t)(b * s.T + t) * HW + (size_t)g4 * 4) * s.post_stride + s.post_off;
+        const float* pp = s.post + ((size_t)(b * s.T + t) * HW + (size_t)(ANY ? min(g4, groups - 1) : g4) * 4) * s.post_stride + s.post_off;
         o.x *= pp[0]; o.y *= pp[s.post_stride]; o.z *= pp[2 * s.post_stride]; o.w *= pp[3 * s.post_stride];
       }
       outv[j] = o;
-      lsum += (o.x + o.y) + (o.z + o.w);
+      if (!ANY || g4 < groups) lsum += (o.x + o.y) + (o.z + o.w);
     }
     // stores after all shared-memory reads of this step (generic-pointer stores would otherwise
     // pin the following loads behind them)
 #pragma unroll
-    for (int j = 0; j < NP; ++j) reinterpret_cast<float4*>(p)[tid + j * ST_THREADS] = outv[j];
+    for (int j = 0; j < NP; ++j)
+      if (!ANY || tid + j * nt < groups) reinterpret_cast<float4*>(p)[tid + j * nt] = outv[j];
     if (s.sums) {
       for (int off = 16; off > 0; off >>= 1) lsum += __shfl_down_sync(0xffffffffu, lsum, off);
-      if (lane == 0) red[t * 8 + warp] = lsum;
+      if (lane == 0) red[t * nw + warp] = lsum;
     }
     if (KSP > 0) __syncthreads();      // all conv reads done before the tile is overwritten
 #pragma unroll
@@ -372,10 +373,9 @@ __global__ void __launch_bounds__(ST_THREADS) plane_stencil_fast_kernel(const St
   }
   if (s.sums) {
     __syncthreads();
-    for (int t = tid; t < s.T; t += ST_THREADS) {
+    for (int t = tid; t < s.T; t += nt) {
       float tot = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) tot += red[t * 8 + w];
+      for (int w = 0; w < nw; ++w) tot += red[t * nw + w];
       s.sums[(size_t)(b * s.T + t) * s.C + c] = tot;
     }
   }
@@ -388,6 +388,7 @@ __global__ void __launch_bounds__(ST_THREADS) plane_stencil_fast_kernel(const St
 // requests the next frame's pixels before it works on this one.  With 3x3 taps its pixels are a strip of a
 // column, so that a tile value read from shared memory serves up to three of them; the tile has a zero
 // halo and there are two in turn (one barrier per frame).
+// (Larger planes of rows of whole float4 groups: the fast path above.)
 // Bound: instruction issue and the shared-memory reads of the taps (floor 8 bytes a pixel: 24 us here).
 // 48 x 8 frames of 14x14x256, 3x3 and four taps: 365 us by the walk above, 121 with pixels dealt out a warp
 // wide, 73 as strips; 16 x 8 x 56x56 x 32: 100 -> 65 us.
@@ -537,13 +538,14 @@ static int launch_stencil_small(const StencilArgs& s, cudaStream_t st, bool* han
   return go(plane_stencil_small_kernel<KSP, 8, false>);
 }
 
-template <int KSP, int KT, int NP>
-static int launch_stencil_fast(const StencilArgs& s, cudaStream_t st) {
-  const size_t smem = ((KSP > 0 ? (size_t)(s.H + 2) * (s.W + 8) : 0) + (size_t)s.T * 8) * sizeof(float);
+template <int KSP, int KT, int NP, bool ANY = false>
+static int launch_stencil_fast(const StencilArgs& s, cudaStream_t st, int nt = ST_THREADS) {
+  const size_t smem = ((KSP > 0 ? (size_t)(s.H + 2) * (s.W + 8) : 0) + (size_t)s.T * (nt / 32)) * sizeof(float);
   if (smem > 200 * 1024) return CSSM_ERR_UNSUPPORTED;
-  cudaError_t e = func_smem(plane_stencil_fast_kernel<KSP, KT, NP>, smem);
+  auto kern = plane_stencil_fast_kernel<KSP, KT, NP, ANY>;
+  cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
-  launch_k(plane_stencil_fast_kernel<KSP, KT, NP>, s.B * s.C, ST_THREADS, smem, st, s);
+  launch_k(kern, s.B * s.C, nt, smem, st, s);
   return check_launch();
 }
 
@@ -556,6 +558,27 @@ static int dispatch_stencil_fast(const StencilArgs& s, cudaStream_t st, bool* ha
   if (s.ksp == 0 && s.kt == 0) return launch_stencil_fast<0, 0, NP>(s, st);
   *handled = false;
   return CSSM_OK;
+}
+
+// Rows of whole float4 groups, four temporal taps and 3x3 or no spatial ones: the groups dealt out to a CTA of as few idle threads as can be.
+// From 192 pixels on; below that the form with a plane a warp is as good or better (122 x 8 x 8 x 8 x 64 87 us a pass, 93 so; 173 x 1 x 12 x 12 x 32
+// 38.4, 39.6; but 30 x 8 x 16 x 16 x 64 72.5, 64.4; 3 x 8 x 48 x 48 x 64 85, 71; of 39 shapes from 16 x 16 to 60 x 60 none more than 1 % behind); a
+// single frame, whose CTAs are over before their loads pay, from 1280 on (33 x 1 x 16 x 16 x 256 twice in the classifier: 620 us a pass, 632 so).
+template <int KSP>
+static int launch_stencil_groups(const StencilArgs& s, cudaStream_t st, bool* handled) {
+  const int groups = s.H * s.W / 4;
+  int best = 0, nt = 0;
+  for (int np = 1; np <= 4; ++np) {
+    const int n = ((groups + np - 1) / np + 31) / 32 * 32;
+    if (n > 512) continue;
+    if (best == 0 || n * np < nt * best || (n * np == nt * best && n >= 128)) { best = np; nt = n; }
+  }
+  *handled = best > 0 && groups >= (s.T > 1 ? 48 : 320);
+  if (!*handled) return CSSM_OK;
+  if (best == 1) return launch_stencil_fast<KSP, 4, 1, true>(s, st, nt);
+  if (best == 2) return launch_stencil_fast<KSP, 4, 2, true>(s, st, nt);
+  if (best == 3) return launch_stencil_fast<KSP, 4, 3, true>(s, st, nt);
+  return launch_stencil_fast<KSP, 4, 4, true>(s, st, nt);
 }
 
 // One source frame for a whole clip: the spatial conv is the same for every frame, and frame f of the temporal one sees
@@ -680,6 +703,11 @@ int launch_plane_stencil(const StencilArgs& s, cudaStream_t st) {
     bool handled = false;
     const int rc = s.H * s.W == 4096 ? dispatch_stencil_fast<4>(s, st, &handled)
                                      : dispatch_stencil_fast<1>(s, st, &handled);
+    if (handled) return rc;
+  }
+  if (s.kt == 4 && (s.ksp == 0 || s.ksp == 3) && s.W % 4 == 0 && (reinterpret_cast<uintptr_t>(s.buf) & 15u) == 0) {
+    bool handled = false;
+    const int rc = s.ksp == 3 ? launch_stencil_groups<3>(s, st, &handled) : launch_stencil_groups<0>(s, st, &handled);
     if (handled) return rc;
   }
   if (s.kt == 4 && (s.ksp == 0 || s.ksp == 3)) {
