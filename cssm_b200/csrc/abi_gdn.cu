@@ -297,6 +297,28 @@ int cssm::gdn_forward_internal(const cssm_gdn_desc* d, const cssm_gdn_weights* w
   ga.ab = (float2*)(ws + l.ab); ga.bkv = (float2*)(ws + l.bkv);
   if ((s = launch_gdn_gates(ga, st)) != CSSM_OK) return s;
 
+  // channel gates: spatial gates sigmoid(Conv1x1(rotated x)) -> planes (BT, 2C, H, W): B_k, B_v; k *= B_k, v *= B_v, by this projection
+  // where it multiplies in place, else with the temporal conv where that is one launch, else by a launch of its own
+  const bool gates_in_place = kv_gates_in_place(*d);      // (no gate planes then: gsp has no room)
+  const bool one_conv = !with_conv && d->short_conv_size >= 2 && d->short_conv_size <= 4 && HW % 4 == 0 && HW != 1024;
+  float* gsp = (float*)(ws + l.gsp);
+  auto spatial_gates = [&]() -> int {
+    GemmArgs q;
+    memset(&q, 0, sizeof(q));
+    q.M = BT * HW; q.N = 2 * C; q.K = C; q.HW = HW;
+    q.A = x; q.rope_t = rt; q.rope_h = rh; q.rope_w = rw; q.rope_nz = rnz;
+    if (x_bcast) { q.a_fdiv = d->T; q.a_fmul = 1; q.a_fadd = 0; }
+    q.Wk = (const float*)(pl + p.gw); q.bias = (const float*)(pl + p.gb);      // packed by plan_init
+    q.out = gsp; q.o_planes = 2 * C; q.o_plane0 = 0;
+    q.T = Tdata; q.H = d->H; q.W = d->W;
+    q.out_act = 2; q.act_n0 = 0;
+    if (((size_t)C * HW) % 8 != 0) return CSSM_ERR_UNSUPPORTED;
+    if (gates_in_place) { q.mul = qkv; q.mul_planes = 3 * C; q.mul_plane0 = C; q.mul_n = 2 * C; }
+    return launch_gemm<false, true>(q, st);
+  };
+  const bool gates_first = chan && d->use_input_gates && !gates_in_place && one_conv;
+  if (gates_first && (s = spatial_gates()) != CSSM_OK) return s;
+
   // 5. causal temporal conv + SiLU on q, k, v planes, input gates on k and v
   mark(4, st);
   bool tconv_done = with_conv;
@@ -305,13 +327,13 @@ int cssm::gdn_forward_internal(const cssm_gdn_desc* d, const cssm_gdn_weights* w
   ta.buf = qkv; ta.B = d->B; ta.T = Tdata; ta.C = C; ta.HW = HW; ta.kt = d->short_conv_size;
   for (int i = 0; i < 3; ++i) { ta.wt[i] = w->conv_t_kernel[i]; ta.bt[i] = w->conv_t_bias[i]; }
   ta.bkv = (d->use_input_gates && !chan) ? (const float2*)(ws + l.bkv) : nullptr;
+  ta.gsp = gates_first ? gsp : nullptr;
   if (with_conv && (s = launch_gemm_qkv_tconv(qkv_proj, ta, st)) != CSSM_OK) return s;
   // one elementwise launch over q, k, v where it measured faster than three per-plane launches
   // (64x64 planes: 1.70 -> 1.36 ms on B=128, T=8; at 32x32 the per-plane kernel is ahead)
-  if (!tconv_done && d->short_conv_size >= 2 && d->short_conv_size <= 4 && HW % 4 == 0 && HW != 1024) {
-    s = launch_qkv_temporal_conv(ta, st);
-    if (s == CSSM_OK) tconv_done = true;
-    else if (s != CSSM_ERR_UNSUPPORTED) return s;
+  if (one_conv) {
+    if ((s = launch_qkv_temporal_conv(ta, st)) != CSSM_OK) return s;
+    tconv_done = true;
   }
   for (int i = 0; i < 3 && !tconv_done; ++i) {
     const bool has_post = d->use_input_gates && !chan && i > 0;
@@ -327,23 +349,10 @@ int cssm::gdn_forward_internal(const cssm_gdn_desc* d, const cssm_gdn_weights* w
     if ((s = launch_plane_stencil(sa, st)) != CSSM_OK) return s;
   }
 
-  if (chan && d->use_input_gates) {
-    // spatial gates sigmoid(Conv1x1(rotated x)) -> planes (BT, 2C, H, W): B_k, B_v; k *= B_k, v *= B_v
-    float* gsp = (float*)(ws + l.gsp);
-    memset(&g, 0, sizeof(g));
-    g.M = BT * HW; g.N = 2 * C; g.K = C; g.HW = HW;
-    g.A = x; g.rope_t = rt; g.rope_h = rh; g.rope_w = rw; g.rope_nz = rnz;
-    if (x_bcast) { g.a_fdiv = d->T; g.a_fmul = 1; g.a_fadd = 0; }
-    g.Wk = (const float*)(pl + p.gw); g.bias = (const float*)(pl + p.gb);      // packed by plan_init
-    g.out = gsp; g.o_planes = 2 * C; g.o_plane0 = 0;
-    g.T = Tdata; g.H = d->H; g.W = d->W;
-    g.out_act = 2; g.act_n0 = 0;
-    if (((size_t)C * HW) % 8 != 0) return CSSM_ERR_UNSUPPORTED;
-    const bool in_place = kv_gates_in_place(*d);      // (no gate planes then: gsp has no room)
-    if (in_place) { g.mul = qkv; g.mul_planes = 3 * C; g.mul_plane0 = C; g.mul_n = 2 * C; }
-    if ((s = launch_gemm<false, true>(g, st)) != CSSM_OK) return s;
+  if (chan && d->use_input_gates && !gates_first) {
+    if ((s = spatial_gates()) != CSSM_OK) return s;
     const size_t per_frame4 = (size_t)2 * C * HW / 4, total4 = per_frame4 * BT;
-    if (!in_place) {
+    if (!gates_in_place) {
       launch_k(gdn_kv_gate_kernel, (unsigned)((total4 + 255) / 256), 256, 0, st, qkv, gsp, per_frame4, total4);
       if ((s = check_launch()) != CSSM_OK) return s;
     }

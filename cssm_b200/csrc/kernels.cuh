@@ -33,6 +33,7 @@ struct QkvTconvArgs {
   int B, T, C, HW, kt;
   const float* wt[3]; const float* bt[3];   // short_conv_q/k/v: (kt,1,C), (C)
   const float2* bkv;              // (B*T, H*W) {B_k, B_v} or nullptr (no input gates)
+  const float* gsp;               // planar (B*T, 2C, H*W): factors of the k and v planes, or nullptr (launch_qkv_temporal_conv only)
 };
 struct GemmArgs;
 // the projection that makes those planes and this conv in one launch (csrc/gemm_qkv_tconv.cu)

@@ -735,8 +735,8 @@ int launch_plane_stencil(const StencilArgs& s, cudaStream_t st) {
 // Causal depthwise temporal conv (KT taps) + SiLU + optional per-pixel input gate on the 3C planar
 // planes of q, k and v in ONE elementwise launch: a thread owns four consecutive pixels of one
 // plane and walks t with the KT-1 previous raw values in registers and the next frame's load in
-// flight, so every plane is read once and written once at full occupancy.
-template <int KT>
+// flight, so every plane is read once and written once at full occupancy.  Gate planes (channel gates) are multiplied on the way.
+template <int KT, bool PLANES>
 __global__ void __launch_bounds__(256) qkv_temporal_conv_kernel(const QkvTconvArgs a) {
   pdl_sync();
   const int HW4 = a.HW >> 2;
@@ -754,16 +754,30 @@ __global__ void __launch_bounds__(256) qkv_temporal_conv_kernel(const QkvTconvAr
   for (int j = 0; j < KT; ++j) w[j] = wtp[(size_t)j * a.C + c];
   const float bias = btp[c];
   const int poff = grp - 1;                                   // k: B_k, v: B_v, q: none
-  const bool gated = a.bkv != nullptr && grp > 0;
+  const bool gated = !PLANES && a.bkv != nullptr && grp > 0, planes = PLANES && grp > 0;
   float4 hist[KT - 1];
 #pragma unroll
   for (int k = 0; k < KT - 1; ++k) hist[k] = make_float4(0.f, 0.f, 0.f, 0.f);
   const size_t fstride = (size_t)3 * a.C * HW4;               // float4 units between frames
   float4* ptr = reinterpret_cast<float4*>(a.buf) + ((size_t)b * a.T * 3 * a.C + p) * HW4 + g4;
-  float4 cur = *ptr;
+  const size_t gstride = (size_t)2 * a.C * HW4;
+  const float4* gpl = planes ? reinterpret_cast<const float4*>(a.gsp) + ((size_t)b * a.T * 2 * a.C + p - a.C) * HW4 + g4 : nullptr;
+  constexpr int AH = PLANES ? 2 : 1;                          // frames on their way (two without gate planes: 1.5 % of a pass slower)
+  const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
+  float4 ring[AH], gr[AH];
+#pragma unroll
+  for (int i = 0; i < AH; ++i) {
+    ring[i] = ptr[(size_t)min(i, a.T - 1) * fstride];
+    gr[i] = planes ? __ldg(gpl + (size_t)min(i, a.T - 1) * gstride) : one;
+  }
   for (int t = 0; t < a.T; ++t) {
-    float4 nxt = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (t + 1 < a.T) nxt = ptr[fstride];
+    const float4 cur = ring[0], gc = gr[0];
+#pragma unroll
+    for (int i = 0; i + 1 < AH; ++i) { ring[i] = ring[i + 1]; gr[i] = gr[i + 1]; }
+    if (t + AH < a.T) {
+      ring[AH - 1] = ptr[AH * fstride];
+      if (planes) gr[AH - 1] = __ldg(gpl + (size_t)(t + AH) * gstride);
+    }
     // out[t] = bias + sum_j w[j] * s[t - (KT-1) + j]; hist[k] holds s[t - (KT-1) + k]
     float4 o = make_float4(fmaf(w[KT - 1], cur.x, bias), fmaf(w[KT - 1], cur.y, bias),
                            fmaf(w[KT - 1], cur.z, bias), fmaf(w[KT - 1], cur.w, bias));
@@ -782,9 +796,9 @@ __global__ void __launch_bounds__(256) qkv_temporal_conv_kernel(const QkvTconvAr
       o.x *= poff ? g0.y : g0.x; o.y *= poff ? g0.w : g0.z;
       o.z *= poff ? g1.y : g1.x; o.w *= poff ? g1.w : g1.z;
     }
+    if (planes) { o.x *= gc.x; o.y *= gc.y; o.z *= gc.z; o.w *= gc.w; }
     *ptr = o;
     ptr += fstride;
-    cur = nxt;
   }
 }
 
@@ -792,10 +806,11 @@ int launch_qkv_temporal_conv(const QkvTconvArgs& a, cudaStream_t st) {
   if (a.HW % 4 != 0 || a.kt < 1) return CSSM_ERR_UNSUPPORTED;
   const long long total = (long long)a.B * 3 * a.C * (a.HW >> 2);
   const unsigned grid = (unsigned)((total + 255) / 256);
+  auto go = [&](auto plain, auto planes) { launch_k(a.gsp != nullptr ? planes : plain, grid, 256, 0, st, a); };
   switch (a.kt) {
-    case 2: launch_k(qkv_temporal_conv_kernel<2>, grid, 256, 0, st, a); break;
-    case 3: launch_k(qkv_temporal_conv_kernel<3>, grid, 256, 0, st, a); break;
-    case 4: launch_k(qkv_temporal_conv_kernel<4>, grid, 256, 0, st, a); break;
+    case 2: go(qkv_temporal_conv_kernel<2, false>, qkv_temporal_conv_kernel<2, true>); break;
+    case 3: go(qkv_temporal_conv_kernel<3, false>, qkv_temporal_conv_kernel<3, true>); break;
+    case 4: go(qkv_temporal_conv_kernel<4, false>, qkv_temporal_conv_kernel<4, true>); break;
     default: return CSSM_ERR_UNSUPPORTED;
   }
   return check_launch();
