@@ -15,7 +15,7 @@
 // 4096 42 / 9.6 / 11; it costs less than 1 % (96 x 14 x 14 x 1024, whole block: 1965 -> 1974 us).
 //
 // Persistent kernel, one CTA per SM, 544 threads, warp-specialised:
-//   warps 0-7  producers : 128-row x 64-k A blocks from global memory (channels-last rows with RoPE
+//   warps 0-7  producers : 128-row x 64-k A blocks (of K <= 32 only the half that the MMAs read) from global memory (channels-last rows with RoPE
 //                          applied, or planar planes times scale and gate), fetched one block ahead
 //                          into registers, split, and written into the 128-byte-swizzled K-major
 //                          operand layout of the ring; with streamed weights also the B blocks;
@@ -269,7 +269,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
     // the lane's two chunks inside a part, rows prow0 (+ 32 r)
     const uint32_t dst0 = tc::sw128_offset(prow0, chunk >> 1) + (chunk & 1) * 8;
     const uint32_t dst1 = tc::sw128_offset(prow0, (chunk >> 1) + 4) + (chunk & 1) * 8;
-    const int prow = tid & 127, kh = tid >> 7;
+    const int prow = tid & 127, kh = tid >> 7, kw = g.K <= 32 ? 16 : 32;      // planar: k values of a thread
     const bool rope = !A_PLANAR && g.rope_t != nullptr;
     const bool remap = g.a_fmul != 0 || g.a_fadd != 0;
     auto fetch = [&](int tile, int kb) {
@@ -296,14 +296,15 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
           const float* p = g.A + row * g.K + k0 + chunk * 4;
 #pragma unroll
           for (int hf = 0; hf < 2; ++hf) {
+            if (hf == 1 && k0 + 32 >= g.K) continue;                 // (the MMAs of such a block end before its second half)
             float* v = pre + 16 * hf + 4 * r;
             if (m < g.M && k0 + (chunk + 8 * hf) * 4 < g.K) ld_stream4(p + 32 * hf, v);
             else v[0] = v[1] = v[2] = v[3] = 0.f;
           }
         }
       } else {
-        const int m = m0 + prow, kk = k0 + kh * 32;
-        const int nk = m < g.M ? g.K - kk : 0;             // valid k values from kk on
+        const int m = m0 + prow, kk = k0 + kh * kw;
+        const int nk = m < g.M ? min(g.K - kk, kw) : 0;    // values of this thread from kk on
         const int fo = q.hw.div(min(m, g.M - 1)), px = min(m, g.M - 1) - fo * g.HW;
         const int fr = remap ? q.fdiv.div(fo) * g.a_fmul + g.a_fadd : fo;
         const float* ap = g.A + ((size_t)fr * g.a_planes + g.a_plane0 + kk) * g.HW + px;
@@ -377,6 +378,7 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
         if (__any_sync(0xffffffffu, !tc::mbar_wait(&empty[s], ((it / NS) & 1) ^ 1))) { atomicExch(&g_split_error, 1); break; }
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
+          if (hf == 1 && k0 + 32 >= g.K) continue;
           unsigned char* dst = a_s + (hf ? dst1 : dst0);
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
@@ -399,10 +401,11 @@ gemm_split_kernel(const GemmArgs g, const SplitGeom q, const __grid_constant__ C
         if (__any_sync(0xffffffffu, !tc::mbar_wait(&empty[s], ((it / NS) & 1) ^ 1))) { atomicExch(&g_split_error, 1); break; }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
+          if (8 * c >= kw) continue;
           float v[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) v[e] = GATE ? pre[8 * c + e] * gpre[GATE ? 8 * c + e : 0] : pre[8 * c + e];
-          store_split8(a_s, tc::sw128_offset(prow, kh * 4 + c), GS_A_PART, v);
+          store_split8(a_s, tc::sw128_offset(prow, kh * (kw >> 3) + c), GS_A_PART, v);
         }
         if (g.rms_scale != nullptr && nkb == 0) { ss_s[((tcnt % GS_SS) * 2 + kh) * 128 + prow] = ss; ss = 0.f; }
         if (ntile < num_tiles) fetch(ntile, nkb);
