@@ -8,7 +8,7 @@
 //
 // Bound: instruction issue (46 to 50 % of the slots, shared-memory pipe 34 to 59 %) at the 12 to 20 warps an SM that registers and planes leave.
 // The folded DFT (O(N) work a value, shared-memory operands) it took over from, passes in us, before -> now:
-// gated 16 x 8 x 56 x 56 x 32 343 -> 240, 3 x 8 x 48 x 48 x 64 152 -> 87, 24 x 8 x 28 x 28 x 64 207 -> 142, 64 x 8 x 14 x 14 x 64 140 -> 116, 159 x 8 x 7 x 7 x 64
+// gated 16 x 8 x 56 x 56 x 32 343 -> 236, 3 x 8 x 48 x 48 x 64 152 -> 87, 24 x 8 x 28 x 28 x 64 207 -> 142, 64 x 8 x 14 x 14 x 64 140 -> 116, 159 x 8 x 7 x 7 x 64
 // 108 -> 89; geometric mean over 44 sides and three batches 1.185 times as fast.  On the way (28 x 28, a pass): frames handed from
 // warp to warp along the recurrence 155 to 223 (a step's bins are then one long chain), passes as calls 189 to 290 (callee-saved registers
 // through local memory, which misses L1 beside this much shared memory).
@@ -153,7 +153,9 @@ __global__ void __launch_bounds__(32 * F) __maxnreg__(65536 / 32 / gated_fft_war
 // Registers and shared memory of a kernel decide F and G together with what the waves look like: a batch of frames costs a warp
 // 3.7 clocks an instruction by itself and 0.17 more for every warp on its SM (two points of 16 x 8 x 56 x 56 x 32: 3.5 warps an SM
 // 150 us, ten 90), half of it whatever the number of planes.  On 63 shapes of nine sides F as chosen is within 2 % of the best of 1, 2
-// and 4 but for two (6 %), always 1, 2 or 4 are 1.27, 1.07 (T > 1) and 1.01 times as slow in the mean.
+// and 4 but for two (6 %), always 1, 2 or 4 are 1.27, 1.07 (T > 1) and 1.01 times as slow in the mean.  Three where it saves a tenth
+// by this count, as where four leave an SM short of a CTA: 16 x 8 x 56 x 56 x 32 243 -> 238 us, 54 x 3 x 16 x 16 x 48 52 -> 48; with a
+// smaller margin one shape in seven of 139 loses 2 to 6 %.
 template <int N>
 static int gated_fft_n(GatedFftArgs& a, cudaStream_t st) {
   typedef Pf<N> P;
@@ -163,7 +165,8 @@ static int gated_fft_n(GatedFftArgs& a, cudaStream_t st) {
   int F = 1, ctas = 1, G = 1;
   for (int g = a.C < P::GMAX ? a.C : P::GMAX; g >= 1; g = g > 1 ? (g + 1) / 2 : 0) {
     const long long groups = (long long)a.B * ((a.C + g - 1) / g);
-    for (int f = 1; f <= 4 && (f == 1 || f / 2 < a.T); f *= 2) {
+    for (int f : {1, 2, 4, 3}) {
+      if (f > 1 && f / 2 >= a.T) continue;
       const size_t smem = (size_t)f * g * P::PLANE * 4 + state;
       int c = (int)(227 * 1024 / (smem + 1024));
       if (c * f > warps) c = warps / f;
@@ -171,7 +174,7 @@ static int gated_fft_n(GatedFftArgs& a, cudaStream_t st) {
       const long long slots = (long long)sms * c, full = groups / slots, rest = (groups % slots + sms - 1) / sms;
       const double one = (a.T + f - 1) / f * (0.5 + 0.5 * g / P::GMAX);
       const double cost = one * (full * (3.7 + 0.17 * c * f) + (rest > 0 ? 3.7 + 0.17 * rest * f : 0));
-      if (cost < best * 0.98) { best = cost; F = f; ctas = c; G = g; }
+      if (cost < best * (f == 3 ? 0.9 : 0.98)) { best = cost; F = f; ctas = c; G = g; }
     }
   }
   const int n = (a.C + G - 1) / G;
@@ -181,7 +184,7 @@ static int gated_fft_n(GatedFftArgs& a, cudaStream_t st) {
   const int slots = sms * ctas, grid = a.groups < slots ? a.groups : slots;
   const PdlOff alone(uneven_rounds(a.groups, ctas));
   const size_t smem = spread_smem((size_t)F * a.G * P::PLANE * 4 + state, grid);
-  auto kern = F == 1 ? gated_spectral_fft<N, 1> : F == 2 ? gated_spectral_fft<N, 2> : gated_spectral_fft<N, 4>;
+  auto kern = F == 1 ? gated_spectral_fft<N, 1> : F == 2 ? gated_spectral_fft<N, 2> : F == 3 ? gated_spectral_fft<N, 3> : gated_spectral_fft<N, 4>;
   const cudaError_t e = func_smem(kern, smem);
   if (e != cudaSuccess) { set_cuda_error(e); return CSSM_ERR_CUDA; }
   launch_k(kern, grid, 32 * F, smem, st, a);

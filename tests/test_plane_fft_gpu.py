@@ -52,7 +52,7 @@ def test_sides(n):
 
 # one frame: planes for every SM; many planes: CTAs of one and two frames, several rounds, a last group of fewer planes
 @pytest.mark.parametrize("B,T,n,C", [(40, 1, 8, 24), (60, 1, 7, 24), (60, 1, 14, 12), (30, 1, 28, 12), (40, 1, 56, 4), (200, 3, 8, 52),
-                                     (300, 2, 7, 36), (37, 3, 20, 20), (75, 3, 14, 36), (20, 3, 40, 36), (19, 2, 56, 32)])
+                                     (300, 2, 7, 36), (37, 3, 20, 20), (75, 3, 14, 36), (20, 3, 40, 36), (19, 2, 56, 32), (54, 3, 16, 48)])
 def test_batches(B, T, n, C):
     _gated(B, T, n, C, "factored")
 
