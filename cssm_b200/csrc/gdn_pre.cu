@@ -1,5 +1,6 @@
 // GDN block, kernels ahead of the spectral stage: RoPE + channels-last depthwise conv with
 // per-row context sums, and the gate maps (alpha, beta per frequency bin; B_k, B_v per pixel).
+#include <type_traits>
 #include "kernels.cuh"
 #include "bf16_ops.cuh"
 #include "gates.cuh"
@@ -28,7 +29,7 @@ __device__ __forceinline__ int dw_pos(int col, int c) {
 // to the two channels' weights: with p = conv(w_e, x_e | w_o, x_o) and q = conv(w_e, x_o | w_o, x_e) of the
 // plane rotated by (h, w),  out_e = p_e cos - q_e sin,  out_o = p_o cos + q_o sin.  So a CTA stages and
 // convolves once (two products) for all T frames instead of T times; what is left is the output's write.
-// 5x5, one 64x64 image over eight frames, batch 128, 64 channels: 1021 -> 372 us.
+// 5x5, one 64x64 image over eight frames, batch 128, 64 channels: 1021 -> 372 us; the frames' stores without a bound and an address each 267.
 template <int K, int DW_CG, bool BC>
 __global__ void __launch_bounds__(DW_THREADS, (K <= 5 ? 2 : 1)) rope_dwconv_cl_kernel(const GdnDwArgs a) {
   pdl_sync();
@@ -189,22 +190,28 @@ __global__ void __launch_bounds__(DW_THREADS, (K <= 5 ? 2 : 1)) rope_dwconv_cl_k
               }
           }
         }
-        for (int f = 0; f < a.T; ++f) {
-          const float2 cf2 = rope ? __ldg(&a.rope_t[f * n2 + pi]) : make_float2(1.f, 0.f);
-          const unsigned long long c2 = pk2(cf2.x, cf2.x), s2 = pk2(-cf2.y, cf2.y);
-          float* orow = a.out + ((((size_t)fr * a.T + f) * a.H + h0 + rc) * W + w0) * C + c0 + 2 * pl;
+        // (whole windows, as all are of planes of a multiple of eight rows and even width, without a test at every store)
+        float* orow = a.out + (((size_t)fr * a.T * a.H + h0 + rc) * W + w0) * C + c0 + 2 * pl;
+        const size_t fstep = (size_t)a.H * W * C;
+        const int wc = W * C;
+        auto frames = [&](auto all) {
+          float* o = orow;
+          float2 cn = rope ? __ldg(&a.rope_t[pi]) : make_float2(1.f, 0.f);
+#pragma unroll 1
+          for (int f = 0; f < a.T; ++f, o += fstep) {
+            const float2 cf2 = cn;
+            if (rope && f + 1 < a.T) cn = __ldg(&a.rope_t[(f + 1) * n2 + pi]);
+            const unsigned long long c2 = pk2(cf2.x, cf2.x), s2 = pk2(-cf2.y, cf2.y);
 #pragma unroll
-          for (int r = 0; r < RC; ++r) {
-            if (h0 + rc + r >= a.H) continue;
+            for (int r = 0; r < RC; ++r)
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
-              if (w0 + j < W) {
-                float ox, oy;
-                upk2(fma2(s2, qx[r][j], fma2(c2, p[r][j], bias2)), ox, oy);
-                *reinterpret_cast<float2*>(orow + ((size_t)r * W + j) * C) = make_float2(ox, oy);
-              }
+              for (int j = 0; j < 2; ++j)
+                if (decltype(all)::value || (h0 + rc + r < a.H && w0 + j < W))
+                  *reinterpret_cast<unsigned long long*>(o + r * wc + j * C) = fma2(s2, qx[r][j], fma2(c2, p[r][j], bias2));
           }
-        }
+        };
+        if (h0 + rc + RC <= a.H && w0 + 1 < W) frames(std::true_type());
+        else frames(std::false_type());
       }
       continue;
     }
