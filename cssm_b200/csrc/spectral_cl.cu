@@ -12,7 +12,7 @@
 // 16-byte accesses, so HBM sees x, z and y once each as full rows.
 //
 // Bound at full batches: the FMA pipe (about 27 operations a value).  14 x 14 x 256, 512 images: 7-point DFTs of every row and column by their
-// definition 80 us a launch, lane FFTs of row pairs 54; the classifier's pass 3619 -> 3566 us.  Few images: a thread's chain of transforms, so
+// definition 80 us a launch, lane FFTs of row pairs 50; the classifier's pass 3619 -> 3566 us.  Few images: a thread's chain of transforms, so
 // sixteen channels a CTA with a thread for every row pair and column (one image 209 -> 200 us a pass).
 #include <cuda_fp16.h>
 #include "kernels.cuh"
